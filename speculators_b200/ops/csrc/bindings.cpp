@@ -673,7 +673,7 @@ void ep_pull(const Tensor& src_ptrs, int64_t capacity, const Tensor& src_rank, c
 // ---- tcgen05 GEMM ------------------------------------------------------------------------
 // out[M,N] = a[M,K] @ b[N,K]^T; epilogue 0 = store, 1 = out += result, 2 = result + residual.
 // `status` (int32[1], device) receives a non-zero code if a bounded wait in the kernel ran out.
-// variant: 0 = choose, 1 = one CTA per 128x256 tile, 2 = CTA pairs on 256x256 tiles.
+// variant: 0 = choose; see launch_gemm_impl.
 void gemm_tn_variant(const Tensor& a, const Tensor& b, Tensor out, const c10::optional<Tensor>& residual, int64_t epilogue, Tensor status,
                      int64_t variant) {
   TORCH_CHECK(a.is_cuda() && b.is_cuda() && out.is_cuda() && status.is_cuda());
@@ -706,7 +706,7 @@ void gemm_tn(const Tensor& a, const Tensor& b, Tensor out, const c10::optional<T
 //   b_mn false: b is [N, K];  true: b is [K, N]
 // dgrad of a linear layer: gemm(dy[T,out], w[out,in], dx, b_mn = true);
 // wgrad: gemm(dy[T,out], x[T,in], dw[out,in], a_mn = b_mn = true, epilogue 1 to accumulate).
-void gemm(const Tensor& a, const Tensor& b, Tensor out, int64_t epilogue, bool a_mn, bool b_mn, Tensor status) {
+void gemm_variant(const Tensor& a, const Tensor& b, Tensor out, int64_t epilogue, bool a_mn, bool b_mn, Tensor status, int64_t variant) {
   TORCH_CHECK(a.is_cuda() && b.is_cuda() && out.is_cuda() && status.is_cuda());
   TORCH_CHECK(a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16 && out.scalar_type() == at::kBFloat16);
   TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && out.dim() == 2 && a.stride(1) == 1 && b.stride(1) == 1 && out.stride(1) == 1);
@@ -718,8 +718,12 @@ void gemm(const Tensor& a, const Tensor& b, Tensor out, int64_t epilogue, bool a
   c10::cuda::CUDAGuard guard(a.device());
   const int rc = sb200::launch_gemm_tcgen05(a.data_ptr(), b.data_ptr(), out.data_ptr(), nullptr, (int)M, (int)N, (int)K, a.stride(0),
                                             b.stride(0), out.stride(0), 0, (int)epilogue, a_mn ? 1 : 0, b_mn ? 1 : 0,
-                                            status.data_ptr<int>(), 0, cur_stream());
+                                            status.data_ptr<int>(), (int)variant, cur_stream());
   TORCH_CHECK(rc == 0, "gemm launch failed (", rc, ")");
+}
+
+void gemm(const Tensor& a, const Tensor& b, Tensor out, int64_t epilogue, bool a_mn, bool b_mn, Tensor status) {
+  gemm_variant(a, b, out, epilogue, a_mn, b_mn, status, 0);
 }
 
 // ---- masked attention ------------------------------------------------------------------
@@ -922,6 +926,7 @@ TORCH_LIBRARY(sb200, m) {
   m.def("hs_pop", &hs_pop);
   m.def("gemm_tn", &gemm_tn);
   m.def("gemm", &gemm);
+  m.def("gemm_variant", &gemm_variant);
   m.def("lmhead_loss_fwd", &lmhead_loss_fwd);
   m.def("moe_group_plan", &moe_group_plan);
   m.def("gemm_grouped_rows", &gemm_grouped_rows);

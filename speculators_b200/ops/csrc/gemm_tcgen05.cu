@@ -1,33 +1,33 @@
 // bf16 GEMM on the 5th-generation tensor cores:  C[M,N] = A[M,K] * B[N,K]^T  (+ epilogue)
 //
 // This is the nn.Linear forward shape: both operands are K-major (row-major with K
-// contiguous), the accumulator is fp32.  Structure of one persistent CTA (192 threads):
+// contiguous), the accumulator is fp32.  Roles of a CTA's warps:
 //
 //   warp 0  TMA producer : cp.async.bulk.tensor (128B-swizzled boxes, no multicast) into a
-//                          4-stage shared-memory ring, completion counted on mbarriers
-//   warp 1  MMA issuer   : allocates all 512 TMEM columns (two 128x256 fp32 accumulators),
-//                          one elected thread issues tcgen05.mma (M=128, N=256, K=16) from
+//                          shared-memory ring, completion counted on mbarriers
+//   warp 1  MMA issuer   : allocates TMEM (two 256-column fp32 accumulators in the persistent
+//                          kernel), one elected thread issues tcgen05.mma from
 //                          shared-memory descriptors and tcgen05.commit's to free ring slots
-//   warps 2-5 epilogue   : tcgen05.ld the finished accumulator (each warp its own 32 TMEM
+//   warps 2.. epilogue   : tcgen05.ld the finished accumulator (each warp its own 32 TMEM
 //                          lanes = 32 output rows), convert to bf16, apply the epilogue and
 //                          store; the MMA warp meanwhile fills the other accumulator
 //
 // Tiles are walked n-major so that CTAs running at the same time share B (weight) tiles in
 // L2.  Ragged M / N / K are handled by TMA zero fill and masked stores.
 //
-// Two kernels share this structure.  gemm_tn_kernel works on 128x256 tiles, one CTA per
-// tile.  gemm_tn_2cta_kernel pairs two SMs (a cluster of two CTAs, tcgen05 cta_group::2)
-// on a 256x256 tile: each CTA stages its own 128 rows of A and 128 of the tile's 256 rows
-// of B (32 KB per stage instead of 48 KB, six stages instead of four), the even CTA's
-// elected thread issues M=256 MMAs that read both CTAs' shared memory and write both
-// CTAs' TMEM, and completion is multicast to the barriers of both CTAs.  Halving the B
-// traffic per SM is what the L2-to-SM path needs to keep the tensor pipe fed.
+// Three kernels share this structure.  gemm_tn_2cta_kernel (large products) pairs two SMs (a cluster
+// of two CTAs, tcgen05 cta_group::2) on a 256x256 tile, persistent over tiles: each CTA stages its own 128
+// rows of A and 128 of the tile's 256 rows of B, the even CTA's elected thread issues M=256 MMAs that read
+// both CTAs' shared memory and write both CTAs' TMEM, and completion is multicast to the barriers of both
+// CTAs.  Halving the B traffic per SM is what the L2-to-SM path needs to keep the tensor pipe fed.
+// gemm_split_kernel runs the same tile on a cluster of two or four pairs that divide the contraction (few
+// tiles, long contraction), gemm_small_kernel one 128x64 tile per CTA (few tiles, short contraction).
 //
 // Operand layouts.  The forward product has both operands K-major (rows of A and of B run
 // along the contraction).  The backward products of a linear layer do not:
 //   dgrad  dX[T,in]  = dY[T,out] * W[out,in]        B is read as stored, [K, N] with N contiguous
 //   wgrad  dW[out,in] (+)= dY[T,out]^T * X[T,in]    A is [K, M] with M contiguous, B is [K, N]
-// The CTA-pair kernel therefore takes each operand either K-major or MN-major (template flags):
+// The kernels therefore take each operand either K-major or MN-major (template flags):
 // an MN-major operand is staged by TMA as boxes of 64 MN-elements x 128 contraction rows (the
 // same 16 KB, 128-byte swizzle) and described to the tensor core with an MN-major shared-memory
 // descriptor plus the transpose bit of the instruction descriptor, so no operand is ever
@@ -37,6 +37,8 @@
 // caller's status word and leaves its loop; the other roles then run out of budget (or
 // see the status word) too, the CTA meets at the final barrier, frees its TMEM and
 // returns.  Nothing traps and nothing spins forever.
+#include <atomic>
+
 #include "loss_stats.cuh"
 #include "tcgen05_utils.cuh"
 
@@ -44,11 +46,8 @@ namespace sb200 {
 
 namespace tc {
 
-constexpr int BM = 128, BN = 256, BK = 64, STAGES = 4;
-constexpr int A_BYTES = BM * BK * 2, B_BYTES = BN * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int THREADS = 192;
+constexpr int BM = 128, BN = 256, BK = 64;
 constexpr int TMEM_COLS = 512;
-constexpr int kDefaultPairVariant = 3;
 
 // kSwiGLU: the weight is the stack [gate rows | up rows] of a gated MLP (N = 2 I).  A tile pairs 128 gate columns
 // with the same 128 up columns (the leader CTA loads the gate rows, its peer the up rows, so the accumulator holds
@@ -117,6 +116,7 @@ struct Params {
   Scatter sc;
   __nv_bfloat16* h;  // kSwiGLU: [M, N / 2] output, row stride ldh
   int64_t ldh;
+  int staged;        // 1: C (and h) leave through shared memory and TMA stores (map_c, map_h)
 };
 
 // First element of the W-column chunk at (row, n0) of the output.
@@ -254,46 +254,48 @@ __device__ __forceinline__ void store_accumulator(const Params& p, uint32_t tadd
 }
 
 // ---- gated MLP: gate | up product with silu(gate) * up formed in the epilogue -------------------
-// One thread = one row; `tlane` = TMEM address of its lane at the first of the 64 gate columns it handles
+// One thread = one row, one warp = 32 rows through its staging area; `tlane` = TMEM address of its lane at the first of the 64 gate columns it handles
 // (the matching up columns sit 128 columns further), col0 = their column in [0, I).  The activation is
 // taken from the bf16-rounded gate and up (what the backward pass reads back), in the element-wise
-// kernel's order: silu(gate) rounded to bf16, times up.  Needs I % 128 == 0, ldc / ldh multiples of 16
-// and 32-byte aligned bases (checked on the host).
-__device__ __forceinline__ void store_accumulator_swiglu(const Params& p, uint32_t tlane, int row, int col0, int row_end) {
+// kernel's order: silu(gate) rounded to bf16, times up.  Needs I % 128 == 0 and staged stores (checked on the host).
+__device__ __forceinline__ void store_accumulator_swiglu(const Params& p, const CUtensorMap* map_c, const CUtensorMap* map_h, uint32_t stage, uint32_t tlane,
+                                                         int row0, int col0, bool live, int lane) {
   const int I = p.N >> 1;
-  __nv_bfloat16* grow = p.c + (int64_t)row * p.ldc + col0;
-  __nv_bfloat16* hrow = p.h + (int64_t)row * p.ldh + col0;
-#pragma unroll 1
+  bf16x8 up[8], hp[8];
+  stage_wait();
+#pragma unroll
   for (int c = 0; c < 2; ++c) {
     uint32_t g[32], u[32];
     tmem_ld32(tlane + c * 32, g);
     tmem_ld32(tlane + 128 + c * 32, u);
     tmem_ld_wait();
-    if (row >= row_end) continue;
-    bf16x8 gp[4], up[4], hp[4];
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
       float gf[8], uf[8], o[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) { gf[j] = __uint_as_float(g[v * 8 + j]); uf[j] = __uint_as_float(u[v * 8 + j]); }
-      gp[v] = pack8(gf);
-      up[v] = pack8(uf);
-      unpack8(gp[v], gf);
-      unpack8(up[v], uf);
+      const bf16x8 gp = pack8(gf);
+      up[c * 4 + v] = pack8(uf);
+      unpack8(gp, gf);
+      unpack8(up[c * 4 + v], uf);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const float sg = 1.f / (1.f + __expf(-gf[j]));
         o[j] = __bfloat162float(__float2bfloat16(gf[j] * sg)) * uf[j];
       }
-      hp[v] = pack8(o);
+      hp[c * 4 + v] = pack8(o);
+      stage_put8(stage, lane, c * 4 + v, gp);
     }
-    st32(grow + c * 32, gp[0], gp[1]);
-    st32(grow + c * 32 + 16, gp[2], gp[3]);
-    st32(grow + I + c * 32, up[0], up[1]);
-    st32(grow + I + c * 32 + 16, up[2], up[3]);
-    st32(hrow + c * 32, hp[0], hp[1]);
-    st32(hrow + c * 32 + 16, hp[2], hp[3]);
   }
+  stage_store(stage, map_c, col0, row0, live);
+  stage_wait();
+#pragma unroll
+  for (int v = 0; v < 8; ++v) stage_put8(stage, lane, v, up[v]);
+  stage_store(stage, map_c, I + col0, row0, live);
+  stage_wait();
+#pragma unroll
+  for (int v = 0; v < 8; ++v) stage_put8(stage, lane, v, hp[v]);
+  stage_store(stage, map_h, col0, row0, live);
 }
 
 // ---- epilogues that read memory (C += result, result + residual) ---------------------------
@@ -313,6 +315,18 @@ __device__ __forceinline__ bool tile_reads_vectorised(const Params& p, int n0) {
   if (p.epilogue == kStore || n0 + W > p.N || (p.ldc & 7) || (reinterpret_cast<uintptr_t>(p.c) & 15)) return false;
   if (p.epilogue == kAddResidual && ((p.ldr & 7) || (reinterpret_cast<uintptr_t>(p.residual) & 15))) return false;
   return true;
+}
+
+// Staged stores take every tile (N is a multiple of 8 then): a chunk past the edge reads as zeros.
+template <int W>
+__device__ __forceinline__ void prefetch_addend_staged(const Params& p, int row, int n0, int row_end, RowPrefetch<W>& pre) {
+  pre.tile_ok = true;
+  pre.valid = row < row_end;
+  if (p.epilogue == kStore) return;
+  const __nv_bfloat16* src = p.epilogue == kAccumulate ? p.c + (int64_t)row * p.ldc + n0 : p.residual + (int64_t)row * p.ldr + n0;
+#pragma unroll
+  for (int i = 0; i < W / 8; ++i)
+    pre.v[i] = pre.valid && n0 + i * 8 < p.N ? __ldg(reinterpret_cast<const uint4*>(src) + i) : make_uint4(0u, 0u, 0u, 0u);
 }
 
 template <int W>
@@ -355,6 +369,57 @@ __device__ __forceinline__ void store_accumulator_prefetched(const Params& p, ui
 #pragma unroll
       for (int v = 0; v < 4; ++v) st8(crow + c * 32 + v * 8, packed[v]);
     }
+  }
+}
+
+// Four finished fp32 values -> row `row`, columns col0 .. col0 + 3 of C with the configured epilogue.
+__device__ __forceinline__ void store_vec4(const Params& p, const float4& t, int row, int col0) {
+  __nv_bfloat16* out = p.c + (int64_t)row * p.ldc + col0;
+  const __nv_bfloat16* add = p.epilogue == kAccumulate ? out : p.residual + (int64_t)row * p.ldr + col0;
+  float f[4] = {t.x, t.y, t.z, t.w};
+  const bool full = col0 + 4 <= p.N && (p.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(p.c) & 7) == 0;
+  if (p.epilogue != kStore) {
+    for (int j = 0; j < 4; ++j)
+      if (col0 + j < p.N) f[j] += __bfloat162float(add[j]);
+  }
+  if (full) {
+    __nv_bfloat162 lo = __floats2bfloat162_rn(f[0], f[1]), hi = __floats2bfloat162_rn(f[2], f[3]);
+    *reinterpret_cast<uint2*>(out) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+  } else {
+    for (int j = 0; j < 4; ++j)
+      if (col0 + j < p.N) out[j] = __float2bfloat16(f[j]);
+  }
+}
+
+// One warp's 32 rows x W columns through its 4 KB staging area, 64 columns at a time.  `row0`: C row of lane 0;
+// `live`: the rows exist; the addend of a reading epilogue is in `pre` (pre.tile_ok) or read here.
+template <int W>
+__device__ __forceinline__ void store_accumulator_staged(const Params& p, const CUtensorMap* map_c, uint32_t stage, uint32_t taddr, int row0, int n0,
+                                                         const RowPrefetch<W>& pre, bool live, bool zero, int lane) {
+#pragma unroll
+  for (int h = 0; h < W / 64; ++h) {
+    stage_wait();
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int c = h * 2 + q;
+      uint32_t r[32];
+      tmem_ld32(taddr + c * 32, r);
+      tmem_ld_wait();
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        float f[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] = zero ? 0.f : __uint_as_float(r[v * 8 + j]);
+        if (p.epilogue != kStore) {
+          float o[8];
+          unpack8(*reinterpret_cast<const bf16x8*>(&pre.v[c * 4 + v]), o);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) f[j] += o[j];
+        }
+        stage_put8(stage, lane, q * 4 + v, pack8(f));
+      }
+    }
+    stage_store(stage, map_c, n0 + h * 64, row0, live && n0 + h * 64 < p.N);
   }
 }
 
@@ -408,103 +473,166 @@ __device__ __forceinline__ void store_accumulator_with_stats(const Params& p, ui
   }
 }
 
-__global__ void __launch_bounds__(THREADS, 1)
-gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const Params p) {
-  extern __shared__ unsigned char smem_raw[];
-  // 1024-byte alignment for the swizzled tiles
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ __align__(8) uint64_t bar_full[STAGES], bar_empty[STAGES], bar_acc_full[2], bar_acc_empty[2];
-  __shared__ uint32_t tmem_base_slot;
+// ---- 128x64 tiles on single CTAs ---------------------------------------------------------------
+// Products that leave most of the chip idle on 256x256 tiles (narrow drafts, short rows, weight gradients of
+// small layers).  Such a launch is latency: load, a few dozen MMAs, one epilogue pass.  So a tile is small, the
+// ring holds four 128-wide contraction steps (192 KB: a contraction of up to 512 is in flight as a whole), there
+// is no persistence and no second accumulator, and where tiles are fewer than SMs a cluster of 2, 4 or 8 CTAs
+// divides the contraction of one tile: every CTA pushes its fp32 partial sums, 128 / splits rows to each
+// member, through distributed shared memory and finishes its own rows in member order (one launch, no
+// workspace, the same bits on every run).  A step is 128 wide because waiting, announcing bytes and committing
+// cost a single thread about 290 cycles each, whatever the step's width.
+// 48 KB per step is three times the L2 traffic per FLOP of a pair tile: larger products do not come here
+// (choose_variant).
+constexpr int S_TILE_N = 64, S_STEP_K = 128, S_STAGES = 4, S_THREADS = 192, S_TMEM_COLS = 64;
+constexpr int S_A_BYTES = BM * S_STEP_K * 2, S_B_BYTES = S_TILE_N * S_STEP_K * 2, S_STAGE_BYTES = S_A_BYTES + S_B_BYTES;
+constexpr int S_RECV_BYTES = BM * S_TILE_N * 4;
 
+__device__ __forceinline__ void st_cluster_f4(uint32_t addr, float a, float b, float c, float d) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+
+template <bool A_MN, bool B_MN>
+__global__ void __launch_bounds__(S_THREADS, 1)
+gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                  const __grid_constant__ CUtensorMap map_c, const Params p, const int log_splits) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ __align__(8) uint64_t bar_full[S_STAGES], bar_empty[S_STAGES], bar_acc_full;
+  __shared__ uint32_t tmem_base_slot;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tiles_m = (p.M + BM - 1) / BM, tiles_n = (p.N + BN - 1) / BN;
-  const int num_tiles = tiles_m * tiles_n;
-  const int num_kb = (p.K + BK - 1) / BK;
+  const int splits = 1 << log_splits, split = blockIdx.x & (splits - 1), tile = blockIdx.x >> log_splits;
+  const int tiles_m = (p.M + BM - 1) / BM;
+  const int m0 = (tile % tiles_m) * BM, n0 = (tile / tiles_m) * S_TILE_N;
+  const int all_kb = (p.K + S_STEP_K - 1) / S_STEP_K;
+  const int kb0 = (split * all_kb) >> log_splits, num_kb = (((split + 1) * all_kb) >> log_splits) - kb0;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < S_STAGES; ++s) {
       mbar_init(smem_addr(&bar_full[s]), 1);
       mbar_init(smem_addr(&bar_empty[s]), 1);
     }
-    for (int a = 0; a < 2; ++a) {
-      mbar_init(smem_addr(&bar_acc_full[a]), 1);
-      mbar_init(smem_addr(&bar_acc_empty[a]), 128);
-    }
+    mbar_init(smem_addr(&bar_acc_full), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_base_slot)), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_base_slot)), "r"(S_TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   fence_before_sync();
   __syncthreads();
   fence_after_sync();
   const uint32_t tmem_base = tmem_base_slot;
+  if (log_splits > 0) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // waited for before the first remote store
 
+  bool ok = true;
+  const int quarter = warp & 3, row = m0 + quarter * 32 + lane;
   if (warp == 0) {
-    // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t stage = 0, phase = 0;
-      bool ok = true;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        const int m0 = (tile % tiles_m) * BM, n0 = (tile / tiles_m) * BN;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!(ok = mbar_wait(smem_addr(&bar_empty[stage]), phase ^ 1, p.status, kTimeoutProducer))) break;
-          const uint32_t full = smem_addr(&bar_full[stage]);
-          mbar_expect_tx(full, STAGE_BYTES);
-          const uint32_t sa = smem_addr(smem + stage * STAGE_BYTES);
-          tma_load_2d(sa, &map_a, full, kb * BK, m0);
-          tma_load_2d(sa + A_BYTES, &map_b, full, kb * BK, n0);
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (kb >= S_STAGES && !mbar_wait(smem_addr(&bar_empty[stage]), phase ^ 1, p.status, kTimeoutProducer)) break;
+        const uint32_t full = smem_addr(&bar_full[stage]), sa = smem_addr(smem + stage * S_STAGE_BYTES), sb = sa + S_A_BYTES;
+        const int k0 = (kb0 + kb) * S_STEP_K;
+        mbar_expect_tx(full, S_STAGE_BYTES);
+        // K-major: boxes of rows x 64 contraction columns; MN-major: boxes of 128 contraction rows x 64 MN-columns
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          if (A_MN) tma_load_2d(sa + u * (S_A_BYTES / 2), &map_a, full, m0 + u * 64, k0);
+          else tma_load_2d(sa + u * (S_A_BYTES / 2), &map_a, full, k0 + u * 64, m0);
         }
+        if (B_MN) {
+          tma_load_2d(sb, &map_b, full, n0, k0);
+        } else {
+          tma_load_2d(sb, &map_b, full, k0, n0);
+          tma_load_2d(sb + S_B_BYTES / 2, &map_b, full, k0 + 64, n0);
+        }
+        if (++stage == S_STAGES) { stage = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = instr_desc_bf16(BM, BN);
+    if (elect_one()) {
+      constexpr uint32_t idesc = instr_desc_ab(BM, S_TILE_N, A_MN, B_MN);
       uint32_t stage = 0, phase = 0;
-      bool ok = true;
-      int local = 0;
-      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local) {
-        const int acc = local & 1;
-        if (!(ok = mbar_wait(smem_addr(&bar_acc_empty[acc]), ((local >> 1) & 1) ^ 1, p.status, kTimeoutMma))) break;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!(ok = mbar_wait(smem_addr(&bar_full[stage]), phase, p.status, kTimeoutMma))) break;
         fence_after_sync();
-        const uint32_t tmem_d = tmem_base + acc * BN;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!(ok = mbar_wait(smem_addr(&bar_full[stage]), phase, p.status, kTimeoutMma))) break;
-          fence_after_sync();
-          const uint32_t sa = smem_addr(smem + stage * STAGE_BYTES);
-          const uint64_t adesc = smem_desc_kmajor_sw128(sa), bdesc = smem_desc_kmajor_sw128(sa + A_BYTES);
+        const uint32_t sa = smem_addr(smem + stage * S_STAGE_BYTES), sb = sa + S_A_BYTES;
+        const uint64_t adesc = A_MN ? smem_desc_mnmajor_sw128(sa, S_A_BYTES / 2) : smem_desc_kmajor_sw128(sa);
+        const uint64_t bdesc = B_MN ? smem_desc_mnmajor_sw128(sb, S_B_BYTES) : smem_desc_kmajor_sw128(sb);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            // advancing 16 K-elements = 32 bytes inside the 128-byte swizzled row: +2 in 16-byte units
-            umma_bf16(tmem_d, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0);
-          }
-          umma_commit(smem_addr(&bar_empty[stage]));  // frees the ring slot once these MMAs retire
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        for (int k = 0; k < 8; ++k) {
+          const uint32_t mn = k * (2048 >> 4), in_row = 2 * (k & 3);
+          umma_bf16(tmem_base, adesc + (A_MN ? mn : (k >> 2) * (S_A_BYTES / 2 >> 4) + in_row),
+                    bdesc + (B_MN ? mn : (k >> 2) * (S_B_BYTES / 2 >> 4) + in_row), idesc, (kb | k) != 0);
         }
-        if (ok) umma_commit(smem_addr(&bar_acc_full[acc]));
+        umma_commit(smem_addr(&bar_empty[stage]));
+        if (++stage == S_STAGES) { stage = 0; phase ^= 1; }
+      }
+      if (ok) umma_commit(smem_addr(&bar_acc_full));
+    }
+  } else if (log_splits == 0) {
+    RowPrefetch<S_TILE_N> pre;
+    if (p.staged) prefetch_addend_staged<S_TILE_N>(p, row, n0, p.M, pre);
+    else prefetch_addend<S_TILE_N>(p, row, n0, p.M, pre);
+    ok = mbar_wait(smem_addr(&bar_acc_full), 0, p.status, kTimeoutEpilogue);
+    ok = __all_sync(0xffffffffu, ok);
+    if (ok) {
+      fence_after_sync();
+      const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16);
+      if (p.staged) {
+        const uint32_t stage = smem_addr(smem + S_STAGES * S_STAGE_BYTES) + quarter * 4096;
+        store_accumulator_staged<S_TILE_N>(p, &map_c, stage, taddr, m0 + quarter * 32, n0, pre, m0 + quarter * 32 < p.M, false, lane);
+        stage_wait();
+      } else if (pre.tile_ok) {
+        store_accumulator_prefetched<S_TILE_N>(p, taddr, row, n0, pre, false);
+      } else {
+        store_accumulator<S_TILE_N>(p, taddr, row, n0, p.M, false);
       }
     }
   } else {
-    // ------------------------------------------------------------------ epilogue (warps 2..5)
-    const int quarter = warp & 3;  // TMEM lanes this warp may touch: 32*quarter .. +31
-    bool ok = true;
-    int local = 0;
-    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++local) {
-      const int acc = local & 1;
-      const int m0 = (tile % tiles_m) * BM, n0 = (tile / tiles_m) * BN;
-      RowPrefetch<BN> pre;
-      prefetch_addend<BN>(p, m0 + quarter * 32 + lane, n0, p.M, pre);
-      ok = mbar_wait(smem_addr(&bar_acc_full[acc]), (local >> 1) & 1, p.status, kTimeoutEpilogue);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
-      fence_after_sync();
-      if (pre.tile_ok) store_accumulator_prefetched<BN>(p, tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN, m0 + quarter * 32 + lane, n0, pre, false);
-      else store_accumulator<BN>(p, tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN, m0 + quarter * 32 + lane, n0, p.M, false);
-      fence_before_sync();
-      mbar_arrive(smem_addr(&bar_acc_empty[acc]));
+    ok = mbar_wait(smem_addr(&bar_acc_full), 0, p.status, kTimeoutEpilogue);
+    ok = __all_sync(0xffffffffu, ok);
+    fence_after_sync();
+  }
+  __syncwarp();
+  if (log_splits > 0) {
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // every member's shared memory is live
+    // Member j finishes rows j * 128 / splits .. of the tile: [source][own row][64 columns] fp32, 16-byte chunks
+    // XOR-swizzled by the row, so that lanes (rows) that push the same columns do not share banks.
+    const int log_rows = 7 - log_splits, tile_row = quarter * 32 + lane, own_rows = 1 << log_rows;
+    const uint32_t recv = smem_addr(smem + S_STAGES * S_STAGE_BYTES);
+    if (warp >= 2 && ok) {
+      const int to = tile_row >> log_rows, r0 = tile_row & (own_rows - 1);
+      const uint32_t dst = map_to_cta(recv, to) + ((split << log_rows) + r0) * 256;
+      const bool empty = num_kb == 0;  // no contraction step ran here: the tensor memory holds nothing
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        uint32_t r[32];
+        tmem_ld32(tmem_base + ((uint32_t)(quarter * 32) << 16) + c * 32, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int v = 0; v < 32; ++v)
+          if (empty) r[v] = 0u;
+#pragma unroll
+        for (int v = 0; v < 8; ++v)
+          st_cluster_f4(dst + (((c * 8 + v) ^ (r0 & 15)) << 4), __uint_as_float(r[v * 4]), __uint_as_float(r[v * 4 + 1]), __uint_as_float(r[v * 4 + 2]),
+                        __uint_as_float(r[v * 4 + 3]));
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();
+    if (warp >= 2 && ok) {
+      const float4* got = reinterpret_cast<const float4*>(smem + S_STAGES * S_STAGE_BYTES);
+      for (int e = threadIdx.x - 64; e < own_rows * 16; e += 128) {  // 16 lanes per row: whole lines
+        const int r0 = e >> 4, c = e & 15, orow = m0 + (split << log_rows) + r0;
+        float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int src = 0; src < splits; ++src) {
+          const float4 o = got[((src << log_rows) + r0) * 16 + (c ^ (r0 & 15))];
+          t.x += o.x; t.y += o.y; t.z += o.z; t.w += o.w;
+        }
+        if (orow < p.M) store_vec4(p, t, orow, n0 + c * 4);
+      }
     }
   }
 
@@ -513,9 +641,8 @@ gemm_tn_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   fence_before_sync();
   __syncthreads();
   if (warp == 1) {
-    __syncwarp();
     fence_after_sync();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(S_TMEM_COLS) : "memory");
   }
 }
 
@@ -528,6 +655,7 @@ constexpr int P_HALF = 128;                                    // rows of A and 
 constexpr int P_A_BYTES = P_HALF * BK * 2, P_B_BYTES = P_HALF * BK * 2, P_SUB_BYTES = P_A_BYTES + P_B_BYTES;
 constexpr int P_TILE_M = 2 * P_HALF, P_TILE_N = 2 * P_HALF;
 constexpr int P_RING_BYTES = 6 * P_SUB_BYTES;
+constexpr int P_STAGE_OUT_BYTES = 8 * 4096;  // one staging area per epilogue warp
 // The pair kernel runs eight epilogue warps: warps w and w + 4 reach the same 32 TMEM lanes (rows) and take 128 of the
 // tile's 256 columns each, so two warps per scheduler share the epilogue's instruction stream (with four warps the row
 // statistics of the lm_head epilogue, and the addend of short-contraction weight gradients, set the pace of the tile).
@@ -535,7 +663,8 @@ constexpr int P_THREADS = 320, P_EPI_COLS = 128;
 
 template <int KSUB, bool A_MN = false, bool B_MN = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P_THREADS, 1)
-gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const Params p) {
+gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                    const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_h, const Params p) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   static_assert(KSUB == 2 || (!A_MN && !B_MN), "MN-major operands are staged as 128-row boxes: KSUB must be 2");
@@ -577,7 +706,7 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t stage = 0, phase = 0;
       bool ok = true;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
@@ -610,7 +739,7 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (leader && lane == 0) {
+    if (leader && elect_one()) {
       constexpr uint32_t idesc = instr_desc_ab(P_TILE_M, P_TILE_N, A_MN, B_MN);
       uint32_t stage = 0, phase = 0;
       bool ok = true;
@@ -649,6 +778,7 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const int quarter = warp & 3;         // TMEM lanes 32 * quarter .. + 31
     const int chalf = (warp - 2) >> 2;    // columns 128 * chalf .. + 127 of the tile
     const uint32_t acc_empty_leader[2] = {map_to_cta(smem_addr(&bar_acc_empty[0]), 0), map_to_cta(smem_addr(&bar_acc_empty[1]), 0)};
+    const uint32_t stage = smem_addr(smem + P_RING_BYTES) + (warp - 2) * 4096;
     bool ok = true;
     int local = 0;
     for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++local) {
@@ -659,43 +789,283 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       RowPrefetch<P_EPI_COLS> pre;
       const bool with_stats = p.rs.targets != nullptr, gated = p.epilogue == kSwiGLU;
       if (with_stats) prefetch_targets<P_EPI_COLS>(p, row, n0, pre);
+      else if (p.staged && !gated) prefetch_addend_staged<P_EPI_COLS>(p, row, n0, ti.row_end, pre);
       else if (!gated) prefetch_addend<P_EPI_COLS>(p, row, n0, ti.row_end, pre);
       ok = mbar_wait(smem_addr(&bar_acc_full[acc]), (local >> 1) & 1, p.status, kTimeoutEpilogue);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       fence_after_sync();
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN + chalf * P_EPI_COLS;
+      const int row0 = ti.c_row0 + quarter * 32;
       if (gated)  // this warp: gate columns 64 * chalf .. + 63 of the tile and the same up columns
-        store_accumulator_swiglu(p, tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN + chalf * 64, row, ti.n0 + chalf * 64, ti.row_end);
+        store_accumulator_swiglu(p, &map_c, &map_h, stage, tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN + chalf * 64, row0, ti.n0 + chalf * 64,
+                                 row0 < ti.row_end, lane);
       else if (with_stats) store_accumulator_with_stats<P_EPI_COLS>(p, taddr, row, n0, ti.tile_n * 2 + chalf, tiles_n * 2, pre);
+      else if (p.staged) store_accumulator_staged<P_EPI_COLS>(p, &map_c, stage, taddr, row0, n0, pre, row0 < ti.row_end, zero, lane);
       else if (pre.tile_ok) store_accumulator_prefetched<P_EPI_COLS>(p, taddr, row, n0, pre, zero);
       else store_accumulator<P_EPI_COLS>(p, taddr, row, n0, ti.row_end, zero);
       fence_before_sync();
-      mbar_arrive_cluster(acc_empty_leader[acc]);
+      mbar_arrive_cluster_relaxed(acc_empty_leader[acc]);
     }
+    stage_wait();
   }
 
   // Both CTAs stay until the pair is done: the peer's copies signal the leader's barriers,
   // the leader's MMAs read the peer's shared memory and write its TMEM.
   fence_before_sync();
   __syncthreads();
-  cluster_sync_all();
+  cluster_sync_relaxed();
   if (warp == 1) {
     fence_after_sync();
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
   }
 }
 
+// ---- 256x256 tiles with the contraction split over the CTA pairs of a cluster -----------------------
+// A product with few tiles and a long contraction (short rows through a wide MLP, Gram-like weight gradients
+// of narrow layers) occupies as many pairs as it has tiles.  Here a cluster of SPLITS pairs shares one tile:
+// every pair runs its part of the contraction at the pair kernel's operand traffic (64 B per clock and SM,
+// where smaller tiles would be bound by L2), then the partial accumulators are reduce-scattered through
+// distributed shared memory: every CTA pushes 128 / SPLITS of its rows in fp32 to each member with its role,
+// into the (now idle) operand ring, and the receiver sums its rows in pair order and stores whole lines.
+// One launch, no workspace, the same bits on every run.
+template <int SPLITS, bool A_MN, bool B_MN>
+__global__ void __cluster_dims__(2 * SPLITS, 1, 1) __launch_bounds__(P_THREADS, 1)
+gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const Params p) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  constexpr int KSUB = 2, STAGES = 6 / KSUB, STAGE_BYTES = KSUB * P_SUB_BYTES, STAGE_K = KSUB * BK;
+  constexpr int OWN_ROWS = P_HALF / SPLITS;  // rows of its 128 that this CTA finishes
+  static_assert(P_HALF * P_TILE_N * 4 <= P_RING_BYTES, "the partial sums must fit the ring");
+  __shared__ __align__(8) uint64_t bar_full[STAGES], bar_empty[STAGES], bar_acc_full;
+  __shared__ uint32_t tmem_base_slot;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t crank = cluster_ctarank(), role = crank & 1, split = crank >> 1;
+  const bool leader = role == 0;
+  const int tiles_m = (p.M + P_TILE_M - 1) / P_TILE_M;
+  const int tile = blockIdx.x / (2 * SPLITS);
+  const int m0 = (tile % tiles_m) * P_TILE_M + role * P_HALF, n0 = (tile / tiles_m) * P_TILE_N;
+  const int all_kb = (p.K + STAGE_K - 1) / STAGE_K, per_kb = (all_kb + SPLITS - 1) / SPLITS;
+  const int kb0 = split * per_kb, num_kb = max(0, min(per_kb, all_kb - kb0));
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(smem_addr(&bar_full[s]), 1);
+      mbar_init(smem_addr(&bar_empty[s]), 1);
+    }
+    mbar_init(smem_addr(&bar_acc_full), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_base_slot)), "r"(P_TILE_N) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  fence_before_sync();
+  cluster_sync_all();
+  fence_after_sync();
+  const uint32_t tmem_base = tmem_base_slot;
+
+  bool ok = true;
+  const int quarter = warp & 3, chalf = (warp - 2) >> 2;
+  if (warp == 0) {
+    if (elect_one()) {
+      uint32_t stage = 0, phase = 0;
+      const int b0 = n0 + role * P_HALF;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!(ok = mbar_wait(smem_addr(&bar_empty[stage]), phase ^ 1, p.status, kTimeoutProducer))) break;
+        const uint32_t full_local = smem_addr(&bar_full[stage]);
+        if (leader) mbar_expect_tx(full_local, 2 * STAGE_BYTES);
+        const uint32_t full_leader = map_to_cta(full_local, crank & ~1u);
+        const uint32_t sa = smem_addr(smem + stage * STAGE_BYTES);
+        const int k0 = (kb0 + kb) * STAGE_K;
+#pragma unroll
+        for (int u = 0; u < KSUB; ++u) {
+          if (A_MN) tma_load_2d_pair(sa + u * P_SUB_BYTES, &map_a, full_leader, m0 + u * 64, k0);
+          else tma_load_2d_pair(sa + u * P_SUB_BYTES, &map_a, full_leader, k0 + u * BK, m0);
+          if (B_MN) tma_load_2d_pair(sa + u * P_SUB_BYTES + P_A_BYTES, &map_b, full_leader, b0 + u * 64, k0);
+          else tma_load_2d_pair(sa + u * P_SUB_BYTES + P_A_BYTES, &map_b, full_leader, k0 + u * BK, b0);
+        }
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+      }
+      for (int s = 0; s < STAGES && ok; ++s) {  // every MMA that reads this CTA's ring has retired
+        ok = mbar_wait(smem_addr(&bar_empty[stage]), phase ^ 1, p.status, kTimeoutProducer);
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+      }
+    }
+  } else if (warp == 1) {
+    if (leader && elect_one()) {
+      constexpr uint32_t idesc = instr_desc_ab(P_TILE_M, P_TILE_N, A_MN, B_MN);
+      const uint16_t mask = (uint16_t)(3u << (crank & ~1u));
+      uint32_t stage = 0, phase = 0;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!(ok = mbar_wait(smem_addr(&bar_full[stage]), phase, p.status, kTimeoutMma))) break;
+        fence_after_sync();
+        const uint32_t sa = smem_addr(smem + stage * STAGE_BYTES);
+        const uint64_t adesc = A_MN ? smem_desc_mnmajor_sw128(sa, P_SUB_BYTES) : smem_desc_kmajor_sw128(sa);
+        const uint64_t bdesc = B_MN ? smem_desc_mnmajor_sw128(sa + P_A_BYTES, P_SUB_BYTES) : smem_desc_kmajor_sw128(sa + P_A_BYTES);
+#pragma unroll
+        for (int u = 0; u < KSUB; ++u) {
+#pragma unroll
+          for (int k = 0; k < BK / 16; ++k) {
+            const uint32_t off_k = u * (P_SUB_BYTES >> 4) + 2 * k, off_mn = (u * (BK / 16) + k) * (2048 >> 4);
+            umma_bf16_pair(tmem_base, adesc + (A_MN ? off_mn : off_k), bdesc + (B_MN ? off_mn : off_k), idesc, (kb | u | k) != 0);
+          }
+        }
+        umma_commit_pair(smem_addr(&bar_empty[stage]), mask);
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+      }
+      if (ok) umma_commit_pair(smem_addr(&bar_acc_full), mask);
+    }
+  } else {
+    ok = mbar_wait(smem_addr(&bar_acc_full), 0, p.status, kTimeoutEpilogue);
+    ok = __all_sync(0xffffffffu, ok);
+    fence_after_sync();
+  }
+  __syncwarp();
+  // Every pair has finished its contraction: nothing reads or writes the rings any more, they can take partial sums.
+  cluster_sync_relaxed();
+  if (warp >= 2 && ok) {
+    // [source pair][own row][256 columns] fp32, 16-byte chunks XOR-swizzled by the row (lanes are rows)
+    const int tile_row = quarter * 32 + lane, to = tile_row / OWN_ROWS, r0 = tile_row % OWN_ROWS;
+    const uint32_t dst = map_to_cta(smem_addr(smem), to * 2 + role) + (split * OWN_ROWS + r0) * (P_TILE_N * 4);
+    const bool empty = num_kb == 0;  // this pair had no contraction step: its tensor memory holds nothing
+#pragma unroll
+    for (int c = 0; c < P_EPI_COLS / 32; ++c) {
+      uint32_t r[32];
+      tmem_ld32(tmem_base + ((uint32_t)(quarter * 32) << 16) + chalf * P_EPI_COLS + c * 32, r);
+      tmem_ld_wait();
+#pragma unroll
+      for (int v = 0; v < 32; ++v)
+        if (empty) r[v] = 0u;
+#pragma unroll
+      for (int v = 0; v < 8; ++v)
+        st_cluster_f4(dst + (((chalf * 32 + c * 8 + v) ^ (r0 & 31)) << 4), __uint_as_float(r[v * 4]), __uint_as_float(r[v * 4 + 1]), __uint_as_float(r[v * 4 + 2]),
+                      __uint_as_float(r[v * 4 + 3]));
+    }
+  }
+  __syncwarp();
+  cluster_sync_all();
+  if (warp >= 2 && ok) {
+    const float4* got = reinterpret_cast<const float4*>(smem);
+#pragma unroll 4
+    for (int e = threadIdx.x - 64; e < OWN_ROWS * (P_TILE_N / 4); e += 256) {  // 64 lanes per row: whole lines
+      const int r0 = e / (P_TILE_N / 4), c = e % (P_TILE_N / 4), row = m0 + split * OWN_ROWS + r0;
+      float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int src = 0; src < SPLITS; ++src) {  // in pair order on every pair
+        const float4 o = got[(src * OWN_ROWS + r0) * (P_TILE_N / 4) + (c ^ (r0 & 31))];
+        t.x += o.x; t.y += o.y; t.z += o.z; t.w += o.w;
+      }
+      if (row < p.M) store_vec4(p, t, row, n0 + c * 4);
+    }
+  }
+  fence_before_sync();
+  __syncthreads();
+  cluster_sync_relaxed();
+  if (warp == 1) {
+    fence_after_sync();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(P_TILE_N) : "memory");
+  }
+}
+
 // ---- host side ---------------------------------------------------------------------------
 }  // namespace tc
+
+template <typename Kernel>
+static bool allow_smem(Kernel kernel, int bytes) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
+}
+
+template <int SPLITS>
+static void launch_split(int a_mn, int b_mn, int tiles, int smem, cudaStream_t stream, const CUtensorMap& map_a, const CUtensorMap& map_b, const tc::Params& p) {
+  const int grid = tiles * 2 * SPLITS;
+  if (a_mn && b_mn) tc::gemm_split_kernel<SPLITS, true, true><<<grid, tc::P_THREADS, smem, stream>>>(map_a, map_b, p);
+  else if (a_mn) tc::gemm_split_kernel<SPLITS, true, false><<<grid, tc::P_THREADS, smem, stream>>>(map_a, map_b, p);
+  else if (b_mn) tc::gemm_split_kernel<SPLITS, false, true><<<grid, tc::P_THREADS, smem, stream>>>(map_a, map_b, p);
+  else tc::gemm_split_kernel<SPLITS, false, false><<<grid, tc::P_THREADS, smem, stream>>>(map_a, map_b, p);
+}
+
+static cudaError_t launch_small(int a_mn, int b_mn, int tiles, int log_splits, int smem, cudaStream_t stream, const CUtensorMap& map_a, const CUtensorMap& map_b,
+                                const CUtensorMap& map_c, const tc::Params& p) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(tiles << log_splits);
+  cfg.blockDim = dim3(tc::S_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 1u << log_splits;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = log_splits > 0 ? 1 : 0;
+  if (a_mn && b_mn) return cudaLaunchKernelEx(&cfg, tc::gemm_small_kernel<true, true>, map_a, map_b, map_c, p, log_splits);
+  if (a_mn) return cudaLaunchKernelEx(&cfg, tc::gemm_small_kernel<true, false>, map_a, map_b, map_c, p, log_splits);
+  if (b_mn) return cudaLaunchKernelEx(&cfg, tc::gemm_small_kernel<false, true>, map_a, map_b, map_c, p, log_splits);
+  return cudaLaunchKernelEx(&cfg, tc::gemm_small_kernel<false, false>, map_a, map_b, map_c, p, log_splits);
+}
+
+enum Variant : int { kPairK64 = 2, kPair = 3, kSplit2 = 4, kSplit4 = 5, kSmall = 10, kSmall2 = 11, kSmall4 = 12, kSmall8 = 13 };
+constexpr int kMaxPairs = kNumSM / 2;
+
+// How many clusters of `size` CTAs (one per SM) the device holds at a time: the GPCs do not divide evenly.
+static int resident_clusters(int size) {
+  static std::atomic<int> cached[64][4];
+  const int dev = PerDeviceOnce::device(), slot = size == 2 ? 0 : size == 4 ? 1 : 2;
+  if (dev >= 0 && cached[dev][slot] > 0) return cached[dev][slot];
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(kNumSM / size * size);
+  cfg.blockDim = dim3(tc::S_THREADS);
+  cfg.dynamicSmemBytes = tc::S_STAGES * tc::S_STAGE_BYTES + tc::S_RECV_BYTES + 1024;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = size;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, tc::gemm_small_kernel<false, false>, &cfg) != cudaSuccess || n < 1) {
+    cudaGetLastError();
+    n = kNumSM / size * 3 / 4;
+  }
+  if (dev >= 0) cached[dev][slot] = n;
+  return n;
+}
+
+// The kernel for a plain product, by predicted time.  Each form costs a fixed part (launch, pipeline fill, epilogue,
+// exchange of partial sums) plus its 128-wide contraction steps; the constants (us) are fits to launches inside CUDA
+// graphs at 128 .. 3072 rows and columns and contractions of 128 .. 32000, all three layouts:
+//   pair tiles     7.0 + 0.56 / step and wave     (2048 x 1024 x 1024: 10.9 us; 1000 x 2048 x 8192: 43.8)
+//   128 x 64 tiles 3.3 + 0.34 / step and wave     (1024 x 1024 x 1024: 6.7; 128 x 256 x 256: 4.0)
+//   the same, contraction over 2, 4, 8 CTAs: 5.0 + 0.34 / step, one wave only   (128 x 512 x 2048: 6.1 at 8, 8.6 unsplit)
+//   pair tiles over 2, 4 pairs: 10.8 + 0.66 / step, one wave only               (1000 x 2048 x 8192: 31.9 at 2)
+// Several waves of small tiles are bound by L2-to-SM traffic, so they pay a full wave each; the model drops them
+// quickly.  Products of more than about two waves of pair tiles always come out as pair tiles.
+static int choose_variant(int M, int N, int K) {
+  using namespace tc;
+  const int64_t small = (int64_t)((M + BM - 1) / BM) * ((N + S_TILE_N - 1) / S_TILE_N);
+  const int64_t big = (int64_t)((M + P_TILE_M - 1) / P_TILE_M) * ((N + P_TILE_N - 1) / P_TILE_N);
+  const int steps = (K + 127) / 128;
+  int best = kPair;
+  float t = 7.0f + 0.56f * steps * ((big + kMaxPairs - 1) / kMaxPairs);
+  auto consider = [&](int variant, float us) {
+    if (us < t) { t = us; best = variant; }
+  };
+  if (small <= 4 * kNumSM) consider(kSmall, 2.0f + (1.3f + 0.34f * steps) * ((small + kNumSM - 1) / kNumSM));
+  for (int log = 1; log <= 3; ++log)
+    if (steps >= (2 << log) && small <= resident_clusters(1 << log)) consider(kSmall + log, 5.0f + 0.34f * ((steps + (1 << log) - 1) >> log));
+  for (int log = 1; log <= 2; ++log)
+    if (steps >= (4 << log) && big <= resident_clusters(2 << log)) consider(log == 1 ? kSplit2 : kSplit4, 10.8f + 0.66f * ((steps + (1 << log) - 1) >> log));
+  return best;
+}
 
 // C[M,N] = op(A) * op(B)^T with epilogue (0 store, 1 C += result, 2 result + residual).
 //   a_mn == 0: A is [M, K] row-major (K-major), lda = row stride;  a_mn == 1: A is [K, M] row-major (M contiguous)
 //   b_mn == 0: B is [N, K] row-major (K-major), ldb = row stride;  b_mn == 1: B is [K, N] row-major (N contiguous)
 // lda / ldb / ldc / ldr in elements; operand rows must be 16-byte aligned (ld multiple of 8).
 // `status` is a device int the kernel writes a non-zero code to if a bounded wait ran out.
-// variant: 0 = choose (CTA pairs when M > 128 or an operand is MN-major), 1 = one CTA per 128x256 tile (K-major
-// only), 2 = CTA pairs with 64-wide K stages (K-major only), 3 = CTA pairs with 128-wide K stages.
+// variant: 0 = choose (choose_variant), 1 or 10 .. 13 = 128x64 tiles on one CTA or a cluster of 2, 4, 8 CTAs, 2 = CTA pairs with 64-wide K stages (K-major only),
+// 3 = CTA pairs with 128-wide K stages, 4 / 5 = clusters of two / four pairs that split the contraction of a tile.
 static int launch_gemm_impl(const void* a, const void* b, void* c, const void* residual, int M, int N, int K, int64_t lda,
                             int64_t ldb, int64_t ldc, int64_t ldr, int epilogue, int a_mn, int b_mn, int* status, int variant,
                             const void* stats_targets, int64_t stats_ldt, int stats_t_rows, int stats_shift, float* stats_partial,
@@ -704,22 +1074,42 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
   using namespace tc;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((lda & 7) || (ldb & 7) || (reinterpret_cast<uintptr_t>(a) & 15) || (reinterpret_cast<uintptr_t>(b) & 15)) return -1;
+  constexpr int smem_pair = P_RING_BYTES + P_STAGE_OUT_BYTES + 1024, smem_small = S_STAGES * S_STAGE_BYTES + S_RECV_BYTES + 1024;
+  static PerDeviceOnce configured;
+  if (configured.needed()) {
+    bool ok = allow_smem(gemm_tn_2cta_kernel<1>, smem_pair) && allow_smem(gemm_tn_2cta_kernel<2>, smem_pair) &&
+              allow_smem(gemm_tn_2cta_kernel<2, false, true>, smem_pair) && allow_smem(gemm_tn_2cta_kernel<2, true, false>, smem_pair) &&
+              allow_smem(gemm_tn_2cta_kernel<2, true, true>, smem_pair);
+    ok = ok && allow_smem(gemm_split_kernel<2, false, false>, smem_pair) && allow_smem(gemm_split_kernel<2, false, true>, smem_pair) &&
+         allow_smem(gemm_split_kernel<2, true, false>, smem_pair) && allow_smem(gemm_split_kernel<2, true, true>, smem_pair);
+    ok = ok && allow_smem(gemm_split_kernel<4, false, false>, smem_pair) && allow_smem(gemm_split_kernel<4, false, true>, smem_pair) &&
+         allow_smem(gemm_split_kernel<4, true, false>, smem_pair) && allow_smem(gemm_split_kernel<4, true, true>, smem_pair);
+    ok = ok && allow_smem(gemm_small_kernel<false, false>, smem_small) && allow_smem(gemm_small_kernel<false, true>, smem_small) &&
+         allow_smem(gemm_small_kernel<true, false>, smem_small) && allow_smem(gemm_small_kernel<true, true>, smem_small);
+    if (!ok) return -2;
+    configured.mark();
+  }
   const bool mn = a_mn || b_mn;
-  if (variant == 0) variant = (M > BM || mn) ? kDefaultPairVariant : 1;
-  if (mn && variant != 3) return -4;
-  const bool pairs = variant >= 2;
+  const bool plain = stats_targets == nullptr && grp == nullptr && scatter == nullptr && epilogue != kSwiGLU;
+  if (variant == 0) variant = plain ? choose_variant(M, N, K) : kPair;
+  if (variant == 1) variant = kSmall;
+  if (variant < kPairK64 || variant > kSmall8 || (variant > kSplit4 && variant < kSmall)) return -4;
+  if (variant == kPairK64 && mn) return -4;
+  if (variant > kPair && !plain) return -4;
+  const bool pairs = variant < kSmall;
   CUtensorMap map_a, map_b;
-  int rc = a_mn ? make_map_bf16(&map_a, a, K, M, lda, 2 * BK) : make_map_bf16(&map_a, a, M, K, lda, BM);
+  constexpr int mn_rows = 2 * BK;  // contraction rows of a transposed operand's box
+  int rc = a_mn ? make_map_bf16(&map_a, a, K, M, lda, mn_rows) : make_map_bf16(&map_a, a, M, K, lda, BM);
   if (rc) return rc;
   // grouped by rows: B is the stack of the experts' matrices
   const int64_t b_stack = (grp != nullptr && grp->mode == kGroupRows) ? grp->num_groups : 1;
-  rc = b_mn ? make_map_bf16(&map_b, b, b_stack * K, N, ldb, 2 * BK) : make_map_bf16(&map_b, b, b_stack * N, K, ldb, pairs ? P_HALF : BN);
+  rc = b_mn ? make_map_bf16(&map_b, b, b_stack * K, N, ldb, mn_rows) : make_map_bf16(&map_b, b, b_stack * N, K, ldb, pairs ? P_HALF : S_TILE_N);
   if (rc) return rc;
   Params p{(__nv_bfloat16*)c, (const __nv_bfloat16*)residual, M, N, K, ldc, ldr, epilogue, status, RowStatsOut{nullptr, 0, 0, 0, nullptr},
-           Grouping{kGroupNone, 0, nullptr, nullptr}, Scatter{}, (__nv_bfloat16*)gated_h, gated_ldh};
+           Grouping{kGroupNone, 0, nullptr, nullptr}, Scatter{}, (__nv_bfloat16*)gated_h, gated_ldh, 0};
   if (epilogue == kSwiGLU) {
-    if (!pairs || a_mn || b_mn || grp != nullptr || stats_targets != nullptr || scatter != nullptr || gated_h == nullptr || (N & 255) || (ldc & 15) ||
-        (gated_ldh & 15) || (reinterpret_cast<uintptr_t>(c) & 31) || (reinterpret_cast<uintptr_t>(gated_h) & 31))
+    if (!pairs || a_mn || b_mn || grp != nullptr || stats_targets != nullptr || scatter != nullptr || gated_h == nullptr || (N & 255) || (ldc & 7) ||
+        (gated_ldh & 7) || (reinterpret_cast<uintptr_t>(c) & 15) || (reinterpret_cast<uintptr_t>(gated_h) & 15))
       return -8;
   }
   if (scatter != nullptr) {
@@ -733,7 +1123,7 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
       if (reinterpret_cast<uintptr_t>(scatter->stage[q]) & 31) return -7;
   }
   if (grp != nullptr) {
-    if (!pairs || variant != 3 || stats_targets != nullptr || residual != nullptr) return -6;
+    if (variant != kPair || stats_targets != nullptr || residual != nullptr) return -6;
     if (grp->mode == kGroupRows && (a_mn || (K & 127) || (N & 255))) return -6;  // experts' matrices must not share a box
     if (grp->mode == kGroupK && !(a_mn && b_mn)) return -6;
     p.grp = *grp;
@@ -744,39 +1134,37 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
       return -5;
     p.rs = RowStatsOut{(const __nv_bfloat16*)stats_targets, stats_ldt, stats_t_rows, stats_shift, stats_partial};
   }
+  // Stores through staging: C must be a matrix that TMA can address, and a warp's 32 rows must not straddle an expert.
+  CUtensorMap map_c = map_a, map_h = map_a;
+  const bool reads_ok = epilogue != kAddResidual || ((ldr & 7) == 0 && (reinterpret_cast<uintptr_t>(residual) & 15) == 0);
+  if (scatter == nullptr && stats_targets == nullptr && (N & 7) == 0 && (ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(c) & 15) == 0 && reads_ok &&
+      (grp == nullptr || grp->mode == kGroupRows || (M & 127) == 0)) {
+    const int64_t rows = grp != nullptr && grp->mode == kGroupK ? (int64_t)grp->num_groups * M : M;
+    rc = make_map_bf16(&map_c, c, rows, N, ldc, 32);
+    if (rc == 0 && epilogue == kSwiGLU) rc = make_map_bf16(&map_h, gated_h, M, N / 2, gated_ldh, 32);
+    if (rc) return rc;
+    p.staged = 1;
+  }
   count_launch(1);
-  if (pairs) {
-    static PerDeviceOnce configured2;
-    constexpr int smem2 = P_RING_BYTES + 1024;
-    if (configured2.needed()) {
-      bool ok = cudaFuncSetAttribute(gemm_tn_2cta_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2) == cudaSuccess;
-      ok = ok && cudaFuncSetAttribute(gemm_tn_2cta_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2) == cudaSuccess;
-      ok = ok && cudaFuncSetAttribute(gemm_tn_2cta_kernel<2, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2) == cudaSuccess;
-      ok = ok && cudaFuncSetAttribute(gemm_tn_2cta_kernel<2, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2) == cudaSuccess;
-      ok = ok && cudaFuncSetAttribute(gemm_tn_2cta_kernel<2, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2) == cudaSuccess;
-      if (!ok) return -2;
-      configured2.mark();
-    }
-    const int max_pairs = kNumSM / 2;
+  const int pair_tiles = ((M + P_TILE_M - 1) / P_TILE_M) * ((N + P_TILE_N - 1) / P_TILE_N);
+  if (variant >= kSmall && variant <= kSmall8) {
+    const int log_splits = variant - kSmall;
+    const int tiles = ((M + BM - 1) / BM) * ((N + S_TILE_N - 1) / S_TILE_N);
+    if (launch_small(a_mn, b_mn, tiles, log_splits, smem_small, stream, map_a, map_b, map_c, p) != cudaSuccess) return -3;
+  } else if (variant == kSplit2) {
+    launch_split<2>(a_mn, b_mn, pair_tiles, smem_pair, stream, map_a, map_b, p);
+  } else if (variant == kSplit4) {
+    launch_split<4>(a_mn, b_mn, pair_tiles, smem_pair, stream, map_a, map_b, p);
+  } else {
     // grouped: the number of tiles is known on the device only; every pair looks for work
-    const int tiles = grp != nullptr ? max_pairs : ((M + P_TILE_M - 1) / P_TILE_M) * ((N + P_TILE_N - 1) / P_TILE_N);
-    const int grid = 2 * (tiles < max_pairs ? tiles : max_pairs);
-    if (a_mn && b_mn) gemm_tn_2cta_kernel<2, true, true><<<grid, P_THREADS, smem2, stream>>>(map_a, map_b, p);
-    else if (a_mn) gemm_tn_2cta_kernel<2, true, false><<<grid, P_THREADS, smem2, stream>>>(map_a, map_b, p);
-    else if (b_mn) gemm_tn_2cta_kernel<2, false, true><<<grid, P_THREADS, smem2, stream>>>(map_a, map_b, p);
-    else if (variant == 3) gemm_tn_2cta_kernel<2><<<grid, P_THREADS, smem2, stream>>>(map_a, map_b, p);
-    else gemm_tn_2cta_kernel<1><<<grid, P_THREADS, smem2, stream>>>(map_a, map_b, p);
-    return cudaGetLastError() == cudaSuccess ? 0 : -3;
+    const int tiles = grp != nullptr ? kMaxPairs : pair_tiles;
+    const int grid = 2 * (tiles < kMaxPairs ? tiles : kMaxPairs);
+    if (a_mn && b_mn) gemm_tn_2cta_kernel<2, true, true><<<grid, P_THREADS, smem_pair, stream>>>(map_a, map_b, map_c, map_h, p);
+    else if (a_mn) gemm_tn_2cta_kernel<2, true, false><<<grid, P_THREADS, smem_pair, stream>>>(map_a, map_b, map_c, map_h, p);
+    else if (b_mn) gemm_tn_2cta_kernel<2, false, true><<<grid, P_THREADS, smem_pair, stream>>>(map_a, map_b, map_c, map_h, p);
+    else if (variant == kPair) gemm_tn_2cta_kernel<2><<<grid, P_THREADS, smem_pair, stream>>>(map_a, map_b, map_c, map_h, p);
+    else gemm_tn_2cta_kernel<1><<<grid, P_THREADS, smem_pair, stream>>>(map_a, map_b, map_c, map_h, p);
   }
-  static PerDeviceOnce configured;
-  constexpr int smem_bytes = STAGES * STAGE_BYTES + 1024;
-  if (configured.needed()) {
-    if (cudaFuncSetAttribute(gemm_tn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess) return -2;
-    configured.mark();
-  }
-  const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  const int grid = tiles < kNumSM ? tiles : kNumSM;
-  gemm_tn_kernel<<<grid, THREADS, smem_bytes, stream>>>(map_a, map_b, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
