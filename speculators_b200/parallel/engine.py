@@ -39,6 +39,7 @@ import contextlib
 import logging
 import math
 import os
+import weakref
 from dataclasses import dataclass, field
 
 import torch
@@ -399,7 +400,10 @@ class TrainEngine:
 
     def _install_lazy_zero_hooks(self) -> None:
         def make(p):
+            ref = weakref.ref(p)  # the hook belongs to p: holding p here would keep every parameter alive for good
+
             def on_grad(g):
+                p = ref()
                 if getattr(p, "_grad_fresh", False):
                     p._grad_fresh = False
                     p._flat_grad.zero_()

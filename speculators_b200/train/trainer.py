@@ -23,6 +23,7 @@ import logging
 import os
 import time
 import warnings
+import weakref
 from pathlib import Path
 from typing import Literal, NamedTuple
 
@@ -168,7 +169,7 @@ class _GraphedStep:
     """CUDA-graph capture of forward + backward (+ optimizer) per input signature."""
 
     def __init__(self, trainer: "Trainer", capture_optimizer: bool):
-        self.trainer = trainer
+        self.trainer = weakref.proxy(trainer)  # a trainer's device memory goes when its last user does, not when the collector runs
         self.capture_optimizer = capture_optimizer
         self.cache: dict[tuple, tuple] = {}
         self.launches_per_capture: dict[tuple, int] = {}  # own-kernel launches recorded per graph
