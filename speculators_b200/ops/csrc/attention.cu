@@ -60,6 +60,7 @@ __device__ __forceinline__ void load_tile_async(__nv_bfloat16* smem, const __nv_
 template <int HD>
 __global__ void __launch_bounds__(kAttnThreads)
 attn_fwd_kernel(const AttnParams p) {
+  pdl_begin();
   constexpr int LD = SmemLayout<HD>::LD;
   constexpr int kTile = SmemLayout<HD>::kTile;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -283,6 +284,7 @@ attn_fwd_kernel(const AttnParams p) {
 template <int HD>
 __global__ void __launch_bounds__(kAttnThreads)
 attn_bwd_dq_kernel(const AttnParams p) {
+  pdl_begin();
   constexpr int LD = SmemLayout<HD>::LD;
   constexpr int kTile = SmemLayout<HD>::kTile;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -513,6 +515,7 @@ attn_bwd_dq_kernel(const AttnParams p) {
 __global__ void __launch_bounds__(256)
 kv_tile_range_kernel(const int* __restrict__ lo, const int* __restrict__ hi, int Tq,
                      int Tc, int* __restrict__ qmin, int* __restrict__ qmax) {
+  pdl_begin();
   __shared__ int smin[8], smax[8];
   const int k0 = blockIdx.x * kBN, k1 = k0 + kBN;
   int mn = 0x7fffffff, mx = 0;
@@ -560,6 +563,7 @@ constexpr int kDkvCols = HD > 128 ? 128 : HD;
 template <int HD>
 __global__ void __launch_bounds__(kAttnThreads)
 attn_bwd_dkv_kernel(const AttnParams p) {
+  pdl_begin();
   constexpr int HDO = kDkvCols<HD>;
   const int c0 = blockIdx.z * HDO;  // first dK / dV column of this CTA
   constexpr int LD = SmemLayout<HD>::LD;
@@ -746,6 +750,7 @@ attn_bwd_dkv_kernel(const AttnParams p) {
 // part: [group, 2, n] fp32 with n = Tc * nkv * HD (n % 8 == 0); dk, dv: [n] bf16.
 __global__ void __launch_bounds__(256)
 dkv_reduce_kernel(const float* __restrict__ part, int group, int64_t n, __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv) {
+  pdl_begin();
   const int64_t nvec = n >> 3;
   for (int64_t vi = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; vi < 2 * nvec; vi += (int64_t)gridDim.x * blockDim.x) {
     const int which = vi >= nvec;
@@ -780,7 +785,7 @@ static int launch_fwd_t(const AttnParams& p, cudaStream_t stream) {
   }
   dim3 grid((p.Tq + kBM - 1) / kBM, p.nh);
   count_launch(1);
-  attn_fwd_kernel<HD><<<grid, kAttnThreads, fwd_smem<HD>(), stream>>>(p);
+  launch_pdl(attn_fwd_kernel<HD>, grid, kAttnThreads, fwd_smem<HD>(), stream, p);
   return 0;
 }
 
@@ -795,15 +800,15 @@ static int launch_bwd_t(const AttnParams& p, int* tile_qmin, int* tile_qmax, cud
   const int n_kv_tiles = (p.Tc + kBN - 1) / kBN;
   count_launch(3);
   dim3 grid_q((p.Tq + kBM - 1) / kBM, p.nh);
-  attn_bwd_dq_kernel<HD><<<grid_q, kAttnThreads, bwd_smem<HD>(), stream>>>(p);
-  kv_tile_range_kernel<<<n_kv_tiles, 256, 0, stream>>>(p.lo, p.hi, p.Tq, p.Tc, tile_qmin, tile_qmax);
+  launch_pdl(attn_bwd_dq_kernel<HD>, grid_q, kAttnThreads, bwd_smem<HD>(), stream, p);
+  launch_pdl(kv_tile_range_kernel, n_kv_tiles, 256, 0, stream, p.lo, p.hi, p.Tq, p.Tc, tile_qmin, tile_qmax);
   dim3 grid_kv(p.nh, n_kv_tiles, HD / kDkvCols<HD>);  // x = head: all heads of the heaviest tile are dispatched first; z = output column part
-  attn_bwd_dkv_kernel<HD><<<grid_kv, kAttnThreads, bwd_smem<HD>(), stream>>>(p);
+  launch_pdl(attn_bwd_dkv_kernel<HD>, grid_kv, kAttnThreads, bwd_smem<HD>(), stream, p);
   if (p.dkv_part != nullptr) {
     const int64_t n = (int64_t)p.Tc * p.nkv * HD;
     const int64_t blocks = (2 * (n >> 3) + 255) / 256;
     count_launch(1);
-    dkv_reduce_kernel<<<(int)(blocks < 8 * kNumSM ? blocks : 8 * kNumSM), 256, 0, stream>>>(p.dkv_part, p.nh / p.nkv, n, p.dk, p.dv);
+    launch_pdl(dkv_reduce_kernel, (int)(blocks < 8 * kNumSM ? blocks : 8 * kNumSM), 256, 0, stream, p.dkv_part, p.nh / p.nkv, n, p.dk, p.dv);
   }
   return 0;
 }
@@ -811,7 +816,7 @@ static int launch_bwd_t(const AttnParams& p, int* tile_qmin, int* tile_qmax, cud
 int launch_kv_tile_range(const AttnParams& p, int* tile_qmin, int* tile_qmax, cudaStream_t stream) {
   const int n_kv_tiles = (p.Tc + kBN - 1) / kBN;
   count_launch(1);
-  kv_tile_range_kernel<<<n_kv_tiles, 256, 0, stream>>>(p.lo, p.hi, p.Tq, p.Tc, tile_qmin, tile_qmax);
+  launch_pdl(kv_tile_range_kernel, n_kv_tiles, 256, 0, stream, p.lo, p.hi, p.Tq, p.Tc, tile_qmin, tile_qmax);
   return 0;
 }
 
@@ -819,7 +824,7 @@ int launch_dkv_reduce(const AttnParams& p, cudaStream_t stream) {
   const int64_t n = (int64_t)p.Tc * p.nkv * 128;
   const int64_t blocks = (2 * (n >> 3) + 255) / 256;
   count_launch(1);
-  dkv_reduce_kernel<<<(int)(blocks < 8 * kNumSM ? blocks : 8 * kNumSM), 256, 0, stream>>>(p.dkv_part, p.nh / p.nkv, n, p.dk, p.dv);
+  launch_pdl(dkv_reduce_kernel, (int)(blocks < 8 * kNumSM ? blocks : 8 * kNumSM), 256, 0, stream, p.dkv_part, p.nh / p.nkv, n, p.dk, p.dv);
   return 0;
 }
 

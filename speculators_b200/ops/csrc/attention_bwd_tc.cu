@@ -90,6 +90,7 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ out, float* __restrict__ delta, int Tq, int nh,
                   int64_t do_rs, int64_t o_rs) {
+  pdl_begin();
   const int lane = threadIdx.x & 31, sub = lane >> 4, l16 = lane & 15;
   const int64_t n = (int64_t)Tq * nh;
   for (int64_t base = ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * 2; base < n; base += (int64_t)gridDim.x * 16) {
@@ -161,6 +162,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   __syncthreads();
   fence_after_sync();
   const uint32_t tmem_base = tmem_base_slot;
+  pdl_begin();
   // TMEM columns: S [0,128)  dP [128,256)  dQ [256,384)  dS of even / odd tiles [384,448) [448,512)
   constexpr uint32_t COL_S = 0, COL_DP = 128, COL_DQ = 256, COL_DS = 384;
 
@@ -193,7 +195,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   const int n_tiles = n_ctx + (p.ext_block > 0 ? 1 : 0);
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t qb = smem_addr(&bar_qdo);
       mbar_expect_tx(qb, 2 * TILE_BYTES);
       tma_load_2d(smem_addr(q_s), &map_q, qb, h * HD, q0);
@@ -220,7 +222,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && n_tiles > 0) {
+    if (n_tiles > 0 && elect_one()) {
       constexpr uint32_t idesc_kk = instr_desc(BM, BN, false);
       constexpr uint32_t idesc_mn = instr_desc(BM, HD, true);
       const uint32_t qa = smem_addr(q_s), da = smem_addr(do_s);
@@ -494,6 +496,7 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   __syncthreads();
   fence_after_sync();
   const uint32_t tmem_base = tmem_base_slot;
+  pdl_begin();
   // TMEM columns: S^T [0,128)  dP^T [128,256)  dV [256,384)  dK [384,512); P^T / dS^T reuse
   // columns [0,32) + [64,96) of the S^T / dP^T block
   constexpr uint32_t COL_ST = 0, COL_DPT = 128, COL_DV = 256, COL_DK = 384;
@@ -513,7 +516,7 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   const int n_keys = ext_mode ? p.Te : p.Tc;
 
   if (warp == 0) {
-    if (lane == 0 && n_tiles > 0) {
+    if (n_tiles > 0 && elect_one()) {
       const uint32_t kvb = smem_addr(&bar_kv);
       mbar_expect_tx(kvb, 2 * TILE_BYTES);
       tma_load_2d(smem_addr(k_s), &map_k, kvb, kvh * HD, key_base);
@@ -534,7 +537,7 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && n_tiles > 0) {
+    if (n_tiles > 0 && elect_one()) {
       constexpr uint32_t idesc_kk = instr_desc(BN, BM, false);
       constexpr uint32_t idesc_mn = instr_desc(BN, HD, true);
       const uint32_t ka = smem_addr(k_s), va = smem_addr(v_s);
@@ -783,18 +786,18 @@ int launch_attn_bwd_tc(const AttnParams& p, int* tile_qmin, int* tile_qmax, int*
   {
     const int64_t pairs = (int64_t)p.Tq * p.nh;
     const int64_t blocks = (pairs + 15) / 16;
-    attn_delta_kernel<<<(int)(blocks < 16 * kNumSM ? blocks : 16 * kNumSM), 256, 0, stream>>>(p.dout, p.out, p.delta, p.Tq, p.nh, p.do_rs, p.o_rs);
+    launch_pdl(attn_delta_kernel, (int)(blocks < 16 * kNumSM ? blocks : 16 * kNumSM), 256, 0, stream, p.dout, p.out, p.delta, p.Tq, p.nh, p.do_rs, p.o_rs);
   }
   dim3 grid_q(p.nh, (p.Tq + BM - 1) / BM);
-  attn_bwd_dq_tc_kernel<<<grid_q, THREADS, SMEM_BYTES, stream>>>(map_q, map_do, map_k, map_v, map_ke, map_ve, p, status);
+  launch_pdl(attn_bwd_dq_tc_kernel, grid_q, THREADS, SMEM_BYTES, stream, map_q, map_do, map_k, map_v, map_ke, map_ve, p, status);
   rc = launch_kv_tile_range(p, tile_qmin, tile_qmax, stream);
   if (rc) return rc;
   dim3 grid_kv(p.nh, (p.Tc + BN - 1) / BN);
-  attn_bwd_dkv_tc_kernel<<<grid_kv, THREADS, SMEM_BYTES, stream>>>(map_q, map_do, map_k, map_v, p, (p.Tc + kAttnKeyTile - 1) / kAttnKeyTile, 0, status);
+  launch_pdl(attn_bwd_dkv_tc_kernel, grid_kv, THREADS, SMEM_BYTES, stream, map_q, map_do, map_k, map_v, p, (p.Tc + kAttnKeyTile - 1) / kAttnKeyTile, 0, status);
   if (p.ext_block > 0) {  // gradients of the extra keys: one key tile per query tile, read from the extra tensors
     count_launch(1);
     dim3 grid_ext(p.nh, (p.Te + BN - 1) / BN);
-    attn_bwd_dkv_tc_kernel<<<grid_ext, THREADS, SMEM_BYTES, stream>>>(map_q, map_do, map_ke, map_ve, p, 0, 1, status);
+    launch_pdl(attn_bwd_dkv_tc_kernel, grid_ext, THREADS, SMEM_BYTES, stream, map_q, map_do, map_ke, map_ve, p, 0, 1, status);
   }
   if (p.dkv_part != nullptr) {
     rc = launch_dkv_reduce(p, stream);

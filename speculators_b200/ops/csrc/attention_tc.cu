@@ -85,6 +85,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   __syncthreads();
   fence_after_sync();
   const uint32_t tmem_base = tmem_base_slot;
+  pdl_begin();
 
   // key range of the CTA: union of the rows' intervals
   int my_lo = 0x7fffffff, my_hi = 0;
@@ -116,7 +117,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0 && (n_tiles > 0 || p.E > 0)) {
+    if ((n_tiles > 0 || p.E > 0) && elect_one()) {
       const uint32_t qb = smem_addr(&bar_q);
       mbar_expect_tx(qb, TILE_BYTES);
       tma_load_2d(smem_addr(q_s), &map_q, qb, h * HD, q0);
@@ -145,7 +146,7 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && n_tiles > 0) {
+    if (n_tiles > 0 && elect_one()) {
       constexpr uint32_t idesc_s = instr_desc(BM, BN, false);  // S = Q K^T: both operands K-major
       constexpr uint32_t idesc_o = instr_desc(BM, HD, true);   // O = P V: V tile is MN-major
       const uint32_t qa = smem_addr(q_s);
@@ -442,7 +443,7 @@ int launch_attn_fwd_tc(const AttnParams& p, int* status, cudaStream_t stream) {
   }
   dim3 grid(p.nh, (p.Tq + BM - 1) / BM);
   count_launch(1);
-  attn_fwd_tc_kernel<<<grid, THREADS, smem_bytes, stream>>>(map_q, map_k, map_v, map_ke, map_ve, p, status);
+  launch_pdl(attn_fwd_tc_kernel, grid, THREADS, smem_bytes, stream, map_q, map_k, map_v, map_ke, map_ve, p, status);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 

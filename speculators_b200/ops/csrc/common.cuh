@@ -63,6 +63,35 @@ struct PerDeviceOnce {
   void mark() { const int d = device(); if (d >= 0) done[d] = true; }
 };
 
+// Programmatic dependent launch.  A step is a chain of hundreds of short kernels; launched the plain way each one
+// starts (scheduling, barrier and tensor-memory set-up: 2 to 3 us) only after its predecessor has drained.  Launched
+// through launch_pdl a kernel's blocks come up while the predecessor still runs and wait in pdl_begin until it has
+// completed and its writes are visible.  Every kernel launched so calls pdl_begin in all threads before it touches
+// global memory (also one that needs no data of its predecessor: the next kernel relies on this one's wait for
+// everything before it).
+__device__ __forceinline__ void pdl_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+inline cudaLaunchAttribute pdl_attribute() {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  return attr;
+}
+template <typename... Params, typename... Args>
+inline cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+  cudaLaunchAttribute attr = pdl_attribute();
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 struct alignas(16) bf16x8 {
   __nv_bfloat162 v[4];
 };

@@ -7,6 +7,7 @@ namespace sb200 {
 // (the gate and up projections run as one GEMM).  h = silu(gate) * up.
 __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gate_up,
                                   __nv_bfloat16* __restrict__ h, int64_t rows, int I) {
+  pdl_begin();
   const int nvec = I >> 3;
   const int64_t total = rows * nvec;
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -31,6 +32,7 @@ __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gate_up,
 __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dh,
                                   const __nv_bfloat16* __restrict__ gate_up,
                                   __nv_bfloat16* __restrict__ dgate_up, int64_t rows, int I) {
+  pdl_begin();
   const int nvec = I >> 3;
   const int64_t total = rows * nvec;
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -64,6 +66,7 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const int64_t* __rest
                             const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                             int64_t tokens, int heads, int hd, int rot, int64_t row_stride,
                             int64_t max_pos, float sign) {
+  pdl_begin();
   const int half = rot >> 1;
   const int64_t total = tokens * heads * half;
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -90,6 +93,7 @@ __global__ void rope_vec8_kernel(__nv_bfloat16* __restrict__ x, const int64_t* _
                                  const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                                  int64_t tokens, int heads, int hd, int rot, int64_t row_stride,
                                  int64_t max_pos, float sign) {
+  pdl_begin();
   const int half = rot >> 1;
   const int hv = half >> 3;
   const int64_t total = tokens * heads * hv;
@@ -130,14 +134,14 @@ static inline int grid_for(int64_t total, int threads) {
 void launch_swiglu_fwd(const void* gate_up, void* h, int64_t rows, int I, cudaStream_t stream) {
   if (rows <= 0) return;
   count_launch(1);
-  swiglu_fwd_kernel<<<grid_for(rows * (I >> 3), 256), 256, 0, stream>>>(
+  launch_pdl(swiglu_fwd_kernel, grid_for(rows * (I >> 3), 256), 256, 0, stream, 
       (const __nv_bfloat16*)gate_up, (__nv_bfloat16*)h, rows, I);
 }
 void launch_swiglu_bwd(const void* dh, const void* gate_up, void* dgate_up, int64_t rows, int I,
                        cudaStream_t stream) {
   if (rows <= 0) return;
   count_launch(1);
-  swiglu_bwd_kernel<<<grid_for(rows * (I >> 3), 256), 256, 0, stream>>>(
+  launch_pdl(swiglu_bwd_kernel, grid_for(rows * (I >> 3), 256), 256, 0, stream, 
       (const __nv_bfloat16*)dh, (const __nv_bfloat16*)gate_up, (__nv_bfloat16*)dgate_up, rows, I);
 }
 void launch_rope(void* x, const int64_t* positions, const float* cos_t, const float* sin_t,
@@ -149,11 +153,11 @@ void launch_rope(void* x, const int64_t* positions, const float* cos_t, const fl
   const bool vec = (half % 8 == 0) && (hd % 8 == 0) && (row_stride % 8 == 0) && ((uintptr_t)x % 16 == 0) &&
                    ((uintptr_t)cos_t % 16 == 0) && ((uintptr_t)sin_t % 16 == 0);
   if (vec) {
-    rope_vec8_kernel<<<grid_for(tokens * heads * (half >> 3), 256), 256, 0, stream>>>(
+    launch_pdl(rope_vec8_kernel, grid_for(tokens * heads * (half >> 3), 256), 256, 0, stream, 
         (__nv_bfloat16*)x, positions, cos_t, sin_t, tokens, heads, hd, rot, row_stride, max_pos, sign);
     return;
   }
-  rope_kernel<<<grid_for(tokens * heads * half, 256), 256, 0, stream>>>(
+  launch_pdl(rope_kernel, grid_for(tokens * heads * half, 256), 256, 0, stream, 
       (__nv_bfloat16*)x, positions, cos_t, sin_t, tokens, heads, hd, rot, row_stride, max_pos, sign);
 }
 

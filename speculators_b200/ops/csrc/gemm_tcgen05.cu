@@ -523,6 +523,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   __syncthreads();
   fence_after_sync();
   const uint32_t tmem_base = tmem_base_slot;
+  pdl_begin();
   if (log_splits > 0) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // waited for before the first remote store
 
   bool ok = true;
@@ -679,9 +680,6 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   const bool leader = rank == 0;
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   const int tiles_m = (p.M + P_TILE_M - 1) / P_TILE_M, tiles_n = (p.N + P_TILE_N - 1) / P_TILE_N;
-  const int num_tiles = p.grp.mode == kGroupRows ? p.grp.tile_start[p.grp.num_groups] * tiles_n
-                        : p.grp.mode == kGroupK  ? p.grp.num_groups * tiles_m * tiles_n
-                                                 : tiles_m * tiles_n;
   const int num_kb = (p.K + STAGE_K - 1) / STAGE_K;
 
   if (threadIdx.x == 0) {
@@ -703,6 +701,10 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   cluster_sync_all();  // barriers of both CTAs are initialised before any remote signal
   fence_after_sync();
   const uint32_t tmem_base = tmem_base_slot;
+  pdl_begin();
+  const int num_tiles = p.grp.mode == kGroupRows ? p.grp.tile_start[p.grp.num_groups] * tiles_n
+                        : p.grp.mode == kGroupK  ? p.grp.num_groups * tiles_m * tiles_n
+                                                 : tiles_m * tiles_n;
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (both CTAs)
@@ -865,6 +867,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   cluster_sync_all();
   fence_after_sync();
   const uint32_t tmem_base = tmem_base_slot;
+  pdl_begin();
 
   bool ok = true;
   const int quarter = warp & 3, chalf = (warp - 2) >> 2;
@@ -980,10 +983,10 @@ static bool allow_smem(Kernel kernel, int bytes) {
 template <int SPLITS>
 static void launch_split(int a_mn, int b_mn, int tiles, int smem, cudaStream_t stream, const CUtensorMap& map_a, const CUtensorMap& map_b, const tc::Params& p) {
   const int grid = tiles * 2 * SPLITS;
-  if (a_mn && b_mn) tc::gemm_split_kernel<SPLITS, true, true><<<grid, tc::P_THREADS, smem, stream>>>(map_a, map_b, p);
-  else if (a_mn) tc::gemm_split_kernel<SPLITS, true, false><<<grid, tc::P_THREADS, smem, stream>>>(map_a, map_b, p);
-  else if (b_mn) tc::gemm_split_kernel<SPLITS, false, true><<<grid, tc::P_THREADS, smem, stream>>>(map_a, map_b, p);
-  else tc::gemm_split_kernel<SPLITS, false, false><<<grid, tc::P_THREADS, smem, stream>>>(map_a, map_b, p);
+  if (a_mn && b_mn) launch_pdl(tc::gemm_split_kernel<SPLITS, true, true>, grid, tc::P_THREADS, smem, stream, map_a, map_b, p);
+  else if (a_mn) launch_pdl(tc::gemm_split_kernel<SPLITS, true, false>, grid, tc::P_THREADS, smem, stream, map_a, map_b, p);
+  else if (b_mn) launch_pdl(tc::gemm_split_kernel<SPLITS, false, true>, grid, tc::P_THREADS, smem, stream, map_a, map_b, p);
+  else launch_pdl(tc::gemm_split_kernel<SPLITS, false, false>, grid, tc::P_THREADS, smem, stream, map_a, map_b, p);
 }
 
 static cudaError_t launch_small(int a_mn, int b_mn, int tiles, int log_splits, int smem, cudaStream_t stream, const CUtensorMap& map_a, const CUtensorMap& map_b,
@@ -993,12 +996,13 @@ static cudaError_t launch_small(int a_mn, int b_mn, int tiles, int log_splits, i
   cfg.blockDim = dim3(tc::S_THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = 1u << log_splits;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = log_splits > 0 ? 1 : 0;
+  cudaLaunchAttribute attr[2] = {};
+  attr[0] = pdl_attribute();
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 1u << log_splits;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = log_splits > 0 ? 2 : 1;
   if (a_mn && b_mn) return cudaLaunchKernelEx(&cfg, tc::gemm_small_kernel<true, true>, map_a, map_b, map_c, p, log_splits);
   if (a_mn) return cudaLaunchKernelEx(&cfg, tc::gemm_small_kernel<true, false>, map_a, map_b, map_c, p, log_splits);
   if (b_mn) return cudaLaunchKernelEx(&cfg, tc::gemm_small_kernel<false, true>, map_a, map_b, map_c, p, log_splits);
@@ -1159,11 +1163,11 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
     // grouped: the number of tiles is known on the device only; every pair looks for work
     const int tiles = grp != nullptr ? kMaxPairs : pair_tiles;
     const int grid = 2 * (tiles < kMaxPairs ? tiles : kMaxPairs);
-    if (a_mn && b_mn) gemm_tn_2cta_kernel<2, true, true><<<grid, P_THREADS, smem_pair, stream>>>(map_a, map_b, map_c, map_h, p);
-    else if (a_mn) gemm_tn_2cta_kernel<2, true, false><<<grid, P_THREADS, smem_pair, stream>>>(map_a, map_b, map_c, map_h, p);
-    else if (b_mn) gemm_tn_2cta_kernel<2, false, true><<<grid, P_THREADS, smem_pair, stream>>>(map_a, map_b, map_c, map_h, p);
-    else if (variant == kPair) gemm_tn_2cta_kernel<2><<<grid, P_THREADS, smem_pair, stream>>>(map_a, map_b, map_c, map_h, p);
-    else gemm_tn_2cta_kernel<1><<<grid, P_THREADS, smem_pair, stream>>>(map_a, map_b, map_c, map_h, p);
+    if (a_mn && b_mn) launch_pdl(gemm_tn_2cta_kernel<2, true, true>, grid, P_THREADS, smem_pair, stream, map_a, map_b, map_c, map_h, p);
+    else if (a_mn) launch_pdl(gemm_tn_2cta_kernel<2, true, false>, grid, P_THREADS, smem_pair, stream, map_a, map_b, map_c, map_h, p);
+    else if (b_mn) launch_pdl(gemm_tn_2cta_kernel<2, false, true>, grid, P_THREADS, smem_pair, stream, map_a, map_b, map_c, map_h, p);
+    else if (variant == kPair) launch_pdl(gemm_tn_2cta_kernel<2>, grid, P_THREADS, smem_pair, stream, map_a, map_b, map_c, map_h, p);
+    else launch_pdl(gemm_tn_2cta_kernel<1>, grid, P_THREADS, smem_pair, stream, map_a, map_b, map_c, map_h, p);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
@@ -1204,6 +1208,7 @@ int launch_gemm_swiglu(const void* x, const void* w, void* gate_up, void* h, int
 // counts[e] rows belong to expert e.  seg[e] = offset of its (128-row aligned) segment in the padded
 // row order, mtile_start[e] = prefix sum of ceil(segment rows / 256).  One block; E <= 4096.
 __global__ void moe_group_plan_kernel(const int* __restrict__ counts, int num_groups, int* __restrict__ seg, int* __restrict__ mtile_start) {
+  pdl_begin();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   int off = 0, tiles = 0;
   for (int e = 0; e < num_groups; ++e) {
@@ -1219,7 +1224,7 @@ __global__ void moe_group_plan_kernel(const int* __restrict__ counts, int num_gr
 
 void launch_moe_group_plan(const int* counts, int num_groups, int* seg, int* mtile_start, cudaStream_t stream) {
   count_launch(1);
-  moe_group_plan_kernel<<<1, 32, 0, stream>>>(counts, num_groups, seg, mtile_start);
+  launch_pdl(moe_group_plan_kernel, 1, 32, 0, stream, counts, num_groups, seg, mtile_start);
 }
 
 // mode 1 (rows grouped): c[R, N] = a[R, K] . b_e^T, b the stack [E, N, K] (b_mn 0) or, for the input
@@ -1254,6 +1259,7 @@ __global__ void __launch_bounds__(128)
 lmhead_combine_kernel(const float* __restrict__ partial, const __nv_bfloat16* __restrict__ logits, const uint8_t* __restrict__ active,
                       float* __restrict__ loss, float* __restrict__ stats, int* __restrict__ argmax_d, int* __restrict__ argmax_t,
                       int rows, int tiles_n, int64_t ld_logits, int op) {
+  pdl_begin();
   const int r = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (r >= rows) return;
   float* st = stats + r;
@@ -1310,7 +1316,7 @@ int launch_lmhead_combine(const float* partial, const void* logits, const uint8_
   if (rows <= 0) return 0;
   if (op != 0 && op != 3) return -1;
   count_launch(1);
-  lmhead_combine_kernel<<<(rows + 3) / 4, 128, 0, stream>>>(partial, (const __nv_bfloat16*)logits, active, loss, stats, argmax_d, argmax_t, rows,
+  launch_pdl(lmhead_combine_kernel, (rows + 3) / 4, 128, 0, stream, partial, (const __nv_bfloat16*)logits, active, loss, stats, argmax_d, argmax_t, rows,
                                                           tiles_n, ld_logits, op);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }

@@ -82,6 +82,7 @@ loss_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* _
                 float* __restrict__ loss, float* __restrict__ stats, int* __restrict__ argmax_d,
                 int* __restrict__ argmax_t, int rows, int V, int64_t ld_logits, int64_t ld_targets,
                 int shift) {
+  pdl_begin();
   __shared__ float scratch[33];
   __shared__ int iscratch[33];
   const int r = blockIdx.x;
@@ -209,6 +210,7 @@ loss_bwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* _
                 const float* __restrict__ grad_out, const float* __restrict__ stats,
                 __nv_bfloat16* __restrict__ dlogits, int rows, int total_rows, int V,
                 int64_t ld_logits, int64_t ld_targets, int64_t ld_dlogits, int shift) {
+  pdl_begin();
   const int r = blockIdx.x;
   if (r >= total_rows) return;
   __nv_bfloat16* d = dlogits + (int64_t)r * ld_dlogits;
@@ -270,7 +272,7 @@ int launch_loss_fwd(int op, const void* logits, const void* targets, const uint8
   if (targets == nullptr && (labels == nullptr || op != kOpCE)) return -3;
   count_launch(1);
 #define SB200_LF(OPV)                                                                            \
-  loss_fwd_kernel<OPV><<<rows, kLossThreads, 0, stream>>>(                                        \
+  launch_pdl(loss_fwd_kernel<OPV>, rows, kLossThreads, 0, stream,                                         \
       (const __nv_bfloat16*)logits, (const __nv_bfloat16*)targets, active, labels, loss, stats,   \
       argmax_d, argmax_t, rows, V, ld_logits, ld_targets, shift)
   switch (op) {
@@ -292,7 +294,7 @@ int launch_loss_bwd(int op, const void* logits, const void* targets, const float
   if (total_rows <= 0) return 0;
   count_launch(1);
 #define SB200_LB(OPV)                                                                         \
-  loss_bwd_kernel<OPV><<<total_rows, kLossThreads, 0, stream>>>(                               \
+  launch_pdl(loss_bwd_kernel<OPV>, total_rows, kLossThreads, 0, stream,                                \
       (const __nv_bfloat16*)logits, (const __nv_bfloat16*)targets, grad_out, stats,            \
       (__nv_bfloat16*)dlogits, rows, total_rows, V, ld_logits, ld_targets, ld_dlogits, shift)
   switch (op) {

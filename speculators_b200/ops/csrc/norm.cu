@@ -25,6 +25,7 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
                    const int64_t* __restrict__ row_index, __nv_bfloat16* __restrict__ y,
                    float* __restrict__ rstd_out, int rows, int H, int64_t x_stride,
                    int64_t y_stride, float eps, int64_t src_rows) {
+  pdl_begin();
   __shared__ float scratch[33];
   const int nvec = H >> 3;
   for (int r = blockIdx.x; r < rows; r += gridDim.x) {
@@ -73,6 +74,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
                    const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd_in,
                    __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_partial, int rows, int H,
                    int64_t dy_stride, int64_t x_stride, int64_t dx_stride, int accumulate_dx) {
+  pdl_begin();
   __shared__ float scratch[33];
   const int nvec = H >> 3;
   float dwacc[NV][8];
@@ -179,6 +181,7 @@ constexpr int kNarrowWarps = kNormThreads / 32;
 __global__ void __launch_bounds__(kNormThreads)
 rmsnorm_fwd_narrow_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
                           float* __restrict__ rstd_out, int rows, int H, int64_t x_stride, int64_t y_stride, float eps) {
+  pdl_begin();
   const int lane = threadIdx.x & 31, nvec = H >> 3;
   const bool on = lane < nvec;
   float wv[8];
@@ -208,6 +211,7 @@ __global__ void __launch_bounds__(kNormThreads)
 rmsnorm_bwd_narrow_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                           const float* __restrict__ rstd_in, __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_partial, int rows, int H,
                           int64_t dy_stride, int64_t x_stride, int64_t dx_stride, int accumulate_dx) {
+  pdl_begin();
   const int lane = threadIdx.x & 31, nvec = H >> 3;
   const bool on = lane < nvec;
   float wv[8], dwacc[8];
@@ -259,6 +263,7 @@ static int narrow_grid(int rows) {
 constexpr int kColsumGroups = 32;
 __global__ void __launch_bounds__(32 * kColsumGroups)
 colsum_kernel(const float* __restrict__ partial, float* __restrict__ dw, int P, int H, int accumulate) {
+  pdl_begin();
   __shared__ float tile[kColsumGroups][33];
   const int c = blockIdx.x * 32 + threadIdx.x;
   float s = 0.f;
@@ -291,13 +296,13 @@ void launch_rmsnorm_fwd(const void* x, const void* w, const int64_t* row_index, 
   if (rows <= 0) return;
   if (H <= kNarrowMaxH && row_index == nullptr) {
     count_launch(1);
-    rmsnorm_fwd_narrow_kernel<<<narrow_grid(rows), kNormThreads, 0, stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
+    launch_pdl(rmsnorm_fwd_narrow_kernel, narrow_grid(rows), kNormThreads, 0, stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
                                                                              (__nv_bfloat16*)y, rstd, rows, H, x_stride, y_stride, eps);
     return;
   }
   int grid = rows < 8 * kNumSM ? rows : 8 * kNumSM;
 #define SB200_FWD(NVV)                                                                         \
-  rmsnorm_fwd_kernel<NVV><<<grid, kNormThreads, 0, stream>>>(                                    \
+  launch_pdl(rmsnorm_fwd_kernel<NVV>, grid, kNormThreads, 0, stream,                                     \
       (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, row_index, (__nv_bfloat16*)y, rstd, rows, \
       H, x_stride, y_stride, eps, src_rows)
   count_launch(1);
@@ -315,18 +320,18 @@ void launch_rmsnorm_bwd(const void* dy, const void* x, const void* w, const floa
   if (H <= kNarrowMaxH) {
     const int g = narrow_grid(rows);
     count_launch(1);
-    rmsnorm_bwd_narrow_kernel<<<g, kNormThreads, 0, stream>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd,
+    launch_pdl(rmsnorm_bwd_narrow_kernel, g, kNormThreads, 0, stream, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd,
                                                             (__nv_bfloat16*)dx, dw_partial, rows, H, dy_stride, x_stride, dx_stride,
                                                             accumulate_dx);
     if (dw_partial && dw) {
       count_launch(1);
-      colsum_kernel<<<(H + 31) / 32, dim3(32, kColsumGroups), 0, stream>>>(dw_partial, dw, g * kNarrowWarps, H, accumulate_dw);
+      launch_pdl(colsum_kernel, (H + 31) / 32, dim3(32, kColsumGroups), 0, stream, dw_partial, dw, g * kNarrowWarps, H, accumulate_dw);
     }
     return;
   }
   const int grid = rmsnorm_bwd_partial_rows(rows, H);
 #define SB200_BWD(NVV)                                                                       \
-  rmsnorm_bwd_kernel<NVV><<<grid, kNormThreads, 0, stream>>>(                                  \
+  launch_pdl(rmsnorm_bwd_kernel<NVV>, grid, kNormThreads, 0, stream,                                   \
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd,         \
       (__nv_bfloat16*)dx, dw_partial, rows, H, dy_stride, x_stride, dx_stride, accumulate_dx)
   count_launch(1);
@@ -336,7 +341,7 @@ void launch_rmsnorm_bwd(const void* dy, const void* x, const void* w, const floa
 #undef SB200_BWD
   if (dw_partial && dw) count_launch(1);
   if (dw_partial && dw)
-    colsum_kernel<<<(H + 31) / 32, dim3(32, kColsumGroups), 0, stream>>>(dw_partial, dw, grid, H, accumulate_dw);
+    launch_pdl(colsum_kernel, (H + 31) / 32, dim3(32, kColsumGroups), 0, stream, dw_partial, dw, grid, H, accumulate_dw);
 }
 
 }  // namespace sb200

@@ -30,6 +30,7 @@ __device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 v) { return _
 template <typename T>
 __global__ void __launch_bounds__(kOptThreads)
 sumsq_partial_kernel(const T* __restrict__ g, int64_t n, float* __restrict__ partial) {
+  pdl_begin();
   __shared__ float scratch[33];
   float acc = 0.f;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -45,6 +46,7 @@ template <>
 __global__ void __launch_bounds__(kOptThreads)
 sumsq_partial_kernel<__nv_bfloat16>(const __nv_bfloat16* __restrict__ g, int64_t n,
                                      float* __restrict__ partial) {
+  pdl_begin();
   __shared__ float scratch[33];
   float acc = 0.f;
   const int64_t nvec = n >> 3;  // buffer base is 16-byte aligned by construction
@@ -67,6 +69,7 @@ sumsq_partial_kernel<__nv_bfloat16>(const __nv_bfloat16* __restrict__ g, int64_t
 // Stage 2: out[0] (+)= sum(partial[0:P]) in a fixed order (deterministic).
 __global__ void sumsq_final_kernel(const float* __restrict__ partial, int P, float* __restrict__ out,
                                    int accumulate) {
+  pdl_begin();
   __shared__ float scratch[33];
   float acc = 0.f;
   for (int i = threadIdx.x; i < P; i += blockDim.x) acc += partial[i];
@@ -81,6 +84,7 @@ __global__ void __launch_bounds__(kOptThreads)
 adamw_kernel(float* __restrict__ master, float* __restrict__ m, float* __restrict__ v,
              const G* __restrict__ grad, __nv_bfloat16* __restrict__ w16, int64_t n,
              const float* __restrict__ hyper, const float* __restrict__ norm_sq) {
+  pdl_begin();
   const float lr = hyper[0], b1 = hyper[1], b2 = hyper[2], eps = hyper[3], wd = hyper[4];
   const float bc1 = hyper[5], bc2 = hyper[6], max_norm = hyper[7];
   float gscale = hyper[8];
@@ -122,6 +126,7 @@ __global__ void __launch_bounds__(kOptThreads)
 muon_momentum_kernel(const G* __restrict__ grad, float* __restrict__ buf, __nv_bfloat16* __restrict__ out, int64_t n,
                      const float* __restrict__ hyper, const float* __restrict__ norm_sq, float momentum, int nesterov,
                      float* __restrict__ partial) {
+  pdl_begin();
   __shared__ float scratch[33];
   const float max_norm = hyper[7];
   float gscale = hyper[8];
@@ -148,6 +153,7 @@ muon_momentum_kernel(const G* __restrict__ grad, float* __restrict__ buf, __nv_b
 __global__ void __launch_bounds__(kOptThreads)
 muon_apply_kernel(float* __restrict__ master, const __nv_bfloat16* __restrict__ update, __nv_bfloat16* __restrict__ w16, int64_t n,
                   const float* __restrict__ hyper, float lr_ratio, float weight_decay, float adjust) {
+  pdl_begin();
   const float lr = hyper[0] * lr_ratio;
   const float keep = 1.f - lr * weight_decay, step = lr * adjust;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -165,12 +171,12 @@ void launch_muon_momentum(const void* grad, int grad_is_bf16, float* buf, void* 
   const int P = 4 * kNumSM;
   count_launch(2);
   if (grad_is_bf16)
-    muon_momentum_kernel<__nv_bfloat16><<<P, kOptThreads, 0, stream>>>((const __nv_bfloat16*)grad, buf, (__nv_bfloat16*)out, n, hyper,
+    launch_pdl(muon_momentum_kernel<__nv_bfloat16>, P, kOptThreads, 0, stream, (const __nv_bfloat16*)grad, buf, (__nv_bfloat16*)out, n, hyper,
                                                                        norm_sq, momentum, nesterov, partial);
   else
-    muon_momentum_kernel<float><<<P, kOptThreads, 0, stream>>>((const float*)grad, buf, (__nv_bfloat16*)out, n, hyper, norm_sq,
+    launch_pdl(muon_momentum_kernel<float>, P, kOptThreads, 0, stream, (const float*)grad, buf, (__nv_bfloat16*)out, n, hyper, norm_sq,
                                                                momentum, nesterov, partial);
-  sumsq_final_kernel<<<1, 256, 0, stream>>>(partial, P, out_sumsq, 0);
+  launch_pdl(sumsq_final_kernel, 1, 256, 0, stream, partial, P, out_sumsq, 0);
 }
 
 void launch_muon_apply(float* master, const void* update, void* w16, int64_t n, const float* hyper, float lr_ratio,
@@ -179,7 +185,7 @@ void launch_muon_apply(float* master, const void* update, void* w16, int64_t n, 
   int64_t blocks = (n + kOptThreads - 1) / kOptThreads;
   const int64_t cap = (int64_t)kNumSM * 16;
   count_launch(1);
-  muon_apply_kernel<<<(int)(blocks < cap ? blocks : cap), kOptThreads, 0, stream>>>(
+  launch_pdl(muon_apply_kernel, (int)(blocks < cap ? blocks : cap), kOptThreads, 0, stream, 
       master, (const __nv_bfloat16*)update, (__nv_bfloat16*)w16, n, hyper, lr_ratio, weight_decay, adjust);
 }
 
@@ -189,6 +195,7 @@ struct HyperVals {
   float v[16];
 };
 __global__ void set_hyper_kernel(float* __restrict__ hyper, const HyperVals vals) {
+  pdl_begin();
   if (threadIdx.x < 16) hyper[threadIdx.x] = vals.v[threadIdx.x];
 }
 
@@ -196,7 +203,7 @@ void launch_set_hyper(float* hyper, const float* host_vals16, cudaStream_t strea
   HyperVals vals;
   for (int i = 0; i < 16; ++i) vals.v[i] = host_vals16[i];
   count_launch(1);
-  set_hyper_kernel<<<1, 32, 0, stream>>>(hyper, vals);
+  launch_pdl(set_hyper_kernel, 1, 32, 0, stream, hyper, vals);
 }
 
 int sumsq_num_partials() { return 4 * kNumSM; }
@@ -206,11 +213,11 @@ void launch_sumsq(const void* g, int is_bf16, int64_t n, float* partial, float* 
   const int P = sumsq_num_partials();
   count_launch(2);
   if (is_bf16)
-    sumsq_partial_kernel<__nv_bfloat16><<<P, kOptThreads, 0, stream>>>((const __nv_bfloat16*)g, n,
+    launch_pdl(sumsq_partial_kernel<__nv_bfloat16>, P, kOptThreads, 0, stream, (const __nv_bfloat16*)g, n,
                                                                         partial);
   else
-    sumsq_partial_kernel<float><<<P, kOptThreads, 0, stream>>>((const float*)g, n, partial);
-  sumsq_final_kernel<<<1, 256, 0, stream>>>(partial, P, out, accumulate);
+    launch_pdl(sumsq_partial_kernel<float>, P, kOptThreads, 0, stream, (const float*)g, n, partial);
+  launch_pdl(sumsq_final_kernel, 1, 256, 0, stream, partial, P, out, accumulate);
 }
 
 void launch_adamw(float* master, float* m, float* v, const void* grad, int grad_is_bf16, void* w16,
@@ -221,10 +228,10 @@ void launch_adamw(float* master, float* m, float* v, const void* grad, int grad_
   const int grid = (int)(blocks < cap ? blocks : cap);
   count_launch(1);
   if (grad_is_bf16)
-    adamw_kernel<__nv_bfloat16><<<grid, kOptThreads, 0, stream>>>(
+    launch_pdl(adamw_kernel<__nv_bfloat16>, grid, kOptThreads, 0, stream, 
         master, m, v, (const __nv_bfloat16*)grad, (__nv_bfloat16*)w16, n, hyper, norm_sq);
   else
-    adamw_kernel<float><<<grid, kOptThreads, 0, stream>>>(master, m, v, (const float*)grad,
+    launch_pdl(adamw_kernel<float>, grid, kOptThreads, 0, stream, master, m, v, (const float*)grad,
                                                           (__nv_bfloat16*)w16, n, hyper, norm_sq);
 }
 

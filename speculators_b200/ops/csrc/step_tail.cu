@@ -21,6 +21,7 @@ __global__ void __launch_bounds__(kTailThreads)
 step_tail_kernel(const float* __restrict__ row_loss, const int* __restrict__ pred, const int* __restrict__ target,
                  const uint8_t* __restrict__ mask, uint8_t* __restrict__ prev, int rows, float decay, float eps,
                  float* __restrict__ out, float* __restrict__ weight) {
+  pdl_begin();
   __shared__ float scratch[33];
   float s_loss = 0.f, s_mask = 0.f, s_prev = 0.f, s_correct = 0.f;
   for (int r = threadIdx.x; r < rows; r += blockDim.x) {
@@ -60,7 +61,7 @@ step_tail_kernel(const float* __restrict__ row_loss, const int* __restrict__ pre
 void launch_step_tail(const float* row_loss, const int* pred, const int* target, const uint8_t* mask, uint8_t* prev, int rows,
                       float decay, float eps, float* out, float* weight, cudaStream_t stream) {
   count_launch(1);
-  step_tail_kernel<<<1, kTailThreads, 0, stream>>>(row_loss, pred, target, mask, prev, rows, decay, eps, out, weight);
+  launch_pdl(step_tail_kernel, 1, kTailThreads, 0, stream, row_loss, pred, target, mask, prev, rows, decay, eps, out, weight);
 }
 
 }  // namespace sb200
