@@ -77,37 +77,82 @@ __global__ void sumsq_final_kernel(const float* __restrict__ partial, int P, flo
   if (threadIdx.x == 0) out[0] = accumulate ? out[0] + acc : acc;
 }
 
+// Eight consecutive fp32 / gradient values with 16-byte accesses.  The optimizer's buffers are read and written once
+// per step and are gigabytes: evict-first, so that they do not displace the weights in L2.
+struct f32x8 {
+  float v[8];
+};
+__device__ __forceinline__ f32x8 ld8s(const float* p) {
+  const float4 a = __ldcs(reinterpret_cast<const float4*>(p)), b = __ldcs(reinterpret_cast<const float4*>(p) + 1);
+  return f32x8{{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}};
+}
+__device__ __forceinline__ f32x8 ld8s(const __nv_bfloat16* p) {
+  const uint4 q = __ldcs(reinterpret_cast<const uint4*>(p));
+  f32x8 r;
+  unpack8(*reinterpret_cast<const bf16x8*>(&q), r.v);
+  return r;
+}
+__device__ __forceinline__ void st8s(float* p, const f32x8& x) {
+  __stcs(reinterpret_cast<float4*>(p), make_float4(x.v[0], x.v[1], x.v[2], x.v[3]));
+  __stcs(reinterpret_cast<float4*>(p) + 1, make_float4(x.v[4], x.v[5], x.v[6], x.v[7]));
+}
+
+struct AdamScalars {
+  float keep, b1, b2, gscale, step_size, inv_sqrt_bc2, eps;
+};
+__device__ __forceinline__ void adam_update(const AdamScalars& s, float g, float& p, float& m, float& v) {
+  g *= s.gscale;
+  p *= s.keep;
+  m = s.b1 * m + (1.f - s.b1) * g;
+  v = s.b2 * v + (1.f - s.b2) * g * g;
+  const float denom = sqrtf(v) * s.inv_sqrt_bc2 + s.eps;
+  p -= s.step_size * (m / denom);
+}
+
 // norm_sq: device scalar holding the (already all-reduced) sum of squares of the
 // *unscaled* gradients; clip coefficient = min(1, max_norm / (grad_scale*sqrt(norm_sq) + 1e-6)).
-template <typename G>
+//
+// Bound by memory: 28 bytes per parameter (bf16 gradient, fp32 master and two moments read and written, bf16
+// weight).  A thread owns eight consecutive parameters and a block 2048, one block per chunk: seven independent
+// 16-byte loads are in flight per thread.  With one parameter per thread and loop step (2- and 4-byte accesses)
+// 1.14 G parameters took 5.58 ms, 5.7 TB/s; this form takes 5.17 ms, 6.2 TB/s (96 % of a plain copy).
+template <typename G, bool VEC>
 __global__ void __launch_bounds__(kOptThreads)
 adamw_kernel(float* __restrict__ master, float* __restrict__ m, float* __restrict__ v,
              const G* __restrict__ grad, __nv_bfloat16* __restrict__ w16, int64_t n,
              const float* __restrict__ hyper, const float* __restrict__ norm_sq) {
   pdl_begin();
-  const float lr = hyper[0], b1 = hyper[1], b2 = hyper[2], eps = hyper[3], wd = hyper[4];
-  const float bc1 = hyper[5], bc2 = hyper[6], max_norm = hyper[7];
-  float gscale = hyper[8];
-  if (max_norm > 0.f && norm_sq) {
-    const float total = gscale * sqrtf(norm_sq[0]);
-    const float coef = max_norm / (total + 1e-6f);
-    if (coef < 1.f) gscale *= coef;
+  AdamScalars s;
+  s.b1 = hyper[1];
+  s.b2 = hyper[2];
+  s.eps = hyper[3];
+  s.keep = 1.f - hyper[0] * hyper[4];
+  s.gscale = hyper[8];
+  if (hyper[7] > 0.f && norm_sq) {
+    const float total = s.gscale * sqrtf(norm_sq[0]);
+    const float coef = hyper[7] / (total + 1e-6f);
+    if (coef < 1.f) s.gscale *= coef;
   }
-  const float step_size = lr / bc1;
-  const float inv_sqrt_bc2 = rsqrtf(bc2);
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const float g = to_f<G>(grad[i]) * gscale;
-    float p = master[i];
-    float mi = m[i], vi = v[i];
-    p *= (1.f - lr * wd);
-    mi = b1 * mi + (1.f - b1) * g;
-    vi = b2 * vi + (1.f - b2) * g * g;
-    const float denom = sqrtf(vi) * inv_sqrt_bc2 + eps;
-    p -= step_size * (mi / denom);
+  s.step_size = hyper[0] / hyper[5];
+  s.inv_sqrt_bc2 = rsqrtf(hyper[6]);
+  const int64_t i0 = ((int64_t)blockIdx.x * kOptThreads + threadIdx.x) * 8;
+  if (VEC && i0 + 8 <= n) {
+    const f32x8 g = ld8s(grad + i0);
+    f32x8 p = ld8s(master + i0), a = ld8s(m + i0), b = ld8s(v + i0);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) adam_update(s, g.v[j], p.v[j], a.v[j], b.v[j]);
+    st8s(master + i0, p);
+    st8s(m + i0, a);
+    st8s(v + i0, b);
+    if (w16) st8(w16 + i0, pack8(p.v));
+    return;
+  }
+  for (int64_t i = i0; i < n && i < i0 + 8; ++i) {
+    float p = master[i], a = m[i], b = v[i];
+    adam_update(s, to_f<G>(grad[i]), p, a, b);
     master[i] = p;
-    m[i] = mi;
-    v[i] = vi;
+    m[i] = a;
+    v[i] = b;
     if (w16) w16[i] = __float2bfloat16(p);
   }
 }
@@ -220,19 +265,22 @@ void launch_sumsq(const void* g, int is_bf16, int64_t n, float* partial, float* 
   launch_pdl(sumsq_final_kernel, 1, 256, 0, stream, partial, P, out, accumulate);
 }
 
+template <typename G>
+static void launch_adamw_as(float* master, float* m, float* v, const G* grad, __nv_bfloat16* w16, int64_t n, const float* hyper,
+                            const float* norm_sq, cudaStream_t stream) {
+  const uintptr_t bits = reinterpret_cast<uintptr_t>(master) | reinterpret_cast<uintptr_t>(m) | reinterpret_cast<uintptr_t>(v) |
+                         reinterpret_cast<uintptr_t>(grad) | reinterpret_cast<uintptr_t>(w16);
+  const int64_t grid = (n + 8 * kOptThreads - 1) / (8 * kOptThreads);
+  if ((bits & 15) == 0) launch_pdl(adamw_kernel<G, true>, (unsigned)grid, kOptThreads, 0, stream, master, m, v, grad, w16, n, hyper, norm_sq);
+  else launch_pdl(adamw_kernel<G, false>, (unsigned)grid, kOptThreads, 0, stream, master, m, v, grad, w16, n, hyper, norm_sq);
+}
+
 void launch_adamw(float* master, float* m, float* v, const void* grad, int grad_is_bf16, void* w16,
                   int64_t n, const float* hyper, const float* norm_sq, cudaStream_t stream) {
   if (n <= 0) return;
-  int64_t blocks = (n + kOptThreads - 1) / kOptThreads;
-  const int64_t cap = (int64_t)kNumSM * 16;
-  const int grid = (int)(blocks < cap ? blocks : cap);
   count_launch(1);
-  if (grad_is_bf16)
-    launch_pdl(adamw_kernel<__nv_bfloat16>, grid, kOptThreads, 0, stream, 
-        master, m, v, (const __nv_bfloat16*)grad, (__nv_bfloat16*)w16, n, hyper, norm_sq);
-  else
-    launch_pdl(adamw_kernel<float>, grid, kOptThreads, 0, stream, master, m, v, (const float*)grad,
-                                                          (__nv_bfloat16*)w16, n, hyper, norm_sq);
+  if (grad_is_bf16) launch_adamw_as(master, m, v, (const __nv_bfloat16*)grad, (__nv_bfloat16*)w16, n, hyper, norm_sq, stream);
+  else launch_adamw_as(master, m, v, (const float*)grad, (__nv_bfloat16*)w16, n, hyper, norm_sq, stream);
 }
 
 }  // namespace sb200
