@@ -66,7 +66,7 @@ def _use_native(t: torch.Tensor) -> bool:
 _GEMM_STATUS: dict[int, torch.Tensor] = {}
 
 
-def _own_gemm_enabled() -> bool:
+def own_gemm_enabled() -> bool:
     import os
 
     return os.environ.get("SB200_LINEAR_GEMM", "tcgen05") != "cublas"
@@ -108,7 +108,7 @@ def _forward_gemm(x2: torch.Tensor, w: torch.Tensor, residual: torch.Tensor | No
     """``x2 @ w.T (+ residual)`` for 2-D operands.  bf16 CUDA operands with 16-byte aligned
     rows run on the package's tcgen05 kernel (the residual is read in its epilogue, no
     copy of it is made); everything else goes to the library."""
-    if _gemm_operand_ok(x2) and _gemm_operand_ok(w) and _own_gemm_enabled() and (
+    if _gemm_operand_ok(x2) and _gemm_operand_ok(w) and own_gemm_enabled() and (
         residual is None or (_gemm_operand_ok(residual) and residual.shape == (x2.shape[0], w.shape[0]))
     ):
         out = torch.empty((x2.shape[0], w.shape[0]), dtype=x2.dtype, device=x2.device)
@@ -138,7 +138,7 @@ def _wgrad_gemm(dy2: torch.Tensor, x2: torch.Tensor, out: torch.Tensor | None, a
 
 def matmul_nt(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
     """``a @ b.T`` for 2-D tensors; bf16 CUDA operands with aligned rows use the tcgen05 kernel."""
-    if _gemm_operand_ok(a) and _gemm_operand_ok(b) and _own_gemm_enabled():
+    if _gemm_operand_ok(a) and _gemm_operand_ok(b) and own_gemm_enabled():
         return _forward_gemm(a, b, None)
     return a @ b.t()
 
@@ -146,7 +146,7 @@ def matmul_nt(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
 def matmul_nn(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, accumulate: bool = False) -> torch.Tensor:
     """``a @ b`` for 2-D tensors (``b`` read as stored, no transpose copy), optionally stored
     into / added to ``out``."""
-    if _gemm_operand_ok(a) and _gemm_operand_ok(b) and _own_gemm_enabled() and (out is None or _gemm_operand_ok(out)):
+    if _gemm_operand_ok(a) and _gemm_operand_ok(b) and own_gemm_enabled() and (out is None or _gemm_operand_ok(out)):
         return _dgrad_gemm(a, b, out, accumulate)
     if out is None:
         return a @ b
@@ -155,7 +155,7 @@ def matmul_nn(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None,
 
 def matmul_tn(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None, accumulate: bool = False) -> torch.Tensor:
     """``a.T @ b`` for 2-D tensors, optionally stored into / added to ``out``."""
-    if _gemm_operand_ok(a) and _gemm_operand_ok(b) and _own_gemm_enabled() and (out is None or _gemm_operand_ok(out)):
+    if _gemm_operand_ok(a) and _gemm_operand_ok(b) and own_gemm_enabled() and (out is None or _gemm_operand_ok(out)):
         return _wgrad_gemm(a, b, out, accumulate)
     if out is None:
         return a.t() @ b
@@ -227,7 +227,7 @@ class _GroupedLinearFn(torch.autograd.Function):
 
 def grouped_linear_ok(x: torch.Tensor, weight: torch.Tensor) -> bool:
     """Whether ``grouped_linear`` can run on the tcgen05 kernel for these operands."""
-    return (_own_gemm_enabled() and _gemm_operand_ok(x) and weight.is_cuda and weight.dtype == torch.bfloat16 and weight.dim() == 3
+    return (own_gemm_enabled() and _gemm_operand_ok(x) and weight.is_cuda and weight.dtype == torch.bfloat16 and weight.dim() == 3
             and weight.is_contiguous() and weight.shape[1] % 256 == 0 and weight.shape[2] % 256 == 0 and x.shape[0] % 128 == 0)
 
 
@@ -275,7 +275,7 @@ def _linear_backward(x2, weight, rows, dy, need_dx: bool, need_dw: bool):
     w = weight if r0 is None else weight[r0:r1]
     dy2 = dy if (dy.stride(-1) == 1 and dy.stride(0) % 8 == 0 and dy.data_ptr() % 16 == 0) else dy.contiguous()
     dx = dw = None
-    own = _own_gemm_enabled() and _gemm_operand_ok(dy2) and _gemm_operand_ok(w) and _gemm_operand_ok(x2)
+    own = own_gemm_enabled() and _gemm_operand_ok(dy2) and _gemm_operand_ok(w) and _gemm_operand_ok(x2)
     if need_dx:
         dx = _dgrad_gemm(dy2, w) if own else dy2 @ w
     if need_dw:
@@ -327,7 +327,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
         return y
     w = weight if rows is None else weight[rows[0] : rows[1]]
     b = bias if (bias is None or rows is None) else bias[rows[0] : rows[1]]
-    if x.is_cuda and x.dtype == torch.bfloat16 and b is None and not torch.is_grad_enabled() and _own_gemm_enabled():
+    if x.is_cuda and x.dtype == torch.bfloat16 and b is None and not torch.is_grad_enabled() and own_gemm_enabled():
         x2 = x.reshape(-1, x.shape[-1])
         res2 = residual.reshape(-1, residual.shape[-1]) if residual is not None else None
         return _forward_gemm(x2, w, res2).view(*x.shape[:-1], w.shape[0])
@@ -487,7 +487,7 @@ def linear_swiglu(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor | None:
     import os
 
     x2 = x.reshape(-1, x.shape[-1])
-    if (not _own_gemm_enabled() or os.environ.get("SB200_FUSED_SWIGLU", "1") == "0" or not _gemm_operand_ok(x2) or not _gemm_operand_ok(weight)
+    if (not own_gemm_enabled() or os.environ.get("SB200_FUSED_SWIGLU", "1") == "0" or not _gemm_operand_ok(x2) or not _gemm_operand_ok(weight)
             or weight.shape[0] % 256 or weight.shape[1] != x2.shape[1]):
         return None
     h = _GateUpSwiGLUFn.apply(x2, weight)
@@ -662,7 +662,7 @@ def lm_head_loss_raw(op: str, hidden: torch.Tensor, weight: torch.Tensor, target
     plain store epilogue), so the two-kernel form is the default."""
     import os
 
-    if (op not in FUSED_HEAD_OPS or not _own_gemm_enabled() or os.environ.get("SB200_FUSED_HEAD", "0") != "1"
+    if (op not in FUSED_HEAD_OPS or not own_gemm_enabled() or os.environ.get("SB200_FUSED_HEAD", "0") != "1"
             or not (_gemm_operand_ok(hidden) and _gemm_operand_ok(weight) and _gemm_operand_ok(targets))
             or weight.shape[0] % 8 or hidden.shape[0] <= 128):
         return None

@@ -34,6 +34,7 @@ int launch_gemm_tn_tcgen05(const void*, const void*, void*, const void*, int, in
                            int*, int, cudaStream_t);
 int launch_gemm_tcgen05(const void*, const void*, void*, const void*, int, int, int, int64_t, int64_t, int64_t, int64_t, int, int, int,
                         int*, int, cudaStream_t);
+int launch_gemm_stack(const void*, const void*, void*, const void*, int, int, int, int, int, int, float, float, int, int*, cudaStream_t);
 void launch_moe_group_plan(const int*, int, int*, int*, cudaStream_t);
 int launch_gemm_grouped(const void*, const void*, void*, int, int, int, int64_t, int64_t, int64_t, int, int, int, const int*, const int*, int, int*,
                         cudaStream_t);
@@ -64,8 +65,10 @@ void launch_sumsq(const void*, int, int64_t, float*, float*, int, cudaStream_t);
 void launch_set_hyper(float*, const float*, cudaStream_t);
 void launch_adamw(float*, float*, float*, const void*, int, void*, int64_t, const float*,
                   const float*, cudaStream_t);
-void launch_muon_momentum(const void*, int, float*, void*, int64_t, const float*, const float*, float, int, float*, float*, cudaStream_t);
-void launch_muon_apply(float*, const void*, void*, int64_t, const float*, float, float, float, cudaStream_t);
+void launch_muon_momentum(const void*, int, float*, void*, const int64_t*, const int*, int, const int*, int, const float*, const float*, float, int, float*,
+                          float*, cudaStream_t);
+void launch_muon_apply(float*, const void*, void*, const int64_t*, const int*, int, const float*, const float*, float, float, cudaStream_t);
+int muon_chunk_elements();
 }  // namespace sb200
 
 namespace {
@@ -333,43 +336,50 @@ void sumsq(const Tensor& g, Tensor out, bool accumulate) {
                       partial.data_ptr<float>(), out.data_ptr<float>(), accumulate, cur_stream());
 }
 
-// Muon, first half: buf <- momentum update of the clipped gradient, out <- bf16 (nesterov) update,
-// out_sumsq[0] <- squared Frobenius norm of out.  partial: fp32[sumsq_num_partials()] scratch.
-void muon_momentum(const Tensor& grad, Tensor buf, Tensor out, const Tensor& hyper, const Tensor& norm_sq, double momentum, bool nesterov,
-                   Tensor partial, Tensor out_sumsq) {
-  const int64_t n = buf.numel();
-  TORCH_CHECK(grad.is_cuda() && grad.is_contiguous() && grad.numel() == n &&
-              (grad.scalar_type() == at::kBFloat16 || grad.scalar_type() == at::kFloat));
+// Muon, both element-wise halves, for every matrix of a table in one launch.
+//   table int64[M, 3]: offset in the flat gradient / weight buffers, elements, offset in the state buffers (offsets multiples of 8)
+//   chunks int32[C, 2]: matrix and chunk of muon_chunk_elements() elements inside it; first_chunk int32[M + 1]
+void check_muon_table(const Tensor& table, const Tensor& chunks) {
+  TORCH_CHECK(table.is_cuda() && table.scalar_type() == at::kLong && table.dim() == 2 && table.size(1) == 3 && table.is_contiguous());
+  TORCH_CHECK(chunks.is_cuda() && chunks.scalar_type() == at::kInt && chunks.dim() == 2 && chunks.size(1) == 2 && chunks.is_contiguous());
+}
+bool aligned16(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; }
+
+// buf <- momentum update of the clipped gradient, out <- bf16 (nesterov) update over its Frobenius norm (inv_norm[M] <- its inverse).
+void muon_momentum(const Tensor& grad, Tensor buf, Tensor out, const Tensor& table, const Tensor& chunks, const Tensor& first_chunk, const Tensor& hyper,
+                   const Tensor& norm_sq, double momentum, bool nesterov, Tensor inv_norm) {
+  check_muon_table(table, chunks);
+  TORCH_CHECK(grad.is_cuda() && grad.is_contiguous() && (grad.scalar_type() == at::kBFloat16 || grad.scalar_type() == at::kFloat));
   TORCH_CHECK(buf.is_cuda() && buf.scalar_type() == at::kFloat && buf.is_contiguous());
-  TORCH_CHECK(out.is_cuda() && out.scalar_type() == at::kBFloat16 && out.is_contiguous() && out.numel() == n);
+  TORCH_CHECK(out.is_cuda() && out.scalar_type() == at::kBFloat16 && out.is_contiguous() && out.numel() == buf.numel());
+  TORCH_CHECK(aligned16(grad) && aligned16(buf) && aligned16(out), "muon_momentum: buffers must be 16-byte aligned");
+  TORCH_CHECK(first_chunk.is_cuda() && first_chunk.scalar_type() == at::kInt && first_chunk.numel() == table.size(0) + 1);
   TORCH_CHECK(hyper.is_cuda() && hyper.scalar_type() == at::kFloat && hyper.numel() >= 9);
   TORCH_CHECK(norm_sq.is_cuda() && norm_sq.scalar_type() == at::kFloat && norm_sq.numel() >= 1);
-  TORCH_CHECK(partial.is_cuda() && partial.scalar_type() == at::kFloat && partial.numel() >= sb200::sumsq_num_partials());
-  TORCH_CHECK(out_sumsq.is_cuda() && out_sumsq.scalar_type() == at::kFloat && out_sumsq.numel() >= 1);
+  TORCH_CHECK(inv_norm.is_cuda() && inv_norm.scalar_type() == at::kFloat && inv_norm.numel() >= table.size(0));
   c10::cuda::CUDAGuard guard(buf.device());
-  sb200::launch_muon_momentum(grad.data_ptr(), grad.scalar_type() == at::kBFloat16, buf.data_ptr<float>(), out.data_ptr(), n,
-                              hyper.data_ptr<float>(), norm_sq.data_ptr<float>(), (float)momentum, nesterov ? 1 : 0,
-                              partial.data_ptr<float>(), out_sumsq.data_ptr<float>(), cur_stream());
+  Tensor partial = at::empty({chunks.size(0)}, inv_norm.options());
+  sb200::launch_muon_momentum(grad.data_ptr(), grad.scalar_type() == at::kBFloat16, buf.data_ptr<float>(), out.data_ptr(), table.data_ptr<int64_t>(),
+                              chunks.data_ptr<int>(), (int)chunks.size(0), first_chunk.data_ptr<int>(), (int)table.size(0), hyper.data_ptr<float>(),
+                              norm_sq.data_ptr<float>(), (float)momentum, nesterov ? 1 : 0, partial.data_ptr<float>(), inv_norm.data_ptr<float>(), cur_stream());
 }
 
-// Muon, second half: master <- master * (1 - lr * wd) - lr * adjust * update, w16 <- bf16(master); lr = hyper[0] * lr_ratio.
-void muon_apply(Tensor master, const Tensor& update, c10::optional<Tensor> w16, const Tensor& hyper, double lr_ratio, double weight_decay,
-                double adjust) {
-  const int64_t n = master.numel();
+// master <- master * (1 - lr * wd) - lr * adjust[matrix] * update, w16 <- bf16(master); lr = hyper[0] * lr_ratio.
+void muon_apply(Tensor master, const Tensor& update, Tensor w16, const Tensor& table, const Tensor& chunks, const Tensor& adjust, const Tensor& hyper,
+                double lr_ratio, double weight_decay) {
+  check_muon_table(table, chunks);
   TORCH_CHECK(master.is_cuda() && master.scalar_type() == at::kFloat && master.is_contiguous());
-  TORCH_CHECK(update.is_cuda() && update.scalar_type() == at::kBFloat16 && update.is_contiguous() && update.numel() == n);
+  TORCH_CHECK(update.is_cuda() && update.scalar_type() == at::kBFloat16 && update.is_contiguous() && update.numel() == master.numel());
+  TORCH_CHECK(w16.is_cuda() && w16.scalar_type() == at::kBFloat16 && w16.is_contiguous());
+  TORCH_CHECK(aligned16(master) && aligned16(update) && aligned16(w16), "muon_apply: buffers must be 16-byte aligned");
+  TORCH_CHECK(adjust.is_cuda() && adjust.scalar_type() == at::kFloat && adjust.is_contiguous() && adjust.numel() == table.size(0));
   TORCH_CHECK(hyper.is_cuda() && hyper.scalar_type() == at::kFloat && hyper.numel() >= 9);
-  void* w = nullptr;
-  if (w16.has_value()) {
-    TORCH_CHECK(w16->is_cuda() && w16->scalar_type() == at::kBFloat16 && w16->numel() == n && w16->is_contiguous());
-    w = w16->data_ptr();
-  }
   c10::cuda::CUDAGuard guard(master.device());
-  sb200::launch_muon_apply(master.data_ptr<float>(), update.data_ptr(), w, n, hyper.data_ptr<float>(), (float)lr_ratio,
-                           (float)weight_decay, (float)adjust, cur_stream());
+  sb200::launch_muon_apply(master.data_ptr<float>(), update.data_ptr(), w16.data_ptr(), table.data_ptr<int64_t>(), chunks.data_ptr<int>(), (int)chunks.size(0),
+                           adjust.data_ptr<float>(), hyper.data_ptr<float>(), (float)lr_ratio, (float)weight_decay, cur_stream());
 }
 
-int64_t sumsq_num_partials_binding() { return sb200::sumsq_num_partials(); }
+int64_t muon_chunk_elements_binding() { return sb200::muon_chunk_elements(); }
 
 // hyper (fp32[16], CUDA) <- vals (<= 16 host doubles), passed as kernel arguments.
 void set_hyper(Tensor hyper, std::vector<double> vals) {
@@ -726,6 +736,24 @@ void gemm(const Tensor& a, const Tensor& b, Tensor out, int64_t epilogue, bool a
   gemm_variant(a, b, out, epilogue, a_mn, b_mn, status, 0);
 }
 
+// Stacks of products: out[z] = alpha op(a[z]) @ op(b[z])^T (+ beta addend[z]), rounded as separate bf16 passes would round.
+// Operands as in gemm, each a dense [batch, ., .] stack; symmetric: the caller knows that the products are.
+void gemm_stack(const Tensor& a, const Tensor& b, Tensor out, const c10::optional<Tensor>& addend, bool a_mn, bool b_mn, double alpha, double beta,
+                bool symmetric, Tensor status) {
+  for (const Tensor* t : std::initializer_list<const Tensor*>{&a, &b, &out})
+    TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kBFloat16 && t->dim() == 3 && t->is_contiguous(), "gemm_stack: contiguous bf16 [batch, rows, cols] expected");
+  const int64_t B = a.size(0), M = a_mn ? a.size(2) : a.size(1), K = a_mn ? a.size(1) : a.size(2), N = b_mn ? b.size(2) : b.size(1);
+  TORCH_CHECK(b.size(0) == B && out.size(0) == B && (b_mn ? b.size(1) : b.size(2)) == K && out.size(1) == M && out.size(2) == N, "gemm_stack: shape mismatch");
+  TORCH_CHECK(!symmetric || M == N, "gemm_stack: a symmetric product is square");
+  if (addend.has_value())
+    TORCH_CHECK(addend->is_cuda() && addend->scalar_type() == at::kBFloat16 && addend->is_contiguous() && addend->sizes() == out.sizes(), "gemm_stack: addend");
+  TORCH_CHECK(status.is_cuda() && status.scalar_type() == at::kInt && status.numel() >= 1);
+  c10::cuda::CUDAGuard guard(a.device());
+  const int rc = sb200::launch_gemm_stack(a.data_ptr(), b.data_ptr(), out.data_ptr(), addend.has_value() ? addend->data_ptr() : nullptr, (int)B, (int)M, (int)N,
+                                          (int)K, a_mn ? 1 : 0, b_mn ? 1 : 0, (float)alpha, (float)beta, symmetric ? 1 : 0, status.data_ptr<int>(), cur_stream());
+  TORCH_CHECK(rc == 0, "gemm_stack launch failed (", rc, ")");
+}
+
 // ---- masked attention ------------------------------------------------------------------
 void check_heads(const Tensor& t, const char* name, int64_t hd) {
   TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.dim() == 3, name, ": bf16 CUDA [T, heads, hd] expected");
@@ -899,7 +927,7 @@ TORCH_LIBRARY(sb200, m) {
   m.def("adamw", &adamw);
   m.def("muon_momentum", &muon_momentum);
   m.def("muon_apply", &muon_apply);
-  m.def("sumsq_num_partials", &sumsq_num_partials_binding);
+  m.def("muon_chunk_elements", &muon_chunk_elements_binding);
   m.def("set_hyper", &set_hyper);
   m.def("launch_count", &launch_count);
   m.def("peer_alloc", &peer_alloc);
@@ -927,6 +955,7 @@ TORCH_LIBRARY(sb200, m) {
   m.def("gemm_tn", &gemm_tn);
   m.def("gemm", &gemm);
   m.def("gemm_variant", &gemm_variant);
+  m.def("gemm_stack", &gemm_stack);
   m.def("lmhead_loss_fwd", &lmhead_loss_fwd);
   m.def("moe_group_plan", &moe_group_plan);
   m.def("gemm_grouped_rows", &gemm_grouped_rows);

@@ -117,15 +117,45 @@ struct Params {
   __nv_bfloat16* h;  // kSwiGLU: [M, N / 2] output, row stride ldh
   int64_t ldh;
   int staged;        // 1: C (and h) leave through shared memory and TMA stores (map_c, map_h)
+  // result = alpha * product (+ beta * addend), rounded where separate element-wise passes over bf16 tensors would round:
+  // alpha * bf16(product) and beta * addend each to bf16 before the sum; alpha = beta = 1 is the plain epilogue
+  float alpha, beta;
+  // a stack of `batch` products: the z-th of each operand's stack, elements apart
+  int batch;
+  int64_t c_batch, r_batch;
+  int symmetric;  // the product is symmetric: tiles above the diagonal are computed and stored twice (map_h: transposed stores)
+};
+
+__device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16(x)); }
+struct Scaling {
+  float alpha, beta;
+  // (the plain epilogue skips the arithmetic as a whole: the conditions are uniform)
+  template <int N>
+  __device__ __forceinline__ void product(float (&f)[N]) const {
+    if (alpha != 1.f) {
+#pragma unroll
+      for (int j = 0; j < N; ++j) f[j] = bf16_round(alpha * bf16_round(f[j]));
+    }
+  }
+  template <int N>
+  __device__ __forceinline__ void add(float (&f)[N], const float (&o)[N]) const {
+    if (beta != 1.f) {
+#pragma unroll
+      for (int j = 0; j < N; ++j) f[j] += bf16_round(beta * o[j]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < N; ++j) f[j] += o[j];
+    }
+  }
 };
 
 // First element of the W-column chunk at (row, n0) of the output.
-__device__ __forceinline__ __nv_bfloat16* c_chunk(const Params& p, int row, int n0) {
+__device__ __forceinline__ __nv_bfloat16* c_chunk(const Params& p, int row, int n0, int z) {
   if (p.sc.world > 0) {
     const int owner = n0 / p.sc.cols;
     return p.sc.stage[owner] + ((int64_t)p.sc.rank * p.M + row) * p.sc.cols + (n0 - owner * p.sc.cols);
   }
-  return p.c + (int64_t)row * p.ldc + n0;
+  return p.c + z * p.c_batch + (int64_t)row * p.ldc + n0;
 }
 
 // Where one 256x256 tile (or this CTA's half of it) sits in the operands.
@@ -137,6 +167,8 @@ struct TileInfo {
   int row_end;     // C rows >= row_end do not exist (for this tile)
   int n0;          // first C column
   int tile_n;      // column-tile index (row statistics)
+  int z;           // which product of the stack
+  bool mirror;     // symmetric product: the tile's transpose is stored too
 };
 
 constexpr int kBandRows = 8;
@@ -144,7 +176,23 @@ constexpr int kBandRows = 8;
 template <bool B_MN>
 __device__ __forceinline__ TileInfo decode_tile(const Params& p, int tile, int tiles_m, int tiles_n, int num_kb, int rank) {
   TileInfo t;
-  if (p.grp.mode == kGroupNone) {
+  t.z = 0;
+  t.mirror = false;
+  if (p.grp.mode == kGroupNone && p.symmetric) {
+    const int per = tiles_m * (tiles_m + 1) / 2;
+    t.z = tile / per;
+    const int local = tile - t.z * per;
+    int j = (int)((sqrtf(8.f * local + 1.f) - 1.f) * 0.5f);  // local = j (j + 1) / 2 + i, i <= j
+    while (j * (j + 1) / 2 > local) --j;
+    while ((j + 1) * (j + 2) / 2 <= local) ++j;
+    const int i = local - j * (j + 1) / 2, m0 = i * 256 + rank * 128;
+    t.mirror = i != j;
+    t.tile_n = j;
+    t.n0 = j * 256;
+    t.a_m = m0; t.a_k0 = 0; t.b_n = t.n0 + rank * 128; t.b_k0 = 0; t.num_kb = num_kb; t.c_row0 = m0; t.row_end = p.M;
+  } else if (p.grp.mode == kGroupNone) {
+    t.z = tile / (tiles_m * tiles_n);
+    tile -= t.z * tiles_m * tiles_n;
     // Tiles run down a band of kBandRows tile rows, column after column, then the next band: the
     // CTA pairs working at the same time cover a near-square patch of C (8 x 9 tiles on 74 pairs),
     // so a wave touches about 17 operand panels instead of 75 and a tall output (a weight
@@ -195,9 +243,9 @@ __device__ __forceinline__ void st32(__nv_bfloat16* ptr, const bf16x8& a, const 
 // Epilogue of one thread: TMEM lane `taddr` (its 256 fp32 columns) -> row `row`, columns
 // n0 .. n0+255 of C, with the configured epilogue.
 template <int W>
-__device__ __forceinline__ void store_accumulator(const Params& p, uint32_t taddr, int row, int n0, int row_end, bool zero) {
-  __nv_bfloat16* crow = c_chunk(p, row, n0);
-  const __nv_bfloat16* rrow = p.residual ? p.residual + (int64_t)row * p.ldr + n0 : nullptr;
+__device__ __forceinline__ void store_accumulator(const Params& p, const Scaling& sc, uint32_t taddr, int row, int n0, int z, int row_end, bool zero) {
+  __nv_bfloat16* crow = c_chunk(p, row, n0, z);
+  const __nv_bfloat16* rrow = p.residual ? p.residual + z * p.r_batch + (int64_t)row * p.ldr + n0 : nullptr;
   const bool vec_ok = ((p.ldc & 7) == 0) && ((reinterpret_cast<uintptr_t>(p.c) & 15) == 0) &&
                       (p.epilogue != kAddResidual || (((p.ldr & 7) == 0) && ((reinterpret_cast<uintptr_t>(p.residual) & 15) == 0)));
   const bool wide_ok = vec_ok && ((p.ldc & 15) == 0) && ((reinterpret_cast<uintptr_t>(p.c) & 31) == 0);
@@ -219,16 +267,15 @@ __device__ __forceinline__ void store_accumulator(const Params& p, uint32_t tadd
           float f[8];
 #pragma unroll
           for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(r[v * 8 + j]);
+          sc.product(f);
           if (p.epilogue == kAccumulate) {
             float o[8];
             unpack8(ld8(crow + c * 32 + v * 8), o);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) f[j] += o[j];
+            sc.add(f, o);
           } else if (p.epilogue == kAddResidual) {
             float o[8];
             unpack8(ld8(rrow + c * 32 + v * 8), o);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) f[j] += o[j];
+            sc.add(f, o);
           }
           packed[v] = pack8(f);
         }
@@ -242,10 +289,13 @@ __device__ __forceinline__ void store_accumulator(const Params& p, uint32_t tadd
       } else {
         for (int j = 0; j < 32; ++j) {
           if (col0 + j < p.N) {
-            float f = __uint_as_float(r[j]);
-            if (p.epilogue == kAccumulate) f += __bfloat162float(crow[c * 32 + j]);
-            else if (p.epilogue == kAddResidual) f += __bfloat162float(rrow[c * 32 + j]);
-            crow[c * 32 + j] = __float2bfloat16(f);
+            float f[1] = {__uint_as_float(r[j])};
+            sc.product(f);
+            if (p.epilogue != kStore) {
+              const float o[1] = {__bfloat162float((p.epilogue == kAccumulate ? crow : rrow)[c * 32 + j])};
+              sc.add(f, o);
+            }
+            crow[c * 32 + j] = __float2bfloat16(f[0]);
           }
         }
       }
@@ -261,41 +311,53 @@ __device__ __forceinline__ void store_accumulator(const Params& p, uint32_t tadd
 __device__ __forceinline__ void store_accumulator_swiglu(const Params& p, const CUtensorMap* map_c, const CUtensorMap* map_h, uint32_t stage, uint32_t tlane,
                                                          int row0, int col0, bool live, int lane) {
   const int I = p.N >> 1;
-  bf16x8 up[8], hp[8];
   stage_wait();
 #pragma unroll
   for (int c = 0; c < 2; ++c) {
-    uint32_t g[32], u[32];
+    uint32_t g[32];
     tmem_ld32(tlane + c * 32, g);
+    tmem_ld_wait();
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      float f[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(g[v * 8 + j]);
+      stage_put8(stage, lane, c * 4 + v, pack8(f));
+    }
+  }
+  stage_store(stage, map_c, col0, row0, 0, live);
+  uint4 row[8];  // the lane's gate values, then its activated ones
+#pragma unroll
+  for (int v = 0; v < 8; ++v) row[v] = stage_get8(stage, lane, v);
+  stage_wait();
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    uint32_t u[32];
     tmem_ld32(tlane + 128 + c * 32, u);
     tmem_ld_wait();
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
       float gf[8], uf[8], o[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) { gf[j] = __uint_as_float(g[v * 8 + j]); uf[j] = __uint_as_float(u[v * 8 + j]); }
-      const bf16x8 gp = pack8(gf);
-      up[c * 4 + v] = pack8(uf);
-      unpack8(gp, gf);
-      unpack8(up[c * 4 + v], uf);
+      for (int j = 0; j < 8; ++j) uf[j] = __uint_as_float(u[v * 8 + j]);
+      const bf16x8 up = pack8(uf);
+      stage_put8(stage, lane, c * 4 + v, up);
+      unpack8(up, uf);
+      unpack8(*reinterpret_cast<const bf16x8*>(&row[c * 4 + v]), gf);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const float sg = 1.f / (1.f + __expf(-gf[j]));
         o[j] = __bfloat162float(__float2bfloat16(gf[j] * sg)) * uf[j];
       }
-      hp[c * 4 + v] = pack8(o);
-      stage_put8(stage, lane, c * 4 + v, gp);
+      const bf16x8 act = pack8(o);
+      row[c * 4 + v] = *reinterpret_cast<const uint4*>(&act);
     }
   }
-  stage_store(stage, map_c, col0, row0, live);
+  stage_store(stage, map_c, I + col0, row0, 0, live);
   stage_wait();
 #pragma unroll
-  for (int v = 0; v < 8; ++v) stage_put8(stage, lane, v, up[v]);
-  stage_store(stage, map_c, I + col0, row0, live);
-  stage_wait();
-#pragma unroll
-  for (int v = 0; v < 8; ++v) stage_put8(stage, lane, v, hp[v]);
-  stage_store(stage, map_h, col0, row0, live);
+  for (int v = 0; v < 8; ++v) stage_put8(stage, lane, v, *reinterpret_cast<const bf16x8*>(&row[v]));
+  stage_store(stage, map_h, col0, row0, 0, live);
 }
 
 // ---- epilogues that read memory (C += result, result + residual) ---------------------------
@@ -319,22 +381,22 @@ __device__ __forceinline__ bool tile_reads_vectorised(const Params& p, int n0) {
 
 // Staged stores take every tile (N is a multiple of 8 then): a chunk past the edge reads as zeros.
 template <int W>
-__device__ __forceinline__ void prefetch_addend_staged(const Params& p, int row, int n0, int row_end, RowPrefetch<W>& pre) {
+__device__ __forceinline__ void prefetch_addend_staged(const Params& p, int row, int n0, int z, int row_end, RowPrefetch<W>& pre) {
   pre.tile_ok = true;
   pre.valid = row < row_end;
   if (p.epilogue == kStore) return;
-  const __nv_bfloat16* src = p.epilogue == kAccumulate ? p.c + (int64_t)row * p.ldc + n0 : p.residual + (int64_t)row * p.ldr + n0;
+  const __nv_bfloat16* src = p.epilogue == kAccumulate ? p.c + z * p.c_batch + (int64_t)row * p.ldc + n0 : p.residual + z * p.r_batch + (int64_t)row * p.ldr + n0;
 #pragma unroll
   for (int i = 0; i < W / 8; ++i)
     pre.v[i] = pre.valid && n0 + i * 8 < p.N ? __ldg(reinterpret_cast<const uint4*>(src) + i) : make_uint4(0u, 0u, 0u, 0u);
 }
 
 template <int W>
-__device__ __forceinline__ void prefetch_addend(const Params& p, int row, int n0, int row_end, RowPrefetch<W>& pre) {
+__device__ __forceinline__ void prefetch_addend(const Params& p, int row, int n0, int z, int row_end, RowPrefetch<W>& pre) {
   pre.tile_ok = tile_reads_vectorised<W>(p, n0);
   pre.valid = pre.tile_ok && row < row_end;
   if (pre.valid) {
-    const __nv_bfloat16* src = p.epilogue == kAccumulate ? p.c + (int64_t)row * p.ldc + n0 : p.residual + (int64_t)row * p.ldr + n0;
+    const __nv_bfloat16* src = p.epilogue == kAccumulate ? p.c + z * p.c_batch + (int64_t)row * p.ldc + n0 : p.residual + z * p.r_batch + (int64_t)row * p.ldr + n0;
 #pragma unroll
     for (int i = 0; i < W / 8; ++i) pre.v[i] = __ldg(reinterpret_cast<const uint4*>(src) + i);
   }
@@ -344,8 +406,9 @@ __device__ __forceinline__ void prefetch_addend(const Params& p, int row, int n0
 // by whole warps (pre.tile_ok); a thread whose row does not exist takes part in the tensor-memory
 // loads and stores nothing.
 template <int W>
-__device__ __forceinline__ void store_accumulator_prefetched(const Params& p, uint32_t taddr, int row, int n0, const RowPrefetch<W>& pre, bool zero) {
-  __nv_bfloat16* crow = p.c + (int64_t)row * p.ldc + n0;
+__device__ __forceinline__ void store_accumulator_prefetched(const Params& p, const Scaling& sc, uint32_t taddr, int row, int n0, int z, const RowPrefetch<W>& pre,
+                                                             bool zero) {
+  __nv_bfloat16* crow = p.c + z * p.c_batch + (int64_t)row * p.ldc + n0;
   const bool wide_ok = ((p.ldc & 15) == 0) && ((reinterpret_cast<uintptr_t>(p.c) & 31) == 0);
 #pragma unroll
   for (int c = 0; c < W / 32; ++c) {
@@ -358,7 +421,9 @@ __device__ __forceinline__ void store_accumulator_prefetched(const Params& p, ui
       float f[8], o[8];
       unpack8(*reinterpret_cast<const bf16x8*>(&pre.v[c * 4 + v]), o);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) f[j] = (zero ? 0.f : __uint_as_float(r[v * 8 + j])) + o[j];
+      for (int j = 0; j < 8; ++j) f[j] = zero ? 0.f : __uint_as_float(r[v * 8 + j]);
+      sc.product(f);
+      sc.add(f, o);
       packed[v] = pack8(f);
     }
     if (!pre.valid) continue;
@@ -373,14 +438,15 @@ __device__ __forceinline__ void store_accumulator_prefetched(const Params& p, ui
 }
 
 // Four finished fp32 values -> row `row`, columns col0 .. col0 + 3 of C with the configured epilogue.
-__device__ __forceinline__ void store_vec4(const Params& p, const float4& t, int row, int col0) {
-  __nv_bfloat16* out = p.c + (int64_t)row * p.ldc + col0;
-  const __nv_bfloat16* add = p.epilogue == kAccumulate ? out : p.residual + (int64_t)row * p.ldr + col0;
-  float f[4] = {t.x, t.y, t.z, t.w};
+__device__ __forceinline__ void store_vec4(const Params& p, const Scaling& sc, const float4& t, int row, int col0, int z) {
+  __nv_bfloat16* out = p.c + z * p.c_batch + (int64_t)row * p.ldc + col0;
+  const __nv_bfloat16* add = p.epilogue == kAccumulate ? out : p.residual + z * p.r_batch + (int64_t)row * p.ldr + col0;
+  float f[4] = {t.x, t.y, t.z, t.w}, o[4];
+  sc.product(f);
   const bool full = col0 + 4 <= p.N && (p.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(p.c) & 7) == 0;
   if (p.epilogue != kStore) {
-    for (int j = 0; j < 4; ++j)
-      if (col0 + j < p.N) f[j] += __bfloat162float(add[j]);
+    for (int j = 0; j < 4; ++j) o[j] = col0 + j < p.N ? __bfloat162float(add[j]) : 0.f;
+    sc.add(f, o);
   }
   if (full) {
     __nv_bfloat162 lo = __floats2bfloat162_rn(f[0], f[1]), hi = __floats2bfloat162_rn(f[2], f[3]);
@@ -394,8 +460,9 @@ __device__ __forceinline__ void store_vec4(const Params& p, const float4& t, int
 // One warp's 32 rows x W columns through its 4 KB staging area, 64 columns at a time.  `row0`: C row of lane 0;
 // `live`: the rows exist; the addend of a reading epilogue is in `pre` (pre.tile_ok) or read here.
 template <int W>
-__device__ __forceinline__ void store_accumulator_staged(const Params& p, const CUtensorMap* map_c, uint32_t stage, uint32_t taddr, int row0, int n0,
-                                                         const RowPrefetch<W>& pre, bool live, bool zero, int lane) {
+__device__ __forceinline__ void store_accumulator_staged(const Params& p, const Scaling& sc, const CUtensorMap* map_c, const CUtensorMap* map_t, uint32_t stage,
+                                                         uint32_t taddr, int row0, int n0, int z, const RowPrefetch<W>& pre, bool live, bool mirror,
+                                                         bool zero, int lane) {
 #pragma unroll
   for (int h = 0; h < W / 64; ++h) {
     stage_wait();
@@ -410,16 +477,32 @@ __device__ __forceinline__ void store_accumulator_staged(const Params& p, const 
         float f[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) f[j] = zero ? 0.f : __uint_as_float(r[v * 8 + j]);
+        sc.product(f);
         if (p.epilogue != kStore) {
           float o[8];
           unpack8(*reinterpret_cast<const bf16x8*>(&pre.v[c * 4 + v]), o);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) f[j] += o[j];
+          sc.add(f, o);
         }
         stage_put8(stage, lane, q * 4 + v, pack8(f));
       }
     }
-    stage_store(stage, map_c, n0 + h * 64, row0, live && n0 + h * 64 < p.N);
+    const bool inside = live && n0 + h * 64 < p.N;
+    stage_store(stage, map_c, n0 + h * 64, row0, z, inside);
+    if (mirror) {  // 64 rows (this half's columns) of 32 elements (the warp's rows); the lanes of a store are neighbours
+      stage_wait();
+      uint4 own[8];
+#pragma unroll
+      for (int v = 0; v < 8; ++v) own[v] = stage_get8(stage, lane, v);
+      __syncwarp();
+#pragma unroll
+      for (int v = 0; v < 8; ++v) {
+        const uint32_t w[4] = {own[v].x, own[v].y, own[v].z, own[v].w};
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          asm volatile("st.shared.b16 [%0], %1;" ::"r"(stage + (v * 8 + j) * 64 + lane * 2), "h"((uint16_t)(w[j >> 1] >> (16 * (j & 1)))) : "memory");
+      }
+      stage_store(stage, map_t, row0, n0 + h * 64, z, inside);
+    }
   }
 }
 
@@ -501,8 +584,9 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   __shared__ __align__(8) uint64_t bar_full[S_STAGES], bar_empty[S_STAGES], bar_acc_full;
   __shared__ uint32_t tmem_base_slot;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int splits = 1 << log_splits, split = blockIdx.x & (splits - 1), tile = blockIdx.x >> log_splits;
-  const int tiles_m = (p.M + BM - 1) / BM;
+  const int splits = 1 << log_splits, split = blockIdx.x & (splits - 1);
+  const int tiles_m = (p.M + BM - 1) / BM, tiles = tiles_m * ((p.N + S_TILE_N - 1) / S_TILE_N);
+  const int z = (int)(blockIdx.x >> log_splits) / tiles, tile = (int)(blockIdx.x >> log_splits) - z * tiles;
   const int m0 = (tile % tiles_m) * BM, n0 = (tile / tiles_m) * S_TILE_N;
   const int all_kb = (p.K + S_STEP_K - 1) / S_STEP_K;
   const int kb0 = (split * all_kb) >> log_splits, num_kb = (((split + 1) * all_kb) >> log_splits) - kb0;
@@ -527,6 +611,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   if (log_splits > 0) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // waited for before the first remote store
 
   bool ok = true;
+  const Scaling sc{p.alpha, p.beta};
   const int quarter = warp & 3, row = m0 + quarter * 32 + lane;
   if (warp == 0) {
     if (elect_one()) {
@@ -539,14 +624,14 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         // K-major: boxes of rows x 64 contraction columns; MN-major: boxes of 128 contraction rows x 64 MN-columns
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
-          if (A_MN) tma_load_2d(sa + u * (S_A_BYTES / 2), &map_a, full, m0 + u * 64, k0);
-          else tma_load_2d(sa + u * (S_A_BYTES / 2), &map_a, full, k0 + u * 64, m0);
+          if (A_MN) tma_load_3d(sa + u * (S_A_BYTES / 2), &map_a, full, m0 + u * 64, k0, z);
+          else tma_load_3d(sa + u * (S_A_BYTES / 2), &map_a, full, k0 + u * 64, m0, z);
         }
         if (B_MN) {
-          tma_load_2d(sb, &map_b, full, n0, k0);
+          tma_load_3d(sb, &map_b, full, n0, k0, z);
         } else {
-          tma_load_2d(sb, &map_b, full, k0, n0);
-          tma_load_2d(sb + S_B_BYTES / 2, &map_b, full, k0 + 64, n0);
+          tma_load_3d(sb, &map_b, full, k0, n0, z);
+          tma_load_3d(sb + S_B_BYTES / 2, &map_b, full, k0 + 64, n0, z);
         }
         if (++stage == S_STAGES) { stage = 0; phase ^= 1; }
       }
@@ -574,8 +659,8 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     }
   } else if (log_splits == 0) {
     RowPrefetch<S_TILE_N> pre;
-    if (p.staged) prefetch_addend_staged<S_TILE_N>(p, row, n0, p.M, pre);
-    else prefetch_addend<S_TILE_N>(p, row, n0, p.M, pre);
+    if (p.staged) prefetch_addend_staged<S_TILE_N>(p, row, n0, z, p.M, pre);
+    else prefetch_addend<S_TILE_N>(p, row, n0, z, p.M, pre);
     ok = mbar_wait(smem_addr(&bar_acc_full), 0, p.status, kTimeoutEpilogue);
     ok = __all_sync(0xffffffffu, ok);
     if (ok) {
@@ -583,12 +668,12 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16);
       if (p.staged) {
         const uint32_t stage = smem_addr(smem + S_STAGES * S_STAGE_BYTES) + quarter * 4096;
-        store_accumulator_staged<S_TILE_N>(p, &map_c, stage, taddr, m0 + quarter * 32, n0, pre, m0 + quarter * 32 < p.M, false, lane);
+        store_accumulator_staged<S_TILE_N>(p, sc, &map_c, &map_c, stage, taddr, m0 + quarter * 32, n0, z, pre, m0 + quarter * 32 < p.M, false, false, lane);
         stage_wait();
       } else if (pre.tile_ok) {
-        store_accumulator_prefetched<S_TILE_N>(p, taddr, row, n0, pre, false);
+        store_accumulator_prefetched<S_TILE_N>(p, sc, taddr, row, n0, z, pre, false);
       } else {
-        store_accumulator<S_TILE_N>(p, taddr, row, n0, p.M, false);
+        store_accumulator<S_TILE_N>(p, sc, taddr, row, n0, z, p.M, false);
       }
     }
   } else {
@@ -632,7 +717,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           const float4 o = got[((src << log_rows) + r0) * 16 + (c ^ (r0 & 15))];
           t.x += o.x; t.y += o.y; t.z += o.z; t.w += o.w;
         }
-        if (orow < p.M) store_vec4(p, t, orow, n0 + c * 4);
+        if (orow < p.M) store_vec4(p, sc, t, orow, n0 + c * 4, z);
       }
     }
   }
@@ -704,7 +789,7 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   pdl_begin();
   const int num_tiles = p.grp.mode == kGroupRows ? p.grp.tile_start[p.grp.num_groups] * tiles_n
                         : p.grp.mode == kGroupK  ? p.grp.num_groups * tiles_m * tiles_n
-                                                 : tiles_m * tiles_n;
+                                                 : p.batch * (p.symmetric ? tiles_m * (tiles_m + 1) / 2 : tiles_m * tiles_n);
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (both CTAs)
@@ -724,10 +809,10 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
           // 64 MN-columns (MN-elements 64u .. 64u+63 of this CTA's 128).  Either way 16 KB at the same place.
 #pragma unroll
           for (int u = 0; u < KSUB; ++u) {
-            if (A_MN) tma_load_2d_pair(sa + u * P_SUB_BYTES, &map_a, full_leader, ti.a_m + u * 64, ti.a_k0 + kb * STAGE_K);
-            else tma_load_2d_pair(sa + u * P_SUB_BYTES, &map_a, full_leader, ti.a_k0 + kb * STAGE_K + u * BK, ti.a_m);
-            if (B_MN) tma_load_2d_pair(sa + u * P_SUB_BYTES + P_A_BYTES, &map_b, full_leader, ti.b_n + u * 64, ti.b_k0 + kb * STAGE_K);
-            else tma_load_2d_pair(sa + u * P_SUB_BYTES + P_A_BYTES, &map_b, full_leader, ti.b_k0 + kb * STAGE_K + u * BK, ti.b_n);
+            if (A_MN) tma_load_3d_pair(sa + u * P_SUB_BYTES, &map_a, full_leader, ti.a_m + u * 64, ti.a_k0 + kb * STAGE_K, ti.z);
+            else tma_load_3d_pair(sa + u * P_SUB_BYTES, &map_a, full_leader, ti.a_k0 + kb * STAGE_K + u * BK, ti.a_m, ti.z);
+            if (B_MN) tma_load_3d_pair(sa + u * P_SUB_BYTES + P_A_BYTES, &map_b, full_leader, ti.b_n + u * 64, ti.b_k0 + kb * STAGE_K, ti.z);
+            else tma_load_3d_pair(sa + u * P_SUB_BYTES + P_A_BYTES, &map_b, full_leader, ti.b_k0 + kb * STAGE_K + u * BK, ti.b_n, ti.z);
           }
           if (++stage == P_STAGES) { stage = 0; phase ^= 1; }
         }
@@ -791,21 +876,22 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       RowPrefetch<P_EPI_COLS> pre;
       const bool with_stats = p.rs.targets != nullptr, gated = p.epilogue == kSwiGLU;
       if (with_stats) prefetch_targets<P_EPI_COLS>(p, row, n0, pre);
-      else if (p.staged && !gated) prefetch_addend_staged<P_EPI_COLS>(p, row, n0, ti.row_end, pre);
-      else if (!gated) prefetch_addend<P_EPI_COLS>(p, row, n0, ti.row_end, pre);
+      else if (p.staged && !gated) prefetch_addend_staged<P_EPI_COLS>(p, row, n0, ti.z, ti.row_end, pre);
+      else if (!gated) prefetch_addend<P_EPI_COLS>(p, row, n0, ti.z, ti.row_end, pre);
       ok = mbar_wait(smem_addr(&bar_acc_full[acc]), (local >> 1) & 1, p.status, kTimeoutEpilogue);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       fence_after_sync();
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN + chalf * P_EPI_COLS;
       const int row0 = ti.c_row0 + quarter * 32;
+      const Scaling sc{p.alpha, p.beta};
       if (gated)  // this warp: gate columns 64 * chalf .. + 63 of the tile and the same up columns
         store_accumulator_swiglu(p, &map_c, &map_h, stage, tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN + chalf * 64, row0, ti.n0 + chalf * 64,
                                  row0 < ti.row_end, lane);
       else if (with_stats) store_accumulator_with_stats<P_EPI_COLS>(p, taddr, row, n0, ti.tile_n * 2 + chalf, tiles_n * 2, pre);
-      else if (p.staged) store_accumulator_staged<P_EPI_COLS>(p, &map_c, stage, taddr, row0, n0, pre, row0 < ti.row_end, zero, lane);
-      else if (pre.tile_ok) store_accumulator_prefetched<P_EPI_COLS>(p, taddr, row, n0, pre, zero);
-      else store_accumulator<P_EPI_COLS>(p, taddr, row, n0, ti.row_end, zero);
+      else if (p.staged) store_accumulator_staged<P_EPI_COLS>(p, sc, &map_c, &map_h, stage, taddr, row0, n0, ti.z, pre, row0 < ti.row_end, ti.mirror, zero, lane);
+      else if (pre.tile_ok) store_accumulator_prefetched<P_EPI_COLS>(p, sc, taddr, row, n0, ti.z, pre, zero);
+      else store_accumulator<P_EPI_COLS>(p, sc, taddr, row, n0, ti.z, ti.row_end, zero);
       fence_before_sync();
       mbar_arrive_cluster_relaxed(acc_empty_leader[acc]);
     }
@@ -846,7 +932,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   const uint32_t crank = cluster_ctarank(), role = crank & 1, split = crank >> 1;
   const bool leader = role == 0;
   const int tiles_m = (p.M + P_TILE_M - 1) / P_TILE_M;
-  const int tile = blockIdx.x / (2 * SPLITS);
+  const int tiles = tiles_m * ((p.N + P_TILE_N - 1) / P_TILE_N);
+  const int z = (int)(blockIdx.x / (2 * SPLITS)) / tiles, tile = (int)(blockIdx.x / (2 * SPLITS)) - z * tiles;
   const int m0 = (tile % tiles_m) * P_TILE_M + role * P_HALF, n0 = (tile / tiles_m) * P_TILE_N;
   const int all_kb = (p.K + STAGE_K - 1) / STAGE_K, per_kb = (all_kb + SPLITS - 1) / SPLITS;
   const int kb0 = split * per_kb, num_kb = max(0, min(per_kb, all_kb - kb0));
@@ -870,6 +957,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   pdl_begin();
 
   bool ok = true;
+  const Scaling sc{p.alpha, p.beta};
   const int quarter = warp & 3, chalf = (warp - 2) >> 2;
   if (warp == 0) {
     if (elect_one()) {
@@ -884,10 +972,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         const int k0 = (kb0 + kb) * STAGE_K;
 #pragma unroll
         for (int u = 0; u < KSUB; ++u) {
-          if (A_MN) tma_load_2d_pair(sa + u * P_SUB_BYTES, &map_a, full_leader, m0 + u * 64, k0);
-          else tma_load_2d_pair(sa + u * P_SUB_BYTES, &map_a, full_leader, k0 + u * BK, m0);
-          if (B_MN) tma_load_2d_pair(sa + u * P_SUB_BYTES + P_A_BYTES, &map_b, full_leader, b0 + u * 64, k0);
-          else tma_load_2d_pair(sa + u * P_SUB_BYTES + P_A_BYTES, &map_b, full_leader, k0 + u * BK, b0);
+          if (A_MN) tma_load_3d_pair(sa + u * P_SUB_BYTES, &map_a, full_leader, m0 + u * 64, k0, z);
+          else tma_load_3d_pair(sa + u * P_SUB_BYTES, &map_a, full_leader, k0 + u * BK, m0, z);
+          if (B_MN) tma_load_3d_pair(sa + u * P_SUB_BYTES + P_A_BYTES, &map_b, full_leader, b0 + u * 64, k0, z);
+          else tma_load_3d_pair(sa + u * P_SUB_BYTES + P_A_BYTES, &map_b, full_leader, k0 + u * BK, b0, z);
         }
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
@@ -960,7 +1048,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         const float4 o = got[(src * OWN_ROWS + r0) * (P_TILE_N / 4) + (c ^ (r0 & 31))];
         t.x += o.x; t.y += o.y; t.z += o.z; t.w += o.w;
       }
-      if (row < p.M) store_vec4(p, t, row, n0 + c * 4);
+      if (row < p.M) store_vec4(p, sc, t, row, n0 + c * 4, z);
     }
   }
   fence_before_sync();
@@ -1012,6 +1100,12 @@ static cudaError_t launch_small(int a_mn, int b_mn, int tiles, int log_splits, i
 enum Variant : int { kPairK64 = 2, kPair = 3, kSplit2 = 4, kSplit4 = 5, kSmall = 10, kSmall2 = 11, kSmall4 = 12, kSmall8 = 13 };
 constexpr int kMaxPairs = kNumSM / 2;
 
+// 256x256 tiles of a stack of products (of a symmetric one: the diagonal and what lies above it).
+static int64_t pair_tile_count(int M, int N, int batch, int symmetric) {
+  const int64_t m = (M + tc::P_TILE_M - 1) / tc::P_TILE_M, n = (N + tc::P_TILE_N - 1) / tc::P_TILE_N;
+  return batch * (symmetric ? m * (m + 1) / 2 : m * n);
+}
+
 // How many clusters of `size` CTAs (one per SM) the device holds at a time: the GPCs do not divide evenly.
 static int resident_clusters(int size) {
   static std::atomic<int> cached[64][4];
@@ -1045,13 +1139,13 @@ static int resident_clusters(int size) {
 //   pair tiles over 2, 4 pairs: 10.8 + 0.66 / step, one wave only               (1000 x 2048 x 8192: 31.9 at 2)
 // Several waves of small tiles are bound by L2-to-SM traffic, so they pay a full wave each; the model drops them
 // quickly.  Products of more than about two waves of pair tiles always come out as pair tiles.
-static int choose_variant(int M, int N, int K) {
+static int choose_variant(int M, int N, int K, int batch, int symmetric) {
   using namespace tc;
-  const int64_t small = (int64_t)((M + BM - 1) / BM) * ((N + S_TILE_N - 1) / S_TILE_N);
-  const int64_t big = (int64_t)((M + P_TILE_M - 1) / P_TILE_M) * ((N + P_TILE_N - 1) / P_TILE_N);
+  const int64_t small = (int64_t)((M + BM - 1) / BM) * ((N + S_TILE_N - 1) / S_TILE_N) * batch;
+  const int64_t big = pair_tile_count(M, N, batch, 0);
   const int steps = (K + 127) / 128;
   int best = kPair;
-  float t = 7.0f + 0.56f * steps * ((big + kMaxPairs - 1) / kMaxPairs);
+  float t = 7.0f + 0.56f * steps * ((pair_tile_count(M, N, batch, symmetric) + kMaxPairs - 1) / kMaxPairs);
   auto consider = [&](int variant, float us) {
     if (us < t) { t = us; best = variant; }
   };
@@ -1062,6 +1156,14 @@ static int choose_variant(int M, int N, int K) {
     if (steps >= (4 << log) && big <= resident_clusters(2 << log)) consider(log == 1 ? kSplit2 : kSplit4, 10.8f + 0.66f * ((steps + (1 << log) - 1) >> log));
   return best;
 }
+
+// What a stack of products adds to a single one; see Params.
+struct BatchSpec {
+  int batch = 1;
+  int64_t a_stride = 0, b_stride = 0, c_stride = 0, r_stride = 0;
+  float alpha = 1.f, beta = 1.f;
+  bool symmetric = false;
+};
 
 // C[M,N] = op(A) * op(B)^T with epilogue (0 store, 1 C += result, 2 result + residual).
 //   a_mn == 0: A is [M, K] row-major (K-major), lda = row stride;  a_mn == 1: A is [K, M] row-major (M contiguous)
@@ -1074,8 +1176,11 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
                             int64_t ldb, int64_t ldc, int64_t ldr, int epilogue, int a_mn, int b_mn, int* status, int variant,
                             const void* stats_targets, int64_t stats_ldt, int stats_t_rows, int stats_shift, float* stats_partial,
                             const tc::Grouping* grp, cudaStream_t stream, const tc::Scatter* scatter = nullptr, void* gated_h = nullptr,
-                            int64_t gated_ldh = 0) {
+                            int64_t gated_ldh = 0, const BatchSpec* batched = nullptr) {
   using namespace tc;
+  static const BatchSpec one{};
+  const BatchSpec& bs = batched != nullptr ? *batched : one;
+  const bool symmetric = bs.symmetric && M == N;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((lda & 7) || (ldb & 7) || (reinterpret_cast<uintptr_t>(a) & 15) || (reinterpret_cast<uintptr_t>(b) & 15)) return -1;
   constexpr int smem_pair = P_RING_BYTES + P_STAGE_OUT_BYTES + 1024, smem_small = S_STAGES * S_STAGE_BYTES + S_RECV_BYTES + 1024;
@@ -1095,7 +1200,7 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
   }
   const bool mn = a_mn || b_mn;
   const bool plain = stats_targets == nullptr && grp == nullptr && scatter == nullptr && epilogue != kSwiGLU;
-  if (variant == 0) variant = plain ? choose_variant(M, N, K) : kPair;
+  if (variant == 0) variant = plain ? choose_variant(M, N, K, bs.batch, symmetric) : kPair;
   if (variant == 1) variant = kSmall;
   if (variant < kPairK64 || variant > kSmall8 || (variant > kSplit4 && variant < kSmall)) return -4;
   if (variant == kPairK64 && mn) return -4;
@@ -1103,14 +1208,16 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
   const bool pairs = variant < kSmall;
   CUtensorMap map_a, map_b;
   constexpr int mn_rows = 2 * BK;  // contraction rows of a transposed operand's box
-  int rc = a_mn ? make_map_bf16(&map_a, a, K, M, lda, mn_rows) : make_map_bf16(&map_a, a, M, K, lda, BM);
+  int rc = a_mn ? make_map_bf16_stack(&map_a, a, K, M, lda, mn_rows, bs.batch, bs.a_stride) : make_map_bf16_stack(&map_a, a, M, K, lda, BM, bs.batch, bs.a_stride);
   if (rc) return rc;
   // grouped by rows: B is the stack of the experts' matrices
   const int64_t b_stack = (grp != nullptr && grp->mode == kGroupRows) ? grp->num_groups : 1;
-  rc = b_mn ? make_map_bf16(&map_b, b, b_stack * K, N, ldb, mn_rows) : make_map_bf16(&map_b, b, b_stack * N, K, ldb, pairs ? P_HALF : S_TILE_N);
+  rc = b_mn ? make_map_bf16_stack(&map_b, b, b_stack * K, N, ldb, mn_rows, bs.batch, bs.b_stride)
+            : make_map_bf16_stack(&map_b, b, b_stack * N, K, ldb, pairs ? P_HALF : S_TILE_N, bs.batch, bs.b_stride);
   if (rc) return rc;
   Params p{(__nv_bfloat16*)c, (const __nv_bfloat16*)residual, M, N, K, ldc, ldr, epilogue, status, RowStatsOut{nullptr, 0, 0, 0, nullptr},
-           Grouping{kGroupNone, 0, nullptr, nullptr}, Scatter{}, (__nv_bfloat16*)gated_h, gated_ldh, 0};
+           Grouping{kGroupNone, 0, nullptr, nullptr}, Scatter{}, (__nv_bfloat16*)gated_h, gated_ldh, 0, bs.alpha, bs.beta, bs.batch,
+           bs.c_stride, bs.r_stride, 0};
   if (epilogue == kSwiGLU) {
     if (!pairs || a_mn || b_mn || grp != nullptr || stats_targets != nullptr || scatter != nullptr || gated_h == nullptr || (N & 255) || (ldc & 7) ||
         (gated_ldh & 7) || (reinterpret_cast<uintptr_t>(c) & 15) || (reinterpret_cast<uintptr_t>(gated_h) & 15))
@@ -1144,16 +1251,20 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
   if (scatter == nullptr && stats_targets == nullptr && (N & 7) == 0 && (ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(c) & 15) == 0 && reads_ok &&
       (grp == nullptr || grp->mode == kGroupRows || (M & 127) == 0)) {
     const int64_t rows = grp != nullptr && grp->mode == kGroupK ? (int64_t)grp->num_groups * M : M;
-    rc = make_map_bf16(&map_c, c, rows, N, ldc, 32);
-    if (rc == 0 && epilogue == kSwiGLU) rc = make_map_bf16(&map_h, gated_h, M, N / 2, gated_ldh, 32);
+    rc = make_map_bf16_stack(&map_c, c, rows, N, ldc, 32, bs.batch, bs.c_stride);
+    if (rc == 0 && epilogue == kSwiGLU) rc = make_map_bf16_stack(&map_h, gated_h, M, N / 2, gated_ldh, 32, 1, 0);
+    if (rc == 0 && symmetric && variant == kPair) {  // transposed stores: 64 rows of 32 elements
+      rc = make_map_bf16_stack(&map_h, c, M, N, ldc, 64, bs.batch, bs.c_stride, 32);
+      p.symmetric = 1;
+    }
     if (rc) return rc;
     p.staged = 1;
   }
   count_launch(1);
-  const int pair_tiles = ((M + P_TILE_M - 1) / P_TILE_M) * ((N + P_TILE_N - 1) / P_TILE_N);
+  const int pair_tiles = (int)pair_tile_count(M, N, bs.batch, p.symmetric);
   if (variant >= kSmall && variant <= kSmall8) {
     const int log_splits = variant - kSmall;
-    const int tiles = ((M + BM - 1) / BM) * ((N + S_TILE_N - 1) / S_TILE_N);
+    const int tiles = ((M + BM - 1) / BM) * ((N + S_TILE_N - 1) / S_TILE_N) * bs.batch;
     if (launch_small(a_mn, b_mn, tiles, log_splits, smem_small, stream, map_a, map_b, map_c, p) != cudaSuccess) return -3;
   } else if (variant == kSplit2) {
     launch_split<2>(a_mn, b_mn, pair_tiles, smem_pair, stream, map_a, map_b, p);
@@ -1181,6 +1292,24 @@ int launch_gemm_tcgen05(const void* a, const void* b, void* c, const void* resid
 int launch_gemm_tn_tcgen05(const void* a, const void* b, void* c, const void* residual, int M, int N, int K, int64_t lda,
                            int64_t ldb, int64_t ldc, int64_t ldr, int epilogue, int* status, int variant, cudaStream_t stream) {
   return launch_gemm_tcgen05(a, b, c, residual, M, N, K, lda, ldb, ldc, ldr, epilogue, 0, 0, status, variant, stream);
+}
+
+// ---- stacks of products (Newton-Schulz iterations of equally shaped matrices) ----------------------
+// c[z] = alpha * op(a[z]) * op(b[z])^T (+ beta * addend[z]), rounded as in Params.
+// All stacks dense: [batch, rows, cols].  `symmetric`: the caller knows that the product is (a Gram matrix, a power of a
+// symmetric matrix): only tiles on and above the diagonal are computed.
+int launch_gemm_stack(const void* a, const void* b, void* c, const void* addend, int batch, int M, int N, int K, int a_mn, int b_mn, float alpha,
+                      float beta, int symmetric, int* status, cudaStream_t stream) {
+  BatchSpec bs;
+  bs.batch = batch;
+  bs.a_stride = (int64_t)M * K;
+  bs.b_stride = (int64_t)N * K;
+  bs.c_stride = bs.r_stride = (int64_t)M * N;
+  bs.alpha = alpha;
+  bs.beta = beta;
+  bs.symmetric = symmetric != 0;
+  return launch_gemm_impl(a, b, c, addend, M, N, K, a_mn ? M : K, b_mn ? N : K, N, N, addend != nullptr ? tc::kAddResidual : tc::kStore, a_mn, b_mn, status, 0,
+                          nullptr, 0, 0, 0, nullptr, nullptr, stream, nullptr, nullptr, 0, &bs);
 }
 
 // ---- row-parallel product with the reduce-scatter's transfer in the epilogue -----------------

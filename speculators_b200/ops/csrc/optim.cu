@@ -158,21 +158,39 @@ adamw_kernel(float* __restrict__ master, float* __restrict__ m, float* __restric
 }
 
 // ---- Muon ------------------------------------------------------------------------------
-// Matrix update of Muon around its Newton-Schulz iteration (which runs as GEMMs):
+// Matrix update of Muon around its Newton-Schulz iteration (which runs as stacks of GEMMs over the matrices of one
+// shape), for all matrices of this rank in one launch each:
 //   muon_momentum: g' = g * grad_scale * clip;  buf = lerp(buf, g', 1 - momentum);
-//                  u = nesterov ? lerp(g', buf, momentum) : buf;  out = bf16(u)
-//                  plus the per-CTA sums of u^2 (for the Frobenius normalisation that
-//                  opens the iteration), one launch for both;
+//                  u = nesterov ? lerp(g', buf, momentum) : buf;  out = bf16(u), and the sums of u^2 per chunk
+//   muon_norms:    inv_norm[matrix] = bf16(1 / (|u| + 1e-7)), summed over the matrix's chunks in order
+//   muon_scale:    x = bf16(u * inv_norm), where the iteration starts
 //   muon_apply:    w = w * (1 - lr * wd) - lr * adjust * o;  w16 = bf16(w)
-// with lr = hyper[0] * lr_ratio (the matrix group follows the schedule of the AdamW group),
-// read from device memory so that the launches can be captured.
+// with lr = hyper[0] * lr_ratio (the matrix group follows the schedule of the AdamW group), read from device memory
+// so that the launches can be captured.  A block handles one chunk of one matrix:
+//   table[matrix] = {offset in the flat gradient / weight buffers, elements, offset in the state buffers},
+//   chunks[block] = {matrix, chunk inside it}.
+// Bound by memory (12 and 12 bytes per parameter plus the gradient): 16-byte accesses, one launch instead of one per
+// matrix (the small matrices of a narrow draft are a few microseconds each).
+constexpr int kMuonChunk = 4 * 8 * kOptThreads;
+
+struct MuonChunk {
+  int64_t flat, state, count;  // first element in the flat / state buffers, elements of the chunk
+  int matrix;
+};
+__device__ __forceinline__ MuonChunk muon_chunk(const int64_t* __restrict__ table, const int2* __restrict__ chunks) {
+  const int2 c = chunks[blockIdx.x];
+  const int64_t first = (int64_t)c.y * kMuonChunk, n = table[c.x * 3 + 1] - first;
+  return MuonChunk{table[c.x * 3] + first, table[c.x * 3 + 2] + first, n < kMuonChunk ? n : kMuonChunk, c.x};
+}
+
 template <typename G>
 __global__ void __launch_bounds__(kOptThreads)
-muon_momentum_kernel(const G* __restrict__ grad, float* __restrict__ buf, __nv_bfloat16* __restrict__ out, int64_t n,
-                     const float* __restrict__ hyper, const float* __restrict__ norm_sq, float momentum, int nesterov,
-                     float* __restrict__ partial) {
+muon_momentum_kernel(const G* __restrict__ grad, float* __restrict__ buf, __nv_bfloat16* __restrict__ out, const int64_t* __restrict__ table,
+                     const int2* __restrict__ chunks, const float* __restrict__ hyper, const float* __restrict__ norm_sq, float momentum,
+                     int nesterov, float* __restrict__ partial) {
   pdl_begin();
   __shared__ float scratch[33];
+  const MuonChunk c = muon_chunk(table, chunks);
   const float max_norm = hyper[7];
   float gscale = hyper[8];
   if (max_norm > 0.f && norm_sq) {
@@ -180,58 +198,121 @@ muon_momentum_kernel(const G* __restrict__ grad, float* __restrict__ buf, __nv_b
     if (coef < 1.f) gscale *= coef;
   }
   float acc = 0.f;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const float g = to_f<G>(grad[i]) * gscale;
-    float b = buf[i];
+  auto update = [&](float g, float& b) -> float {
+    g *= gscale;
     b += (g - b) * (1.f - momentum);
-    buf[i] = b;
-    const float u = nesterov ? g + (b - g) * momentum : b;
-    const __nv_bfloat16 r = __float2bfloat16(u);
-    out[i] = r;
-    const float ur = __bfloat162float(r);
-    acc += ur * ur;
+    return nesterov ? g + (b - g) * momentum : b;
+  };
+#pragma unroll
+  for (int it = 0; it < 4; ++it) {
+    const int64_t i = (int64_t)(it * kOptThreads + threadIdx.x) * 8;
+    if (i + 8 <= c.count) {
+      const f32x8 g = ld8s(grad + c.flat + i);
+      f32x8 b = ld8s(buf + c.state + i), u;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) u.v[j] = update(g.v[j], b.v[j]);
+      st8s(buf + c.state + i, b);
+      const bf16x8 r = pack8(u.v);
+      st8(out + c.state + i, r);
+      unpack8(r, u.v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc += u.v[j] * u.v[j];
+    } else {
+      for (int64_t k = i; k < c.count; ++k) {
+        float b = buf[c.state + k];
+        const __nv_bfloat16 r = __float2bfloat16(update(to_f<G>(grad[c.flat + k]), b));
+        buf[c.state + k] = b;
+        out[c.state + k] = r;
+        acc += __bfloat162float(r) * __bfloat162float(r);
+      }
+    }
   }
   acc = block_sum(acc, scratch);
   if (threadIdx.x == 0) partial[blockIdx.x] = acc;
 }
 
 __global__ void __launch_bounds__(kOptThreads)
-muon_apply_kernel(float* __restrict__ master, const __nv_bfloat16* __restrict__ update, __nv_bfloat16* __restrict__ w16, int64_t n,
-                  const float* __restrict__ hyper, float lr_ratio, float weight_decay, float adjust) {
+muon_norms_kernel(const float* __restrict__ partial, const int* __restrict__ first_chunk, float* __restrict__ inv_norm) {
   pdl_begin();
-  const float lr = hyper[0] * lr_ratio;
-  const float keep = 1.f - lr * weight_decay, step = lr * adjust;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const float w = master[i] * keep - step * __bfloat162float(update[i]);
-    master[i] = w;
-    if (w16) w16[i] = __float2bfloat16(w);
+  __shared__ float scratch[33];
+  float acc = 0.f;
+  for (int i = first_chunk[blockIdx.x] + threadIdx.x; i < first_chunk[blockIdx.x + 1]; i += blockDim.x) acc += partial[i];
+  acc = block_sum(acc, scratch);
+  if (threadIdx.x == 0) inv_norm[blockIdx.x] = __bfloat162float(__float2bfloat16(1.f / (sqrtf(acc) + 1e-7f)));
+}
+
+__global__ void __launch_bounds__(kOptThreads)
+muon_scale_kernel(__nv_bfloat16* __restrict__ x, const int64_t* __restrict__ table, const int2* __restrict__ chunks, const float* __restrict__ inv_norm) {
+  pdl_begin();
+  const MuonChunk c = muon_chunk(table, chunks);
+  const float s = inv_norm[c.matrix];
+#pragma unroll
+  for (int it = 0; it < 4; ++it) {
+    const int64_t i = (int64_t)(it * kOptThreads + threadIdx.x) * 8;
+    if (i + 8 <= c.count) {
+      float u[8];
+      unpack8(ld8(x + c.state + i), u);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) u[j] *= s;
+      st8(x + c.state + i, pack8(u));
+    } else {
+      for (int64_t k = i; k < c.count; ++k) x[c.state + k] = __float2bfloat16(__bfloat162float(x[c.state + k]) * s);
+    }
   }
 }
 
-// partial: [sumsq_num_partials()] scratch; out_sumsq[0] = sum of squares of the bf16 update
-void launch_muon_momentum(const void* grad, int grad_is_bf16, float* buf, void* out, int64_t n, const float* hyper,
-                          const float* norm_sq, float momentum, int nesterov, float* partial, float* out_sumsq,
-                          cudaStream_t stream) {
-  if (n <= 0) return;
-  const int P = 4 * kNumSM;
-  count_launch(2);
-  if (grad_is_bf16)
-    launch_pdl(muon_momentum_kernel<__nv_bfloat16>, P, kOptThreads, 0, stream, (const __nv_bfloat16*)grad, buf, (__nv_bfloat16*)out, n, hyper,
-                                                                       norm_sq, momentum, nesterov, partial);
-  else
-    launch_pdl(muon_momentum_kernel<float>, P, kOptThreads, 0, stream, (const float*)grad, buf, (__nv_bfloat16*)out, n, hyper, norm_sq,
-                                                               momentum, nesterov, partial);
-  launch_pdl(sumsq_final_kernel, 1, 256, 0, stream, partial, P, out_sumsq, 0);
+__global__ void __launch_bounds__(kOptThreads)
+muon_apply_kernel(float* __restrict__ master, const __nv_bfloat16* __restrict__ update, __nv_bfloat16* __restrict__ w16,
+                  const int64_t* __restrict__ table, const int2* __restrict__ chunks, const float* __restrict__ adjust,
+                  const float* __restrict__ hyper, float lr_ratio, float weight_decay) {
+  pdl_begin();
+  const MuonChunk c = muon_chunk(table, chunks);
+  const float lr = hyper[0] * lr_ratio;
+  const float keep = 1.f - lr * weight_decay, step = lr * adjust[c.matrix];
+#pragma unroll
+  for (int it = 0; it < 4; ++it) {
+    const int64_t i = (int64_t)(it * kOptThreads + threadIdx.x) * 8;
+    if (i + 8 <= c.count) {
+      const f32x8 u = ld8s(update + c.state + i);
+      f32x8 w = ld8s(master + c.state + i);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) w.v[j] = w.v[j] * keep - step * u.v[j];
+      st8s(master + c.state + i, w);
+      st8(w16 + c.flat + i, pack8(w.v));
+    } else {
+      for (int64_t k = i; k < c.count; ++k) {
+        const float w = master[c.state + k] * keep - step * __bfloat162float(update[c.state + k]);
+        master[c.state + k] = w;
+        w16[c.flat + k] = __float2bfloat16(w);
+      }
+    }
+  }
 }
 
-void launch_muon_apply(float* master, const void* update, void* w16, int64_t n, const float* hyper, float lr_ratio,
-                       float weight_decay, float adjust, cudaStream_t stream) {
-  if (n <= 0) return;
-  int64_t blocks = (n + kOptThreads - 1) / kOptThreads;
-  const int64_t cap = (int64_t)kNumSM * 16;
+int muon_chunk_elements() { return kMuonChunk; }
+
+// partial: fp32[num_chunks] scratch; inv_norm: fp32[num_matrices]
+void launch_muon_momentum(const void* grad, int grad_is_bf16, float* buf, void* out, const int64_t* table, const int* chunks, int num_chunks,
+                          const int* first_chunk, int num_matrices, const float* hyper, const float* norm_sq, float momentum, int nesterov,
+                          float* partial, float* inv_norm, cudaStream_t stream) {
+  if (num_chunks <= 0) return;
+  count_launch(3);
+  if (grad_is_bf16)
+    launch_pdl(muon_momentum_kernel<__nv_bfloat16>, num_chunks, kOptThreads, 0, stream, (const __nv_bfloat16*)grad, buf, (__nv_bfloat16*)out, table,
+               (const int2*)chunks, hyper, norm_sq, momentum, nesterov, partial);
+  else
+    launch_pdl(muon_momentum_kernel<float>, num_chunks, kOptThreads, 0, stream, (const float*)grad, buf, (__nv_bfloat16*)out, table, (const int2*)chunks,
+               hyper, norm_sq, momentum, nesterov, partial);
+  launch_pdl(muon_norms_kernel, num_matrices, kOptThreads, 0, stream, partial, first_chunk, inv_norm);
+  launch_pdl(muon_scale_kernel, num_chunks, kOptThreads, 0, stream, (__nv_bfloat16*)out, table, (const int2*)chunks, inv_norm);
+}
+
+void launch_muon_apply(float* master, const void* update, void* w16, const int64_t* table, const int* chunks, int num_chunks, const float* adjust,
+                       const float* hyper, float lr_ratio, float weight_decay, cudaStream_t stream) {
+  if (num_chunks <= 0) return;
   count_launch(1);
-  launch_pdl(muon_apply_kernel, (int)(blocks < cap ? blocks : cap), kOptThreads, 0, stream, 
-      master, (const __nv_bfloat16*)update, (__nv_bfloat16*)w16, n, hyper, lr_ratio, weight_decay, adjust);
+  launch_pdl(muon_apply_kernel, num_chunks, kOptThreads, 0, stream, master, (const __nv_bfloat16*)update, (__nv_bfloat16*)w16, table, (const int2*)chunks,
+             adjust, hyper, lr_ratio, weight_decay);
 }
 
 // Hyper-parameters travel as kernel arguments (copied at launch), so the host can

@@ -201,12 +201,17 @@ __device__ __forceinline__ void stage_put8(uint32_t stage, int lane, int chunk, 
   const uint4 x = *reinterpret_cast<const uint4*>(&v);
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(stage + lane * 128 + ((chunk ^ (lane & 7)) << 4)), "r"(x.x), "r"(x.y), "r"(x.z), "r"(x.w) : "memory");
 }
+__device__ __forceinline__ uint4 stage_get8(uint32_t stage, int lane, int chunk) {
+  uint4 x;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w) : "r"(stage + lane * 128 + ((chunk ^ (lane & 7)) << 4)) : "memory");
+  return x;
+}
 // The whole warp calls this once its 4 KB (1024-byte aligned) are written; `live`: the tile exists in the matrix.
-__device__ __forceinline__ void stage_store(uint32_t stage, const CUtensorMap* map, int x, int y, bool live) {
+__device__ __forceinline__ void stage_store(uint32_t stage, const CUtensorMap* map, int x, int y, int z, bool live) {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   __syncwarp();
   if (elect_one()) {
-    if (live) asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map), "r"(stage), "r"(x), "r"(y) : "memory");
+    if (live) asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(map), "r"(stage), "r"(x), "r"(y), "r"(z) : "memory");
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
   }
 }
@@ -245,11 +250,17 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
 __device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
-// TMA load whose completion bytes are counted on a barrier that may live in the peer CTA
-__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t cluster_bar, int x, int y) {
+// (_pair: the completion bytes are counted on a barrier that may live in the peer CTA)
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(dst), "l"(map), "r"(cluster_bar), "r"(x), "r"(y)
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap* map, uint32_t cluster_bar, int x, int y, int z) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(dst), "l"(map), "r"(cluster_bar), "r"(x), "r"(y), "r"(z)
       : "memory");
 }
 __device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
@@ -286,18 +297,14 @@ inline EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// Tensor map over a row-major [rows, cols] bf16 matrix with row stride `ld` elements; box =
-// 64 columns x `box_rows` rows, 128-byte swizzle, zero fill outside the matrix.
-inline int make_map_bf16(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int64_t ld, int box_rows) {
+inline int encode_map(CUtensorMap* map, const void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box,
+                      CUtensorMapSwizzle swizzle) {
   EncodeTiledFn fn = encode_fn();
   if (fn == nullptr) return -10;
-  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-  const cuuint32_t box[2] = {64u, (cuuint32_t)box_rows};
-  const cuuint32_t estr[2] = {1, 1};
+  const cuuint32_t estr[3] = {1, 1, 1};
   auto encode = [&]() {
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-              CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   };
   CUresult rc = encode();
   if (rc == CUDA_ERROR_INVALID_CONTEXT) {
@@ -307,6 +314,25 @@ inline int make_map_bf16(CUtensorMap* map, const void* base, int64_t rows, int64
     if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) rc = encode();
   }
   return rc == CUDA_SUCCESS ? 0 : -(1000 + (int)rc);  // -(1000 + CUresult)
+}
+
+// Tensor map over a row-major [rows, cols] bf16 matrix with row stride `ld` elements; box =
+// 64 columns x `box_rows` rows, 128-byte swizzle, zero fill outside the matrix.
+inline int make_map_bf16(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int64_t ld, int box_rows) {
+  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
+  const cuuint32_t box[2] = {64u, (cuuint32_t)box_rows};
+  return encode_map(map, base, 2, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+// The same over a stack of `batch` such matrices, `batch_stride` elements apart; boxes do not reach into the next one.
+// box_cols 64: 128-byte swizzle; any other width: rows as they are.
+inline int make_map_bf16_stack(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int64_t ld, int box_rows, int64_t batch,
+                               int64_t batch_stride, int box_cols = 64) {
+  const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)batch};
+  const cuuint64_t strides[2] = {(cuuint64_t)ld * 2, (cuuint64_t)(batch > 1 ? batch_stride : ld) * 2};
+  const cuuint32_t box[3] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 1u};
+  return encode_map(map, base, 3, dims, strides, box, box_cols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
 }  // namespace tc

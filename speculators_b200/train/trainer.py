@@ -18,6 +18,8 @@ a different execution model:
 
 from __future__ import annotations
 
+import contextlib
+import gc
 import json
 import logging
 import os
@@ -165,6 +167,33 @@ def _with_lookahead(iterable):
     yield cur, None
 
 
+@contextlib.contextmanager
+def _capturing(graph: torch.cuda.CUDAGraph, stream: torch.cuda.Stream):
+    """Capture the body into ``graph`` on ``stream`` (the one the warm-up ran on).
+
+    ``torch.cuda.graph`` collects garbage and gives the allocator's whole cache back to the driver first (0.1 s to
+    seconds once another trainer's memory has been freed), because a capture cannot do so when it runs short.  The
+    warm-up left behind what the step needs as cached blocks, so the cache has to go only if that much is not free
+    beside it.  The collector stays off meanwhile: what it frees could make calls that a capture forbids."""
+    torch.cuda.synchronize()
+    free, _ = torch.cuda.mem_get_info()
+    cached = torch.cuda.memory_reserved() - torch.cuda.memory_allocated()
+    if free < cached + cached // 8 + (1 << 30):
+        torch.cuda.empty_cache()
+    collecting = gc.isenabled()
+    gc.disable()
+    try:
+        with torch.cuda.stream(stream):
+            graph.capture_begin()
+            try:
+                yield
+            finally:
+                graph.capture_end()
+    finally:
+        if collecting:
+            gc.enable()
+
+
 class _GraphedStep:
     """CUDA-graph capture of forward + backward (+ optimizer) per input signature."""
 
@@ -185,6 +214,16 @@ class _GraphedStep:
     def signature(batch: dict) -> tuple:
         return tuple(sorted((k, tuple(v.shape), str(v.dtype)) for k, v in batch.items() if isinstance(v, torch.Tensor)))
 
+    _capture_streams: dict[torch.device, torch.cuda.Stream] = {}
+
+    @classmethod
+    def _capture_stream(cls, device: torch.device) -> torch.cuda.Stream:
+        """One stream per device for warm-ups and captures: the allocator keeps freed blocks per stream, so a stream of
+        its own for every signature would leave a warm-up's worth of memory behind each time."""
+        if device not in cls._capture_streams:
+            cls._capture_streams[device] = torch.cuda.Stream(device)
+        return cls._capture_streams[device]
+
     def _capture(self, batch: dict):
         tr = self.trainer
         dev = tr.device
@@ -195,7 +234,7 @@ class _GraphedStep:
         for k, v in static_in.items():
             v.copy_(batch[k], non_blocking=True)
         kwargs = tr.config.train_call_kwargs or {}
-        side = torch.cuda.Stream()
+        side = self._capture_stream(dev)
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):
             for _ in range(2):  # warm-up without touching the weights
@@ -205,7 +244,7 @@ class _GraphedStep:
         torch.cuda.current_stream().wait_stream(side)
         graph = torch.cuda.CUDAGraph()
         count_capture = ops.native().launch_count()
-        with torch.cuda.graph(graph):
+        with _capturing(graph, side):
             tr.engine.zero_grad()
             _, loss, metrics = tr.model(**static_in, **kwargs)
             loss.backward()
