@@ -56,8 +56,10 @@ class DFlashDecoderLayer(nn.Module):
         self.post_attention_layernorm = RMSNorm(config.hidden_size, config.rms_norm_eps)
 
     def forward(self, noise, target_hidden, noise_positions, all_positions, rotary, spec):
-        noise = self.self_attn(self.input_layernorm(noise), target_hidden, noise_positions, all_positions, rotary, spec, residual=noise)
-        return self.mlp(self.post_attention_layernorm(noise), residual=noise)
+        normed, noise = self.input_layernorm.fork(noise)
+        noise = self.self_attn(normed, target_hidden, noise_positions, all_positions, rotary, spec, residual=noise)
+        normed, noise = self.post_attention_layernorm.fork(noise)
+        return self.mlp(normed, residual=noise)
 
 
 # names of the reference's Hugging-Face-based classes (src/speculators/models/dflash/model_definitions.py:47,158)

@@ -67,7 +67,8 @@ class Eagle3FirstLayer(nn.Module):
         )
         residual = normed_hidden if self.norm_before_residual else hidden
         h = self.self_attn(x, positions, rotary, spec, past, ctx_len, residual=residual)
-        return self.mlp(self.post_attention_layernorm(h), residual=h)
+        normed, h = self.post_attention_layernorm.fork(h)
+        return self.mlp(normed, residual=h)
 
 
 @SpeculatorModel.register("eagle3")

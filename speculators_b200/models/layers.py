@@ -44,6 +44,10 @@ class RMSNorm(nn.Module):
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         return ops.rms_norm(x, self.weight, self.variance_epsilon)
 
+    def fork(self, x: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
+        """``(self(x), x)``: the input of a pre-norm block and its residual branch."""
+        return ops.rms_norm_fork(x, self.weight, self.variance_epsilon)
+
     def extra_repr(self) -> str:
         return f"{tuple(self.weight.shape)}, eps={self.variance_epsilon}"
 
@@ -322,5 +326,7 @@ class DecoderLayer(nn.Module):
         self.post_attention_layernorm = RMSNorm(config.hidden_size, config.rms_norm_eps)
 
     def forward(self, x, positions, rotary, spec, past=None, ctx_len=None) -> torch.Tensor:
-        x = self.self_attn(self.input_layernorm(x), positions, rotary, spec, past, ctx_len, residual=x)
-        return self.mlp(self.post_attention_layernorm(x), residual=x)
+        normed, x = self.input_layernorm.fork(x)
+        x = self.self_attn(normed, positions, rotary, spec, past, ctx_len, residual=x)
+        normed, x = self.post_attention_layernorm.fork(x)
+        return self.mlp(normed, residual=x)

@@ -52,9 +52,10 @@ class ZeroCenteredRMSNorm(nn.Module):
         self.variance_epsilon = eps
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        xf = x.float()
-        xf = xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + self.variance_epsilon)
-        return (xf * (1.0 + self.weight.float())).to(x.dtype)
+        return ops.rms_norm(x, self.weight, self.variance_epsilon, centred=True)
+
+    def fork(self, x: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
+        return ops.rms_norm_fork(x, self.weight, self.variance_epsilon, centred=True)
 
 
 class GatedAttention(nn.Module):

@@ -42,6 +42,7 @@ __all__ = [
     "masked_attention_reference",
     "native",
     "rms_norm",
+    "rms_norm_fork",
     "rope_",
     "rope_split",
     "sum_of_squares",
@@ -336,55 +337,93 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
 
 
 # --------------------------------------------------------------------------- rmsnorm
-_RMSNORM_MAX_WIDTH = 16384
+_RMSNORM_MAX_WIDTH = 32768
 
 
-def _rms_norm_ref(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
+def _rms_norm_ref(x: torch.Tensor, weight: torch.Tensor, eps: float, centred: bool = False) -> torch.Tensor:
     dt = x.dtype
     xf = x.float()
     xf = xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + eps)
-    return weight * xf.to(dt)
+    return (xf * (1.0 + weight.float())).to(dt) if centred else weight * xf.to(dt)
+
+
+def _grad_rows(d: torch.Tensor | None, width: int) -> torch.Tensor | None:
+    """A gradient as the ``[rows, width]`` layout the kernels read."""
+    if d is None:
+        return None
+    d2 = d.reshape(-1, width)
+    return d2 if d2.stride(-1) == 1 and d2.stride(0) % 8 == 0 and d2.data_ptr() % 16 == 0 else d2.contiguous()
+
+
+def _param_grad_target(weight: torch.Tensor) -> tuple[torch.Tensor, bool, bool]:
+    """Where a kernel puts a parameter's gradient: ``(buffer, accumulate, attached)``.  With a flat gradient view attached
+    by the training engine that view (stored into by the first gradient after ``zero_grad``, which left it uncleared, added
+    to by later ones; autograd then gets ``None``), else a fresh tensor."""
+    flat = getattr(weight, "_flat_grad", None)
+    if flat is None:
+        return torch.empty_like(weight), False, False
+    fresh = getattr(weight, "_grad_fresh", False)
+    weight._grad_fresh = False
+    return flat, not fresh, True
+
+
+def _norm_backward(dy, dy2, x2, weight, rstd, residual_grad, need_dx: bool, need_dw: bool, centred: bool):
+    """``(dx, dw)`` of a norm over ``x2 [rows, H]``; ``dw`` is ``None`` when it went into the engine's flat buffer."""
+    dx = torch.empty_like(x2) if need_dx else None
+    dw, accumulate, attached = _param_grad_target(weight) if need_dw else (None, False, False)
+    if need_dx or need_dw:
+        native().rmsnorm_bwd(dy, dy2, x2, weight, rstd, residual_grad if need_dx else None, dx, dw, accumulate, centred)
+    return dx, None if attached else dw
 
 
 class _RMSNormFn(torch.autograd.Function):
+    """Norm of ``x``; with ``fork`` the result is ``(normalised, x)`` and the gradient that comes back through the second
+    (a residual branch) is added inside the norm's backward kernel instead of a pass of autograd's own."""
+
     @staticmethod
-    def forward(ctx, x, weight, eps):
+    def forward(ctx, x, weight, eps, centred, fork):
         H = x.shape[-1]
         x2 = x.reshape(-1, H)
-        if x2.stride(-1) != 1:
+        if x2.stride(-1) != 1 or x2.stride(0) % 8 or x2.data_ptr() % 16:
             x2 = x2.contiguous()
         # allocated in the caller's shape and returned as it is: a view made in here could not be
         # modified in place afterwards (the rotary kernel does that to normalised q / k heads)
         y = torch.empty(x.shape, dtype=x.dtype, device=x.device)
         rstd = torch.empty(x2.shape[0], dtype=torch.float32, device=x.device)
-        native().rmsnorm_fwd(x2, weight, None, y.view(-1, H), rstd, eps)
+        native().norm_fwd(x2, weight, None, y.view(-1, H), rstd, eps, centred)
         ctx.save_for_backward(x2, weight, rstd)
-        ctx.shape = x.shape
-        return y
+        ctx.shape, ctx.centred = x.shape, centred
+        ctx.set_materialize_grads(False)
+        return (y, x.view_as(x)) if fork else y
 
     @staticmethod
-    def backward(ctx, dy):
+    def backward(ctx, dy, dres=None):
+        if dy is None:
+            return dres, None, None, None, None
         x2, weight, rstd = ctx.saved_tensors
         H = x2.shape[-1]
-        dy2 = dy.reshape(-1, H)
-        if dy2.stride(-1) != 1 or dy2.stride(0) % 8:
-            dy2 = dy2.contiguous()
-        dx = torch.empty_like(x2)
-        dw = None
-        if ctx.needs_input_grad[1]:
-            dw = torch.empty(H, dtype=torch.float32, device=x2.device)
-        native().rmsnorm_bwd(dy2, x2, weight, rstd, dx, dw, False, False)
-        return dx.view(ctx.shape), (dw.to(weight.dtype) if dw is not None else None), None
+        dx, dw = _norm_backward(_grad_rows(dy, H), None, x2, weight, rstd, _grad_rows(dres, H), ctx.needs_input_grad[0], ctx.needs_input_grad[1], ctx.centred)
+        return (dx.view(ctx.shape) if dx is not None else None), dw, None, None, None
 
 
-def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
-    """RMSNorm over the last dim: ``weight * (x / rms(x))`` with fp32 statistics.  Rows of up to
-    16384 elements run on the package's kernels (one row per CTA with the row in registers; one row
-    per warp for rows of up to 256); wider rows (the concatenated auxiliary states of a 70B-class
-    verifier: 3 x 8192) use the element-wise formulation."""
-    if _use_native(x) and x.shape[-1] <= _RMSNORM_MAX_WIDTH and x.shape[-1] % 8 == 0:
-        return _RMSNormFn.apply(x, weight, eps)
-    return _rms_norm_ref(x, weight, eps)
+def _norm_native(x: torch.Tensor) -> bool:
+    return _use_native(x) and x.dtype == torch.bfloat16 and x.shape[-1] <= _RMSNORM_MAX_WIDTH and x.shape[-1] % 8 == 0
+
+
+def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float, centred: bool = False) -> torch.Tensor:
+    """RMSNorm over the last dim: ``weight * (x / rms(x))`` with fp32 statistics (``centred``: ``(1 + weight)``, applied
+    before rounding).  bf16 CUDA rows of up to 32768 elements run on the package's kernels (one row per CTA with the row in
+    registers; one row per warp for rows of up to 256)."""
+    if _norm_native(x):
+        return _RMSNormFn.apply(x, weight, eps, centred, False)
+    return _rms_norm_ref(x, weight, eps, centred)
+
+
+def rms_norm_fork(x: torch.Tensor, weight: torch.Tensor, eps: float, centred: bool = False) -> tuple[torch.Tensor, torch.Tensor]:
+    """``(rms_norm(x), x)`` for a pre-norm block: the second result is the residual branch."""
+    if _norm_native(x) and torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad):
+        return _RMSNormFn.apply(x, weight, eps, centred, True)
+    return rms_norm(x, weight, eps, centred), x
 
 
 class _Eagle3InputFn(torch.autograd.Function):
@@ -413,27 +452,11 @@ class _Eagle3InputFn(torch.autograd.Function):
         T, H = hidden.shape
         if dout is None:
             dout = torch.zeros((T, 2 * H), dtype=hidden.dtype, device=hidden.device)
-        if dout.stride(1) != 1 or dout.stride(0) % 8:
-            dout = dout.contiguous()
-        nat = native()
+        dout = _grad_rows(dout, 2 * H)
         need_e, need_h, need_we, need_wh = ctx.needs_input_grad[:4]
-        d_e = d_h = dw_e = dw_h = None
-        if need_e or need_we:
-            d_e = torch.empty_like(embeds)
-            dw_e = torch.empty(H, dtype=torch.float32, device=hidden.device) if need_we else None
-            nat.rmsnorm_bwd(dout[:, :H], embeds, w_e, rs_e, d_e, dw_e, False, False)
-        if need_h or need_wh:
-            d_h = torch.empty_like(hidden)
-            dw_h = torch.empty(H, dtype=torch.float32, device=hidden.device) if need_wh else None
-            dy_h = dout[:, H:] if dhalf is None else dout[:, H:] + dhalf
-            nat.rmsnorm_bwd(dy_h, hidden, w_h, rs_h, d_h, dw_h, False, False)
-        return (
-            d_e if need_e else None,
-            d_h if need_h else None,
-            dw_e.to(w_e.dtype) if dw_e is not None else None,
-            dw_h.to(w_h.dtype) if dw_h is not None else None,
-            None,
-        )
+        d_e, dw_e = _norm_backward(dout[:, :H], None, embeds, w_e, rs_e, None, need_e, need_we, False)
+        d_h, dw_h = _norm_backward(dout[:, H:], _grad_rows(dhalf, H), hidden, w_h, rs_h, None, need_h, need_wh, False)
+        return d_e, d_h, dw_e, dw_h, None
 
 
 def eagle3_input_concat(embeds, hidden, w_embed_norm, w_hidden_norm, eps, return_hidden_half: bool = False):

@@ -9,9 +9,9 @@
 #include <ATen/ATen.h>
 
 namespace sb200 {
-int rmsnorm_bwd_partial_rows(int rows, int H);
+int rmsnorm_bwd_partial_rows(int rows, int H, bool with_dx);
 void launch_rmsnorm_fwd(const void*, const void*, const int64_t*, void*, float*, int, int, int64_t,
-                        int64_t, float, int64_t, cudaStream_t);
+                        int64_t, float, int64_t, int, cudaStream_t);
 struct BoundsRecord {
   int site;
   long long index;
@@ -19,8 +19,8 @@ struct BoundsRecord {
 };
 int read_bounds_norm(BoundsRecord*);
 int read_bounds_ep(BoundsRecord*);
-void launch_rmsnorm_bwd(const void*, const void*, const void*, const float*, void*, float*, float*,
-                        int, int, int64_t, int64_t, int64_t, int, int, cudaStream_t);
+void launch_rmsnorm_bwd(const void*, int64_t, const void*, int64_t, const void*, int64_t, const void*, const float*, const void*, int64_t, void*, int64_t,
+                        float*, void*, int, int, int, int, cudaStream_t);
 void launch_swiglu_fwd(const void*, void*, int64_t, int, cudaStream_t);
 void launch_swiglu_bwd(const void*, const void*, void*, int64_t, int, cudaStream_t);
 void launch_rope(void*, const int64_t*, const float*, const float*, int64_t, int, int, int, int64_t,
@@ -85,8 +85,8 @@ void check_rows(const Tensor& t, const char* name) {
               " rows must be 16-byte aligned");
 }
 
-void rmsnorm_fwd(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& row_index, Tensor y,
-                 c10::optional<Tensor> rstd, double eps) {
+void norm_fwd(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& row_index, Tensor y,
+              c10::optional<Tensor> rstd, double eps, bool centred) {
   check_rows(x, "x");
   check_rows(y, "y");
   const int H = (int)y.size(1);
@@ -94,7 +94,7 @@ void rmsnorm_fwd(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& 
   TORCH_CHECK(x.size(1) == H && w.numel() == H && w.is_contiguous() &&
                   w.scalar_type() == at::kBFloat16,
               "rmsnorm: shape/dtype mismatch");
-  TORCH_CHECK(H % 8 == 0 && H <= 16384, "rmsnorm: H must be a multiple of 8 and <= 16384");
+  TORCH_CHECK(H % 8 == 0 && H <= 32768, "rmsnorm: H must be a multiple of 8 and <= 32768");
   const int64_t* idx = nullptr;
   if (row_index.has_value()) {
     TORCH_CHECK(row_index->scalar_type() == at::kLong && row_index->is_contiguous() &&
@@ -111,30 +111,40 @@ void rmsnorm_fwd(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& 
   }
   c10::cuda::CUDAGuard guard(x.device());
   sb200::launch_rmsnorm_fwd(x.data_ptr(), w.data_ptr(), idx, y.data_ptr(), rs, rows, H, x.stride(0),
-                            y.stride(0), (float)eps, x.size(0), cur_stream());
+                            y.stride(0), (float)eps, x.size(0), centred ? 1 : 0, cur_stream());
+}
+void rmsnorm_fwd(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& row_index, Tensor y, c10::optional<Tensor> rstd, double eps) {
+  norm_fwd(x, w, row_index, y, rstd, eps, false);
 }
 
-void rmsnorm_bwd(const Tensor& dy, const Tensor& x, const Tensor& w, const Tensor& rstd, Tensor dx,
-                 c10::optional<Tensor> dw, bool accumulate_dx, bool accumulate_dw) {
-  check_rows(dy, "dy");
-  check_rows(x, "x");
-  check_rows(dx, "dx");
-  const int rows = (int)x.size(0), H = (int)x.size(1);
-  TORCH_CHECK(dy.size(0) == rows && dy.size(1) == H && dx.size(0) == rows && dx.size(1) == H);
-  TORCH_CHECK(H % 8 == 0 && H <= 16384);
+// dx = norm gradient of (dy + dy2) (+ add), dw bf16[H] (=, +=); dy2, add, dx, dw optional.  centred: the weight is 1 + w.
+void rmsnorm_bwd(const Tensor& dy, const c10::optional<Tensor>& dy2, const Tensor& x, const Tensor& w, const Tensor& rstd, const c10::optional<Tensor>& add,
+                 c10::optional<Tensor> dx, c10::optional<Tensor> dw, bool accumulate_dw, bool centred) {
+  const int64_t rows = x.size(0), H = x.size(1);
+  auto rows_of = [&](const c10::optional<Tensor>& t, const char* name, int64_t& stride) -> void* {
+    if (!t.has_value()) return nullptr;
+    check_rows(*t, name);
+    TORCH_CHECK(t->size(0) == rows && t->size(1) == H, "rmsnorm_bwd: ", name, " has another shape");
+    stride = t->stride(0);
+    return t->data_ptr();
+  };
+  int64_t sy = 0, sy2 = 0, sx = 0, sa = 0, sd = 0;
+  void* py = rows_of(dy, "dy", sy);
+  void* py2 = rows_of(dy2, "dy2", sy2);
+  void* px = rows_of(x, "x", sx);
+  void* pa = rows_of(add, "add", sa);
+  void* pd = rows_of(dx, "dx", sd);
+  TORCH_CHECK(H % 8 == 0 && H <= 32768 && w.numel() == H && w.scalar_type() == at::kBFloat16 && w.is_contiguous());
+  TORCH_CHECK(rstd.scalar_type() == at::kFloat && rstd.numel() == rows && rstd.is_contiguous());
   c10::cuda::CUDAGuard guard(x.device());
-  float* dwp = nullptr;
-  float* dwo = nullptr;
   Tensor partial;
   if (dw.has_value()) {
-    TORCH_CHECK(dw->scalar_type() == at::kFloat && dw->numel() == H && dw->is_contiguous());
-    partial = at::empty({sb200::rmsnorm_bwd_partial_rows(rows, H), H}, dw->options());
-    dwp = partial.data_ptr<float>();
-    dwo = dw->data_ptr<float>();
+    TORCH_CHECK(dw->scalar_type() == at::kBFloat16 && dw->numel() == H && dw->is_contiguous());
+    partial = at::empty({sb200::rmsnorm_bwd_partial_rows((int)rows, (int)H, pd != nullptr), H}, rstd.options());
+    if (rows == 0 && !accumulate_dw) dw->zero_();
   }
-  sb200::launch_rmsnorm_bwd(dy.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr<float>(),
-                            dx.data_ptr(), dwp, dwo, rows, H, dy.stride(0), x.stride(0),
-                            dx.stride(0), accumulate_dx, accumulate_dw, cur_stream());
+  sb200::launch_rmsnorm_bwd(py, sy, py2, sy2, px, sx, w.data_ptr(), rstd.data_ptr<float>(), pa, sa, pd, sd, dw.has_value() ? partial.data_ptr<float>() : nullptr,
+                            dw.has_value() ? dw->data_ptr() : nullptr, (int)rows, (int)H, accumulate_dw ? 1 : 0, centred ? 1 : 0, cur_stream());
 }
 
 Tensor swiglu_fwd(const Tensor& gate_up) {
@@ -916,6 +926,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> attn_bwd(
 
 TORCH_LIBRARY(sb200, m) {
   m.def("rmsnorm_fwd", &rmsnorm_fwd);
+  m.def("norm_fwd", &norm_fwd);
   m.def("rmsnorm_bwd", &rmsnorm_bwd);
   m.def("swiglu_fwd", &swiglu_fwd);
   m.def("swiglu_bwd", &swiglu_bwd);

@@ -320,8 +320,7 @@ class TrainEngine:
         for p, o in zip(self.params, self.offsets):
             p.data = self.flat_w[o : o + p.numel()].view(p.shape)
             p.grad = self.flat_g[o : o + p.numel()].view(p.shape)
-            if p.ndim == 2:  # ops.linear accumulates weight gradients straight into this view
-                p._flat_grad = p.grad
+            p._flat_grad = p.grad  # the ops' backward passes put parameter gradients straight into this view
         self._init32 = init32
 
     def _init_state(self) -> None:
@@ -379,24 +378,19 @@ class TrainEngine:
 
     # ------------------------------------------------------------------ step
     def zero_grad(self) -> None:
-        """Clear the gradient buffer.  On CUDA the matrices (almost all of the buffer) are
-        not written: they are flagged ``_grad_fresh`` and whoever produces their first
-        gradient of the step stores it instead of accumulating (``ops.linear``'s weight
-        gradient GEMM, or the hook below for gradients that arrive through autograd's own
-        accumulation); ``apply`` clears the ones nothing touched."""
+        """Clear the gradient buffer.  On CUDA nothing is written: the parameters are flagged
+        ``_grad_fresh`` and whoever produces the first gradient of the step stores it instead of
+        accumulating (the backward passes of ``ops``, or the hook below for gradients that arrive
+        through autograd's own accumulation); ``apply`` clears the ones nothing touched."""
         lazy = self._lazy_zero
         if not lazy:
             self.flat_g.zero_()
         for p, o in zip(self.params, self.offsets):  # re-attach if something replaced .grad
             if p.grad is None or p.grad.data_ptr() != self.flat_g.data_ptr() + o * self.flat_g.element_size():
                 p.grad = self.flat_g[o : o + p.numel()].view(p.shape)
-                if p.ndim == 2:
-                    p._flat_grad = p.grad
+                p._flat_grad = p.grad
             if lazy:
-                if p.ndim == 2:
-                    p._grad_fresh = True
-                else:
-                    p.grad.zero_()
+                p._grad_fresh = True
 
     def _install_lazy_zero_hooks(self) -> None:
         def make(p):
@@ -412,20 +406,18 @@ class TrainEngine:
             return on_grad
 
         for p in self.params:
-            if p.ndim == 2:
-                p._grad_fresh = False
-                p.register_hook(make(p))
+            p._grad_fresh = False
+            p.register_hook(make(p))
 
     def mark_grads_written(self) -> None:
         """Call after writing gradients into ``flat_g`` / ``p.grad`` directly (not through
         backward): tells ``apply`` that the matrices' regions hold this step's gradients."""
         for p in self.params:
-            if p.ndim == 2:
-                p._grad_fresh = False
+            p._grad_fresh = False
 
     def _settle_untouched_grads(self) -> None:
         for p in self.params:
-            if p.ndim == 2 and getattr(p, "_grad_fresh", False):
+            if getattr(p, "_grad_fresh", False):
                 p._grad_fresh = False
                 p._flat_grad.zero_()
 

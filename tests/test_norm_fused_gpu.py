@@ -1,0 +1,62 @@
+"""RMSNorm variants against fp32: zero-centred weights, the residual gradient added in the backward kernel, rows up to 32768,
+the weight gradient alone, and gradients that go into an attached flat buffer."""
+
+import pytest
+import torch
+
+from speculators_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+
+def _reference(x, w, eps, centred):
+    xf = x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + eps)
+    return xf * (1 + w if centred else w)
+
+
+# narrow rows, one block per row at every register budget, the widest rows; one row and more rows than blocks
+@pytest.mark.parametrize("rows,H", [(1, 8), (700, 128), (300, 264), (33, 4104), (50, 9000), (40, 16392), (700, 24576), (3, 32768)])
+@pytest.mark.parametrize("centred", [False, True])
+@pytest.mark.parametrize("input_grad", [True, False])
+def test_fork_backward(rows, H, centred, input_grad):
+    torch.manual_seed(H)
+    x = torch.randn(rows, H, device="cuda").bfloat16().requires_grad_(input_grad)
+    w = (torch.rand(H, device="cuda") - (0.5 if centred else -0.5)).bfloat16().requires_grad_()
+    dy, dres = torch.randn(rows, H, device="cuda").bfloat16(), torch.randn(rows, H, device="cuda").bfloat16()
+    y, res = ops.rms_norm_fork(x, w, 1e-5, centred)
+    torch.autograd.backward([y, res] if input_grad else [y], [dy, dres] if input_grad else [dy])
+    xf, wf = x.detach().float().requires_grad_(), w.detach().float().requires_grad_()
+    yf = _reference(xf, wf, 1e-5, centred)
+    yf.backward(dy.float())
+    assert (y.float() - yf).abs().max() <= 0.02 * yf.abs().max()
+    assert (w.grad.float() - wf.grad).abs().max() <= 0.01 * wf.grad.abs().max() + 0.02
+    if input_grad:
+        want = xf.grad + dres.float()
+        assert (x.grad.float() - want).abs().max() <= 0.02 * want.abs().max()
+
+
+def test_weight_gradient_goes_to_the_flat_buffer():
+    torch.manual_seed(0)
+    x = torch.randn(100, 512, device="cuda").bfloat16()
+    w = torch.ones(512, device="cuda", dtype=torch.bfloat16).requires_grad_()
+    w._flat_grad, w._grad_fresh = torch.full_like(w, float("nan")), True  # the first gradient is stored, the second added
+    dy = torch.randn_like(x)
+    for _ in range(2):
+        ops.rms_norm(x, w, 1e-5).backward(dy)
+    xf = x.float() * torch.rsqrt(x.float().pow(2).mean(-1, keepdim=True) + 1e-5)
+    want = 2 * (dy.float() * xf).sum(0)
+    assert w.grad is None and (w._flat_grad.float() - want).abs().max() <= 0.02 * want.abs().max()
+
+
+def test_eagle3_input_adds_the_half_gradient():
+    torch.manual_seed(0)
+    T, H = 130, 256
+    e, h = torch.randn(T, H, device="cuda").bfloat16(), torch.randn(T, H, device="cuda").bfloat16().requires_grad_()
+    we, wh = (torch.rand(H, device="cuda").bfloat16().requires_grad_() for _ in range(2))
+    out, half = ops.eagle3_input_concat(e, h, we, wh, 1e-5, return_hidden_half=True)
+    d, dh = torch.randn_like(out), torch.randn(T, H, device="cuda").bfloat16()
+    torch.autograd.backward([out, half], [d, dh])
+    hf, wf = h.detach().float().requires_grad_(), wh.detach().float().requires_grad_()
+    _reference(hf, wf, 1e-5, False).backward(d[:, H:].float() + dh.float())
+    assert (h.grad.float() - hf.grad).abs().max() <= 0.02 * hf.grad.abs().max() + 0.02
+    assert (wh.grad.float() - wf.grad).abs().max() <= 0.02 * wf.grad.abs().max() and torch.isfinite(we.grad).all()
