@@ -39,6 +39,7 @@ from speculators_b200.layer_config import TransformerLayerConfig
 from speculators_b200.models.layers import FusedLinear, Linear, RotaryTable
 from speculators_b200.models.mtp.model_definitions import _MTPMixin
 from speculators_b200.ops import AttnSpec
+from speculators_b200.ops.moe import moe_experts, moe_experts_ok
 
 __all__ = ["GatedAttention", "MoEDecoderLayer", "MoEMTPLayer", "SparseMoeBlock", "ZeroCenteredRMSNorm", "expert_forward"]
 
@@ -73,9 +74,17 @@ class GatedAttention(nn.Module):
         self.q_norm = ZeroCenteredRMSNorm(self.hd, config.rms_norm_eps)
         self.k_norm = ZeroCenteredRMSNorm(self.hd, config.rms_norm_eps)
 
-    def forward(self, x, positions, rotary: RotaryTable, spec: AttnSpec) -> torch.Tensor:
+    def forward(self, x, positions, rotary: RotaryTable, spec: AttnSpec, residual: torch.Tensor | None = None) -> torch.Tensor:
         T = x.shape[0]
         qg = self.q_proj(x).view(T, self.nh, 2 * self.hd)
+        split = ops.split_gated_query(qg, self.q_norm.weight, self.q_norm.variance_epsilon)
+        if split is not None:
+            q, gate = split
+            k = self.k_norm(self.k_proj(x).view(T, self.nkv, self.hd))
+            q = ops.rope_(q, positions, rotary.cos, rotary.sin, self.nh, self.hd, self.rot)
+            k = ops.rope_(k, positions, rotary.cos, rotary.sin, self.nkv, self.hd, self.rot)
+            out = ops.masked_attention(q, k, self.v_proj(x).view(T, self.nkv, self.hd), spec, scale=self.scaling)
+            return self.o_proj(ops.gated(out, gate).view(T, self.nh * self.hd), residual=residual)
         q, gate = qg[..., : self.hd], qg[..., self.hd :].reshape(T, self.nh * self.hd)
         q = self.q_norm(q).reshape(T, self.nh * self.hd)
         k = self.k_norm(self.k_proj(x).view(T, self.nkv, self.hd)).reshape(T, self.nkv * self.hd)
@@ -83,7 +92,7 @@ class GatedAttention(nn.Module):
         q = ops.rope_(q.contiguous(), positions, rotary.cos, rotary.sin, self.nh, self.hd, self.rot).view(T, self.nh, self.hd)
         k = ops.rope_(k.contiguous(), positions, rotary.cos, rotary.sin, self.nkv, self.hd, self.rot).view(T, self.nkv, self.hd)
         out = ops.masked_attention(q, k, v, spec, scale=self.scaling).reshape(T, self.nh * self.hd)
-        return self.o_proj(out * torch.sigmoid(gate))
+        return self.o_proj(out * torch.sigmoid(gate), residual=residual)
 
 
 class _Experts(nn.Module):
@@ -227,7 +236,17 @@ class SparseMoeBlock(nn.Module):
             top_p = top_p / top_p.sum(dim=-1, keepdim=True)
         return top_p.to(x.dtype), top_e
 
-    def forward(self, x: torch.Tensor) -> torch.Tensor:
+    def forward(self, x: torch.Tensor, residual: torch.Tensor | None = None) -> torch.Tensor:
+        """The block's output, plus ``residual`` when given."""
+        if self.ep_size == 1 and moe_experts_ok(x, self.experts.gate_up_proj, self.experts.down_proj):
+            top_p, top_e = self.route(x)
+            shared, gate = (None, None) if self.shared_expert is None else (self.shared_expert(x), self.shared_expert_gate(x))
+            return moe_experts(x, top_p, top_e, self.experts.gate_up_proj, self.experts.down_proj, shared, gate, residual)
+        out = self._sorted_forward(x)
+        return out if residual is None else residual + out
+
+    def _sorted_forward(self, x: torch.Tensor) -> torch.Tensor:
+        """Rows sorted by expert through autograd's own indexing: expert parallelism, and operands outside the fused path."""
         T, H = x.shape
         top_p, top_e = self.route(x)
         if self.ep_size > 1 and self._peer_exchange_ok(x):
@@ -337,8 +356,10 @@ class MoEDecoderLayer(nn.Module):
         self.post_attention_layernorm = ZeroCenteredRMSNorm(H, eps)
 
     def forward(self, x, positions, rotary, spec) -> torch.Tensor:
-        x = x + self.self_attn(self.input_layernorm(x), positions, rotary, spec)
-        return x + self.mlp(self.post_attention_layernorm(x))
+        normed, x = self.input_layernorm.fork(x)
+        x = self.self_attn(normed, positions, rotary, spec, residual=x)
+        normed, x = self.post_attention_layernorm.fork(x)
+        return self.mlp(normed, residual=x)
 
 
 class MoEMTPLayer(_MTPMixin, MoEDecoderLayer):

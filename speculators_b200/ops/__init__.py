@@ -15,6 +15,8 @@ kernels via ``torch.autograd.Function``.
 
 from __future__ import annotations
 
+import math
+
 import torch
 import torch.nn.functional as F
 
@@ -27,6 +29,7 @@ __all__ = [
     "adamw_step_",
     "eagle3_input_concat",
     "fused_row_loss",
+    "gated",
     "check_gemm_status",
     "gemm_status",
     "GroupPlan",
@@ -45,6 +48,7 @@ __all__ = [
     "rms_norm_fork",
     "rope_",
     "rope_split",
+    "split_gated_query",
     "sum_of_squares",
     "swiglu",
     "token_cross_entropy",
@@ -221,8 +225,9 @@ class _GroupedLinearFn(torch.autograd.Function):
             dx = torch.empty_like(x_pad)
             native().gemm_grouped_rows(dy, weight, dx, True, seg, mts, status)
         if ctx.needs_input_grad[1]:
-            dw = torch.empty_like(weight)
-            native().gemm_grouped_wgrad(dy, x_pad, dw, False, seg, mts, status)
+            dw, accumulate, attached = _param_grad_target(weight)
+            native().gemm_grouped_wgrad(dy, x_pad, dw, accumulate, seg, mts, status)
+            dw = None if attached else dw
         return dx, dw, None, None
 
 
@@ -541,42 +546,51 @@ def _rope_ref(x, positions, cos_t, sin_t, heads, hd, rot, sign):
     return torch.cat([y.reshape(T, heads * hd), x[:, heads * hd :]], dim=-1)
 
 
+def _unrotate(dq, dk, dv, positions, cos_t, sin_t, heads, hd, rot):
+    """Gradient of a rotation: the ``[T, .]`` gradients side by side in a fresh buffer (an incoming one may be shared with
+    other consumers), the first ``heads`` heads rotated back."""
+    parts = [_grad_rows(d, math.prod(d.shape[1:])) if d is not None else None for d in (dq, dk, dv)]
+    merge = rot % 16 == 0 and all(p is None or (p.shape[1] % hd == 0 and p.data_ptr() % 16 == 0) for p in parts)
+    nq = parts[0].shape[1] // hd
+    rotate_k = heads > nq
+    if merge and heads == nq + (parts[1].shape[1] // hd if rotate_k else 0) and positions.is_contiguous():
+        return native().rope_merge(*parts, rotate_k, positions, cos_t, sin_t, hd, rot, -1.0)
+    d = parts[0].clone() if dk is None else torch.cat([p for p in parts if p is not None], dim=-1)
+    native().rope_(d, positions, cos_t, sin_t, heads, hd, rot, -1.0)
+    return d
+
+
 class _RopeFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, positions, cos_t, sin_t, heads, hd, rot):
         ctx.save_for_backward(positions, cos_t, sin_t)
         ctx.cfg = (heads, hd, rot)
-        native().rope_(x, positions, cos_t, sin_t, heads, hd, rot, 1.0)
+        native().rope_(x.view(x.shape[0], -1), positions, cos_t, sin_t, heads, hd, rot, 1.0)
         ctx.mark_dirty(x)
         return x
 
     @staticmethod
     def backward(ctx, dx):
-        positions, cos_t, sin_t = ctx.saved_tensors
-        heads, hd, rot = ctx.cfg
-        dx = dx.clone()  # the incoming gradient may be shared with other consumers
-        native().rope_(dx, positions, cos_t, sin_t, heads, hd, rot, -1.0)
-        return dx, None, None, None, None, None, None
+        return _unrotate(dx, None, None, *ctx.saved_tensors, *ctx.cfg).view(dx.shape), None, None, None, None, None, None
 
 
 def rope_(x, positions, cos_t, sin_t, heads: int, hd: int, rot: int):
     """Neox rotary embedding of the first ``heads`` heads of every row of ``x``
-    (``[T, >= heads*hd]``), rotating the first ``rot`` channels of each head.
+    (``[T, >= heads*hd]`` or ``[T, heads, hd]``), rotating the first ``rot`` channels of each head.
     In place on CUDA; returns the rotated tensor."""
     if _use_native(x):
-        if x._is_view() or x.stride(-1) != 1:  # noqa: SLF001
+        if x._is_view() or x.stride(-1) != 1 or (x.dim() == 3 and not x.is_contiguous()):  # noqa: SLF001
             # rotating a view in place would rewrite its base's history (and is refused outright for
             # views that custom functions hand out): work on a private copy instead
             x = x.clone(memory_format=torch.contiguous_format)
         return _RopeFn.apply(x, positions, cos_t, sin_t, heads, hd, rot)
-    return _rope_ref(x, positions, cos_t, sin_t, heads, hd, rot, 1.0)
+    return _rope_ref(x.reshape(x.shape[0], -1), positions, cos_t, sin_t, heads, hd, rot, 1.0).view(x.shape)
 
 
 class _RopeSplitFn(torch.autograd.Function):
     """Rotate the q|k heads of a fused projection buffer in place and hand out the
-    q / k / v column blocks as views.  Backward gathers the three gradients into one
-    fresh buffer (a single concatenation instead of three zero-filled slice
-    gradients and their sums) and un-rotates it in place."""
+    q / k / v column blocks as views.  Backward lays the three gradients side by side in one
+    fresh buffer and un-rotates them on the way, in one pass."""
 
     @staticmethod
     def forward(ctx, qkv, positions, cos_t, sin_t, heads, hd, rot, nq, nk):
@@ -589,11 +603,68 @@ class _RopeSplitFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dq, dk, dv):
-        positions, cos_t, sin_t = ctx.saved_tensors
-        heads, hd, rot = ctx.cfg
-        d = torch.cat([dq, dk, dv], dim=-1)
-        native().rope_(d, positions, cos_t, sin_t, heads, hd, rot, -1.0)
-        return d, None, None, None, None, None, None, None, None
+        return _unrotate(dq, dk, dv, *ctx.saved_tensors, *ctx.cfg), None, None, None, None, None, None, None, None
+
+
+# --------------------------------------------------------------------------- gated attention
+class _SplitGatedQueryFn(torch.autograd.Function):
+    """``(centred_rms_norm(qg[..., :hd]), qg[..., hd:])``; the query half is read and its gradient written in place inside the
+    ``[T, heads, 2 * hd]`` buffer, into the other half of which ``_GatedFn`` has put the gate's gradient."""
+
+    @staticmethod
+    def forward(ctx, qg, weight, eps):
+        T, heads, two = qg.shape
+        hd = two // 2
+        x2 = qg.view(T * heads, two)[:, :hd]
+        q = torch.empty((T, heads, hd), dtype=qg.dtype, device=qg.device)
+        rstd = torch.empty(T * heads, dtype=torch.float32, device=qg.device)
+        native().norm_fwd(x2, weight, None, q.view(T * heads, hd), rstd, eps, True)
+        ctx.save_for_backward(qg, weight, rstd)
+        return q, qg[..., hd:]
+
+    @staticmethod
+    def backward(ctx, dq, dgate):
+        qg, weight, rstd = ctx.saved_tensors
+        T, heads, two = qg.shape
+        hd = two // 2
+        in_place = (dgate.dtype == qg.dtype and dgate.stride() == (heads * two, two, 1) and dgate.storage_offset() == hd
+                    and dgate.untyped_storage().nbytes() == qg.numel() * qg.element_size())
+        if in_place:
+            d = dgate.as_strided(qg.shape, (heads * two, two, 1), 0)
+        else:
+            d = torch.empty_like(qg)
+            d[..., hd:] = dgate
+        rows = T * heads
+        dw, accumulate, attached = _param_grad_target(weight) if ctx.needs_input_grad[1] else (None, False, False)
+        native().rmsnorm_bwd(_grad_rows(dq, hd), None, qg.view(rows, two)[:, :hd], weight, rstd, None, d.view(rows, two)[:, :hd], dw, accumulate, True)
+        return d, None if attached else dw, None
+
+
+class _GatedFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, out, gate):
+        ctx.save_for_backward(out, gate)
+        return native().gate_mul_fwd(out, gate)
+
+    @staticmethod
+    def backward(ctx, dy):
+        out, gate = ctx.saved_tensors
+        T, heads, hd = out.shape
+        dgate = torch.empty((T, heads, gate.stride(1)), dtype=out.dtype, device=out.device)[..., -hd:]  # of a projection: its second half
+        return native().gate_mul_bwd(dy.contiguous(), out, gate, dgate), dgate
+
+
+def split_gated_query(qg: torch.Tensor, weight: torch.Tensor, eps: float):
+    """Query and gate of a gated attention from the ``[T, heads, 2 * hd]`` projection: the query normalised with a zero-centred
+    weight, the gate as a view.  ``None`` where the kernels do not take the tensor and the caller runs the steps one by one."""
+    if not (_norm_native(qg) and qg.is_contiguous() and qg.shape[-1] % 16 == 0):
+        return None
+    return _SplitGatedQueryFn.apply(qg, weight, eps)
+
+
+def gated(out: torch.Tensor, gate: torch.Tensor) -> torch.Tensor:
+    """``out * sigmoid(gate)`` for ``[T, heads, hd]`` CUDA tensors, ``gate`` as ``split_gated_query`` returns it."""
+    return _GatedFn.apply(out.contiguous(), gate)
 
 
 def rope_split(qkv, positions, cos_t, sin_t, heads: int, hd: int, rot: int, nq: int, nk: int):

@@ -21,8 +21,20 @@ int read_bounds_norm(BoundsRecord*);
 int read_bounds_ep(BoundsRecord*);
 void launch_rmsnorm_bwd(const void*, int64_t, const void*, int64_t, const void*, int64_t, const void*, const float*, const void*, int64_t, void*, int64_t,
                         float*, void*, int, int, int, int, cudaStream_t);
-void launch_swiglu_fwd(const void*, void*, int64_t, int, cudaStream_t);
-void launch_swiglu_bwd(const void*, const void*, void*, int64_t, int, cudaStream_t);
+void launch_swiglu_fwd(const void*, void*, int64_t, int, const int*, cudaStream_t);
+void launch_swiglu_bwd(const void*, const void*, void*, int64_t, int, const int*, cudaStream_t);
+void launch_rope_merge(const void* const*, const int64_t*, const int*, const int*, void*, int64_t, const int64_t*, const float*, const float*, int64_t, int, int,
+                       int, float, cudaStream_t);
+void launch_gate_mul_fwd(const void*, const void*, void*, int, int, int, int64_t, int, cudaStream_t);
+void launch_gate_mul_bwd(const void*, const void*, const void*, void*, void*, int, int, int, int64_t, int, int64_t, cudaStream_t);
+int moe_plan_blocks(int);
+int launch_moe_plan(const int64_t*, int, int, int, int*, int*, int*, int*, int*, cudaStream_t);
+void launch_moe_gather(const void*, int64_t, const int*, const int*, int, void*, int, int, cudaStream_t);
+void launch_moe_gather_bwd(const void*, const int*, int, void*, int, int, cudaStream_t);
+void launch_moe_combine(const void*, const int*, const void*, int, const void*, const void*, const void*, void*, int, int, cudaStream_t);
+void launch_moe_combine_bwd(const void*, const void*, const int*, const int*, const void*, int, void*, void*, const void*, const void*, void*, void*, int, int, int,
+                            cudaStream_t);
+int launch_gemm_grouped_swiglu(const void*, const void*, void*, void*, int, int, int, int64_t, int64_t, const int*, const int*, int, int*, cudaStream_t);
 void launch_rope(void*, const int64_t*, const float*, const float*, int64_t, int, int, int, int64_t,
                  int64_t, float, cudaStream_t);
 int launch_loss_fwd(int, const void*, const void*, const uint8_t*, const int64_t*, float*, float*, int*,
@@ -147,6 +159,13 @@ void rmsnorm_bwd(const Tensor& dy, const c10::optional<Tensor>& dy2, const Tenso
                             dw.has_value() ? dw->data_ptr() : nullptr, (int)rows, (int)H, accumulate_dw ? 1 : 0, centred ? 1 : 0, cur_stream());
 }
 
+// rows_used (optional int32[1] on the device): rows past it are left alone.
+const int* used_rows(const c10::optional<Tensor>& rows_used) {
+  if (!rows_used.has_value()) return nullptr;
+  TORCH_CHECK(rows_used->is_cuda() && rows_used->scalar_type() == at::kInt && rows_used->numel() >= 1);
+  return rows_used->data_ptr<int>();
+}
+
 Tensor swiglu_fwd(const Tensor& gate_up) {
   check_rows(gate_up, "gate_up");
   TORCH_CHECK(gate_up.is_contiguous() && gate_up.size(1) % 16 == 0);
@@ -154,19 +173,146 @@ Tensor swiglu_fwd(const Tensor& gate_up) {
   const int I = (int)(gate_up.size(1) / 2);
   c10::cuda::CUDAGuard guard(gate_up.device());
   Tensor h = at::empty({rows, I}, gate_up.options());
-  sb200::launch_swiglu_fwd(gate_up.data_ptr(), h.data_ptr(), rows, I, cur_stream());
+  sb200::launch_swiglu_fwd(gate_up.data_ptr(), h.data_ptr(), rows, I, nullptr, cur_stream());
   return h;
 }
 
-Tensor swiglu_bwd(const Tensor& dh, const Tensor& gate_up) {
+Tensor swiglu_bwd_rows(const Tensor& dh, const Tensor& gate_up, const c10::optional<Tensor>& rows_used) {
   check_rows(gate_up, "gate_up");
   check_rows(dh, "dh");
   TORCH_CHECK(gate_up.is_contiguous() && dh.is_contiguous() && dh.size(1) * 2 == gate_up.size(1));
   c10::cuda::CUDAGuard guard(gate_up.device());
   Tensor out = at::empty_like(gate_up);
   sb200::launch_swiglu_bwd(dh.data_ptr(), gate_up.data_ptr(), out.data_ptr(), gate_up.size(0),
-                           (int)dh.size(1), cur_stream());
+                           (int)dh.size(1), used_rows(rows_used), cur_stream());
   return out;
+}
+Tensor swiglu_bwd(const Tensor& dh, const Tensor& gate_up) { return swiglu_bwd_rows(dh, gate_up, c10::nullopt); }
+
+// [q | k | v] gradients (2-D rows, k and v optional) side by side, rotated back where marked (q always, k with rotate_k).
+Tensor rope_merge(const Tensor& q, const c10::optional<Tensor>& k, const c10::optional<Tensor>& v, bool rotate_k, const Tensor& positions, const Tensor& cos_t,
+                  const Tensor& sin_t, int64_t hd, int64_t rot, double sign) {
+  TORCH_CHECK(rot % 16 == 0 && rot <= hd && hd % 8 == 0, "rope_merge: rot a multiple of 16, hd of 8");
+  const Tensor* parts[3] = {&q, k.has_value() ? &*k : nullptr, v.has_value() ? &*v : nullptr};
+  const void* src[3] = {nullptr, nullptr, nullptr};
+  int64_t stride[3] = {0, 0, 0}, width = 0;
+  int heads[3] = {0, 0, 0}, rotate[3] = {1, rotate_k ? 1 : 0, 0};
+  for (int i = 0; i < 3; ++i) {
+    if (parts[i] == nullptr) continue;
+    check_rows(*parts[i], "rope_merge input");
+    TORCH_CHECK(parts[i]->size(0) == q.size(0) && parts[i]->size(1) % hd == 0, "rope_merge: whole heads of the same rows expected");
+    src[i] = parts[i]->data_ptr();
+    stride[i] = parts[i]->stride(0);
+    heads[i] = (int)(parts[i]->size(1) / hd);
+    width += parts[i]->size(1);
+  }
+  TORCH_CHECK(positions.scalar_type() == at::kLong && positions.is_contiguous() && positions.numel() == q.size(0));
+  TORCH_CHECK(cos_t.scalar_type() == at::kFloat && sin_t.scalar_type() == at::kFloat && cos_t.is_contiguous() && sin_t.is_contiguous() && cos_t.dim() == 2 &&
+              cos_t.size(1) == rot / 2 && sin_t.sizes() == cos_t.sizes() && (reinterpret_cast<uintptr_t>(cos_t.data_ptr()) & 15) == 0 &&
+              (reinterpret_cast<uintptr_t>(sin_t.data_ptr()) & 15) == 0);
+  c10::cuda::CUDAGuard guard(q.device());
+  Tensor out = at::empty({q.size(0), width}, q.options());
+  sb200::launch_rope_merge(src, stride, heads, rotate, out.data_ptr(), width, positions.data_ptr<int64_t>(), cos_t.data_ptr<float>(), sin_t.data_ptr<float>(),
+                           cos_t.size(0), (int)q.size(0), (int)hd, (int)rot, (float)sign, cur_stream());
+  return out;
+}
+
+// ---- gated attention ---------------------------------------------------------------------------
+// out: contiguous [T, heads, hd]; gate: [T, heads, hd] view with unit inner stride (a half of each head's projection).
+void check_gate(const Tensor& out, const Tensor& gate, const char* name) {
+  TORCH_CHECK(out.is_cuda() && out.scalar_type() == at::kBFloat16 && out.dim() == 3 && out.is_contiguous() && out.size(2) % 8 == 0);
+  TORCH_CHECK(gate.is_cuda() && gate.scalar_type() == at::kBFloat16 && gate.sizes() == out.sizes() && gate.stride(2) == 1 && gate.stride(1) % 8 == 0 &&
+              gate.stride(0) % 8 == 0 && (reinterpret_cast<uintptr_t>(gate.data_ptr()) & 15) == 0, name, ": strided [T, heads, hd] with aligned rows expected");
+}
+Tensor gate_mul_fwd(const Tensor& out, const Tensor& gate) {
+  check_gate(out, gate, "gate");
+  c10::cuda::CUDAGuard guard(out.device());
+  Tensor y = at::empty_like(out);
+  sb200::launch_gate_mul_fwd(out.data_ptr(), gate.data_ptr(), y.data_ptr(), (int)out.size(0), (int)out.size(1), (int)out.size(2), gate.stride(0),
+                             (int)gate.stride(1), cur_stream());
+  return y;
+}
+Tensor gate_mul_bwd(const Tensor& dy, const Tensor& out, const Tensor& gate, Tensor dgate) {
+  check_gate(out, gate, "gate");
+  check_gate(out, dgate, "dgate");
+  TORCH_CHECK(dy.sizes() == out.sizes() && dy.is_contiguous() && dy.scalar_type() == at::kBFloat16 && dgate.stride(1) == gate.stride(1));
+  c10::cuda::CUDAGuard guard(out.device());
+  Tensor dout = at::empty_like(out);
+  sb200::launch_gate_mul_bwd(dy.data_ptr(), out.data_ptr(), gate.data_ptr(), dout.data_ptr(), dgate.data_ptr(), (int)out.size(0), (int)out.size(1),
+                             (int)out.size(2), gate.stride(0), (int)gate.stride(1), dgate.stride(0), cur_stream());
+  return dout;
+}
+
+// ---- mixture-of-experts row movement ---------------------------------------------------------------
+// expert int64[T, k] -> (seg int32[E + 1], 256-row tile prefix int32[E + 1], slot_row int32[T * k], row_slot int32[capacity]).
+std::tuple<Tensor, Tensor, Tensor, Tensor> moe_plan(const Tensor& expert, int64_t E, int64_t capacity) {
+  TORCH_CHECK(expert.is_cuda() && expert.scalar_type() == at::kLong && expert.is_contiguous() && expert.numel() > 0);
+  TORCH_CHECK(E >= 1 && E <= 1024 && capacity >= (expert.numel() + 127 * E + 127) / 128 * 128, "moe_plan: at most 1024 experts and room for every padded segment");
+  c10::cuda::CUDAGuard guard(expert.device());
+  auto opt = expert.options().dtype(at::kInt);
+  const int n = (int)expert.numel();
+  Tensor hist = at::empty({sb200::moe_plan_blocks(n), E}, opt), seg = at::empty({E + 1}, opt), tiles = at::empty({E + 1}, opt);
+  Tensor slot_row = at::empty({n}, opt), row_slot = at::empty({capacity}, opt);
+  const int rc = sb200::launch_moe_plan(expert.data_ptr<int64_t>(), n, (int)E, (int)capacity, hist.data_ptr<int>(), seg.data_ptr<int>(), tiles.data_ptr<int>(),
+                                        slot_row.data_ptr<int>(), row_slot.data_ptr<int>(), cur_stream());
+  TORCH_CHECK(rc == 0, "moe_plan launch failed (", rc, ")");
+  return {seg, tiles, slot_row, row_slot};
+}
+const int* int_ptr(const Tensor& t, int64_t least, const char* name) {
+  TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kInt && t.is_contiguous() && t.numel() >= least, name, ": int32 CUDA tensor expected");
+  return t.data_ptr<int>();
+}
+// the used row count is the last entry of seg
+const int* rows_used_of(const Tensor& seg) { return int_ptr(seg, 2, "seg") + (seg.numel() - 1); }
+
+Tensor moe_gather(const Tensor& x, const Tensor& row_slot, const Tensor& seg, int64_t k) {
+  check_rows(x, "x");
+  const int64_t cap = row_slot.numel(), H = x.size(1);
+  TORCH_CHECK(H % 8 == 0);
+  c10::cuda::CUDAGuard guard(x.device());
+  Tensor out = at::empty({cap, H}, x.options());
+  sb200::launch_moe_gather(x.data_ptr(), x.stride(0), int_ptr(row_slot, 1, "row_slot"), rows_used_of(seg), (int)k, out.data_ptr(), (int)cap, (int)H, cur_stream());
+  return out;
+}
+Tensor moe_gather_bwd(const Tensor& d_pad, const Tensor& slot_row, int64_t k) {
+  check_rows(d_pad, "d_pad");
+  TORCH_CHECK(d_pad.is_contiguous() && d_pad.size(1) % 8 == 0 && slot_row.numel() % k == 0);
+  const int64_t T = slot_row.numel() / k, H = d_pad.size(1);
+  c10::cuda::CUDAGuard guard(d_pad.device());
+  Tensor dx = at::empty({T, H}, d_pad.options());
+  sb200::launch_moe_gather_bwd(d_pad.data_ptr(), int_ptr(slot_row, 1, "slot_row"), (int)k, dx.data_ptr(), (int)T, (int)H, cur_stream());
+  return dx;
+}
+const void* token_rows(const c10::optional<Tensor>& t, int64_t T, int64_t W, const char* name) {
+  if (!t.has_value()) return nullptr;
+  TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kBFloat16 && t->is_contiguous() && t->numel() == T * W, name, ": contiguous bf16 [T, .] expected");
+  return t->data_ptr();
+}
+Tensor moe_combine(const Tensor& y_pad, const Tensor& slot_row, const Tensor& p, const c10::optional<Tensor>& shared, const c10::optional<Tensor>& gate,
+                   const c10::optional<Tensor>& residual) {
+  check_rows(y_pad, "y_pad");
+  TORCH_CHECK(y_pad.is_contiguous() && p.dim() == 2 && p.is_contiguous() && p.scalar_type() == at::kBFloat16 && p.numel() == slot_row.numel());
+  TORCH_CHECK(shared.has_value() == gate.has_value(), "moe_combine: the shared expert comes with its gate");
+  const int64_t T = p.size(0), k = p.size(1), H = y_pad.size(1);
+  c10::cuda::CUDAGuard guard(y_pad.device());
+  Tensor out = at::empty({T, H}, y_pad.options());
+  sb200::launch_moe_combine(y_pad.data_ptr(), int_ptr(slot_row, 1, "slot_row"), p.data_ptr(), (int)k, token_rows(shared, T, H, "shared"), token_rows(gate, T, 1, "gate"),
+                            token_rows(residual, T, H, "residual"), out.data_ptr(), (int)T, (int)H, cur_stream());
+  return out;
+}
+// -> (dy_pad, dp, dshared, dgate); the last two empty without a shared expert
+std::tuple<Tensor, Tensor, Tensor, Tensor> moe_combine_bwd(const Tensor& dout, const Tensor& y_pad, const Tensor& row_slot, const Tensor& seg, const Tensor& p,
+                                                           const c10::optional<Tensor>& shared, const c10::optional<Tensor>& gate) {
+  check_rows(y_pad, "y_pad");
+  const int64_t T = p.size(0), k = p.size(1), H = y_pad.size(1), cap = row_slot.numel();
+  TORCH_CHECK(y_pad.is_contiguous() && y_pad.size(0) == cap && p.is_contiguous() && p.scalar_type() == at::kBFloat16);
+  c10::cuda::CUDAGuard guard(y_pad.device());
+  Tensor dy_pad = at::empty_like(y_pad), dp = at::empty_like(p);
+  Tensor dshared = at::empty({shared.has_value() ? T : 0, H}, y_pad.options()), dgate = at::empty({shared.has_value() ? T : 0, 1}, y_pad.options());
+  sb200::launch_moe_combine_bwd(token_rows(dout, T, H, "dout"), y_pad.data_ptr(), int_ptr(row_slot, 1, "row_slot"), rows_used_of(seg), p.data_ptr(), (int)k,
+                                dy_pad.data_ptr(), dp.data_ptr(), token_rows(shared, T, H, "shared"), token_rows(gate, T, 1, "gate"), dshared.data_ptr(),
+                                dgate.data_ptr(), (int)T, (int)cap, (int)H, cur_stream());
+  return {dy_pad, dp, dshared, dgate};
 }
 
 // x: [tokens, >= heads*hd] view (row stride arbitrary); rotates the first `heads` heads in place.
@@ -244,6 +390,21 @@ void gemm_grouped_rows(const Tensor& x, const Tensor& w, Tensor out, bool transp
                                             out.stride(0), 0, 1, transposed ? 1 : 0, seg.data_ptr<int>(), mts.data_ptr<int>(), (int)E,
                                             status.data_ptr<int>(), cur_stream());
   TORCH_CHECK(rc == 0, "gemm_grouped_rows launch failed (", rc, ")");
+}
+
+// (gate_up [R, 2 I], h [R, I] = silu(gate) * up) for stacked [gate; up] experts w: [E, 2 I, K].
+std::tuple<Tensor, Tensor> gemm_grouped_swiglu(const Tensor& x, const Tensor& w, const Tensor& seg, const Tensor& mts, Tensor status) {
+  check_rows(x, "x");
+  TORCH_CHECK(w.is_cuda() && w.scalar_type() == at::kBFloat16 && w.dim() == 3 && w.is_contiguous(), "w must be a contiguous bf16 [E, 2 I, K] stack");
+  const int64_t E = w.size(0), R = x.size(0), K = x.size(1), I = w.size(1) / 2;
+  TORCH_CHECK(w.size(2) == K && K % 128 == 0 && w.size(1) == 2 * I && I % 128 == 0 && R % 128 == 0, "gemm_grouped_swiglu: shape mismatch");
+  TORCH_CHECK(seg.is_cuda() && seg.scalar_type() == at::kInt && seg.numel() == E + 1 && mts.scalar_type() == at::kInt && mts.numel() == E + 1);
+  c10::cuda::CUDAGuard guard(x.device());
+  Tensor gate_up = at::empty({R, 2 * I}, x.options()), h = at::empty({R, I}, x.options());
+  const int rc = sb200::launch_gemm_grouped_swiglu(x.data_ptr(), w.data_ptr(), gate_up.data_ptr(), h.data_ptr(), (int)R, (int)I, (int)K, x.stride(0), K,
+                                                   seg.data_ptr<int>(), mts.data_ptr<int>(), (int)E, status.data_ptr<int>(), cur_stream());
+  TORCH_CHECK(rc == 0, "gemm_grouped_swiglu launch failed (", rc, ")");
+  return {gate_up, h};
 }
 
 // dw[e] (=, +=) dy[seg_e, :]^T . x[seg_e, :]  (dw: [E, M, N], dy: [R, M], x: [R, N]); an expert without rows gets zeros (store) / is left alone (accumulate).
@@ -930,6 +1091,16 @@ TORCH_LIBRARY(sb200, m) {
   m.def("rmsnorm_bwd", &rmsnorm_bwd);
   m.def("swiglu_fwd", &swiglu_fwd);
   m.def("swiglu_bwd", &swiglu_bwd);
+  m.def("swiglu_bwd_rows", &swiglu_bwd_rows);
+  m.def("rope_merge", &rope_merge);
+  m.def("gate_mul_fwd", &gate_mul_fwd);
+  m.def("gate_mul_bwd", &gate_mul_bwd);
+  m.def("moe_plan", &moe_plan);
+  m.def("moe_gather", &moe_gather);
+  m.def("moe_gather_bwd", &moe_gather_bwd);
+  m.def("moe_combine", &moe_combine);
+  m.def("moe_combine_bwd", &moe_combine_bwd);
+  m.def("gemm_grouped_swiglu", &gemm_grouped_swiglu);
   m.def("rope_", &rope_);
   m.def("loss_fwd", &loss_fwd);
   m.def("loss_bwd", &loss_bwd);

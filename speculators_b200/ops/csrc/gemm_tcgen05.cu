@@ -221,6 +221,10 @@ __device__ __forceinline__ TileInfo decode_tile(const Params& p, int tile, int t
     t.a_m = m0; t.a_k0 = 0; t.num_kb = num_kb; t.c_row0 = m0; t.row_end = s1;
     t.b_n = (B_MN ? 0 : e * p.N) + t.n0 + rank * 128;
     t.b_k0 = B_MN ? e * p.K : 0;
+    if (p.epilogue == kSwiGLU) {
+      t.n0 = t.tile_n * 128;
+      t.b_n = e * p.N + t.n0 + rank * (p.N >> 1);
+    }
   } else {
     const int per = tiles_m * tiles_n, e = tile / per, local = tile % per;
     const int m0 = (local % tiles_m) * 256 + rank * 128, s0 = p.grp.seg[e];
@@ -1219,7 +1223,7 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
            Grouping{kGroupNone, 0, nullptr, nullptr}, Scatter{}, (__nv_bfloat16*)gated_h, gated_ldh, 0, bs.alpha, bs.beta, bs.batch,
            bs.c_stride, bs.r_stride, 0};
   if (epilogue == kSwiGLU) {
-    if (!pairs || a_mn || b_mn || grp != nullptr || stats_targets != nullptr || scatter != nullptr || gated_h == nullptr || (N & 255) || (ldc & 7) ||
+    if (!pairs || a_mn || b_mn || (grp != nullptr && grp->mode != kGroupRows) || stats_targets != nullptr || scatter != nullptr || gated_h == nullptr || (N & 255) || (ldc & 7) ||
         (gated_ldh & 7) || (reinterpret_cast<uintptr_t>(c) & 15) || (reinterpret_cast<uintptr_t>(gated_h) & 15))
       return -8;
   }
@@ -1366,6 +1370,14 @@ int launch_gemm_grouped(const void* a, const void* b, void* c, int M, int N, int
   const int a_mn = mode == tc::kGroupK ? 1 : 0;
   return launch_gemm_impl(a, b, c, nullptr, M, N, K, lda, ldb, ldc, 0, epilogue, a_mn, mode == tc::kGroupK ? 1 : b_mn, status, 3, nullptr, 0, 0, 0,
                           nullptr, &grp, stream);
+}
+
+// mode 1 with stacked [gate; up] experts [E, 2 I, K]: gate_up[R, 2 I] and h[R, I] = silu(gate) * up.
+int launch_gemm_grouped_swiglu(const void* a, const void* b, void* gate_up, void* h, int M, int I, int K, int64_t lda, int64_t ldb, const int* seg,
+                               const int* mtile_start, int num_groups, int* status, cudaStream_t stream) {
+  const tc::Grouping grp{tc::kGroupRows, num_groups, seg, mtile_start};
+  return launch_gemm_impl(a, b, gate_up, nullptr, M, 2 * I, K, lda, ldb, 2 * I, 0, tc::kSwiGLU, 0, 0, status, 3, nullptr, 0, 0, 0, nullptr, &grp, stream,
+                          nullptr, h, I);
 }
 
 // ---- lm_head product fused with the row loss (KL divergence / cross-entropy on the argmax) -----
