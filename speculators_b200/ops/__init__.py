@@ -96,6 +96,7 @@ _WAIT_CODES = {
     31: "attention forward producer", 32: "attention forward MMA issuer", 33: "attention forward softmax",
     41: "attention dQ producer", 42: "attention dQ MMA issuer", 43: "attention dQ element-wise warps",
     44: "attention dK/dV producer", 45: "attention dK/dV MMA issuer", 46: "attention dK/dV element-wise warps",
+    51: "attention (head dim 256) producer", 52: "attention (head dim 256) MMA issuer", 53: "attention (head dim 256) element-wise warps",
 }
 
 

@@ -1,12 +1,12 @@
 """CUDA path of ``masked_attention``: autograd wrapper around the sm_100a kernels
 (head dims 64, 128 and 256).  Other head dims use the dense formulation.
 
-Forward and backward at head dim 128 run on the tcgen05 tensor cores
-(``csrc/attention_tc.cu``, ``csrc/attention_bwd_tc.cu``: TMA tiles, TMEM accumulators,
-probability tiles handed to the next product through TMEM); ``FWD_IMPL`` / ``BWD_IMPL`` =
-``"mma"`` (or ``SB200_ATTN_FWD=mma`` / ``SB200_ATTN_BWD=mma``) select the ``mma.sync``
-kernels of ``csrc/attention.cu``, which also serve head dims 64 and 256 (256: the gated
-full-attention heads of Qwen3-Next style MTP layers)."""
+Forward and backward at head dim 128, and at 256 without extra keys (the gated full-attention
+heads of Qwen3-Next style MTP layers), run on the tcgen05 tensor cores
+(``csrc/attention_tc.cu``, ``csrc/attention_bwd_tc.cu``, ``csrc/attention_wide_tc.cu``: TMA tiles,
+TMEM accumulators, probability tiles handed to the next product through TMEM); ``FWD_IMPL`` /
+``BWD_IMPL`` = ``"mma"`` (or ``SB200_ATTN_FWD=mma`` / ``SB200_ATTN_BWD=mma``) select the
+``mma.sync`` kernels of ``csrc/attention.cu``, which also serve head dim 64 and 256 with extra keys."""
 
 from __future__ import annotations
 
@@ -32,14 +32,20 @@ def _rows_ok(t: torch.Tensor) -> torch.Tensor:
     return t.contiguous()
 
 
+def _tensor_core_shape(q: torch.Tensor, ext_idx: torch.Tensor | None) -> bool:
+    """Whether the tcgen05 kernels take the call: head dim 128, or 256 (their own kernels, whose shared memory is filled by
+    128 resident rows and leaves none to stage individually addressed extra keys in)."""
+    return q.shape[2] == 128 or (q.shape[2] == 256 and ext_idx is None)
+
+
 class _MaskedAttentionFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, lo, hi, k_ext, v_ext, ext_idx, scale, ext_block, ext_causal):
         q, k, v = _rows_ok(q), _rows_ok(k), _rows_ok(v)
         if ext_idx is not None:
             k_ext, v_ext = _rows_ok(k_ext), _rows_ok(v_ext)
-        tc_fwd = FWD_IMPL == "tc" and q.shape[2] == 128
-        tc_bwd = BWD_IMPL == "tc" and q.shape[2] == 128
+        tc_shape = _tensor_core_shape(q, ext_idx)
+        tc_fwd, tc_bwd = FWD_IMPL == "tc" and tc_shape, BWD_IMPL == "tc" and tc_shape
         # block-structured extras run as one more key tile on the tensor cores; both directions must take
         # that route (or neither), since the forward's statistics feed the backward either way
         block = int(ext_block) if (ext_idx is not None and tc_fwd and tc_bwd and BLOCK_EXTRAS and ext_block and 128 % int(ext_block) == 0
@@ -58,7 +64,7 @@ class _MaskedAttentionFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout):
         q, k, v, out, lse2, lo, hi, k_ext, v_ext, ext_idx = ctx.saved_tensors
-        if BWD_IMPL == "tc" and q.shape[2] == 128:
+        if BWD_IMPL == "tc" and _tensor_core_shape(q, ext_idx):
             from speculators_b200.ops import gemm_status
 
             impl, status = 1, gemm_status(q.device)

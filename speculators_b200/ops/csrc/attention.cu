@@ -804,13 +804,7 @@ static int launch_bwd_t(const AttnParams& p, int* tile_qmin, int* tile_qmax, cud
   launch_pdl(kv_tile_range_kernel, n_kv_tiles, 256, 0, stream, p.lo, p.hi, p.Tq, p.Tc, tile_qmin, tile_qmax);
   dim3 grid_kv(p.nh, n_kv_tiles, HD / kDkvCols<HD>);  // x = head: all heads of the heaviest tile are dispatched first; z = output column part
   launch_pdl(attn_bwd_dkv_kernel<HD>, grid_kv, kAttnThreads, bwd_smem<HD>(), stream, p);
-  if (p.dkv_part != nullptr) {
-    const int64_t n = (int64_t)p.Tc * p.nkv * HD;
-    const int64_t blocks = (2 * (n >> 3) + 255) / 256;
-    count_launch(1);
-    launch_pdl(dkv_reduce_kernel, (int)(blocks < 8 * kNumSM ? blocks : 8 * kNumSM), 256, 0, stream, p.dkv_part, p.nh / p.nkv, n, p.dk, p.dv);
-  }
-  return 0;
+  return p.dkv_part != nullptr ? launch_dkv_reduce(p, HD, stream) : 0;
 }
 
 int launch_kv_tile_range(const AttnParams& p, int* tile_qmin, int* tile_qmax, cudaStream_t stream) {
@@ -820,8 +814,8 @@ int launch_kv_tile_range(const AttnParams& p, int* tile_qmin, int* tile_qmax, cu
   return 0;
 }
 
-int launch_dkv_reduce(const AttnParams& p, cudaStream_t stream) {
-  const int64_t n = (int64_t)p.Tc * p.nkv * 128;
+int launch_dkv_reduce(const AttnParams& p, int hd, cudaStream_t stream) {
+  const int64_t n = (int64_t)p.Tc * p.nkv * hd;
   const int64_t blocks = (2 * (n >> 3) + 255) / 256;
   count_launch(1);
   launch_pdl(dkv_reduce_kernel, (int)(blocks < 8 * kNumSM ? blocks : 8 * kNumSM), 256, 0, stream, p.dkv_part, p.nh / p.nkv, n, p.dk, p.dv);

@@ -86,27 +86,29 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
 }
 
 // ---------------------------------------------------------------------------------- delta
-// delta[h, row] = sum_c dO[row, h, c] * O[row, h, c]: 16 lanes per (row, head), 16 bytes per lane.
+// delta[h, row] = sum_c dO[row, h, c] * O[row, h, c]: W / 8 lanes per (row, head), 16 bytes per lane.
+template <int W>
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ out, float* __restrict__ delta, int Tq, int nh,
                   int64_t do_rs, int64_t o_rs) {
   pdl_begin();
-  const int lane = threadIdx.x & 31, sub = lane >> 4, l16 = lane & 15;
+  constexpr int L = W / 8, PER_WARP = 32 / L;
+  const int lane = threadIdx.x & 31, sub = lane / L, part = lane % L;
   const int64_t n = (int64_t)Tq * nh;
-  for (int64_t base = ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * 2; base < n; base += (int64_t)gridDim.x * 16) {
+  for (int64_t base = ((int64_t)blockIdx.x * 8 + (threadIdx.x >> 5)) * PER_WARP; base < n; base += (int64_t)gridDim.x * 8 * PER_WARP) {
     const int64_t idx = base + sub;
     float acc = 0.f;
     if (idx < n) {
       const int row = (int)(idx / nh), h = (int)(idx % nh);
       float a[8], b[8];
-      unpack8(ld8(dout + (int64_t)row * do_rs + h * HD + l16 * 8), a);
-      unpack8(ld8(out + (int64_t)row * o_rs + h * HD + l16 * 8), b);
+      unpack8(ld8(dout + (int64_t)row * do_rs + h * W + part * 8), a);
+      unpack8(ld8(out + (int64_t)row * o_rs + h * W + part * 8), b);
 #pragma unroll
       for (int i = 0; i < 8; ++i) acc = fmaf(a[i], b[i], acc);
     }
 #pragma unroll
-    for (int o = 8; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if (l16 == 0 && idx < n) delta[(int64_t)(idx % nh) * Tq + idx / nh] = acc;
+    for (int o = L / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (part == 0 && idx < n) delta[(int64_t)(idx % nh) * Tq + idx / nh] = acc;
   }
 }
 
@@ -755,6 +757,14 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 
 }  // namespace abtc
 
+void launch_attn_delta(const AttnParams& p, int hd, cudaStream_t stream) {
+  const int64_t blocks = ((int64_t)p.Tq * p.nh * (hd / 8) + 255) / 256;
+  const int grid = (int)(blocks < 16 * kNumSM ? blocks : 16 * kNumSM);
+  count_launch(1);
+  if (hd == 256) launch_pdl(abtc::attn_delta_kernel<256>, grid, 256, 0, stream, p.dout, p.out, p.delta, p.Tq, p.nh, p.do_rs, p.o_rs);
+  else launch_pdl(abtc::attn_delta_kernel<128>, grid, 256, 0, stream, p.dout, p.out, p.delta, p.Tq, p.nh, p.do_rs, p.o_rs);
+}
+
 // head_dim 128; tile_qmin / tile_qmax: scratch of one int per 64-key tile, fully written here.
 int launch_attn_bwd_tc(const AttnParams& p, int* tile_qmin, int* tile_qmax, int* status, cudaStream_t stream) {
   using namespace abtc;
@@ -782,12 +792,8 @@ int launch_attn_bwd_tc(const AttnParams& p, int* tile_qmin, int* tile_qmax, int*
     if (cudaFuncSetAttribute(attn_bwd_dkv_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess) return -2;
     configured.mark();
   }
-  count_launch(3);
-  {
-    const int64_t pairs = (int64_t)p.Tq * p.nh;
-    const int64_t blocks = (pairs + 15) / 16;
-    launch_pdl(attn_delta_kernel, (int)(blocks < 16 * kNumSM ? blocks : 16 * kNumSM), 256, 0, stream, p.dout, p.out, p.delta, p.Tq, p.nh, p.do_rs, p.o_rs);
-  }
+  count_launch(2);
+  launch_attn_delta(p, HD, stream);
   dim3 grid_q(p.nh, (p.Tq + BM - 1) / BM);
   launch_pdl(attn_bwd_dq_tc_kernel, grid_q, THREADS, SMEM_BYTES, stream, map_q, map_do, map_k, map_v, map_ke, map_ve, p, status);
   rc = launch_kv_tile_range(p, tile_qmin, tile_qmax, stream);
@@ -800,7 +806,7 @@ int launch_attn_bwd_tc(const AttnParams& p, int* tile_qmin, int* tile_qmax, int*
     launch_pdl(attn_bwd_dkv_tc_kernel, grid_ext, THREADS, SMEM_BYTES, stream, map_q, map_do, map_ke, map_ve, p, 0, 1, status);
   }
   if (p.dkv_part != nullptr) {
-    rc = launch_dkv_reduce(p, stream);
+    rc = launch_dkv_reduce(p, HD, stream);
     if (rc) return rc;
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -3;

@@ -51,8 +51,12 @@ constexpr int kAttnKeyTile = 64;
 // tcgen05 backward (dQ kernel, dK/dV kernel), head_dim 128; same scratch and status conventions.
 int launch_attn_bwd_tc(const AttnParams& p, int* tile_qmin, int* tile_qmax, int* status, cudaStream_t stream);
 // Pieces of the backward shared by both implementations: per-64-key-tile query row ranges,
-// and the head-ordered sum of the fp32 dK / dV partials of grouped queries (head_dim 128).
+// the head-ordered sum of the fp32 dK / dV partials of grouped queries, and delta = rowsum(dO * O) (head dims 128, 256).
 int launch_kv_tile_range(const AttnParams& p, int* tile_qmin, int* tile_qmax, cudaStream_t stream);
-int launch_dkv_reduce(const AttnParams& p, cudaStream_t stream);
+int launch_dkv_reduce(const AttnParams& p, int hd, cudaStream_t stream);
+void launch_attn_delta(const AttnParams& p, int hd, cudaStream_t stream);
+// The same two at head dim 256, without extra keys.
+int launch_attn_fwd_wide_tc(const AttnParams& p, int* status, cudaStream_t stream);
+int launch_attn_bwd_wide_tc(const AttnParams& p, int* tile_qmin, int* tile_qmax, int* status, cudaStream_t stream);
 
 }  // namespace sb200

@@ -196,3 +196,9 @@ def test_anchored_blocks_run_their_block_keys_as_a_tile(window, non_causal, n_an
         tol = 3e-2 * float(b.grad.abs().max()) + 2e-2
         assert float((a.float() - b.grad).abs().max()) < tol, (name, float((a.float() - b.grad).abs().max()), tol)
         assert float((a.float() - c.float()).abs().max()) < tol, (name, "vs per-row path")
+
+
+@pytest.mark.parametrize("T,nh,nkv,window,pattern", [(1, 2, 2, None, "single"), (65, 3, 3, None, "single"), (700, 6, 2, 100, "multi_pad"), (449, 2, 1, None, "multi_pad")])
+def test_head_dim_256_tensor_core_kernels(T, nh, nkv, window, pattern):
+    """One row, ungrouped heads, windows that start and end inside a tile, documents, padding rows that see nothing."""
+    _run(T, nh, nkv, 256, step=0, window=window, pattern=pattern)
