@@ -35,15 +35,13 @@ class DFlashAttention(nn.Module):
     def forward(self, noise, target_hidden, noise_positions, all_positions, rotary: RotaryTable, spec: AttnSpec, residual=None):
         nq = noise.shape[0]
         T = target_hidden.shape[0]
-        q = self.qkv_proj.forward_parts(noise, 0, 1).view(nq, self.nh, self.hd)
+        q = self.qkv_proj.forward_parts(noise, 0, 1)
         kv = self.qkv_proj.forward_parts(torch.cat([target_hidden, noise], dim=0), 1, 3)
-        k = kv[:, : self.nkv * self.hd].reshape(T + nq, self.nkv, self.hd)
-        v = kv[:, self.nkv * self.hd :].view(T + nq, self.nkv, self.hd)
-        q = self.q_norm(q).reshape(nq, self.nh * self.hd)
-        k = self.k_norm(k).reshape(T + nq, self.nkv * self.hd)
-        q = ops.rope_(q, noise_positions, rotary.cos, rotary.sin, self.nh, self.hd, self.rot).view(nq, self.nh, self.hd)
-        k = ops.rope_(k, all_positions, rotary.cos, rotary.sin, self.nkv, self.hd, self.rot).view(T + nq, self.nkv, self.hd)
-        out = ops.masked_attention(q, k[:T], v[:T], spec, k[T:], v[T:], scale=self.scaling)
+        (q,) = ops.norm_rope_heads(q, self.q_norm.weight, None, self.q_norm.variance_epsilon, noise_positions, rotary.cos, rotary.sin,
+                                   (self.nh, 0, 0), self.hd, self.rot)
+        k_ctx, k_ext, v_ctx, v_ext = ops.norm_rope_heads(kv, self.k_norm.weight, None, self.k_norm.variance_epsilon, all_positions, rotary.cos,
+                                                         rotary.sin, (self.nkv, 0, self.nkv), self.hd, self.rot, split=T)
+        out = ops.masked_attention(q, k_ctx, v_ctx, spec, k_ext, v_ext, scale=self.scaling)
         return self.o_proj(out.reshape(nq, self.nh * self.hd), residual=residual)
 
 

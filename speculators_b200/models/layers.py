@@ -233,23 +233,19 @@ class Attention(nn.Module):
         self.q_norm = RMSNorm(self.hd, config.rms_norm_eps) if use_qk_norm else None
         self.k_norm = RMSNorm(self.hd, config.rms_norm_eps) if use_qk_norm else None
 
-    def project_qkv(self, x: torch.Tensor, positions: torch.Tensor, rotary: RotaryTable):
+    def project_qkv(self, x: torch.Tensor, positions: torch.Tensor, rotary: RotaryTable, split: int | None = None):
         """x [T, in] -> (q [T, nh, hd], k [T, nkv, hd], v [T, nkv, hd]) with per-head
-        norms (if any) and rotary embedding applied.  The three results are views
-        of one fused projection buffer."""
+        norms (if any) and rotary embedding applied; with ``split`` k and v come as
+        two tensors each, the rows below it and the rows from it on."""
         T = x.shape[0]
         nq, nk = self.nh * self.hd, self.nkv * self.hd
         qkv = self.qkv_proj(x)
         if self.q_norm is not None:
-            q = self.q_norm(qkv[:, :nq].reshape(T, self.nh, self.hd))
-            k = self.k_norm(qkv[:, nq : nq + nk].reshape(T, self.nkv, self.hd))
-            qk = torch.cat([q.reshape(T, nq), k.reshape(T, nk)], dim=-1)
-            qk = ops.rope_(qk, positions, rotary.cos, rotary.sin, self.nh + self.nkv, self.hd, self.rot)
-            q, k = qk[:, :nq], qk[:, nq:]
-            v = qkv[:, nq + nk :]
-        else:
-            q, k, v = ops.rope_split(qkv, positions, rotary.cos, rotary.sin, self.nh + self.nkv, self.hd, self.rot, nq, nk)
-        return q.view(T, self.nh, self.hd), k.view(T, self.nkv, self.hd), v.view(T, self.nkv, self.hd)
+            return ops.norm_rope_heads(qkv, self.q_norm.weight, self.k_norm.weight, self.q_norm.variance_epsilon, positions, rotary.cos,
+                                       rotary.sin, (self.nh, self.nkv, self.nkv), self.hd, self.rot, split)
+        q, k, v = ops.rope_split(qkv, positions, rotary.cos, rotary.sin, self.nh + self.nkv, self.hd, self.rot, nq, nk)
+        q, k, v = q.view(T, self.nh, self.hd), k.view(T, self.nkv, self.hd), v.view(T, self.nkv, self.hd)
+        return (q, k, v) if split is None else (q, k[:split], k[split:], v[:split], v[split:])
 
     def forward(self, x, positions, rotary, spec: AttnSpec, past: list | None = None, ctx_len: int | None = None,
                 residual: torch.Tensor | None = None) -> torch.Tensor:
@@ -261,10 +257,12 @@ class Attention(nn.Module):
         ``ctx_len`` (P-EAGLE): the first ``ctx_len`` rows of this pass are the
         interval-addressed context, the remaining rows are the extra keys."""
         T = x.shape[0]
-        q, k, v = self.project_qkv(x, positions, rotary)
         if ctx_len is not None and ctx_len < T:
-            out = ops.masked_attention(q, k[:ctx_len], v[:ctx_len], spec, k[ctx_len:], v[ctx_len:], scale=self.scaling)
-        elif past is None:
+            q, k_ctx, k_ext, v_ctx, v_ext = self.project_qkv(x, positions, rotary, split=ctx_len)
+            out = ops.masked_attention(q, k_ctx, v_ctx, spec, k_ext, v_ext, scale=self.scaling)
+            return self.o_proj(out.reshape(T, self.nh * self.hd), residual=residual)
+        q, k, v = self.project_qkv(x, positions, rotary)
+        if past is None:
             out = ops.masked_attention(q, k, v, spec, scale=self.scaling)
         else:
             past.append((k, v))

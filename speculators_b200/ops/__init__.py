@@ -31,6 +31,7 @@ __all__ = [
     "fused_row_loss",
     "gated",
     "check_gemm_status",
+    "clear_fresh_grad",
     "gemm_status",
     "GroupPlan",
     "grouped_linear",
@@ -44,6 +45,7 @@ __all__ = [
     "matmul_tn",
     "masked_attention_reference",
     "native",
+    "norm_rope_heads",
     "rms_norm",
     "rms_norm_fork",
     "rope_",
@@ -288,20 +290,14 @@ def _linear_backward(x2, weight, rows, dy, need_dx: bool, need_dw: bool):
     if need_dw:
         flat = getattr(weight, "_flat_grad", None)
         if flat is not None:
-            target = flat if r0 is None else flat[r0:r1]
-            fresh = getattr(weight, "_grad_fresh", False)
-            if fresh:
-                # first gradient of this weight since the engine's zero_grad, which left
-                # the buffer uncleared: store instead of accumulate
-                weight._grad_fresh = False
-                if r0 is not None:
-                    flat.zero_()
+            # the first gradient of these rows since the engine's zero_grad, which left the buffer uncleared, is stored
+            target, accumulate = _param_grad_target(weight)[:2] if r0 is None else _row_grad_target(weight, r0, r1)
             if own and _gemm_operand_ok(target):
-                _wgrad_gemm(dy2, x2, target, accumulate=not fresh or r0 is not None)
-            elif fresh and r0 is None:
-                torch.mm(dy2.t(), x2, out=flat)
-            else:
+                _wgrad_gemm(dy2, x2, target, accumulate=accumulate)
+            elif accumulate:
                 target.addmm_(dy2.t(), x2)
+            else:
+                torch.mm(dy2.t(), x2, out=target)
         elif r0 is None:
             dw = _wgrad_gemm(dy2, x2, None, accumulate=False) if own else dy2.t() @ x2
         else:
@@ -368,9 +364,40 @@ def _param_grad_target(weight: torch.Tensor) -> tuple[torch.Tensor, bool, bool]:
     flat = getattr(weight, "_flat_grad", None)
     if flat is None:
         return torch.empty_like(weight), False, False
-    fresh = getattr(weight, "_grad_fresh", False)
-    weight._grad_fresh = False
+    fresh = getattr(weight, "_grad_fresh", False) is True
+    if fresh:
+        weight._grad_fresh = False
+    else:
+        clear_fresh_grad(weight)
     return flat, not fresh, True
+
+
+def clear_fresh_grad(p: torch.Tensor) -> None:
+    """Zero what no gradient has been stored into since the engine's ``zero_grad``: all of the flat view
+    (``_grad_fresh`` is ``True``) or the row intervals that ``_row_grad_target`` has left."""
+    fresh = getattr(p, "_grad_fresh", False)
+    if fresh is False:
+        return
+    p._grad_fresh = False
+    for r0, r1 in [(0, p.shape[0])] if fresh is True else fresh:
+        p._flat_grad[r0:r1].zero_()
+
+
+def _row_grad_target(weight: torch.Tensor, r0: int, r1: int) -> tuple[torch.Tensor, bool]:
+    """``(rows of the flat gradient view, accumulate)`` for a gradient of rows ``r0 .. r1`` alone: stored where nothing has been
+    stored since ``zero_grad``; the intervals still unwritten stay noted on the weight."""
+    fresh = getattr(weight, "_grad_fresh", False)
+    if fresh is True:
+        fresh = [(0, weight.shape[0])]
+    inside = [iv for iv in fresh or [] if iv[0] <= r0 and r1 <= iv[1]]
+    if not inside:
+        if any(a < r1 and r0 < b for a, b in fresh or []):  # partly written
+            clear_fresh_grad(weight)
+        return weight._flat_grad[r0:r1], True
+    (a, b), = inside
+    rest = [iv for iv in fresh if iv != (a, b)] + [iv for iv in ((a, r0), (r1, b)) if iv[0] < iv[1]]
+    weight._grad_fresh = rest or False
+    return weight._flat_grad[r0:r1], False
 
 
 def _norm_backward(dy, dy2, x2, weight, rstd, residual_grad, need_dx: bool, need_dw: bool, centred: bool):
@@ -605,6 +632,68 @@ class _RopeSplitFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dq, dk, dv):
         return _unrotate(dq, dk, dv, *ctx.saved_tensors, *ctx.cfg), None, None, None, None, None, None, None, None
+
+
+# --------------------------------------------------------------------------- per-head norms and rotation
+def _is_split(block: int, nb: int, split) -> bool:
+    """Queries (the first of two rotated blocks) stay whole."""
+    return split is not None and not (block == 0 and nb)
+
+
+def _head_blocks(blocks, split):
+    nb = blocks[1] is not None
+    return tuple(x for i, b in enumerate(blocks) if b is not None for x in ((b[:split], b[split:]) if _is_split(i, nb, split) else (b,)))
+
+
+class _NormRopeHeadsFn(torch.autograd.Function):
+    """Head norms and rotation of a projection ``[a heads | b heads | plain heads]``; see ``norm_rope_heads``."""
+
+    @staticmethod
+    def forward(ctx, src, w_a, w_b, positions, cos_t, sin_t, eps, heads, hd, rot, split):
+        T, (na, nb, nv) = src.shape[0], heads
+        src = src.detach()
+        out, rstd = native().heads_fwd(src, w_a, na, w_b, nb, eps, positions, cos_t, sin_t, hd, rot)
+        ctx.save_for_backward(src, w_a, w_b, rstd, positions, cos_t, sin_t)
+        ctx.cfg = (heads, hd, rot, split)
+        ctx.set_materialize_grads(False)
+        blocks = [out[:, : na * hd], out[:, na * hd :], src[:, (na + nb) * hd : (na + nb + nv) * hd]]
+        return _head_blocks([b.view(T, n, hd) if n else None for b, n in zip(blocks, heads)], split)
+
+    @staticmethod
+    def backward(ctx, *grads):
+        src, w_a, w_b, rstd, positions, cos_t, sin_t = ctx.saved_tensors
+        (na, nb, nv), hd, rot, split = ctx.cfg
+        it = iter(grads)
+        rows = []  # gradients of rows below and from the split on, for each of the three blocks
+        for block, n in enumerate((na, nb, nv)):
+            for half in range(2):
+                g = next(it) if n and half < (2 if _is_split(block, nb, split) else 1) else None
+                rows.append(_grad_rows(g, n * hd) if g is not None and g.shape[0] else None)
+        dw_a, acc_a, flat_a = _param_grad_target(w_a) if ctx.needs_input_grad[1] else (None, False, False)
+        dw_b, acc_b, flat_b = _param_grad_target(w_b) if nb and ctx.needs_input_grad[2] else (None, False, False)
+        d = native().heads_bwd(rows, src.shape[0] if split is None else split, src, rstd, w_a, na, w_b, nb, nv, dw_a, acc_a, dw_b, acc_b, positions, cos_t, sin_t, hd, rot)
+        return d, None if flat_a else dw_a, None if flat_b else dw_b, None, None, None, None, None, None, None, None
+
+
+def norm_rope_heads(src: torch.Tensor, w_a, w_b, eps: float, positions, cos_t, sin_t, heads: tuple[int, int, int], hd: int, rot: int,
+                    split: int | None = None):
+    """Per-head RMSNorm (weights ``w_a``, ``w_b``) and rotary embedding of the first ``heads[0]`` and next ``heads[1]`` heads of
+    a projection ``[T, sum(heads) * hd]``; the last ``heads[2]`` heads pass through.  Returns a ``[T, n, hd]`` tensor for every
+    block that has heads, or with ``split`` two (rows below it, rows from it on) for every block but the queries, the first of
+    two rotated ones.  One launch each way on CUDA (head
+    dims 64, 128, 256); the gradients of all results are gathered into one buffer of the projection's layout."""
+    na, nb, nv = heads
+    if (_use_native(src) and src.dtype == torch.bfloat16 and hd in (64, 128, 256) and rot % 16 == 0 and rot <= hd and src.stride(-1) == 1
+            and src.stride(0) % 8 == 0 and src.data_ptr() % 16 == 0 and positions.is_contiguous() and all(w is None or w.dtype == src.dtype for w in (w_a, w_b))):
+        return _NormRopeHeadsFn.apply(src, w_a, w_b, positions, cos_t, sin_t, eps, heads, hd, rot, split)
+    T, blocks, col = src.shape[0], [], 0
+    for n, w in ((na, w_a), (nb, w_b), (nv, None)):
+        x = src[:, col : col + n * hd].reshape(T, n, hd) if n else None
+        col += n * hd
+        if n and w is not None:
+            x = rope_(rms_norm(x, w, eps).reshape(T, n * hd), positions, cos_t, sin_t, n, hd, rot).view(T, n, hd)
+        blocks.append(x)
+    return _head_blocks(blocks, split)
 
 
 # --------------------------------------------------------------------------- gated attention

@@ -21,6 +21,11 @@ int read_bounds_norm(BoundsRecord*);
 int read_bounds_ep(BoundsRecord*);
 void launch_rmsnorm_bwd(const void*, int64_t, const void*, int64_t, const void*, int64_t, const void*, const float*, const void*, int64_t, void*, int64_t,
                         float*, void*, int, int, int, int, cudaStream_t);
+void launch_heads_fwd(const void*, int64_t, const void* const*, const int*, void*, float*, int, float, const int64_t*, const float*, const float*, int64_t, int,
+                      int, cudaStream_t);
+int heads_bwd_groups(int, int);
+void launch_heads_bwd(const void* const*, const int64_t*, const int*, const void*, int64_t, const void* const*, const float*, float* const*, void* const*,
+                      const int*, const int*, void*, int64_t, int, const int64_t*, const float*, const float*, int64_t, int, int, cudaStream_t);
 void launch_swiglu_fwd(const void*, void*, int64_t, int, const int*, cudaStream_t);
 void launch_swiglu_bwd(const void*, const void*, void*, int64_t, int, const int*, cudaStream_t);
 void launch_rope_merge(const void* const*, const int64_t*, const int*, const int*, void*, int64_t, const int64_t*, const float*, const float*, int64_t, int, int,
@@ -159,6 +164,82 @@ void rmsnorm_bwd(const Tensor& dy, const c10::optional<Tensor>& dy2, const Tenso
                             dw.has_value() ? dw->data_ptr() : nullptr, (int)rows, (int)H, accumulate_dw ? 1 : 0, centred ? 1 : 0, cur_stream());
 }
 
+void check_rotation(const Tensor& positions, const Tensor& cos_t, const Tensor& sin_t, int64_t tokens, int64_t hd, int64_t rot) {
+  TORCH_CHECK(rot % 16 == 0 && rot <= hd && hd % 8 == 0, "rotation: rot a multiple of 16, hd of 8");
+  TORCH_CHECK(positions.scalar_type() == at::kLong && positions.is_contiguous() && positions.numel() == tokens);
+  TORCH_CHECK(cos_t.scalar_type() == at::kFloat && sin_t.scalar_type() == at::kFloat && cos_t.is_contiguous() && sin_t.is_contiguous() && cos_t.dim() == 2 &&
+              cos_t.size(1) == rot / 2 && sin_t.sizes() == cos_t.sizes() && (reinterpret_cast<uintptr_t>(cos_t.data_ptr()) & 15) == 0 &&
+              (reinterpret_cast<uintptr_t>(sin_t.data_ptr()) & 15) == 0, "rotation: aligned fp32 [positions, rot / 2] tables expected");
+}
+const void* head_weight(const c10::optional<Tensor>& w, int64_t heads, int64_t hd) {
+  if (heads == 0) return nullptr;
+  TORCH_CHECK(w.has_value() && w->scalar_type() == at::kBFloat16 && w->is_contiguous() && w->numel() == hd && (reinterpret_cast<uintptr_t>(w->data_ptr()) & 15) == 0);
+  return w->data_ptr();
+}
+
+// -> (rotated normalised heads [T, (na + nb) hd], rstd [T na] then [T nb])
+std::tuple<Tensor, Tensor> heads_fwd(const Tensor& src, const c10::optional<Tensor>& w_a, int64_t na, const c10::optional<Tensor>& w_b, int64_t nb, double eps,
+                                     const Tensor& positions, const Tensor& cos_t, const Tensor& sin_t, int64_t hd, int64_t rot) {
+  check_rows(src, "src");
+  TORCH_CHECK((hd == 64 || hd == 128 || hd == 256) && na >= 1 && nb >= 0 && src.size(1) >= (na + nb) * hd);
+  check_rotation(positions, cos_t, sin_t, src.size(0), hd, rot);
+  c10::cuda::CUDAGuard guard(src.device());
+  Tensor out = at::empty({src.size(0), (na + nb) * hd}, src.options());
+  Tensor rstd = at::empty({src.size(0) * (na + nb)}, src.options().dtype(at::kFloat));
+  const void* w[2] = {head_weight(w_a, na, hd), head_weight(w_b, nb, hd)};
+  const int heads[2] = {(int)na, (int)nb};
+  sb200::launch_heads_fwd(src.data_ptr(), src.stride(0), w, heads, out.data_ptr(), rstd.data_ptr<float>(), (int)src.size(0), (float)eps,
+                          positions.data_ptr<int64_t>(), cos_t.data_ptr<float>(), sin_t.data_ptr<float>(), cos_t.size(0), (int)hd, (int)rot, cur_stream());
+  return {out, rstd};
+}
+
+// d: gradients (or None) of the a, b and plain blocks, each below and from `split` on (a whole when there is a b)
+Tensor heads_bwd(const c10::List<c10::optional<Tensor>>& d, int64_t split, const Tensor& src, const Tensor& rstd, const c10::optional<Tensor>& w_a, int64_t na,
+                 const c10::optional<Tensor>& w_b, int64_t nb, int64_t nv, const c10::optional<Tensor>& dw_a, bool acc_a, const c10::optional<Tensor>& dw_b,
+                 bool acc_b, const Tensor& positions, const Tensor& cos_t, const Tensor& sin_t, int64_t hd, int64_t rot) {
+  check_rows(src, "src");
+  const int64_t T = src.size(0);
+  TORCH_CHECK(d.size() == 6 && (hd == 64 || hd == 128 || hd == 256) && src.size(1) >= (na + nb + nv) * hd && split >= 0 && split <= T);
+  TORCH_CHECK(rstd.scalar_type() == at::kFloat && rstd.is_contiguous() && rstd.numel() == T * (na + nb));
+  check_rotation(positions, cos_t, sin_t, T, hd, rot);
+  const int heads[3] = {(int)na, (int)nb, (int)nv};
+  const void* ptr[6];
+  int64_t stride[6];
+  const int splits[3] = {(int)(nb > 0 ? T : split), (int)split, (int)split};
+  std::vector<Tensor> hold;
+  for (int i = 0; i < 6; ++i) {
+    ptr[i] = nullptr;
+    stride[i] = 0;
+    const c10::optional<Tensor> g = d.get(i);
+    if (!g.has_value()) continue;
+    check_rows(*g, "gradient");
+    TORCH_CHECK(g->size(1) == heads[i / 2] * hd && g->size(0) == (i % 2 ? T - splits[i / 2] : splits[i / 2]), "heads_bwd: gradient of another shape");
+    hold.push_back(*g);
+    ptr[i] = g->data_ptr();
+    stride[i] = g->stride(0);
+  }
+  c10::cuda::CUDAGuard guard(src.device());
+  Tensor out = at::empty({T, src.size(1)}, src.options());
+  if (src.size(1) > (na + nb + nv) * hd) out.zero_();
+  const c10::optional<Tensor>* dws[2] = {&dw_a, &dw_b};
+  Tensor partial[2];
+  float* pp[2] = {nullptr, nullptr};
+  void* pw[2] = {nullptr, nullptr};
+  for (int i = 0; i < 2; ++i) {
+    if (!dws[i]->has_value() || heads[i] == 0) continue;
+    TORCH_CHECK((*dws[i])->scalar_type() == at::kBFloat16 && (*dws[i])->numel() == hd && (*dws[i])->is_contiguous());
+    if (T == 0 && !(i ? acc_b : acc_a)) (*dws[i])->zero_();
+    partial[i] = at::empty({sb200::heads_bwd_groups((int)T, heads[i]), hd}, rstd.options());
+    pp[i] = partial[i].data_ptr<float>();
+    pw[i] = (*dws[i])->data_ptr();
+  }
+  const void* w[2] = {head_weight(w_a, na, hd), head_weight(w_b, nb, hd)};
+  const int acc[2] = {acc_a ? 1 : 0, acc_b ? 1 : 0};
+  sb200::launch_heads_bwd(ptr, stride, splits, src.data_ptr(), src.stride(0), w, rstd.data_ptr<float>(), pp, pw, acc, heads, out.data_ptr(), out.stride(0), (int)T,
+                          positions.data_ptr<int64_t>(), cos_t.data_ptr<float>(), sin_t.data_ptr<float>(), cos_t.size(0), (int)hd, (int)rot, cur_stream());
+  return out;
+}
+
 // rows_used (optional int32[1] on the device): rows past it are left alone.
 const int* used_rows(const c10::optional<Tensor>& rows_used) {
   if (!rows_used.has_value()) return nullptr;
@@ -192,7 +273,7 @@ Tensor swiglu_bwd(const Tensor& dh, const Tensor& gate_up) { return swiglu_bwd_r
 // [q | k | v] gradients (2-D rows, k and v optional) side by side, rotated back where marked (q always, k with rotate_k).
 Tensor rope_merge(const Tensor& q, const c10::optional<Tensor>& k, const c10::optional<Tensor>& v, bool rotate_k, const Tensor& positions, const Tensor& cos_t,
                   const Tensor& sin_t, int64_t hd, int64_t rot, double sign) {
-  TORCH_CHECK(rot % 16 == 0 && rot <= hd && hd % 8 == 0, "rope_merge: rot a multiple of 16, hd of 8");
+  check_rotation(positions, cos_t, sin_t, q.size(0), hd, rot);
   const Tensor* parts[3] = {&q, k.has_value() ? &*k : nullptr, v.has_value() ? &*v : nullptr};
   const void* src[3] = {nullptr, nullptr, nullptr};
   int64_t stride[3] = {0, 0, 0}, width = 0;
@@ -206,10 +287,6 @@ Tensor rope_merge(const Tensor& q, const c10::optional<Tensor>& k, const c10::op
     heads[i] = (int)(parts[i]->size(1) / hd);
     width += parts[i]->size(1);
   }
-  TORCH_CHECK(positions.scalar_type() == at::kLong && positions.is_contiguous() && positions.numel() == q.size(0));
-  TORCH_CHECK(cos_t.scalar_type() == at::kFloat && sin_t.scalar_type() == at::kFloat && cos_t.is_contiguous() && sin_t.is_contiguous() && cos_t.dim() == 2 &&
-              cos_t.size(1) == rot / 2 && sin_t.sizes() == cos_t.sizes() && (reinterpret_cast<uintptr_t>(cos_t.data_ptr()) & 15) == 0 &&
-              (reinterpret_cast<uintptr_t>(sin_t.data_ptr()) & 15) == 0);
   c10::cuda::CUDAGuard guard(q.device());
   Tensor out = at::empty({q.size(0), width}, q.options());
   sb200::launch_rope_merge(src, stride, heads, rotate, out.data_ptr(), width, positions.data_ptr<int64_t>(), cos_t.data_ptr<float>(), sin_t.data_ptr<float>(),
@@ -1094,6 +1171,8 @@ TORCH_LIBRARY(sb200, m) {
   m.def("swiglu_fwd", &swiglu_fwd);
   m.def("swiglu_bwd", &swiglu_bwd);
   m.def("swiglu_bwd_rows", &swiglu_bwd_rows);
+  m.def("heads_fwd", &heads_fwd);
+  m.def("heads_bwd", &heads_bwd);
   m.def("rope_merge", &rope_merge);
   m.def("gate_mul_fwd", &gate_mul_fwd);
   m.def("gate_mul_bwd", &gate_mul_bwd);

@@ -397,10 +397,7 @@ class TrainEngine:
             ref = weakref.ref(p)  # the hook belongs to p: holding p here would keep every parameter alive for good
 
             def on_grad(g):
-                p = ref()
-                if getattr(p, "_grad_fresh", False):
-                    p._grad_fresh = False
-                    p._flat_grad.zero_()
+                ops.clear_fresh_grad(ref())
                 return g
 
             return on_grad
@@ -417,9 +414,7 @@ class TrainEngine:
 
     def _settle_untouched_grads(self) -> None:
         for p in self.params:
-            if getattr(p, "_grad_fresh", False):
-                p._grad_fresh = False
-                p._flat_grad.zero_()
+            ops.clear_fresh_grad(p)
 
     def prepare_hyper(self, lr: float | None = None) -> None:
         """Host side of a step: bump the step counter and stage lr / bias corrections

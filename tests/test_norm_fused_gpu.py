@@ -60,3 +60,50 @@ def test_eagle3_input_adds_the_half_gradient():
     _reference(hf, wf, 1e-5, False).backward(d[:, H:].float() + dh.float())
     assert (h.grad.float() - hf.grad).abs().max() <= 0.02 * hf.grad.abs().max() + 0.02
     assert (wh.grad.float() - wf.grad).abs().max() <= 0.02 * wf.grad.abs().max() and torch.isfinite(we.grad).all()
+
+
+@pytest.mark.parametrize("hd,rot,T", [(64, 64, 1), (128, 128, 700), (256, 64, 77)])
+@pytest.mark.parametrize("heads,split", [((3, 0, 0), None), ((2, 0, 2), 5), ((4, 2, 2), None), ((6, 1, 1), 40)])
+def test_norm_rope_heads_has_the_bits_of_the_separate_steps(hd, rot, T, heads, split):
+    torch.manual_seed(hd)
+    split = min(split, T) if split is not None else None
+    src = torch.randn(T, sum(heads) * hd, device="cuda").bfloat16()
+    angle = torch.rand(300, rot // 2, device="cuda")
+    pos = torch.randint(0, 300, (T,), device="cuda")
+    weights = [(torch.rand(hd, device="cuda") + 0.5).bfloat16() for _ in range(2)]
+
+    def run(fused):
+        x, wa, wb = (t.clone().requires_grad_() for t in (src, *weights))
+        args = (wa, wb if heads[1] else None, 1e-6, pos, angle.cos(), angle.sin(), heads, hd, rot, split)
+        if fused:
+            out = ops.norm_rope_heads(x, *args)
+        else:
+            blocks, col = [], 0
+            for n, w in zip(heads, (wa, wb, None)):
+                b = x[:, col: col + n * hd].reshape(T, n, hd) if n else None
+                col += n * hd
+                if n and w is not None:
+                    b = ops.rope_(ops.rms_norm(b, w, 1e-6).reshape(T, n * hd), pos, angle.cos(), angle.sin(), n, hd, rot).view(T, n, hd)
+                blocks.append(b)
+            out = ops._head_blocks(blocks, split)
+        g = torch.Generator(device="cuda").manual_seed(1)
+        torch.autograd.backward(out, [torch.randn(o.shape, device="cuda", generator=g).bfloat16() for o in out])
+        return [*out, x.grad, wa.grad, *([wb.grad] if heads[1] else [])]
+
+    for a, b in zip(run(True), run(False), strict=True):
+        assert torch.equal(a, b)
+
+
+def test_row_slices_of_a_flat_gradient_are_stored_then_added():
+    torch.manual_seed(0)
+    w = torch.randn(384, 256, device="cuda").bfloat16().requires_grad_()
+    w._flat_grad, w._grad_fresh = torch.full_like(w, float("nan")), True
+    x = torch.randn(200, 256, device="cuda").bfloat16()
+    want = torch.zeros(384, 256, device="cuda")
+    for r0, r1 in ((128, 256), (0, 128), (128, 256)):
+        dy = torch.randn(200, r1 - r0, device="cuda").bfloat16()
+        ops.linear(x, w, rows=(r0, r1)).backward(dy)
+        want[r0:r1] += dy.float().t() @ x.float()
+    assert torch.isnan(w._flat_grad[256:]).all()
+    ops.clear_fresh_grad(w)
+    assert (w._flat_grad[256:] == 0).all() and (w._flat_grad.float() - want).abs().max() <= 0.02 * want.abs().max()
