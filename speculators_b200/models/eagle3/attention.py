@@ -18,6 +18,7 @@ from __future__ import annotations
 
 import torch
 
+from speculators_b200 import ops
 from speculators_b200.ops import AttnSpec
 
 __all__ = [
@@ -30,6 +31,8 @@ def causal_document_interval(document_ids: torch.Tensor, sliding_window: int | N
     """``(lo, hi)`` int32 [T]: allowed context keys of each query under causal +
     same-document (+ window) masking."""
     doc = document_ids.reshape(-1)
+    if doc.is_cuda and doc.dtype == torch.int64:
+        return ops.native().document_interval(doc.contiguous(), int(sliding_window or 0))  # one launch
     T = doc.shape[0]
     idx = torch.arange(T, device=doc.device)
     new_run = torch.ones(T, dtype=torch.bool, device=doc.device)

@@ -59,14 +59,17 @@ class Eagle3FirstLayer(nn.Module):
         self.hidden_norm = RMSNorm(H, config.rms_norm_eps)
         self.post_attention_layernorm = RMSNorm(H, config.rms_norm_eps)
 
-    def forward(self, embeds, hidden, positions, rotary, spec, past=None, ctx_len=None):
+    def forward(self, embeds, hidden, positions, rotary, spec, past=None, ctx_len=None, repeated=False):
+        """``repeated`` (P-EAGLE): the inputs hold ``ctx_len + 2`` rows, the rows from ``ctx_len`` on share one."""
         H = self.hidden_size
         x, normed_hidden = ops.eagle3_input_concat(
             embeds, hidden, self.input_layernorm.weight, self.hidden_norm.weight, self.hidden_norm.variance_epsilon,
             return_hidden_half=True,
         )
         residual = normed_hidden if self.norm_before_residual else hidden
-        h = self.self_attn(x, positions, rotary, spec, past, ctx_len, residual=residual)
+        if repeated:
+            residual = ops.repeat_rows(residual, positions.shape[0])
+        h = self.self_attn(x, positions, rotary, spec, past, ctx_len, residual=residual, repeated=repeated)
         normed, h = self.post_attention_layernorm.fork(h)
         return self.mlp(normed, residual=h)
 

@@ -233,32 +233,36 @@ class Attention(nn.Module):
         self.q_norm = RMSNorm(self.hd, config.rms_norm_eps) if use_qk_norm else None
         self.k_norm = RMSNorm(self.hd, config.rms_norm_eps) if use_qk_norm else None
 
-    def project_qkv(self, x: torch.Tensor, positions: torch.Tensor, rotary: RotaryTable, split: int | None = None):
+    def project_qkv(self, x: torch.Tensor, positions: torch.Tensor, rotary: RotaryTable, split: int | None = None, repeated: bool = False):
         """x [T, in] -> (q [T, nh, hd], k [T, nkv, hd], v [T, nkv, hd]) with per-head
         norms (if any) and rotary embedding applied; with ``split`` k and v come as
-        two tensors each, the rows below it and the rows from it on."""
-        T = x.shape[0]
+        two tensors each, the rows below it and the rows from it on.  ``repeated``: ``x`` has
+        ``split + 2`` rows, the rows from ``split`` on all read row ``split`` (``ops.repeat_rows``)."""
+        T = positions.shape[0]
         nq, nk = self.nh * self.hd, self.nkv * self.hd
         qkv = self.qkv_proj(x)
         if self.q_norm is not None:
             return ops.norm_rope_heads(qkv, self.q_norm.weight, self.k_norm.weight, self.q_norm.variance_epsilon, positions, rotary.cos,
-                                       rotary.sin, (self.nh, self.nkv, self.nkv), self.hd, self.rot, split)
+                                       rotary.sin, (self.nh, self.nkv, self.nkv), self.hd, self.rot, split, repeated)
+        if repeated:
+            qkv = ops.repeat_rows(qkv, T)
         q, k, v = ops.rope_split(qkv, positions, rotary.cos, rotary.sin, self.nh + self.nkv, self.hd, self.rot, nq, nk)
         q, k, v = q.view(T, self.nh, self.hd), k.view(T, self.nkv, self.hd), v.view(T, self.nkv, self.hd)
         return (q, k, v) if split is None else (q, k[:split], k[split:], v[:split], v[split:])
 
     def forward(self, x, positions, rotary, spec: AttnSpec, past: list | None = None, ctx_len: int | None = None,
-                residual: torch.Tensor | None = None) -> torch.Tensor:
+                residual: torch.Tensor | None = None, repeated: bool = False) -> torch.Tensor:
         """``past`` (EAGLE-3 TTT): list of (k, v) of earlier passes over the same
         positions.  Entry 0 is the context the interval part of ``spec`` indexes;
         later entries and this pass's own keys are reachable through
         ``spec.extra_idx`` (row ``(j-1)*T + i`` = key ``i`` of pass ``j``).
 
         ``ctx_len`` (P-EAGLE): the first ``ctx_len`` rows of this pass are the
-        interval-addressed context, the remaining rows are the extra keys."""
-        T = x.shape[0]
+        interval-addressed context, the remaining rows are the extra keys; ``repeated``
+        says that ``x`` holds those only once (``project_qkv``)."""
+        T = positions.shape[0]
         if ctx_len is not None and ctx_len < T:
-            q, k_ctx, k_ext, v_ctx, v_ext = self.project_qkv(x, positions, rotary, split=ctx_len)
+            q, k_ctx, k_ext, v_ctx, v_ext = self.project_qkv(x, positions, rotary, split=ctx_len, repeated=repeated)
             out = ops.masked_attention(q, k_ctx, v_ctx, spec, k_ext, v_ext, scale=self.scaling)
             return self.o_proj(out.reshape(T, self.nh * self.hd), residual=residual)
         q, k, v = self.project_qkv(x, positions, rotary)

@@ -19,6 +19,7 @@ from __future__ import annotations
 
 import torch
 
+from speculators_b200 import ops
 from speculators_b200.models.eagle3.attention import causal_document_interval
 from speculators_b200.ops import AttnSpec
 
@@ -34,6 +35,10 @@ def peagle_attn_spec(anchor_pos, depth, document_ids, num_depths: int, sliding_w
     n = anchor_pos.shape[0]
     device = doc.device
     doc_lo, _ = causal_document_interval(doc, None)
+    if doc.is_cuda and all(t.dtype == torch.int64 for t in (doc, anchor_pos, depth)):
+        lo, hi, extra = ops.native().peagle_spec(anchor_pos.contiguous(), depth.contiguous(), row_valid, doc.contiguous(), doc_lo, num_depths,
+                                                 int(sliding_window or 0))
+        return AttnSpec(lo=lo, hi=hi, extra_idx=extra if extra.numel() else None)
     lo = doc_lo[anchor_pos].to(torch.int64)
     if sliding_window is not None:
         lo = torch.maximum(lo, anchor_pos + depth - int(sliding_window) + 1)

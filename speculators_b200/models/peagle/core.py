@@ -89,12 +89,17 @@ class PEagleDraftModel(Eagle3DraftModel):
                 down_sample_ratio_min=down_sample_ratio_min, max_anchors=max_anchors,
             )
         orig = anchor_pos + depth
-        depth0 = depth == 0
-        ids = torch.where(depth0, input_ids.reshape(-1)[orig], torch.full_like(orig, self.mask_token_id))
-        embeds = self.embed_tokens(ids).to(dtype)
+        n = orig.shape[0]
+        # Every row deeper than 0 (they follow the T rows of depth 0) reads the mask token and the mask state: the products
+        # up to the first attention are formed once for all of them, as row T (kept twice, see ``ops.repeat_rows``).
+        repeated = n > T
+        ids = input_ids.reshape(-1)
         aux = hidden_states.reshape(T, -1).to(dtype)
-        sampled = torch.where(depth0.unsqueeze(-1), aux[orig], self.mask_hidden.reshape(1, -1).to(dtype).expand(orig.shape[0], -1))
-        hidden = self._project_aux(sampled)
+        if repeated:
+            ids = torch.cat([ids, torch.full((2,), self.mask_token_id, dtype=ids.dtype, device=device)])
+            aux = torch.cat([aux, self.mask_hidden.reshape(1, -1).to(dtype).expand(2, -1)])
+        embeds = ops.embedding(ids, self.embed_tokens.weight, self.embed_tokens.padding_idx).to(dtype)
+        hidden = self._project_aux(aux)
 
         doc = document_ids.reshape(-1).to(device)
         full_spec = peagle_attn_spec(anchor_pos, depth, doc, num_depths, None, row_valid) if self.uses_full_attn else None
@@ -104,13 +109,15 @@ class PEagleDraftModel(Eagle3DraftModel):
         for li, layer in enumerate(self.layers):
             spec = win_spec if li in self.sliding_window_indices else full_spec
             if li == 0:
-                hidden = layer(embeds, hidden, orig, self.rotary_emb, spec, None, T)
+                hidden = layer(embeds, hidden, orig, self.rotary_emb, spec, None, T, repeated)
             else:
                 hidden = layer(hidden, orig, self.rotary_emb, spec, None, T)
         logits = ops.linear(self.norm(hidden), self.lm_head.weight)
         with torch.no_grad():
-            vl = verifier_last_hidden_states.reshape(T, -1).to(dtype)[orig]
+            # rows of one position share their target: T rows of the verifier's head, then a gather
+            vl = verifier_last_hidden_states.reshape(T, -1).to(dtype)
             targets = ops.linear(self.verifier_norm(vl), self.verifier_lm_head.weight)
+            targets = targets.index_select(0, orig) if repeated else targets
         loss, metrics = compute_metrics(
             logits.unsqueeze(0), targets.unsqueeze(0), loss_mask, anchor_pos, depth, num_depths, loss_config=loss_config,
             row_valid=row_valid,

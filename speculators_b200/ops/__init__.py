@@ -28,6 +28,7 @@ __all__ = [
     "LOSS_OPS",
     "adamw_step_",
     "eagle3_input_concat",
+    "embedding",
     "fused_row_loss",
     "gated",
     "check_gemm_status",
@@ -46,6 +47,7 @@ __all__ = [
     "masked_attention_reference",
     "native",
     "norm_rope_heads",
+    "repeat_rows",
     "rms_norm",
     "rms_norm_fork",
     "rope_",
@@ -649,20 +651,24 @@ class _NormRopeHeadsFn(torch.autograd.Function):
     """Head norms and rotation of a projection ``[a heads | b heads | plain heads]``; see ``norm_rope_heads``."""
 
     @staticmethod
-    def forward(ctx, src, w_a, w_b, positions, cos_t, sin_t, eps, heads, hd, rot, split):
-        T, (na, nb, nv) = src.shape[0], heads
+    def forward(ctx, src, w_a, w_b, positions, cos_t, sin_t, eps, heads, hd, rot, split, repeated):
+        na, nb, nv = heads
         src = src.detach()
-        out, rstd = native().heads_fwd(src, w_a, na, w_b, nb, eps, positions, cos_t, sin_t, hd, rot)
+        out, rstd = native().heads_fwd(src, w_a, na, w_b, nb, eps, positions, cos_t, sin_t, hd, rot, repeated)
         ctx.save_for_backward(src, w_a, w_b, rstd, positions, cos_t, sin_t)
-        ctx.cfg = (heads, hd, rot, split)
+        ctx.cfg = (heads, hd, rot, split, repeated)
         ctx.set_materialize_grads(False)
         blocks = [out[:, : na * hd], out[:, na * hd :], src[:, (na + nb) * hd : (na + nb + nv) * hd]]
-        return _head_blocks([b.view(T, n, hd) if n else None for b, n in zip(blocks, heads)], split)
+        blocks = [b.unflatten(1, (n, hd)) if n else None for b, n in zip(blocks, heads)]
+        if repeated:
+            v = blocks[2]
+            return blocks[0], blocks[1][:split], blocks[1][split:], v[:split], v[split : split + 1].expand(out.shape[0] - split, nv, hd)
+        return _head_blocks(blocks, split)
 
     @staticmethod
     def backward(ctx, *grads):
         src, w_a, w_b, rstd, positions, cos_t, sin_t = ctx.saved_tensors
-        (na, nb, nv), hd, rot, split = ctx.cfg
+        (na, nb, nv), hd, rot, split, repeated = ctx.cfg
         it = iter(grads)
         rows = []  # gradients of rows below and from the split on, for each of the three blocks
         for block, n in enumerate((na, nb, nv)):
@@ -671,21 +677,28 @@ class _NormRopeHeadsFn(torch.autograd.Function):
                 rows.append(_grad_rows(g, n * hd) if g is not None and g.shape[0] else None)
         dw_a, acc_a, flat_a = _param_grad_target(w_a) if ctx.needs_input_grad[1] else (None, False, False)
         dw_b, acc_b, flat_b = _param_grad_target(w_b) if nb and ctx.needs_input_grad[2] else (None, False, False)
-        d = native().heads_bwd(rows, src.shape[0] if split is None else split, src, rstd, w_a, na, w_b, nb, nv, dw_a, acc_a, dw_b, acc_b, positions, cos_t, sin_t, hd, rot)
-        return d, None if flat_a else dw_a, None if flat_b else dw_b, None, None, None, None, None, None, None, None
+        d = native().heads_bwd(rows, src.shape[0] if split is None else split, src, rstd, w_a, na, w_b, nb, nv, dw_a, acc_a, dw_b, acc_b, positions, cos_t, sin_t, hd, rot, repeated)
+        return d, None if flat_a else dw_a, None if flat_b else dw_b, None, None, None, None, None, None, None, None, None
 
 
 def norm_rope_heads(src: torch.Tensor, w_a, w_b, eps: float, positions, cos_t, sin_t, heads: tuple[int, int, int], hd: int, rot: int,
-                    split: int | None = None):
+                    split: int | None = None, repeated: bool = False):
     """Per-head RMSNorm (weights ``w_a``, ``w_b``) and rotary embedding of the first ``heads[0]`` and next ``heads[1]`` heads of
     a projection ``[T, sum(heads) * hd]``; the last ``heads[2]`` heads pass through.  Returns a ``[T, n, hd]`` tensor for every
     block that has heads, or with ``split`` two (rows below it, rows from it on) for every block but the queries, the first of
     two rotated ones.  One launch each way on CUDA (head
-    dims 64, 128, 256); the gradients of all results are gathered into one buffer of the projection's layout."""
+    dims 64, 128, 256); the gradients of all results are gathered into one buffer of the projection's layout.
+
+    ``repeated``: ``src`` holds ``split + 2`` rows, and every row from ``split`` on (``positions`` has them all) stands for row
+    ``split`` at its own position, as ``repeat_rows`` would lay them out."""
     na, nb, nv = heads
+    if repeated and not (nb and nv and _norm_native(src)):
+        src, repeated = repeat_rows(src, positions.shape[0]), False
     if (_use_native(src) and src.dtype == torch.bfloat16 and hd in (64, 128, 256) and rot % 16 == 0 and rot <= hd and src.stride(-1) == 1
             and src.stride(0) % 8 == 0 and src.data_ptr() % 16 == 0 and positions.is_contiguous() and all(w is None or w.dtype == src.dtype for w in (w_a, w_b))):
-        return _NormRopeHeadsFn.apply(src, w_a, w_b, positions, cos_t, sin_t, eps, heads, hd, rot, split)
+        return _NormRopeHeadsFn.apply(src, w_a, w_b, positions, cos_t, sin_t, eps, heads, hd, rot, split, repeated)
+    if repeated:
+        src = repeat_rows(src, positions.shape[0])
     T, blocks, col = src.shape[0], [], 0
     for n, w in ((na, w_a), (nb, w_b), (nv, None)):
         x = src[:, col : col + n * hd].reshape(T, n, hd) if n else None
@@ -694,6 +707,65 @@ def norm_rope_heads(src: torch.Tensor, w_a, w_b, eps: float, positions, cos_t, s
             x = rope_(rms_norm(x, w, eps).reshape(T, n * hd), positions, cos_t, sin_t, n, hd, rot).view(T, n, hd)
         blocks.append(x)
     return _head_blocks(blocks, split)
+
+
+# --------------------------------------------------------------------------- repeated rows, embedding
+class _RepeatRowsFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, n):
+        T = x.shape[0] - 2
+        out = torch.empty((n, x.shape[1]), dtype=x.dtype, device=x.device)
+        out[:T] = x[:T]
+        out[T:] = x[T]
+        ctx.T = T
+        return out
+
+    @staticmethod
+    def backward(ctx, d):
+        T = ctx.T
+        dx = torch.empty((T + 2, d.shape[1]), dtype=d.dtype, device=d.device)
+        dx[:T] = d[:T]
+        native().repeated_rows_sum(_grad_rows(d[T:], d.shape[1]), dx[T:])
+        return dx, None
+
+
+def repeat_rows(x: torch.Tensor, n: int) -> torch.Tensor:
+    """``[T + 2, W] -> [n, W]``: the first ``T`` rows, then row ``T`` as often as it takes (``n > T``).  The last two rows of
+    ``x`` hold the same values; a gradient reaches them as the rounded sum over the repeated rows and the rest that rounding
+    left, so products with the two keep the sum at twice the precision of bf16."""
+    T = x.shape[0] - 2
+    if _use_native(x) and x.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and torch.is_grad_enabled() and x.requires_grad:
+        return _RepeatRowsFn.apply(x, n)
+    return torch.cat([x[:T], x[T : T + 1].expand(n - T, -1)])
+
+
+class _EmbeddingFn(torch.autograd.Function):
+    """Rows of ``weight``; the gradient goes straight into the engine's flat buffer (a dense one of autograd's own was zeroed,
+    filled and then added to it: 3.7 GB of traffic for a 152k x 4096 table), duplicates summed in fp32 in a fixed order."""
+
+    @staticmethod
+    def forward(ctx, ids, weight, padding_idx):
+        ctx.save_for_backward(ids, weight)
+        ctx.padding_idx = padding_idx
+        return F.embedding(ids, weight)
+
+    @staticmethod
+    def backward(ctx, d):
+        ids, weight = ctx.saved_tensors
+        dw, accumulate, attached = _param_grad_target(weight)
+        if not accumulate:
+            dw.zero_()
+        order = torch.sort(ids, stable=True)
+        native().embedding_bwd(order.values, order.indices, _grad_rows(d, d.shape[1]), -1 if ctx.padding_idx is None else ctx.padding_idx, dw, accumulate)
+        return None, None if attached else dw, None
+
+
+def embedding(ids: torch.Tensor, weight: torch.Tensor, padding_idx: int | None = None) -> torch.Tensor:
+    """``F.embedding`` of flat ``ids`` for a table that is trained."""
+    if (_use_native(weight) and weight.dtype == torch.bfloat16 and weight.requires_grad and torch.is_grad_enabled() and weight.shape[1] % 8 == 0
+            and ids.dtype == torch.int64):
+        return _EmbeddingFn.apply(ids.reshape(-1), weight, padding_idx)
+    return F.embedding(ids, weight, padding_idx)
 
 
 # --------------------------------------------------------------------------- gated attention

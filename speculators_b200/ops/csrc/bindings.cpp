@@ -21,11 +21,18 @@ int read_bounds_norm(BoundsRecord*);
 int read_bounds_ep(BoundsRecord*);
 void launch_rmsnorm_bwd(const void*, int64_t, const void*, int64_t, const void*, int64_t, const void*, const float*, const void*, int64_t, void*, int64_t,
                         float*, void*, int, int, int, int, cudaStream_t);
-void launch_heads_fwd(const void*, int64_t, const void* const*, const int*, void*, float*, int, float, const int64_t*, const float*, const float*, int64_t, int,
-                      int, cudaStream_t);
+void launch_heads_fwd(const void*, int64_t, const void* const*, const int*, void*, float*, int, int, float, const int64_t*, const float*, const float*, int64_t,
+                      int, int, cudaStream_t);
 int heads_bwd_groups(int, int);
+int64_t repeated_part_floats(int, int, int);
 void launch_heads_bwd(const void* const*, const int64_t*, const int*, const void*, int64_t, const void* const*, const float*, float* const*, void* const*,
-                      const int*, const int*, void*, int64_t, int, const int64_t*, const float*, const float*, int64_t, int, int, cudaStream_t);
+                      const int*, const int*, void*, int64_t, int, int, float*, const int64_t*, const float*, const float*, int64_t, int, int, cudaStream_t);
+void launch_repeated_rows_sum(const void*, int64_t, int, int, float*, void*, int64_t, cudaStream_t);
+void launch_document_interval(const int64_t*, int, int, int*, int*, cudaStream_t);
+void launch_compact(const bool*, int, int64_t*, int*, cudaStream_t);
+void launch_cod_step(const int64_t*, const int64_t*, int, const bool*, int, int, int, unsigned char*, int64_t*, int64_t*, int64_t*, int64_t*, int*, cudaStream_t);
+void launch_peagle_spec(const int64_t*, const int64_t*, const bool*, const int64_t*, const int*, int, int, int, int, int*, int*, int*, int*, cudaStream_t);
+void launch_embedding_bwd(const int64_t*, const int64_t*, const void*, int64_t, int, int, int64_t, int64_t, void*, int, cudaStream_t);
 void launch_swiglu_fwd(const void*, void*, int64_t, int, const int*, cudaStream_t);
 void launch_swiglu_bwd(const void*, const void*, void*, int64_t, int, const int*, cudaStream_t);
 void launch_rope_merge(const void* const*, const int64_t*, const int*, const int*, void*, int64_t, const int64_t*, const float*, const float*, int64_t, int, int,
@@ -177,18 +184,22 @@ const void* head_weight(const c10::optional<Tensor>& w, int64_t heads, int64_t h
   return w->data_ptr();
 }
 
-// -> (rotated normalised heads [T, (na + nb) hd], rstd [T na] then [T nb])
+// -> (rotated normalised heads [T, (na + nb) hd], rstd [T na] then [T nb]); repeated: src holds two rows more than the
+// first tokens, and the tokens after those (positions has them all) read the first of the two
 std::tuple<Tensor, Tensor> heads_fwd(const Tensor& src, const c10::optional<Tensor>& w_a, int64_t na, const c10::optional<Tensor>& w_b, int64_t nb, double eps,
-                                     const Tensor& positions, const Tensor& cos_t, const Tensor& sin_t, int64_t hd, int64_t rot) {
+                                     const Tensor& positions, const Tensor& cos_t, const Tensor& sin_t, int64_t hd, int64_t rot, bool repeated) {
   check_rows(src, "src");
+  const int64_t T = repeated ? positions.numel() : src.size(0);
   TORCH_CHECK((hd == 64 || hd == 128 || hd == 256) && na >= 1 && nb >= 0 && src.size(1) >= (na + nb) * hd);
-  check_rotation(positions, cos_t, sin_t, src.size(0), hd, rot);
+  TORCH_CHECK(!repeated || (src.size(0) >= 2 && T > src.size(0) - 2), "heads_fwd: two rows for the repeated tokens expected");
+  check_rotation(positions, cos_t, sin_t, T, hd, rot);
   c10::cuda::CUDAGuard guard(src.device());
-  Tensor out = at::empty({src.size(0), (na + nb) * hd}, src.options());
-  Tensor rstd = at::empty({src.size(0) * (na + nb)}, src.options().dtype(at::kFloat));
+  Tensor out = at::empty({T, (na + nb) * hd}, src.options());
+  Tensor rstd = at::empty({T * (na + nb)}, src.options().dtype(at::kFloat));
   const void* w[2] = {head_weight(w_a, na, hd), head_weight(w_b, nb, hd)};
   const int heads[2] = {(int)na, (int)nb};
-  sb200::launch_heads_fwd(src.data_ptr(), src.stride(0), w, heads, out.data_ptr(), rstd.data_ptr<float>(), (int)src.size(0), (float)eps,
+  sb200::launch_heads_fwd(src.data_ptr(), src.stride(0), w, heads, out.data_ptr(), rstd.data_ptr<float>(), (int)T,
+                          (int)(repeated ? src.size(0) - 2 : src.size(0)), (float)eps,
                           positions.data_ptr<int64_t>(), cos_t.data_ptr<float>(), sin_t.data_ptr<float>(), cos_t.size(0), (int)hd, (int)rot, cur_stream());
   return {out, rstd};
 }
@@ -196,9 +207,10 @@ std::tuple<Tensor, Tensor> heads_fwd(const Tensor& src, const c10::optional<Tens
 // d: gradients (or None) of the a, b and plain blocks, each below and from `split` on (a whole when there is a b)
 Tensor heads_bwd(const c10::List<c10::optional<Tensor>>& d, int64_t split, const Tensor& src, const Tensor& rstd, const c10::optional<Tensor>& w_a, int64_t na,
                  const c10::optional<Tensor>& w_b, int64_t nb, int64_t nv, const c10::optional<Tensor>& dw_a, bool acc_a, const c10::optional<Tensor>& dw_b,
-                 bool acc_b, const Tensor& positions, const Tensor& cos_t, const Tensor& sin_t, int64_t hd, int64_t rot) {
+                 bool acc_b, const Tensor& positions, const Tensor& cos_t, const Tensor& sin_t, int64_t hd, int64_t rot, bool repeated) {
   check_rows(src, "src");
-  const int64_t T = src.size(0);
+  const int64_t T = positions.numel(), tokens = repeated ? src.size(0) - 2 : src.size(0);
+  TORCH_CHECK(repeated ? (tokens >= 0 && T > tokens && split == tokens && nb > 0) : T == tokens, "heads_bwd: rows and positions do not match");
   TORCH_CHECK(d.size() == 6 && (hd == 64 || hd == 128 || hd == 256) && src.size(1) >= (na + nb + nv) * hd && split >= 0 && split <= T);
   TORCH_CHECK(rstd.scalar_type() == at::kFloat && rstd.is_contiguous() && rstd.numel() == T * (na + nb));
   check_rotation(positions, cos_t, sin_t, T, hd, rot);
@@ -219,8 +231,8 @@ Tensor heads_bwd(const c10::List<c10::optional<Tensor>>& d, int64_t split, const
     stride[i] = g->stride(0);
   }
   c10::cuda::CUDAGuard guard(src.device());
-  Tensor out = at::empty({T, src.size(1)}, src.options());
-  if (src.size(1) > (na + nb + nv) * hd) out.zero_();
+  Tensor out = at::empty({src.size(0), src.size(1)}, src.options());
+  if (src.size(1) > (na + nb + nv) * hd || tokens == 0) out.zero_();
   const c10::optional<Tensor>* dws[2] = {&dw_a, &dw_b};
   Tensor partial[2];
   float* pp[2] = {nullptr, nullptr};
@@ -228,16 +240,93 @@ Tensor heads_bwd(const c10::List<c10::optional<Tensor>>& d, int64_t split, const
   for (int i = 0; i < 2; ++i) {
     if (!dws[i]->has_value() || heads[i] == 0) continue;
     TORCH_CHECK((*dws[i])->scalar_type() == at::kBFloat16 && (*dws[i])->numel() == hd && (*dws[i])->is_contiguous());
-    if (T == 0 && !(i ? acc_b : acc_a)) (*dws[i])->zero_();
-    partial[i] = at::empty({sb200::heads_bwd_groups((int)T, heads[i]), hd}, rstd.options());
+    if (tokens == 0 && !(i ? acc_b : acc_a)) (*dws[i])->zero_();
+    partial[i] = at::empty({sb200::heads_bwd_groups((int)tokens, heads[i]) + (repeated ? heads[i] : 0), hd}, rstd.options());
     pp[i] = partial[i].data_ptr<float>();
     pw[i] = (*dws[i])->data_ptr();
   }
   const void* w[2] = {head_weight(w_a, na, hd), head_weight(w_b, nb, hd)};
   const int acc[2] = {acc_a ? 1 : 0, acc_b ? 1 : 0};
-  sb200::launch_heads_bwd(ptr, stride, splits, src.data_ptr(), src.stride(0), w, rstd.data_ptr<float>(), pp, pw, acc, heads, out.data_ptr(), out.stride(0), (int)T,
-                          positions.data_ptr<int64_t>(), cos_t.data_ptr<float>(), sin_t.data_ptr<float>(), cos_t.size(0), (int)hd, (int)rot, cur_stream());
+  Tensor sums;
+  if (repeated) sums = at::empty({sb200::repeated_part_floats((int)(T - tokens), (int)(na + nb + nv), (int)hd)}, rstd.options());
+  sb200::launch_heads_bwd(ptr, stride, splits, src.data_ptr(), src.stride(0), w, rstd.data_ptr<float>(), pp, pw, acc, heads, out.data_ptr(), out.stride(0), (int)tokens, (int)T,
+                          repeated ? sums.data_ptr<float>() : nullptr, positions.data_ptr<int64_t>(), cos_t.data_ptr<float>(), sin_t.data_ptr<float>(), cos_t.size(0), (int)hd, (int)rot, cur_stream());
   return out;
+}
+
+// dst[0], dst[1] = the fp32 sum of all rows of d as a rounded row and what the rounding left
+void repeated_rows_sum(const Tensor& d, Tensor dst) {
+  check_rows(d, "d");
+  check_rows(dst, "dst");
+  TORCH_CHECK(d.size(0) >= 1 && dst.size(0) == 2 && dst.size(1) == d.size(1) && d.size(1) % 8 == 0);
+  c10::cuda::CUDAGuard guard(d.device());
+  Tensor part = at::empty({sb200::repeated_part_floats((int)d.size(0), (int)d.size(1), 1)}, d.options().dtype(at::kFloat));
+  sb200::launch_repeated_rows_sum(d.data_ptr(), d.stride(0), (int)d.size(0), (int)d.size(1), part.data_ptr<float>(), dst.data_ptr(), dst.stride(0), cur_stream());
+}
+
+// ---- row bookkeeping -------------------------------------------------------------------------------
+const int64_t* long_ptr(const Tensor& t, const char* name) {
+  TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kLong && t.is_contiguous(), name, ": contiguous int64 CUDA tensor expected");
+  return t.data_ptr<int64_t>();
+}
+const bool* bool_ptr(const Tensor& t, int64_t n, const char* name) {
+  TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kBool && t.is_contiguous() && t.numel() == n, name, ": contiguous bool CUDA tensor expected");
+  return t.data_ptr<bool>();
+}
+std::tuple<Tensor, Tensor> document_interval(const Tensor& doc, int64_t window) {
+  const int64_t* d = long_ptr(doc, "document_ids");
+  c10::cuda::CUDAGuard guard(doc.device());
+  Tensor both = at::empty({2, doc.numel()}, doc.options().dtype(at::kInt));
+  Tensor lo = both.select(0, 0), hi = both.select(0, 1);
+  sb200::launch_document_interval(d, (int)doc.numel(), (int)window, lo.data_ptr<int>(), hi.data_ptr<int>(), cur_stream());
+  return {lo, hi};
+}
+// positions of the set entries -> (int64[T] of which the first count are filled, int32[1] count)
+std::tuple<Tensor, Tensor> compact_rows(const Tensor& valid) {
+  const bool* v = bool_ptr(valid, valid.numel(), "valid");
+  c10::cuda::CUDAGuard guard(valid.device());
+  Tensor list = at::empty({valid.numel()}, valid.options().dtype(at::kLong)), count = at::empty({1}, valid.options().dtype(at::kInt));
+  sb200::launch_compact(v, (int)valid.numel(), list.data_ptr<int64_t>(), count.data_ptr<int>(), cur_stream());
+  return {list, count};
+}
+// anchor / depths: int64[take] views the step fills; -> (picked int64[take], next pool int64[take], its size int32[1])
+std::tuple<Tensor, Tensor, Tensor> cod_step(const Tensor& pool, const c10::optional<Tensor>& perm, int64_t take, const Tensor& valid, int64_t depth,
+                                            bool filter_zero, Tensor anchor, Tensor depths) {
+  const int64_t T = valid.numel();
+  TORCH_CHECK(take >= 0 && take <= pool.numel() && anchor.numel() == take && depths.numel() == take && (!perm.has_value() || perm->numel() >= take));
+  const bool* v = bool_ptr(valid, T, "valid");
+  c10::cuda::CUDAGuard guard(valid.device());
+  auto opt = valid.options();
+  Tensor flags = at::empty({perm.has_value() ? T : 0}, opt.dtype(at::kByte)), picked = at::empty({take}, opt.dtype(at::kLong));
+  Tensor next = at::empty({take}, opt.dtype(at::kLong)), count = at::empty({1}, opt.dtype(at::kInt));
+  sb200::launch_cod_step(long_ptr(pool, "pool"), perm.has_value() ? long_ptr(*perm, "perm") : nullptr, (int)take, v, (int)T, (int)depth, filter_zero ? 1 : 0,
+                         flags.data_ptr<uint8_t>(), picked.data_ptr<int64_t>(), const_cast<int64_t*>(long_ptr(anchor, "anchor")),
+                         const_cast<int64_t*>(long_ptr(depths, "depths")), next.data_ptr<int64_t>(), count.data_ptr<int>(), cur_stream());
+  return {picked, next, count};
+}
+// -> (lo, hi int32[n], extra int32[n, num_depths - 1] or empty)
+std::tuple<Tensor, Tensor, Tensor> peagle_spec(const Tensor& anchor, const Tensor& depth, const c10::optional<Tensor>& row_valid, const Tensor& doc,
+                                               const Tensor& doc_lo, int64_t num_depths, int64_t window) {
+  const int64_t n = anchor.numel(), T = doc.numel();
+  TORCH_CHECK(depth.numel() == n && doc_lo.numel() == T && doc_lo.scalar_type() == at::kInt && doc_lo.is_contiguous() && T > 0);
+  c10::cuda::CUDAGuard guard(doc.device());
+  auto opt = doc.options().dtype(at::kInt);
+  const bool extras = num_depths > 1 && n > T;
+  Tensor lo = at::empty({n}, opt), hi = at::empty({n}, opt), extra = at::empty({extras ? n : 0, num_depths - 1}, opt);
+  Tensor table = extras ? at::full({num_depths, T}, -1, opt) : at::empty({0}, opt);
+  sb200::launch_peagle_spec(long_ptr(anchor, "anchor_pos"), long_ptr(depth, "depth"), row_valid.has_value() ? bool_ptr(*row_valid, n, "row_valid") : nullptr,
+                            long_ptr(doc, "document_ids"), doc_lo.data_ptr<int>(), (int)n, (int)T, (int)num_depths, (int)window, table.data_ptr<int>(),
+                            lo.data_ptr<int>(), hi.data_ptr<int>(), extras ? extra.data_ptr<int>() : nullptr, cur_stream());
+  return {lo, hi, extra};
+}
+// dw rows of the ids (ascending, `order` their source rows of d) stored or added to
+void embedding_bwd(const Tensor& ids, const Tensor& order, const Tensor& d, int64_t padding, Tensor dw, bool accumulate) {
+  check_rows(d, "d");
+  TORCH_CHECK(ids.numel() == d.size(0) && order.numel() == d.size(0) && dw.dim() == 2 && dw.is_contiguous() && dw.scalar_type() == at::kBFloat16 &&
+              dw.size(1) == d.size(1) && d.size(1) % 8 == 0 && (reinterpret_cast<uintptr_t>(dw.data_ptr()) & 15) == 0);
+  c10::cuda::CUDAGuard guard(d.device());
+  sb200::launch_embedding_bwd(long_ptr(ids, "ids"), long_ptr(order, "order"), d.data_ptr(), d.stride(0), (int)d.size(0), (int)d.size(1), dw.size(0), padding,
+                              dw.data_ptr(), accumulate ? 1 : 0, cur_stream());
 }
 
 // rows_used (optional int32[1] on the device): rows past it are left alone.
@@ -1174,6 +1263,12 @@ TORCH_LIBRARY(sb200, m) {
   m.def("heads_fwd", &heads_fwd);
   m.def("heads_bwd", &heads_bwd);
   m.def("rope_merge", &rope_merge);
+  m.def("repeated_rows_sum", &repeated_rows_sum);
+  m.def("document_interval", &document_interval);
+  m.def("compact_rows", &compact_rows);
+  m.def("cod_step", &cod_step);
+  m.def("peagle_spec", &peagle_spec);
+  m.def("embedding_bwd", &embedding_bwd);
   m.def("gate_mul_fwd", &gate_mul_fwd);
   m.def("gate_mul_bwd", &gate_mul_bwd);
   m.def("moe_plan", &moe_plan);

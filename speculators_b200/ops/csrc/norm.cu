@@ -419,7 +419,7 @@ struct HeadsFwdArgs {
   int heads[2];
   __nv_bfloat16* out;  // [T, (heads[0] + heads[1]) * hd]
   float* rstd;         // [T * heads[0]] then [T * heads[1]]
-  int tokens;
+  int tokens, src_last;  // tokens from src_last on read that row of src
   float eps;
   HeadsRope rope;
 };
@@ -438,7 +438,7 @@ __global__ void __launch_bounds__(256) heads_fwd_kernel(const HeadsFwdArgs p) {
     float xv[8], wv[8], ss = 0.f;
 #pragma unroll
     for (int j = 0; j < 8; ++j) xv[j] = 0.f;
-    if (on) unpack8(ld8(p.src + t * p.src_stride + c * HD + l * 8), xv);
+    if (on) unpack8(ld8(p.src + min(t, (int64_t)p.src_last) * p.src_stride + c * HD + l * 8), xv);
 #pragma unroll
     for (int j = 0; j < 8; ++j) ss += xv[j] * xv[j];
     nw.load(p.w[which] + l * 8, wv);
@@ -458,7 +458,7 @@ struct HeadsBwdArgs {
   const __nv_bfloat16* src;
   int64_t src_stride;
   const __nv_bfloat16* w[2];
-  const float* rstd;
+  const float* rstd[2];
   float* partial[2];  // weight gradient sums, one row per group
   int heads[3], groups[3];
   __nv_bfloat16* dst;
@@ -505,7 +505,7 @@ __global__ void __launch_bounds__(256) heads_bwd_kernel(const HeadsBwdArgs p) {
 #pragma unroll
   for (int j = 0; j < 8; ++j) dwacc[j] = 0.f;
   nw.load(p.w[which] + l * 8, wv);
-  const float* rstd_of = p.rstd + (which ? (int64_t)p.tokens * p.heads[0] : 0);
+  const float* rstd_of = p.rstd[which];
   const int trips = (int)((rows + groups - 1) / groups);  // the same in all groups: every lane shuffles
   int64_t t;
   int h;
@@ -548,6 +548,89 @@ __global__ void __launch_bounds__(256) heads_bwd_kernel(const HeadsBwdArgs p) {
     float4* o4 = reinterpret_cast<float4*>(p.partial[which] + (int64_t)g * HD + l * 8);
     o4[0] = make_float4(dwacc[0], dwacc[1], dwacc[2], dwacc[3]);
     o4[1] = make_float4(dwacc[4], dwacc[5], dwacc[6], dwacc[7]);
+  }
+}
+
+// Rows that were one row of the projection (P-EAGLE's deeper samples all read the same mask token and mask state, so the
+// products are formed once): their gradients, rotated back, are summed in fp32 and taken through the norm as one row.
+// The result is kept as two bf16 rows, the rounded sum and what the rounding left over, so that the products of the
+// backward pass see it at twice the precision.  Two launches: slices of rows by 2048 columns, then one block per head.
+struct RepeatedArgs {
+  const __nv_bfloat16* d[3];  // gradients of the repeated rows
+  int64_t d_stride[3];
+  int heads[3], hd, rows, slices;
+  float* part;  // [slices][all columns]
+  HeadsRope rope;  // positions of the repeated rows
+  const __nv_bfloat16* w[2];
+  const __nv_bfloat16* src;  // the row of the projection they read
+  const float* rstd[2];      // of its heads
+  float* dw_part[2];         // one row of hd floats per head
+  __nv_bfloat16* dst;        // two rows
+  int64_t dst_stride;
+};
+__global__ void __launch_bounds__(256) repeated_sum_kernel(const RepeatedArgs p) {
+  pdl_begin();
+  const int64_t cols = (int64_t)(p.heads[0] + p.heads[1] + p.heads[2]) * p.hd, c = ((int64_t)blockIdx.x * 256 + threadIdx.x) * 8;
+  if (c >= cols) return;
+  int head = (int)(c / p.hd), which = 0;
+  const int at = (int)(c - (int64_t)head * p.hd), half = p.rope.rot >> 1;
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    if (which == i && head >= p.heads[i]) { head -= p.heads[i]; ++which; }
+  const __nv_bfloat16* d = p.d[which];
+  const int64_t stride = p.d_stride[which];
+  const int col = head * p.hd + at;
+  const bool rotated = which < 2 && at < p.rope.rot, first = at < half;
+  float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (d != nullptr) {
+    for (int r = blockIdx.y; r < p.rows; r += gridDim.y) {
+      float v[8];
+      unpack8(ld8(d + (int64_t)r * stride + col), v);
+      if (!rotated) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[j] += v[j];
+        continue;
+      }
+      float o[8];
+      unpack8(ld8(d + (int64_t)r * stride + (first ? col + half : col - half)), o);
+      int64_t pos = p.rope.positions[r];
+      pos = pos < 0 ? 0 : (pos >= p.rope.max_pos ? p.rope.max_pos - 1 : pos);
+      const float* cs = p.rope.cos_t + pos * half + (first ? at : at - half);
+      const float* sn = p.rope.sin_t + pos * half + (first ? at : at - half);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[j] += first ? v[j] * cs[j] + o[j] * sn[j] : v[j] * cs[j] - o[j] * sn[j];
+    }
+  }
+  float4* out = reinterpret_cast<float4*>(p.part + (int64_t)blockIdx.y * cols + c);
+  out[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+  out[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+}
+__global__ void __launch_bounds__(256) repeated_finish_kernel(const RepeatedArgs p) {
+  pdl_begin();
+  __shared__ float scratch[33];
+  int head = blockIdx.x, which = 0;
+  const int64_t cols = (int64_t)gridDim.x * p.hd;
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    if (which == i && head >= p.heads[i]) { head -= p.heads[i]; ++which; }
+  for (int at = threadIdx.x; at < ((p.hd + 255) & ~255); at += 256) {
+    const int64_t c = (int64_t)blockIdx.x * p.hd + at;
+    const bool on = at < p.hd;
+    float s = 0.f;
+    if (on)
+      for (int i = 0; i < p.slices; ++i) s += p.part[(int64_t)i * cols + c];
+    if (which < 2) {  // a head is at most 256 wide: one trip
+      const float rstd = p.rstd[which][head], w = on ? __bfloat162float(p.w[which][at]) : 0.f;
+      const float xh = on ? __bfloat162float(p.src[c]) * rstd : 0.f;
+      const float dot = block_sum(s * w * xh, scratch) / (float)p.hd;
+      if (on && p.dw_part[which] != nullptr) p.dw_part[which][(int64_t)head * p.hd + at] = s * xh;
+      s = rstd * (s * w - xh * dot);
+    }
+    if (on) {
+      const __nv_bfloat16 hi = __float2bfloat16(s);
+      p.dst[c] = hi;
+      p.dst[p.dst_stride + c] = __float2bfloat16(s - __bfloat162float(hi));
+    }
   }
 }
 
@@ -623,11 +706,12 @@ void launch_rmsnorm_bwd(const void* dy, int64_t dy_stride, const void* dy2, int6
   } while (0)
 
 // heads: a, b; hd 64, 128 or 256; rot a multiple of 16
-void launch_heads_fwd(const void* src, int64_t src_stride, const void* const* w, const int* heads, void* out, float* rstd, int tokens, float eps,
+// src_last: tokens from there on read that row of src (tokens or more: every token its own)
+void launch_heads_fwd(const void* src, int64_t src_stride, const void* const* w, const int* heads, void* out, float* rstd, int tokens, int src_last, float eps,
                       const int64_t* positions, const float* cos_t, const float* sin_t, int64_t max_pos, int hd, int rot, cudaStream_t stream) {
   if (tokens <= 0) return;
   typedef const __nv_bfloat16* In;
-  const HeadsFwdArgs a{(In)src, src_stride, {(In)w[0], (In)w[1]}, {heads[0], heads[1]}, (__nv_bfloat16*)out, rstd, tokens, eps,
+  const HeadsFwdArgs a{(In)src, src_stride, {(In)w[0], (In)w[1]}, {heads[0], heads[1]}, (__nv_bfloat16*)out, rstd, tokens, src_last, eps,
                        HeadsRope{positions, cos_t, sin_t, max_pos, rot}};
   const int64_t blocks = ((int64_t)tokens * (heads[0] + heads[1]) * (hd / 8) + 255) / 256;
   const int grid = (int)(blocks < 16 * kNumSM ? blocks : 16 * kNumSM);
@@ -637,31 +721,44 @@ void launch_heads_fwd(const void* src, int64_t src_stride, const void* const* w,
 
 int heads_bwd_groups(int tokens, int heads) { return heads > 0 ? narrow_grid(tokens * heads) * kNarrowWarps : 0; }
 
-// d / d_stride: [3][2] gradients of the a, b and plain blocks below and from `split` on; partial[i]: heads_bwd_groups rows of hd floats
+static int repeated_slices(int rows) { return rows < 96 ? rows : 96; }
+int64_t repeated_part_floats(int rows, int heads, int hd) { return (int64_t)repeated_slices(rows) * heads * hd; }
+
+// d / d_stride: [3][2] gradients of the a, b and plain blocks below and from `split` on; rstd: [all_tokens * a] then
+// [all_tokens * b]; partial[i]: heads_bwd_groups rows of hd floats, and one more per head with repeated rows.
+// all_tokens > tokens: the gradients of the rest (the second of each pair; the a block's rows follow its first ones)
+// belong to row `tokens` of src, positions go on, and two more rows of dst receive their sum; part: repeated_part_floats.
 void launch_heads_bwd(const void* const* d, const int64_t* d_stride, const int* split, const void* src, int64_t src_stride, const void* const* w,
                       const float* rstd, float* const* partial, void* const* dw, const int* accumulate, const int* heads, void* dst, int64_t dst_stride,
-                      int tokens, const int64_t* positions, const float* cos_t, const float* sin_t, int64_t max_pos, int hd, int rot, cudaStream_t stream) {
+                      int tokens, int all_tokens, float* part, const int64_t* positions, const float* cos_t, const float* sin_t, int64_t max_pos, int hd,
+                      int rot, cudaStream_t stream) {
   if (tokens <= 0) return;
   typedef const __nv_bfloat16* In;
+  const bool repeated = all_tokens > tokens;
   HeadsBwdArgs a{};
+  RepeatedArgs q{};
   int64_t groups = 0;
   for (int i = 0; i < 3; ++i) {
     for (int k = 0; k < 2; ++k) {
       a.d[i][k] = (In)d[2 * i + k];
       a.d_stride[i][k] = d_stride[2 * i + k];
     }
-    a.split[i] = split[i];
-    a.heads[i] = heads[i];
+    q.d[i] = i == 0 ? (d[0] != nullptr ? (In)d[0] + (int64_t)tokens * d_stride[0] : nullptr) : (In)d[2 * i + 1];
+    q.d_stride[i] = d_stride[i == 0 ? 0 : 2 * i + 1];
+    q.heads[i] = a.heads[i] = heads[i];
+    a.split[i] = repeated ? tokens : split[i];
     a.groups[i] = heads_bwd_groups(tokens, heads[i]);
     groups += a.groups[i];
   }
   for (int i = 0; i < 2; ++i) {
-    a.w[i] = (In)w[i];
+    q.w[i] = a.w[i] = (In)w[i];
     a.partial[i] = partial[i];
+    a.rstd[i] = rstd + (i ? (int64_t)all_tokens * heads[0] : 0);
+    q.rstd[i] = a.rstd[i] + (int64_t)tokens * heads[i];
+    q.dw_part[i] = partial[i] != nullptr ? partial[i] + (int64_t)a.groups[i] * hd : nullptr;
   }
   a.src = (In)src;
   a.src_stride = src_stride;
-  a.rstd = rstd;
   a.dst = (__nv_bfloat16*)dst;
   a.dst_stride = dst_stride;
   a.tokens = tokens;
@@ -669,19 +766,50 @@ void launch_heads_bwd(const void* const* d, const int64_t* d_stride, const int* 
   const int grid = (int)((groups * (hd / 8) + 255) / 256);
   count_launch(1);
   SB200_HEADS(heads_bwd_kernel, grid, a);
+  if (repeated) {
+    q.hd = hd;
+    q.rows = all_tokens - tokens;
+    q.slices = repeated_slices(q.rows);
+    q.part = part;
+    q.rope = HeadsRope{positions + tokens, cos_t, sin_t, max_pos, rot};
+    q.src = (In)src + (int64_t)tokens * src_stride;
+    q.dst = a.dst + (int64_t)tokens * dst_stride;
+    q.dst_stride = dst_stride;
+    const int all = heads[0] + heads[1] + heads[2];
+    count_launch(2);
+    launch_pdl(repeated_sum_kernel, dim3((all * hd + 2047) / 2048, q.slices), 256, 0, stream, q);
+    launch_pdl(repeated_finish_kernel, all, 256, 0, stream, q);
+  }
   ColsumJobs jobs{};
   int n = 0;
   for (int i = 0; i < 2; ++i)
     if (partial[i] != nullptr && dw[i] != nullptr) {
       jobs.partial[n] = partial[i];
       jobs.dw[n] = (__nv_bfloat16*)dw[i];
-      jobs.rows[n] = a.groups[i];
+      jobs.rows[n] = a.groups[i] + (repeated ? heads[i] : 0);
       jobs.accumulate[n++] = accumulate[i];
     }
   if (n > 0) {
     count_launch(1);
     launch_pdl(colsum_kernel, dim3((hd + 31) / 32, n), dim3(32, kColsumGroups), 0, stream, jobs, hd);
   }
+}
+
+// dst[0 .. 2): the sum of `rows` rows of d in fp32, as a rounded row and the rest; width a multiple of 8
+void launch_repeated_rows_sum(const void* d, int64_t d_stride, int rows, int width, float* part, void* dst, int64_t dst_stride, cudaStream_t stream) {
+  RepeatedArgs q{};
+  q.d[2] = (const __nv_bfloat16*)d;
+  q.d_stride[2] = d_stride;
+  q.hd = width % 256 == 0 ? 256 : 8;
+  q.heads[2] = width / q.hd;
+  q.rows = rows;
+  q.slices = repeated_slices(rows);
+  q.part = part;
+  q.dst = (__nv_bfloat16*)dst;
+  q.dst_stride = dst_stride;
+  count_launch(2);
+  launch_pdl(repeated_sum_kernel, dim3((width + 2047) / 2048, q.slices), 256, 0, stream, q);
+  launch_pdl(repeated_finish_kernel, q.heads[2], 256, 0, stream, q);
 }
 #undef SB200_HEADS
 

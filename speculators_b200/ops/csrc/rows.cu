@@ -1,0 +1,217 @@
+// Row bookkeeping of the drafts' steps: document intervals, P-EAGLE's sampling and mask, embedding gradients.
+//
+// All of it is latency, not bandwidth: the torch formulations were 10 to 60 launches of 2 us each (and, in the sampler,
+// two host synchronisations per depth) on a few thousand indices.  Single-block kernels scan 8 consecutive entries per
+// thread, 8192 per round, so a packed row of ordinary length takes one round.
+#include "common.cuh"
+
+namespace sb200 {
+namespace rows {
+
+constexpr int kT = 1024, kPer = 8;
+
+// inclusive scan over the block; `scratch`: 32 values
+template <typename Op>
+__device__ __forceinline__ int block_scan(int v, Op op, int* scratch) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v = op(v, u);
+  }
+  __syncthreads();
+  if (lane == 31) scratch[warp] = v;
+  __syncthreads();
+  int before = scratch[0];
+  for (int w = 1; w < warp; ++w) before = op(before, scratch[w]);
+  return warp > 0 ? op(v, before) : v;
+}
+
+// lo / hi of every row under causal + same-document (+ window) masking: equal ids form runs, -1 is padding.
+__global__ void __launch_bounds__(kT) document_interval_kernel(const int64_t* __restrict__ doc, int T, int window, int* __restrict__ lo, int* __restrict__ hi) {
+  pdl_begin();
+  __shared__ int scratch[32], carry;
+  if (threadIdx.x == 0) carry = 0;
+  for (int base = 0; base < T; base += kT * kPer) {
+    const int i0 = base + threadIdx.x * kPer;
+    int start[kPer], last = 0;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const int i = i0 + j;
+      if (i < T && (i == 0 || doc[i] != doc[i - 1])) last = i;
+      start[j] = last;
+    }
+    __syncthreads();  // carry of the round before
+    const int from = carry;
+    const int all = block_scan(last, [](int a, int b) { return max(a, b); }, scratch);
+    // what the threads before this one reached
+    const int up = __shfl_up_sync(0xffffffffu, all, 1);
+    int before = from;
+    if ((threadIdx.x & 31) != 0) before = max(before, up);
+    else for (int w = 0; w < (int)(threadIdx.x >> 5); ++w) before = max(before, scratch[w]);
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const int i = i0 + j;
+      if (i < T) {
+        int l = max(start[j], before);
+        if (window > 0) l = max(l, i - window + 1);
+        lo[i] = doc[i] == -1 ? i : l;
+        hi[i] = i + 1;
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x == kT - 1) carry = max(from, all);
+  }
+}
+
+// Ordered compaction over n candidates: put(rank, i) for every i with keep(i); returns how many (valid in all threads).
+template <typename Keep, typename Put>
+__device__ __forceinline__ int compact(int n, Keep keep, Put put, int* scratch, int* total) {
+  __syncthreads();
+  if (threadIdx.x == 0) *total = 0;
+  for (int base = 0; base < n; base += kT * kPer) {
+    const int i0 = base + threadIdx.x * kPer;
+    unsigned bits = 0;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j)
+      if (i0 + j < n && keep(i0 + j)) bits |= 1u << j;
+    const int mine = __popc(bits);
+    __syncthreads();
+    const int from = *total;
+    const int upto = block_scan(mine, [](int a, int b) { return a + b; }, scratch);
+    int rank = from + upto - mine;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j)
+      if (bits >> j & 1) put(rank++, i0 + j);
+    __syncthreads();
+    if (threadIdx.x == kT - 1) *total = from + upto;
+  }
+  __syncthreads();
+  return *total;
+}
+
+__global__ void __launch_bounds__(kT) compact_kernel(const bool* __restrict__ valid, int T, int64_t* __restrict__ list, int* __restrict__ count) {
+  pdl_begin();
+  __shared__ int scratch[32], total;
+  const int n = compact(T, [&](int i) { return valid[i]; }, [&](int rank, int i) { list[rank] = i; }, scratch, &total);
+  if (threadIdx.x == 0) *count = n;
+}
+
+// One depth of the sampler: the `take` entries of `pool` that `perm` puts first, ascending (all of it as it is without a
+// permutation); their anchors and depths; the successors that are still inside the mask as the next pool.
+__global__ void __launch_bounds__(kT)
+cod_step_kernel(const int64_t* __restrict__ pool, const int64_t* __restrict__ perm, int take, const bool* __restrict__ valid, int T, int depth, int filter_zero,
+                unsigned char* __restrict__ flags, int64_t* __restrict__ picked, int64_t* __restrict__ anchor, int64_t* __restrict__ depths,
+                int64_t* __restrict__ next, int* __restrict__ count) {
+  pdl_begin();
+  __shared__ int scratch[32], total;
+  auto put = [&](int rank, int64_t at) {
+    picked[rank] = at;
+    anchor[rank] = at - depth;
+    depths[rank] = depth;
+  };
+  if (perm != nullptr) {
+    for (int i = threadIdx.x; i < T; i += kT) flags[i] = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < take; i += kT) flags[pool[perm[i]]] = 1;
+    __syncthreads();
+    compact(T, [&](int i) { return flags[i] != 0; }, [&](int rank, int i) { put(rank, i); }, scratch, &total);
+  } else {
+    for (int i = threadIdx.x; i < take; i += kT) put(i, pool[i]);
+  }
+  __syncthreads();
+  auto successor = [&](int i) { const int64_t s = picked[i] + 1; return s >= T ? s - T : s; };
+  const int n = compact(take, [&](int i) { const int64_t s = successor(i); return (s != 0 || !filter_zero) && valid[s]; },
+                        [&](int rank, int i) { next[rank] = successor(i); }, scratch, &total);
+  if (threadIdx.x == 0) *count = n;
+}
+
+// table[depth, anchor] = row - T for the rows of depth >= 1 (the caller has filled it with -1)
+__global__ void __launch_bounds__(256)
+peagle_table_kernel(const int64_t* __restrict__ anchor, const int64_t* __restrict__ depth, const bool* __restrict__ row_valid, int n, int T, int num_depths,
+                    int* __restrict__ table) {
+  pdl_begin();
+  const int r = blockIdx.x * 256 + threadIdx.x;
+  if (r >= n || (row_valid != nullptr && !row_valid[r])) return;
+  const int64_t d = depth[r], a = anchor[r] < 0 ? anchor[r] + T : anchor[r];
+  if (d >= 1 && d < num_depths && a >= 0 && a < T) table[d * T + a] = r - T;
+}
+__global__ void __launch_bounds__(256)
+peagle_spec_kernel(const int64_t* __restrict__ anchor, const int64_t* __restrict__ depth, const bool* __restrict__ row_valid, const int64_t* __restrict__ doc,
+                   const int* __restrict__ doc_lo, int n, int T, int num_depths, int window, const int* __restrict__ table, int* __restrict__ lo,
+                   int* __restrict__ hi, int* __restrict__ extra) {
+  pdl_begin();
+  const int r = blockIdx.x * 256 + threadIdx.x;
+  if (r >= n) return;
+  const int64_t d = depth[r], a0 = anchor[r];
+  const int64_t a = min(max(a0 < 0 ? a0 + T : a0, (int64_t)0), (int64_t)T - 1);
+  const bool pad = doc[a] == -1 || (row_valid != nullptr && !row_valid[r]);
+  int64_t l = doc_lo[a];
+  if (window > 0) l = max(l, a0 + d - window + 1);
+  lo[r] = pad ? 0 : (int)l;
+  hi[r] = pad ? 0 : (int)(a0 + 1);
+  if (extra != nullptr)
+    for (int e = 1; e < num_depths; ++e) extra[(int64_t)r * (num_depths - 1) + e - 1] = d >= e && !pad ? table[(int64_t)e * T + a] : -1;
+}
+
+// Gradient rows of an embedding from ids in ascending order (`order`: where each came from): one block sums the rows of
+// one id in fp32 and stores, or adds to, its row of dw.  Rows of other ids are not touched.
+__global__ void __launch_bounds__(256)
+embedding_bwd_kernel(const int64_t* __restrict__ ids, const int64_t* __restrict__ order, const __nv_bfloat16* __restrict__ d, int64_t d_stride, int n, int H,
+                     int64_t vocab, int64_t padding, __nv_bfloat16* __restrict__ dw, int accumulate) {
+  pdl_begin();
+  const int i = blockIdx.x;
+  const int64_t id = ids[i];
+  if ((i > 0 && ids[i - 1] == id) || id == padding || id < 0 || id >= vocab) return;
+  for (int c = threadIdx.x * 8; c < H; c += 256 * 8) {
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, v[8];
+    for (int j = i; j < n && ids[j] == id; ++j) {
+      unpack8(ld8(d + order[j] * d_stride + c), v);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) acc[u] += v[u];
+    }
+    __nv_bfloat16* out = dw + id * (int64_t)H + c;
+    if (accumulate) {
+      unpack8(ld8(out), v);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) acc[u] = __bfloat162float(__float2bfloat16(acc[u])) + v[u];
+    }
+    st8(out, pack8(acc));
+  }
+}
+
+}  // namespace rows
+
+void launch_document_interval(const int64_t* doc, int T, int window, int* lo, int* hi, cudaStream_t stream) {
+  if (T <= 0) return;
+  count_launch(1);
+  launch_pdl(rows::document_interval_kernel, 1, rows::kT, 0, stream, doc, T, window, lo, hi);
+}
+void launch_compact(const bool* valid, int T, int64_t* list, int* count, cudaStream_t stream) {
+  count_launch(1);
+  launch_pdl(rows::compact_kernel, 1, rows::kT, 0, stream, valid, T, list, count);
+}
+void launch_cod_step(const int64_t* pool, const int64_t* perm, int take, const bool* valid, int T, int depth, int filter_zero, unsigned char* flags,
+                     int64_t* picked, int64_t* anchor, int64_t* depths, int64_t* next, int* count, cudaStream_t stream) {
+  count_launch(1);
+  launch_pdl(rows::cod_step_kernel, 1, rows::kT, 0, stream, pool, perm, take, valid, T, depth, filter_zero, flags, picked, anchor, depths, next, count);
+}
+void launch_peagle_spec(const int64_t* anchor, const int64_t* depth, const bool* row_valid, const int64_t* doc, const int* doc_lo, int n, int T, int num_depths,
+                        int window, int* table, int* lo, int* hi, int* extra, cudaStream_t stream) {
+  if (n <= 0) return;
+  const int grid = (n + 255) / 256;
+  if (extra != nullptr) {
+    count_launch(1);
+    launch_pdl(rows::peagle_table_kernel, grid, 256, 0, stream, anchor, depth, row_valid, n, T, num_depths, table);
+  }
+  count_launch(1);
+  launch_pdl(rows::peagle_spec_kernel, grid, 256, 0, stream, anchor, depth, row_valid, doc, doc_lo, n, T, num_depths, window, (const int*)table, lo, hi, extra);
+}
+void launch_embedding_bwd(const int64_t* ids, const int64_t* order, const void* d, int64_t d_stride, int n, int H, int64_t vocab, int64_t padding, void* dw,
+                          int accumulate, cudaStream_t stream) {
+  if (n <= 0) return;
+  count_launch(1);
+  launch_pdl(rows::embedding_bwd_kernel, n, 256, 0, stream, ids, order, (const __nv_bfloat16*)d, d_stride, n, H, vocab, padding, (__nv_bfloat16*)dw, accumulate);
+}
+
+}  // namespace sb200

@@ -1,0 +1,107 @@
+"""Row bookkeeping kernels (document intervals, P-EAGLE sampling and mask, repeated rows, embedding gradients) against the
+CPU formulations and fp32 autograd."""
+
+import pytest
+import torch
+
+from speculators_b200 import ops
+from speculators_b200.models.eagle3.attention import causal_document_interval
+from speculators_b200.models.peagle.attention import peagle_attn_spec
+from speculators_b200.models.peagle.data import generate_cod_sample_indices
+
+pytestmark = pytest.mark.gpu
+
+
+def _docs(T, n):
+    cuts = torch.randint(0, T, (n,)).sort().values
+    doc = torch.bucketize(torch.arange(T), cuts, right=True)
+    doc[T - T // 9:] = -1
+    return doc
+
+
+# less than one vector, around the 8192 entries of a round, several rounds
+@pytest.mark.parametrize("T,n", [(1, 1), (77, 3), (8192, 5), (8193, 40), (20001, 2)])
+@pytest.mark.parametrize("window", [None, 50])
+def test_document_interval(T, n, window):
+    torch.manual_seed(T)
+    doc = _docs(T, n)
+    for a, b in zip(causal_document_interval(doc.cuda(), window), causal_document_interval(doc, window)):
+        assert torch.equal(a.cpu(), b)
+
+
+@pytest.mark.parametrize("T,share,max_anchors,filter_zero", [(1, 1.0, None, True), (300, 0.5, None, True), (300, 0.9, 40, False), (9000, 0.6, 4000, True), (64, 0.0, None, True)])
+def test_sampler_and_mask(T, share, max_anchors, filter_zero, monkeypatch):
+    torch.manual_seed(T)
+    mask = (torch.rand(1, T) < share).float()
+    doc = _docs(T, 4)
+
+    def perm(n, device=None):
+        g = torch.Generator().manual_seed(n)
+        return torch.rand(n, generator=g).argsort().to(device)
+
+    monkeypatch.setattr(torch, "randperm", perm)
+    kw = dict(num_depths=6, max_anchors=max_anchors, filter_position_zero=filter_zero)
+    a, d = generate_cod_sample_indices(T, mask.cuda(), **kw)
+    ra, rd = generate_cod_sample_indices(T, mask, **kw)
+    assert torch.equal(a.cpu(), ra) and torch.equal(d.cpu(), rd)
+    for window, valid in ((None, None), (20, None), (None, torch.rand(len(ra)) < 0.8)):
+        got = peagle_attn_spec(a, d, doc.cuda(), 6, window, None if valid is None else valid.cuda())
+        want = peagle_attn_spec(ra, rd, doc, 6, window, valid)
+        assert torch.equal(got.lo.cpu(), want.lo) and torch.equal(got.hi.cpu(), want.hi)
+        assert (got.extra_idx is None) == (want.extra_idx is None)
+        assert got.extra_idx is None or torch.equal(got.extra_idx.cpu(), want.extra_idx)
+
+
+@pytest.mark.parametrize("T,n,hd,rot", [(1, 2, 64, 64), (130, 131, 128, 128), (300, 900, 128, 64), (40, 77, 256, 256)])
+def test_repeated_rows(T, n, hd, rot):
+    """Shared rows through heads and residual against the same rows laid out; the two gradient rows hold the sum to fp32's digits."""
+    torch.manual_seed(n)
+    heads = (4, 2, 2)
+    src = torch.randn(T + 2, 8 * hd, device="cuda").bfloat16()
+    src[T + 1] = src[T]
+    pos = torch.randint(0, 500, (n,), device="cuda")
+    angle = torch.rand(500, rot // 2, device="cuda")
+    wa, wb = ((torch.rand(hd, device="cuda") + 0.5).bfloat16().requires_grad_() for _ in range(2))
+    x = src.clone().requires_grad_()
+    out = ops.norm_rope_heads(x, wa, wb, 1e-6, pos, angle.cos(), angle.sin(), heads, hd, rot, split=T, repeated=True)
+    res = ops.repeat_rows(x, n)
+    grads = [torch.randn(o.shape, device="cuda").bfloat16() for o in (*out, res)]
+    torch.autograd.backward([*out, res], grads)
+
+    xf = src.float().requires_grad_()
+    wf = [w.detach().float().requires_grad_() for w in (wa, wb)]
+    laid = torch.cat([xf[:T], xf[T:T + 1].expand(n - T, -1)])
+    rotated, col = [], 0
+    for h, w in zip(heads, (*wf, None)):
+        b = laid[:, col: col + h * hd].reshape(n, h, hd)
+        col += h * hd
+        if w is not None:
+            b = ops._rms_norm_ref(b, w, 1e-6)
+            b = ops._rope_ref(b.reshape(n, -1), pos, angle.cos(), angle.sin(), h, hd, rot, 1.0).view(n, h, hd)
+        rotated.append(b)
+    want = (rotated[0], rotated[1][:T], rotated[1][T:], rotated[2][:T], rotated[2][T:], laid)
+    torch.autograd.backward(want, [g.float() for g in grads])
+    for a, b in zip((*out, res), want):
+        assert a.shape == b.shape and (a.float() - b).abs().max() <= 0.02 * b.abs().max()
+    scale = xf.grad.abs().max()
+    assert (x.grad[:T].float() - xf.grad[:T]).abs().max() <= 0.02 * scale
+    assert (x.grad[T].float() + x.grad[T + 1].float() - xf.grad[T]).abs().max() <= 0.02 * scale
+    for a, b in zip((wa, wb), wf):
+        assert (a.grad.float() - b.grad).abs().max() <= 0.02 * b.grad.abs().max() + 0.02
+
+
+@pytest.mark.parametrize("n,H,vocab,padding", [(1, 8, 5, None), (700, 264, 50, 3), (64, 4096, 1000, None)])
+@pytest.mark.parametrize("attached", [False, True])
+def test_embedding_gradient(n, H, vocab, padding, attached):
+    torch.manual_seed(n)
+    w = torch.randn(vocab, H, device="cuda").bfloat16().requires_grad_()
+    if attached:
+        w._flat_grad, w._grad_fresh = torch.full_like(w, float("nan")), True
+    ids = torch.randint(0, vocab, (n,), device="cuda")
+    d = torch.randn(n, H, device="cuda").bfloat16()
+    wf = w.detach().float().requires_grad_()
+    for _ in range(2):
+        ops.embedding(ids, w, padding).backward(d)
+        torch.nn.functional.embedding(ids, wf, padding).backward(d.float())
+    got = w._flat_grad if attached else w.grad
+    assert (got.float() - wf.grad).abs().max() <= 0.01 * wf.grad.abs().max()
