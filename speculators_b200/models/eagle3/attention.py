@@ -50,8 +50,7 @@ def ttt_attn_spec(document_ids: torch.Tensor, ttt_step: int, sliding_window: int
     T = lo.shape[0]
     extra = None
     if ttt_step > 0:
-        idx = torch.arange(T, device=lo.device, dtype=torch.int32)
-        extra = torch.stack([idx + j * T for j in range(ttt_step)], dim=1).contiguous()
+        extra = torch.arange(ttt_step * T, device=lo.device, dtype=torch.int32).view(ttt_step, T).t().contiguous()
     return AttnSpec(lo=lo, hi=hi, extra_idx=extra)
 
 

@@ -185,7 +185,7 @@ class Eagle3DraftModel(DraftVocabMixin, SpeculatorModel):
             with torch.no_grad():
                 vl = verifier_last_hidden_states.reshape(T, -1).to(dtype)
                 targets = ops.linear(self.verifier_norm(vl), self.verifier_lm_head.weight)  # [T, Vd]
-            loss = torch.zeros((), device=device, dtype=torch.float32)
+            loss = None
             prev_correct = (
                 loss_mask.to(torch.bool).clone() if loss_mask is not None
                 else torch.ones(1, T, device=device, dtype=torch.bool)
@@ -209,7 +209,7 @@ class Eagle3DraftModel(DraftVocabMixin, SpeculatorModel):
                 else:
                     hidden = layer(hidden, positions, self.rotary_emb, spec, past[li])
             if self.config.norm_output:
-                hidden = head_in = self.norm(hidden)
+                hidden, head_in = ops.rms_norm_pair(hidden, self.norm.weight, self.norm.variance_epsilon)
             else:
                 head_in = self.norm(hidden)
             fused = None
@@ -217,27 +217,30 @@ class Eagle3DraftModel(DraftVocabMixin, SpeculatorModel):
                 # lm_head GEMM with the loss's forward reduction in its epilogue (CUDA, bf16, KL / CE)
                 fused = compute_metrics_from_hidden(
                     head_in, self.lm_head.weight, targets.unsqueeze(0), loss_mask, prev_correct, step, ttt_step_loss_decay,
-                    loss_config=loss_config,
+                    loss_config=loss_config, earlier=loss,
                 )
             if fused is None:
                 logits = ops.linear(head_in, self.lm_head.weight)
                 if return_loss:
                     fused = compute_metrics(
                         logits.unsqueeze(0), targets.unsqueeze(0), loss_mask, prev_correct, step,
-                        ttt_step_loss_decay, loss_config=loss_config,
+                        ttt_step_loss_decay, loss_config=loss_config, earlier=loss,
                     )
             if return_loss:
-                loss = loss + fused[0]
+                loss = fused[0]
                 metrics.update(fused[1])
 
             if return_draft_tokens:
                 draft_tokens.append(torch.argmax(logits.detach(), dim=-1).unsqueeze(0))
             ids = padded_ids[1 + step : 1 + step + T]
-            positions = positions + 1
+            if step + 1 < ttt_steps:
+                positions = positions + 1
 
         if return_loss:
+            if loss is None:  # no passes
+                loss = torch.zeros((), device=device)
             metrics["loss_sum"] = loss.detach().clone()
-            metrics["loss_total"] = torch.ones((), device=device)
+            metrics["loss_total"] = metrics["loss_0_total"] if ttt_steps else torch.ones((), device=device)
             return draft_tokens, loss, metrics
         return draft_tokens
 

@@ -45,11 +45,12 @@ def _single_fused_primitive(loss_config: LossConfig) -> tuple[str, float] | None
     return (name, float(weight)) if name in _PRIMITIVES and _is_fused(fn) else None
 
 
-def _compute_metrics_fused(logits, targets, loss_mask, prev_correct, ttt_step: int, decay: float, op: str, weight: float, head=None):
+def _compute_metrics_fused(logits, targets, loss_mask, prev_correct, ttt_step: int, decay: float, op: str, weight: float, head=None, earlier=None):
     """CUDA fast path for one fused loss term: row-loss kernel + one tail kernel (masked
     mean, decay, accuracy counters, ``prev_correct`` update) instead of ~30 small ops.  With
     ``head = (hidden [T, H], lm_head weight)`` instead of ``logits`` the head's GEMM and the
-    forward reduction of the loss run as one kernel (``None`` is returned if that does not apply)."""
+    forward reduction of the loss run as one kernel (``None`` is returned if that does not apply).
+    The first result is the pass's loss added to ``earlier`` (the loss of the passes before)."""
     from speculators_b200 import ops
     from speculators_b200.losses.utils import _REDUCTION_EPS
 
@@ -58,21 +59,20 @@ def _compute_metrics_fused(logits, targets, loss_mask, prev_correct, ttt_step: i
     mask_u8 = loss_mask.reshape(-1)[ttt_step:]
     if mask_u8.dtype not in (torch.bool, torch.uint8):
         mask_u8 = mask_u8 != 0
-    prev_flat = prev_correct.reshape(-1)
-    active = mask_u8.bool() | prev_flat[:rows]
+    mask_u8, prev_flat, targets = mask_u8.contiguous(), prev_correct.reshape(-1), targets.reshape(targets.shape[1], -1)
     if head is None:
-        row_loss, pred, tgt = ops.fused_row_loss_raw(op, logits.reshape(T, -1), targets.reshape(targets.shape[1], -1), ttt_step, rows, active)
+        loss, stats = ops.ttt_step_loss(op, logits.reshape(T, -1), targets, earlier, ttt_step, rows, mask_u8, prev_flat, decay * weight, _REDUCTION_EPS)
+        step_loss, one = stats[0], stats[4]
     else:
-        fused = ops.lm_head_loss_raw(op, head[0], head[1], targets.reshape(targets.shape[1], -1), ttt_step, rows, active)
-        if fused is None:
+        if not ops.lm_head_loss_ok(op, *head, targets):
             return None
-        row_loss, pred, tgt = fused
-    out = ops.ttt_step_tail(row_loss, pred, tgt, mask_u8.contiguous(), prev_flat, decay, _REDUCTION_EPS)
-    loss = out[0] * weight if weight != 1.0 else out[0]
-    stats = out.detach()
-    one = torch.ones((), device=row_loss.device)
+        row_loss, pred, tgt = ops.lm_head_loss_raw(op, *head, targets, ttt_step, rows, mask_u8.bool() | prev_flat[:rows])
+        out = ops.ttt_step_tail(row_loss, pred, tgt, mask_u8, prev_flat, decay, _REDUCTION_EPS)
+        loss = out[0] * weight
+        stats, step_loss, one = out.detach(), loss.detach(), torch.ones((), device=out.device)
+        loss = loss if earlier is None else earlier + loss
     metrics = {
-        f"loss_{ttt_step}_sum": stats[0] * weight if weight != 1.0 else stats[0], f"loss_{ttt_step}_total": one,
+        f"loss_{ttt_step}_sum": step_loss, f"loss_{ttt_step}_total": one,
         f"full_acc_{ttt_step}_sum": stats[1], f"full_acc_{ttt_step}_total": stats[2],
         f"cond_acc_{ttt_step}_sum": stats[1], f"cond_acc_{ttt_step}_total": stats[3],
     }
@@ -80,7 +80,7 @@ def _compute_metrics_fused(logits, targets, loss_mask, prev_correct, ttt_step: i
 
 
 def compute_metrics_from_hidden(hidden, head_weight, targets, loss_mask, prev_correct, ttt_step: int, ttt_step_loss_decay: float,
-                                loss_config: LossConfig | None = None):
+                                loss_config: LossConfig | None = None, earlier=None):
     """``compute_metrics`` of ``hidden @ head_weight.T`` without a separate pass over the
     logits: the lm_head GEMM's epilogue reduces each tile for the loss.  Returns ``None`` when
     that path does not apply (not CUDA bf16, a loss other than one fused KL / CE term, ...);
@@ -94,17 +94,20 @@ def compute_metrics_from_hidden(hidden, head_weight, targets, loss_mask, prev_co
     if single is None:
         return None
     return _compute_metrics_fused(None, targets, loss_mask, prev_correct, ttt_step, float(ttt_step_loss_decay) ** ttt_step, *single,
-                                  head=(hidden, head_weight))
+                                  head=(hidden, head_weight), earlier=earlier)
 
 
-def compute_metrics(logits, targets, loss_mask, prev_correct, ttt_step: int, ttt_step_loss_decay: float, loss_config: LossConfig | None = None):
-    """Returns ``(step_loss, metrics)``; updates ``prev_correct`` in place."""
+def compute_metrics(logits, targets, loss_mask, prev_correct, ttt_step: int, ttt_step_loss_decay: float, loss_config: LossConfig | None = None,
+                    earlier=None):
+    """Returns ``(step_loss, metrics)``, the loss added to that of the ``earlier`` passes when given; updates
+    ``prev_correct`` in place."""
     if loss_config is None:
         loss_config = {"kl_div": (kl_div_loss, 1.0)}
     if USE_FUSED_TAIL and logits.is_cuda and logits.dtype == torch.bfloat16 and loss_mask is not None and prev_correct is not None and prev_correct.dtype == torch.bool:
         single = _single_fused_primitive(loss_config)
         if single is not None and prev_correct.is_contiguous():
-            return _compute_metrics_fused(logits, targets, loss_mask, prev_correct, ttt_step, float(ttt_step_loss_decay) ** ttt_step, *single)
+            return _compute_metrics_fused(logits, targets, loss_mask, prev_correct, ttt_step, float(ttt_step_loss_decay) ** ttt_step, *single,
+                                          earlier=earlier)
     T = logits.shape[1]
     rows = T - ttt_step
     device = logits.device
@@ -139,4 +142,4 @@ def compute_metrics(logits, targets, loss_mask, prev_correct, ttt_step: int, ttt
     metrics[f"full_acc_{ttt_step}_total"] = full_t
     metrics[f"cond_acc_{ttt_step}_sum"] = cond_c
     metrics[f"cond_acc_{ttt_step}_total"] = cond_t
-    return total, metrics
+    return (total if earlier is None else earlier + total), metrics

@@ -272,8 +272,7 @@ class Attention(nn.Module):
             past.append((k, v))
             k_ctx, v_ctx = past[0]
             if len(past) > 1:
-                k_ext = torch.cat([kv[0] for kv in past[1:]], dim=0)
-                v_ext = torch.cat([kv[1] for kv in past[1:]], dim=0)
+                k_ext, v_ext = past[1] if len(past) == 2 else (torch.cat([kv[i] for kv in past[1:]], dim=0) for i in range(2))
                 out = ops.masked_attention(q, k_ctx, v_ctx, spec, k_ext, v_ext, scale=self.scaling)
             else:
                 out = ops.masked_attention(q, k_ctx, v_ctx, spec, scale=self.scaling)

@@ -39,6 +39,7 @@ __all__ = [
     "grouped_linear_ok",
     "linear",
     "linear_swiglu",
+    "lm_head_loss_ok",
     "lm_head_loss_raw",
     "masked_attention",
     "matmul_nn",
@@ -50,12 +51,14 @@ __all__ = [
     "repeat_rows",
     "rms_norm",
     "rms_norm_fork",
+    "rms_norm_pair",
     "rope_",
     "rope_split",
     "split_gated_query",
     "sum_of_squares",
     "swiglu",
     "token_cross_entropy",
+    "ttt_step_loss",
     "ttt_step_tail",
 ]
 
@@ -409,6 +412,36 @@ def _norm_backward(dy, dy2, x2, weight, rstd, residual_grad, need_dx: bool, need
     if need_dx or need_dw:
         native().rmsnorm_bwd(dy, dy2, x2, weight, rstd, residual_grad if need_dx else None, dx, dw, accumulate, centred)
     return dx, None if attached else dw
+
+
+class _RMSNormPairFn(torch.autograd.Function):
+    """Norm of ``x`` handed out twice, for two consumers whose gradients meet in the backward kernel."""
+
+    @staticmethod
+    def forward(ctx, x, weight, eps):
+        y = torch.empty_like(x)
+        rstd = torch.empty(x.shape[0], dtype=torch.float32, device=x.device)
+        native().norm_fwd(x, weight, None, y, rstd, eps, False)
+        ctx.save_for_backward(x, weight, rstd)
+        ctx.set_materialize_grads(False)
+        return y, y.view_as(y)
+
+    @staticmethod
+    def backward(ctx, d1, d2):
+        d1, d2 = (d1, d2) if d1 is not None else (d2, None)
+        if d1 is None:
+            return None, None, None
+        x, weight, rstd = ctx.saved_tensors
+        H = x.shape[1]
+        return *_norm_backward(_grad_rows(d1, H), _grad_rows(d2, H), x, weight, rstd, None, ctx.needs_input_grad[0], ctx.needs_input_grad[1], False), None
+
+
+def rms_norm_pair(x: torch.Tensor, weight: torch.Tensor, eps: float) -> tuple[torch.Tensor, torch.Tensor]:
+    """``rms_norm(x)`` twice, for two consumers."""
+    if _norm_native(x) and x.dim() == 2 and x.is_contiguous() and torch.is_grad_enabled() and x.requires_grad:
+        return _RMSNormPairFn.apply(x, weight, eps)
+    y = rms_norm(x, weight, eps)
+    return y, y
 
 
 class _RMSNormFn(torch.autograd.Function):
@@ -908,6 +941,15 @@ class _LmHeadLossFn(torch.autograd.Function):
 FUSED_HEAD_OPS = ("kl_div", "ce")
 
 
+def lm_head_loss_ok(op: str, hidden: torch.Tensor, weight: torch.Tensor, targets: torch.Tensor) -> bool:
+    """Whether the fused head of ``lm_head_loss_raw`` applies and is switched on."""
+    import os
+
+    return (op in FUSED_HEAD_OPS and os.environ.get("SB200_FUSED_HEAD", "0") == "1" and own_gemm_enabled()
+            and _gemm_operand_ok(hidden) and _gemm_operand_ok(weight) and _gemm_operand_ok(targets)
+            and weight.shape[0] % 8 == 0 and hidden.shape[0] > 128)
+
+
 def lm_head_loss_raw(op: str, hidden: torch.Tensor, weight: torch.Tensor, targets: torch.Tensor, shift: int, rows: int, active):
     """Per-row loss between ``(hidden @ weight.T)[r]`` and ``targets[r + shift]`` for ``r < rows``
     plus both argmaxes (int32), like ``fused_row_loss_raw`` on the product; ``None`` when the
@@ -916,11 +958,7 @@ def lm_head_loss_raw(op: str, hidden: torch.Tensor, weight: torch.Tensor, target
     fused kernel measured 0.466 ms against 0.443 ms for the GEMM followed by the row-loss
     kernel (its statistics epilogue holds the tensor pipe at 70 % active against 88 % for the
     plain store epilogue), so the two-kernel form is the default."""
-    import os
-
-    if (op not in FUSED_HEAD_OPS or not own_gemm_enabled() or os.environ.get("SB200_FUSED_HEAD", "0") != "1"
-            or not (_gemm_operand_ok(hidden) and _gemm_operand_ok(weight) and _gemm_operand_ok(targets))
-            or weight.shape[0] % 8 or hidden.shape[0] <= 128):
+    if not lm_head_loss_ok(op, hidden, weight, targets):
         return None
     return _LmHeadLossFn.apply(hidden, weight, targets, LOSS_OPS[op], shift, rows, active)
 
@@ -928,7 +966,8 @@ def lm_head_loss_raw(op: str, hidden: torch.Tensor, weight: torch.Tensor, target
 class _StepTailFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, row_loss, pred, target, mask, prev, decay, eps):
-        out, weight = native().step_tail(row_loss, pred, target, mask, prev, decay, eps)
+        out, weight, _ = native().step_tail(row_loss, pred, target, mask, prev, decay, eps, None)
+        out = out[:4]
         ctx.save_for_backward(weight)
         ctx.mark_dirty(prev)
         ctx.mark_non_differentiable(prev)
@@ -938,6 +977,39 @@ class _StepTailFn(torch.autograd.Function):
     def backward(ctx, dout, _dprev):
         (weight,) = ctx.saved_tensors
         return weight * dout[0], None, None, None, None, None, None
+
+
+class _StepLossFn(torch.autograd.Function):
+    """Row loss and tail of one training-time-test pass: two launches forward, one backward.  As separate functions autograd
+    put a zero fill in front of every result that is not differentiated, and a copy and a product around the loss itself:
+    fourteen launches more in each pass, on steps whose kernels take 2 us."""
+
+    @staticmethod
+    def forward(ctx, logits, targets, earlier, op, shift, rows, mask, prev, decay, eps):
+        row_loss, stats, pred, tgt = native().loss_fwd_either(op, logits, targets, mask, prev, shift, rows)
+        out, weight, total = native().step_tail(row_loss, pred, tgt, mask, prev, decay, eps, earlier)
+        ctx.save_for_backward(logits, targets, stats, weight)
+        ctx.cfg = (op, shift, rows)
+        ctx.mark_non_differentiable(out)
+        ctx.set_materialize_grads(False)
+        return total, out
+
+    @staticmethod
+    def backward(ctx, dtotal, _dout):
+        if dtotal is None:
+            return (None,) * 10
+        logits, targets, stats, weight = ctx.saved_tensors
+        op, shift, rows = ctx.cfg
+        d = native().loss_bwd_scaled(op, logits, targets, weight, dtotal.float(), stats, shift, rows)
+        return d, None, dtotal if ctx.needs_input_grad[2] else None, None, None, None, None, None, None, None
+
+
+def ttt_step_loss(op: str, logits, targets, earlier, shift: int, rows: int, mask, prev_correct, decay: float, eps: float):
+    """``fused_row_loss_raw`` over the rows marked in ``mask`` or ``prev_correct`` followed by ``ttt_step_tail`` (CUDA, bf16
+    logits).  Returns ``(earlier + loss, out)`` with ``out`` = loss, correct, total, cond_total, 1; ``earlier``: the loss of
+    the passes before or ``None``; the loss itself is differentiable through the first result."""
+    logits, targets = (t if t.stride(-1) == 1 else t.contiguous() for t in (logits, targets))
+    return _StepLossFn.apply(logits, targets, earlier, LOSS_OPS[op], shift, rows, mask, prev_correct, float(decay), float(eps))
 
 
 def ttt_step_tail(row_loss, pred_ids, target_ids, mask, prev_correct, decay: float, eps: float):

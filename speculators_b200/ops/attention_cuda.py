@@ -73,7 +73,7 @@ class _MaskedAttentionFn(torch.autograd.Function):
         dq, dk, dv, dke, dve = _ext.lib().attn_bwd(
             _rows_ok(dout), q, k, v, out, lse2, lo, hi, k_ext, v_ext, ext_idx, ctx.scale, impl, status, ctx.block[0], ctx.block[1])
         if ext_idx is not None:
-            return dq, dk, dv, None, None, dke.to(q.dtype), dve.to(q.dtype), None, None, None, None
+            return dq, dk, dv, None, None, dke, dve, None, None, None, None
         return dq, dk, dv, None, None, None, None, None, None, None, None
 
 

@@ -49,9 +49,9 @@ void launch_moe_combine_bwd(const void*, const void*, const int*, const int*, co
 int launch_gemm_grouped_swiglu(const void*, const void*, void*, void*, int, int, int, int64_t, int64_t, const int*, const int*, int, int*, cudaStream_t);
 void launch_rope(void*, const int64_t*, const float*, const float*, int64_t, int, int, int, int64_t,
                  int64_t, float, cudaStream_t);
-int launch_loss_fwd(int, const void*, const void*, const uint8_t*, const int64_t*, float*, float*, int*,
+int launch_loss_fwd(int, const void*, const void*, const uint8_t*, const uint8_t*, const int64_t*, float*, float*, int*,
                     int*, int, int, int64_t, int64_t, int, cudaStream_t);
-int launch_loss_bwd(int, const void*, const void*, const float*, const float*, void*, int, int, int,
+int launch_loss_bwd(int, const void*, const void*, const float*, const float*, const float*, void*, int, int, int,
                     int64_t, int64_t, int64_t, int, cudaStream_t);
 int64_t launch_count();
 int launch_gemm_tn_tcgen05(const void*, const void*, void*, const void*, int, int, int, int64_t, int64_t, int64_t, int64_t, int,
@@ -84,7 +84,7 @@ int launch_tp_reduce_broadcast(int, int, int, int, const void*, void* const*, vo
 int hs_ring_ctl_words_per_slot();
 int launch_hs_push(const void*, int64_t, void*, uint32_t*, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t*, int*, cudaStream_t);
 int launch_hs_pop(void*, int64_t, const void*, uint32_t*, uint32_t, uint32_t, uint32_t*, int*, cudaStream_t);
-void launch_step_tail(const float*, const int*, const int*, const uint8_t*, uint8_t*, int, float, float, float*, float*, cudaStream_t);
+void launch_step_tail(const float*, const int*, const int*, const uint8_t*, uint8_t*, int, float, float, float*, float*, const float*, float*, cudaStream_t);
 void launch_sumsq(const void*, int, int64_t, float*, float*, int, cudaStream_t);
 void launch_set_hyper(float*, const float*, cudaStream_t);
 void launch_adamw(float*, float*, float*, const void*, int, void*, int64_t, const float*,
@@ -497,10 +497,14 @@ void rope_(Tensor x, const Tensor& positions, const Tensor& cos_t, const Tensor&
                      cos_t.size(0), (float)sign, cur_stream());
 }
 
-std::tuple<Tensor, Tensor, Tensor, Tensor> loss_fwd(int64_t op, const Tensor& logits,
-                                                    const Tensor& targets,
-                                                    const c10::optional<Tensor>& active,
-                                                    int64_t shift, int64_t rows) {
+const uint8_t* row_flags(const c10::optional<Tensor>& t, int64_t rows) {
+  if (!t.has_value()) return nullptr;
+  TORCH_CHECK((t->scalar_type() == at::kBool || t->scalar_type() == at::kByte) && t->is_contiguous() && t->numel() >= rows, "bool / uint8 row flags expected");
+  return reinterpret_cast<const uint8_t*>(t->data_ptr());
+}
+
+std::tuple<Tensor, Tensor, Tensor, Tensor> loss_fwd_either(int64_t op, const Tensor& logits, const Tensor& targets, const c10::optional<Tensor>& active,
+                                                           const c10::optional<Tensor>& also, int64_t shift, int64_t rows) {
   TORCH_CHECK(logits.is_cuda() && targets.is_cuda());
   TORCH_CHECK(logits.scalar_type() == at::kBFloat16 && targets.scalar_type() == at::kBFloat16);
   TORCH_CHECK(logits.dim() == 2 && targets.dim() == 2 && logits.stride(1) == 1 &&
@@ -512,19 +516,17 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> loss_fwd(int64_t op, const Tensor& lo
   Tensor stats = at::empty({5, rows}, fopt);
   Tensor am_d = at::empty({rows}, logits.options().dtype(at::kInt));
   Tensor am_t = at::empty({rows}, logits.options().dtype(at::kInt));
-  const uint8_t* act = nullptr;
-  if (active.has_value()) {
-    TORCH_CHECK((active->scalar_type() == at::kBool || active->scalar_type() == at::kByte) &&
-                active->is_contiguous() && active->numel() == rows);
-    act = reinterpret_cast<const uint8_t*>(active->data_ptr());
-  }
-  const int rc = sb200::launch_loss_fwd((int)op, logits.data_ptr(), targets.data_ptr(), act, nullptr,
+  const int rc = sb200::launch_loss_fwd((int)op, logits.data_ptr(), targets.data_ptr(), row_flags(active, rows), row_flags(also, rows), nullptr,
                                         loss.data_ptr<float>(), stats.data_ptr<float>(),
                                         am_d.data_ptr<int>(), am_t.data_ptr<int>(), (int)rows,
                                         (int)logits.size(1), logits.stride(0), targets.stride(0),
                                         (int)shift, cur_stream());
   TORCH_CHECK(rc == 0, "loss_fwd: unknown op ", op);
   return {loss, stats, am_d, am_t};
+}
+std::tuple<Tensor, Tensor, Tensor, Tensor> loss_fwd(int64_t op, const Tensor& logits, const Tensor& targets, const c10::optional<Tensor>& active, int64_t shift,
+                                                    int64_t rows) {
+  return loss_fwd_either(op, logits, targets, active, c10::nullopt, shift, rows);
 }
 
 // ---- grouped (mixture-of-experts) products ----------------------------------------------------
@@ -641,15 +643,16 @@ std::tuple<Tensor, Tensor> ce_label_fwd(const Tensor& logits, const Tensor& labe
     TORCH_CHECK((keep->scalar_type() == at::kBool || keep->scalar_type() == at::kByte) && keep->is_contiguous() && keep->numel() == rows);
     act = reinterpret_cast<const uint8_t*>(keep->data_ptr());
   }
-  const int rc = sb200::launch_loss_fwd(3, logits.data_ptr(), nullptr, act, labels.data_ptr<int64_t>(), loss.data_ptr<float>(),
+  const int rc = sb200::launch_loss_fwd(3, logits.data_ptr(), nullptr, act, nullptr, labels.data_ptr<int64_t>(), loss.data_ptr<float>(),
                                         stats.data_ptr<float>(), nullptr, nullptr, (int)rows, (int)logits.size(1),
                                         logits.stride(0), logits.stride(0), 0, cur_stream());
   TORCH_CHECK(rc == 0, "ce_label_fwd failed (", rc, ")");
   return {loss, stats};
 }
 
-Tensor loss_bwd(int64_t op, const Tensor& logits, const Tensor& targets, const Tensor& grad_out,
-                const Tensor& stats, int64_t shift, int64_t rows) {
+Tensor loss_bwd_scaled(int64_t op, const Tensor& logits, const Tensor& targets, const Tensor& grad_out, const c10::optional<Tensor>& grad_scale,
+                       const Tensor& stats, int64_t shift, int64_t rows) {
+  TORCH_CHECK(!grad_scale.has_value() || (grad_scale->is_cuda() && grad_scale->scalar_type() == at::kFloat && grad_scale->numel() == 1));
   TORCH_CHECK(grad_out.scalar_type() == at::kFloat && grad_out.is_contiguous() &&
               grad_out.numel() == rows);
   TORCH_CHECK(stats.scalar_type() == at::kFloat && stats.is_contiguous() && stats.size(0) == 5 &&
@@ -658,10 +661,13 @@ Tensor loss_bwd(int64_t op, const Tensor& logits, const Tensor& targets, const T
   Tensor d = at::empty({logits.size(0), logits.size(1)}, logits.options());
   const int rc = sb200::launch_loss_bwd(
       (int)op, logits.data_ptr(), targets.data_ptr(), grad_out.data_ptr<float>(),
-      stats.data_ptr<float>(), d.data_ptr(), (int)rows, (int)logits.size(0), (int)logits.size(1),
+      grad_scale.has_value() ? grad_scale->data_ptr<float>() : nullptr, stats.data_ptr<float>(), d.data_ptr(), (int)rows, (int)logits.size(0), (int)logits.size(1),
       logits.stride(0), targets.stride(0), d.stride(0), (int)shift, cur_stream());
   TORCH_CHECK(rc == 0, "loss_bwd: unknown op ", op);
   return d;
+}
+Tensor loss_bwd(int64_t op, const Tensor& logits, const Tensor& targets, const Tensor& grad_out, const Tensor& stats, int64_t shift, int64_t rows) {
+  return loss_bwd_scaled(op, logits, targets, grad_out, c10::nullopt, stats, shift, rows);
 }
 
 void sumsq(const Tensor& g, Tensor out, bool accumulate) {
@@ -784,8 +790,10 @@ int64_t fused_optim_ctl_words() { return sb200::fused_optim_ctl_words(); }
 // ---- tail of a training-time-test pass --------------------------------------------------------
 // row_loss fp32[rows], pred / target int32[rows], mask uint8[rows] (0 / non-0), prev uint8 or bool [rows] (updated in place).
 // Returns (out fp32[4] = loss, correct, total, cond_total; weight fp32[rows] = d loss / d row_loss).
-std::tuple<Tensor, Tensor> step_tail(const Tensor& row_loss, const Tensor& pred, const Tensor& target, const Tensor& mask, Tensor prev,
-                                     double decay, double eps) {
+// -> (out float[5]: loss, correct, total, cond_total, 1; weight float[rows]; earlier + loss)
+std::tuple<Tensor, Tensor, Tensor> step_tail(const Tensor& row_loss, const Tensor& pred, const Tensor& target, const Tensor& mask, Tensor prev,
+                                             double decay, double eps, const c10::optional<Tensor>& earlier) {
+  TORCH_CHECK(!earlier.has_value() || (earlier->is_cuda() && earlier->scalar_type() == at::kFloat && earlier->numel() == 1));
   const int64_t rows = row_loss.numel();
   TORCH_CHECK(row_loss.is_cuda() && row_loss.scalar_type() == at::kFloat && row_loss.is_contiguous());
   TORCH_CHECK(pred.scalar_type() == at::kInt && target.scalar_type() == at::kInt && pred.is_contiguous() && target.is_contiguous());
@@ -793,12 +801,13 @@ std::tuple<Tensor, Tensor> step_tail(const Tensor& row_loss, const Tensor& pred,
   TORCH_CHECK((mask.scalar_type() == at::kByte || mask.scalar_type() == at::kBool) && mask.is_contiguous());
   TORCH_CHECK((prev.scalar_type() == at::kByte || prev.scalar_type() == at::kBool) && prev.is_contiguous());
   c10::cuda::CUDAGuard guard(row_loss.device());
-  Tensor out = at::empty({4}, row_loss.options());
+  Tensor out = at::empty({5}, row_loss.options()), total = at::empty({}, row_loss.options());
   Tensor weight = at::empty({rows}, row_loss.options());
   sb200::launch_step_tail(row_loss.data_ptr<float>(), pred.data_ptr<int>(), target.data_ptr<int>(),
                           static_cast<const uint8_t*>(mask.data_ptr()), static_cast<uint8_t*>(prev.data_ptr()), (int)rows, (float)decay,
-                          (float)eps, out.data_ptr<float>(), weight.data_ptr<float>(), cur_stream());
-  return {out, weight};
+                          (float)eps, out.data_ptr<float>(), weight.data_ptr<float>(), earlier.has_value() ? earlier->data_ptr<float>() : nullptr,
+                           total.data_ptr<float>(), cur_stream());
+  return {out, weight, total};
 }
 
 // ---- hidden-state ring (device-to-device hand-off) -----------------------------------------
@@ -1216,8 +1225,9 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> attn_bwd(
   Tensor delta = at::empty({q.size(1), q.size(0)}, lse2.options());
   Tensor dke, dve;
   if (p.E > 0 || p.ext_block > 0) {
-    dke = at::zeros({p.Te, p.nkv, hd}, lse2.options());
-    dve = at::zeros({p.Te, p.nkv, hd}, lse2.options());
+    const Tensor both = at::zeros({2, p.Te, p.nkv, hd}, lse2.options());
+    dke = both.select(0, 0);
+    dve = both.select(0, 1);
     p.dke = dke.data_ptr<float>();
     p.dve = dve.data_ptr<float>();
   } else {
@@ -1248,6 +1258,11 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> attn_bwd(
                  : impl == 1 ? sb200::launch_attn_bwd_tc(p, qmin.data_ptr<int>(), qmax.data_ptr<int>(), status->data_ptr<int>(), cur_stream())
                            : sb200::launch_attn_bwd(p, (int)hd, qmin.data_ptr<int>(), qmax.data_ptr<int>(), cur_stream());
   TORCH_CHECK(rc == 0, "attn_bwd launch failed (", rc, ")");
+  if (dke.numel() > 0) {  // both gradients of the extra keys in the inputs' type with one conversion
+    const Tensor both = at::as_strided(dke, {2, p.Te, p.nkv, hd}, {(int64_t)p.Te * p.nkv * hd, p.nkv * hd, hd, 1}).to(q.scalar_type());
+    dke = both.select(0, 0);
+    dve = both.select(0, 1);
+  }
   return {dq, dk, dv, dke, dve};
 }
 
@@ -1263,6 +1278,8 @@ TORCH_LIBRARY(sb200, m) {
   m.def("heads_fwd", &heads_fwd);
   m.def("heads_bwd", &heads_bwd);
   m.def("rope_merge", &rope_merge);
+  m.def("loss_fwd_either", &loss_fwd_either);
+  m.def("loss_bwd_scaled", &loss_bwd_scaled);
   m.def("repeated_rows_sum", &repeated_rows_sum);
   m.def("document_interval", &document_interval);
   m.def("compact_rows", &compact_rows);

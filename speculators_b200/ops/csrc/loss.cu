@@ -78,7 +78,7 @@ __device__ __forceinline__ void block_combine(RowStats& s, float* scratch, int* 
 template <int OP>
 __global__ void __launch_bounds__(kLossThreads)
 loss_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* __restrict__ targets,
-                const uint8_t* __restrict__ active, const int64_t* __restrict__ labels,
+                const uint8_t* __restrict__ active, const uint8_t* __restrict__ also, const int64_t* __restrict__ labels,
                 float* __restrict__ loss, float* __restrict__ stats, int* __restrict__ argmax_d,
                 int* __restrict__ argmax_t, int rows, int V, int64_t ld_logits, int64_t ld_targets,
                 int shift) {
@@ -88,7 +88,7 @@ loss_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* _
   const int r = blockIdx.x;
   if (r >= rows) return;
   float* st = stats + r;
-  if (active && !active[r]) {
+  if (active && !active[r] && !(also && also[r])) {
     if (threadIdx.x == 0) {
       loss[r] = 0.f;
 #pragma unroll
@@ -207,7 +207,7 @@ loss_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* _
 template <int OP>
 __global__ void __launch_bounds__(kLossThreads)
 loss_bwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* __restrict__ targets,
-                const float* __restrict__ grad_out, const float* __restrict__ stats,
+                const float* __restrict__ grad_out, const float* __restrict__ grad_scale, const float* __restrict__ stats,
                 __nv_bfloat16* __restrict__ dlogits, int rows, int total_rows, int V,
                 int64_t ld_logits, int64_t ld_targets, int64_t ld_dlogits, int shift) {
   pdl_begin();
@@ -217,7 +217,7 @@ loss_bwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* _
   const bool vec_ok =
       ((V & 7) == 0) && ((ld_logits & 7) == 0) && ((ld_targets & 7) == 0) && ((ld_dlogits & 7) == 0);
   const int nvec = vec_ok ? (V >> 3) : 0;
-  const float go = r < rows ? grad_out[r] : 0.f;
+  const float go = r < rows ? grad_out[r] * (grad_scale != nullptr ? *grad_scale : 1.f) : 0.f;
   // a row the forward skipped (inactive) has all-zero statistics; its sum-exp would be >= 1
   // otherwise.  Such a row gets no gradient whatever the upstream value is.
   const bool skipped = r < rows && stats[(int64_t)rows + r] == 0.f;
@@ -265,7 +265,8 @@ loss_bwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* _
         grad(__bfloat162float(x[c]), OP != kOpCE ? __bfloat162float(t[c]) : 0.f, c));
 }
 
-int launch_loss_fwd(int op, const void* logits, const void* targets, const uint8_t* active,
+// active / also (optional): rows marked in neither are skipped
+int launch_loss_fwd(int op, const void* logits, const void* targets, const uint8_t* active, const uint8_t* also,
                     const int64_t* labels, float* loss, float* stats, int* argmax_d, int* argmax_t, int rows, int V,
                     int64_t ld_logits, int64_t ld_targets, int shift, cudaStream_t stream) {
   if (rows <= 0) return 0;
@@ -273,7 +274,7 @@ int launch_loss_fwd(int op, const void* logits, const void* targets, const uint8
   count_launch(1);
 #define SB200_LF(OPV)                                                                            \
   launch_pdl(loss_fwd_kernel<OPV>, rows, kLossThreads, 0, stream,                                         \
-      (const __nv_bfloat16*)logits, (const __nv_bfloat16*)targets, active, labels, loss, stats,   \
+      (const __nv_bfloat16*)logits, (const __nv_bfloat16*)targets, active, also, labels, loss, stats,   \
       argmax_d, argmax_t, rows, V, ld_logits, ld_targets, shift)
   switch (op) {
     case kOpKL: SB200_LF(kOpKL); break;
@@ -287,15 +288,16 @@ int launch_loss_fwd(int op, const void* logits, const void* targets, const uint8
   return 0;
 }
 
+// grad_scale (optional, device): a factor of every grad_out
 int launch_loss_bwd(int op, const void* logits, const void* targets, const float* grad_out,
-                    const float* stats, void* dlogits, int rows, int total_rows, int V,
+                    const float* grad_scale, const float* stats, void* dlogits, int rows, int total_rows, int V,
                     int64_t ld_logits, int64_t ld_targets, int64_t ld_dlogits, int shift,
                     cudaStream_t stream) {
   if (total_rows <= 0) return 0;
   count_launch(1);
 #define SB200_LB(OPV)                                                                         \
   launch_pdl(loss_bwd_kernel<OPV>, total_rows, kLossThreads, 0, stream,                                \
-      (const __nv_bfloat16*)logits, (const __nv_bfloat16*)targets, grad_out, stats,            \
+      (const __nv_bfloat16*)logits, (const __nv_bfloat16*)targets, grad_out, grad_scale, stats,            \
       (__nv_bfloat16*)dlogits, rows, total_rows, V, ld_logits, ld_targets, ld_dlogits, shift)
   switch (op) {
     case kOpKL: SB200_LB(kOpKL); break;

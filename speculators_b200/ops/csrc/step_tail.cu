@@ -8,6 +8,7 @@
 //   correct     = sum_r (prev[r] & mask[r])         (after the update)
 //   total       = sum_r mask[r]
 //   weight[r]   = decay * mask[r] / (sum mask + eps)     (d loss / d row_loss[r], for backward)
+//   total_loss  = loss of the earlier passes + loss      (optional: the passes' sum without an addition of its own)
 //
 // One CTA (rows are a few thousand): two passes over the rows, block-wide sums in between.
 #include "common.cuh"
@@ -20,7 +21,7 @@ constexpr int kTailThreads = 1024;
 __global__ void __launch_bounds__(kTailThreads)
 step_tail_kernel(const float* __restrict__ row_loss, const int* __restrict__ pred, const int* __restrict__ target,
                  const uint8_t* __restrict__ mask, uint8_t* __restrict__ prev, int rows, float decay, float eps,
-                 float* __restrict__ out, float* __restrict__ weight) {
+                 float* __restrict__ out, float* __restrict__ weight, const float* __restrict__ earlier, float* __restrict__ total_loss) {
   pdl_begin();
   __shared__ float scratch[33];
   float s_loss = 0.f, s_mask = 0.f, s_prev = 0.f, s_correct = 0.f;
@@ -49,6 +50,8 @@ step_tail_kernel(const float* __restrict__ row_loss, const int* __restrict__ pre
     out[1] = s_correct;
     out[2] = s_mask;
     out[3] = s_prev;
+    out[4] = 1.f;  // how many passes the sums above cover
+    if (total_loss != nullptr) *total_loss = (earlier != nullptr ? *earlier : 0.f) + s_loss * scale;
   }
   __syncthreads();
   const float scale = scale_s;
@@ -57,11 +60,11 @@ step_tail_kernel(const float* __restrict__ row_loss, const int* __restrict__ pre
 
 }  // namespace
 
-// out: float[4] = loss, correct, total, cond_total.  weight: float[rows].
+// out: float[5] = loss, correct, total, cond_total, 1.  weight: float[rows].
 void launch_step_tail(const float* row_loss, const int* pred, const int* target, const uint8_t* mask, uint8_t* prev, int rows,
-                      float decay, float eps, float* out, float* weight, cudaStream_t stream) {
+                      float decay, float eps, float* out, float* weight, const float* earlier, float* total_loss, cudaStream_t stream) {
   count_launch(1);
-  launch_pdl(step_tail_kernel, 1, kTailThreads, 0, stream, row_loss, pred, target, mask, prev, rows, decay, eps, out, weight);
+  launch_pdl(step_tail_kernel, 1, kTailThreads, 0, stream, row_loss, pred, target, mask, prev, rows, decay, eps, out, weight, earlier, total_loss);
 }
 
 }  // namespace sb200
