@@ -1,12 +1,13 @@
 """CUDA path of ``masked_attention``: autograd wrapper around the sm_100a kernels
 (head dims 64, 128 and 256).  Other head dims use the dense formulation.
 
-Forward and backward at head dim 128, and at 256 without extra keys (the gated full-attention
+Forward and backward at head dims 64 and 128, and at 256 without extra keys (the gated full-attention
 heads of Qwen3-Next style MTP layers), run on the tcgen05 tensor cores
 (``csrc/attention_tc.cu``, ``csrc/attention_bwd_tc.cu``, ``csrc/attention_wide_tc.cu``: TMA tiles,
 TMEM accumulators, probability tiles handed to the next product through TMEM); ``FWD_IMPL`` /
 ``BWD_IMPL`` = ``"mma"`` (or ``SB200_ATTN_FWD=mma`` / ``SB200_ATTN_BWD=mma``) select the
-``mma.sync`` kernels of ``csrc/attention.cu``, which also serve head dim 64 and 256 with extra keys."""
+``mma.sync`` kernels of ``csrc/attention.cu``, which also serve head dim 256 with extra keys and
+short inputs at head dim 64."""
 
 from __future__ import annotations
 
@@ -33,9 +34,13 @@ def _rows_ok(t: torch.Tensor) -> torch.Tensor:
 
 
 def _tensor_core_shape(q: torch.Tensor, ext_idx: torch.Tensor | None) -> bool:
-    """Whether the tcgen05 kernels take the call: head dim 128, or 256 (their own kernels, whose shared memory is filled by
-    128 resident rows and leaves none to stage individually addressed extra keys in)."""
-    return q.shape[2] == 128 or (q.shape[2] == 256 and ext_idx is None)
+    """Whether the tcgen05 kernels take the call: head dim 128; 256 without extra keys (its own kernels, whose shared memory
+    is filled by 128 resident rows and leaves none to stage individually addressed extra keys in); 64 from 513 query rows on -
+    up to there a head is a few key tiles, and setting up tensor memory costs what the products save (128 tokens, 4 heads:
+    10 / 55 us forward / backward on mma.sync, 11 / 61 here; 512 tokens 15 / 61 and 15 / 68; 1001 tokens, 32 heads 42 / 117
+    and 26 / 73; 8192 tokens 1189 / 3543 and 593 / 1644)."""
+    hd = q.shape[2]
+    return hd == 128 or (hd == 64 and q.shape[0] > 512) or (hd == 256 and ext_idx is None)
 
 
 class _MaskedAttentionFn(torch.autograd.Function):

@@ -1,4 +1,4 @@
-// Masked attention backward on the 5th-generation tensor cores (head_dim 128): two kernels
+// Masked attention backward on the 5th-generation tensor cores (head dims 64 and 128): two kernels
 // with the same role split as the forward (warp 0 TMA producer, warp 1 single-thread MMA
 // issuer and TMEM owner, warps 2-9 element-wise work, two threads per TMEM lane with 64
 // columns each).  Every product runs on tcgen05.mma with fp32 accumulators in TMEM; the
@@ -31,11 +31,11 @@ namespace abtc {
 
 using namespace tc;
 
-constexpr int BM = 128, BN = 128, HD = 128, THREADS = 320;
+constexpr int BM = 128, BN = 128, THREADS = 320;
 constexpr int SUB_BYTES = 128 * 64 * 2;    // one [128 rows x 64 columns] bf16 sub-tile
-constexpr int TILE_BYTES = 2 * SUB_BYTES;  // a [128 x 128] operand tile
+template <int HD> constexpr int kTile = HD / 64 * SUB_BYTES;  // a [128 x HD] operand tile
 constexpr int TMEM_COLS = 512;
-constexpr int SMEM_BYTES = 6 * TILE_BYTES + 1024;
+template <int HD> constexpr int kSmem = 6 * kTile<HD> + 1024;
 constexpr float kLog2e = 1.4426950408889634f;
 
 enum Status : int {
@@ -43,16 +43,22 @@ enum Status : int {
   kTimeoutDkvProducer = 44, kTimeoutDkvMma = 45, kTimeoutDkvCompute = 46,
 };
 
-// D (+)= A B^T, both operands [128 rows x 128] K-major tiles in shared memory
+template <int HD>
+__device__ __forceinline__ void load_tile(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
+#pragma unroll
+  for (int c = 0; c < HD / 64; ++c) tma_load_2d(dst + c * SUB_BYTES, map, bar, x + c * 64, y);
+}
+// D (+)= A B^T, both operands [128 rows x HD] K-major tiles in shared memory
+template <int HD>
 __device__ __forceinline__ void mma_ss(uint32_t tmem_d, uint32_t a_tile, uint32_t b_tile, uint32_t idesc) {
 #pragma unroll
-  for (int kk = 0; kk < 8; ++kk) {
+  for (int kk = 0; kk < HD / 16; ++kk) {
     const uint32_t off = (kk >> 2) * SUB_BYTES;
     umma_bf16(tmem_d, smem_desc_kmajor_sw128(a_tile + off) + 2 * (kk & 3), smem_desc_kmajor_sw128(b_tile + off) + 2 * (kk & 3), idesc, kk != 0);
   }
 }
 // D (+)= A B with A [128 x 128] as bf16 pairs in TMEM (contraction index 0..63 from column
-// a0, 64..127 from column a1) and B a [128 contraction rows x 128] tile read MN-major
+// a0, 64..127 from column a1) and B a [128 contraction rows x HD] tile read MN-major
 __device__ __forceinline__ void mma_ts(uint32_t tmem_d, uint32_t a0, uint32_t a1, uint32_t b_tile, uint32_t idesc, bool accumulate) {
 #pragma unroll
   for (int kk = 0; kk < 8; ++kk) {
@@ -61,21 +67,10 @@ __device__ __forceinline__ void mma_ts(uint32_t tmem_d, uint32_t a0, uint32_t a1
   }
 }
 
-// like tc::store_rows64_f32, adding into global memory (several query heads of a group meet on one KV head)
-__device__ __forceinline__ void atomic_rows64_f32(unsigned char* stage, const float (&vals)[64], float* gbase, int64_t row_stride, int rows_valid,
-                                                  int lane) {
-  __syncwarp();
-  float4* mine = reinterpret_cast<float4*>(stage + lane * 256);
-#pragma unroll
-  for (int c = 0; c < 16; ++c) mine[c ^ (lane & 7)] = make_float4(vals[c * 4], vals[c * 4 + 1], vals[c * 4 + 2], vals[c * 4 + 3]);
-  __syncwarp();
-#pragma unroll
-  for (int it = 0; it < 16; ++it) {
-    const int r = it * 2 + (lane >> 4), pc = lane & 15;
-    const float4 v = reinterpret_cast<const float4*>(stage + r * 256)[pc ^ (r & 7)];
-    if (r < rows_valid) atomicAdd(reinterpret_cast<float4*>(gbase + (int64_t)r * row_stride + pc * 4), v);
-  }
-  __syncwarp();
+// like tc::store_rows_f32, adding into global memory (several query heads of a group meet on one KV head)
+template <int W>
+__device__ __forceinline__ void atomic_rows_f32(unsigned char* stage, const float (&vals)[W], float* gbase, int64_t row_stride, int rows_valid, int lane) {
+  stage_rows_f32(stage, vals, rows_valid, lane, [&](int r, int c, float4 v) { atomicAdd(reinterpret_cast<float4*>(gbase + (int64_t)r * row_stride + c), v); });
 }
 
 __device__ __forceinline__ void pair_barrier(int quarter) { asm volatile("bar.sync %0, 64;" ::"r"(1 + quarter) : "memory"); }
@@ -113,11 +108,13 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* _
 }
 
 // ------------------------------------------------------------------------------------- dQ
+template <int HD>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_do,
                       const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                       const __grid_constant__ CUtensorMap map_ke, const __grid_constant__ CUtensorMap map_ve,
                       const AttnParams p, int* status) {
+  constexpr int TILE_BYTES = kTile<HD>, HO = HD / 2, STAGE = HD * 128;  // HO: head-dim columns of a thread; STAGE: staging bytes of a warp
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* q_s = smem;
@@ -200,10 +197,8 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     if (elect_one()) {
       const uint32_t qb = smem_addr(&bar_qdo);
       mbar_expect_tx(qb, 2 * TILE_BYTES);
-      tma_load_2d(smem_addr(q_s), &map_q, qb, h * HD, q0);
-      tma_load_2d(smem_addr(q_s) + SUB_BYTES, &map_q, qb, h * HD + 64, q0);
-      tma_load_2d(smem_addr(do_s), &map_do, qb, h * HD, q0);
-      tma_load_2d(smem_addr(do_s) + SUB_BYTES, &map_do, qb, h * HD + 64, q0);
+      load_tile<HD>(smem_addr(q_s), &map_q, qb, h * HD, q0);
+      load_tile<HD>(smem_addr(do_s), &map_do, qb, h * HD, q0);
       for (int t = 0; t < n_tiles; ++t) {
         const int st = t % 3;
         const bool ext = t >= n_ctx;
@@ -214,13 +209,11 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         const uint32_t kfull = smem_addr(&bar_k_full[st]);
         mbar_expect_tx(kfull, TILE_BYTES);
         const uint32_t ka = smem_addr(k_s + st * TILE_BYTES), va = smem_addr(v_s);
-        tma_load_2d(ka, mk, kfull, kvh * HD, key0);
-        tma_load_2d(ka + SUB_BYTES, mk, kfull, kvh * HD + 64, key0);
+        load_tile<HD>(ka, mk, kfull, kvh * HD, key0);
         if (!mbar_wait(smem_addr(&bar_v_empty), (t & 1) ^ 1, status, kTimeoutDqProducer)) break;
         const uint32_t vfull = smem_addr(&bar_v_full);
         mbar_expect_tx(vfull, TILE_BYTES);
-        tma_load_2d(va, mv, vfull, kvh * HD, key0);
-        tma_load_2d(va + SUB_BYTES, mv, vfull, kvh * HD + 64, key0);
+        load_tile<HD>(va, mv, vfull, kvh * HD, key0);
       }
     }
   } else if (warp == 1) {
@@ -229,8 +222,8 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       constexpr uint32_t idesc_mn = instr_desc(BM, HD, true);
       const uint32_t qa = smem_addr(q_s), da = smem_addr(do_s);
       auto issue_scores = [&](int t) {  // S = Q K_t^T and dP = dO V_t^T
-        mma_ss(tmem_base + COL_S, qa, smem_addr(k_s + (t % 3) * TILE_BYTES), idesc_kk);
-        mma_ss(tmem_base + COL_DP, da, smem_addr(v_s), idesc_kk);
+        mma_ss<HD>(tmem_base + COL_S, qa, smem_addr(k_s + (t % 3) * TILE_BYTES), idesc_kk);
+        mma_ss<HD>(tmem_base + COL_DP, da, smem_addr(v_s), idesc_kk);
         umma_commit(smem_addr(&bar_sdp_full));
         umma_commit(smem_addr(&bar_v_empty));  // the V buffer may be refilled
       };
@@ -270,7 +263,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     const int ehi = (row_ok && p.ext_block > 0) ? min(p.ext_causal ? row + 1 : elo + p.ext_block, p.Te) : 0;
     const float sc = p.scale * kLog2e;
     const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
-    const int colh = half * 64;
+    const int colh = half * 64, colo = half * HO;  // first key, first head-dim column of this thread
     const int sw = prow & 7;
     int xc = 0;
     auto exchange = [&](float2 mine) -> float2 {
@@ -283,8 +276,10 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
 
     bool ok = mbar_wait(smem_addr(&bar_qdo), 0, status, kTimeoutDqCompute);
     ok = __all_sync(0xffffffffu, ok);
-    const unsigned char* q_row = q_s + half * SUB_BYTES + prow * 128;    // this thread's 64 head-dim columns of q
-    const unsigned char* do_row = do_s + half * SUB_BYTES + prow * 128;  // ... and of dO
+    constexpr int L = HO / 8;  // 16-byte chunks of a half row
+    const int half_at = HD == 128 ? half * SUB_BYTES : 0, qc0 = HD == 128 ? 0 : half * L;
+    const unsigned char* q_row = q_s + half_at + prow * 128;    // this thread's head-dim columns of q (from chunk qc0)
+    const unsigned char* do_row = do_s + half_at + prow * 128;  // ... and of dO
     const float delta = row_ok ? p.delta[(int64_t)h * p.Tq + row] : 0.f;  // rowsum(dO * O), from attn_delta_kernel
 
     for (int t = 0; t < n_tiles; ++t) {
@@ -334,17 +329,17 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       if (lane == 0) mbar_arrive(smem_addr(&bar_ds_ready));
     }
 
-    float dq[64];
+    float dq[HO];
 #pragma unroll
-    for (int i = 0; i < 64; ++i) dq[i] = 0.f;
+    for (int i = 0; i < HO; ++i) dq[i] = 0.f;
     if (n_tiles > 0) {
       if (ok) ok = mbar_wait(smem_addr(&bar_dq_done), (n_tiles - 1) & 1, status, kTimeoutDqCompute);
       ok = __all_sync(0xffffffffu, ok);
       fence_after_sync();
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
+      for (int c = 0; c < HO / 32; ++c) {
         uint32_t a[32];
-        tmem_ld32(lane_base + COL_DQ + colh + c * 32, a);
+        tmem_ld32(lane_base + COL_DQ + colo + c * 32, a);
         tmem_ld_wait();
 #pragma unroll
         for (int i = 0; i < 32; ++i) dq[c * 32 + i] = __uint_as_float(a[i]);
@@ -352,40 +347,39 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       fence_before_sync();
     }
 
-    // Individually addressed extra keys: each thread of the pair takes 64 of the 128
+    // Individually addressed extra keys: each thread of the pair takes half of the
     // dimensions of q.k and dO.v, the halves meet through the exchange slots.  Rows of the
     // extra K / V tensors and the dK / dV contributions travel through a per-warp staging
     // area (the K / V stages, idle once the tile loop has drained) so that global loads and
     // atomics are issued warp-wide over whole rows instead of one row per lane.
     if (p.E > 0) {
-      unsigned char* stage = k_s + (warp - 2) * 16384;  // 16 KB per warp
+      unsigned char* stage = k_s + (warp - 2) * STAGE;
+      constexpr int V_AT = 32 * HO * 2, F_AT = 2 * V_AT;  // staged K rows, V rows, fp32 rows
       for (int e = 0; e < p.E; ++e) {
         const int idx = row_ok ? p.ext_idx[(int64_t)row * p.E + e] : -1;
         const bool valid = idx >= 0 && idx < p.Te;
         const int idc = valid ? idx : 0;
-        // stage in: 8 lanes fetch the 128 bytes of one row's half, 4 rows per instruction
+        // stage in: L lanes fetch one row's half, 32 / L rows per instruction
         __syncwarp();
 #pragma unroll
-        for (int it = 0; it < 8; ++it) {
-          const int r = it * 4 + (lane >> 3), pc = lane & 7;
+        for (int it = 0; it < L; ++it) {
+          const int r = it * (32 / L) + lane / L, pc = lane % L;
           const int64_t ir = __shfl_sync(0xffffffffu, idc, r);
-          const bf16x8 kx = ld8(p.ke + ir * p.ke_rs + kvh * HD + colh + pc * 8);
-          const bf16x8 vx = ld8(p.ve + ir * p.ve_rs + kvh * HD + colh + pc * 8);
-          *reinterpret_cast<bf16x8*>(stage + r * 128 + ((pc ^ (r & 7)) << 4)) = kx;
-          *reinterpret_cast<bf16x8*>(stage + 4096 + r * 128 + ((pc ^ (r & 7)) << 4)) = vx;
+          const bf16x8 kx = ld8(p.ke + ir * p.ke_rs + kvh * HD + colo + pc * 8);
+          const bf16x8 vx = ld8(p.ve + ir * p.ve_rs + kvh * HD + colo + pc * 8);
+          *reinterpret_cast<bf16x8*>(stage + stage_row_chunk<HO>(r, pc)) = kx;
+          *reinterpret_cast<bf16x8*>(stage + V_AT + stage_row_chunk<HO>(r, pc)) = vx;
         }
         __syncwarp();
-        const unsigned char* k_row = stage + lane * 128;
-        const unsigned char* v_row = stage + 4096 + lane * 128;
         const int lsw = lane & 7;
         float dot = 0.f, dpe = 0.f;
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
+        for (int c = 0; c < L; ++c) {
           float a[8], b[8], g[8], w[8];
-          unpack8(*reinterpret_cast<const bf16x8*>(q_row + ((c ^ sw) << 4)), a);
-          unpack8(*reinterpret_cast<const bf16x8*>(k_row + ((c ^ lsw) << 4)), b);
-          unpack8(*reinterpret_cast<const bf16x8*>(do_row + ((c ^ sw) << 4)), g);
-          unpack8(*reinterpret_cast<const bf16x8*>(v_row + ((c ^ lsw) << 4)), w);
+          unpack8(*reinterpret_cast<const bf16x8*>(q_row + (((qc0 + c) ^ sw) << 4)), a);
+          unpack8(*reinterpret_cast<const bf16x8*>(stage + stage_row_chunk<HO>(lane, c)), b);
+          unpack8(*reinterpret_cast<const bf16x8*>(do_row + (((qc0 + c) ^ sw) << 4)), g);
+          unpack8(*reinterpret_cast<const bf16x8*>(stage + V_AT + stage_row_chunk<HO>(lane, c)), w);
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             dot = fmaf(a[i], b[i], dot);
@@ -397,34 +391,34 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
         const float dse = pe * (dpe + other.y - delta);
         const float dss = dse * p.scale;
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
+        for (int c = 0; c < L; ++c) {
           float b[8];
-          unpack8(*reinterpret_cast<const bf16x8*>(k_row + ((c ^ lsw) << 4)), b);
+          unpack8(*reinterpret_cast<const bf16x8*>(stage + stage_row_chunk<HO>(lane, c)), b);
 #pragma unroll
           for (int i = 0; i < 8; ++i) dq[c * 8 + i] = fmaf(dse, b[i], dq[c * 8 + i]);
         }
         // contributions to the extra keys' dK (dss * q) then dV (pe * dO): each lane lays its
-        // row's 64 floats into the staging area, then 16 lanes add one row's 256 bytes
+        // row's HO floats into the staging area, then HO / 4 lanes add one row
 #pragma unroll 1
         for (int which = 0; which < 2; ++which) {
           const unsigned char* src_row = which ? do_row : q_row;
           const float mul = which ? pe : dss;
-          float* dst_base = (which ? p.dve : p.dke) + kvh * HD + colh;
+          float* dst_base = (which ? p.dve : p.dke) + kvh * HD + colo;
           __syncwarp();
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
+          for (int c = 0; c < L; ++c) {
             float a[8];
-            unpack8(*reinterpret_cast<const bf16x8*>(src_row + ((c ^ sw) << 4)), a);
-            float4* out4 = reinterpret_cast<float4*>(stage + 8192 + lane * 256);
+            unpack8(*reinterpret_cast<const bf16x8*>(src_row + (((qc0 + c) ^ sw) << 4)), a);
+            float4* out4 = reinterpret_cast<float4*>(stage + F_AT + lane * (HO * 4));
             out4[(2 * c) ^ lsw] = make_float4(mul * a[0], mul * a[1], mul * a[2], mul * a[3]);
             out4[(2 * c + 1) ^ lsw] = make_float4(mul * a[4], mul * a[5], mul * a[6], mul * a[7]);
           }
           __syncwarp();
 #pragma unroll
-          for (int it = 0; it < 16; ++it) {
-            const int r = it * 2 + (lane >> 4), pc = lane & 15;
+          for (int it = 0; it < 2 * L; ++it) {
+            const int r = it * (16 / L) + lane / (2 * L), pc = lane % (2 * L);
             const int ir = __shfl_sync(0xffffffffu, valid && ok ? idx : -1, r);
-            const float4 val = reinterpret_cast<const float4*>(stage + 8192 + r * 256)[pc ^ (r & 7)];
+            const float4 val = reinterpret_cast<const float4*>(stage + F_AT + r * (HO * 4))[pc ^ (r & 7)];
             if (ir >= 0) atomicAdd(reinterpret_cast<float4*>(dst_base + (int64_t)ir * p.nkv * HD + pc * 4), val);
           }
         }
@@ -434,7 +428,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     if (__all_sync(0xffffffffu, ok)) {
       // whole rows through the warp's staging area (the K / V stages are idle by now)
       const int warp_row0 = q0 + quarter * 32;
-      store_rows64_bf16(k_s + (warp - 2) * 16384, dq, p.scale, p.dq + (int64_t)warp_row0 * p.dq_rs + h * HD + colh, p.dq_rs, p.Tq - warp_row0, lane);
+      store_rows_bf16(k_s + (warp - 2) * STAGE, dq, p.scale, p.dq + (int64_t)warp_row0 * p.dq_rs + h * HD + colo, p.dq_rs, p.Tq - warp_row0, lane);
     }
   }
 
@@ -448,6 +442,7 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
 }
 
 // ---------------------------------------------------------------------------------- dK / dV
+template <int HD>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_do,
                        const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
@@ -455,6 +450,7 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   // ext_mode (block-structured extras): the key tiles are tiles of the extra K / V tensors (the caller passes their
   // tensor maps as map_k / map_v); key tile j is seen by query tile j alone, under the block mask, and the result is
   // added (fp32 atomics over the query heads of a group) into dke / dve.
+  constexpr int TILE_BYTES = kTile<HD>, HO = HD / 2, STAGE = HD * 128;  // HO: head-dim columns of a thread; STAGE: staging bytes of a warp
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* k_s = smem;
@@ -521,10 +517,8 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     if (n_tiles > 0 && elect_one()) {
       const uint32_t kvb = smem_addr(&bar_kv);
       mbar_expect_tx(kvb, 2 * TILE_BYTES);
-      tma_load_2d(smem_addr(k_s), &map_k, kvb, kvh * HD, key_base);
-      tma_load_2d(smem_addr(k_s) + SUB_BYTES, &map_k, kvb, kvh * HD + 64, key_base);
-      tma_load_2d(smem_addr(v_s), &map_v, kvb, kvh * HD, key_base);
-      tma_load_2d(smem_addr(v_s) + SUB_BYTES, &map_v, kvb, kvh * HD + 64, key_base);
+      load_tile<HD>(smem_addr(k_s), &map_k, kvb, kvh * HD, key_base);
+      load_tile<HD>(smem_addr(v_s), &map_v, kvb, kvh * HD, key_base);
       for (int t = 0; t < n_tiles; ++t) {
         const int st = t & 1;
         if (!mbar_wait(smem_addr(&bar_qdo_empty[st]), ((t >> 1) & 1) ^ 1, status, kTimeoutDkvProducer)) break;
@@ -532,10 +526,8 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         mbar_expect_tx(full, 2 * TILE_BYTES);
         const int r0 = (i0 + t) * BM;
         const uint32_t qa = smem_addr(q_s + st * TILE_BYTES), da = smem_addr(do_s + st * TILE_BYTES);
-        tma_load_2d(qa, &map_q, full, h * HD, r0);
-        tma_load_2d(qa + SUB_BYTES, &map_q, full, h * HD + 64, r0);
-        tma_load_2d(da, &map_do, full, h * HD, r0);
-        tma_load_2d(da + SUB_BYTES, &map_do, full, h * HD + 64, r0);
+        load_tile<HD>(qa, &map_q, full, h * HD, r0);
+        load_tile<HD>(da, &map_do, full, h * HD, r0);
       }
     }
   } else if (warp == 1) {
@@ -547,9 +539,9 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       bool ok = mbar_wait(smem_addr(&bar_kv), 0, status, kTimeoutDkvMma) && mbar_wait(smem_addr(&bar_qdo_full[0]), 0, status, kTimeoutDkvMma);
       if (ok) {
         fence_after_sync();
-        mma_ss(t_st, ka, smem_addr(q_s), idesc_kk);  // S^T = K Q^T
+        mma_ss<HD>(t_st, ka, smem_addr(q_s), idesc_kk);  // S^T = K Q^T
         umma_commit(smem_addr(&bar_s_full));
-        mma_ss(t_dpt, va, smem_addr(do_s), idesc_kk);  // dP^T = V dO^T
+        mma_ss<HD>(t_dpt, va, smem_addr(do_s), idesc_kk);  // dP^T = V dO^T
         umma_commit(smem_addr(&bar_dp_full));
       }
       for (int t = 0; t < n_tiles && ok; ++t) {
@@ -564,7 +556,7 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           // P^T of tile t shares its columns with S^T: wait until the product above has read it
           if (!(ok = mbar_wait(smem_addr(&bar_dv_done), t & 1, status, kTimeoutDkvMma))) break;
           fence_after_sync();
-          mma_ss(t_st, ka, q_n, idesc_kk);
+          mma_ss<HD>(t_st, ka, q_n, idesc_kk);
           umma_commit(smem_addr(&bar_s_full));
         }
         if (!(ok = mbar_wait(smem_addr(&bar_ds_ready), t & 1, status, kTimeoutDkvMma))) break;
@@ -575,7 +567,7 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         if (t + 1 < n_tiles) {
           if (!(ok = mbar_wait(smem_addr(&bar_dk_done), t & 1, status, kTimeoutDkvMma))) break;
           fence_after_sync();
-          mma_ss(t_dpt, va, do_n, idesc_kk);
+          mma_ss<HD>(t_dpt, va, do_n, idesc_kk);
           umma_commit(smem_addr(&bar_dp_full));
         }
       }
@@ -588,7 +580,7 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     const int ct = (warp - 2) * 32 + lane;  // 0..255: loader index for the per-query statistics
     const float sc = p.scale * kLog2e;
     const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
-    const int colh = half * 64;  // this thread's 64 queries of the tile / 64 head-dim columns of the outputs
+    const int colh = half * 64, colo = half * HO;  // this thread's first query of the tile / head-dim column of the outputs
     bool ok = true;
 
     // statistics of query `i0 * BM + ..` go through registers one tile ahead
@@ -708,22 +700,22 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       if (t + 1 < n_tiles) stash_stats(t + 1);
     }
 
-    // results: this thread's key row, 64 head-dim columns of dV and of dK
-    float acc[64];
+    // results: this thread's key row, HO head-dim columns of dV and of dK
+    float acc[HO];
     const int64_t plane = (int64_t)p.Tc * p.nkv * HD;
 #pragma unroll 1
     for (int which = 0; which < 2; ++which) {  // 0: dK, 1: dV
 #pragma unroll
-      for (int i = 0; i < 64; ++i) acc[i] = 0.f;
+      for (int i = 0; i < HO; ++i) acc[i] = 0.f;
       if (n_tiles > 0) {
         if (ok) ok = mbar_wait(smem_addr(which ? &bar_dv_done : &bar_dk_done), (n_tiles - 1) & 1, status, kTimeoutDkvCompute);
         ok = __all_sync(0xffffffffu, ok);
         fence_after_sync();
         const float mul = which ? 1.f : p.scale;
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
+        for (int c = 0; c < HO / 32; ++c) {
           uint32_t a[32];
-          tmem_ld32(lane_base + (which ? COL_DV : COL_DK) + colh + c * 32, a);
+          tmem_ld32(lane_base + (which ? COL_DV : COL_DK) + colo + c * 32, a);
           tmem_ld_wait();
 #pragma unroll
           for (int i = 0; i < 32; ++i) acc[c * 32 + i] = __uint_as_float(a[i]) * mul;
@@ -732,16 +724,16 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       }
       if (__all_sync(0xffffffffu, ok)) {
         // whole rows through the warp's staging area (the Q / dO stages are idle by now)
-        unsigned char* stage = q_s + (warp - 2) * 16384;
+        unsigned char* stage = q_s + (warp - 2) * STAGE;
         const int warp_key0 = key_base + quarter * 32;
-        const int64_t off0 = ((int64_t)warp_key0 * p.nkv + kvh) * HD + colh;
+        const int64_t off0 = ((int64_t)warp_key0 * p.nkv + kvh) * HD + colo;
         if (ext_mode)
-          atomic_rows64_f32(stage, acc, (which ? p.dve : p.dke) + off0, (int64_t)p.nkv * HD, n_keys - warp_key0, lane);
+          atomic_rows_f32(stage, acc, (which ? p.dve : p.dke) + off0, (int64_t)p.nkv * HD, n_keys - warp_key0, lane);
         else if (p.dkv_part != nullptr)
-          store_rows64_f32(stage, acc, p.dkv_part + (int64_t)(h - kvh * group) * 2 * plane + which * plane + off0, (int64_t)p.nkv * HD,
+          store_rows_f32(stage, acc, p.dkv_part + (int64_t)(h - kvh * group) * 2 * plane + which * plane + off0, (int64_t)p.nkv * HD,
                            p.Tc - warp_key0, lane);
         else
-          store_rows64_bf16(stage, acc, 1.f, (which ? p.dv : p.dk) + off0, (int64_t)p.nkv * HD, p.Tc - warp_key0, lane);
+          store_rows_bf16(stage, acc, 1.f, (which ? p.dv : p.dk) + off0, (int64_t)p.nkv * HD, p.Tc - warp_key0, lane);
       }
     }
   }
@@ -762,11 +754,12 @@ void launch_attn_delta(const AttnParams& p, int hd, cudaStream_t stream) {
   const int grid = (int)(blocks < 16 * kNumSM ? blocks : 16 * kNumSM);
   count_launch(1);
   if (hd == 256) launch_pdl(abtc::attn_delta_kernel<256>, grid, 256, 0, stream, p.dout, p.out, p.delta, p.Tq, p.nh, p.do_rs, p.o_rs);
+  else if (hd == 64) launch_pdl(abtc::attn_delta_kernel<64>, grid, 256, 0, stream, p.dout, p.out, p.delta, p.Tq, p.nh, p.do_rs, p.o_rs);
   else launch_pdl(abtc::attn_delta_kernel<128>, grid, 256, 0, stream, p.dout, p.out, p.delta, p.Tq, p.nh, p.do_rs, p.o_rs);
 }
 
-// head_dim 128; tile_qmin / tile_qmax: scratch of one int per 64-key tile, fully written here.
-int launch_attn_bwd_tc(const AttnParams& p, int* tile_qmin, int* tile_qmax, int* status, cudaStream_t stream) {
+template <int HD>
+static int launch_bwd(const AttnParams& p, int* tile_qmin, int* tile_qmax, int* status, cudaStream_t stream) {
   using namespace abtc;
   if (p.Tq <= 0) return 0;
   CUtensorMap map_q, map_do, map_k, map_v;
@@ -788,28 +781,33 @@ int launch_attn_bwd_tc(const AttnParams& p, int* tile_qmin, int* tile_qmax, int*
   }
   static PerDeviceOnce configured;
   if (configured.needed()) {
-    if (cudaFuncSetAttribute(attn_bwd_dq_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess) return -2;
-    if (cudaFuncSetAttribute(attn_bwd_dkv_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess) return -2;
+    if (cudaFuncSetAttribute(attn_bwd_dq_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem<HD>) != cudaSuccess) return -2;
+    if (cudaFuncSetAttribute(attn_bwd_dkv_tc_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem<HD>) != cudaSuccess) return -2;
     configured.mark();
   }
   count_launch(2);
   launch_attn_delta(p, HD, stream);
   dim3 grid_q(p.nh, (p.Tq + BM - 1) / BM);
-  launch_pdl(attn_bwd_dq_tc_kernel, grid_q, THREADS, SMEM_BYTES, stream, map_q, map_do, map_k, map_v, map_ke, map_ve, p, status);
+  launch_pdl(attn_bwd_dq_tc_kernel<HD>, grid_q, THREADS, kSmem<HD>, stream, map_q, map_do, map_k, map_v, map_ke, map_ve, p, status);
   rc = launch_kv_tile_range(p, tile_qmin, tile_qmax, stream);
   if (rc) return rc;
   dim3 grid_kv(p.nh, (p.Tc + BN - 1) / BN);
-  launch_pdl(attn_bwd_dkv_tc_kernel, grid_kv, THREADS, SMEM_BYTES, stream, map_q, map_do, map_k, map_v, p, (p.Tc + kAttnKeyTile - 1) / kAttnKeyTile, 0, status);
+  launch_pdl(attn_bwd_dkv_tc_kernel<HD>, grid_kv, THREADS, kSmem<HD>, stream, map_q, map_do, map_k, map_v, p, (p.Tc + kAttnKeyTile - 1) / kAttnKeyTile, 0, status);
   if (p.ext_block > 0) {  // gradients of the extra keys: one key tile per query tile, read from the extra tensors
     count_launch(1);
     dim3 grid_ext(p.nh, (p.Te + BN - 1) / BN);
-    launch_pdl(attn_bwd_dkv_tc_kernel, grid_ext, THREADS, SMEM_BYTES, stream, map_q, map_do, map_ke, map_ve, p, 0, 1, status);
+    launch_pdl(attn_bwd_dkv_tc_kernel<HD>, grid_ext, THREADS, kSmem<HD>, stream, map_q, map_do, map_ke, map_ve, p, 0, 1, status);
   }
   if (p.dkv_part != nullptr) {
     rc = launch_dkv_reduce(p, HD, stream);
     if (rc) return rc;
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
+// head_dim 64 or 128; tile_qmin / tile_qmax: scratch of one int per 64-key tile, fully written here.
+int launch_attn_bwd_tc(const AttnParams& p, int hd, int* tile_qmin, int* tile_qmax, int* status, cudaStream_t stream) {
+  return hd == 64 ? launch_bwd<64>(p, tile_qmin, tile_qmax, status, stream) : launch_bwd<128>(p, tile_qmin, tile_qmax, status, stream);
 }
 
 }  // namespace sb200

@@ -420,13 +420,13 @@ wide_kernel(const __grid_constant__ CUtensorMap map_r0, const __grid_constant__ 
       const int warp_row0 = row0 + quarter * 32;
       if constexpr (QRES) {
         const int64_t rs = MODE == kFwd ? p.o_rs : p.dq_rs;
-        store_rows64_bf16(stage, acc, 1.f, (MODE == kFwd ? p.out : p.dq) + (int64_t)warp_row0 * rs + h * HD + col, rs, p.Tq - warp_row0, lane);
+        store_rows_bf16(stage, acc, 1.f, (MODE == kFwd ? p.out : p.dq) + (int64_t)warp_row0 * rs + h * HD + col, rs, p.Tq - warp_row0, lane);
       } else {
         const int64_t rs = (int64_t)p.nkv * HD, off = (int64_t)warp_row0 * rs + kvh * HD + col, plane = (int64_t)p.Tc * rs;
         if (p.dkv_part != nullptr)
-          store_rows64_f32(stage, acc, p.dkv_part + ((int64_t)(h - kvh * group) * 2 + (MODE == kDv ? 1 : 0)) * plane + off, rs, p.Tc - warp_row0, lane);
+          store_rows_f32(stage, acc, p.dkv_part + ((int64_t)(h - kvh * group) * 2 + (MODE == kDv ? 1 : 0)) * plane + off, rs, p.Tc - warp_row0, lane);
         else
-          store_rows64_bf16(stage, acc, 1.f, (MODE == kDv ? p.dv : p.dk) + off, rs, p.Tc - warp_row0, lane);
+          store_rows_bf16(stage, acc, 1.f, (MODE == kDv ? p.dv : p.dk) + off, rs, p.Tc - warp_row0, lane);
       }
     }
     fence_before_sync();

@@ -1178,7 +1178,7 @@ std::tuple<Tensor, Tensor> attn_fwd(const Tensor& q, const Tensor& k, const Tens
   return {out, lse2};
 }
 
-// Forward on the tcgen05 tensor cores (head_dim 128, or 256 without extra keys).  `status` (int32[1], device) receives a
+// Forward on the tcgen05 tensor cores (head_dim 64 or 128, or 256 without extra keys).  `status` (int32[1], device) receives a
 // non-zero code if a bounded wait in the kernel ran out.
 std::tuple<Tensor, Tensor> attn_fwd_tc(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& lo, const Tensor& hi,
                                        const c10::optional<Tensor>& ke, const c10::optional<Tensor>& ve,
@@ -1186,7 +1186,7 @@ std::tuple<Tensor, Tensor> attn_fwd_tc(const Tensor& q, const Tensor& k, const T
                                        bool ext_causal) {
   sb200::AttnParams p = make_params(q, k, v, lo, hi, ke, ve, ext_idx, scale);
   use_block_extras(p, q, ext_block, ext_causal);
-  TORCH_CHECK(q.size(2) == 128 || (q.size(2) == 256 && p.E == 0 && p.ext_block == 0), "attn_fwd_tc: head_dim must be 128, or 256 without extra keys");
+  TORCH_CHECK(q.size(2) == 64 || q.size(2) == 128 || (q.size(2) == 256 && p.E == 0 && p.ext_block == 0), "attn_fwd_tc: head_dim must be 64 or 128, or 256 without extra keys");
   TORCH_CHECK(status.is_cuda() && status.scalar_type() == at::kInt && status.numel() >= 1);
   c10::cuda::CUDAGuard guard(q.device());
   Tensor out = at::empty({q.size(0), q.size(1), q.size(2)}, q.options());
@@ -1195,7 +1195,7 @@ std::tuple<Tensor, Tensor> attn_fwd_tc(const Tensor& q, const Tensor& k, const T
   p.o_rs = out.stride(0);
   p.lse2 = lse2.data_ptr<float>();
   const int rc = q.size(2) == 256 ? sb200::launch_attn_fwd_wide_tc(p, status.data_ptr<int>(), cur_stream())
-                                  : sb200::launch_attn_fwd_tc(p, status.data_ptr<int>(), cur_stream());
+                                  : sb200::launch_attn_fwd_tc(p, (int)q.size(2), status.data_ptr<int>(), cur_stream());
   TORCH_CHECK(rc == 0, "attn_fwd_tc launch failed (", rc, ")");
   return {out, lse2};
 }
@@ -1205,13 +1205,13 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> attn_bwd(
     const Tensor& lo, const Tensor& hi, const c10::optional<Tensor>& ke, const c10::optional<Tensor>& ve,
     const c10::optional<Tensor>& ext_idx, double scale, int64_t impl, const c10::optional<Tensor>& status, int64_t ext_block,
     bool ext_causal) {
-  // impl 0: mma.sync kernels; 1: tcgen05 kernels (head_dim 128, or 256 without extra keys; `status` receives a code if a bounded wait ran out)
+  // impl 0: mma.sync kernels; 1: tcgen05 kernels (head_dim 64 or 128, or 256 without extra keys; `status` receives a code if a bounded wait ran out)
   sb200::AttnParams p = make_params(q, k, v, lo, hi, ke, ve, ext_idx, scale);
   TORCH_CHECK(ext_block <= 0 || impl == 1, "block-structured extras run on the tcgen05 kernels only");
   use_block_extras(p, q, ext_block, ext_causal);
   const int64_t hd = q.size(2);
   if (impl == 1) {
-    TORCH_CHECK(hd == 128 || (hd == 256 && p.E == 0 && p.ext_block == 0), "attn_bwd: the tcgen05 kernels need head_dim 128, or 256 without extra keys");
+    TORCH_CHECK(hd == 64 || hd == 128 || (hd == 256 && p.E == 0 && p.ext_block == 0), "attn_bwd: the tcgen05 kernels need head_dim 64 or 128, or 256 without extra keys");
     TORCH_CHECK(status.has_value() && status->is_cuda() && status->scalar_type() == at::kInt && status->numel() >= 1);
   }
   check_heads(dout, "dout", hd);
@@ -1255,7 +1255,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> attn_bwd(
   p.tile_qmin = qmin.data_ptr<int>();
   p.tile_qmax = qmax.data_ptr<int>();
   const int rc = impl == 1 && hd == 256 ? sb200::launch_attn_bwd_wide_tc(p, qmin.data_ptr<int>(), qmax.data_ptr<int>(), status->data_ptr<int>(), cur_stream())
-                 : impl == 1 ? sb200::launch_attn_bwd_tc(p, qmin.data_ptr<int>(), qmax.data_ptr<int>(), status->data_ptr<int>(), cur_stream())
+                 : impl == 1 ? sb200::launch_attn_bwd_tc(p, (int)hd, qmin.data_ptr<int>(), qmax.data_ptr<int>(), status->data_ptr<int>(), cur_stream())
                            : sb200::launch_attn_bwd(p, (int)hd, qmin.data_ptr<int>(), qmax.data_ptr<int>(), cur_stream());
   TORCH_CHECK(rc == 0, "attn_bwd launch failed (", rc, ")");
   if (dke.numel() > 0) {  // both gradients of the extra keys in the inputs' type with one conversion

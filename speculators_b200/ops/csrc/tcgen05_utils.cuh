@@ -156,41 +156,53 @@ __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence
 // (partial sectors, one line per lane).  Instead the warp lays its 32 rows into shared memory
 // (16-byte chunks XOR-swizzled by the row so that neither side has bank conflicts) and then
 // writes whole rows: 8 lanes per 128-byte bf16 row, 16 lanes per 256-byte fp32 row.
-// `stage`: 4 KB (bf16) / 8 KB (fp32) private to the warp; `rows_valid`: rows of the warp's 32
-// that exist; `gbase`: element 0 of the warp's row 0; vals[i] is column i of the lane's row.
-__device__ __forceinline__ void store_rows64_bf16(unsigned char* stage, const float (&vals)[64], float mul, __nv_bfloat16* gbase,
-                                                  int64_t row_stride, int rows_valid, int lane) {
+// `stage`: 64 W bytes (bf16) / 128 W bytes (fp32) private to the warp, W = 32 or 64 columns; `rows_valid`: rows of the
+// warp's 32 that exist; `gbase`: element 0 of the warp's row 0; vals[i] is column i of the lane's row.
+template <int W>
+__device__ __forceinline__ uint32_t stage_row_chunk(int row, int chunk) {  // byte offset of a 16-byte chunk of a W-column bf16 row
+  return row * (W * 2) + ((chunk ^ (W == 64 ? row & 7 : (row >> 1) & 3)) << 4);
+}
+template <int W>
+__device__ __forceinline__ void store_rows_bf16(unsigned char* stage, const float (&vals)[W], float mul, __nv_bfloat16* gbase, int64_t row_stride,
+                                                int rows_valid, int lane) {
+  constexpr int L = W / 8;  // lanes a row
   __syncwarp();
 #pragma unroll
-  for (int c = 0; c < 8; ++c) {
+  for (int c = 0; c < L; ++c) {
     float f[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) f[i] = vals[c * 8 + i] * mul;
-    *reinterpret_cast<bf16x8*>(stage + lane * 128 + ((c ^ (lane & 7)) << 4)) = pack8(f);
+    *reinterpret_cast<bf16x8*>(stage + stage_row_chunk<W>(lane, c)) = pack8(f);
   }
   __syncwarp();
 #pragma unroll
-  for (int it = 0; it < 8; ++it) {
-    const int r = it * 4 + (lane >> 3), pc = lane & 7;
-    const bf16x8 v = *reinterpret_cast<const bf16x8*>(stage + r * 128 + ((pc ^ (r & 7)) << 4));
+  for (int it = 0; it < L; ++it) {
+    const int r = it * (32 / L) + lane / L, pc = lane % L;
+    const bf16x8 v = *reinterpret_cast<const bf16x8*>(stage + stage_row_chunk<W>(r, pc));
     if (r < rows_valid) st8(gbase + (int64_t)r * row_stride + pc * 8, v);
   }
   __syncwarp();
 }
-__device__ __forceinline__ void store_rows64_f32(unsigned char* stage, const float (&vals)[64], float* gbase, int64_t row_stride,
-                                                 int rows_valid, int lane) {
+// fp32 rows: `put(r, column, value)` for each of the warp's existing rows, 4 W bytes at a time across W / 4 lanes
+template <int W, typename Put>
+__device__ __forceinline__ void stage_rows_f32(unsigned char* stage, const float (&vals)[W], int rows_valid, int lane, Put put) {
+  constexpr int L = W / 4;
   __syncwarp();
-  float4* mine = reinterpret_cast<float4*>(stage + lane * 256);
+  float4* mine = reinterpret_cast<float4*>(stage + lane * (W * 4));
 #pragma unroll
-  for (int c = 0; c < 16; ++c) mine[c ^ (lane & 7)] = make_float4(vals[c * 4], vals[c * 4 + 1], vals[c * 4 + 2], vals[c * 4 + 3]);
+  for (int c = 0; c < L; ++c) mine[c ^ (lane & 7)] = make_float4(vals[c * 4], vals[c * 4 + 1], vals[c * 4 + 2], vals[c * 4 + 3]);
   __syncwarp();
 #pragma unroll
-  for (int it = 0; it < 16; ++it) {
-    const int r = it * 2 + (lane >> 4), pc = lane & 15;
-    const float4 v = reinterpret_cast<const float4*>(stage + r * 256)[pc ^ (r & 7)];
-    if (r < rows_valid) *reinterpret_cast<float4*>(gbase + (int64_t)r * row_stride + pc * 4) = v;
+  for (int it = 0; it < L; ++it) {
+    const int r = it * (32 / L) + lane / L, pc = lane % L;
+    const float4 v = reinterpret_cast<const float4*>(stage + r * (W * 4))[pc ^ (r & 7)];
+    if (r < rows_valid) put(r, pc * 4, v);
   }
   __syncwarp();
+}
+template <int W>
+__device__ __forceinline__ void store_rows_f32(unsigned char* stage, const float (&vals)[W], float* gbase, int64_t row_stride, int rows_valid, int lane) {
+  stage_rows_f32(stage, vals, rows_valid, lane, [&](int r, int c, float4 v) { *reinterpret_cast<float4*>(gbase + (int64_t)r * row_stride + c) = v; });
 }
 
 // ---- tile stores through shared memory -----------------------------------------------------

@@ -202,3 +202,9 @@ def test_anchored_blocks_run_their_block_keys_as_a_tile(window, non_causal, n_an
 def test_head_dim_256_tensor_core_kernels(T, nh, nkv, window, pattern):
     """One row, ungrouped heads, windows that start and end inside a tile, documents, padding rows that see nothing."""
     _run(T, nh, nkv, 256, step=0, window=window, pattern=pattern)
+
+
+@pytest.mark.parametrize("T,nh,nkv,step,window,pattern", [(513, 2, 2, 0, None, "single"), (700, 6, 2, 2, 100, "multi_pad"), (897, 4, 1, 1, None, "multi_pad")])
+def test_head_dim_64_tensor_core_kernels(T, nh, nkv, step, window, pattern):
+    """Ungrouped heads, windows that start and end inside a tile, extra keys, padding rows that see only them."""
+    _run(T, nh, nkv, 64, step=step, window=window, pattern=pattern)
