@@ -173,12 +173,13 @@ def _capturing(graph: torch.cuda.CUDAGraph, stream: torch.cuda.Stream):
 
     ``torch.cuda.graph`` collects garbage and gives the allocator's whole cache back to the driver first (0.1 s to
     seconds once another trainer's memory has been freed), because a capture cannot do so when it runs short.  The
-    warm-up left behind what the step needs as cached blocks, so the cache has to go only if that much is not free
-    beside it.  The collector stays off meanwhile: what it frees could make calls that a capture forbids."""
+    warm-up left behind what the step needs as cached blocks of its stream, so the cache has to go only if that much is
+    not free beside it.  The collector stays off meanwhile: what it frees could make calls that a capture forbids."""
     torch.cuda.synchronize()
     free, _ = torch.cuda.mem_get_info()
-    cached = torch.cuda.memory_reserved() - torch.cuda.memory_allocated()
-    if free < cached + cached // 8 + (1 << 30):
+    needed = sum(s["total_size"] - s["allocated_size"] for s in torch.cuda.memory_snapshot()
+                 if s["stream"] == stream.cuda_stream and tuple(s.get("segment_pool_id", (0, 0))) == (0, 0))
+    if free < needed + needed // 8 + (1 << 30):
         torch.cuda.empty_cache()
     collecting = gc.isenabled()
     gc.disable()
