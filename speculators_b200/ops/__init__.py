@@ -282,6 +282,90 @@ class _LinearFn(torch.autograd.Function):
         return dx, dw, dres, None, None
 
 
+_MAX_USES = 4  # of a weight in one product (the kernel's operand maps)
+# Half a wave of 256 x 256 tiles: below, the product runs on smaller tiles use by use, and is best started at once
+_GATHER_ELEMENTS = 37 * 65536
+
+
+class _SideWork:
+    """Weight gradients of one backward pass: gathered over the uses of a weight, run on a stream of their own."""
+
+    def __init__(self, main: torch.cuda.Stream):
+        self.main, self.stream = main, torch.cuda.Stream(main.device)
+        self.task = -1
+        self.held = []  # operands of what the side stream has queued
+        self.weights = []
+        self.pending: dict[tuple, tuple] = {}  # (weight's id, rows) -> (weight, uses gathered, launch)
+
+    def begin(self, task: int) -> None:
+        if self.task != task:
+            self.pending.clear()  # of a pass that ended in an exception
+            torch.autograd.Variable._execution_engine.queue_callback(self.finish)
+            self.task = task
+
+    def run(self, key: tuple) -> None:
+        weight, uses, launch = self.pending.pop(key)
+        self.stream.wait_stream(self.main)
+        with torch.cuda.stream(self.stream):
+            launch(uses)
+        self.held.append(uses)
+        self.weights.append(weight)
+        weight._side_work = self
+
+    def finish(self) -> None:
+        for key in list(self.pending):
+            self.pending[key][0]._grad_uses.pop(key[1:], None)  # uses that no gradient came back from
+            self.run(key)
+        self.main.wait_stream(self.stream)
+        for w in self.weights:
+            w._side_work = None
+        self.held.clear()  # memory goes back to the main stream's order, which now follows the side stream's
+        self.weights.clear()
+        self.task = -1
+
+
+_SIDE_WORK: dict[tuple[int, int], _SideWork] = {}  # by device and main stream (torch hands out streams from a fixed pool)
+
+
+def _wait_for_side_work(weight: torch.Tensor) -> None:
+    work = getattr(weight, "_side_work", None)
+    if work is not None:
+        torch.cuda.current_stream(weight.device).wait_stream(work.stream)
+
+
+def _note_use(weight: torch.Tensor, *rows) -> None:
+    """Called where a differentiated product uses ``weight`` (or rows of it): how many gradients to expect."""
+    if getattr(weight, "_flat_grad", None) is not None:
+        uses = weight.__dict__.setdefault("_grad_uses", {})
+        uses[rows] = uses.get(rows, 0) + 1
+
+
+def _gather_use(weight: torch.Tensor, rows: tuple, use: tuple, launch) -> None:
+    """One use's operands of a gradient that goes into the flat buffer.  ``launch(uses)`` forms the gradient of all uses as one
+    product once the last expected one (or ``_MAX_USES``) has come: training-time-test passes read and wrote every gradient
+    once a pass (uses of a small weight, whose product is bound by neither, are not waited for: ``_GATHER_ELEMENTS``).  It runs beside the rest of the backward pass, where nothing needs its result: on its own stream it fills
+    the SMs that the chain of input gradients leaves idle - the last wave of a product, the short element-wise kernels.  The
+    pass's end runs what is left and joins the streams, and so does any other gradient of the same weight."""
+    task = torch._C._current_graph_task_id()
+    if task < 0:
+        launch([use])
+        return
+    main = torch.cuda.current_stream(weight.device)
+    work = _SIDE_WORK.get((main.device_index, main.cuda_stream))
+    if work is None:
+        work = _SIDE_WORK[(main.device_index, main.cuda_stream)] = _SideWork(main)
+    work.begin(task)
+    key = (id(weight), *rows)
+    _, uses, _ = work.pending.setdefault(key, (weight, [], launch))
+    uses.append(use)
+    expected = weight.__dict__.setdefault("_grad_uses", {})
+    expected[rows] = expected.get(rows, 0) - 1
+    if expected[rows] <= 0 or len(uses) == _MAX_USES or weight.numel() < _GATHER_ELEMENTS:
+        if expected[rows] <= 0:
+            del expected[rows]
+        work.run(key)
+
+
 def _linear_backward(x2, weight, rows, dy, need_dx: bool, need_dw: bool):
     """``(dx, dw)`` of ``y = x2 @ weight[rows].T``; ``dw`` is ``None`` when the gradient went
     straight into the flat buffer the training engine attached to the weight."""
@@ -294,12 +378,16 @@ def _linear_backward(x2, weight, rows, dy, need_dx: bool, need_dw: bool):
         dx = _dgrad_gemm(dy2, w) if own else dy2 @ w
     if need_dw:
         flat = getattr(weight, "_flat_grad", None)
-        if flat is not None:
-            # the first gradient of these rows since the engine's zero_grad, which left the buffer uncleared, is stored
+        if flat is not None and own and _gemm_operand_ok(flat if r0 is None else flat[r0:r1]) and x2.shape[0] > 0:
+            def launch(uses):
+                # the first gradient of these rows since the engine's zero_grad, which left the buffer uncleared, is stored
+                target, accumulate = _param_grad_target(weight, beside=True)[:2] if r0 is None else _row_grad_target(weight, r0, r1)
+                native().gemm_wgrad_parts([u[0] for u in uses], [u[1] for u in uses], target, accumulate, gemm_status(target.device))
+
+            _gather_use(weight, (r0, r1), (dy2, x2), launch)
+        elif flat is not None:
             target, accumulate = _param_grad_target(weight)[:2] if r0 is None else _row_grad_target(weight, r0, r1)
-            if own and _gemm_operand_ok(target):
-                _wgrad_gemm(dy2, x2, target, accumulate=accumulate)
-            elif accumulate:
+            if accumulate:
                 target.addmm_(dy2.t(), x2)
             else:
                 torch.mm(dy2.t(), x2, out=target)
@@ -327,6 +415,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
         lead = x.shape[:-1]
         x2 = x.reshape(-1, x.shape[-1])
         res2 = residual.reshape(-1, residual.shape[-1]) if residual is not None else None
+        if weight.requires_grad:
+            _note_use(weight, r0, r1)
         y = _LinearFn.apply(x2, weight, res2, r0, r1)
         if len(lead) != 1:
             y = y.view(*lead, y.shape[-1])
@@ -362,10 +452,12 @@ def _grad_rows(d: torch.Tensor | None, width: int) -> torch.Tensor | None:
     return d2 if d2.stride(-1) == 1 and d2.stride(0) % 8 == 0 and d2.data_ptr() % 16 == 0 else d2.contiguous()
 
 
-def _param_grad_target(weight: torch.Tensor) -> tuple[torch.Tensor, bool, bool]:
+def _param_grad_target(weight: torch.Tensor, beside: bool = False) -> tuple[torch.Tensor, bool, bool]:
     """Where a kernel puts a parameter's gradient: ``(buffer, accumulate, attached)``.  With a flat gradient view attached
     by the training engine that view (stored into by the first gradient after ``zero_grad``, which left it uncleared, added
-    to by later ones; autograd then gets ``None``), else a fresh tensor."""
+    to by later ones; autograd then gets ``None``), else a fresh tensor.  ``beside``: called by what ``_gather_use`` runs."""
+    if not beside:
+        _wait_for_side_work(weight)
     flat = getattr(weight, "_flat_grad", None)
     if flat is None:
         return torch.empty_like(weight), False, False
@@ -380,6 +472,7 @@ def _param_grad_target(weight: torch.Tensor) -> tuple[torch.Tensor, bool, bool]:
 def clear_fresh_grad(p: torch.Tensor) -> None:
     """Zero what no gradient has been stored into since the engine's ``zero_grad``: all of the flat view
     (``_grad_fresh`` is ``True``) or the row intervals that ``_row_grad_target`` has left."""
+    _wait_for_side_work(p)
     fresh = getattr(p, "_grad_fresh", False)
     if fresh is False:
         return
@@ -581,6 +674,8 @@ def linear_swiglu(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor | None:
     if (not own_gemm_enabled() or os.environ.get("SB200_FUSED_SWIGLU", "1") == "0" or not _gemm_operand_ok(x2) or not _gemm_operand_ok(weight)
             or weight.shape[0] % 256 or weight.shape[1] != x2.shape[1]):
         return None
+    if weight.requires_grad and torch.is_grad_enabled():
+        _note_use(weight, None, None)
     h = _GateUpSwiGLUFn.apply(x2, weight)
     return h.view(*x.shape[:-1], h.shape[-1])
 
@@ -960,6 +1055,8 @@ def lm_head_loss_raw(op: str, hidden: torch.Tensor, weight: torch.Tensor, target
     plain store epilogue), so the two-kernel form is the default."""
     if not lm_head_loss_ok(op, hidden, weight, targets):
         return None
+    if weight.requires_grad and torch.is_grad_enabled():
+        _note_use(weight, None, None)
     return _LmHeadLossFn.apply(hidden, weight, targets, LOSS_OPS[op], shift, rows, active)
 
 

@@ -58,6 +58,9 @@ int launch_gemm_tn_tcgen05(const void*, const void*, void*, const void*, int, in
                            int*, int, cudaStream_t);
 int launch_gemm_tcgen05(const void*, const void*, void*, const void*, int, int, int, int64_t, int64_t, int64_t, int64_t, int, int, int,
                         int*, int, cudaStream_t);
+int launch_gemm_parts(int, const void* const*, const void* const*, const int*, const int64_t*, const int64_t*, void*, int, int, int64_t, int, int*, cudaStream_t);
+int launch_gemm_grouped_parts(int, const void* const*, const void* const*, const int*, const int64_t*, const int64_t*, const int* const*, void*, int, int, int,
+                              const int*, int, int*, cudaStream_t);
 int launch_gemm_stack(const void*, const void*, void*, const void*, int, int, int, int, int, int, float, float, int, int*, cudaStream_t);
 void launch_moe_group_plan(const int*, int, int*, int*, cudaStream_t);
 int launch_gemm_grouped(const void*, const void*, void*, int, int, int, int64_t, int64_t, int64_t, int, int, int, const int*, const int*, int, int*,
@@ -576,18 +579,61 @@ std::tuple<Tensor, Tensor> gemm_grouped_swiglu(const Tensor& x, const Tensor& w,
 }
 
 // dw[e] (=, +=) dy[seg_e, :]^T . x[seg_e, :]  (dw: [E, M, N], dy: [R, M], x: [R, N]); an expert without rows gets zeros (store) / is left alone (accumulate).
-void gemm_grouped_wgrad(const Tensor& dy, const Tensor& x, Tensor dw, bool accumulate, const Tensor& seg, const Tensor& mts, Tensor status) {
-  check_rows(dy, "dy");
-  check_rows(x, "x");
+void gemm_grouped_wgrad_parts(const std::vector<Tensor>& dy, const std::vector<Tensor>& x, Tensor dw, bool accumulate, const std::vector<Tensor>& seg,
+                              const Tensor& mts, Tensor status) {
   TORCH_CHECK(dw.is_cuda() && dw.scalar_type() == at::kBFloat16 && dw.dim() == 3 && dw.is_contiguous());
-  const int64_t E = dw.size(0), M = dw.size(1), N = dw.size(2), R = dy.size(0);
-  TORCH_CHECK(dy.size(1) == M && x.size(1) == N && x.size(0) == R && R % 128 == 0, "gemm_grouped_wgrad: shape mismatch");
-  TORCH_CHECK(seg.is_cuda() && seg.scalar_type() == at::kInt && seg.numel() == E + 1);
-  c10::cuda::CUDAGuard guard(x.device());
-  const int rc = sb200::launch_gemm_grouped(dy.data_ptr(), x.data_ptr(), dw.data_ptr(), (int)M, (int)N, (int)R, dy.stride(0), x.stride(0), N,
-                                            accumulate ? 1 : 0, 2, 1, seg.data_ptr<int>(), mts.data_ptr<int>(), (int)E, status.data_ptr<int>(),
-                                            cur_stream());
+  const int64_t E = dw.size(0), M = dw.size(1), N = dw.size(2);
+  const size_t n = dy.size();
+  TORCH_CHECK(n >= 1 && n <= 4 && x.size() == n && seg.size() == n, "gemm_grouped_wgrad: one to four uses");
+  const void *a[4], *b[4];
+  const int* sp[4];
+  int K[4];
+  int64_t lda[4], ldb[4];
+  for (size_t i = 0; i < n; ++i) {
+    check_rows(dy[i], "dy");
+    check_rows(x[i], "x");
+    TORCH_CHECK(dy[i].size(1) == M && x[i].size(1) == N && x[i].size(0) == dy[i].size(0) && dy[i].size(0) % 128 == 0, "gemm_grouped_wgrad: shape mismatch");
+    TORCH_CHECK(seg[i].is_cuda() && seg[i].scalar_type() == at::kInt && seg[i].numel() == E + 1);
+    a[i] = dy[i].data_ptr();
+    b[i] = x[i].data_ptr();
+    sp[i] = seg[i].data_ptr<int>();
+    K[i] = (int)dy[i].size(0);
+    lda[i] = dy[i].stride(0);
+    ldb[i] = x[i].stride(0);
+  }
+  c10::cuda::CUDAGuard guard(dw.device());
+  const int rc = sb200::launch_gemm_grouped_parts((int)n, a, b, K, lda, ldb, sp, dw.data_ptr(), (int)M, (int)N, accumulate ? 1 : 0, mts.data_ptr<int>(), (int)E,
+                                                  status.data_ptr<int>(), cur_stream());
   TORCH_CHECK(rc == 0, "gemm_grouped_wgrad launch failed (", rc, ")");
+}
+void gemm_grouped_wgrad(const Tensor& dy, const Tensor& x, Tensor dw, bool accumulate, const Tensor& seg, const Tensor& mts, Tensor status) {
+  gemm_grouped_wgrad_parts({dy}, {x}, dw, accumulate, {seg}, mts, status);
+}
+
+// dw (+)= sum_i dy_i^T . x_i: the weight gradient over several uses of a weight
+void gemm_wgrad_parts(const std::vector<Tensor>& dy, const std::vector<Tensor>& x, Tensor dw, bool accumulate, Tensor status) {
+  check_rows(dw, "dw");
+  const int64_t M = dw.size(0), N = dw.size(1);
+  const size_t n = dy.size();
+  TORCH_CHECK(n >= 1 && n <= 4 && x.size() == n, "gemm_wgrad_parts: one to four uses");
+  const void *a[4], *b[4];
+  int K[4];
+  int64_t lda[4], ldb[4];
+  for (size_t i = 0; i < n; ++i) {
+    check_rows(dy[i], "dy");
+    check_rows(x[i], "x");
+    TORCH_CHECK(dy[i].size(1) == M && x[i].size(1) == N && x[i].size(0) == dy[i].size(0) && dy[i].size(0) > 0, "gemm_wgrad_parts: shape mismatch");
+    a[i] = dy[i].data_ptr();
+    b[i] = x[i].data_ptr();
+    K[i] = (int)dy[i].size(0);
+    lda[i] = dy[i].stride(0);
+    ldb[i] = x[i].stride(0);
+  }
+  TORCH_CHECK(status.is_cuda() && status.scalar_type() == at::kInt && status.numel() >= 1);
+  c10::cuda::CUDAGuard guard(dw.device());
+  const int rc = sb200::launch_gemm_parts((int)n, a, b, K, lda, ldb, dw.data_ptr(), (int)M, (int)N, dw.stride(0), accumulate ? 1 : 0, status.data_ptr<int>(),
+                                          cur_stream());
+  TORCH_CHECK(rc == 0, "gemm_wgrad_parts launch failed (", rc, ")");
 }
 
 // lm_head product fused with the row loss: logits = x @ w^T on the tcgen05 kernel whose epilogue also
@@ -1335,6 +1381,8 @@ TORCH_LIBRARY(sb200, m) {
   m.def("moe_group_plan", &moe_group_plan);
   m.def("gemm_grouped_rows", &gemm_grouped_rows);
   m.def("gemm_grouped_wgrad", &gemm_grouped_wgrad);
+  m.def("gemm_wgrad_parts", &gemm_wgrad_parts);
+  m.def("gemm_grouped_wgrad_parts", &gemm_grouped_wgrad_parts);
   m.def("gemm_tn_variant", &gemm_tn_variant);
   m.def("attn_fwd", &attn_fwd);
   m.def("attn_fwd_tc", &attn_fwd_tc);

@@ -751,12 +751,44 @@ constexpr int P_STAGE_OUT_BYTES = 8 * 4096;  // one staging area per epilogue wa
 // statistics of the lm_head epilogue, and the addend of short-contraction weight gradients, set the pace of the tile).
 constexpr int P_THREADS = 320, P_EPI_COLS = 128;
 
-template <int KSUB, bool A_MN = false, bool B_MN = false>
+// A contraction in parts: the weight gradients of a weight that was used several times (training-time-test passes), each
+// use with its own pair of operands.  As one product per use every product but the first read and wrote the gradient once
+// more, and its tiles were short: at 736 rows the epilogue took longer than the products.  One tile loop over all parts
+// accumulates them in tensor memory - in fp32, without the roundings in between.
+//   24576 x 4096 x 736, three uses: 463 us as separate products, 286 as one; 16384 x 2048 x 1001: 191 and 133 us.
+constexpr int kMoreParts = 3;
+struct MoreParts {
+  CUtensorMap a[kMoreParts], b[kMoreParts];
+  const int* seg[kMoreParts];  // grouped contraction: the part's own segments
+  int num_kb[kMoreParts];
+  int n;
+};
+struct NoParts {};
+template <bool PARTS> struct PartsArg { typedef NoParts type; };
+template <> struct PartsArg<true> { typedef MoreParts type; };
+// 128-wide contraction steps of part i for this tile, and where they start
+__device__ __forceinline__ int part_steps(const Params& p, const MoreParts& more, int i, int tile, int per, int& k0) {
+  k0 = 0;
+  if (p.grp.mode != kGroupK) return more.num_kb[i];
+  const int e = tile / per;
+  k0 = more.seg[i][e];
+  return (more.seg[i][e + 1] - k0) >> 7;
+}
+__device__ __forceinline__ int more_steps(const Params& p, const MoreParts& more, int tile, int per) {
+  int sum = 0, k0;
+  for (int i = 0; i < more.n; ++i) sum += part_steps(p, more, i, tile, per, k0);
+  return sum;
+}
+__device__ __forceinline__ int more_steps(const Params&, const NoParts&, int, int) { return 0; }
+
+template <int KSUB, bool A_MN = false, bool B_MN = false, bool PARTS = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P_THREADS, 1)
 gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                    const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_h, const Params p) {
+                    const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_h, const Params p,
+                    const __grid_constant__ typename PartsArg<PARTS>::type more) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  static_assert(!PARTS || (A_MN && B_MN), "parts are those of weight gradients");
   static_assert(KSUB == 2 || (!A_MN && !B_MN), "MN-major operands are staged as 128-row boxes: KSUB must be 2");
   constexpr int P_STAGES = 6 / KSUB;
   constexpr int P_STAGE_BYTES = KSUB * P_SUB_BYTES;
@@ -802,23 +834,33 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       bool ok = true;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
         const TileInfo ti = decode_tile<B_MN>(p, tile, tiles_m, tiles_n, num_kb, (int)rank);
-        for (int kb = 0; kb < ti.num_kb; ++kb) {
-          if (!(ok = mbar_wait(smem_addr(&bar_empty[stage]), phase ^ 1, p.status, kTimeoutProducer))) break;
-          const uint32_t full_local = smem_addr(&bar_full[stage]);
-          if (leader) mbar_expect_tx(full_local, 2 * P_STAGE_BYTES);
-          const uint32_t full_leader = map_to_cta(full_local, 0);
-          const uint32_t sa = smem_addr(smem + stage * P_STAGE_BYTES);
-          // Elements outside the matrices read as zeros (TMA fill).  K-major operand: sub-tile u =
-          // 128 rows x 64 contraction columns.  MN-major operand: sub-tile u = 128 contraction rows x
-          // 64 MN-columns (MN-elements 64u .. 64u+63 of this CTA's 128).  Either way 16 KB at the same place.
+        auto load_steps = [&](const CUtensorMap* ma, const CUtensorMap* mb, int a_k0, int b_k0, int steps) {
+          for (int kb = 0; kb < steps; ++kb) {
+            if (!(ok = mbar_wait(smem_addr(&bar_empty[stage]), phase ^ 1, p.status, kTimeoutProducer))) break;
+            const uint32_t full_local = smem_addr(&bar_full[stage]);
+            if (leader) mbar_expect_tx(full_local, 2 * P_STAGE_BYTES);
+            const uint32_t full_leader = map_to_cta(full_local, 0);
+            const uint32_t sa = smem_addr(smem + stage * P_STAGE_BYTES);
+            // Elements outside the matrices read as zeros (TMA fill).  K-major operand: sub-tile u =
+            // 128 rows x 64 contraction columns.  MN-major operand: sub-tile u = 128 contraction rows x
+            // 64 MN-columns (MN-elements 64u .. 64u+63 of this CTA's 128).  Either way 16 KB at the same place.
 #pragma unroll
-          for (int u = 0; u < KSUB; ++u) {
-            if (A_MN) tma_load_3d_pair(sa + u * P_SUB_BYTES, &map_a, full_leader, ti.a_m + u * 64, ti.a_k0 + kb * STAGE_K, ti.z);
-            else tma_load_3d_pair(sa + u * P_SUB_BYTES, &map_a, full_leader, ti.a_k0 + kb * STAGE_K + u * BK, ti.a_m, ti.z);
-            if (B_MN) tma_load_3d_pair(sa + u * P_SUB_BYTES + P_A_BYTES, &map_b, full_leader, ti.b_n + u * 64, ti.b_k0 + kb * STAGE_K, ti.z);
-            else tma_load_3d_pair(sa + u * P_SUB_BYTES + P_A_BYTES, &map_b, full_leader, ti.b_k0 + kb * STAGE_K + u * BK, ti.b_n, ti.z);
+            for (int u = 0; u < KSUB; ++u) {
+              if (A_MN) tma_load_3d_pair(sa + u * P_SUB_BYTES, ma, full_leader, ti.a_m + u * 64, a_k0 + kb * STAGE_K, ti.z);
+              else tma_load_3d_pair(sa + u * P_SUB_BYTES, ma, full_leader, a_k0 + kb * STAGE_K + u * BK, ti.a_m, ti.z);
+              if (B_MN) tma_load_3d_pair(sa + u * P_SUB_BYTES + P_A_BYTES, mb, full_leader, ti.b_n + u * 64, b_k0 + kb * STAGE_K, ti.z);
+              else tma_load_3d_pair(sa + u * P_SUB_BYTES + P_A_BYTES, mb, full_leader, b_k0 + kb * STAGE_K + u * BK, ti.b_n, ti.z);
+            }
+            if (++stage == P_STAGES) { stage = 0; phase ^= 1; }
           }
-          if (++stage == P_STAGES) { stage = 0; phase ^= 1; }
+        };
+        load_steps(&map_a, &map_b, ti.a_k0, ti.b_k0, ti.num_kb);
+        if constexpr (PARTS) {
+          for (int i = 0; i < more.n && ok; ++i) {
+            int k0;
+            const int steps = part_steps(p, more, i, tile, tiles_m * tiles_n, k0);
+            load_steps(&more.a[i], &more.b[i], k0, k0, steps);
+          }
         }
       }
       // tail: stay until the MMAs that read this CTA's last slots have retired (their
@@ -840,7 +882,7 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         if (!(ok = mbar_wait(smem_addr(&bar_acc_empty[acc]), ((local >> 1) & 1) ^ 1, p.status, kTimeoutMma))) break;
         fence_after_sync();
         const uint32_t tmem_d = tmem_base + acc * BN;
-        const int tile_kb = decode_tile<B_MN>(p, tile, tiles_m, tiles_n, num_kb, 0).num_kb;
+        const int tile_kb = decode_tile<B_MN>(p, tile, tiles_m, tiles_n, num_kb, 0).num_kb + more_steps(p, more, tile, tiles_m * tiles_n);
         for (int kb = 0; kb < tile_kb; ++kb) {
           if (!(ok = mbar_wait(smem_addr(&bar_full[stage]), phase, p.status, kTimeoutMma))) break;
           fence_after_sync();
@@ -876,7 +918,7 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       const int acc = local & 1;
       const TileInfo ti = decode_tile<B_MN>(p, tile, tiles_m, tiles_n, num_kb, (int)rank);
       const int row = ti.c_row0 + quarter * 32 + lane, n0 = ti.n0 + chalf * P_EPI_COLS;
-      const bool zero = ti.num_kb == 0;
+      const bool zero = ti.num_kb + more_steps(p, more, tile, tiles_m * tiles_n) == 0;
       RowPrefetch<P_EPI_COLS> pre;
       const bool with_stats = p.rs.targets != nullptr, gated = p.epilogue == kSwiGLU;
       if (with_stats) prefetch_targets<P_EPI_COLS>(p, row, n0, pre);
@@ -1161,6 +1203,16 @@ static int choose_variant(int M, int N, int K, int batch, int symmetric) {
   return best;
 }
 
+// Further uses of a weight whose gradient is one product (see MoreParts); the first is the plain a, b, K.
+struct PartsSpec {
+  int n = 0;
+  const void* a[tc::kMoreParts];
+  const void* b[tc::kMoreParts];
+  int K[tc::kMoreParts];
+  int64_t lda[tc::kMoreParts], ldb[tc::kMoreParts];
+  const int* seg[tc::kMoreParts];
+};
+
 // What a stack of products adds to a single one; see Params.
 struct BatchSpec {
   int batch = 1;
@@ -1180,7 +1232,7 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
                             int64_t ldb, int64_t ldc, int64_t ldr, int epilogue, int a_mn, int b_mn, int* status, int variant,
                             const void* stats_targets, int64_t stats_ldt, int stats_t_rows, int stats_shift, float* stats_partial,
                             const tc::Grouping* grp, cudaStream_t stream, const tc::Scatter* scatter = nullptr, void* gated_h = nullptr,
-                            int64_t gated_ldh = 0, const BatchSpec* batched = nullptr) {
+                            int64_t gated_ldh = 0, const BatchSpec* batched = nullptr, const PartsSpec* parts = nullptr) {
   using namespace tc;
   static const BatchSpec one{};
   const BatchSpec& bs = batched != nullptr ? *batched : one;
@@ -1192,7 +1244,7 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
   if (configured.needed()) {
     bool ok = allow_smem(gemm_tn_2cta_kernel<1>, smem_pair) && allow_smem(gemm_tn_2cta_kernel<2>, smem_pair) &&
               allow_smem(gemm_tn_2cta_kernel<2, false, true>, smem_pair) && allow_smem(gemm_tn_2cta_kernel<2, true, false>, smem_pair) &&
-              allow_smem(gemm_tn_2cta_kernel<2, true, true>, smem_pair);
+              allow_smem(gemm_tn_2cta_kernel<2, true, true>, smem_pair) && allow_smem(gemm_tn_2cta_kernel<2, true, true, true>, smem_pair);
     ok = ok && allow_smem(gemm_split_kernel<2, false, false>, smem_pair) && allow_smem(gemm_split_kernel<2, false, true>, smem_pair) &&
          allow_smem(gemm_split_kernel<2, true, false>, smem_pair) && allow_smem(gemm_split_kernel<2, true, true>, smem_pair);
     ok = ok && allow_smem(gemm_split_kernel<4, false, false>, smem_pair) && allow_smem(gemm_split_kernel<4, false, true>, smem_pair) &&
@@ -1252,7 +1304,12 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
   // Stores through staging: C must be a matrix that TMA can address, and a warp's 32 rows must not straddle an expert.
   CUtensorMap map_c = map_a, map_h = map_a;
   const bool reads_ok = epilogue != kAddResidual || ((ldr & 7) == 0 && (reinterpret_cast<uintptr_t>(residual) & 15) == 0);
-  if (scatter == nullptr && stats_targets == nullptr && (N & 7) == 0 && (ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(c) & 15) == 0 && reads_ok &&
+  // An epilogue that reads C or a residual on pair tiles stores whole sectors straight from registers: with the addend's loads
+  // it is the epilogue that sets the pace at short contractions, and waiting for the staging area to be read lengthens it
+  // (weight gradients added up: 24576 x 4096 x 736 195 us staged, 175 direct; 4096 x 14336 x 2048 214 and 194).
+  const bool direct = (epilogue == kAccumulate || epilogue == kAddResidual) && variant == kPair && !symmetric && (N & 127) == 0 && (ldc & 15) == 0 &&
+                      (reinterpret_cast<uintptr_t>(c) & 31) == 0;
+  if (!direct && scatter == nullptr && stats_targets == nullptr && (N & 7) == 0 && (ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(c) & 15) == 0 && reads_ok &&
       (grp == nullptr || grp->mode == kGroupRows || (M & 127) == 0)) {
     const int64_t rows = grp != nullptr && grp->mode == kGroupK ? (int64_t)grp->num_groups * M : M;
     rc = make_map_bf16_stack(&map_c, c, rows, N, ldc, 32, bs.batch, bs.c_stride);
@@ -1263,6 +1320,19 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
     }
     if (rc) return rc;
     p.staged = 1;
+  }
+  MoreParts more{};
+  if (parts != nullptr) {
+    if (!a_mn || !b_mn || variant != kPair || bs.batch != 1 || parts->n > kMoreParts) return -9;
+    more.n = parts->n;
+    for (int i = 0; i < parts->n; ++i) {
+      if ((parts->lda[i] & 7) || (parts->ldb[i] & 7) || (reinterpret_cast<uintptr_t>(parts->a[i]) & 15) || (reinterpret_cast<uintptr_t>(parts->b[i]) & 15)) return -1;
+      rc = make_map_bf16_stack(&more.a[i], parts->a[i], parts->K[i], M, parts->lda[i], mn_rows, 1, 0);
+      if (rc == 0) rc = make_map_bf16_stack(&more.b[i], parts->b[i], parts->K[i], N, parts->ldb[i], mn_rows, 1, 0);
+      if (rc) return rc;
+      more.num_kb[i] = (parts->K[i] + 2 * BK - 1) / (2 * BK);
+      more.seg[i] = parts->seg[i];
+    }
   }
   count_launch(1);
   const int pair_tiles = (int)pair_tile_count(M, N, bs.batch, p.symmetric);
@@ -1278,11 +1348,12 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
     // grouped: the number of tiles is known on the device only; every pair looks for work
     const int tiles = grp != nullptr ? kMaxPairs : pair_tiles;
     const int grid = 2 * (tiles < kMaxPairs ? tiles : kMaxPairs);
-    if (a_mn && b_mn) launch_pdl(gemm_tn_2cta_kernel<2, true, true>, grid, P_THREADS, smem_pair, stream, map_a, map_b, map_c, map_h, p);
-    else if (a_mn) launch_pdl(gemm_tn_2cta_kernel<2, true, false>, grid, P_THREADS, smem_pair, stream, map_a, map_b, map_c, map_h, p);
-    else if (b_mn) launch_pdl(gemm_tn_2cta_kernel<2, false, true>, grid, P_THREADS, smem_pair, stream, map_a, map_b, map_c, map_h, p);
-    else if (variant == kPair) launch_pdl(gemm_tn_2cta_kernel<2>, grid, P_THREADS, smem_pair, stream, map_a, map_b, map_c, map_h, p);
-    else launch_pdl(gemm_tn_2cta_kernel<1>, grid, P_THREADS, smem_pair, stream, map_a, map_b, map_c, map_h, p);
+    if (more.n > 0) launch_pdl(gemm_tn_2cta_kernel<2, true, true, true>, grid, P_THREADS, smem_pair, stream, map_a, map_b, map_c, map_h, p, more);
+    else if (a_mn && b_mn) launch_pdl(gemm_tn_2cta_kernel<2, true, true>, grid, P_THREADS, smem_pair, stream, map_a, map_b, map_c, map_h, p, NoParts{});
+    else if (a_mn) launch_pdl(gemm_tn_2cta_kernel<2, true, false>, grid, P_THREADS, smem_pair, stream, map_a, map_b, map_c, map_h, p, NoParts{});
+    else if (b_mn) launch_pdl(gemm_tn_2cta_kernel<2, false, true>, grid, P_THREADS, smem_pair, stream, map_a, map_b, map_c, map_h, p, NoParts{});
+    else if (variant == kPair) launch_pdl(gemm_tn_2cta_kernel<2>, grid, P_THREADS, smem_pair, stream, map_a, map_b, map_c, map_h, p, NoParts{});
+    else launch_pdl(gemm_tn_2cta_kernel<1>, grid, P_THREADS, smem_pair, stream, map_a, map_b, map_c, map_h, p, NoParts{});
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
@@ -1296,6 +1367,36 @@ int launch_gemm_tcgen05(const void* a, const void* b, void* c, const void* resid
 int launch_gemm_tn_tcgen05(const void* a, const void* b, void* c, const void* residual, int M, int N, int K, int64_t lda,
                            int64_t ldb, int64_t ldc, int64_t ldr, int epilogue, int* status, int variant, cudaStream_t stream) {
   return launch_gemm_tcgen05(a, b, c, residual, M, N, K, lda, ldb, ldc, ldr, epilogue, 0, 0, status, variant, stream);
+}
+
+// c[M, N] (+)= sum_i a_i[K_i, M]^T . b_i[K_i, N]: one launch where pair tiles are the form for the whole contraction, else one each
+// (small products are not bound by their epilogue, and have better forms).
+int launch_gemm_parts(int n, const void* const* a, const void* const* b, const int* K, const int64_t* lda, const int64_t* ldb, void* c, int M, int N,
+                      int64_t ldc, int accumulate, int* status, cudaStream_t stream) {
+  if (n < 1 || n > tc::kMoreParts + 1) return -9;
+  int total = 0;
+  PartsSpec parts;
+  for (int i = 0; i < n; ++i) {
+    if (K[i] <= 0) return -9;
+    total += (K[i] + 127) / 128 * 128;
+    if (i == 0) continue;
+    parts.a[i - 1] = a[i];
+    parts.b[i - 1] = b[i];
+    parts.K[i - 1] = K[i];
+    parts.lda[i - 1] = lda[i];
+    parts.ldb[i - 1] = ldb[i];
+    parts.seg[i - 1] = nullptr;
+  }
+  parts.n = n - 1;
+  if (n > 1 && choose_variant(M, N, total, 1, 0) == kPair)
+    return launch_gemm_impl(a[0], b[0], c, nullptr, M, N, K[0], lda[0], ldb[0], ldc, 0, accumulate ? 1 : 0, 1, 1, status, kPair, nullptr, 0, 0, 0, nullptr,
+                            nullptr, stream, nullptr, nullptr, 0, nullptr, &parts);
+  for (int i = 0; i < n; ++i) {
+    const int rc = launch_gemm_impl(a[i], b[i], c, nullptr, M, N, K[i], lda[i], ldb[i], ldc, 0, accumulate || i > 0 ? 1 : 0, 1, 1, status, 0, nullptr, 0, 0, 0,
+                                    nullptr, nullptr, stream);
+    if (rc) return rc;
+  }
+  return 0;
 }
 
 // ---- stacks of products (Newton-Schulz iterations of equally shaped matrices) ----------------------
@@ -1370,6 +1471,25 @@ int launch_gemm_grouped(const void* a, const void* b, void* c, int M, int N, int
   const int a_mn = mode == tc::kGroupK ? 1 : 0;
   return launch_gemm_impl(a, b, c, nullptr, M, N, K, lda, ldb, ldc, 0, epilogue, a_mn, mode == tc::kGroupK ? 1 : b_mn, status, 3, nullptr, 0, 0, 0,
                           nullptr, &grp, stream);
+}
+
+// mode 2 over several uses, each with its own operands and segments: c_e (+)= sum_i a_i[seg_i,e, M]^T . b_i[seg_i,e, N]
+int launch_gemm_grouped_parts(int n, const void* const* a, const void* const* b, const int* K, const int64_t* lda, const int64_t* ldb, const int* const* seg,
+                              void* c, int M, int N, int accumulate, const int* mtile_start, int num_groups, int* status, cudaStream_t stream) {
+  if (n < 1 || n > tc::kMoreParts + 1) return -9;
+  PartsSpec parts;
+  parts.n = n - 1;
+  for (int i = 1; i < n; ++i) {
+    parts.a[i - 1] = a[i];
+    parts.b[i - 1] = b[i];
+    parts.K[i - 1] = K[i];
+    parts.lda[i - 1] = lda[i];
+    parts.ldb[i - 1] = ldb[i];
+    parts.seg[i - 1] = seg[i];
+  }
+  const tc::Grouping grp{tc::kGroupK, num_groups, seg[0], mtile_start};
+  return launch_gemm_impl(a[0], b[0], c, nullptr, M, N, K[0], lda[0], ldb[0], N, 0, accumulate ? 1 : 0, 1, 1, status, kPair, nullptr, 0, 0, 0, nullptr, &grp,
+                          stream, nullptr, nullptr, 0, nullptr, n > 1 ? &parts : nullptr);
 }
 
 // mode 1 with stacked [gate; up] experts [E, 2 I, K]: gate_up[R, 2 I] and h[R, I] = silu(gate) * up.

@@ -54,9 +54,19 @@ class _MoEExpertsFn(torch.autograd.Function):
         def weight_gradient(needed, dy, rows, w):
             if not needed:
                 return None
-            dw, accumulate, attached = ops._param_grad_target(w)  # noqa: SLF001
-            nat.gemm_grouped_wgrad(dy, rows, dw, accumulate, seg, tiles, status)
-            return None if attached else dw
+            flat = getattr(w, "_flat_grad", None)
+            if flat is None:
+                dw = torch.empty_like(w)
+                nat.gemm_grouped_wgrad(dy, rows, dw, False, seg, tiles, status)
+                return dw
+
+            def launch(uses):
+                target, accumulate, _ = ops._param_grad_target(w, beside=True)  # noqa: SLF001
+                dys, xs, segs = (list(part) for part in zip(*uses))
+                nat.gemm_grouped_wgrad_parts(dys, xs, target, accumulate, segs, tiles, status)
+
+            ops._gather_use(w, ("experts",), (dy, rows, seg), launch)  # noqa: SLF001
+            return None
 
         dw_d = weight_gradient(need[4], dy_pad, h, w_d)
         dx = dw_gu = None
@@ -80,4 +90,8 @@ def moe_experts(x, top_p, top_e, gate_up, down, shared=None, shared_gate=None, r
     def rows(t):
         return None if t is None else t.contiguous()
 
+    if torch.is_grad_enabled():
+        for w in (gate_up, down):
+            if w.requires_grad:
+                ops._note_use(w, "experts")  # noqa: SLF001
     return _MoEExpertsFn.apply(rows(x), rows(top_p), rows(top_e), gate_up, down, rows(shared), rows(shared_gate), rows(residual))

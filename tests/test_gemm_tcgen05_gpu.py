@@ -242,3 +242,42 @@ def test_gate_up_product_with_swiglu_epilogue_matches_two_step_form(T, H, I, mon
     # same accumulation and the same rounding points as the two-step form
     assert torch.equal(h1, h0)
     assert torch.equal(dx1, dx0) and torch.equal(dw1, dw0)
+
+
+# ---- gradients of a weight that is used several times ---------------------------------------------------
+# small products (one launch each), pair tiles with one to four uses, ragged rows, every contraction remainder
+@pytest.mark.parametrize("M,N,Ks", [(128, 64, (128, 100)), (2048, 4096, (300,)), (4096, 2560, (1001, 128)), (5120, 2048, (64, 1, 257)), (2048, 8192, (736, 735, 734, 733))])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_weight_gradient_over_several_uses(M, N, Ks, accumulate):
+    torch.manual_seed(M)
+    dy = [(torch.randn(k, M, device="cuda") * 0.1).bfloat16() for k in Ks]
+    x = [torch.randn(k, N, device="cuda").bfloat16() for k in Ks]
+    dw = torch.randn(M, N, device="cuda").bfloat16()
+    want = sum(a.float().t() @ b.float() for a, b in zip(dy, x)) + (dw.float() if accumulate else 0)
+    ops.native().gemm_wgrad_parts(dy, x, dw, accumulate, ops.gemm_status(dw.device))
+    ops.check_gemm_status()
+    assert (dw.float() - want).abs().max() <= 0.01 * want.abs().max()
+
+
+@pytest.mark.parametrize("counts", [[[300, 0, 17], [0, 0, 5]], [[1, 200, 0], [128, 0, 0], [0, 3, 400], [256, 256, 0]]])
+def test_grouped_weight_gradient_over_several_uses(counts):
+    """Segments of each use's own; an expert without rows in any of them gets zeros."""
+    torch.manual_seed(0)
+    E, M, N = 3, 512, 256
+    dys, xs, segs, want = [], [], [], torch.zeros(E, M, N, device="cuda")
+    for c in counts:
+        plan = ops.GroupPlan(torch.tensor(c, device="cuda"), sum(c))
+        dy, x = torch.zeros(plan.capacity, M, device="cuda"), torch.zeros(plan.capacity, N, device="cuda")
+        seg = plan.seg.tolist()
+        for e, n in enumerate(c):
+            dy[seg[e]: seg[e] + n], x[seg[e]: seg[e] + n] = torch.randn(n, M, device="cuda") * 0.1, torch.randn(n, N, device="cuda")
+        dys.append(dy.bfloat16())
+        xs.append(x.bfloat16())
+        segs.append(plan.seg)
+        for e in range(E):
+            rows = slice(seg[e], seg[e + 1])
+            want[e] += dys[-1][rows].float().t() @ xs[-1][rows].float()
+    dw = torch.full((E, M, N), float("nan"), device="cuda", dtype=torch.bfloat16)
+    ops.native().gemm_grouped_wgrad_parts(dys, xs, dw, False, segs, plan.mtile_start, ops.gemm_status(dw.device))
+    ops.check_gemm_status()
+    assert (dw.float() - want).abs().max() <= 0.01 * want.abs().max()

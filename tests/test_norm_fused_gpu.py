@@ -107,3 +107,34 @@ def test_row_slices_of_a_flat_gradient_are_stored_then_added():
     assert torch.isnan(w._flat_grad[256:]).all()
     ops.clear_fresh_grad(w)
     assert (w._flat_grad[256:] == 0).all() and (w._flat_grad.float() - want).abs().max() <= 0.02 * want.abs().max()
+
+
+@pytest.mark.parametrize("rows,K,N", [(64, 128, 128), (1001, 512, 768)])
+def test_weight_gradients_beside_the_backward_pass(rows, K, N):
+    """Several uses of a weight, a gradient that reaches it another way, and a pass that ends in an exception."""
+    torch.manual_seed(rows)
+    w = torch.randn(N, K, device="cuda").bfloat16().requires_grad_()
+    x = torch.randn(rows, K, device="cuda").bfloat16().requires_grad_()
+    w._flat_grad, w._grad_fresh = torch.full_like(w, float("nan")), True
+    w.grad = w._flat_grad
+
+    def hook(g):
+        ops.clear_fresh_grad(w)
+        return g
+
+    w.register_hook(hook)
+    stop = ops.linear(x, w)
+    stop.register_hook(lambda g: (_ for _ in ()).throw(RuntimeError("stop")))
+    with pytest.raises(RuntimeError, match="stop"):
+        (ops.linear(stop.new_ones(rows, K) * 0, w).sum() + stop.sum()).backward()
+    w._grad_fresh = True
+    y = ops.linear(x, w)
+    z = ops.linear(y[:, :K].contiguous(), w) if N >= K else y
+    (z.float().pow(2).mean() + (w.float() * 0.5).sum()).backward()
+    got = w._flat_grad.float()
+    xf, wf = x.detach().float().requires_grad_(), w.detach().float().requires_grad_()
+    yf = xf @ wf.t()
+    zf = yf[:, :K].bfloat16().float().detach() + (yf[:, :K] - yf[:, :K].detach())
+    zf = zf @ wf.t() if N >= K else yf
+    (zf.pow(2).mean() + (wf * 0.5).sum()).backward()
+    assert (got - wf.grad).abs().max() <= 0.02 * wf.grad.abs().max()
