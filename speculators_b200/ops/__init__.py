@@ -360,7 +360,10 @@ def _gather_use(weight: torch.Tensor, rows: tuple, use: tuple, launch) -> None:
     uses.append(use)
     expected = weight.__dict__.setdefault("_grad_uses", {})
     expected[rows] = expected.get(rows, 0) - 1
-    if expected[rows] <= 0 or len(uses) == _MAX_USES or weight.numel() < _GATHER_ELEMENTS:
+    # contractions of 8192 rows are long enough on their own (28672 x 4096, three uses: 4380 us apart, 4430 together;
+    # of 2048 rows 1150 and 1075); rows grouped by expert are few for each
+    whole = weight.numel() < _GATHER_ELEMENTS or (weight.dim() == 2 and use[0].shape[0] > 6144)
+    if expected[rows] <= 0 or len(uses) == _MAX_USES or whole:
         if expected[rows] <= 0:
             del expected[rows]
         work.run(key)

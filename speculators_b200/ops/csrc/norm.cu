@@ -40,49 +40,89 @@ __device__ __forceinline__ float round_bf16(float v) { return __bfloat162float(_
 
 SB200_BOUNDS_RECORD
 
+// Sum over the block with one barrier: `slot` alternates, so that a slot is written again only after everybody has passed
+// the barrier behind its last reading.  The order of the additions is block_sum's.
+template <int THREADS>
+__device__ __forceinline__ float row_sum(float v, float (&scratch)[2][THREADS / 32], int slot) {
+  constexpr int W = THREADS / 32;
+  v = warp_sum(v);
+  if ((threadIdx.x & 31) == 0) scratch[slot][threadIdx.x >> 5] = v;
+  __syncthreads();
+  float s[W];
+#pragma unroll
+  for (int i = 0; i < W; ++i) s[i] = scratch[slot][i];
+#pragma unroll
+  for (int half = W / 2; half > 0; half >>= 1)
+#pragma unroll
+    for (int i = 0; i < half; ++i) s[i] += s[i + half];
+  return s[0];
+}
+
+// Blocks an SM runs at once, by registers; the grid is no larger (a second, part-filled wave took as long as the first),
+// and evens out how many rows its blocks walk.
+template <int NV, int THREADS> constexpr int kFwdBlocks = THREADS == 512 ? 1 : NV == 2 ? 5 : NV == 4 ? 4 : 2;
+
 template <int NV, int THREADS>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, kFwdBlocks<NV, THREADS>)
 rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                    const int64_t* __restrict__ row_index, __nv_bfloat16* __restrict__ y,
                    float* __restrict__ rstd_out, int rows, int H, int64_t x_stride,
                    int64_t y_stride, float eps, int64_t src_rows, NormWeight nw) {
   pdl_begin();
-  __shared__ float scratch[33];
+  __shared__ float scratch[2][THREADS / 32];
   const int nvec = H >> 3;
-  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
+  bf16x8 cur[NV], next[NV];
+  bool ok = false, next_ok = false;  // false only in the debug build
+  auto fetch = [&](int r, bf16x8 (&to)[NV]) -> bool {
     const int64_t src = row_index ? row_index[r] : (int64_t)r;
-    if (!SB200_IN_RANGE(src, src_rows, 1)) continue;  // debug build only
+    if (!SB200_IN_RANGE(src, src_rows, 1)) return false;
     const __nv_bfloat16* xr = x + src * x_stride;
-    float cache[NV][8];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int v = threadIdx.x + i * THREADS;
+      if (v < nvec) to[i] = ld8(xr + (v << 3));
+    }
+    return true;
+  };
+  int r = blockIdx.x, slot = 0;
+  if (r < rows) ok = fetch(r, cur);
+  for (; r < rows; r += gridDim.x, slot ^= 1) {
+    if (r + (int)gridDim.x < rows) next_ok = fetch(r + gridDim.x, next);  // in flight during this row's reduction
     float ss = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int v = threadIdx.x + i * THREADS;
-      if (v < nvec) {
-        unpack8(ld8(xr + (v << 3)), cache[i]);
+      if (ok && v < nvec) {
+        float xv[8];
+        unpack8(cur[i], xv);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) ss += cache[i][j] * cache[i][j];
+        for (int j = 0; j < 8; ++j) ss += xv[j] * xv[j];
       }
     }
-    ss = block_sum(ss, scratch);
+    ss = row_sum<THREADS>(ss, scratch, slot);
     const float rstd = rsqrtf(ss / (float)H + eps);
-    if (threadIdx.x == 0 && rstd_out) rstd_out[r] = rstd;
+    if (ok && threadIdx.x == 0 && rstd_out) rstd_out[r] = rstd;
     __nv_bfloat16* yr = y + (int64_t)r * y_stride;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int v = threadIdx.x + i * THREADS;
-      if (v < nvec) {
-        float wv[8], o[8];
+      if (ok && v < nvec) {
+        float xv[8], wv[8], o[8];
+        unpack8(cur[i], xv);
         nw.load(w + (v << 3), wv);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = nw.apply(cache[i][j] * rstd, wv[j]);
+        for (int j = 0; j < 8; ++j) o[j] = nw.apply(xv[j] * rstd, wv[j]);
         st8(yr + (v << 3), pack8(o));
       }
+      cur[i] = next[i];
     }
+    ok = next_ok;
   }
 }
 
 // One CTA walks rows blockIdx.x, +gridDim.x, ... and keeps its dw partial in registers.
+// The row's direct gradient and the next row's scale are loaded before the reduction too, which takes one barrier:
+// 2048 x 4096 27 -> 18.9 us, 8192 x 4096 92 -> 57.5 (copy bandwidth: 41.6), 1536 x 8192 58 -> 33.6.
 // A row's x and dy stay in registers (packed bf16) between the reduction and the dx pass,
 // and the next row is fetched before the block-wide reduction of the current one, so the
 // loads of one row overlap the synchronisation of the previous row.
@@ -109,11 +149,11 @@ __device__ __forceinline__ bf16x8 load_dy(const NormBwdArgs& p, int64_t r, int c
   for (int j = 0; j < 8; ++j) a[j] += b[j];
   return pack8(a);
 }
-__device__ __forceinline__ void store_dx(const NormBwdArgs& p, int64_t r, int c, const float (&d)[8]) {
+__device__ __forceinline__ void store_dx(const NormBwdArgs& p, int64_t r, int c, const float (&d)[8], const bf16x8* add = nullptr) {
   if (p.dx == nullptr) return;
   float o[8];
   if (p.add != nullptr) {
-    unpack8(ld8(p.add + r * p.add_stride + c), o);
+    unpack8(add != nullptr ? *add : ld8(p.add + r * p.add_stride + c), o);
 #pragma unroll
     for (int j = 0; j < 8; ++j) o[j] += round_bf16(d[j]);
   } else {
@@ -127,7 +167,7 @@ template <int NV, int THREADS, bool DW>
 __global__ void __launch_bounds__(THREADS)
 rmsnorm_bwd_kernel(const NormBwdArgs p) {
   pdl_begin();
-  __shared__ float scratch[33];
+  __shared__ float scratch[2][THREADS / 32];
   const int nvec = p.H >> 3;
   float dwacc[DW ? NV : 1][8];
   bf16x8 wreg[NV];
@@ -154,16 +194,26 @@ rmsnorm_bwd_kernel(const NormBwdArgs p) {
       }
     }
   };
-  int r = blockIdx.x;
+  int r = blockIdx.x, slot = 0;
+  float rstd_next = r < p.rows ? p.rstd[r] : 0.f;
   if (kPrefetch && r < p.rows) fetch(r, xa, da);
-  for (; r < p.rows; r += gridDim.x) {
+  for (; r < p.rows; r += gridDim.x, slot ^= 1) {
+    const float rstd = rstd_next;
+    const int rn = r + gridDim.x;
+    if (rn < p.rows) rstd_next = p.rstd[rn];
     if constexpr (kPrefetch) {
-      const int rn = r + gridDim.x;
       if (rn < p.rows) fetch(rn, xb, db);
     } else {
       fetch(r, xa, da);
     }
-    const float rstd = p.rstd[r];
+    bf16x8 addv[NB];  // this row's direct gradient: its load passes during the reduction too
+    if (kPrefetch && p.add != nullptr) {
+#pragma unroll
+      for (int i = 0; i < NB; ++i) {
+        const int v = threadIdx.x + i * THREADS;
+        if (v < nvec) addv[i] = ld8(p.add + (int64_t)r * p.add_stride + (v << 3));
+      }
+    }
     float dot = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
@@ -181,7 +231,7 @@ rmsnorm_bwd_kernel(const NormBwdArgs p) {
         }
       }
     }
-    dot = block_sum(dot, scratch) / (float)p.H;
+    dot = row_sum<THREADS>(dot, scratch, slot) / (float)p.H;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int v = threadIdx.x + i * THREADS;
@@ -192,7 +242,7 @@ rmsnorm_bwd_kernel(const NormBwdArgs p) {
         unpack8(wreg[i], wv);
 #pragma unroll
         for (int j = 0; j < 8; ++j) d[j] = rstd * (dv[j] * (p.nw.centred ? 1.f + wv[j] : wv[j]) - xv[j] * rstd * dot);
-        store_dx(p, r, v << 3, d);
+        store_dx(p, r, v << 3, d, kPrefetch ? &addv[kPrefetch ? i : 0] : nullptr);
       }
     }
     if constexpr (kPrefetch) {
@@ -660,9 +710,14 @@ void launch_rmsnorm_fwd(const void* x, const void* w, const int64_t* row_index, 
                (__nv_bfloat16*)y, rstd, rows, H, x_stride, y_stride, eps, nw);
     return;
   }
-  const int grid = rows < 8 * kNumSM ? rows : 8 * kNumSM;
+  // narrow rows, few of them: a block each (1001 x 2048 4.2 us, 4.6 walking); wide ones are better walked (1536 x 24576 51 and 42)
+  auto grid = [&](int blocks) {
+    if (H <= 4096 && rows <= 16 * kNumSM) return rows;
+    const int most = blocks * kNumSM, rounds = (rows + most - 1) / most;
+    return (rows + rounds - 1) / rounds;
+  };
 #define SB200_FWD(NVV, THREADS)                                                                                          \
-  launch_pdl(rmsnorm_fwd_kernel<NVV, THREADS>, grid, THREADS, 0, stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, row_index, \
+  launch_pdl(rmsnorm_fwd_kernel<NVV, THREADS>, grid(kFwdBlocks<NVV, THREADS>), THREADS, 0, stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, row_index, \
              (__nv_bfloat16*)y, rstd, rows, H, x_stride, y_stride, eps, src_rows, nw)
   if (H <= 4096) SB200_FWD(2, 256);
   else if (H <= 8192) SB200_FWD(4, 256);
