@@ -290,18 +290,14 @@ _GATHER_ELEMENTS = 37 * 65536
 class _SideWork:
     """Weight gradients of one backward pass: gathered over the uses of a weight, run on a stream of their own."""
 
-    def __init__(self, main: torch.cuda.Stream):
-        self.main, self.stream = main, torch.cuda.Stream(main.device)
-        self.task = -1
+    def __init__(self, main: torch.cuda.Stream, key: tuple[int, int, int]):
+        self.main, self.key = main, key
+        self.stream = _SIDE_STREAMS.get(key[:2])
+        if self.stream is None:
+            self.stream = _SIDE_STREAMS[key[:2]] = torch.cuda.Stream(main.device)
         self.held = []  # operands of what the side stream has queued
         self.weights = []
         self.pending: dict[tuple, tuple] = {}  # (weight's id, rows) -> (weight, uses gathered, launch)
-
-    def begin(self, task: int) -> None:
-        if self.task != task:
-            self.pending.clear()  # of a pass that ended in an exception
-            torch.autograd.Variable._execution_engine.queue_callback(self.finish)
-            self.task = task
 
     def run(self, key: tuple) -> None:
         weight, uses, launch = self.pending.pop(key)
@@ -319,12 +315,13 @@ class _SideWork:
         self.main.wait_stream(self.stream)
         for w in self.weights:
             w._side_work = None
-        self.held.clear()  # memory goes back to the main stream's order, which now follows the side stream's
-        self.weights.clear()
-        self.task = -1
+        # the operands' memory goes back to the main stream's order, which now follows the side stream's
+        _SIDE_WORK.pop(self.key, None)
 
 
-_SIDE_WORK: dict[tuple[int, int], _SideWork] = {}  # by device and main stream (torch hands out streams from a fixed pool)
+_SIDE_STREAMS: dict[tuple[int, int], torch.cuda.Stream] = {}  # by device and main stream (torch hands out streams from a fixed pool)
+_SIDE_WORK: dict[tuple[int, int, int], _SideWork] = {}  # by device, main stream and backward pass (threads may run several at once)
+_SIDE_WORK_KEPT = 32  # passes; what an exception ended never finishes and goes when that many others have begun
 
 
 def _wait_for_side_work(weight: torch.Tensor) -> None:
@@ -343,18 +340,22 @@ def _note_use(weight: torch.Tensor, *rows) -> None:
 def _gather_use(weight: torch.Tensor, rows: tuple, use: tuple, launch) -> None:
     """One use's operands of a gradient that goes into the flat buffer.  ``launch(uses)`` forms the gradient of all uses as one
     product once the last expected one (or ``_MAX_USES``) has come: training-time-test passes read and wrote every gradient
-    once a pass (uses of a small weight, whose product is bound by neither, are not waited for: ``_GATHER_ELEMENTS``).  It runs beside the rest of the backward pass, where nothing needs its result: on its own stream it fills
-    the SMs that the chain of input gradients leaves idle - the last wave of a product, the short element-wise kernels.  The
+    once a pass.  It runs beside the rest of the backward pass, where nothing needs its result: on its own stream it fills
+    the SMs that the chain of input gradients leaves idle - the last wave of a product, the short element-wise kernels.
+    Waiting for further uses does not pay for small weights (``_GATHER_ELEMENTS``), whose products are bound by neither.  The
     pass's end runs what is left and joins the streams, and so does any other gradient of the same weight."""
     task = torch._C._current_graph_task_id()
     if task < 0:
         launch([use])
         return
     main = torch.cuda.current_stream(weight.device)
-    work = _SIDE_WORK.get((main.device_index, main.cuda_stream))
+    at = (main.device_index, main.cuda_stream, task)
+    work = _SIDE_WORK.get(at)
     if work is None:
-        work = _SIDE_WORK[(main.device_index, main.cuda_stream)] = _SideWork(main)
-    work.begin(task)
+        for old in [k for k in list(_SIDE_WORK) if k[2] < task - _SIDE_WORK_KEPT]:
+            _SIDE_WORK.pop(old, None)
+        work = _SIDE_WORK[at] = _SideWork(main, at)
+        torch.autograd.Variable._execution_engine.queue_callback(work.finish)
     key = (id(weight), *rows)
     _, uses, _ = work.pending.setdefault(key, (weight, [], launch))
     uses.append(use)

@@ -109,7 +109,7 @@ def test_row_slices_of_a_flat_gradient_are_stored_then_added():
     assert (w._flat_grad[256:] == 0).all() and (w._flat_grad.float() - want).abs().max() <= 0.02 * want.abs().max()
 
 
-@pytest.mark.parametrize("rows,K,N", [(64, 128, 128), (1001, 512, 768)])
+@pytest.mark.parametrize("rows,K,N", [(64, 128, 128), (1001, 512, 768), (300, 1536, 2048)])
 def test_weight_gradients_beside_the_backward_pass(rows, K, N):
     """Several uses of a weight, a gradient that reaches it another way, and a pass that ends in an exception."""
     torch.manual_seed(rows)
