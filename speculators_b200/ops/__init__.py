@@ -309,10 +309,17 @@ class _SideWork:
         weight._side_work = self
 
     def finish(self) -> None:
+        # The engine runs this on the stream that ``backward()`` was called on, once that stream waits for those of the leaves.
+        # It is not ``main`` where forward ran on another one, and whoever reads the gradients reads them there.
+        current = torch.cuda.current_stream(self.main.device)
+        if self.pending and current != self.main:
+            self.stream.wait_stream(current)  # gradients of the same weights that came through autograd's own accumulation
         for key in list(self.pending):
             self.pending[key][0]._grad_uses.pop(key[1:], None)  # uses that no gradient came back from
             self.run(key)
         self.main.wait_stream(self.stream)
+        if current != self.main:
+            current.wait_stream(self.main)
         for w in self.weights:
             w._side_work = None
         # the operands' memory goes back to the main stream's order, which now follows the side stream's
