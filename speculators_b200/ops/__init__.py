@@ -392,7 +392,7 @@ def _linear_backward(x2, weight, rows, dy, need_dx: bool, need_dw: bool):
         if flat is not None and own and _gemm_operand_ok(flat if r0 is None else flat[r0:r1]) and x2.shape[0] > 0:
             def launch(uses):
                 # the first gradient of these rows since the engine's zero_grad, which left the buffer uncleared, is stored
-                target, accumulate = _param_grad_target(weight, beside=True)[:2] if r0 is None else _row_grad_target(weight, r0, r1)
+                target, accumulate = _param_grad_target(weight, beside=True)[:2] if r0 is None else _row_grad_target(weight, r0, r1, beside=True)
                 native().gemm_wgrad_parts([u[0] for u in uses], [u[1] for u in uses], target, accumulate, gemm_status(target.device))
 
             _gather_use(weight, (r0, r1), (dy2, x2), launch)
@@ -492,9 +492,12 @@ def clear_fresh_grad(p: torch.Tensor) -> None:
         p._flat_grad[r0:r1].zero_()
 
 
-def _row_grad_target(weight: torch.Tensor, r0: int, r1: int) -> tuple[torch.Tensor, bool]:
+def _row_grad_target(weight: torch.Tensor, r0: int, r1: int, beside: bool = False) -> tuple[torch.Tensor, bool]:
     """``(rows of the flat gradient view, accumulate)`` for a gradient of rows ``r0 .. r1`` alone: stored where nothing has been
-    stored since ``zero_grad``; the intervals still unwritten stay noted on the weight."""
+    stored since ``zero_grad``; the intervals still unwritten stay noted on the weight.  ``beside`` as in ``_param_grad_target``:
+    anyone else waits for what earlier uses of the rows have launched."""
+    if not beside:
+        _wait_for_side_work(weight)
     fresh = getattr(weight, "_grad_fresh", False)
     if fresh is True:
         fresh = [(0, weight.shape[0])]

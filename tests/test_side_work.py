@@ -86,3 +86,20 @@ def test_the_stream_that_called_backward_waits_for_the_gradients(streams, width)
     assert behind == [width == 64]
     assert "dw" in main.behind and "dw" in caller.behind
     assert width == 64 or "accumulated" in ops._SIDE_STREAMS[0, main.cuda_stream].behind
+
+
+@pytest.mark.parametrize("rows", [(None, None), (0, 32)])
+def test_a_gradient_on_the_main_stream_comes_behind_those_beside_it(streams, rows):
+    """A use whose operands the kernel does not take (the library product) after one that it does."""
+    _, main = streams
+    w, x = _weight(), torch.ones(4, 64, requires_grad=True)
+    w._flat_grad = torch.zeros(64, 64)
+    before = []
+
+    def library(d):
+        r0, r1 = rows
+        ops._linear_backward(x.detach(), w, rows, d if r0 is None else d[:, r0:r1], False, True)
+        before.append("dw" in main.behind)
+
+    _use(x, w, main, "dw", library).sum().backward()
+    assert before == [True]
