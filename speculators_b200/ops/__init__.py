@@ -15,7 +15,10 @@ kernels via ``torch.autograd.Function``.
 
 from __future__ import annotations
 
+import collections
+import contextlib
 import math
+import weakref
 
 import torch
 import torch.nn.functional as F
@@ -264,22 +267,22 @@ class _LinearFn(torch.autograd.Function):
     """
 
     @staticmethod
-    def forward(ctx, x, weight, residual, r0, r1):
+    def forward(ctx, x, weight, residual, r0, r1, use):
         # x is [rows, in]; the result is a fresh tensor (never a view), so callers may
         # rotate / normalise it in place
         w = weight if r0 is None else weight[r0:r1]
         y = _forward_gemm(x, w, residual)
         ctx.save_for_backward(x, weight)
-        ctx.rows = (r0, r1)
+        ctx.rows, ctx.use = (r0, r1), use
         ctx.has_residual = residual is not None
         return y
 
     @staticmethod
     def backward(ctx, dy):
         x2, weight = ctx.saved_tensors
-        dx, dw = _linear_backward(x2, weight, ctx.rows, dy, ctx.needs_input_grad[0], ctx.needs_input_grad[1])
+        dx, dw = _linear_backward(x2, weight, ctx.rows, ctx.use, dy, ctx.needs_input_grad[0], ctx.needs_input_grad[1])
         dres = dy if ctx.has_residual and ctx.needs_input_grad[2] else None
-        return dx, dw, dres, None, None
+        return dx, dw, dres, None, None, None
 
 
 _MAX_USES = 4  # of a weight in one product (the kernel's operand maps)
@@ -288,25 +291,32 @@ _GATHER_ELEMENTS = 37 * 65536
 
 
 class _SideWork:
-    """Weight gradients of one backward pass: gathered over the uses of a weight, run on a stream of their own."""
+    """Weight gradients of one backward pass: gathered over the uses of a weight, run on a stream of their own.
 
-    def __init__(self, main: torch.cuda.Stream, key: tuple[int, int, int]):
-        self.main, self.key = main, key
-        self.stream = _SIDE_STREAMS.get(key[:2])
+    The pass's own end-of-pass callback holds the only reference that lasts, so a pass that an exception ends gives its
+    operands back when the engine drops it."""
+
+    def __init__(self, main: torch.cuda.Stream, at: tuple[int, int]):
+        self.main = main
+        self.stream = _SIDE_STREAMS.get(at)
         if self.stream is None:
-            self.stream = _SIDE_STREAMS[key[:2]] = torch.cuda.Stream(main.device)
-        self.held = []  # operands of what the side stream has queued
-        self.weights = []
+            self.stream = _SIDE_STREAMS[at] = torch.cuda.Stream(main.device)
+        self.held: collections.deque = collections.deque()  # (event behind a launch, its operands, itself with what it reads), the oldest first
+        self.weights: list[torch.Tensor] = []
         self.pending: dict[tuple, tuple] = {}  # (weight's id, rows) -> (weight, uses gathered, launch)
 
     def run(self, key: tuple) -> None:
         weight, uses, launch = self.pending.pop(key)
         self.stream.wait_stream(self.main)
         with torch.cuda.stream(self.stream):
+            _wait_for_side_work(weight)  # of another stream's pass
             launch(uses)
-        self.held.append(uses)
         self.weights.append(weight)
-        weight._side_work = self
+        weight._side_stream = self.stream
+        self.held.append((self.stream.record_event(), uses, launch))
+        while len(self.held) > _SIDE_HELD:
+            self.main.wait_event(self.held[0][0])  # the memory goes back to the main stream's order
+            self.held.popleft()
 
     def finish(self) -> None:
         # The engine runs this on the stream that ``backward()`` was called on, once that stream waits for those of the leaves.
@@ -315,71 +325,102 @@ class _SideWork:
         if self.pending and current != self.main:
             self.stream.wait_stream(current)  # gradients of the same weights that came through autograd's own accumulation
         for key in list(self.pending):
-            self.pending[key][0]._grad_uses.pop(key[1:], None)  # uses that no gradient came back from
             self.run(key)
         self.main.wait_stream(self.stream)
         if current != self.main:
             current.wait_stream(self.main)
         for w in self.weights:
-            w._side_work = None
-        # the operands' memory goes back to the main stream's order, which now follows the side stream's
-        _SIDE_WORK.pop(self.key, None)
+            if w._side_stream is self.stream:
+                w._side_stream = None
+        self.held.clear()
+
+    def __del__(self):
+        if self.held:  # the pass did not come to its end
+            with contextlib.suppress(RuntimeError):  # a capture that the exception ended, too
+                self.main.wait_stream(self.stream)
 
 
 _SIDE_STREAMS: dict[tuple[int, int], torch.cuda.Stream] = {}  # by device and main stream (torch hands out streams from a fixed pool)
-_SIDE_WORK: dict[tuple[int, int, int], _SideWork] = {}  # by device, main stream and backward pass (threads may run several at once)
-_SIDE_WORK_KEPT = 32  # passes; what an exception ended never finishes and goes when that many others have begun
+# by device, main stream and backward pass (threads may run several at once)
+_SIDE_WORK: weakref.WeakValueDictionary[tuple[int, int, int], _SideWork] = weakref.WeakValueDictionary()
+# Bounds on what a pass keeps allocated for its weight gradients, however deep the model: operands of launches that the main
+# stream has not waited for yet, and weights with uses gathered but not launched.  Four launches are a layer's; steps of one to
+# five layers take the same time with any bound (five layers of 8192 rows 58.7 ms, 59.9 without one) but for the smallest,
+# whose chain feels a wait for every launch (0.441 ms, 0.445 at a bound of one).
+_SIDE_HELD = 4
+_SIDE_PENDING = 16
 
 
 def _wait_for_side_work(weight: torch.Tensor) -> None:
-    work = getattr(weight, "_side_work", None)
-    if work is not None:
-        torch.cuda.current_stream(weight.device).wait_stream(work.stream)
+    stream = getattr(weight, "_side_stream", None)
+    if stream is not None:
+        current = torch.cuda.current_stream(weight.device)
+        if current != stream:
+            current.wait_stream(stream)
 
 
-def _note_use(weight: torch.Tensor, *rows) -> None:
-    """Called where a differentiated product uses ``weight`` (or rows of it): how many gradients to expect."""
-    if getattr(weight, "_flat_grad", None) is not None:
-        uses = weight.__dict__.setdefault("_grad_uses", {})
-        uses[rows] = uses.get(rows, 0) + 1
+class _Use:
+    """A differentiated product's use of a weight (or of rows of it) whose gradient is still to come: held by the product's
+    node, so that it goes with the graph if no gradient comes."""
+
+    def __init__(self, weight: torch.Tensor, rows: tuple):
+        self.counts, self.rows = weight.__dict__.setdefault("_grad_uses", {}), rows
+        self.counts[rows] = self.counts.get(rows, 0) + 1
+
+    def left(self) -> int:
+        """Count this use as come; how many others of the same rows are still to come."""
+        counts, self.counts = self.counts, None
+        if counts is None:  # the node's second pass
+            return 0
+        n = counts[self.rows] - 1
+        if n:
+            counts[self.rows] = n
+        else:
+            del counts[self.rows]
+        return n
+
+    def __del__(self):
+        self.left()
 
 
-def _gather_use(weight: torch.Tensor, rows: tuple, use: tuple, launch) -> None:
+def _note_use(weight: torch.Tensor, *rows) -> _Use | None:
+    """Called where a differentiated product uses ``weight`` (or rows of it): for the product's node to keep."""
+    return _Use(weight, rows) if getattr(weight, "_flat_grad", None) is not None else None
+
+
+def _gather_use(weight: torch.Tensor, rows: tuple, use: _Use | None, operands: tuple, launch) -> None:
     """One use's operands of a gradient that goes into the flat buffer.  ``launch(uses)`` forms the gradient of all uses as one
     product once the last expected one (or ``_MAX_USES``) has come: training-time-test passes read and wrote every gradient
     once a pass.  It runs beside the rest of the backward pass, where nothing needs its result: on its own stream it fills
     the SMs that the chain of input gradients leaves idle - the last wave of a product, the short element-wise kernels.
     Waiting for further uses does not pay for small weights (``_GATHER_ELEMENTS``), whose products are bound by neither.  The
     pass's end runs what is left and joins the streams, and so does any other gradient of the same weight."""
+    left = use.left() if use is not None else 0
     task = torch._C._current_graph_task_id()
     if task < 0:
-        launch([use])
+        launch([operands])
         return
     main = torch.cuda.current_stream(weight.device)
     at = (main.device_index, main.cuda_stream, task)
     work = _SIDE_WORK.get(at)
     if work is None:
-        for old in [k for k in list(_SIDE_WORK) if k[2] < task - _SIDE_WORK_KEPT]:
-            _SIDE_WORK.pop(old, None)
-        work = _SIDE_WORK[at] = _SideWork(main, at)
+        work = _SIDE_WORK[at] = _SideWork(main, at[:2])
         torch.autograd.Variable._execution_engine.queue_callback(work.finish)
     key = (id(weight), *rows)
     _, uses, _ = work.pending.setdefault(key, (weight, [], launch))
-    uses.append(use)
-    expected = weight.__dict__.setdefault("_grad_uses", {})
-    expected[rows] = expected.get(rows, 0) - 1
+    uses.append(operands)
     # contractions of 8192 rows are long enough on their own (28672 x 4096, three uses: 4380 us apart, 4430 together;
     # of 2048 rows 1150 and 1075); rows grouped by expert are few for each
-    whole = weight.numel() < _GATHER_ELEMENTS or (weight.dim() == 2 and use[0].shape[0] > 6144)
-    if expected[rows] <= 0 or len(uses) == _MAX_USES or whole:
-        if expected[rows] <= 0:
-            del expected[rows]
+    whole = weight.numel() < _GATHER_ELEMENTS or (weight.dim() == 2 and operands[0].shape[0] > 6144)
+    if left == 0 or len(uses) == _MAX_USES or whole:
         work.run(key)
+    elif len(work.pending) > _SIDE_PENDING:
+        work.run(next(iter(work.pending)))
 
 
-def _linear_backward(x2, weight, rows, dy, need_dx: bool, need_dw: bool):
+def _linear_backward(x2, weight, rows, use, dy, need_dx: bool, need_dw: bool):
     """``(dx, dw)`` of ``y = x2 @ weight[rows].T``; ``dw`` is ``None`` when the gradient went
-    straight into the flat buffer the training engine attached to the weight."""
+    straight into the flat buffer the training engine attached to the weight.  ``use``: what ``_note_use`` gave the product."""
     r0, r1 = rows
     w = weight if r0 is None else weight[r0:r1]
     dy2 = dy if (dy.stride(-1) == 1 and dy.stride(0) % 8 == 0 and dy.data_ptr() % 16 == 0) else dy.contiguous()
@@ -395,8 +436,10 @@ def _linear_backward(x2, weight, rows, dy, need_dx: bool, need_dw: bool):
                 target, accumulate = _param_grad_target(weight, beside=True)[:2] if r0 is None else _row_grad_target(weight, r0, r1, beside=True)
                 native().gemm_wgrad_parts([u[0] for u in uses], [u[1] for u in uses], target, accumulate, gemm_status(target.device))
 
-            _gather_use(weight, (r0, r1), (dy2, x2), launch)
+            _gather_use(weight, (r0, r1), use, (dy2, x2), launch)
         elif flat is not None:
+            if use is not None:
+                use.left()
             target, accumulate = _param_grad_target(weight)[:2] if r0 is None else _row_grad_target(weight, r0, r1)
             if accumulate:
                 target.addmm_(dy2.t(), x2)
@@ -426,9 +469,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
         lead = x.shape[:-1]
         x2 = x.reshape(-1, x.shape[-1])
         res2 = residual.reshape(-1, residual.shape[-1]) if residual is not None else None
-        if weight.requires_grad:
-            _note_use(weight, r0, r1)
-        y = _LinearFn.apply(x2, weight, res2, r0, r1)
+        y = _LinearFn.apply(x2, weight, res2, r0, r1, _note_use(weight, r0, r1) if weight.requires_grad else None)
         if len(lead) != 1:
             y = y.view(*lead, y.shape[-1])
         if bias is not None:
@@ -664,17 +705,18 @@ class _GateUpSwiGLUFn(torch.autograd.Function):
     gate | up product (saved for the backward pass) and the activated product."""
 
     @staticmethod
-    def forward(ctx, x2, weight):
+    def forward(ctx, x2, weight, use):
         gate_up, h = native().gemm_swiglu(x2, weight, gemm_status(x2.device))
         ctx.save_for_backward(x2, weight, gate_up)
+        ctx.use = use
         return h
 
     @staticmethod
     def backward(ctx, dh):
         x2, weight, gate_up = ctx.saved_tensors
         dgu = native().swiglu_bwd(dh.contiguous(), gate_up)
-        dx, dw = _linear_backward(x2, weight, (None, None), dgu, ctx.needs_input_grad[0], ctx.needs_input_grad[1])
-        return dx, dw
+        dx, dw = _linear_backward(x2, weight, (None, None), ctx.use, dgu, ctx.needs_input_grad[0], ctx.needs_input_grad[1])
+        return dx, dw, None
 
 
 def linear_swiglu(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor | None:
@@ -688,9 +730,8 @@ def linear_swiglu(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor | None:
     if (not own_gemm_enabled() or os.environ.get("SB200_FUSED_SWIGLU", "1") == "0" or not _gemm_operand_ok(x2) or not _gemm_operand_ok(weight)
             or weight.shape[0] % 256 or weight.shape[1] != x2.shape[1]):
         return None
-    if weight.requires_grad and torch.is_grad_enabled():
-        _note_use(weight, None, None)
-    h = _GateUpSwiGLUFn.apply(x2, weight)
+    use = _note_use(weight, None, None) if weight.requires_grad and torch.is_grad_enabled() else None
+    h = _GateUpSwiGLUFn.apply(x2, weight, use)
     return h.view(*x.shape[:-1], h.shape[-1])
 
 
@@ -1031,10 +1072,10 @@ class _LmHeadLossFn(torch.autograd.Function):
     the row-loss backward kernel followed by the input-gradient GEMM."""
 
     @staticmethod
-    def forward(ctx, hidden, weight, targets, op, shift, rows, active):
+    def forward(ctx, hidden, weight, targets, op, shift, rows, active, use):
         logits, loss, stats, am_d, am_t = native().lmhead_loss_fwd(op, hidden, weight, targets, active, shift, rows, gemm_status(hidden.device))
         ctx.save_for_backward(hidden, weight, targets, logits, stats)
-        ctx.cfg = (op, shift, rows)
+        ctx.cfg, ctx.use = (op, shift, rows), use
         ctx.mark_non_differentiable(am_d, am_t)
         return loss, am_d, am_t
 
@@ -1043,8 +1084,8 @@ class _LmHeadLossFn(torch.autograd.Function):
         hidden, weight, targets, logits, stats = ctx.saved_tensors
         op, shift, rows = ctx.cfg
         d = native().loss_bwd(op, logits, targets, dloss.contiguous().float(), stats, shift, rows)
-        dx, dw = _linear_backward(hidden, weight, (None, None), d, ctx.needs_input_grad[0], ctx.needs_input_grad[1])
-        return dx, dw, None, None, None, None, None
+        dx, dw = _linear_backward(hidden, weight, (None, None), ctx.use, d, ctx.needs_input_grad[0], ctx.needs_input_grad[1])
+        return dx, dw, None, None, None, None, None, None
 
 
 FUSED_HEAD_OPS = ("kl_div", "ce")
@@ -1069,9 +1110,8 @@ def lm_head_loss_raw(op: str, hidden: torch.Tensor, weight: torch.Tensor, target
     plain store epilogue), so the two-kernel form is the default."""
     if not lm_head_loss_ok(op, hidden, weight, targets):
         return None
-    if weight.requires_grad and torch.is_grad_enabled():
-        _note_use(weight, None, None)
-    return _LmHeadLossFn.apply(hidden, weight, targets, LOSS_OPS[op], shift, rows, active)
+    use = _note_use(weight, None, None) if weight.requires_grad and torch.is_grad_enabled() else None
+    return _LmHeadLossFn.apply(hidden, weight, targets, LOSS_OPS[op], shift, rows, active, use)
 
 
 class _StepTailFn(torch.autograd.Function):

@@ -29,7 +29,7 @@ def moe_experts_ok(x: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor) -
 
 class _MoEExpertsFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, top_p, top_e, w_gu, w_d, shared, gate, residual):
+    def forward(ctx, x, top_p, top_e, w_gu, w_d, shared, gate, residual, uses):
         nat, status = ops.native(), ops.gemm_status(x.device)
         k, E = top_e.shape[1], w_gu.shape[0]
         capacity = (top_e.numel() + 127 * E + 127) // 128 * 128  # worst case: every expert's tail padded by 127 rows
@@ -40,7 +40,7 @@ class _MoEExpertsFn(torch.autograd.Function):
         nat.gemm_grouped_rows(h, w_d, y_pad, False, seg, tiles, status)
         out = nat.moe_combine(y_pad, slot_row, top_p, shared, gate, residual)
         ctx.save_for_backward(x_pad, gate_up, h, y_pad, top_p, w_gu, w_d, shared, gate, seg, tiles, slot_row, row_slot)
-        ctx.with_residual = residual is not None
+        ctx.with_residual, ctx.uses = residual is not None, uses
         return out
 
     @staticmethod
@@ -51,7 +51,7 @@ class _MoEExpertsFn(torch.autograd.Function):
         dout = dout.contiguous()
         dy_pad, dp, dshared, dgate = nat.moe_combine_bwd(dout, y_pad, row_slot, seg, top_p, shared, gate)
 
-        def weight_gradient(needed, dy, rows, w):
+        def weight_gradient(needed, dy, rows, w, use):
             if not needed:
                 return None
             flat = getattr(w, "_flat_grad", None)
@@ -65,22 +65,22 @@ class _MoEExpertsFn(torch.autograd.Function):
                 dys, xs, segs = (list(part) for part in zip(*uses))
                 nat.gemm_grouped_wgrad_parts(dys, xs, target, accumulate, segs, tiles, status)
 
-            ops._gather_use(w, ("experts",), (dy, rows, seg), launch)  # noqa: SLF001
+            ops._gather_use(w, ("experts",), use, (dy, rows, seg), launch)  # noqa: SLF001
             return None
 
-        dw_d = weight_gradient(need[4], dy_pad, h, w_d)
+        dw_d = weight_gradient(need[4], dy_pad, h, w_d, ctx.uses[1])
         dx = dw_gu = None
         if need[0] or need[3]:
             dh = torch.empty_like(h)
             nat.gemm_grouped_rows(dy_pad, w_d, dh, True, seg, tiles, status)
             dgu = nat.swiglu_bwd_rows(dh, gate_up, seg[-1:])
-            dw_gu = weight_gradient(need[3], dgu, x_pad, w_gu)
+            dw_gu = weight_gradient(need[3], dgu, x_pad, w_gu, ctx.uses[0])
             if need[0]:
                 dx_pad = torch.empty_like(x_pad)
                 nat.gemm_grouped_rows(dgu, w_gu, dx_pad, True, seg, tiles, status)
                 dx = nat.moe_gather_bwd(dx_pad, slot_row, top_p.shape[1])
         with_shared = shared is not None
-        return dx, dp, None, dw_gu, dw_d, dshared if with_shared else None, dgate if with_shared else None, dout if ctx.with_residual else None
+        return dx, dp, None, dw_gu, dw_d, dshared if with_shared else None, dgate if with_shared else None, dout if ctx.with_residual else None, None
 
 
 def moe_experts(x, top_p, top_e, gate_up, down, shared=None, shared_gate=None, residual=None) -> torch.Tensor:
@@ -90,8 +90,6 @@ def moe_experts(x, top_p, top_e, gate_up, down, shared=None, shared_gate=None, r
     def rows(t):
         return None if t is None else t.contiguous()
 
-    if torch.is_grad_enabled():
-        for w in (gate_up, down):
-            if w.requires_grad:
-                ops._note_use(w, "experts")  # noqa: SLF001
-    return _MoEExpertsFn.apply(rows(x), rows(top_p), rows(top_e), gate_up, down, rows(shared), rows(shared_gate), rows(residual))
+    grad = torch.is_grad_enabled()
+    uses = tuple(ops._note_use(w, "experts") if grad and w.requires_grad else None for w in (gate_up, down))  # noqa: SLF001
+    return _MoEExpertsFn.apply(rows(x), rows(top_p), rows(top_e), gate_up, down, rows(shared), rows(shared_gate), rows(residual), uses)

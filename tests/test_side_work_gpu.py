@@ -44,3 +44,57 @@ def test_forward_on_one_stream_and_backward_from_another(late, rows, cols):
     (2 * (x.float() @ wf.t()).pow(2).mean()).backward()
     # dy is rounded to bf16 and so is the sum: two roundings of 2^-9 of the largest terms, and cancellation in between
     assert (got - wf.grad).abs().max() <= 0.02 * wf.grad.abs().max()
+
+
+@pytest.mark.parametrize("width,rows", [(1024, 2048), (2048, 512)])  # launched at once, gathered where another use is expected
+def test_memory_of_a_pass_does_not_grow_with_its_layers(width, rows):
+    """Behind the bounds every further layer adds what its forward pass keeps, and no operands of weight gradients."""
+    torch.manual_seed(0)
+    x = torch.randn(rows, width, device="cuda").bfloat16()
+
+    def extra(layers):
+        weights = [_weight(width, width) for _ in range(layers)]
+        ops.linear(x, weights[0]).sum().backward()  # allocations of the first call
+        y = x
+        for w in weights:
+            y = ops.linear(y, w)
+        loss = y.sum()
+        del y
+        torch.cuda.synchronize()
+        start = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        loss.backward()
+        torch.cuda.synchronize()
+        return (torch.cuda.max_memory_allocated() - start) / (rows * width * 2)
+
+    bound = ops._SIDE_HELD + ops._SIDE_PENDING
+    # in units of one activation: the pass frees a layer's input for each gradient that it forms
+    assert extra(3 * bound) <= extra(bound) + 1
+
+
+def test_memory_after_a_pass_that_an_exception_ended():
+    torch.manual_seed(0)
+    w = _weight(512, 512)
+
+    def stop(g):
+        raise RuntimeError("stop")
+
+    def failing():
+        x = torch.randn(4096, 512, device="cuda").bfloat16().requires_grad_()
+        y = ops.linear(x, w)
+        y.register_hook(stop)
+        with pytest.raises(RuntimeError, match="stop"):
+            ops.linear(y, w).sum().backward()
+
+    failing()
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    for _ in range(3):
+        failing()
+    torch.cuda.synchronize()
+    assert torch.cuda.memory_allocated() == before
+    w._grad_fresh = True
+    x = torch.randn(64, 512, device="cuda").bfloat16()
+    ops.linear(x, w).sum().backward()
+    want = torch.ones(64, 512, device="cuda").t() @ x.float()
+    assert (w._flat_grad.float() - want).abs().max() <= 0.01 * want.abs().max()
