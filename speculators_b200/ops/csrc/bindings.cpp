@@ -32,7 +32,8 @@ void launch_document_interval(const int64_t*, int, int, int*, int*, cudaStream_t
 void launch_compact(const bool*, int, int64_t*, int*, cudaStream_t);
 void launch_cod_step(const int64_t*, const int64_t*, int, const bool*, int, int, int, unsigned char*, int64_t*, int64_t*, int64_t*, int64_t*, int*, cudaStream_t);
 void launch_peagle_spec(const int64_t*, const int64_t*, const bool*, const int64_t*, const int*, int, int, int, int, int*, int*, int*, int*, cudaStream_t);
-void launch_embedding_bwd(const int64_t*, const int64_t*, const void*, int64_t, int, int, int64_t, int64_t, void*, int, cudaStream_t);
+int embedding_bwd_partial_rows(int);
+void launch_embedding_bwd(const int64_t*, const int64_t*, const void*, int64_t, int, int, int64_t, int64_t, void*, int, float*, cudaStream_t);
 void launch_swiglu_fwd(const void*, void*, int64_t, int, const int*, cudaStream_t);
 void launch_swiglu_bwd(const void*, const void*, void*, int64_t, int, const int*, cudaStream_t);
 void launch_rope_merge(const void* const*, const int64_t*, const int*, const int*, void*, int64_t, const int64_t*, const float*, const float*, int64_t, int, int,
@@ -328,8 +329,9 @@ void embedding_bwd(const Tensor& ids, const Tensor& order, const Tensor& d, int6
   TORCH_CHECK(ids.numel() == d.size(0) && order.numel() == d.size(0) && dw.dim() == 2 && dw.is_contiguous() && dw.scalar_type() == at::kBFloat16 &&
               dw.size(1) == d.size(1) && d.size(1) % 8 == 0 && (reinterpret_cast<uintptr_t>(dw.data_ptr()) & 15) == 0);
   c10::cuda::CUDAGuard guard(d.device());
+  Tensor part = at::empty({sb200::embedding_bwd_partial_rows((int)d.size(0)), d.size(1)}, d.options().dtype(at::kFloat));
   sb200::launch_embedding_bwd(long_ptr(ids, "ids"), long_ptr(order, "order"), d.data_ptr(), d.stride(0), (int)d.size(0), (int)d.size(1), dw.size(0), padding,
-                              dw.data_ptr(), accumulate ? 1 : 0, cur_stream());
+                              dw.data_ptr(), accumulate ? 1 : 0, part.data_ptr<float>(), cur_stream());
 }
 
 // rows_used (optional int32[1] on the device): rows past it are left alone.

@@ -112,6 +112,7 @@ __device__ __forceinline__ bf16x8 pack8(const float (&f)[8]) {
   return p;
 }
 
+__device__ __forceinline__ float round_bf16(float v) { return __bfloat162float(__float2bfloat16(v)); }
 __device__ __forceinline__ bf16x8 ld8(const __nv_bfloat16* ptr) {
   return *reinterpret_cast<const bf16x8*>(ptr);
 }

@@ -36,7 +36,6 @@ struct NormWeight {
   // the plain module normalises in fp32, rounds to bf16, then scales
   __device__ __forceinline__ float apply(float xhat, float w) const { return centred ? xhat * w : __bfloat162float(__float2bfloat16(xhat)) * w; }
 };
-__device__ __forceinline__ float round_bf16(float v) { return __bfloat162float(__float2bfloat16(v)); }
 
 SB200_BOUNDS_RECORD
 

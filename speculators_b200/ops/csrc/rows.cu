@@ -154,29 +154,124 @@ peagle_spec_kernel(const int64_t* __restrict__ anchor, const int64_t* __restrict
     for (int e = 1; e < num_depths; ++e) extra[(int64_t)r * (num_depths - 1) + e - 1] = d >= e && !pad ? table[(int64_t)e * T + a] : -1;
 }
 
-// Gradient rows of an embedding from ids in ascending order (`order`: where each came from): one block sums the rows of
-// one id in fp32 and stores, or adds to, its row of dw.  Rows of other ids are not touched.
+// Gradient rows of an embedding from ids in ascending order (`order`: where each came from), summed in fp32 in a fixed order
+// and stored into, or added to, the id's row of dw.  Rows of other ids are not touched.
+//
+// The positions are cut into slices of 32, and a block sums what one id has in one slice: its loads do not depend on one
+// another, and however often an id comes (frequent tokens, the padding of a batch) no block walks more than 32 rows.  An id
+// that lies in one slice is done then; one that crosses into others leaves a partial row per slice (an id has at most two
+// kinds in a slice: it starts there, row 2 k + 1, or it comes from the slice before, row 2 k), and embedding_join_kernel
+// sums those.  As one block per id, the loop's exit hanging on a load, a step with real text waited for its most frequent id:
+// added to a 152k x 4096 table, 8194 rows with Zipf's frequencies (673 of one id) 841 -> 46 us, a quarter of them padding
+// 2545 -> 50, all one id 9926 -> 50; ids that hardly repeat 47 -> 52 (2050 rows: 18.5 -> 21.5), the second launch.
+constexpr int kSlice = 32;
+__device__ __forceinline__ bool embedding_id_ok(int64_t id, int64_t vocab, int64_t padding) { return id != padding && id >= 0 && id < vocab; }
+
 __global__ void __launch_bounds__(256)
 embedding_bwd_kernel(const int64_t* __restrict__ ids, const int64_t* __restrict__ order, const __nv_bfloat16* __restrict__ d, int64_t d_stride, int n, int H,
-                     int64_t vocab, int64_t padding, __nv_bfloat16* __restrict__ dw, int accumulate) {
+                     int64_t vocab, int64_t padding, __nv_bfloat16* __restrict__ dw, int accumulate, float* __restrict__ part) {
   pdl_begin();
-  const int i = blockIdx.x;
-  const int64_t id = ids[i];
-  if ((i > 0 && ids[i - 1] == id) || id == padding || id < 0 || id >= vocab) return;
+  __shared__ int64_t rows[kSlice];
+  const int i = blockIdx.x, slice = i / kSlice, stop = slice * kSlice + min(n - slice * kSlice, kSlice), lane = threadIdx.x & 31;
+  // one round of loads for all that the block has to know, whether it needs it or not
+  const int at = i + min(lane, stop - i - 1);
+  const int64_t id = ids[i], before = ids[max(i - 1, 0)], mine = ids[at], next = ids[min(stop, n - 1)], row = order[at];
+  const bool starts = i == 0 || before != id;
+  if ((!starts && i % kSlice != 0) || !embedding_id_ok(id, vocab, padding)) return;
+  const bool same = lane < stop - i && mine == id, more = stop < n && next == id;
+  const int len = __popc(__ballot_sync(0xffffffffu, same));  // ascending: the equal ones come first
+  if (threadIdx.x < len) rows[threadIdx.x] = row;
+  __syncthreads();
+  const bool whole = starts && !(more && i + len == stop);
   for (int c = threadIdx.x * 8; c < H; c += 256 * 8) {
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, v[8];
-    for (int j = i; j < n && ids[j] == id; ++j) {
-      unpack8(ld8(d + order[j] * d_stride + c), v);
+#pragma unroll 4
+    for (int j = 0; j < len; ++j) {
+      unpack8(ld8(d + rows[j] * d_stride + c), v);
 #pragma unroll
       for (int u = 0; u < 8; ++u) acc[u] += v[u];
+    }
+    if (!whole) {
+      float4* out = reinterpret_cast<float4*>(part + (2 * (int64_t)slice + starts) * H + c);
+      out[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+      out[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+      continue;
     }
     __nv_bfloat16* out = dw + id * (int64_t)H + c;
     if (accumulate) {
       unpack8(ld8(out), v);
 #pragma unroll
-      for (int u = 0; u < 8; ++u) acc[u] = __bfloat162float(__float2bfloat16(acc[u])) + v[u];
+      for (int u = 0; u < 8; ++u) acc[u] = round_bf16(acc[u]) + v[u];
     }
     st8(out, pack8(acc));
+  }
+}
+
+// One block: 128 columns of the ids that start in one of 8 slices and cross into the next.  A warp takes a slice and sums an id
+// that comes into few others by itself; for longer ones the eight warps share the partial rows and meet in shared memory (8194 rows in runs of 40: 46 us, 58 where the
+// block took one id after the other).
+constexpr int kJoinSlices = 8, kJoinAlone = 8;
+__device__ __forceinline__ void add4(float4& a, const float4& b) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; }
+__device__ __forceinline__ void embedding_store4(__nv_bfloat16* dw, int accumulate, float4 v) {
+  __nv_bfloat162* out = reinterpret_cast<__nv_bfloat162*>(dw);
+  if (accumulate) {
+    const float2 a = __bfloat1622float2(out[0]), b = __bfloat1622float2(out[1]);
+    v = make_float4(round_bf16(v.x) + a.x, round_bf16(v.y) + a.y, round_bf16(v.z) + b.x, round_bf16(v.w) + b.y);
+  }
+  out[0] = __floats2bfloat162_rn(v.x, v.y);
+  out[1] = __floats2bfloat162_rn(v.z, v.w);
+}
+__global__ void __launch_bounds__(32 * kJoinSlices)
+embedding_join_kernel(const int64_t* __restrict__ ids, const float* __restrict__ part, int n, int H, int64_t vocab, int64_t padding,
+                      __nv_bfloat16* __restrict__ dw, int accumulate) {
+  pdl_begin();
+  constexpr int kThreads = 32 * kJoinSlices;
+  __shared__ float4 tile[kJoinSlices][32];
+  __shared__ int shared_by_all[kJoinSlices];
+  const int slices = (n - 1) / kSlice + 1, k0 = blockIdx.x * kJoinSlices, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.y * 128 + lane * 4;
+  // the warp's slice: what starts in it and comes into `further` others, as far as 32 lanes see
+  const int mine = k0 + warp;
+  int further = 0;
+  if (mine + 1 < slices) {
+    const int begin = mine * kSlice;
+    const int64_t id = ids[begin + kSlice], last = ids[begin + kSlice - 1], before = ids[max(begin - 1, 0)];
+    const int m = mine + 1 + min(lane, slices - 2 - mine);
+    const bool same = lane < slices - 1 - mine && ids[m * kSlice] == id;
+    if (last == id && (begin == 0 || before != id) && embedding_id_ok(id, vocab, padding)) further = __popc(__ballot_sync(0xffffffffu, same));
+    if (further > 0 && further <= kJoinAlone && c < H) {
+      float4 acc = *reinterpret_cast<const float4*>(part + (2 * (int64_t)mine + 1) * H + c);
+#pragma unroll
+      for (int r = 1; r <= kJoinAlone; ++r)
+        if (r <= further) add4(acc, *reinterpret_cast<const float4*>(part + 2 * (int64_t)(mine + r) * H + c));
+      embedding_store4(dw + id * (int64_t)H + c, accumulate, acc);
+    }
+  }
+  if (lane == 0) shared_by_all[warp] = further > kJoinAlone;
+  __syncthreads();
+  for (int s = 0; s < kJoinSlices; ++s) {
+    if (!shared_by_all[s]) continue;
+    const int k = k0 + s;
+    const int64_t id = ids[(k + 1) * kSlice];
+    int got;
+    further = 0;
+    do {
+      const int m = k + 1 + further + threadIdx.x;
+      got = __syncthreads_count(m < slices && ids[min(m, slices - 1) * kSlice] == id);
+      further += got;
+    } while (got == kThreads);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (c < H) {
+#pragma unroll 4
+      for (int r = warp; r <= further; r += kJoinSlices) add4(acc, *reinterpret_cast<const float4*>(part + (2 * (int64_t)(k + r) + (r == 0)) * H + c));
+    }
+    tile[warp][lane] = acc;
+    __syncthreads();
+    if (warp == 0 && c < H) {
+#pragma unroll
+      for (int w = 1; w < kJoinSlices; ++w) add4(acc, tile[w][lane]);
+      embedding_store4(dw + id * (int64_t)H + c, accumulate, acc);
+    }
+    __syncthreads();  // the tile is written again
   }
 }
 
@@ -207,11 +302,17 @@ void launch_peagle_spec(const int64_t* anchor, const int64_t* depth, const bool*
   count_launch(1);
   launch_pdl(rows::peagle_spec_kernel, grid, 256, 0, stream, anchor, depth, row_valid, doc, doc_lo, n, T, num_depths, window, (const int*)table, lo, hi, extra);
 }
+int embedding_bwd_partial_rows(int n) { return n > rows::kSlice ? ((n - 1) / rows::kSlice + 1) * 2 : 0; }
 void launch_embedding_bwd(const int64_t* ids, const int64_t* order, const void* d, int64_t d_stride, int n, int H, int64_t vocab, int64_t padding, void* dw,
-                          int accumulate, cudaStream_t stream) {
+                          int accumulate, float* part, cudaStream_t stream) {
   if (n <= 0) return;
-  count_launch(1);
-  launch_pdl(rows::embedding_bwd_kernel, n, 256, 0, stream, ids, order, (const __nv_bfloat16*)d, d_stride, n, H, vocab, padding, (__nv_bfloat16*)dw, accumulate);
+  const int slices = (n - 1) / rows::kSlice + 1;
+  count_launch(slices > 1 ? 2 : 1);
+  launch_pdl(rows::embedding_bwd_kernel, n, 256, 0, stream, ids, order, (const __nv_bfloat16*)d, d_stride, n, H, vocab, padding, (__nv_bfloat16*)dw, accumulate,
+             part);
+  if (slices > 1)
+    launch_pdl(rows::embedding_join_kernel, dim3((slices - 1 + rows::kJoinSlices - 1) / rows::kJoinSlices, (H + 127) / 128), 256, 0, stream, ids,
+               (const float*)part, n, H, vocab, padding, (__nv_bfloat16*)dw, accumulate);
 }
 
 }  // namespace sb200

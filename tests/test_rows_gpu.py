@@ -105,3 +105,24 @@ def test_embedding_gradient(n, H, vocab, padding, attached):
         torch.nn.functional.embedding(ids, wf, padding).backward(d.float())
     got = w._flat_grad if attached else w.grad
     assert (got.float() - wf.grad).abs().max() <= 0.01 * wf.grad.abs().max()
+
+
+# an id that fills a slice of 32 positions, crosses one edge, two, 8 and 9 (the last that a warp sums alone), many (a padded tail), more
+# than 256 slices; H in part of a 128-column block
+@pytest.mark.parametrize("lengths,H", [([32, 32, 1], 8), ([31, 257, 256, 288, 289, 33], 264), ([33, 31, 1], 136), ([1, 31, 64, 3, 70], 2056), ([5, 2048, 7, 300], 256), ([8300], 24), ([17] * 40, 128), ([8] * 3 + [8192], 64)])
+@pytest.mark.parametrize("padding", [None, 1])
+@pytest.mark.parametrize("attached", [False, True])
+def test_embedding_gradient_of_frequent_ids(lengths, H, padding, attached):
+    torch.manual_seed(H)
+    ids = torch.repeat_interleave(torch.arange(len(lengths)) * 3, torch.tensor(lengths))[torch.randperm(sum(lengths))].cuda()
+    w = torch.zeros(3 * len(lengths) + 1, H, device="cuda").bfloat16().requires_grad_()
+    if attached:
+        w._flat_grad, w._grad_fresh = torch.full_like(w, float("nan")), True
+    d = torch.randn(ids.numel(), H, device="cuda").bfloat16()
+    for _ in range(2):
+        ops.embedding(ids, w, padding).backward(d)
+    got = (w._flat_grad if attached else w.grad).double()
+    keep = (ids != padding) if padding is not None else torch.ones_like(ids, dtype=torch.bool)
+    want, size = (torch.zeros(w.shape, dtype=torch.double, device="cuda").index_add_(0, ids[keep], 2 * x.double()[keep]) for x in (d, d.abs()))
+    # fp32 sums of at most max(lengths) terms; the sum is rounded to bf16, and so is its double
+    assert ((got - want).abs() <= 2.0**-8 * want.abs() + max(lengths) * 2.0**-24 * size).all()
