@@ -40,6 +40,7 @@
 #include <atomic>
 
 #include "loss_stats.cuh"
+#include "remember.h"
 #include "tcgen05_utils.cuh"
 
 namespace sb200 {
@@ -1152,28 +1153,26 @@ static int64_t pair_tile_count(int M, int N, int batch, int symmetric) {
   return batch * (symmetric ? m * (m + 1) / 2 : m * n);
 }
 
-// How many clusters of `size` CTAs (one per SM) the device holds at a time: the GPCs do not divide evenly.
+// How many clusters of `size` CTAs (one per SM) the device holds at a time: the GPCs do not divide evenly.  Where the runtime
+// does not say, three quarters of the SMs; a call with more clusters than fit takes a second wave.
 static int resident_clusters(int size) {
-  static std::atomic<int> cached[64][4];
+  static std::atomic<int> known[64][3];
   const int dev = PerDeviceOnce::device(), slot = size == 2 ? 0 : size == 4 ? 1 : 2;
-  if (dev >= 0 && cached[dev][slot] > 0) return cached[dev][slot];
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(kNumSM / size * size);
-  cfg.blockDim = dim3(tc::S_THREADS);
-  cfg.dynamicSmemBytes = tc::S_STAGES * tc::S_STAGE_BYTES + tc::S_RECV_BYTES + 1024;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = size;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, tc::gemm_small_kernel<false, false>, &cfg) != cudaSuccess || n < 1) {
+  return remember(dev >= 0 ? &known[dev][slot] : nullptr, [size](int* n) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(kNumSM / size * size);
+    cfg.blockDim = dim3(tc::S_THREADS);
+    cfg.dynamicSmemBytes = tc::S_STAGES * tc::S_STAGE_BYTES + tc::S_RECV_BYTES + 1024;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = size;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(n, tc::gemm_small_kernel<false, false>, &cfg) == cudaSuccess) return true;
     cudaGetLastError();
-    n = kNumSM / size * 3 / 4;
-  }
-  if (dev >= 0) cached[dev][slot] = n;
-  return n;
+    return false;
+  }, kNumSM / size * 3 / 4);
 }
 
 // The kernel for a plain product, by predicted time.  Each form costs a fixed part (launch, pipeline fill, epilogue,

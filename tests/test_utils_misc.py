@@ -185,3 +185,33 @@ def test_gated_mlp_activations():
         assert torch.allclose(mlp(x), (fn(gate) * up) @ mlp.down_proj.weight.t(), atol=1e-6)
     with pytest.raises(ValueError, match="not supported"):
         MLP(TransformerLayerConfig(**base, hidden_act="tanh"))
+
+
+def test_a_failed_query_is_asked_again(tmp_path):
+    """``csrc/remember.h``: the guess that stands in for a failed query is not kept, what the query says is."""
+    import shutil
+    import subprocess
+
+    from speculators_b200.ops import _build
+
+    gxx = shutil.which("g++")
+    if gxx is None:
+        pytest.skip("no g++")
+    src = tmp_path / "t.cpp"
+    src.write_text("""
+        #include "remember.h"
+        int main() {
+          std::atomic<int> kept{0};
+          int asked = 0;
+          bool ok = false;
+          auto query = [&](int* n) { ++asked; *n = 70; return ok; };
+          if (sb200::remember(&kept, query, 55) != 55 || sb200::remember(&kept, query, 54) != 54 || asked != 2) return 1;
+          ok = true;
+          if (sb200::remember(&kept, query, 55) != 70 || asked != 3) return 2;
+          ok = false;
+          if (sb200::remember(&kept, query, 55) != 70 || asked != 3) return 3;
+          return sb200::remember(nullptr, query, 55) != 55 || asked != 4 ? 4 : 0;
+        }
+    """)
+    subprocess.run([gxx, "-std=c++17", "-I", str(_build.CSRC), str(src), "-o", str(tmp_path / "t")], check=True)
+    assert subprocess.run([str(tmp_path / "t")]).returncode == 0
