@@ -120,6 +120,11 @@ __device__ __forceinline__ void st8(__nv_bfloat16* ptr, const bf16x8& v) {
   *reinterpret_cast<bf16x8*>(ptr) = v;
 }
 
+// A rotated channel pair, (x1 c - x2 s, x2 c + x1 s): the product with s rounds, the one with c is fused into the sum.  Spelled
+// out, so that every kernel that rotates gives the same bits however the compiler would contract the expression.
+__device__ __forceinline__ float rotate_first(float x1, float x2, float c, float s) { return __fmaf_rn(x1, c, -__fmul_rn(x2, s)); }
+__device__ __forceinline__ float rotate_second(float x1, float x2, float c, float s) { return __fmaf_rn(x2, c, __fmul_rn(x1, s)); }
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

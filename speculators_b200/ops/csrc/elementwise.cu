@@ -85,8 +85,8 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const int64_t* __rest
     __nv_bfloat16* p = x + t * row_stride + (int64_t)h * hd;
     const float x1 = __bfloat162float(p[i]);
     const float x2 = __bfloat162float(p[i + half]);
-    p[i] = __float2bfloat16(x1 * c - x2 * s);
-    p[i + half] = __float2bfloat16(x2 * c + x1 * s);
+    p[i] = __float2bfloat16(rotate_first(x1, x2, c, s));
+    p[i + half] = __float2bfloat16(rotate_second(x1, x2, c, s));
   }
 }
 
@@ -120,8 +120,8 @@ __global__ void rope_vec8_kernel(__nv_bfloat16* __restrict__ x, const int64_t* _
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const float sj = sign * sn[j];
-      y1[j] = x1[j] * c[j] - x2[j] * sj;
-      y2[j] = x2[j] * c[j] + x1[j] * sj;
+      y1[j] = rotate_first(x1[j], x2[j], c[j], sj);
+      y2[j] = rotate_second(x1[j], x2[j], c[j], sj);
     }
     st8(p, pack8(y1));
     st8(p + half, pack8(y2));
@@ -188,8 +188,8 @@ __global__ void __launch_bounds__(256) rope_merge_kernel(const RopeMerge a) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const float sj = a.sign * sn[j];
-      y1[j] = x1[j] * c[j] - x2[j] * sj;
-      y2[j] = x2[j] * c[j] + x1[j] * sj;
+      y1[j] = rotate_first(x1[j], x2[j], c[j], sj);
+      y2[j] = rotate_second(x1[j], x2[j], c[j], sj);
     }
     st8(dst + at, pack8(y1));
     st8(dst + at + half, pack8(y2));

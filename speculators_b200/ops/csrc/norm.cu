@@ -309,6 +309,30 @@ rmsnorm_dw_kernel(const NormBwdArgs p) {
 constexpr int kNarrowMaxH = 256;
 constexpr int kNarrowWarps = kNormThreads / 32;
 
+// The arithmetic of a narrow row's eight elements, rounding by rounding: the kernels below and the ones that do head norms and
+// rotation at once share it and give the same bits.  Sums take one fused multiply-add per element; x-hat = x rstd rounds, and
+// so does dy w; dx = rstd (dy w - x-hat dot) rounds x-hat dot, fuses dy w into the difference and rounds the product with rstd.
+__device__ __forceinline__ float narrow_squares(const float (&x)[8]) {
+  float ss = 0.f;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) ss = __fmaf_rn(x[j], x[j], ss);
+  return ss;
+}
+__device__ __forceinline__ float narrow_sums(const float (&dy)[8], const float (&w)[8], const float (&x)[8], float rstd, float (&dw)[8]) {
+  float dot = 0.f;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float xh = __fmul_rn(x[j], rstd);
+    dot = __fmaf_rn(__fmul_rn(dy[j], w[j]), xh, dot);
+    dw[j] = __fmaf_rn(dy[j], xh, dw[j]);
+  }
+  return dot;
+}
+__device__ __forceinline__ void narrow_dx(const float (&dy)[8], const float (&w)[8], const float (&x)[8], float rstd, float dot, float (&dx)[8]) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) dx[j] = __fmul_rn(rstd, __fmaf_rn(dy[j], w[j], -__fmul_rn(__fmul_rn(x[j], rstd), dot)));
+}
+
 __global__ void __launch_bounds__(kNormThreads)
 rmsnorm_fwd_narrow_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
                           float* __restrict__ rstd_out, int rows, int H, int64_t x_stride, int64_t y_stride, float eps, NormWeight nw) {
@@ -322,8 +346,7 @@ rmsnorm_fwd_narrow_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
     float xv[8], ss = 0.f;
     if (on) {
       unpack8(ld8(x + (int64_t)r * x_stride + (lane << 3)), xv);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) ss += xv[j] * xv[j];
+      ss = narrow_squares(xv);
     }
     ss = warp_sum(ss);
     const float rstd = rsqrtf(ss / (float)H + eps);
@@ -354,18 +377,12 @@ rmsnorm_bwd_narrow_kernel(const NormBwdArgs p) {
     if (on) {
       unpack8(ld8(p.x + (int64_t)r * p.x_stride + (lane << 3)), xv);
       unpack8(load_dy(p, r, lane << 3), dv);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float xh = xv[j] * rstd;
-        dot += dv[j] * wv[j] * xh;
-        dwacc[j] += dv[j] * xh;
-      }
+      dot = narrow_sums(dv, wv, xv, rstd, dwacc);
     }
     dot = warp_sum(dot) / (float)p.H;
     if (on) {
       float d[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) d[j] = rstd * (dv[j] * wv[j] - xv[j] * rstd * dot);
+      narrow_dx(dv, wv, xv, rstd, dot, d);
       store_dx(p, r, lane << 3, d);
     }
   }
@@ -450,8 +467,7 @@ __device__ __forceinline__ void rotate8(const HeadsRope& p, int64_t t, bool on, 
   for (int j = 0; j < 8; ++j) {
     const float sj = sign * sn[j];
     const float x1 = first ? v[j] : other[j], x2 = first ? other[j] : v[j];
-    // spelled out: what the compiler makes of x1 c - x2 s and x2 c + x1 s in the rotation kernels
-    v[j] = first ? __fmaf_rn(x1, c[j], -__fmul_rn(x2, sj)) : __fmaf_rn(x2, c[j], __fmul_rn(x1, sj));
+    v[j] = first ? rotate_first(x1, x2, c[j], sj) : rotate_second(x1, x2, c[j], sj);
   }
 }
 template <int L>
@@ -484,12 +500,11 @@ __global__ void __launch_bounds__(256) heads_fwd_kernel(const HeadsFwdArgs p) {
     const bool on = r < rows;
     const int64_t t = on ? r / all : 0;
     const int c = on ? (int)(r - t * all) : 0, which = c >= p.heads[0], h = which ? c - p.heads[0] : c;
-    float xv[8], wv[8], ss = 0.f;
+    float xv[8], wv[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) xv[j] = 0.f;
     if (on) unpack8(ld8(p.src + min(t, (int64_t)p.src_last) * p.src_stride + c * HD + l * 8), xv);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) ss += xv[j] * xv[j];
+    const float ss = narrow_squares(xv);
     nw.load(p.w[which] + l * 8, wv);
     const float rstd = rsqrtf(lanes_sum<L>(ss) / (float)HD + p.eps);
     if (on && l == 0) p.rstd[(which ? (int64_t)p.tokens * p.heads[0] : 0) + t * p.heads[which] + h] = rstd;
@@ -567,7 +582,7 @@ __global__ void __launch_bounds__(256) heads_bwd_kernel(const HeadsBwdArgs p) {
     const int64_t ct = t;
     const int ch = h;
     const float rstd = rn;
-    float xv[8], dv[8], dot = 0.f;
+    float xv[8], dv[8];
     unpack8(dn, dv);
     unpack8(xn, xv);
     if (i + 1 < trips) {  // the next row's loads are in flight during this one's sums
@@ -579,17 +594,11 @@ __global__ void __launch_bounds__(256) heads_bwd_kernel(const HeadsBwdArgs p) {
     }
     rotate8(p.rope, ct, cur_on, l, -1.f, dv);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      dv[j] = cur_on ? round_bf16(dv[j]) : 0.f;
-      const float xh = xv[j] * rstd;
-      dot += dv[j] * wv[j] * xh;
-      dwacc[j] += dv[j] * xh;
-    }
-    dot = lanes_sum<L>(dot) / (float)HD;
+    for (int j = 0; j < 8; ++j) dv[j] = cur_on ? round_bf16(dv[j]) : 0.f;
+    const float dot = lanes_sum<L>(narrow_sums(dv, wv, xv, rstd, dwacc)) / (float)HD;
     if (cur_on) {
       float d[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) d[j] = rstd * __fmaf_rn(dv[j], wv[j], -__fmul_rn(__fmul_rn(xv[j], rstd), dot));  // as in the narrow kernel
+      narrow_dx(dv, wv, xv, rstd, dot, d);
       st8(p.dst + ct * p.dst_stride + col0 + ch * HD + l * 8, pack8(d));
     }
   }
