@@ -8,6 +8,7 @@ import pytest
 import torch
 
 import speculators_b200 as sb
+from speculators_b200 import ops
 from speculators_b200.train import Trainer, TrainerConfig
 from speculators_b200.train.synthetic import SyntheticLoader
 
@@ -234,3 +235,40 @@ def test_muon_on_gpu_tracks_the_fp32_engine():
         # matrices: Newton-Schulz in bf16 against fp32; vectors (AdamW): the first steps are sign-like, bf16 gradients flip a few
         tol = 0.15 if w.ndim == 2 else 0.4
         assert (w - g_).abs().max() < tol * moved + 1e-4, (name, float((w - g_).abs().max()), float(moved))
+
+
+@pytest.mark.parametrize("name", ["kl_div", "ce"])
+def test_fused_head_and_default_head_give_the_same_passes(name, monkeypatch):
+    """The switch ``SB200_FUSED_HEAD`` has a tail of its own behind its row losses: running loss, counters, ``prev_correct`` and
+    the gradient of the hidden states over three passes against the default's."""
+    from speculators_b200.losses.utils import resolve_loss_config
+    from speculators_b200.models.eagle3 import metrics as em
+
+    torch.manual_seed(0)
+    T, H, V = 300, 128, 512
+    weight = (torch.randn(V, H, device="cuda") * 0.3).bfloat16()
+    states = [(torch.randn(T, H, device="cuda")).bfloat16() for _ in range(3)]
+    targets = states[0] @ weight.t()  # the first pass is right everywhere, the others in places
+    for s, hidden in enumerate(states[1:], 1):
+        hidden[: T // 2] = states[0].roll(-s, 0)[: T // 2]
+    mask = torch.rand(1, T, device="cuda") > 0.4
+    config, results = resolve_loss_config(f'{{"{name}": 0.5}}'), []
+    for fused in (True, False):
+        monkeypatch.setenv("SB200_FUSED_HEAD", "1" if fused else "0")
+        prev, loss, log, grads = mask.clone(), None, {}, []
+        xs = [h.clone().requires_grad_() for h in states]
+        for step, x in enumerate(xs):
+            if fused:
+                loss, m = em.compute_metrics_from_hidden(x, weight, targets.unsqueeze(0), mask, prev, step, 0.8, config, earlier=loss)
+            else:
+                loss, m = em.compute_metrics(ops.linear(x, weight).unsqueeze(0), targets.unsqueeze(0), mask, prev, step, 0.8, config, earlier=loss)
+            log.update({k: float(v) for k, v in m.items()})
+        loss.backward()
+        results.append((float(loss), log, prev, [x.grad.float() for x in xs]))
+    (la, ma, pa, ga), (lb, mb, pb, gb) = results
+    # the same bf16 logits, statistics summed in another order; the gradients are bf16
+    assert abs(la - lb) <= 1e-4 * abs(lb) and torch.equal(pa, pb) and set(ma) == set(mb)
+    assert all(abs(ma[k] - mb[k]) <= 1e-4 * abs(mb[k]) + 1e-6 for k in mb)
+    assert 0 < mb["cond_acc_2_total"] < mb["cond_acc_1_total"]
+    for a, b in zip(ga, gb):
+        assert (a - b).abs().max() <= 0.01 * b.abs().max()
