@@ -409,8 +409,11 @@ def _gather_use(weight: torch.Tensor, rows: tuple, use: _Use | None, operands: t
     key = (id(weight), *rows)
     _, uses, _ = work.pending.setdefault(key, (weight, [], launch))
     uses.append(operands)
-    # contractions of 8192 rows are long enough on their own (28672 x 4096, three uses: 4380 us apart, 4430 together;
-    # of 2048 rows 1150 and 1075); rows grouped by expert are few for each
+    # Three uses as one product against three, weights of 4096 x 4096 to 57344 x 8192: of 736 rows 1.7 to 2.1 times as fast, of
+    # 2048 rows 1.04 to 1.16, of 4096 1.01 to 1.05, of 6144 0.996 to 1.03, of 8192 1.01 to 1.02 (28672 x 4096: 665 and 388 us,
+    # 1106 and 1049, 1989 and 1949, 2835 and 2846, 4134 and 4104).  Past 6144 rows that is within the spread of the runs and not
+    # worth keeping the uses' operands for; only the smallest that are gathered would still gain there (2048 x 2048, 8192 rows:
+    # 1.16, some 25 us).  Rows grouped by expert are few for each.
     whole = weight.numel() < _GATHER_ELEMENTS or (weight.dim() == 2 and operands[0].shape[0] > 6144)
     if left == 0 or len(uses) == _MAX_USES or whole:
         work.run(key)

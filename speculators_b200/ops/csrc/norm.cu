@@ -718,7 +718,12 @@ void launch_rmsnorm_fwd(const void* x, const void* w, const int64_t* row_index, 
                (__nv_bfloat16*)y, rstd, rows, H, x_stride, y_stride, eps, nw);
     return;
   }
-  // narrow rows, few of them: a block each (1001 x 2048 4.2 us, 4.6 walking); wide ones are better walked (1536 x 24576 51 and 42)
+  // A block a row, or blocks that walk rows with the next one in flight.  Measured at 512 to 24576 columns, 128 to 16384 rows
+  // (us, a block each and walking).  From L2, back to back: up to 4096 columns walking never gains up to 2368 rows and loses
+  // up to a third (1536 x 4096 7.2 and 9.7, 2048 x 2048 6.2 and 6.4), behind them 2 to 20 % (3000 x 2048 8.4 and 9.9, 8192 x
+  // 4096 33.8 and 35.9).  From memory it is level or gains a tenth there (8192 x 2048 28.7 and 26.8, 2368 x 4096 18.4 and
+  // 16.4) and 15 to 20 % on wide rows, where a block's loads are long (1536 x 24576 57 and 47, from L2 51 and 42).  The line
+  // gives few narrow rows, which the step's kernels find in L2, a block each.
   auto grid = [&](int blocks) {
     if (H <= 4096 && rows <= 16 * kNumSM) return rows;
     const int most = blocks * kNumSM, rounds = (rows + most - 1) / most;

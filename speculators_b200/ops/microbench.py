@@ -236,7 +236,7 @@ def main(argv: list[str] | None = None) -> int:
     ap.add_argument("--warmup", type=int, default=3)
     ap.add_argument("--no-flush", action="store_true", help="do not rewrite an L2-sized buffer between iterations")
     ap.add_argument("--peaks", default=None, help="JSON file with measured hbm_gbs and bf16_tflops")
-    ap.add_argument("--variant", type=int, default=0, help="gemm: 0 choose, 1 one CTA per tile, 2 CTA pairs")
+    ap.add_argument("--variant", type=int, default=0, help="gemm: 0 choose, 10 .. 13 tiles of 128 x 64 on 1, 2, 4, 8 CTAs, 3 CTA pairs (2: 64-wide K stages), 4 / 5 over 2 / 4 pairs")
     ap.add_argument("-m", type=int, default=2048)
     ap.add_argument("-n", type=int, default=6144)
     ap.add_argument("-k", type=int, default=8192)
