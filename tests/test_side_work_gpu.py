@@ -98,3 +98,35 @@ def test_memory_after_a_pass_that_an_exception_ended():
     ops.linear(x, w).sum().backward()
     want = torch.ones(64, 512, device="cuda").t() @ x.float()
     assert (w._flat_grad.float() - want).abs().max() <= 0.01 * want.abs().max()
+
+
+def test_an_exception_inside_a_capture_leaves_the_streams_usable():
+    torch.manual_seed(0)
+    w = _weight(512, 512)
+    x = torch.randn(256, 512, device="cuda").bfloat16().requires_grad_()
+    stream = torch.cuda.Stream()
+
+    def step(fail):
+        w._grad_fresh = True
+        y = ops.linear(x, w)
+        if fail:
+            y.register_hook(lambda g: (_ for _ in ()).throw(RuntimeError("stop")))
+        torch.autograd.backward(ops.linear(y, w).float().pow(2).mean(), inputs=[x, w])
+
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        step(False)
+    torch.cuda.current_stream().wait_stream(stream)
+    want = w._flat_grad.clone()
+    with pytest.raises(RuntimeError, match="stop"):
+        with torch.cuda.graph(torch.cuda.CUDAGraph(), stream=stream):
+            step(True)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        step(False)
+    w._flat_grad.fill_(float("nan"))
+    graph.replay()
+    assert torch.equal(w._flat_grad, want)
+    w._flat_grad.fill_(float("nan"))
+    step(False)
+    assert torch.equal(w._flat_grad, want)
