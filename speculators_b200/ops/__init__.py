@@ -397,7 +397,8 @@ def _gather_use(weight: torch.Tensor, rows: tuple, use: _Use | None, operands: t
     pass's end runs what is left and joins the streams, and so does any other gradient of the same weight."""
     left = use.left() if use is not None else 0
     task = torch._C._current_graph_task_id()
-    if task < 0:
+    if task < 0:  # a node's backward called by hand
+        _wait_for_side_work(weight)  # of a pass that an exception ended
         launch([operands])
         return
     main = torch.cuda.current_stream(weight.device)

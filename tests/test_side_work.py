@@ -160,3 +160,17 @@ def test_a_pass_that_an_exception_ends_gives_its_operands_back(streams, width):
     launched = []
     _product(x, w, main, "d", lambda _: launched.append("d" in ops._SIDE_STREAMS[0, main.cuda_stream].behind)).sum().backward()
     assert launched == [True]
+
+
+def test_a_gradient_outside_a_pass_comes_behind_one_that_an_exception_ended(streams):
+    caller, main = streams
+    w, x = _weight(), torch.ones(4, 64, requires_grad=True)
+
+    def stop(_):
+        raise ValueError("stop")
+
+    with pytest.raises(ValueError, match="stop"):
+        _product(x, w, main, "a", stop).sum().backward()
+    before = []
+    ops._gather_use(w, (None, None), None, (x, x), lambda uses: before.append("a" in caller.behind))
+    assert before == [True]
