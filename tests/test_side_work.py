@@ -37,8 +37,10 @@ def streams(monkeypatch):
     @contextlib.contextmanager
     def stream(s):
         now.append(s)
-        yield
-        now.pop()
+        try:
+            yield
+        finally:
+            now.pop()
 
     monkeypatch.setattr(torch.cuda, "Stream", _Stream)
     monkeypatch.setattr(torch.cuda, "stream", stream)
