@@ -17,7 +17,7 @@ from speculators_b200.losses import LossConfig, exp_loss_decay, kl_div_loss, red
 from speculators_b200.losses.rowwise import rowwise_terms
 from speculators_b200.models.metrics import compute_accuracy_single_step
 
-__all__ = ["align_for_step", "compute_metrics", "compute_metrics_from_hidden"]
+__all__ = ["align_for_step", "compute_metrics", "compute_metrics_from_hidden", "compute_metrics_of_rows", "step_tail_is_fused"]
 
 
 def align_for_step(logits, targets, loss_mask, prev_correct, ttt_step: int):
@@ -71,12 +71,31 @@ def _compute_metrics_fused(logits, targets, loss_mask, prev_correct, ttt_step: i
         loss = out[0] * weight
         stats, step_loss, one = out.detach(), loss.detach(), torch.ones((), device=out.device)
         loss = loss if earlier is None else earlier + loss
-    metrics = {
+    return loss, _fused_metrics(ttt_step, stats, step_loss, one)
+
+
+def _fused_metrics(ttt_step: int, stats, step_loss, one) -> dict[str, torch.Tensor]:
+    return {
         f"loss_{ttt_step}_sum": step_loss, f"loss_{ttt_step}_total": one,
         f"full_acc_{ttt_step}_sum": stats[1], f"full_acc_{ttt_step}_total": stats[2],
         f"cond_acc_{ttt_step}_sum": stats[1], f"cond_acc_{ttt_step}_total": stats[3],
     }
-    return loss, metrics
+
+
+def step_tail_is_fused(loss_config: LossConfig | None) -> bool:
+    """Whether a pass's loss and counters run as one row-loss kernel and one tail (given bf16 CUDA logits and a loss mask)."""
+    return USE_FUSED_TAIL and (loss_config is None or _single_fused_primitive(loss_config) is not None)
+
+
+def compute_metrics_of_rows(logits, targets, rows, ttt_step: int, ttt_step_loss_decay: float, loss_config: LossConfig | None = None, earlier=None):
+    """``compute_metrics`` where ``logits`` and ``targets`` hold the rows that ``ops.step_rows`` lists."""
+    from speculators_b200 import ops
+    from speculators_b200.losses.utils import _REDUCTION_EPS
+
+    op, weight = _single_fused_primitive(loss_config or {"kl_div": (kl_div_loss, 1.0)})
+    loss, stats = ops.ttt_step_loss(op, logits, targets, earlier, 0, logits.shape[0], rows.mask[ttt_step], rows.prev_correct,
+                                    float(ttt_step_loss_decay) ** ttt_step * weight, _REDUCTION_EPS, target_row=rows.target_row[ttt_step], live=rows.live)
+    return loss, _fused_metrics(ttt_step, stats, stats[0], stats[4])
 
 
 def compute_metrics_from_hidden(hidden, head_weight, targets, loss_mask, prev_correct, ttt_step: int, ttt_step_loss_decay: float,

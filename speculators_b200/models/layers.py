@@ -41,12 +41,12 @@ class RMSNorm(nn.Module):
         self.weight = nn.Parameter(torch.ones(hidden_size))
         self.variance_epsilon = eps
 
-    def forward(self, x: torch.Tensor) -> torch.Tensor:
-        return ops.rms_norm(x, self.weight, self.variance_epsilon)
+    def forward(self, x: torch.Tensor, live: torch.Tensor | None = None) -> torch.Tensor:
+        return ops.rms_norm(x, self.weight, self.variance_epsilon, live=live)
 
-    def fork(self, x: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
+    def fork(self, x: torch.Tensor, live: torch.Tensor | None = None) -> tuple[torch.Tensor, torch.Tensor]:
         """``(self(x), x)``: the input of a pre-norm block and its residual branch."""
-        return ops.rms_norm_fork(x, self.weight, self.variance_epsilon)
+        return ops.rms_norm_fork(x, self.weight, self.variance_epsilon, live=live)
 
     def extra_repr(self) -> str:
         return f"{tuple(self.weight.shape)}, eps={self.variance_epsilon}"
@@ -70,10 +70,10 @@ class Linear(nn.Module):
         self.row_parallel = None
         _init_linear_(self.weight, std)
 
-    def forward(self, x: torch.Tensor, residual: torch.Tensor | None = None) -> torch.Tensor:
+    def forward(self, x: torch.Tensor, residual: torch.Tensor | None = None, live: torch.Tensor | None = None) -> torch.Tensor:
         if self.row_parallel is not None and self.bias is None:
             return self.row_parallel(x, self.weight, residual)
-        return ops.linear(x, self.weight, self.bias, residual=residual)
+        return ops.linear(x, self.weight, self.bias, residual=residual, live=live)
 
     def extra_repr(self) -> str:
         return f"in={self.in_features}, out={self.out_features}, bias={self.bias is not None}"
@@ -119,8 +119,8 @@ class FusedLinear(nn.Module):
             acc += s
         return out
 
-    def forward(self, x: torch.Tensor) -> torch.Tensor:
-        return ops.linear(x, self.weight, self.bias)
+    def forward(self, x: torch.Tensor, live: torch.Tensor | None = None) -> torch.Tensor:
+        return ops.linear(x, self.weight, self.bias, live=live)
 
     def forward_parts(self, x: torch.Tensor, first: int, last: int) -> torch.Tensor:
         """Apply only parts ``first .. last-1`` (row slice of the fused weight)."""
@@ -233,25 +233,26 @@ class Attention(nn.Module):
         self.q_norm = RMSNorm(self.hd, config.rms_norm_eps) if use_qk_norm else None
         self.k_norm = RMSNorm(self.hd, config.rms_norm_eps) if use_qk_norm else None
 
-    def project_qkv(self, x: torch.Tensor, positions: torch.Tensor, rotary: RotaryTable, split: int | None = None, repeated: bool = False):
+    def project_qkv(self, x: torch.Tensor, positions: torch.Tensor, rotary: RotaryTable, split: int | None = None, repeated: bool = False,
+                    live: torch.Tensor | None = None):
         """x [T, in] -> (q [T, nh, hd], k [T, nkv, hd], v [T, nkv, hd]) with per-head
         norms (if any) and rotary embedding applied; with ``split`` k and v come as
         two tensors each, the rows below it and the rows from it on.  ``repeated``: ``x`` has
         ``split + 2`` rows, the rows from ``split`` on all read row ``split`` (``ops.repeat_rows``)."""
         T = positions.shape[0]
         nq, nk = self.nh * self.hd, self.nkv * self.hd
-        qkv = self.qkv_proj(x)
+        qkv = self.qkv_proj(x, live)
         if self.q_norm is not None:
             return ops.norm_rope_heads(qkv, self.q_norm.weight, self.k_norm.weight, self.q_norm.variance_epsilon, positions, rotary.cos,
-                                       rotary.sin, (self.nh, self.nkv, self.nkv), self.hd, self.rot, split, repeated)
+                                       rotary.sin, (self.nh, self.nkv, self.nkv), self.hd, self.rot, split, repeated, live)
         if repeated:
             qkv = ops.repeat_rows(qkv, T)
-        q, k, v = ops.rope_split(qkv, positions, rotary.cos, rotary.sin, self.nh + self.nkv, self.hd, self.rot, nq, nk)
+        q, k, v = ops.rope_split(qkv, positions, rotary.cos, rotary.sin, self.nh + self.nkv, self.hd, self.rot, nq, nk, live)
         q, k, v = q.view(T, self.nh, self.hd), k.view(T, self.nkv, self.hd), v.view(T, self.nkv, self.hd)
         return (q, k, v) if split is None else (q, k[:split], k[split:], v[:split], v[split:])
 
     def forward(self, x, positions, rotary, spec: AttnSpec, past: list | None = None, ctx_len: int | None = None,
-                residual: torch.Tensor | None = None, repeated: bool = False) -> torch.Tensor:
+                residual: torch.Tensor | None = None, repeated: bool = False, rows: ops.StepRows | None = None, dense: bool = False) -> torch.Tensor:
         """``past`` (EAGLE-3 TTT): list of (k, v) of earlier passes over the same
         positions.  Entry 0 is the context the interval part of ``spec`` indexes;
         later entries and this pass's own keys are reachable through
@@ -259,13 +260,21 @@ class Attention(nn.Module):
 
         ``ctx_len`` (P-EAGLE): the first ``ctx_len`` rows of this pass are the
         interval-addressed context, the remaining rows are the extra keys; ``repeated``
-        says that ``x`` holds those only once (``project_qkv``)."""
+        says that ``x`` holds those only once (``project_qkv``).
+
+        ``rows``: the rows that the step needs (``ops.step_rows``).  The inputs are of those rows, or of the whole batch
+        (``dense``: keys and values of all rows are context), the result and ``spec`` are of those rows."""
         T = positions.shape[0]
+        live = rows.live if rows is not None and not dense else None
         if ctx_len is not None and ctx_len < T:
             q, k_ctx, k_ext, v_ctx, v_ext = self.project_qkv(x, positions, rotary, split=ctx_len, repeated=repeated)
             out = ops.masked_attention(q, k_ctx, v_ctx, spec, k_ext, v_ext, scale=self.scaling)
             return self.o_proj(out.reshape(T, self.nh * self.hd), residual=residual)
-        q, k, v = self.project_qkv(x, positions, rotary)
+        q, k, v = self.project_qkv(x, positions, rotary, live=live)
+        if dense:
+            live = rows.live
+            q, residual = ops.take_rows(rows.index, rows.inverse, live, q.reshape(T, -1), residual)
+            q = q.view(T, self.nh, self.hd)
         if past is None:
             out = ops.masked_attention(q, k, v, spec, scale=self.scaling)
         else:
@@ -276,7 +285,7 @@ class Attention(nn.Module):
                 out = ops.masked_attention(q, k_ctx, v_ctx, spec, k_ext, v_ext, scale=self.scaling)
             else:
                 out = ops.masked_attention(q, k_ctx, v_ctx, spec, scale=self.scaling)
-        return self.o_proj(out.reshape(T, self.nh * self.hd), residual=residual)
+        return self.o_proj(out.reshape(T, self.nh * self.hd), residual=residual, live=live)
 
 
 _GATE_ACTIVATIONS = {
@@ -301,19 +310,19 @@ class MLP(nn.Module):
         self.gate_up_proj = FusedLinear(config.hidden_size, ["gate_proj", "up_proj"], [inter, inter], bias=bool(config.mlp_bias)).attach(self, "gate_up_proj")
         self.down_proj = Linear(inter, config.hidden_size, bias=bool(config.mlp_bias))
 
-    def forward(self, x: torch.Tensor, residual: torch.Tensor | None = None) -> torch.Tensor:
+    def forward(self, x: torch.Tensor, residual: torch.Tensor | None = None, live: torch.Tensor | None = None) -> torch.Tensor:
         silu = self.hidden_act in ("silu", "swish")
         if silu and self.gate_up_proj.bias is None:
-            hidden = ops.linear_swiglu(x, self.gate_up_proj.weight)  # activation in the GEMM's epilogue
+            hidden = ops.linear_swiglu(x, self.gate_up_proj.weight, live)  # activation in the GEMM's epilogue
             if hidden is not None:
-                return self.down_proj(hidden, residual=residual)
-        gate_up = self.gate_up_proj(x)
+                return self.down_proj(hidden, residual=residual, live=live)
+        gate_up = self.gate_up_proj(x, live)
         if silu:
-            hidden = ops.swiglu(gate_up)
+            hidden = ops.swiglu(gate_up, live)
         else:
             gate, up = gate_up.chunk(2, dim=-1)
             hidden = _GATE_ACTIVATIONS[self.hidden_act](gate) * up
-        return self.down_proj(hidden, residual=residual)
+        return self.down_proj(hidden, residual=residual, live=live)
 
 
 class DecoderLayer(nn.Module):
@@ -326,8 +335,10 @@ class DecoderLayer(nn.Module):
         self.input_layernorm = RMSNorm(config.hidden_size, config.rms_norm_eps)
         self.post_attention_layernorm = RMSNorm(config.hidden_size, config.rms_norm_eps)
 
-    def forward(self, x, positions, rotary, spec, past=None, ctx_len=None) -> torch.Tensor:
-        normed, x = self.input_layernorm.fork(x)
-        x = self.self_attn(normed, positions, rotary, spec, past, ctx_len, residual=x)
-        normed, x = self.post_attention_layernorm.fork(x)
-        return self.mlp(normed, residual=x)
+    def forward(self, x, positions, rotary, spec, past=None, ctx_len=None, rows=None, dense=False) -> torch.Tensor:
+        """``rows``, ``dense``: as in ``Attention``."""
+        live = rows.live if rows is not None else None
+        normed, x = self.input_layernorm.fork(x, None if dense else live)
+        x = self.self_attn(normed, positions, rotary, spec, past, ctx_len, residual=x, rows=rows, dense=dense)
+        normed, x = self.post_attention_layernorm.fork(x, live)
+        return self.mlp(normed, residual=x, live=live)

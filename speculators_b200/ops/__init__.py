@@ -19,6 +19,7 @@ import collections
 import contextlib
 import math
 import weakref
+from typing import NamedTuple
 
 import torch
 import torch.nn.functional as F
@@ -28,6 +29,7 @@ from speculators_b200.ops.attention import AttnSpec, masked_attention, masked_at
 
 __all__ = [
     "AttnSpec",
+    "StepRows",
     "LOSS_OPS",
     "adamw_step_",
     "eagle3_input_concat",
@@ -55,11 +57,14 @@ __all__ = [
     "rms_norm",
     "rms_norm_fork",
     "rms_norm_pair",
+    "rms_norm_taken",
     "rope_",
     "rope_split",
     "split_gated_query",
+    "step_rows",
     "sum_of_squares",
     "swiglu",
+    "take_rows",
     "token_cross_entropy",
     "ttt_step_loss",
     "ttt_step_tail",
@@ -120,7 +125,16 @@ def check_gemm_status() -> None:
             raise RuntimeError(f"a tcgen05 kernel on cuda:{idx} gave up waiting (code {code}: {_WAIT_CODES.get(code, 'unknown wait')})")
 
 
-def _forward_gemm(x2: torch.Tensor, w: torch.Tensor, residual: torch.Tensor | None) -> torch.Tensor:
+# ``live`` (here and below): an int32 tensor on the device that says how many of the rows hold anything (``step_rows``).  The
+# kernels neither read nor write the rows behind; what runs elsewhere takes all rows, and a sum over rows leaves those out.
+def _without_unused(x2: torch.Tensor, live: torch.Tensor | None) -> torch.Tensor:
+    if live is None:
+        return x2
+    used = torch.arange(x2.shape[0], device=x2.device) < live
+    return torch.where(used[:, None], x2, torch.zeros((), dtype=x2.dtype, device=x2.device))
+
+
+def _forward_gemm(x2: torch.Tensor, w: torch.Tensor, residual: torch.Tensor | None, live: torch.Tensor | None = None) -> torch.Tensor:
     """``x2 @ w.T (+ residual)`` for 2-D operands.  bf16 CUDA operands with 16-byte aligned
     rows run on the package's tcgen05 kernel (the residual is read in its epilogue, no
     copy of it is made); everything else goes to the library."""
@@ -128,27 +142,28 @@ def _forward_gemm(x2: torch.Tensor, w: torch.Tensor, residual: torch.Tensor | No
         residual is None or (_gemm_operand_ok(residual) and residual.shape == (x2.shape[0], w.shape[0]))
     ):
         out = torch.empty((x2.shape[0], w.shape[0]), dtype=x2.dtype, device=x2.device)
-        native().gemm_tn(x2, w, out, residual, 2 if residual is not None else 0, gemm_status(x2.device))
+        native().gemm_tn(x2, w, out, residual, 2 if residual is not None else 0, gemm_status(x2.device), live)
         return out
     if residual is not None:
         return torch.addmm(residual, x2, w.t())
     return x2 @ w.t()
 
 
-def _dgrad_gemm(dy2: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, accumulate: bool = False) -> torch.Tensor:
+def _dgrad_gemm(dy2: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, accumulate: bool = False,
+                live: torch.Tensor | None = None) -> torch.Tensor:
     """``dy2 @ w`` (input gradient of a linear layer) on the tcgen05 kernel: the weight is read
     as stored, ``[out, in]`` with ``in`` contiguous, as an MN-major B operand."""
     dx = out if out is not None else torch.empty((dy2.shape[0], w.shape[1]), dtype=dy2.dtype, device=dy2.device)
-    native().gemm(dy2, w, dx, 1 if accumulate else 0, False, True, gemm_status(dy2.device))
+    native().gemm(dy2, w, dx, 1 if accumulate else 0, False, True, gemm_status(dy2.device), live)
     return dx
 
 
-def _wgrad_gemm(dy2: torch.Tensor, x2: torch.Tensor, out: torch.Tensor | None, accumulate: bool) -> torch.Tensor:
+def _wgrad_gemm(dy2: torch.Tensor, x2: torch.Tensor, out: torch.Tensor | None, accumulate: bool, live: torch.Tensor | None = None) -> torch.Tensor:
     """``dy2.T @ x2`` (weight gradient) on the tcgen05 kernel, both operands read in place as
     MN-major tiles, stored into or added to ``out`` in the epilogue."""
     if out is None:
         out = torch.empty((dy2.shape[1], x2.shape[1]), dtype=dy2.dtype, device=dy2.device)
-    native().gemm(dy2, x2, out, 1 if accumulate else 0, True, True, gemm_status(dy2.device))
+    native().gemm(dy2, x2, out, 1 if accumulate else 0, True, True, gemm_status(dy2.device), live)
     return out
 
 
@@ -267,22 +282,22 @@ class _LinearFn(torch.autograd.Function):
     """
 
     @staticmethod
-    def forward(ctx, x, weight, residual, r0, r1, use):
+    def forward(ctx, x, weight, residual, r0, r1, use, live):
         # x is [rows, in]; the result is a fresh tensor (never a view), so callers may
         # rotate / normalise it in place
         w = weight if r0 is None else weight[r0:r1]
-        y = _forward_gemm(x, w, residual)
-        ctx.save_for_backward(x, weight)
+        y = _forward_gemm(x, w, residual, live)
+        ctx.save_for_backward(x, weight, live)
         ctx.rows, ctx.use = (r0, r1), use
         ctx.has_residual = residual is not None
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        x2, weight = ctx.saved_tensors
-        dx, dw = _linear_backward(x2, weight, ctx.rows, ctx.use, dy, ctx.needs_input_grad[0], ctx.needs_input_grad[1])
+        x2, weight, live = ctx.saved_tensors
+        dx, dw = _linear_backward(x2, weight, ctx.rows, ctx.use, dy, ctx.needs_input_grad[0], ctx.needs_input_grad[1], live)
         dres = dy if ctx.has_residual and ctx.needs_input_grad[2] else None
-        return dx, dw, dres, None, None, None
+        return dx, dw, dres, None, None, None, None
 
 
 _MAX_USES = 4  # of a weight in one product (the kernel's operand maps)
@@ -422,7 +437,7 @@ def _gather_use(weight: torch.Tensor, rows: tuple, use: _Use | None, operands: t
         work.run(next(iter(work.pending)))
 
 
-def _linear_backward(x2, weight, rows, use, dy, need_dx: bool, need_dw: bool):
+def _linear_backward(x2, weight, rows, use, dy, need_dx: bool, need_dw: bool, live=None):
     """``(dx, dw)`` of ``y = x2 @ weight[rows].T``; ``dw`` is ``None`` when the gradient went
     straight into the flat buffer the training engine attached to the weight.  ``use``: what ``_note_use`` gave the product."""
     r0, r1 = rows
@@ -431,49 +446,58 @@ def _linear_backward(x2, weight, rows, use, dy, need_dx: bool, need_dw: bool):
     dx = dw = None
     own = own_gemm_enabled() and _gemm_operand_ok(dy2) and _gemm_operand_ok(w) and _gemm_operand_ok(x2)
     if need_dx:
-        dx = _dgrad_gemm(dy2, w) if own else dy2 @ w
+        dx = _dgrad_gemm(dy2, w, live=live) if own else dy2 @ w
+    if need_dw and not own:
+        dy2, x2 = _without_unused(dy2, live), _without_unused(x2, live)
     if need_dw:
         flat = getattr(weight, "_flat_grad", None)
         if flat is not None and own and _gemm_operand_ok(flat if r0 is None else flat[r0:r1]) and x2.shape[0] > 0:
             def launch(uses):
                 # the first gradient of these rows since the engine's zero_grad, which left the buffer uncleared, is stored
                 target, accumulate = _param_grad_target(weight, beside=True)[:2] if r0 is None else _row_grad_target(weight, r0, r1, beside=True)
-                native().gemm_wgrad_parts([u[0] for u in uses], [u[1] for u in uses], target, accumulate, gemm_status(target.device))
+                status = gemm_status(target.device)
+                all_rows = status[:0]
+                native().gemm_wgrad_parts_rows([u[0] for u in uses], [u[1] for u in uses], target, accumulate, status,
+                                               [all_rows if u[2] is None else u[2] for u in uses])
 
-            _gather_use(weight, (r0, r1), use, (dy2, x2), launch)
+            _gather_use(weight, (r0, r1), use, (dy2, x2, live), launch)
         elif flat is not None:
             if use is not None:
                 use.left()
+            dy2, x2 = (_without_unused(t, live if own else None) for t in (dy2, x2))
             target, accumulate = _param_grad_target(weight)[:2] if r0 is None else _row_grad_target(weight, r0, r1)
             if accumulate:
                 target.addmm_(dy2.t(), x2)
             else:
                 torch.mm(dy2.t(), x2, out=target)
         elif r0 is None:
-            dw = _wgrad_gemm(dy2, x2, None, accumulate=False) if own else dy2.t() @ x2
+            dw = _wgrad_gemm(dy2, x2, None, accumulate=False, live=live) if own else dy2.t() @ x2
         else:
             dw = torch.zeros_like(weight)
             if own and _gemm_operand_ok(dw[r0:r1]):
-                _wgrad_gemm(dy2, x2, dw[r0:r1], accumulate=False)
+                _wgrad_gemm(dy2, x2, dw[r0:r1], accumulate=False, live=live)
             else:
+                dy2, x2 = (_without_unused(t, live if own else None) for t in (dy2, x2))
                 dw[r0:r1] = dy2.t() @ x2
     return dx, dw
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = None, residual: torch.Tensor | None = None,
-           rows: tuple[int, int] | None = None) -> torch.Tensor:
+           rows: tuple[int, int] | None = None, live: torch.Tensor | None = None) -> torch.Tensor:
     """``x @ weight[rows].T (+ bias) (+ residual)``.  On CUDA in bf16 the forward product
     runs on the package's tcgen05 GEMM with the residual read in its epilogue
     (``SB200_LINEAR_GEMM=cublas`` sends it to the library instead); the two backward
     products run on the same kernel with the transposed operands read in place (MN-major
     tiles), the weight gradient accumulating in the epilogue into the engine's flat
-    gradient buffer."""
+    gradient buffer.  ``live``: see ``step_rows`` (no bias then)."""
+    if live is not None and bias is not None:
+        raise ValueError("linear: a bias takes all rows")
     if x.is_cuda and (weight.requires_grad or x.requires_grad) and torch.is_grad_enabled():
         r0, r1 = rows if rows is not None else (None, None)
         lead = x.shape[:-1]
         x2 = x.reshape(-1, x.shape[-1])
         res2 = residual.reshape(-1, residual.shape[-1]) if residual is not None else None
-        y = _LinearFn.apply(x2, weight, res2, r0, r1, _note_use(weight, r0, r1) if weight.requires_grad else None)
+        y = _LinearFn.apply(x2, weight, res2, r0, r1, _note_use(weight, r0, r1) if weight.requires_grad else None, live)
         if len(lead) != 1:
             y = y.view(*lead, y.shape[-1])
         if bias is not None:
@@ -484,7 +508,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
     if x.is_cuda and x.dtype == torch.bfloat16 and b is None and not torch.is_grad_enabled() and own_gemm_enabled():
         x2 = x.reshape(-1, x.shape[-1])
         res2 = residual.reshape(-1, residual.shape[-1]) if residual is not None else None
-        return _forward_gemm(x2, w, res2).view(*x.shape[:-1], w.shape[0])
+        return _forward_gemm(x2, w, res2, live).view(*x.shape[:-1], w.shape[0])
     y = F.linear(x, w, b)
     return y if residual is None else y + residual
 
@@ -557,12 +581,12 @@ def _row_grad_target(weight: torch.Tensor, r0: int, r1: int, beside: bool = Fals
     return weight._flat_grad[r0:r1], False
 
 
-def _norm_backward(dy, dy2, x2, weight, rstd, residual_grad, need_dx: bool, need_dw: bool, centred: bool):
+def _norm_backward(dy, dy2, x2, weight, rstd, residual_grad, need_dx: bool, need_dw: bool, centred: bool, live=None):
     """``(dx, dw)`` of a norm over ``x2 [rows, H]``; ``dw`` is ``None`` when it went into the engine's flat buffer."""
     dx = torch.empty_like(x2) if need_dx else None
     dw, accumulate, attached = _param_grad_target(weight) if need_dw else (None, False, False)
     if need_dx or need_dw:
-        native().rmsnorm_bwd(dy, dy2, x2, weight, rstd, residual_grad if need_dx else None, dx, dw, accumulate, centred)
+        native().rmsnorm_bwd(dy, dy2, x2, weight, rstd, residual_grad if need_dx else None, dx, dw, accumulate, centred, live)
     return dx, None if attached else dw
 
 
@@ -570,11 +594,11 @@ class _RMSNormPairFn(torch.autograd.Function):
     """Norm of ``x`` handed out twice, for two consumers whose gradients meet in the backward kernel."""
 
     @staticmethod
-    def forward(ctx, x, weight, eps):
+    def forward(ctx, x, weight, eps, live):
         y = torch.empty_like(x)
         rstd = torch.empty(x.shape[0], dtype=torch.float32, device=x.device)
-        native().norm_fwd(x, weight, None, y, rstd, eps, False)
-        ctx.save_for_backward(x, weight, rstd)
+        native().norm_fwd(x, weight, None, y, rstd, eps, False, live)
+        ctx.save_for_backward(x, weight, rstd, live)
         ctx.set_materialize_grads(False)
         return y, y.view_as(y)
 
@@ -582,17 +606,17 @@ class _RMSNormPairFn(torch.autograd.Function):
     def backward(ctx, d1, d2):
         d1, d2 = (d1, d2) if d1 is not None else (d2, None)
         if d1 is None:
-            return None, None, None
-        x, weight, rstd = ctx.saved_tensors
+            return None, None, None, None
+        x, weight, rstd, live = ctx.saved_tensors
         H = x.shape[1]
-        return *_norm_backward(_grad_rows(d1, H), _grad_rows(d2, H), x, weight, rstd, None, ctx.needs_input_grad[0], ctx.needs_input_grad[1], False), None
+        return *_norm_backward(_grad_rows(d1, H), _grad_rows(d2, H), x, weight, rstd, None, ctx.needs_input_grad[0], ctx.needs_input_grad[1], False, live), None, None
 
 
-def rms_norm_pair(x: torch.Tensor, weight: torch.Tensor, eps: float) -> tuple[torch.Tensor, torch.Tensor]:
+def rms_norm_pair(x: torch.Tensor, weight: torch.Tensor, eps: float, live: torch.Tensor | None = None) -> tuple[torch.Tensor, torch.Tensor]:
     """``rms_norm(x)`` twice, for two consumers."""
     if _norm_native(x) and x.dim() == 2 and x.is_contiguous() and torch.is_grad_enabled() and x.requires_grad:
-        return _RMSNormPairFn.apply(x, weight, eps)
-    y = rms_norm(x, weight, eps)
+        return _RMSNormPairFn.apply(x, weight, eps, live)
+    y = rms_norm(x, weight, eps, live=live)
     return y, y
 
 
@@ -601,7 +625,7 @@ class _RMSNormFn(torch.autograd.Function):
     (a residual branch) is added inside the norm's backward kernel instead of a pass of autograd's own."""
 
     @staticmethod
-    def forward(ctx, x, weight, eps, centred, fork):
+    def forward(ctx, x, weight, eps, centred, fork, live):
         H = x.shape[-1]
         x2 = x.reshape(-1, H)
         if x2.stride(-1) != 1 or x2.stride(0) % 8 or x2.data_ptr() % 16:
@@ -610,8 +634,8 @@ class _RMSNormFn(torch.autograd.Function):
         # modified in place afterwards (the rotary kernel does that to normalised q / k heads)
         y = torch.empty(x.shape, dtype=x.dtype, device=x.device)
         rstd = torch.empty(x2.shape[0], dtype=torch.float32, device=x.device)
-        native().norm_fwd(x2, weight, None, y.view(-1, H), rstd, eps, centred)
-        ctx.save_for_backward(x2, weight, rstd)
+        native().norm_fwd(x2, weight, None, y.view(-1, H), rstd, eps, centred, live)
+        ctx.save_for_backward(x2, weight, rstd, live)
         ctx.shape, ctx.centred = x.shape, centred
         ctx.set_materialize_grads(False)
         return (y, x.view_as(x)) if fork else y
@@ -619,31 +643,33 @@ class _RMSNormFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy, dres=None):
         if dy is None:
-            return dres, None, None, None, None
-        x2, weight, rstd = ctx.saved_tensors
+            return dres, None, None, None, None, None
+        x2, weight, rstd, live = ctx.saved_tensors
         H = x2.shape[-1]
-        dx, dw = _norm_backward(_grad_rows(dy, H), None, x2, weight, rstd, _grad_rows(dres, H), ctx.needs_input_grad[0], ctx.needs_input_grad[1], ctx.centred)
-        return (dx.view(ctx.shape) if dx is not None else None), dw, None, None, None
+        dx, dw = _norm_backward(_grad_rows(dy, H), None, x2, weight, rstd, _grad_rows(dres, H), ctx.needs_input_grad[0], ctx.needs_input_grad[1], ctx.centred,
+                                live)
+        return (dx.view(ctx.shape) if dx is not None else None), dw, None, None, None, None
 
 
 def _norm_native(x: torch.Tensor) -> bool:
     return _use_native(x) and x.dtype == torch.bfloat16 and x.shape[-1] <= _RMSNORM_MAX_WIDTH and x.shape[-1] % 8 == 0
 
 
-def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float, centred: bool = False) -> torch.Tensor:
+def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float, centred: bool = False, live: torch.Tensor | None = None) -> torch.Tensor:
     """RMSNorm over the last dim: ``weight * (x / rms(x))`` with fp32 statistics (``centred``: ``(1 + weight)``, applied
     before rounding).  bf16 CUDA rows of up to 32768 elements run on the package's kernels (one row per CTA with the row in
     registers; one row per warp for rows of up to 256)."""
     if _norm_native(x):
-        return _RMSNormFn.apply(x, weight, eps, centred, False)
+        return _RMSNormFn.apply(x, weight, eps, centred, False, live)
     return _rms_norm_ref(x, weight, eps, centred)
 
 
-def rms_norm_fork(x: torch.Tensor, weight: torch.Tensor, eps: float, centred: bool = False) -> tuple[torch.Tensor, torch.Tensor]:
+def rms_norm_fork(x: torch.Tensor, weight: torch.Tensor, eps: float, centred: bool = False,
+                  live: torch.Tensor | None = None) -> tuple[torch.Tensor, torch.Tensor]:
     """``(rms_norm(x), x)`` for a pre-norm block: the second result is the residual branch."""
     if _norm_native(x) and torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad):
-        return _RMSNormFn.apply(x, weight, eps, centred, True)
-    return rms_norm(x, weight, eps, centred), x
+        return _RMSNormFn.apply(x, weight, eps, centred, True, live)
+    return rms_norm(x, weight, eps, centred, live), x
 
 
 class _Eagle3InputFn(torch.autograd.Function):
@@ -651,15 +677,15 @@ class _Eagle3InputFn(torch.autograd.Function):
     strided launches into one [T, 2H] buffer (no separate concat copy)."""
 
     @staticmethod
-    def forward(ctx, embeds, hidden, w_e, w_h, eps):
+    def forward(ctx, embeds, hidden, w_e, w_h, eps, live):
         T, H = hidden.shape
         out = torch.empty((T, 2 * H), dtype=hidden.dtype, device=hidden.device)
         rs_e = torch.empty(T, dtype=torch.float32, device=hidden.device)
         rs_h = torch.empty(T, dtype=torch.float32, device=hidden.device)
         nat = native()
-        nat.rmsnorm_fwd(embeds, w_e, None, out[:, :H], rs_e, eps)
-        nat.rmsnorm_fwd(hidden, w_h, None, out[:, H:], rs_h, eps)
-        ctx.save_for_backward(embeds, hidden, w_e, w_h, rs_e, rs_h)
+        nat.rmsnorm_fwd(embeds, w_e, None, out[:, :H], rs_e, eps, live)
+        nat.rmsnorm_fwd(hidden, w_h, None, out[:, H:], rs_h, eps, live)
+        ctx.save_for_backward(embeds, hidden, w_e, w_h, rs_e, rs_h, live)
         ctx.set_materialize_grads(False)
         # second result: the normalised-hidden half on its own, so that a consumer of just
         # that half (the residual branch) hands its gradient back as [T, H] instead of
@@ -668,23 +694,23 @@ class _Eagle3InputFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dout, dhalf):
-        embeds, hidden, w_e, w_h, rs_e, rs_h = ctx.saved_tensors
+        embeds, hidden, w_e, w_h, rs_e, rs_h, live = ctx.saved_tensors
         T, H = hidden.shape
         if dout is None:
             dout = torch.zeros((T, 2 * H), dtype=hidden.dtype, device=hidden.device)
         dout = _grad_rows(dout, 2 * H)
         need_e, need_h, need_we, need_wh = ctx.needs_input_grad[:4]
-        d_e, dw_e = _norm_backward(dout[:, :H], None, embeds, w_e, rs_e, None, need_e, need_we, False)
-        d_h, dw_h = _norm_backward(dout[:, H:], _grad_rows(dhalf, H), hidden, w_h, rs_h, None, need_h, need_wh, False)
-        return d_e, d_h, dw_e, dw_h, None
+        d_e, dw_e = _norm_backward(dout[:, :H], None, embeds, w_e, rs_e, None, need_e, need_we, False, live)
+        d_h, dw_h = _norm_backward(dout[:, H:], _grad_rows(dhalf, H), hidden, w_h, rs_h, None, need_h, need_wh, False, live)
+        return d_e, d_h, dw_e, dw_h, None, None
 
 
-def eagle3_input_concat(embeds, hidden, w_embed_norm, w_hidden_norm, eps, return_hidden_half: bool = False):
+def eagle3_input_concat(embeds, hidden, w_embed_norm, w_hidden_norm, eps, return_hidden_half: bool = False, live: torch.Tensor | None = None):
     """First-layer input of an EAGLE-3 draft: both halves normalised, concatenated
     (``[T, 2H]``).  With ``return_hidden_half`` also returns the normalised-hidden half
     ``[T, H]`` as a result of its own (a view of the first on CUDA)."""
     if _use_native(hidden):
-        out, half = _Eagle3InputFn.apply(embeds.contiguous(), hidden.contiguous(), w_embed_norm, w_hidden_norm, eps)
+        out, half = _Eagle3InputFn.apply(embeds.contiguous(), hidden.contiguous(), w_embed_norm, w_hidden_norm, eps, live)
     else:
         out = torch.cat([_rms_norm_ref(embeds, w_embed_norm, eps), _rms_norm_ref(hidden, w_hidden_norm, eps)], dim=-1)
         half = out[:, hidden.shape[-1]:]
@@ -694,14 +720,14 @@ def eagle3_input_concat(embeds, hidden, w_embed_norm, w_hidden_norm, eps, return
 # --------------------------------------------------------------------------- swiglu
 class _SwiGLUFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, gate_up):
-        ctx.save_for_backward(gate_up)
-        return native().swiglu_fwd(gate_up)
+    def forward(ctx, gate_up, live):
+        ctx.save_for_backward(gate_up, live)
+        return native().swiglu_fwd(gate_up, live)
 
     @staticmethod
     def backward(ctx, dh):
-        (gate_up,) = ctx.saved_tensors
-        return native().swiglu_bwd(dh.contiguous(), gate_up)
+        gate_up, live = ctx.saved_tensors
+        return native().swiglu_bwd_rows(dh.contiguous(), gate_up, live), None
 
 
 class _GateUpSwiGLUFn(torch.autograd.Function):
@@ -709,21 +735,21 @@ class _GateUpSwiGLUFn(torch.autograd.Function):
     gate | up product (saved for the backward pass) and the activated product."""
 
     @staticmethod
-    def forward(ctx, x2, weight, use):
-        gate_up, h = native().gemm_swiglu(x2, weight, gemm_status(x2.device))
-        ctx.save_for_backward(x2, weight, gate_up)
+    def forward(ctx, x2, weight, use, live):
+        gate_up, h = native().gemm_swiglu(x2, weight, gemm_status(x2.device), live)
+        ctx.save_for_backward(x2, weight, gate_up, live)
         ctx.use = use
         return h
 
     @staticmethod
     def backward(ctx, dh):
-        x2, weight, gate_up = ctx.saved_tensors
-        dgu = native().swiglu_bwd(dh.contiguous(), gate_up)
-        dx, dw = _linear_backward(x2, weight, (None, None), ctx.use, dgu, ctx.needs_input_grad[0], ctx.needs_input_grad[1])
-        return dx, dw, None
+        x2, weight, gate_up, live = ctx.saved_tensors
+        dgu = native().swiglu_bwd_rows(dh.contiguous(), gate_up, live)
+        dx, dw = _linear_backward(x2, weight, (None, None), ctx.use, dgu, ctx.needs_input_grad[0], ctx.needs_input_grad[1], live)
+        return dx, dw, None, None
 
 
-def linear_swiglu(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor | None:
+def linear_swiglu(x: torch.Tensor, weight: torch.Tensor, live: torch.Tensor | None = None) -> torch.Tensor | None:
     """``swiglu(linear(x, weight))`` for a stacked ``[gate; up]`` weight in one launch: the
     activation is formed in the GEMM's epilogue from the accumulator (``SB200_FUSED_SWIGLU=0``
     switches it off).  ``None`` when the operands do not suit the kernel (other dtype or device,
@@ -735,15 +761,15 @@ def linear_swiglu(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor | None:
             or weight.shape[0] % 256 or weight.shape[1] != x2.shape[1]):
         return None
     use = _note_use(weight, None, None) if weight.requires_grad and torch.is_grad_enabled() else None
-    h = _GateUpSwiGLUFn.apply(x2, weight, use)
+    h = _GateUpSwiGLUFn.apply(x2, weight, use, live)
     return h.view(*x.shape[:-1], h.shape[-1])
 
 
-def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
+def swiglu(gate_up: torch.Tensor, live: torch.Tensor | None = None) -> torch.Tensor:
     """``silu(gate) * up`` where ``gate_up = [gate | up]`` along the last dim."""
     if _use_native(gate_up):
         shape = gate_up.shape
-        out = _SwiGLUFn.apply(gate_up.reshape(-1, shape[-1]).contiguous())
+        out = _SwiGLUFn.apply(gate_up.reshape(-1, shape[-1]).contiguous(), live)
         return out.view(*shape[:-1], shape[-1] // 2)
     gate, up = gate_up.chunk(2, dim=-1)
     return F.silu(gate) * up
@@ -763,7 +789,7 @@ def _rope_ref(x, positions, cos_t, sin_t, heads, hd, rot, sign):
     return torch.cat([y.reshape(T, heads * hd), x[:, heads * hd :]], dim=-1)
 
 
-def _unrotate(dq, dk, dv, positions, cos_t, sin_t, heads, hd, rot):
+def _unrotate(dq, dk, dv, positions, cos_t, sin_t, heads, hd, rot, live=None):
     """Gradient of a rotation: the ``[T, .]`` gradients side by side in a fresh buffer (an incoming one may be shared with
     other consumers), the first ``heads`` heads rotated back."""
     parts = [_grad_rows(d, math.prod(d.shape[1:])) if d is not None else None for d in (dq, dk, dv)]
@@ -771,9 +797,9 @@ def _unrotate(dq, dk, dv, positions, cos_t, sin_t, heads, hd, rot):
     nq = parts[0].shape[1] // hd
     rotate_k = heads > nq
     if merge and heads == nq + (parts[1].shape[1] // hd if rotate_k else 0) and positions.is_contiguous():
-        return native().rope_merge(*parts, rotate_k, positions, cos_t, sin_t, hd, rot, -1.0)
+        return native().rope_merge(*parts, rotate_k, positions, cos_t, sin_t, hd, rot, -1.0, live)
     d = parts[0].clone() if dk is None else torch.cat([p for p in parts if p is not None], dim=-1)
-    native().rope_(d, positions, cos_t, sin_t, heads, hd, rot, -1.0)
+    native().rope_(d, positions, cos_t, sin_t, heads, hd, rot, -1.0, live)
     return d
 
 
@@ -810,17 +836,18 @@ class _RopeSplitFn(torch.autograd.Function):
     fresh buffer and un-rotates them on the way, in one pass."""
 
     @staticmethod
-    def forward(ctx, qkv, positions, cos_t, sin_t, heads, hd, rot, nq, nk):
-        ctx.save_for_backward(positions, cos_t, sin_t)
+    def forward(ctx, qkv, positions, cos_t, sin_t, heads, hd, rot, nq, nk, live):
+        ctx.save_for_backward(positions, cos_t, sin_t, live)
         ctx.cfg = (heads, hd, rot)
         qkv = qkv.detach()
-        native().rope_(qkv, positions, cos_t, sin_t, heads, hd, rot, 1.0)
+        native().rope_(qkv, positions, cos_t, sin_t, heads, hd, rot, 1.0, live)
         q, k, v = qkv[:, :nq], qkv[:, nq : nq + nk], qkv[:, nq + nk :]
         return q, k, v
 
     @staticmethod
     def backward(ctx, dq, dk, dv):
-        return _unrotate(dq, dk, dv, *ctx.saved_tensors, *ctx.cfg), None, None, None, None, None, None, None, None
+        *tables, live = ctx.saved_tensors
+        return _unrotate(dq, dk, dv, *tables, *ctx.cfg, live), None, None, None, None, None, None, None, None, None
 
 
 # --------------------------------------------------------------------------- per-head norms and rotation
@@ -838,11 +865,11 @@ class _NormRopeHeadsFn(torch.autograd.Function):
     """Head norms and rotation of a projection ``[a heads | b heads | plain heads]``; see ``norm_rope_heads``."""
 
     @staticmethod
-    def forward(ctx, src, w_a, w_b, positions, cos_t, sin_t, eps, heads, hd, rot, split, repeated):
+    def forward(ctx, src, w_a, w_b, positions, cos_t, sin_t, eps, heads, hd, rot, split, repeated, live):
         na, nb, nv = heads
         src = src.detach()
-        out, rstd = native().heads_fwd(src, w_a, na, w_b, nb, eps, positions, cos_t, sin_t, hd, rot, repeated)
-        ctx.save_for_backward(src, w_a, w_b, rstd, positions, cos_t, sin_t)
+        out, rstd = native().heads_fwd(src, w_a, na, w_b, nb, eps, positions, cos_t, sin_t, hd, rot, repeated, live)
+        ctx.save_for_backward(src, w_a, w_b, rstd, positions, cos_t, sin_t, live)
         ctx.cfg = (heads, hd, rot, split, repeated)
         ctx.set_materialize_grads(False)
         blocks = [out[:, : na * hd], out[:, na * hd :], src[:, (na + nb) * hd : (na + nb + nv) * hd]]
@@ -854,7 +881,7 @@ class _NormRopeHeadsFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, *grads):
-        src, w_a, w_b, rstd, positions, cos_t, sin_t = ctx.saved_tensors
+        src, w_a, w_b, rstd, positions, cos_t, sin_t, live = ctx.saved_tensors
         (na, nb, nv), hd, rot, split, repeated = ctx.cfg
         it = iter(grads)
         rows = []  # gradients of rows below and from the split on, for each of the three blocks
@@ -864,12 +891,12 @@ class _NormRopeHeadsFn(torch.autograd.Function):
                 rows.append(_grad_rows(g, n * hd) if g is not None and g.shape[0] else None)
         dw_a, acc_a, flat_a = _param_grad_target(w_a) if ctx.needs_input_grad[1] else (None, False, False)
         dw_b, acc_b, flat_b = _param_grad_target(w_b) if nb and ctx.needs_input_grad[2] else (None, False, False)
-        d = native().heads_bwd(rows, src.shape[0] if split is None else split, src, rstd, w_a, na, w_b, nb, nv, dw_a, acc_a, dw_b, acc_b, positions, cos_t, sin_t, hd, rot, repeated)
-        return d, None if flat_a else dw_a, None if flat_b else dw_b, None, None, None, None, None, None, None, None, None
+        d = native().heads_bwd(rows, src.shape[0] if split is None else split, src, rstd, w_a, na, w_b, nb, nv, dw_a, acc_a, dw_b, acc_b, positions, cos_t, sin_t, hd, rot, repeated, live)
+        return d, None if flat_a else dw_a, None if flat_b else dw_b, None, None, None, None, None, None, None, None, None, None
 
 
 def norm_rope_heads(src: torch.Tensor, w_a, w_b, eps: float, positions, cos_t, sin_t, heads: tuple[int, int, int], hd: int, rot: int,
-                    split: int | None = None, repeated: bool = False):
+                    split: int | None = None, repeated: bool = False, live: torch.Tensor | None = None):
     """Per-head RMSNorm (weights ``w_a``, ``w_b``) and rotary embedding of the first ``heads[0]`` and next ``heads[1]`` heads of
     a projection ``[T, sum(heads) * hd]``; the last ``heads[2]`` heads pass through.  Returns a ``[T, n, hd]`` tensor for every
     block that has heads, or with ``split`` two (rows below it, rows from it on) for every block but the queries, the first of
@@ -883,7 +910,7 @@ def norm_rope_heads(src: torch.Tensor, w_a, w_b, eps: float, positions, cos_t, s
         src, repeated = repeat_rows(src, positions.shape[0]), False
     if (_use_native(src) and src.dtype == torch.bfloat16 and hd in (64, 128, 256) and rot % 16 == 0 and rot <= hd and src.stride(-1) == 1
             and src.stride(0) % 8 == 0 and src.data_ptr() % 16 == 0 and positions.is_contiguous() and all(w is None or w.dtype == src.dtype for w in (w_a, w_b))):
-        return _NormRopeHeadsFn.apply(src, w_a, w_b, positions, cos_t, sin_t, eps, heads, hd, rot, split, repeated)
+        return _NormRopeHeadsFn.apply(src, w_a, w_b, positions, cos_t, sin_t, eps, heads, hd, rot, split, repeated, live)
     if repeated:
         src = repeat_rows(src, positions.shape[0])
     T, blocks, col = src.shape[0], [], 0
@@ -894,6 +921,94 @@ def norm_rope_heads(src: torch.Tensor, w_a, w_b, eps: float, positions, cos_t, s
             x = rope_(rms_norm(x, w, eps).reshape(T, n * hd), positions, cos_t, sin_t, n, hd, rot).view(T, n, hd)
         blocks.append(x)
     return _head_blocks(blocks, split)
+
+
+# --------------------------------------------------------------------------- rows that a step needs
+class StepRows(NamedTuple):
+    """Rows of a packed batch that a training-time-test step needs, and what its passes read of them (``step_rows``).
+
+    A tensor "of the rows" has one row per listed row of the batch and as many rows in all as the batch, of which the first
+    ``live`` are in use: shapes do not depend on the mask, and the count stays on the device."""
+
+    index: torch.Tensor  # int64 [T]: the batch's row
+    inverse: torch.Tensor  # int32 [T]: where a row of the batch is listed, -1: nowhere
+    live: torch.Tensor  # int32 [1]
+    target_index: torch.Tensor  # the same for the verifier's rows
+    target_live: torch.Tensor
+    ids: torch.Tensor  # int64 [passes, T], shifted by the pass
+    positions: torch.Tensor
+    mask: torch.Tensor  # bool [passes, T]
+    prev_correct: torch.Tensor  # bool [T]
+    target_row: torch.Tensor  # int32 [passes, T]: the verifier's listed row to compare with, -1: none
+    intervals: list  # of (lo, hi)
+    extra: list  # per pass: None, then int32 [T, pass]
+
+
+def step_rows(mask: torch.Tensor, ids: torch.Tensor, positions: torch.Tensor, intervals: list, passes: int) -> StepRows:
+    """Which rows of a packed batch the passes of a training-time-test step need, the batch in their order.
+
+    Pass ``s`` compares row ``t`` with the verifier's row ``t + s`` where ``mask[t + s]`` is set, and follows the rows that
+    were right in every pass from where ``mask[t]`` is.  A later pass sees a row's own keys of the passes before and nothing
+    else of them, so a row that no comparison reads serves as context keys in pass 0 only.  ``mask`` bool / uint8 ``[T]``,
+    ``intervals``: up to two key intervals ``(lo, hi)`` of the rows.  Rows are listed in ascending order; the count is a
+    multiple of 256 or all of them (on the CPU exact), filled up with rows that nobody asked for."""
+    T = ids.shape[0]
+    if _use_native(ids):
+        both = [lo._base if lo._base is not None and lo._base is hi._base and lo._base.shape == (2, T) else torch.stack([lo, hi]) for lo, hi in intervals]
+        index, inverse, count, ids, positions, mask, prev, target_row, spans, extra = native().step_rows(mask.contiguous(), ids, positions, both, passes)
+        offsets = [T * s * (s - 1) // 2 for s in range(passes)]
+        extra = [None] + [extra.view(-1)[offsets[s] : offsets[s] + T * s].view(T, s) for s in range(1, passes)]
+        return StepRows(index[0], inverse[0], count[:1], index[1], count[1:], ids, positions, mask, prev, target_row, [(s[0], s[1]) for s in spans], extra)
+    m = torch.cat([mask.bool(), torch.zeros(passes, dtype=torch.bool)])
+    lists = []
+    for wanted in (torch.stack([m[s : s + T] for s in range(passes)]).any(0),
+                   torch.stack([torch.cat([torch.zeros(s, dtype=torch.bool), m[: T - s]]) for s in range(passes) if s < T]).any(0)):
+        at = wanted.nonzero().view(-1)
+        inverse = torch.full((T,), -1, dtype=torch.int32)
+        inverse[at] = torch.arange(at.numel(), dtype=torch.int32)
+        lists.append((torch.cat([at, at.new_zeros(T - at.numel())]), inverse, torch.tensor([at.numel()], dtype=torch.int32)))
+    (index, inverse, live), (target_index, target_inverse, target_live) = lists
+    on = torch.arange(T) < live
+    u = index + torch.arange(passes)[:, None]
+    there = on & (u < T)
+    u = u.clamp(max=T - 1)
+    zero = torch.zeros((), dtype=torch.long)
+    extra = [None] + [torch.where(on[:, None], torch.arange(s, dtype=torch.int32) * T + torch.arange(T, dtype=torch.int32)[:, None], -1) for s in range(1, passes)]
+    return StepRows(index, inverse, live, target_index, target_live, torch.where(there, ids[u], zero),
+                    torch.where(on, positions[index] + torch.arange(passes)[:, None], zero), there & m[u], on & m[index],
+                    torch.where(there, target_inverse[u], -1), [tuple(torch.where(on, v[index], 0) for v in pair) for pair in intervals], extra)
+
+
+class _TakeRowsFn(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, index, inverse, live, *xs):
+        ctx.save_for_backward(inverse)
+        ctx.set_materialize_grads(False)
+        return tuple(native().take_rows(xs, index, live))
+
+    @staticmethod
+    def backward(ctx, *ds):
+        (inverse,) = ctx.saved_tensors
+        given = [i for i, d in enumerate(ds) if d is not None and ctx.needs_input_grad[3 + i]]
+        grads = iter(native().put_rows([_grad_rows(ds[i], ds[i].shape[1]) for i in given], inverse)) if given else None
+        return None, None, None, *(next(grads) if i in given else None for i in range(len(ds)))
+
+
+def take_rows(index: torch.Tensor, inverse: torch.Tensor, live: torch.Tensor, *xs: torch.Tensor) -> tuple[torch.Tensor, ...]:
+    """Rows ``index`` of one or two matrices ``[T, W]``, as ``step_rows`` lists them; the rows from ``live`` on are not written
+    (zero on the CPU).  The gradient is a row copy, zero where a row was not taken."""
+    if _use_native(index):
+        return _TakeRowsFn.apply(index, inverse, live, *(_grad_rows(x, x.shape[1]) for x in xs))
+    return tuple(_without_unused(x[index], live) for x in xs)
+
+
+def rms_norm_taken(x: torch.Tensor, weight: torch.Tensor, eps: float, index: torch.Tensor, live: torch.Tensor) -> torch.Tensor:
+    """``rms_norm`` of the rows ``index`` of ``x``, where nothing is differentiated."""
+    if _norm_native(x):
+        y = torch.empty((index.shape[0], x.shape[1]), dtype=x.dtype, device=x.device)
+        native().norm_fwd(_grad_rows(x, x.shape[1]), weight, index, y, None, eps, False, live)
+        return y
+    return rms_norm(_without_unused(x[index], live), weight, eps)
 
 
 # --------------------------------------------------------------------------- repeated rows, embedding
@@ -1016,13 +1131,13 @@ def gated(out: torch.Tensor, gate: torch.Tensor) -> torch.Tensor:
     return _GatedFn.apply(out.contiguous(), gate)
 
 
-def rope_split(qkv, positions, cos_t, sin_t, heads: int, hd: int, rot: int, nq: int, nk: int):
+def rope_split(qkv, positions, cos_t, sin_t, heads: int, hd: int, rot: int, nq: int, nk: int, live: torch.Tensor | None = None):
     """``rope_`` on the first ``heads`` heads of ``qkv`` ([T, nq + nk + nv]) followed by
     the split into ``(q [T, nq], k [T, nk], v [T, rest])``.  On CUDA the buffer is
     rotated in place and the results are views of it: the caller must own ``qkv``
     (a fresh projection output) and must not modify the views in place."""
     if _use_native(qkv) and qkv.requires_grad and torch.is_grad_enabled():
-        return _RopeSplitFn.apply(qkv, positions, cos_t, sin_t, heads, hd, rot, nq, nk)
+        return _RopeSplitFn.apply(qkv, positions, cos_t, sin_t, heads, hd, rot, nq, nk, live)
     out = rope_(qkv, positions, cos_t, sin_t, heads, hd, rot)
     return out[:, :nq], out[:, nq : nq + nk], out[:, nq + nk :]
 
@@ -1095,11 +1210,15 @@ class _LmHeadLossFn(torch.autograd.Function):
 FUSED_HEAD_OPS = ("kl_div", "ce")
 
 
-def lm_head_loss_ok(op: str, hidden: torch.Tensor, weight: torch.Tensor, targets: torch.Tensor) -> bool:
-    """Whether the fused head of ``lm_head_loss_raw`` applies and is switched on."""
+def fused_head_enabled() -> bool:
     import os
 
-    return (op in FUSED_HEAD_OPS and os.environ.get("SB200_FUSED_HEAD", "0") == "1" and own_gemm_enabled()
+    return os.environ.get("SB200_FUSED_HEAD", "0") == "1"
+
+
+def lm_head_loss_ok(op: str, hidden: torch.Tensor, weight: torch.Tensor, targets: torch.Tensor) -> bool:
+    """Whether the fused head of ``lm_head_loss_raw`` applies and is switched on."""
+    return (op in FUSED_HEAD_OPS and fused_head_enabled() and own_gemm_enabled()
             and _gemm_operand_ok(hidden) and _gemm_operand_ok(weight) and _gemm_operand_ok(targets)
             and weight.shape[0] % 8 == 0 and hidden.shape[0] > 128)
 
@@ -1140,10 +1259,10 @@ class _StepLossFn(torch.autograd.Function):
     fourteen launches more in each pass, on steps whose kernels take 2 us."""
 
     @staticmethod
-    def forward(ctx, logits, targets, earlier, op, shift, rows, mask, prev, decay, eps):
-        row_loss, stats, pred, tgt = native().loss_fwd_either(op, logits, targets, mask, prev, shift, rows)
-        out, weight, total = native().step_tail(row_loss, pred, tgt, mask, prev, decay, eps, earlier)
-        ctx.save_for_backward(logits, targets, stats, weight)
+    def forward(ctx, logits, targets, earlier, op, shift, rows, mask, prev, decay, eps, target_row, live):
+        row_loss, stats, pred, tgt = native().loss_fwd_either(op, logits, targets, mask, prev, shift, rows, target_row)
+        out, weight, total = native().step_tail(row_loss, pred, tgt, mask, prev, decay, eps, earlier, target_row)
+        ctx.save_for_backward(logits, targets, stats, weight, target_row, live)
         ctx.cfg = (op, shift, rows)
         ctx.mark_non_differentiable(out)
         ctx.set_materialize_grads(False)
@@ -1152,19 +1271,29 @@ class _StepLossFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dtotal, _dout):
         if dtotal is None:
-            return (None,) * 10
-        logits, targets, stats, weight = ctx.saved_tensors
+            return (None,) * 12
+        logits, targets, stats, weight, target_row, live = ctx.saved_tensors
         op, shift, rows = ctx.cfg
-        d = native().loss_bwd_scaled(op, logits, targets, weight, dtotal.float(), stats, shift, rows)
-        return d, None, dtotal if ctx.needs_input_grad[2] else None, None, None, None, None, None, None, None
+        d = native().loss_bwd_scaled(op, logits, targets, weight, dtotal.float(), stats, shift, rows, target_row, live)
+        return d, None, dtotal if ctx.needs_input_grad[2] else None, None, None, None, None, None, None, None, None, None
 
 
-def ttt_step_loss(op: str, logits, targets, earlier, shift: int, rows: int, mask, prev_correct, decay: float, eps: float):
+def ttt_step_loss(op: str, logits, targets, earlier, shift: int, rows: int, mask, prev_correct, decay: float, eps: float, target_row=None, live=None):
     """``fused_row_loss_raw`` over the rows marked in ``mask`` or ``prev_correct`` followed by ``ttt_step_tail`` (CUDA, bf16
     logits).  Returns ``(earlier + loss, out)`` with ``out`` = loss, correct, total, cond_total, 1; ``earlier``: the loss of
-    the passes before or ``None``; the loss itself is differentiable through the first result."""
+    the passes before or ``None``; the loss itself is differentiable through the first result.  ``target_row`` (int32
+    ``[rows]``): the row of ``targets`` to compare with in place of ``shift``, -1 for none (``step_rows``)."""
+    if not _use_native(logits):
+        there = torch.ones(rows, dtype=torch.bool) if target_row is None else target_row >= 0
+        mask, was = mask[:rows].bool() & there, prev_correct[:rows] & there
+        tg = targets[shift : shift + rows] if target_row is None else targets[target_row.clamp(min=0).long()]
+        row_loss, pred, tgt = fused_row_loss(op, logits[:rows], tg, active=mask | was)
+        out = ttt_step_tail(row_loss, pred, tgt, mask, was, decay, eps)
+        prev_correct[:rows] = torch.where(there, was, prev_correct[:rows])
+        total = out[0] if earlier is None else earlier + out[0]
+        return total, torch.cat([out.detach(), out.new_ones(1)])
     logits, targets = (t if t.stride(-1) == 1 else t.contiguous() for t in (logits, targets))
-    return _StepLossFn.apply(logits, targets, earlier, LOSS_OPS[op], shift, rows, mask, prev_correct, float(decay), float(eps))
+    return _StepLossFn.apply(logits, targets, earlier, LOSS_OPS[op], shift, rows, mask, prev_correct, float(decay), float(eps), target_row, live)
 
 
 def ttt_step_tail(row_loss, pred_ids, target_ids, mask, prev_correct, decay: float, eps: float):

@@ -11,7 +11,7 @@
 namespace sb200 {
 int rmsnorm_bwd_partial_rows(int rows, int H, bool with_dx);
 void launch_rmsnorm_fwd(const void*, const void*, const int64_t*, void*, float*, int, int, int64_t,
-                        int64_t, float, int64_t, int, cudaStream_t);
+                        int64_t, float, int64_t, int, const int*, cudaStream_t);
 struct BoundsRecord {
   int site;
   long long index;
@@ -20,24 +20,29 @@ struct BoundsRecord {
 int read_bounds_norm(BoundsRecord*);
 int read_bounds_ep(BoundsRecord*);
 void launch_rmsnorm_bwd(const void*, int64_t, const void*, int64_t, const void*, int64_t, const void*, const float*, const void*, int64_t, void*, int64_t,
-                        float*, void*, int, int, int, int, cudaStream_t);
+                        float*, void*, int, int, int, int, const int*, cudaStream_t);
 void launch_heads_fwd(const void*, int64_t, const void* const*, const int*, void*, float*, int, int, float, const int64_t*, const float*, const float*, int64_t,
-                      int, int, cudaStream_t);
+                      int, int, const int*, cudaStream_t);
 int heads_bwd_groups(int, int);
 int64_t repeated_part_floats(int, int, int);
 void launch_heads_bwd(const void* const*, const int64_t*, const int*, const void*, int64_t, const void* const*, const float*, float* const*, void* const*,
-                      const int*, const int*, void*, int64_t, int, int, float*, const int64_t*, const float*, const float*, int64_t, int, int, cudaStream_t);
+                      const int*, const int*, void*, int64_t, int, int, float*, const int64_t*, const float*, const float*, int64_t, int, int, const int*,
+                      cudaStream_t);
 void launch_repeated_rows_sum(const void*, int64_t, int, int, float*, void*, int64_t, cudaStream_t);
 void launch_document_interval(const int64_t*, int, int, int*, int*, cudaStream_t);
 void launch_compact(const bool*, int, int64_t*, int*, cudaStream_t);
 void launch_cod_step(const int64_t*, const int64_t*, int, const bool*, int, int, int, unsigned char*, int64_t*, int64_t*, int64_t*, int64_t*, int*, cudaStream_t);
 void launch_peagle_spec(const int64_t*, const int64_t*, const bool*, const int64_t*, const int*, int, int, int, int, int*, int*, int*, int*, cudaStream_t);
+void launch_step_rows(const uint8_t*, const int64_t*, const int64_t*, const int* const*, int, int, int64_t*, int*, int*, int64_t*, int64_t*, uint8_t*, uint8_t*,
+                      int*, int* const*, int*, cudaStream_t);
+void launch_take_rows(int, const void* const*, const int64_t*, const int*, void* const*, const int64_t*, const int*, int, cudaStream_t);
+void launch_put_rows(int, const void* const*, const int64_t*, const int*, void* const*, const int*, int, cudaStream_t);
 int embedding_bwd_partial_rows(int);
 void launch_embedding_bwd(const int64_t*, const int64_t*, const void*, int64_t, int, int, int64_t, int64_t, void*, int, float*, cudaStream_t);
 void launch_swiglu_fwd(const void*, void*, int64_t, int, const int*, cudaStream_t);
 void launch_swiglu_bwd(const void*, const void*, void*, int64_t, int, const int*, cudaStream_t);
 void launch_rope_merge(const void* const*, const int64_t*, const int*, const int*, void*, int64_t, const int64_t*, const float*, const float*, int64_t, int, int,
-                       int, float, cudaStream_t);
+                       int, float, const int*, cudaStream_t);
 void launch_gate_mul_fwd(const void*, const void*, void*, int, int, int, int64_t, int, cudaStream_t);
 void launch_gate_mul_bwd(const void*, const void*, const void*, void*, void*, int, int, int, int64_t, int, int64_t, cudaStream_t);
 int moe_plan_blocks(int);
@@ -49,17 +54,17 @@ void launch_moe_combine_bwd(const void*, const void*, const int*, const int*, co
                             cudaStream_t);
 int launch_gemm_grouped_swiglu(const void*, const void*, void*, void*, int, int, int, int64_t, int64_t, const int*, const int*, int, int*, cudaStream_t);
 void launch_rope(void*, const int64_t*, const float*, const float*, int64_t, int, int, int, int64_t,
-                 int64_t, float, cudaStream_t);
+                 int64_t, float, const int*, cudaStream_t);
 int launch_loss_fwd(int, const void*, const void*, const uint8_t*, const uint8_t*, const int64_t*, float*, float*, int*,
-                    int*, int, int, int64_t, int64_t, int, cudaStream_t);
+                    int*, int, int, int64_t, int64_t, int, const int*, cudaStream_t);
 int launch_loss_bwd(int, const void*, const void*, const float*, const float*, const float*, void*, int, int, int,
-                    int64_t, int64_t, int64_t, int, cudaStream_t);
+                    int64_t, int64_t, int64_t, int, const int*, const int*, cudaStream_t);
 int64_t launch_count();
 int launch_gemm_tn_tcgen05(const void*, const void*, void*, const void*, int, int, int, int64_t, int64_t, int64_t, int64_t, int,
-                           int*, int, cudaStream_t);
+                           int*, int, const int*, cudaStream_t);
 int launch_gemm_tcgen05(const void*, const void*, void*, const void*, int, int, int, int64_t, int64_t, int64_t, int64_t, int, int, int,
-                        int*, int, cudaStream_t);
-int launch_gemm_parts(int, const void* const*, const void* const*, const int*, const int64_t*, const int64_t*, void*, int, int, int64_t, int, int*, cudaStream_t);
+                        int*, int, const int*, cudaStream_t);
+int launch_gemm_parts(int, const void* const*, const void* const*, const int*, const int64_t*, const int64_t*, const int* const*, void*, int, int, int64_t, int, int*, cudaStream_t);
 int launch_gemm_grouped_parts(int, const void* const*, const void* const*, const int*, const int64_t*, const int64_t*, const int* const*, void*, int, int, int,
                               const int*, int, int*, cudaStream_t);
 int launch_gemm_stack(const void*, const void*, void*, const void*, int, int, int, int, int, int, float, float, int, int*, cudaStream_t);
@@ -81,14 +86,15 @@ int fused_optim_ctl_words();
 int fused_optim_num_partials();
 int launch_fused_sharded_adamw(int, int, int64_t, const void* const*, void* const*, void* const*, const void*, void*, float*, float*,
                                float*, float*, float*, const float*, int*, uint32_t, cudaStream_t);
-int launch_gemm_swiglu(const void*, const void*, void*, void*, int, int, int, int64_t, int64_t, int64_t, int64_t, int*, cudaStream_t);
+int launch_gemm_swiglu(const void*, const void*, void*, void*, int, int, int, int64_t, int64_t, int64_t, int64_t, int*, const int*, cudaStream_t);
 int launch_gemm_scatter(const void*, const void*, void* const*, int, int, int, int, int, int64_t, int64_t, int*, cudaStream_t);
 int tp_allreduce_ctl_words();
 int launch_tp_reduce_broadcast(int, int, int, int, const void*, void* const*, void*, const void*, void* const*, int, int*, uint32_t, cudaStream_t);
 int hs_ring_ctl_words_per_slot();
 int launch_hs_push(const void*, int64_t, void*, uint32_t*, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t*, int*, cudaStream_t);
 int launch_hs_pop(void*, int64_t, const void*, uint32_t*, uint32_t, uint32_t, uint32_t*, int*, cudaStream_t);
-void launch_step_tail(const float*, const int*, const int*, const uint8_t*, uint8_t*, int, float, float, float*, float*, const float*, float*, cudaStream_t);
+void launch_step_tail(const float*, const int*, const int*, const uint8_t*, uint8_t*, int, float, float, float*, float*, const float*, float*, const int*,
+                      cudaStream_t);
 void launch_sumsq(const void*, int, int64_t, float*, float*, int, cudaStream_t);
 void launch_set_hyper(float*, const float*, cudaStream_t);
 void launch_adamw(float*, float*, float*, const void*, int, void*, int64_t, const float*,
@@ -113,8 +119,20 @@ void check_rows(const Tensor& t, const char* name) {
               " rows must be 16-byte aligned");
 }
 
+// rows_used (optional int32[1] on the device): rows past it are left alone.
+const int* used_rows(const c10::optional<Tensor>& rows_used) {
+  if (!rows_used.has_value()) return nullptr;
+  TORCH_CHECK(rows_used->is_cuda() && rows_used->scalar_type() == at::kInt && rows_used->numel() >= 1);
+  return rows_used->data_ptr<int>();
+}
+const uint8_t* row_flags(const c10::optional<Tensor>& t, int64_t rows) {
+  if (!t.has_value()) return nullptr;
+  TORCH_CHECK((t->scalar_type() == at::kBool || t->scalar_type() == at::kByte) && t->is_contiguous() && t->numel() >= rows, "bool / uint8 row flags expected");
+  return reinterpret_cast<const uint8_t*>(t->data_ptr());
+}
+
 void norm_fwd(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& row_index, Tensor y,
-              c10::optional<Tensor> rstd, double eps, bool centred) {
+              c10::optional<Tensor> rstd, double eps, bool centred, const c10::optional<Tensor>& live) {
   check_rows(x, "x");
   check_rows(y, "y");
   const int H = (int)y.size(1);
@@ -139,15 +157,16 @@ void norm_fwd(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& row
   }
   c10::cuda::CUDAGuard guard(x.device());
   sb200::launch_rmsnorm_fwd(x.data_ptr(), w.data_ptr(), idx, y.data_ptr(), rs, rows, H, x.stride(0),
-                            y.stride(0), (float)eps, x.size(0), centred ? 1 : 0, cur_stream());
+                            y.stride(0), (float)eps, x.size(0), centred ? 1 : 0, used_rows(live), cur_stream());
 }
-void rmsnorm_fwd(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& row_index, Tensor y, c10::optional<Tensor> rstd, double eps) {
-  norm_fwd(x, w, row_index, y, rstd, eps, false);
+void rmsnorm_fwd(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& row_index, Tensor y, c10::optional<Tensor> rstd, double eps,
+                 const c10::optional<Tensor>& live) {
+  norm_fwd(x, w, row_index, y, rstd, eps, false, live);
 }
 
 // dx = norm gradient of (dy + dy2) (+ add), dw bf16[H] (=, +=); dy2, add, dx, dw optional.  centred: the weight is 1 + w.
 void rmsnorm_bwd(const Tensor& dy, const c10::optional<Tensor>& dy2, const Tensor& x, const Tensor& w, const Tensor& rstd, const c10::optional<Tensor>& add,
-                 c10::optional<Tensor> dx, c10::optional<Tensor> dw, bool accumulate_dw, bool centred) {
+                 c10::optional<Tensor> dx, c10::optional<Tensor> dw, bool accumulate_dw, bool centred, const c10::optional<Tensor>& live) {
   const int64_t rows = x.size(0), H = x.size(1);
   auto rows_of = [&](const c10::optional<Tensor>& t, const char* name, int64_t& stride) -> void* {
     if (!t.has_value()) return nullptr;
@@ -172,7 +191,7 @@ void rmsnorm_bwd(const Tensor& dy, const c10::optional<Tensor>& dy2, const Tenso
     if (rows == 0 && !accumulate_dw) dw->zero_();
   }
   sb200::launch_rmsnorm_bwd(py, sy, py2, sy2, px, sx, w.data_ptr(), rstd.data_ptr<float>(), pa, sa, pd, sd, dw.has_value() ? partial.data_ptr<float>() : nullptr,
-                            dw.has_value() ? dw->data_ptr() : nullptr, (int)rows, (int)H, accumulate_dw ? 1 : 0, centred ? 1 : 0, cur_stream());
+                            dw.has_value() ? dw->data_ptr() : nullptr, (int)rows, (int)H, accumulate_dw ? 1 : 0, centred ? 1 : 0, used_rows(live), cur_stream());
 }
 
 void check_rotation(const Tensor& positions, const Tensor& cos_t, const Tensor& sin_t, int64_t tokens, int64_t hd, int64_t rot) {
@@ -191,7 +210,9 @@ const void* head_weight(const c10::optional<Tensor>& w, int64_t heads, int64_t h
 // -> (rotated normalised heads [T, (na + nb) hd], rstd [T na] then [T nb]); repeated: src holds two rows more than the
 // first tokens, and the tokens after those (positions has them all) read the first of the two
 std::tuple<Tensor, Tensor> heads_fwd(const Tensor& src, const c10::optional<Tensor>& w_a, int64_t na, const c10::optional<Tensor>& w_b, int64_t nb, double eps,
-                                     const Tensor& positions, const Tensor& cos_t, const Tensor& sin_t, int64_t hd, int64_t rot, bool repeated) {
+                                     const Tensor& positions, const Tensor& cos_t, const Tensor& sin_t, int64_t hd, int64_t rot, bool repeated,
+                                     const c10::optional<Tensor>& live) {
+  TORCH_CHECK(!repeated || !live.has_value(), "heads_fwd: a row count and repeated rows exclude each other");
   check_rows(src, "src");
   const int64_t T = repeated ? positions.numel() : src.size(0);
   TORCH_CHECK((hd == 64 || hd == 128 || hd == 256) && na >= 1 && nb >= 0 && src.size(1) >= (na + nb) * hd);
@@ -204,14 +225,16 @@ std::tuple<Tensor, Tensor> heads_fwd(const Tensor& src, const c10::optional<Tens
   const int heads[2] = {(int)na, (int)nb};
   sb200::launch_heads_fwd(src.data_ptr(), src.stride(0), w, heads, out.data_ptr(), rstd.data_ptr<float>(), (int)T,
                           (int)(repeated ? src.size(0) - 2 : src.size(0)), (float)eps,
-                          positions.data_ptr<int64_t>(), cos_t.data_ptr<float>(), sin_t.data_ptr<float>(), cos_t.size(0), (int)hd, (int)rot, cur_stream());
+                          positions.data_ptr<int64_t>(), cos_t.data_ptr<float>(), sin_t.data_ptr<float>(), cos_t.size(0), (int)hd, (int)rot, used_rows(live), cur_stream());
   return {out, rstd};
 }
 
 // d: gradients (or None) of the a, b and plain blocks, each below and from `split` on (a whole when there is a b)
 Tensor heads_bwd(const c10::List<c10::optional<Tensor>>& d, int64_t split, const Tensor& src, const Tensor& rstd, const c10::optional<Tensor>& w_a, int64_t na,
                  const c10::optional<Tensor>& w_b, int64_t nb, int64_t nv, const c10::optional<Tensor>& dw_a, bool acc_a, const c10::optional<Tensor>& dw_b,
-                 bool acc_b, const Tensor& positions, const Tensor& cos_t, const Tensor& sin_t, int64_t hd, int64_t rot, bool repeated) {
+                 bool acc_b, const Tensor& positions, const Tensor& cos_t, const Tensor& sin_t, int64_t hd, int64_t rot, bool repeated,
+                 const c10::optional<Tensor>& live) {
+  TORCH_CHECK(!repeated || !live.has_value(), "heads_bwd: a row count and repeated rows exclude each other");
   check_rows(src, "src");
   const int64_t T = positions.numel(), tokens = repeated ? src.size(0) - 2 : src.size(0);
   TORCH_CHECK(repeated ? (tokens >= 0 && T > tokens && split == tokens && nb > 0) : T == tokens, "heads_bwd: rows and positions do not match");
@@ -254,7 +277,7 @@ Tensor heads_bwd(const c10::List<c10::optional<Tensor>>& d, int64_t split, const
   Tensor sums;
   if (repeated) sums = at::empty({sb200::repeated_part_floats((int)(T - tokens), (int)(na + nb + nv), (int)hd)}, rstd.options());
   sb200::launch_heads_bwd(ptr, stride, splits, src.data_ptr(), src.stride(0), w, rstd.data_ptr<float>(), pp, pw, acc, heads, out.data_ptr(), out.stride(0), (int)tokens, (int)T,
-                          repeated ? sums.data_ptr<float>() : nullptr, positions.data_ptr<int64_t>(), cos_t.data_ptr<float>(), sin_t.data_ptr<float>(), cos_t.size(0), (int)hd, (int)rot, cur_stream());
+                          repeated ? sums.data_ptr<float>() : nullptr, positions.data_ptr<int64_t>(), cos_t.data_ptr<float>(), sin_t.data_ptr<float>(), cos_t.size(0), (int)hd, (int)rot, used_rows(live), cur_stream());
   return out;
 }
 
@@ -323,6 +346,68 @@ std::tuple<Tensor, Tensor, Tensor> peagle_spec(const Tensor& anchor, const Tenso
                             lo.data_ptr<int>(), hi.data_ptr<int>(), extras ? extra.data_ptr<int>() : nullptr, cur_stream());
   return {lo, hi, extra};
 }
+// The rows a training-time-test step of S passes needs (see wanted_rows_kernel): every tensor is fully written.
+// -> (index int64[2, T], inverse int32[2, T], count int32[2]; ids, positions int64[S, T], mask bool[S, T], prev bool[T], target_row int32[S, T],
+//     intervals int32[n, 2, T] as given, extra keys int32[S (S - 1) / 2, T] flat)
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor> step_rows(const Tensor& mask, const Tensor& ids, const Tensor& positions,
+                                                                                                     const std::vector<Tensor>& intervals, int64_t passes) {
+  const int64_t T = ids.numel(), S = passes;
+  TORCH_CHECK(T > 0 && T < (int64_t{1} << 31) / std::max<int64_t>(S * S, 1) && S >= 1 && intervals.size() <= 2 && positions.numel() == T && mask.numel() == T &&
+              mask.is_cuda());
+  c10::cuda::CUDAGuard guard(ids.device());
+  const auto l = ids.options().dtype(at::kLong), n = ids.options().dtype(at::kInt), b = ids.options().dtype(at::kBool);
+  Tensor index = at::empty({2, T}, l), inverse = at::empty({2, T}, n), count = at::empty({2}, n);
+  Tensor ids_out = at::empty({S, T}, l), pos_out = at::empty({S, T}, l), mask_out = at::empty({S, T}, b), prev = at::empty({T}, b);
+  Tensor target_row = at::empty({S, T}, n), spans = at::empty({(int64_t)intervals.size(), 2, T}, n), extra = at::empty({S * (S - 1) / 2, T}, n);
+  const int* in[2] = {nullptr, nullptr};
+  int* out[2] = {nullptr, nullptr};
+  for (size_t k = 0; k < intervals.size(); ++k) {
+    TORCH_CHECK(intervals[k].is_cuda() && intervals[k].scalar_type() == at::kInt && intervals[k].is_contiguous() && intervals[k].dim() == 2 && intervals[k].size(0) == 2 &&
+                intervals[k].size(1) == T, "step_rows: intervals are contiguous int32 [2, T]");
+    in[k] = intervals[k].data_ptr<int>();
+    out[k] = spans.select(0, (int64_t)k).data_ptr<int>();
+  }
+  sb200::launch_step_rows(row_flags(mask, T), long_ptr(ids, "ids"), long_ptr(positions, "positions"), in, (int)T, (int)S, index.data_ptr<int64_t>(),
+                          inverse.data_ptr<int>(), count.data_ptr<int>(), ids_out.data_ptr<int64_t>(), pos_out.data_ptr<int64_t>(),
+                          reinterpret_cast<uint8_t*>(mask_out.data_ptr()), reinterpret_cast<uint8_t*>(prev.data_ptr()), target_row.data_ptr<int>(), out,
+                          extra.data_ptr<int>(), cur_stream());
+  return {index, inverse, count, ids_out, pos_out, mask_out, prev, target_row, spans, extra};
+}
+struct RowCopyArgs {
+  const void* from[2];
+  void* to[2];
+  int64_t stride[2];
+  int W[2];
+  std::vector<Tensor> out;
+};
+RowCopyArgs row_copy_args(const std::vector<Tensor>& x, int64_t rows) {
+  TORCH_CHECK(x.size() == 1 || x.size() == 2, "one or two matrices");
+  RowCopyArgs a{};
+  for (size_t i = 0; i < x.size(); ++i) {
+    check_rows(x[i], "rows");
+    TORCH_CHECK(x[i].size(1) % 8 == 0 && x[i].device() == x[0].device());
+    a.out.push_back(at::empty({rows, x[i].size(1)}, x[i].options()));
+    a.from[i] = x[i].data_ptr();
+    a.to[i] = a.out[i].data_ptr();
+    a.stride[i] = x[i].stride(0);
+    a.W[i] = (int)x[i].size(1);
+  }
+  return a;
+}
+// out[r] = x[index[r]] for r < live, for one or two matrices (index: rows of x, not checked); put_rows is its gradient
+std::vector<Tensor> take_rows(const std::vector<Tensor>& x, const Tensor& index, const c10::optional<Tensor>& live) {
+  c10::cuda::CUDAGuard guard(index.device());
+  RowCopyArgs a = row_copy_args(x, index.numel());
+  sb200::launch_take_rows((int)x.size(), a.from, a.stride, a.W, a.to, long_ptr(index, "index"), used_rows(live), (int)index.numel(), cur_stream());
+  return a.out;
+}
+std::vector<Tensor> put_rows(const std::vector<Tensor>& d, const Tensor& inverse) {
+  TORCH_CHECK(inverse.is_cuda() && inverse.scalar_type() == at::kInt && inverse.is_contiguous());
+  c10::cuda::CUDAGuard guard(inverse.device());
+  RowCopyArgs a = row_copy_args(d, inverse.numel());
+  sb200::launch_put_rows((int)d.size(), a.from, a.stride, a.W, a.to, inverse.data_ptr<int>(), (int)inverse.numel(), cur_stream());
+  return a.out;
+}
 // dw rows of the ids (ascending, `order` their source rows of d) stored or added to
 void embedding_bwd(const Tensor& ids, const Tensor& order, const Tensor& d, int64_t padding, Tensor dw, bool accumulate) {
   check_rows(d, "d");
@@ -334,21 +419,14 @@ void embedding_bwd(const Tensor& ids, const Tensor& order, const Tensor& d, int6
                               dw.data_ptr(), accumulate ? 1 : 0, part.data_ptr<float>(), cur_stream());
 }
 
-// rows_used (optional int32[1] on the device): rows past it are left alone.
-const int* used_rows(const c10::optional<Tensor>& rows_used) {
-  if (!rows_used.has_value()) return nullptr;
-  TORCH_CHECK(rows_used->is_cuda() && rows_used->scalar_type() == at::kInt && rows_used->numel() >= 1);
-  return rows_used->data_ptr<int>();
-}
-
-Tensor swiglu_fwd(const Tensor& gate_up) {
+Tensor swiglu_fwd(const Tensor& gate_up, const c10::optional<Tensor>& rows_used) {
   check_rows(gate_up, "gate_up");
   TORCH_CHECK(gate_up.is_contiguous() && gate_up.size(1) % 16 == 0);
   const int64_t rows = gate_up.size(0);
   const int I = (int)(gate_up.size(1) / 2);
   c10::cuda::CUDAGuard guard(gate_up.device());
   Tensor h = at::empty({rows, I}, gate_up.options());
-  sb200::launch_swiglu_fwd(gate_up.data_ptr(), h.data_ptr(), rows, I, nullptr, cur_stream());
+  sb200::launch_swiglu_fwd(gate_up.data_ptr(), h.data_ptr(), rows, I, used_rows(rows_used), cur_stream());
   return h;
 }
 
@@ -366,7 +444,7 @@ Tensor swiglu_bwd(const Tensor& dh, const Tensor& gate_up) { return swiglu_bwd_r
 
 // [q | k | v] gradients (2-D rows, k and v optional) side by side, rotated back where marked (q always, k with rotate_k).
 Tensor rope_merge(const Tensor& q, const c10::optional<Tensor>& k, const c10::optional<Tensor>& v, bool rotate_k, const Tensor& positions, const Tensor& cos_t,
-                  const Tensor& sin_t, int64_t hd, int64_t rot, double sign) {
+                  const Tensor& sin_t, int64_t hd, int64_t rot, double sign, const c10::optional<Tensor>& live) {
   check_rotation(positions, cos_t, sin_t, q.size(0), hd, rot);
   const Tensor* parts[3] = {&q, k.has_value() ? &*k : nullptr, v.has_value() ? &*v : nullptr};
   const void* src[3] = {nullptr, nullptr, nullptr};
@@ -384,7 +462,7 @@ Tensor rope_merge(const Tensor& q, const c10::optional<Tensor>& k, const c10::op
   c10::cuda::CUDAGuard guard(q.device());
   Tensor out = at::empty({q.size(0), width}, q.options());
   sb200::launch_rope_merge(src, stride, heads, rotate, out.data_ptr(), width, positions.data_ptr<int64_t>(), cos_t.data_ptr<float>(), sin_t.data_ptr<float>(),
-                           cos_t.size(0), (int)q.size(0), (int)hd, (int)rot, (float)sign, cur_stream());
+                           cos_t.size(0), (int)q.size(0), (int)hd, (int)rot, (float)sign, used_rows(live), cur_stream());
   return out;
 }
 
@@ -488,7 +566,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> moe_combine_bwd(const Tensor& dout, c
 
 // x: [tokens, >= heads*hd] view (row stride arbitrary); rotates the first `heads` heads in place.
 void rope_(Tensor x, const Tensor& positions, const Tensor& cos_t, const Tensor& sin_t, int64_t heads,
-           int64_t hd, int64_t rot, double sign) {
+           int64_t hd, int64_t rot, double sign, const c10::optional<Tensor>& live) {
   TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.dim() == 2 && x.stride(1) == 1);
   TORCH_CHECK(x.size(1) >= heads * hd && rot % 2 == 0 && rot <= hd);
   TORCH_CHECK(positions.scalar_type() == at::kLong && positions.is_contiguous() &&
@@ -499,22 +577,26 @@ void rope_(Tensor x, const Tensor& positions, const Tensor& cos_t, const Tensor&
   c10::cuda::CUDAGuard guard(x.device());
   sb200::launch_rope(x.data_ptr(), positions.data_ptr<int64_t>(), cos_t.data_ptr<float>(),
                      sin_t.data_ptr<float>(), x.size(0), (int)heads, (int)hd, (int)rot, x.stride(0),
-                     cos_t.size(0), (float)sign, cur_stream());
+                     cos_t.size(0), (float)sign, used_rows(live), cur_stream());
 }
 
-const uint8_t* row_flags(const c10::optional<Tensor>& t, int64_t rows) {
+
+// int32[rows]: the row of the targets each row is compared with, -1 for none
+const int* row_targets(const c10::optional<Tensor>& t, int64_t rows) {
   if (!t.has_value()) return nullptr;
-  TORCH_CHECK((t->scalar_type() == at::kBool || t->scalar_type() == at::kByte) && t->is_contiguous() && t->numel() >= rows, "bool / uint8 row flags expected");
-  return reinterpret_cast<const uint8_t*>(t->data_ptr());
+  TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kInt && t->is_contiguous() && t->numel() >= rows, "int32 target rows expected");
+  return t->data_ptr<int>();
 }
 
+// target_row: rows of `targets` to compare with, in place of a shift (they are not checked against its size)
 std::tuple<Tensor, Tensor, Tensor, Tensor> loss_fwd_either(int64_t op, const Tensor& logits, const Tensor& targets, const c10::optional<Tensor>& active,
-                                                           const c10::optional<Tensor>& also, int64_t shift, int64_t rows) {
+                                                           const c10::optional<Tensor>& also, int64_t shift, int64_t rows,
+                                                           const c10::optional<Tensor>& target_row) {
   TORCH_CHECK(logits.is_cuda() && targets.is_cuda());
   TORCH_CHECK(logits.scalar_type() == at::kBFloat16 && targets.scalar_type() == at::kBFloat16);
   TORCH_CHECK(logits.dim() == 2 && targets.dim() == 2 && logits.stride(1) == 1 &&
               targets.stride(1) == 1 && logits.size(1) == targets.size(1));
-  TORCH_CHECK(rows >= 0 && rows <= logits.size(0) && rows + shift <= targets.size(0) && shift >= 0);
+  TORCH_CHECK(rows >= 0 && rows <= logits.size(0) && (target_row.has_value() || (rows + shift <= targets.size(0) && shift >= 0)));
   c10::cuda::CUDAGuard guard(logits.device());
   auto fopt = logits.options().dtype(at::kFloat);
   Tensor loss = at::empty({rows}, fopt);
@@ -525,13 +607,13 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> loss_fwd_either(int64_t op, const Ten
                                         loss.data_ptr<float>(), stats.data_ptr<float>(),
                                         am_d.data_ptr<int>(), am_t.data_ptr<int>(), (int)rows,
                                         (int)logits.size(1), logits.stride(0), targets.stride(0),
-                                        (int)shift, cur_stream());
+                                        (int)shift, row_targets(target_row, rows), cur_stream());
   TORCH_CHECK(rc == 0, "loss_fwd: unknown op ", op);
   return {loss, stats, am_d, am_t};
 }
 std::tuple<Tensor, Tensor, Tensor, Tensor> loss_fwd(int64_t op, const Tensor& logits, const Tensor& targets, const c10::optional<Tensor>& active, int64_t shift,
                                                     int64_t rows) {
-  return loss_fwd_either(op, logits, targets, active, c10::nullopt, shift, rows);
+  return loss_fwd_either(op, logits, targets, active, c10::nullopt, shift, rows, c10::nullopt);
 }
 
 // ---- grouped (mixture-of-experts) products ----------------------------------------------------
@@ -613,18 +695,22 @@ void gemm_grouped_wgrad(const Tensor& dy, const Tensor& x, Tensor dw, bool accum
 }
 
 // dw (+)= sum_i dy_i^T . x_i: the weight gradient over several uses of a weight
-void gemm_wgrad_parts(const std::vector<Tensor>& dy, const std::vector<Tensor>& x, Tensor dw, bool accumulate, Tensor status) {
+// live: how many rows of each use count (one int32 per use, an empty tensor: all; an empty list: all of every use)
+void gemm_wgrad_parts_rows(const std::vector<Tensor>& dy, const std::vector<Tensor>& x, Tensor dw, bool accumulate, Tensor status,
+                           const std::vector<Tensor>& live) {
   check_rows(dw, "dw");
   const int64_t M = dw.size(0), N = dw.size(1);
   const size_t n = dy.size();
-  TORCH_CHECK(n >= 1 && n <= 4 && x.size() == n, "gemm_wgrad_parts: one to four uses");
+  TORCH_CHECK(n >= 1 && n <= 4 && x.size() == n && (live.empty() || live.size() == n), "gemm_wgrad_parts: one to four uses");
   const void *a[4], *b[4];
+  const int* rows_of[4];
   int K[4];
   int64_t lda[4], ldb[4];
   for (size_t i = 0; i < n; ++i) {
     check_rows(dy[i], "dy");
     check_rows(x[i], "x");
     TORCH_CHECK(dy[i].size(1) == M && x[i].size(1) == N && x[i].size(0) == dy[i].size(0) && dy[i].size(0) > 0, "gemm_wgrad_parts: shape mismatch");
+    rows_of[i] = live.empty() || live[i].numel() == 0 ? nullptr : used_rows(live[i]);
     a[i] = dy[i].data_ptr();
     b[i] = x[i].data_ptr();
     K[i] = (int)dy[i].size(0);
@@ -633,9 +719,13 @@ void gemm_wgrad_parts(const std::vector<Tensor>& dy, const std::vector<Tensor>& 
   }
   TORCH_CHECK(status.is_cuda() && status.scalar_type() == at::kInt && status.numel() >= 1);
   c10::cuda::CUDAGuard guard(dw.device());
-  const int rc = sb200::launch_gemm_parts((int)n, a, b, K, lda, ldb, dw.data_ptr(), (int)M, (int)N, dw.stride(0), accumulate ? 1 : 0, status.data_ptr<int>(),
+  const int rc = sb200::launch_gemm_parts((int)n, a, b, K, lda, ldb, rows_of, dw.data_ptr(), (int)M, (int)N, dw.stride(0), accumulate ? 1 : 0, status.data_ptr<int>(),
                                           cur_stream());
   TORCH_CHECK(rc == 0, "gemm_wgrad_parts launch failed (", rc, ")");
+}
+
+void gemm_wgrad_parts(const std::vector<Tensor>& dy, const std::vector<Tensor>& x, Tensor dw, bool accumulate, Tensor status) {
+  gemm_wgrad_parts_rows(dy, x, dw, accumulate, status, {});
 }
 
 // lm_head product fused with the row loss: logits = x @ w^T on the tcgen05 kernel whose epilogue also
@@ -693,13 +783,13 @@ std::tuple<Tensor, Tensor> ce_label_fwd(const Tensor& logits, const Tensor& labe
   }
   const int rc = sb200::launch_loss_fwd(3, logits.data_ptr(), nullptr, act, nullptr, labels.data_ptr<int64_t>(), loss.data_ptr<float>(),
                                         stats.data_ptr<float>(), nullptr, nullptr, (int)rows, (int)logits.size(1),
-                                        logits.stride(0), logits.stride(0), 0, cur_stream());
+                                        logits.stride(0), logits.stride(0), 0, nullptr, cur_stream());
   TORCH_CHECK(rc == 0, "ce_label_fwd failed (", rc, ")");
   return {loss, stats};
 }
 
 Tensor loss_bwd_scaled(int64_t op, const Tensor& logits, const Tensor& targets, const Tensor& grad_out, const c10::optional<Tensor>& grad_scale,
-                       const Tensor& stats, int64_t shift, int64_t rows) {
+                       const Tensor& stats, int64_t shift, int64_t rows, const c10::optional<Tensor>& target_row, const c10::optional<Tensor>& live) {
   TORCH_CHECK(!grad_scale.has_value() || (grad_scale->is_cuda() && grad_scale->scalar_type() == at::kFloat && grad_scale->numel() == 1));
   TORCH_CHECK(grad_out.scalar_type() == at::kFloat && grad_out.is_contiguous() &&
               grad_out.numel() == rows);
@@ -710,12 +800,12 @@ Tensor loss_bwd_scaled(int64_t op, const Tensor& logits, const Tensor& targets, 
   const int rc = sb200::launch_loss_bwd(
       (int)op, logits.data_ptr(), targets.data_ptr(), grad_out.data_ptr<float>(),
       grad_scale.has_value() ? grad_scale->data_ptr<float>() : nullptr, stats.data_ptr<float>(), d.data_ptr(), (int)rows, (int)logits.size(0), (int)logits.size(1),
-      logits.stride(0), targets.stride(0), d.stride(0), (int)shift, cur_stream());
+      logits.stride(0), targets.stride(0), d.stride(0), (int)shift, row_targets(target_row, rows), used_rows(live), cur_stream());
   TORCH_CHECK(rc == 0, "loss_bwd: unknown op ", op);
   return d;
 }
 Tensor loss_bwd(int64_t op, const Tensor& logits, const Tensor& targets, const Tensor& grad_out, const Tensor& stats, int64_t shift, int64_t rows) {
-  return loss_bwd_scaled(op, logits, targets, grad_out, c10::nullopt, stats, shift, rows);
+  return loss_bwd_scaled(op, logits, targets, grad_out, c10::nullopt, stats, shift, rows, c10::nullopt, c10::nullopt);
 }
 
 void sumsq(const Tensor& g, Tensor out, bool accumulate) {
@@ -840,7 +930,7 @@ int64_t fused_optim_ctl_words() { return sb200::fused_optim_ctl_words(); }
 // Returns (out fp32[4] = loss, correct, total, cond_total; weight fp32[rows] = d loss / d row_loss).
 // -> (out float[5]: loss, correct, total, cond_total, 1; weight float[rows]; earlier + loss)
 std::tuple<Tensor, Tensor, Tensor> step_tail(const Tensor& row_loss, const Tensor& pred, const Tensor& target, const Tensor& mask, Tensor prev,
-                                             double decay, double eps, const c10::optional<Tensor>& earlier) {
+                                             double decay, double eps, const c10::optional<Tensor>& earlier, const c10::optional<Tensor>& target_row) {
   TORCH_CHECK(!earlier.has_value() || (earlier->is_cuda() && earlier->scalar_type() == at::kFloat && earlier->numel() == 1));
   const int64_t rows = row_loss.numel();
   TORCH_CHECK(row_loss.is_cuda() && row_loss.scalar_type() == at::kFloat && row_loss.is_contiguous());
@@ -854,7 +944,7 @@ std::tuple<Tensor, Tensor, Tensor> step_tail(const Tensor& row_loss, const Tenso
   sb200::launch_step_tail(row_loss.data_ptr<float>(), pred.data_ptr<int>(), target.data_ptr<int>(),
                           static_cast<const uint8_t*>(mask.data_ptr()), static_cast<uint8_t*>(prev.data_ptr()), (int)rows, (float)decay,
                           (float)eps, out.data_ptr<float>(), weight.data_ptr<float>(), earlier.has_value() ? earlier->data_ptr<float>() : nullptr,
-                           total.data_ptr<float>(), cur_stream());
+                           total.data_ptr<float>(), row_targets(target_row, rows), cur_stream());
   return {out, weight, total};
 }
 
@@ -919,7 +1009,7 @@ void fused_sharded_adamw(int64_t world, int64_t rank, int64_t shard, const Tenso
 
 // ---- gated MLP: gate | up product with the activation in the GEMM epilogue ------------------------
 // w: [2 I, K], gate rows first.  Returns (gate_up [M, 2 I], h [M, I] = silu(gate) * up).
-std::tuple<Tensor, Tensor> gemm_swiglu(const Tensor& x, const Tensor& w, Tensor status) {
+std::tuple<Tensor, Tensor> gemm_swiglu(const Tensor& x, const Tensor& w, Tensor status, const c10::optional<Tensor>& live) {
   check_rows(x, "x");
   check_rows(w, "w");
   const int64_t M = x.size(0), K = x.size(1), I = w.size(0) / 2;
@@ -929,7 +1019,7 @@ std::tuple<Tensor, Tensor> gemm_swiglu(const Tensor& x, const Tensor& w, Tensor 
   Tensor gate_up = at::empty({M, 2 * I}, x.options());
   Tensor h = at::empty({M, I}, x.options());
   const int rc = sb200::launch_gemm_swiglu(x.data_ptr(), w.data_ptr(), gate_up.data_ptr(), h.data_ptr(), (int)M, (int)I, (int)K, x.stride(0), w.stride(0),
-                                           2 * I, I, status.data_ptr<int>(), cur_stream());
+                                           2 * I, I, status.data_ptr<int>(), used_rows(live), cur_stream());
   TORCH_CHECK(rc == 0, "gemm_swiglu launch failed (", rc, ")");
   return {gate_up, h};
 }
@@ -1079,7 +1169,7 @@ void ep_pull(const Tensor& src_ptrs, int64_t capacity, const Tensor& src_rank, c
 // `status` (int32[1], device) receives a non-zero code if a bounded wait in the kernel ran out.
 // variant: 0 = choose; see launch_gemm_impl.
 void gemm_tn_variant(const Tensor& a, const Tensor& b, Tensor out, const c10::optional<Tensor>& residual, int64_t epilogue, Tensor status,
-                     int64_t variant) {
+                     int64_t variant, const c10::optional<Tensor>& live) {
   TORCH_CHECK(a.is_cuda() && b.is_cuda() && out.is_cuda() && status.is_cuda());
   TORCH_CHECK(a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16 && out.scalar_type() == at::kBFloat16);
   TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && out.dim() == 2 && a.stride(1) == 1 && b.stride(1) == 1 && out.stride(1) == 1);
@@ -1097,12 +1187,13 @@ void gemm_tn_variant(const Tensor& a, const Tensor& b, Tensor out, const c10::op
   c10::cuda::CUDAGuard guard(a.device());
   const int rc = sb200::launch_gemm_tn_tcgen05(a.data_ptr(), b.data_ptr(), out.data_ptr(), res, (int)a.size(0), (int)b.size(0),
                                                (int)a.size(1), a.stride(0), b.stride(0), out.stride(0), ldr, (int)epilogue,
-                                               status.data_ptr<int>(), (int)variant, cur_stream());
+                                               status.data_ptr<int>(), (int)variant, used_rows(live), cur_stream());
   TORCH_CHECK(rc == 0, "gemm_tn launch failed (", rc, ")");
 }
 
-void gemm_tn(const Tensor& a, const Tensor& b, Tensor out, const c10::optional<Tensor>& residual, int64_t epilogue, Tensor status) {
-  gemm_tn_variant(a, b, out, residual, epilogue, status, 0);
+void gemm_tn(const Tensor& a, const Tensor& b, Tensor out, const c10::optional<Tensor>& residual, int64_t epilogue, Tensor status,
+             const c10::optional<Tensor>& live) {
+  gemm_tn_variant(a, b, out, residual, epilogue, status, 0, live);
 }
 
 // out[M,N] (=, +=) op(a) @ op(b)^T with either operand stored transposed:
@@ -1110,7 +1201,9 @@ void gemm_tn(const Tensor& a, const Tensor& b, Tensor out, const c10::optional<T
 //   b_mn false: b is [N, K];  true: b is [K, N]
 // dgrad of a linear layer: gemm(dy[T,out], w[out,in], dx, b_mn = true);
 // wgrad: gemm(dy[T,out], x[T,in], dw[out,in], a_mn = b_mn = true, epilogue 1 to accumulate).
-void gemm_variant(const Tensor& a, const Tensor& b, Tensor out, int64_t epilogue, bool a_mn, bool b_mn, Tensor status, int64_t variant) {
+// live (device int32): how many rows of the activations count - the rows of a and out, or with both operands transposed the sum's
+void gemm_variant(const Tensor& a, const Tensor& b, Tensor out, int64_t epilogue, bool a_mn, bool b_mn, Tensor status, int64_t variant,
+                  const c10::optional<Tensor>& live) {
   TORCH_CHECK(a.is_cuda() && b.is_cuda() && out.is_cuda() && status.is_cuda());
   TORCH_CHECK(a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16 && out.scalar_type() == at::kBFloat16);
   TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && out.dim() == 2 && a.stride(1) == 1 && b.stride(1) == 1 && out.stride(1) == 1);
@@ -1122,12 +1215,12 @@ void gemm_variant(const Tensor& a, const Tensor& b, Tensor out, int64_t epilogue
   c10::cuda::CUDAGuard guard(a.device());
   const int rc = sb200::launch_gemm_tcgen05(a.data_ptr(), b.data_ptr(), out.data_ptr(), nullptr, (int)M, (int)N, (int)K, a.stride(0),
                                             b.stride(0), out.stride(0), 0, (int)epilogue, a_mn ? 1 : 0, b_mn ? 1 : 0,
-                                            status.data_ptr<int>(), (int)variant, cur_stream());
+                                            status.data_ptr<int>(), (int)variant, used_rows(live), cur_stream());
   TORCH_CHECK(rc == 0, "gemm launch failed (", rc, ")");
 }
 
-void gemm(const Tensor& a, const Tensor& b, Tensor out, int64_t epilogue, bool a_mn, bool b_mn, Tensor status) {
-  gemm_variant(a, b, out, epilogue, a_mn, b_mn, status, 0);
+void gemm(const Tensor& a, const Tensor& b, Tensor out, int64_t epilogue, bool a_mn, bool b_mn, Tensor status, const c10::optional<Tensor>& live) {
+  gemm_variant(a, b, out, epilogue, a_mn, b_mn, status, 0, live);
 }
 
 // Stacks of products: out[z] = alpha op(a[z]) @ op(b[z])^T (+ beta addend[z]), rounded as separate bf16 passes would round.
@@ -1317,17 +1410,27 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> attn_bwd(
 }  // namespace
 
 TORCH_LIBRARY(sb200, m) {
-  m.def("rmsnorm_fwd", &rmsnorm_fwd);
-  m.def("norm_fwd", &norm_fwd);
-  m.def("rmsnorm_bwd", &rmsnorm_bwd);
-  m.def("swiglu_fwd", &swiglu_fwd);
+  // a trailing `live` (int32[1] on the device): how many of the rows are in use
+  m.def("rmsnorm_fwd(Tensor x, Tensor w, Tensor? row_index, Tensor y, Tensor? rstd, float eps, Tensor? live=None) -> ()", &rmsnorm_fwd);
+  m.def("norm_fwd(Tensor x, Tensor w, Tensor? row_index, Tensor y, Tensor? rstd, float eps, bool centred, Tensor? live=None) -> ()", &norm_fwd);
+  m.def("rmsnorm_bwd(Tensor dy, Tensor? dy2, Tensor x, Tensor w, Tensor rstd, Tensor? add, Tensor? dx, Tensor? dw, bool accumulate_dw, bool centred, "
+        "Tensor? live=None) -> ()", &rmsnorm_bwd);
+  m.def("step_rows", &step_rows);
+  m.def("take_rows", &take_rows);
+  m.def("put_rows", &put_rows);
+  m.def("swiglu_fwd(Tensor gate_up, Tensor? rows_used=None) -> Tensor", &swiglu_fwd);
   m.def("swiglu_bwd", &swiglu_bwd);
   m.def("swiglu_bwd_rows", &swiglu_bwd_rows);
-  m.def("heads_fwd", &heads_fwd);
-  m.def("heads_bwd", &heads_bwd);
-  m.def("rope_merge", &rope_merge);
-  m.def("loss_fwd_either", &loss_fwd_either);
-  m.def("loss_bwd_scaled", &loss_bwd_scaled);
+  m.def("heads_fwd(Tensor src, Tensor? w_a, int na, Tensor? w_b, int nb, float eps, Tensor positions, Tensor cos, Tensor sin, int hd, int rot, bool repeated, "
+        "Tensor? live=None) -> (Tensor, Tensor)", &heads_fwd);
+  m.def("heads_bwd(Tensor?[] d, int split, Tensor src, Tensor rstd, Tensor? w_a, int na, Tensor? w_b, int nb, int nv, Tensor? dw_a, bool acc_a, Tensor? dw_b, "
+        "bool acc_b, Tensor positions, Tensor cos, Tensor sin, int hd, int rot, bool repeated, Tensor? live=None) -> Tensor", &heads_bwd);
+  m.def("rope_merge(Tensor q, Tensor? k, Tensor? v, bool rotate_k, Tensor positions, Tensor cos, Tensor sin, int hd, int rot, float sign, Tensor? live=None) -> "
+        "Tensor", &rope_merge);
+  m.def("loss_fwd_either(int op, Tensor logits, Tensor targets, Tensor? active, Tensor? also, int shift, int rows, Tensor? target_row=None) -> "
+        "(Tensor, Tensor, Tensor, Tensor)", &loss_fwd_either);
+  m.def("loss_bwd_scaled(int op, Tensor logits, Tensor targets, Tensor grad_out, Tensor? grad_scale, Tensor stats, int shift, int rows, "
+        "Tensor? target_row=None, Tensor? live=None) -> Tensor", &loss_bwd_scaled);
   m.def("repeated_rows_sum", &repeated_rows_sum);
   m.def("document_interval", &document_interval);
   m.def("compact_rows", &compact_rows);
@@ -1342,7 +1445,7 @@ TORCH_LIBRARY(sb200, m) {
   m.def("moe_combine", &moe_combine);
   m.def("moe_combine_bwd", &moe_combine_bwd);
   m.def("gemm_grouped_swiglu", &gemm_grouped_swiglu);
-  m.def("rope_", &rope_);
+  m.def("rope_(Tensor x, Tensor positions, Tensor cos, Tensor sin, int heads, int hd, int rot, float sign, Tensor? live=None) -> ()", &rope_);
   m.def("loss_fwd", &loss_fwd);
   m.def("loss_bwd", &loss_bwd);
   m.def("ce_label_fwd", &ce_label_fwd);
@@ -1361,11 +1464,12 @@ TORCH_LIBRARY(sb200, m) {
   m.def("peer_tensor", &peer_tensor);
   m.def("fused_optim_ctl_words", &fused_optim_ctl_words);
   m.def("fused_sharded_adamw", &fused_sharded_adamw);
-  m.def("gemm_swiglu", &gemm_swiglu);
+  m.def("gemm_swiglu(Tensor x, Tensor w, Tensor status, Tensor? live=None) -> (Tensor, Tensor)", &gemm_swiglu);
   m.def("gemm_scatter", &gemm_scatter);
   m.def("tp_allreduce_ctl_words", &tp_allreduce_ctl_words);
   m.def("tp_reduce_broadcast", &tp_reduce_broadcast);
-  m.def("step_tail", &step_tail);
+  m.def("step_tail(Tensor row_loss, Tensor pred, Tensor target, Tensor mask, Tensor prev, float decay, float eps, Tensor? earlier, Tensor? target_row=None) -> "
+        "(Tensor, Tensor, Tensor)", &step_tail);
   m.def("checked_build", &checked_build);
   m.def("bounds_report", &bounds_report);
   m.def("ep_push", &ep_push);
@@ -1375,17 +1479,18 @@ TORCH_LIBRARY(sb200, m) {
   m.def("hs_ring_ctl_words", &hs_ring_ctl_words);
   m.def("hs_push", &hs_push);
   m.def("hs_pop", &hs_pop);
-  m.def("gemm_tn", &gemm_tn);
-  m.def("gemm", &gemm);
-  m.def("gemm_variant", &gemm_variant);
+  m.def("gemm_tn(Tensor a, Tensor b, Tensor out, Tensor? residual, int epilogue, Tensor status, Tensor? live=None) -> ()", &gemm_tn);
+  m.def("gemm(Tensor a, Tensor b, Tensor out, int epilogue, bool a_mn, bool b_mn, Tensor status, Tensor? live=None) -> ()", &gemm);
+  m.def("gemm_variant(Tensor a, Tensor b, Tensor out, int epilogue, bool a_mn, bool b_mn, Tensor status, int variant, Tensor? live=None) -> ()", &gemm_variant);
   m.def("gemm_stack", &gemm_stack);
   m.def("lmhead_loss_fwd", &lmhead_loss_fwd);
   m.def("moe_group_plan", &moe_group_plan);
   m.def("gemm_grouped_rows", &gemm_grouped_rows);
   m.def("gemm_grouped_wgrad", &gemm_grouped_wgrad);
   m.def("gemm_wgrad_parts", &gemm_wgrad_parts);
+  m.def("gemm_wgrad_parts_rows", &gemm_wgrad_parts_rows);
   m.def("gemm_grouped_wgrad_parts", &gemm_grouped_wgrad_parts);
-  m.def("gemm_tn_variant", &gemm_tn_variant);
+  m.def("gemm_tn_variant(Tensor a, Tensor b, Tensor out, Tensor? residual, int epilogue, Tensor status, int variant, Tensor? live=None) -> ()", &gemm_tn_variant);
   m.def("attn_fwd", &attn_fwd);
   m.def("attn_fwd_tc", &attn_fwd_tc);
   m.def("attn_bwd", &attn_bwd);

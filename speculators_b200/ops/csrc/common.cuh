@@ -92,6 +92,10 @@ inline cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, 
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
 
+// How many of a buffer's rows hold anything, where the device alone knows (nullptr: all of them).  Rows behind are neither
+// read nor written.  Read after pdl_begin.
+__device__ __forceinline__ int live_rows(const int* live, int rows) { return live != nullptr ? min(rows, max(*live, 0)) : rows; }
+
 struct alignas(16) bf16x8 {
   __nv_bfloat162 v[4];
 };

@@ -68,8 +68,9 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ dh,
 __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const int64_t* __restrict__ positions,
                             const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                             int64_t tokens, int heads, int hd, int rot, int64_t row_stride,
-                            int64_t max_pos, float sign) {
+                            int64_t max_pos, float sign, const int* __restrict__ live) {
   pdl_begin();
+  tokens = live_rows(live, (int)tokens);
   const int half = rot >> 1;
   const int64_t total = tokens * heads * half;
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -95,8 +96,9 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const int64_t* __rest
 __global__ void rope_vec8_kernel(__nv_bfloat16* __restrict__ x, const int64_t* __restrict__ positions,
                                  const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                                  int64_t tokens, int heads, int hd, int rot, int64_t row_stride,
-                                 int64_t max_pos, float sign) {
+                                 int64_t max_pos, float sign, const int* __restrict__ live) {
   pdl_begin();
+  tokens = live_rows(live, (int)tokens);
   const int half = rot >> 1;
   const int hv = half >> 3;
   const int64_t total = tokens * heads * hv;
@@ -147,6 +149,7 @@ struct RopeMerge {
   int64_t max_pos;
   int tokens, hd, rot;
   float sign;
+  const int* live;  // optional: tokens in use
 };
 __global__ void __launch_bounds__(256) rope_merge_kernel(const RopeMerge a) {
   pdl_begin();
@@ -154,7 +157,7 @@ __global__ void __launch_bounds__(256) rope_merge_kernel(const RopeMerge a) {
   int units[3], all = 0;
 #pragma unroll
   for (int i = 0; i < 3; ++i) { units[i] = a.part[i].heads * (a.part[i].rotate ? rotated : plain); all += units[i]; }
-  const int64_t total = (int64_t)a.tokens * all;
+  const int64_t total = (int64_t)live_rows(a.live, a.tokens) * all;
   for (int64_t idx = (int64_t)blockIdx.x * 256 + threadIdx.x; idx < total; idx += (int64_t)gridDim.x * 256) {
     const int t = (int)(idx / all);
     int u = (int)(idx - (int64_t)t * all), col = 0, which = 0;
@@ -259,7 +262,7 @@ void launch_swiglu_bwd(const void* dh, const void* gate_up, void* dgate_up, int6
 }
 void launch_rope(void* x, const int64_t* positions, const float* cos_t, const float* sin_t,
                  int64_t tokens, int heads, int hd, int rot, int64_t row_stride, int64_t max_pos,
-                 float sign, cudaStream_t stream) {
+                 float sign, const int* live, cudaStream_t stream) {
   if (tokens <= 0) return;
   count_launch(1);
   const int half = rot >> 1;
@@ -267,17 +270,17 @@ void launch_rope(void* x, const int64_t* positions, const float* cos_t, const fl
                    ((uintptr_t)cos_t % 16 == 0) && ((uintptr_t)sin_t % 16 == 0);
   if (vec) {
     launch_pdl(rope_vec8_kernel, grid_for(tokens * heads * (half >> 3), 256), 256, 0, stream, 
-        (__nv_bfloat16*)x, positions, cos_t, sin_t, tokens, heads, hd, rot, row_stride, max_pos, sign);
+        (__nv_bfloat16*)x, positions, cos_t, sin_t, tokens, heads, hd, rot, row_stride, max_pos, sign, live);
     return;
   }
   launch_pdl(rope_kernel, grid_for(tokens * heads * half, 256), 256, 0, stream, 
-      (__nv_bfloat16*)x, positions, cos_t, sin_t, tokens, heads, hd, rot, row_stride, max_pos, sign);
+      (__nv_bfloat16*)x, positions, cos_t, sin_t, tokens, heads, hd, rot, row_stride, max_pos, sign, live);
 }
 
 // srcs / strides / heads / rotate: three column blocks (heads 0: absent).  rot and hd multiples of 16 and 8, rows 16-byte aligned.
 void launch_rope_merge(const void* const* srcs, const int64_t* strides, const int* heads, const int* rotate, void* dst, int64_t dst_stride,
                        const int64_t* positions, const float* cos_t, const float* sin_t, int64_t max_pos, int tokens, int hd, int rot, float sign,
-                       cudaStream_t stream) {
+                       const int* live, cudaStream_t stream) {
   if (tokens <= 0) return;
   RopeMerge a{};
   int64_t units = 0;
@@ -295,6 +298,7 @@ void launch_rope_merge(const void* const* srcs, const int64_t* strides, const in
   a.hd = hd;
   a.rot = rot;
   a.sign = sign;
+  a.live = live;
   count_launch(1);
   launch_pdl(rope_merge_kernel, grid_for(tokens * units, 256), 256, 0, stream, a);
 }

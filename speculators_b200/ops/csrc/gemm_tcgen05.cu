@@ -125,6 +125,9 @@ struct Params {
   int batch;
   int64_t c_batch, r_batch;
   int symmetric;  // the product is symmetric: tiles above the diagonal are computed and stored twice (map_h: transposed stores)
+  // Device-side row count of the activations (live_rows).  It bounds M, and where both operands are MN-major (a weight
+  // gradient, which sums over the rows) K.  A multiple of 256 or all rows: no tile and no contraction step straddles it.
+  const int* live;
 };
 
 __device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16(x)); }
@@ -175,7 +178,7 @@ struct TileInfo {
 constexpr int kBandRows = 8;
 
 template <bool B_MN>
-__device__ __forceinline__ TileInfo decode_tile(const Params& p, int tile, int tiles_m, int tiles_n, int num_kb, int rank) {
+__device__ __forceinline__ TileInfo decode_tile(const Params& p, int M, int tile, int tiles_m, int tiles_n, int num_kb, int rank) {
   TileInfo t;
   t.z = 0;
   t.mirror = false;
@@ -190,7 +193,7 @@ __device__ __forceinline__ TileInfo decode_tile(const Params& p, int tile, int t
     t.mirror = i != j;
     t.tile_n = j;
     t.n0 = j * 256;
-    t.a_m = m0; t.a_k0 = 0; t.b_n = t.n0 + rank * 128; t.b_k0 = 0; t.num_kb = num_kb; t.c_row0 = m0; t.row_end = p.M;
+    t.a_m = m0; t.a_k0 = 0; t.b_n = t.n0 + rank * 128; t.b_k0 = 0; t.num_kb = num_kb; t.c_row0 = m0; t.row_end = M;
   } else if (p.grp.mode == kGroupNone) {
     t.z = tile / (tiles_m * tiles_n);
     tile -= t.z * tiles_m * tiles_n;
@@ -203,7 +206,7 @@ __device__ __forceinline__ TileInfo decode_tile(const Params& p, int tile, int t
     const int m0 = (first + local % rows) * 256 + rank * 128;
     t.tile_n = local / rows;
     t.n0 = t.tile_n * 256;
-    t.a_m = m0; t.a_k0 = 0; t.b_n = t.n0 + rank * 128; t.b_k0 = 0; t.num_kb = num_kb; t.c_row0 = m0; t.row_end = p.M;
+    t.a_m = m0; t.a_k0 = 0; t.b_n = t.n0 + rank * 128; t.b_k0 = 0; t.num_kb = num_kb; t.c_row0 = m0; t.row_end = M;
     if (p.epilogue == kSwiGLU) {  // 128 gate rows for the leader, the matching up rows for its peer
       t.n0 = t.tile_n * 128;
       t.b_n = t.n0 + rank * (p.N >> 1);
@@ -593,9 +596,6 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   const int tiles_m = (p.M + BM - 1) / BM, tiles = tiles_m * ((p.N + S_TILE_N - 1) / S_TILE_N);
   const int z = (int)(blockIdx.x >> log_splits) / tiles, tile = (int)(blockIdx.x >> log_splits) - z * tiles;
   const int m0 = (tile % tiles_m) * BM, n0 = (tile / tiles_m) * S_TILE_N;
-  const int all_kb = (p.K + S_STEP_K - 1) / S_STEP_K;
-  const int kb0 = (split * all_kb) >> log_splits, num_kb = (((split + 1) * all_kb) >> log_splits) - kb0;
-
   if (threadIdx.x == 0) {
     for (int s = 0; s < S_STAGES; ++s) {
       mbar_init(smem_addr(&bar_full[s]), 1);
@@ -613,6 +613,11 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   fence_after_sync();
   const uint32_t tmem_base = tmem_base_slot;
   pdl_begin();
+  constexpr bool kSumsRows = A_MN && B_MN;
+  const int M = kSumsRows ? p.M : live_rows(p.live, p.M), K = kSumsRows ? live_rows(p.live, p.K) : p.K;
+  const bool dead = m0 >= M;  // the whole cluster: nothing is loaded, multiplied or stored
+  const int all_kb = dead ? 0 : (K + S_STEP_K - 1) / S_STEP_K;
+  const int kb0 = (split * all_kb) >> log_splits, num_kb = (((split + 1) * all_kb) >> log_splits) - kb0;
   if (log_splits > 0) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // waited for before the first remote store
 
   bool ok = true;
@@ -664,8 +669,8 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     }
   } else if (log_splits == 0) {
     RowPrefetch<S_TILE_N> pre;
-    if (p.staged) prefetch_addend_staged<S_TILE_N>(p, row, n0, z, p.M, pre);
-    else prefetch_addend<S_TILE_N>(p, row, n0, z, p.M, pre);
+    if (p.staged) prefetch_addend_staged<S_TILE_N>(p, row, n0, z, M, pre);
+    else prefetch_addend<S_TILE_N>(p, row, n0, z, M, pre);
     ok = mbar_wait(smem_addr(&bar_acc_full), 0, p.status, kTimeoutEpilogue);
     ok = __all_sync(0xffffffffu, ok);
     if (ok) {
@@ -673,12 +678,12 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16);
       if (p.staged) {
         const uint32_t stage = smem_addr(smem + S_STAGES * S_STAGE_BYTES) + quarter * 4096;
-        store_accumulator_staged<S_TILE_N>(p, sc, &map_c, &map_c, stage, taddr, m0 + quarter * 32, n0, z, pre, m0 + quarter * 32 < p.M, false, false, lane);
+        store_accumulator_staged<S_TILE_N>(p, sc, &map_c, &map_c, stage, taddr, m0 + quarter * 32, n0, z, pre, m0 + quarter * 32 < M, false, num_kb == 0, lane);
         stage_wait();
       } else if (pre.tile_ok) {
-        store_accumulator_prefetched<S_TILE_N>(p, sc, taddr, row, n0, z, pre, false);
+        store_accumulator_prefetched<S_TILE_N>(p, sc, taddr, row, n0, z, pre, num_kb == 0);
       } else {
-        store_accumulator<S_TILE_N>(p, sc, taddr, row, n0, z, p.M, false);
+        store_accumulator<S_TILE_N>(p, sc, taddr, row, n0, z, M, num_kb == 0);
       }
     }
   } else {
@@ -722,7 +727,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           const float4 o = got[((src << log_rows) + r0) * 16 + (c ^ (r0 & 15))];
           t.x += o.x; t.y += o.y; t.z += o.z; t.w += o.w;
         }
-        if (orow < p.M) store_vec4(p, sc, t, orow, n0 + c * 4, z);
+        if (orow < M) store_vec4(p, sc, t, orow, n0 + c * 4, z);
       }
     }
   }
@@ -760,27 +765,39 @@ constexpr int P_THREADS = 320, P_EPI_COLS = 128;
 constexpr int kMoreParts = 3;
 struct MoreParts {
   CUtensorMap a[kMoreParts], b[kMoreParts];
-  const int* seg[kMoreParts];  // grouped contraction: the part's own segments
-  int num_kb[kMoreParts];
+  const int* seg[kMoreParts];   // grouped contraction: the part's own segments
+  const int* live[kMoreParts];  // as Params::live
+  int rows[kMoreParts];
   int n;
 };
 struct NoParts {};
 template <bool PARTS> struct PartsArg { typedef NoParts type; };
 template <> struct PartsArg<true> { typedef MoreParts type; };
-// 128-wide contraction steps of part i for this tile, and where they start
-__device__ __forceinline__ int part_steps(const Params& p, const MoreParts& more, int i, int tile, int per, int& k0) {
+// 128-wide contraction steps of the parts of a plain product, read once per thread
+template <bool PARTS> struct PartSteps {
+  __device__ __forceinline__ explicit PartSteps(const NoParts&) {}
+};
+template <> struct PartSteps<true> {
+  int kb[kMoreParts];
+  __device__ __forceinline__ explicit PartSteps(const MoreParts& more) {
+#pragma unroll
+    for (int i = 0; i < kMoreParts; ++i) kb[i] = i < more.n ? (live_rows(more.live[i], more.rows[i]) + 127) >> 7 : 0;
+  }
+};
+// ... of part i for this tile, and where they start
+__device__ __forceinline__ int part_steps(const Params& p, const MoreParts& more, const PartSteps<true>& steps, int i, int tile, int per, int& k0) {
   k0 = 0;
-  if (p.grp.mode != kGroupK) return more.num_kb[i];
+  if (p.grp.mode != kGroupK) return i == 0 ? steps.kb[0] : i == 1 ? steps.kb[1] : steps.kb[2];
   const int e = tile / per;
   k0 = more.seg[i][e];
   return (more.seg[i][e + 1] - k0) >> 7;
 }
-__device__ __forceinline__ int more_steps(const Params& p, const MoreParts& more, int tile, int per) {
+__device__ __forceinline__ int more_steps(const Params& p, const MoreParts& more, const PartSteps<true>& steps, int tile, int per) {
   int sum = 0, k0;
-  for (int i = 0; i < more.n; ++i) sum += part_steps(p, more, i, tile, per, k0);
+  for (int i = 0; i < more.n; ++i) sum += part_steps(p, more, steps, i, tile, per, k0);
   return sum;
 }
-__device__ __forceinline__ int more_steps(const Params&, const NoParts&, int, int) { return 0; }
+__device__ __forceinline__ int more_steps(const Params&, const NoParts&, const PartSteps<false>&, int, int) { return 0; }
 
 template <int KSUB, bool A_MN = false, bool B_MN = false, bool PARTS = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P_THREADS, 1)
@@ -801,9 +818,6 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
-  const int tiles_m = (p.M + P_TILE_M - 1) / P_TILE_M, tiles_n = (p.N + P_TILE_N - 1) / P_TILE_N;
-  const int num_kb = (p.K + STAGE_K - 1) / STAGE_K;
-
   if (threadIdx.x == 0) {
     for (int s = 0; s < P_STAGES; ++s) {
       mbar_init(smem_addr(&bar_full[s]), 1);   // the leader's expect_tx arrival; bytes come from both CTAs' copies
@@ -824,6 +838,11 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   fence_after_sync();
   const uint32_t tmem_base = tmem_base_slot;
   pdl_begin();
+  constexpr bool kSumsRows = A_MN && B_MN;
+  const int M = kSumsRows ? p.M : live_rows(p.live, p.M), K = kSumsRows ? live_rows(p.live, p.K) : p.K;
+  const int tiles_m = (M + P_TILE_M - 1) / P_TILE_M, tiles_n = (p.N + P_TILE_N - 1) / P_TILE_N;
+  const int num_kb = (K + STAGE_K - 1) / STAGE_K;
+  [[maybe_unused]] const PartSteps<PARTS> steps(more);
   const int num_tiles = p.grp.mode == kGroupRows ? p.grp.tile_start[p.grp.num_groups] * tiles_n
                         : p.grp.mode == kGroupK  ? p.grp.num_groups * tiles_m * tiles_n
                                                  : p.batch * (p.symmetric ? tiles_m * (tiles_m + 1) / 2 : tiles_m * tiles_n);
@@ -834,9 +853,9 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       uint32_t stage = 0, phase = 0;
       bool ok = true;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
-        const TileInfo ti = decode_tile<B_MN>(p, tile, tiles_m, tiles_n, num_kb, (int)rank);
-        auto load_steps = [&](const CUtensorMap* ma, const CUtensorMap* mb, int a_k0, int b_k0, int steps) {
-          for (int kb = 0; kb < steps; ++kb) {
+        const TileInfo ti = decode_tile<B_MN>(p, M, tile, tiles_m, tiles_n, num_kb, (int)rank);
+        auto load_steps = [&](const CUtensorMap* ma, const CUtensorMap* mb, int a_k0, int b_k0, int count) {
+          for (int kb = 0; kb < count; ++kb) {
             if (!(ok = mbar_wait(smem_addr(&bar_empty[stage]), phase ^ 1, p.status, kTimeoutProducer))) break;
             const uint32_t full_local = smem_addr(&bar_full[stage]);
             if (leader) mbar_expect_tx(full_local, 2 * P_STAGE_BYTES);
@@ -859,8 +878,8 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         if constexpr (PARTS) {
           for (int i = 0; i < more.n && ok; ++i) {
             int k0;
-            const int steps = part_steps(p, more, i, tile, tiles_m * tiles_n, k0);
-            load_steps(&more.a[i], &more.b[i], k0, k0, steps);
+            const int count = part_steps(p, more, steps, i, tile, tiles_m * tiles_n, k0);
+            load_steps(&more.a[i], &more.b[i], k0, k0, count);
           }
         }
       }
@@ -883,7 +902,7 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         if (!(ok = mbar_wait(smem_addr(&bar_acc_empty[acc]), ((local >> 1) & 1) ^ 1, p.status, kTimeoutMma))) break;
         fence_after_sync();
         const uint32_t tmem_d = tmem_base + acc * BN;
-        const int tile_kb = decode_tile<B_MN>(p, tile, tiles_m, tiles_n, num_kb, 0).num_kb + more_steps(p, more, tile, tiles_m * tiles_n);
+        const int tile_kb = decode_tile<B_MN>(p, M, tile, tiles_m, tiles_n, num_kb, 0).num_kb + more_steps(p, more, steps, tile, tiles_m * tiles_n);
         for (int kb = 0; kb < tile_kb; ++kb) {
           if (!(ok = mbar_wait(smem_addr(&bar_full[stage]), phase, p.status, kTimeoutMma))) break;
           fence_after_sync();
@@ -917,9 +936,9 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     int local = 0;
     for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++local) {
       const int acc = local & 1;
-      const TileInfo ti = decode_tile<B_MN>(p, tile, tiles_m, tiles_n, num_kb, (int)rank);
+      const TileInfo ti = decode_tile<B_MN>(p, M, tile, tiles_m, tiles_n, num_kb, (int)rank);
       const int row = ti.c_row0 + quarter * 32 + lane, n0 = ti.n0 + chalf * P_EPI_COLS;
-      const bool zero = ti.num_kb + more_steps(p, more, tile, tiles_m * tiles_n) == 0;
+      const bool zero = ti.num_kb + more_steps(p, more, steps, tile, tiles_m * tiles_n) == 0;
       RowPrefetch<P_EPI_COLS> pre;
       const bool with_stats = p.rs.targets != nullptr, gated = p.epilogue == kSwiGLU;
       if (with_stats) prefetch_targets<P_EPI_COLS>(p, row, n0, pre);
@@ -982,9 +1001,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   const int tiles = tiles_m * ((p.N + P_TILE_N - 1) / P_TILE_N);
   const int z = (int)(blockIdx.x / (2 * SPLITS)) / tiles, tile = (int)(blockIdx.x / (2 * SPLITS)) - z * tiles;
   const int m0 = (tile % tiles_m) * P_TILE_M + role * P_HALF, n0 = (tile / tiles_m) * P_TILE_N;
-  const int all_kb = (p.K + STAGE_K - 1) / STAGE_K, per_kb = (all_kb + SPLITS - 1) / SPLITS;
-  const int kb0 = split * per_kb, num_kb = max(0, min(per_kb, all_kb - kb0));
-
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(smem_addr(&bar_full[s]), 1);
@@ -1002,6 +1018,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   fence_after_sync();
   const uint32_t tmem_base = tmem_base_slot;
   pdl_begin();
+  constexpr bool kSumsRows = A_MN && B_MN;
+  const int M = kSumsRows ? p.M : live_rows(p.live, p.M), K = kSumsRows ? live_rows(p.live, p.K) : p.K;
+  const bool dead = (tile % tiles_m) * P_TILE_M >= M;  // the whole cluster
+  const int all_kb = dead ? 0 : (K + STAGE_K - 1) / STAGE_K, per_kb = (all_kb + SPLITS - 1) / SPLITS;
+  const int kb0 = split * per_kb, num_kb = max(0, min(per_kb, all_kb - kb0));
 
   bool ok = true;
   const Scaling sc{p.alpha, p.beta};
@@ -1095,7 +1116,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         const float4 o = got[(src * OWN_ROWS + r0) * (P_TILE_N / 4) + (c ^ (r0 & 31))];
         t.x += o.x; t.y += o.y; t.z += o.z; t.w += o.w;
       }
-      if (row < p.M) store_vec4(p, sc, t, row, n0 + c * 4, z);
+      if (row < M) store_vec4(p, sc, t, row, n0 + c * 4, z);
     }
   }
   fence_before_sync();
@@ -1210,6 +1231,7 @@ struct PartsSpec {
   int K[tc::kMoreParts];
   int64_t lda[tc::kMoreParts], ldb[tc::kMoreParts];
   const int* seg[tc::kMoreParts];
+  const int* live[tc::kMoreParts];
 };
 
 // What a stack of products adds to a single one; see Params.
@@ -1231,7 +1253,7 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
                             int64_t ldb, int64_t ldc, int64_t ldr, int epilogue, int a_mn, int b_mn, int* status, int variant,
                             const void* stats_targets, int64_t stats_ldt, int stats_t_rows, int stats_shift, float* stats_partial,
                             const tc::Grouping* grp, cudaStream_t stream, const tc::Scatter* scatter = nullptr, void* gated_h = nullptr,
-                            int64_t gated_ldh = 0, const BatchSpec* batched = nullptr, const PartsSpec* parts = nullptr) {
+                            int64_t gated_ldh = 0, const BatchSpec* batched = nullptr, const PartsSpec* parts = nullptr, const int* live = nullptr) {
   using namespace tc;
   static const BatchSpec one{};
   const BatchSpec& bs = batched != nullptr ? *batched : one;
@@ -1272,7 +1294,8 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
   if (rc) return rc;
   Params p{(__nv_bfloat16*)c, (const __nv_bfloat16*)residual, M, N, K, ldc, ldr, epilogue, status, RowStatsOut{nullptr, 0, 0, 0, nullptr},
            Grouping{kGroupNone, 0, nullptr, nullptr}, Scatter{}, (__nv_bfloat16*)gated_h, gated_ldh, 0, bs.alpha, bs.beta, bs.batch,
-           bs.c_stride, bs.r_stride, 0};
+           bs.c_stride, bs.r_stride, 0, live};
+  if (live != nullptr && (grp != nullptr || scatter != nullptr || stats_targets != nullptr || bs.batch != 1 || (a_mn && !b_mn))) return -10;
   if (epilogue == kSwiGLU) {
     if (!pairs || a_mn || b_mn || (grp != nullptr && grp->mode != kGroupRows) || stats_targets != nullptr || scatter != nullptr || gated_h == nullptr || (N & 255) || (ldc & 7) ||
         (gated_ldh & 7) || (reinterpret_cast<uintptr_t>(c) & 15) || (reinterpret_cast<uintptr_t>(gated_h) & 15))
@@ -1329,8 +1352,9 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
       rc = make_map_bf16_stack(&more.a[i], parts->a[i], parts->K[i], M, parts->lda[i], mn_rows, 1, 0);
       if (rc == 0) rc = make_map_bf16_stack(&more.b[i], parts->b[i], parts->K[i], N, parts->ldb[i], mn_rows, 1, 0);
       if (rc) return rc;
-      more.num_kb[i] = (parts->K[i] + 2 * BK - 1) / (2 * BK);
+      more.rows[i] = parts->K[i];
       more.seg[i] = parts->seg[i];
+      more.live[i] = parts->live[i];
     }
   }
   count_launch(1);
@@ -1358,20 +1382,21 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
 }
 
 int launch_gemm_tcgen05(const void* a, const void* b, void* c, const void* residual, int M, int N, int K, int64_t lda,
-                        int64_t ldb, int64_t ldc, int64_t ldr, int epilogue, int a_mn, int b_mn, int* status, int variant,
+                        int64_t ldb, int64_t ldc, int64_t ldr, int epilogue, int a_mn, int b_mn, int* status, int variant, const int* live,
                         cudaStream_t stream) {
-  return launch_gemm_impl(a, b, c, residual, M, N, K, lda, ldb, ldc, ldr, epilogue, a_mn, b_mn, status, variant, nullptr, 0, 0, 0, nullptr, nullptr, stream);
+  return launch_gemm_impl(a, b, c, residual, M, N, K, lda, ldb, ldc, ldr, epilogue, a_mn, b_mn, status, variant, nullptr, 0, 0, 0, nullptr, nullptr, stream,
+                          nullptr, nullptr, 0, nullptr, nullptr, live);
 }
 
 int launch_gemm_tn_tcgen05(const void* a, const void* b, void* c, const void* residual, int M, int N, int K, int64_t lda,
-                           int64_t ldb, int64_t ldc, int64_t ldr, int epilogue, int* status, int variant, cudaStream_t stream) {
-  return launch_gemm_tcgen05(a, b, c, residual, M, N, K, lda, ldb, ldc, ldr, epilogue, 0, 0, status, variant, stream);
+                           int64_t ldb, int64_t ldc, int64_t ldr, int epilogue, int* status, int variant, const int* live, cudaStream_t stream) {
+  return launch_gemm_tcgen05(a, b, c, residual, M, N, K, lda, ldb, ldc, ldr, epilogue, 0, 0, status, variant, live, stream);
 }
 
 // c[M, N] (+)= sum_i a_i[K_i, M]^T . b_i[K_i, N]: one launch where pair tiles are the form for the whole contraction, else one each
 // (small products are not bound by their epilogue, and have better forms).
-int launch_gemm_parts(int n, const void* const* a, const void* const* b, const int* K, const int64_t* lda, const int64_t* ldb, void* c, int M, int N,
-                      int64_t ldc, int accumulate, int* status, cudaStream_t stream) {
+int launch_gemm_parts(int n, const void* const* a, const void* const* b, const int* K, const int64_t* lda, const int64_t* ldb, const int* const* live,
+                      void* c, int M, int N, int64_t ldc, int accumulate, int* status, cudaStream_t stream) {
   if (n < 1 || n > tc::kMoreParts + 1) return -9;
   int total = 0;
   PartsSpec parts;
@@ -1385,14 +1410,15 @@ int launch_gemm_parts(int n, const void* const* a, const void* const* b, const i
     parts.lda[i - 1] = lda[i];
     parts.ldb[i - 1] = ldb[i];
     parts.seg[i - 1] = nullptr;
+    parts.live[i - 1] = live[i];
   }
   parts.n = n - 1;
   if (n > 1 && choose_variant(M, N, total, 1, 0) == kPair)
     return launch_gemm_impl(a[0], b[0], c, nullptr, M, N, K[0], lda[0], ldb[0], ldc, 0, accumulate ? 1 : 0, 1, 1, status, kPair, nullptr, 0, 0, 0, nullptr,
-                            nullptr, stream, nullptr, nullptr, 0, nullptr, &parts);
+                            nullptr, stream, nullptr, nullptr, 0, nullptr, &parts, live[0]);
   for (int i = 0; i < n; ++i) {
     const int rc = launch_gemm_impl(a[i], b[i], c, nullptr, M, N, K[i], lda[i], ldb[i], ldc, 0, accumulate || i > 0 ? 1 : 0, 1, 1, status, 0, nullptr, 0, 0, 0,
-                                    nullptr, nullptr, stream);
+                                    nullptr, nullptr, stream, nullptr, nullptr, 0, nullptr, nullptr, live[i]);
     if (rc) return rc;
   }
   return 0;
@@ -1432,9 +1458,9 @@ int launch_gemm_scatter(const void* a, const void* b, void* const* stage, int wo
 // ---- gate | up product of a gated MLP with the activation in the epilogue ---------------------
 // gate_up[M, 2 I] = x[M, K] . w[2 I, K]^T (gate rows first) and h[M, I] = silu(gate) * up.  I % 128 == 0.
 int launch_gemm_swiglu(const void* x, const void* w, void* gate_up, void* h, int M, int I, int K, int64_t ldx, int64_t ldw, int64_t ldc, int64_t ldh,
-                       int* status, cudaStream_t stream) {
+                       int* status, const int* live, cudaStream_t stream) {
   return launch_gemm_impl(x, w, gate_up, nullptr, M, 2 * I, K, ldx, ldw, ldc, 0, tc::kSwiGLU, 0, 0, status, 3, nullptr, 0, 0, 0, nullptr, nullptr, stream,
-                          nullptr, h, ldh);
+                          nullptr, h, ldh, nullptr, nullptr, live);
 }
 
 // ---- grouped products for mixture-of-experts layers -----------------------------------------
@@ -1485,6 +1511,7 @@ int launch_gemm_grouped_parts(int n, const void* const* a, const void* const* b,
     parts.lda[i - 1] = lda[i];
     parts.ldb[i - 1] = ldb[i];
     parts.seg[i - 1] = seg[i];
+    parts.live[i - 1] = nullptr;
   }
   const tc::Grouping grp{tc::kGroupK, num_groups, seg[0], mtile_start};
   return launch_gemm_impl(a[0], b[0], c, nullptr, M, N, K[0], lda[0], ldb[0], N, 0, accumulate ? 1 : 0, 1, 1, status, kPair, nullptr, 0, 0, 0, nullptr, &grp,

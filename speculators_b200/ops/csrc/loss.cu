@@ -81,14 +81,15 @@ loss_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* _
                 const uint8_t* __restrict__ active, const uint8_t* __restrict__ also, const int64_t* __restrict__ labels,
                 float* __restrict__ loss, float* __restrict__ stats, int* __restrict__ argmax_d,
                 int* __restrict__ argmax_t, int rows, int V, int64_t ld_logits, int64_t ld_targets,
-                int shift) {
+                int shift, const int* __restrict__ target_row) {
   pdl_begin();
   __shared__ float scratch[33];
   __shared__ int iscratch[33];
   const int r = blockIdx.x;
   if (r >= rows) return;
   float* st = stats + r;
-  if (active && !active[r] && !(also && also[r])) {
+  const int tr = target_row != nullptr ? target_row[r] : r + shift;
+  if (tr < 0 || (active && !active[r] && !(also && also[r]))) {
     if (threadIdx.x == 0) {
       loss[r] = 0.f;
 #pragma unroll
@@ -101,7 +102,7 @@ loss_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* _
   const __nv_bfloat16* x = logits + (int64_t)r * ld_logits;
   // with integer labels (token cross-entropy) there is no target row to read
   const bool has_t = targets != nullptr;
-  const __nv_bfloat16* t = has_t ? targets + (int64_t)(r + shift) * ld_targets : x;
+  const __nv_bfloat16* t = has_t ? targets + (int64_t)tr * ld_targets : x;
   const bool vec_ok = ((V & 7) == 0) && ((ld_logits & 7) == 0) && ((ld_targets & 7) == 0);
   const int nvec = vec_ok ? (V >> 3) : 0;
 
@@ -132,7 +133,7 @@ loss_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* _
   } else {
     stt.m = 0.f;
     stt.z = 1.f;
-    int lab = labels ? (int)labels[r + shift] : 0;
+    int lab = labels ? (int)labels[tr] : 0;
     stt.best_idx = lab < 0 ? 0 : (lab >= V ? V - 1 : lab);
   }
   const float lse_d = sd.m + __logf(sd.z);
@@ -209,10 +210,11 @@ __global__ void __launch_bounds__(kLossThreads)
 loss_bwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* __restrict__ targets,
                 const float* __restrict__ grad_out, const float* __restrict__ grad_scale, const float* __restrict__ stats,
                 __nv_bfloat16* __restrict__ dlogits, int rows, int total_rows, int V,
-                int64_t ld_logits, int64_t ld_targets, int64_t ld_dlogits, int shift) {
+                int64_t ld_logits, int64_t ld_targets, int64_t ld_dlogits, int shift, const int* __restrict__ target_row,
+                const int* __restrict__ live) {
   pdl_begin();
   const int r = blockIdx.x;
-  if (r >= total_rows) return;
+  if (r >= live_rows(live, total_rows)) return;
   __nv_bfloat16* d = dlogits + (int64_t)r * ld_dlogits;
   const bool vec_ok =
       ((V & 7) == 0) && ((ld_logits & 7) == 0) && ((ld_targets & 7) == 0) && ((ld_dlogits & 7) == 0);
@@ -230,7 +232,7 @@ loss_bwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* _
     return;
   }
   const __nv_bfloat16* x = logits + (int64_t)r * ld_logits;
-  const __nv_bfloat16* t = targets + (int64_t)(r + shift) * ld_targets;
+  const __nv_bfloat16* t = targets + (int64_t)(target_row != nullptr ? target_row[r] : r + shift) * ld_targets;  // not negative: the forward did not skip it
   const float* st = stats + r;
   const float lse_d = st[0] + __logf(st[(int64_t)rows]);
   const float lse_t = (OP == kOpCE) ? 0.f : st[(int64_t)2 * rows] + __logf(st[(int64_t)3 * rows]);
@@ -265,17 +267,18 @@ loss_bwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* _
         grad(__bfloat162float(x[c]), OP != kOpCE ? __bfloat162float(t[c]) : 0.f, c));
 }
 
-// active / also (optional): rows marked in neither are skipped
+// active / also (optional): rows marked in neither are skipped.  target_row (optional): the row of `targets` that each row is
+// compared with, instead of its own + shift; rows with a negative one are skipped.
 int launch_loss_fwd(int op, const void* logits, const void* targets, const uint8_t* active, const uint8_t* also,
                     const int64_t* labels, float* loss, float* stats, int* argmax_d, int* argmax_t, int rows, int V,
-                    int64_t ld_logits, int64_t ld_targets, int shift, cudaStream_t stream) {
+                    int64_t ld_logits, int64_t ld_targets, int shift, const int* target_row, cudaStream_t stream) {
   if (rows <= 0) return 0;
   if (targets == nullptr && (labels == nullptr || op != kOpCE)) return -3;
   count_launch(1);
 #define SB200_LF(OPV)                                                                            \
   launch_pdl(loss_fwd_kernel<OPV>, rows, kLossThreads, 0, stream,                                         \
       (const __nv_bfloat16*)logits, (const __nv_bfloat16*)targets, active, also, labels, loss, stats,   \
-      argmax_d, argmax_t, rows, V, ld_logits, ld_targets, shift)
+      argmax_d, argmax_t, rows, V, ld_logits, ld_targets, shift, target_row)
   switch (op) {
     case kOpKL: SB200_LF(kOpKL); break;
     case kOpRKL: SB200_LF(kOpRKL); break;
@@ -288,17 +291,18 @@ int launch_loss_fwd(int op, const void* logits, const void* targets, const uint8
   return 0;
 }
 
-// grad_scale (optional, device): a factor of every grad_out
+// grad_scale (optional, device): a factor of every grad_out; target_row as in launch_loss_fwd; live (optional, device): rows of
+// dlogits in use, those behind are not written
 int launch_loss_bwd(int op, const void* logits, const void* targets, const float* grad_out,
                     const float* grad_scale, const float* stats, void* dlogits, int rows, int total_rows, int V,
-                    int64_t ld_logits, int64_t ld_targets, int64_t ld_dlogits, int shift,
-                    cudaStream_t stream) {
+                    int64_t ld_logits, int64_t ld_targets, int64_t ld_dlogits, int shift, const int* target_row,
+                    const int* live, cudaStream_t stream) {
   if (total_rows <= 0) return 0;
   count_launch(1);
 #define SB200_LB(OPV)                                                                         \
   launch_pdl(loss_bwd_kernel<OPV>, total_rows, kLossThreads, 0, stream,                                \
       (const __nv_bfloat16*)logits, (const __nv_bfloat16*)targets, grad_out, grad_scale, stats,            \
-      (__nv_bfloat16*)dlogits, rows, total_rows, V, ld_logits, ld_targets, ld_dlogits, shift)
+      (__nv_bfloat16*)dlogits, rows, total_rows, V, ld_logits, ld_targets, ld_dlogits, shift, target_row, live)
   switch (op) {
     case kOpKL: SB200_LB(kOpKL); break;
     case kOpRKL: SB200_LB(kOpRKL); break;

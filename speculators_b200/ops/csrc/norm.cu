@@ -66,8 +66,9 @@ __global__ void __launch_bounds__(THREADS, kFwdBlocks<NV, THREADS>)
 rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                    const int64_t* __restrict__ row_index, __nv_bfloat16* __restrict__ y,
                    float* __restrict__ rstd_out, int rows, int H, int64_t x_stride,
-                   int64_t y_stride, float eps, int64_t src_rows, NormWeight nw) {
+                   int64_t y_stride, float eps, int64_t src_rows, NormWeight nw, const int* __restrict__ live) {
   pdl_begin();
+  rows = live_rows(live, rows);
   __shared__ float scratch[2][THREADS / 32];
   const int nvec = H >> 3;
   bf16x8 cur[NV], next[NV];
@@ -137,6 +138,7 @@ struct NormBwdArgs {
   int rows, H;
   int64_t dy_stride, dy2_stride, x_stride, add_stride, dx_stride;
   NormWeight nw;
+  const int* live;  // optional: rows in use
 };
 __device__ __forceinline__ bf16x8 load_dy(const NormBwdArgs& p, int64_t r, int c) {
   const bf16x8 d = ld8(p.dy + r * p.dy_stride + c);
@@ -166,6 +168,7 @@ template <int NV, int THREADS, bool DW>
 __global__ void __launch_bounds__(THREADS)
 rmsnorm_bwd_kernel(const NormBwdArgs p) {
   pdl_begin();
+  const int rows = live_rows(p.live, p.rows);
   __shared__ float scratch[2][THREADS / 32];
   const int nvec = p.H >> 3;
   float dwacc[DW ? NV : 1][8];
@@ -194,14 +197,14 @@ rmsnorm_bwd_kernel(const NormBwdArgs p) {
     }
   };
   int r = blockIdx.x, slot = 0;
-  float rstd_next = r < p.rows ? p.rstd[r] : 0.f;
-  if (kPrefetch && r < p.rows) fetch(r, xa, da);
-  for (; r < p.rows; r += gridDim.x, slot ^= 1) {
+  float rstd_next = r < rows ? p.rstd[r] : 0.f;
+  if (kPrefetch && r < rows) fetch(r, xa, da);
+  for (; r < rows; r += gridDim.x, slot ^= 1) {
     const float rstd = rstd_next;
     const int rn = r + gridDim.x;
-    if (rn < p.rows) rstd_next = p.rstd[rn];
+    if (rn < rows) rstd_next = p.rstd[rn];
     if constexpr (kPrefetch) {
-      if (rn < p.rows) fetch(rn, xb, db);
+      if (rn < rows) fetch(rn, xb, db);
     } else {
       fetch(r, xa, da);
     }
@@ -273,6 +276,7 @@ constexpr int kDwGroups = 8;
 __global__ void __launch_bounds__(32 * kDwGroups)
 rmsnorm_dw_kernel(const NormBwdArgs p) {
   pdl_begin();
+  const int rows = live_rows(p.live, p.rows);
   __shared__ float tile[kDwGroups][32 * 8 + 8];
   const int c = (blockIdx.x * 32 + threadIdx.x) * 8;
   float acc[8];
@@ -280,7 +284,7 @@ rmsnorm_dw_kernel(const NormBwdArgs p) {
   for (int j = 0; j < 8; ++j) acc[j] = 0.f;
   if (c < p.H) {
 #pragma unroll 4
-    for (int r = blockIdx.y * kDwGroups + threadIdx.y; r < p.rows; r += gridDim.y * kDwGroups) {
+    for (int r = blockIdx.y * kDwGroups + threadIdx.y; r < rows; r += gridDim.y * kDwGroups) {
       float xv[8], dv[8];
       const float rstd = p.rstd[r];
       unpack8(ld8(p.x + (int64_t)r * p.x_stride + c), xv);
@@ -335,8 +339,9 @@ __device__ __forceinline__ void narrow_dx(const float (&dy)[8], const float (&w)
 
 __global__ void __launch_bounds__(kNormThreads)
 rmsnorm_fwd_narrow_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
-                          float* __restrict__ rstd_out, int rows, int H, int64_t x_stride, int64_t y_stride, float eps, NormWeight nw) {
+                          float* __restrict__ rstd_out, int rows, int H, int64_t x_stride, int64_t y_stride, float eps, NormWeight nw, const int* __restrict__ live) {
   pdl_begin();
+  rows = live_rows(live, rows);
   const int lane = threadIdx.x & 31, nvec = H >> 3;
   const bool on = lane < nvec;
   float wv[8];
@@ -364,6 +369,7 @@ rmsnorm_fwd_narrow_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat
 __global__ void __launch_bounds__(kNormThreads)
 rmsnorm_bwd_narrow_kernel(const NormBwdArgs p) {
   pdl_begin();
+  const int rows = live_rows(p.live, p.rows);
   const int lane = threadIdx.x & 31, nvec = p.H >> 3;
   const bool on = lane < nvec;
   float wv[8], dwacc[8];
@@ -371,7 +377,7 @@ rmsnorm_bwd_narrow_kernel(const NormBwdArgs p) {
   for (int j = 0; j < 8; ++j) { wv[j] = 0.f; dwacc[j] = 0.f; }
   if (on) p.nw.load(p.w + (lane << 3), wv);
   const int warps = gridDim.x * kNarrowWarps, warp_id = blockIdx.x * kNarrowWarps + (threadIdx.x >> 5);
-  for (int r = warp_id; r < p.rows; r += warps) {
+  for (int r = warp_id; r < rows; r += warps) {
     float xv[8], dv[8], dot = 0.f;
     const float rstd = p.rstd[r];
     if (on) {
@@ -487,13 +493,14 @@ struct HeadsFwdArgs {
   int tokens, src_last;  // tokens from src_last on read that row of src
   float eps;
   HeadsRope rope;
+  const int* live;  // optional: tokens in use
 };
 template <int L>
 __global__ void __launch_bounds__(256) heads_fwd_kernel(const HeadsFwdArgs p) {
   pdl_begin();
   constexpr int HD = L * 8;
   const int l = threadIdx.x % L, all = p.heads[0] + p.heads[1];
-  const int64_t rows = (int64_t)p.tokens * all, groups = (int64_t)gridDim.x * (256 / L);
+  const int64_t rows = (int64_t)live_rows(p.live, p.tokens) * all, groups = (int64_t)gridDim.x * (256 / L);
   const NormWeight nw{false};
   for (int64_t base = (int64_t)blockIdx.x * (256 / L) + (threadIdx.x & ~31) / L; base < rows; base += groups) {
     const int64_t r = base + (threadIdx.x & 31) / L;
@@ -529,6 +536,7 @@ struct HeadsBwdArgs {
   int64_t dst_stride;
   int tokens;
   HeadsRope rope;
+  const int* live;  // optional: tokens in use
 };
 template <int L>
 __global__ void __launch_bounds__(256) heads_bwd_kernel(const HeadsBwdArgs p) {
@@ -542,7 +550,7 @@ __global__ void __launch_bounds__(256) heads_bwd_kernel(const HeadsBwdArgs p) {
   if (g >= p.groups[which]) return;  // whole warps
   const int heads = which == 0 ? p.heads[0] : which == 1 ? p.heads[1] : p.heads[2], groups = p.groups[which], split = p.split[which];
   const int col0 = (which > 0 ? p.heads[0] * HD : 0) + (which > 1 ? p.heads[1] * HD : 0);
-  const int64_t rows = (int64_t)p.tokens * heads;
+  const int64_t rows = (int64_t)live_rows(p.live, p.tokens) * heads;
   const __nv_bfloat16* d0 = p.d[which][0];
   const __nv_bfloat16* d1 = p.d[which][1];
   const int64_t s0 = p.d_stride[which][0], s1 = p.d_stride[which][1];
@@ -707,15 +715,16 @@ int rmsnorm_bwd_partial_rows(int rows, int H, bool with_dx) {
 SB200_BOUNDS_READER(read_bounds_norm)
 
 // src_rows: number of rows of `x` (what `row_index` may address).
+// live (optional, device): how many of the rows are in use.
 void launch_rmsnorm_fwd(const void* x, const void* w, const int64_t* row_index, void* y,
                         float* rstd, int rows, int H, int64_t x_stride, int64_t y_stride, float eps,
-                        int64_t src_rows, int centred, cudaStream_t stream) {
+                        int64_t src_rows, int centred, const int* live, cudaStream_t stream) {
   if (rows <= 0) return;
   const NormWeight nw{centred != 0};
   count_launch(1);
   if (H <= kNarrowMaxH && row_index == nullptr) {
     launch_pdl(rmsnorm_fwd_narrow_kernel, narrow_grid(rows), kNormThreads, 0, stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
-               (__nv_bfloat16*)y, rstd, rows, H, x_stride, y_stride, eps, nw);
+               (__nv_bfloat16*)y, rstd, rows, H, x_stride, y_stride, eps, nw, live);
     return;
   }
   // A block a row, or blocks that walk rows with the next one in flight.  Measured at 512 to 24576 columns, 128 to 16384 rows
@@ -731,7 +740,7 @@ void launch_rmsnorm_fwd(const void* x, const void* w, const int64_t* row_index, 
   };
 #define SB200_FWD(NVV, THREADS)                                                                                          \
   launch_pdl(rmsnorm_fwd_kernel<NVV, THREADS>, grid(kFwdBlocks<NVV, THREADS>), THREADS, 0, stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, row_index, \
-             (__nv_bfloat16*)y, rstd, rows, H, x_stride, y_stride, eps, src_rows, nw)
+             (__nv_bfloat16*)y, rstd, rows, H, x_stride, y_stride, eps, src_rows, nw, live)
   if (H <= 4096) SB200_FWD(2, 256);
   else if (H <= 8192) SB200_FWD(4, 256);
   else if (H <= 16384) SB200_FWD(8, 256);
@@ -741,11 +750,11 @@ void launch_rmsnorm_fwd(const void* x, const void* w, const int64_t* row_index, 
 
 void launch_rmsnorm_bwd(const void* dy, int64_t dy_stride, const void* dy2, int64_t dy2_stride, const void* x, int64_t x_stride, const void* w,
                         const float* rstd, const void* add, int64_t add_stride, void* dx, int64_t dx_stride, float* dw_partial, void* dw, int rows,
-                        int H, int accumulate_dw, int centred, cudaStream_t stream) {
+                        int H, int accumulate_dw, int centred, const int* live, cudaStream_t stream) {
   if (rows <= 0) return;
   typedef const __nv_bfloat16* In;
   const NormBwdArgs p{(In)dy, (In)dy2, (In)x, (In)w, rstd, (In)add, (__nv_bfloat16*)dx, dw_partial, rows, H, dy_stride, dy2_stride, x_stride,
-                      add_stride, dx_stride, NormWeight{centred != 0}};
+                      add_stride, dx_stride, NormWeight{centred != 0}, live};
   const int partial_rows = rmsnorm_bwd_partial_rows(rows, H, dx != nullptr), grid = rows < 2 * kNumSM ? rows : 2 * kNumSM;
   const bool alone = norm_dw_alone(H, dx != nullptr);
 #define SB200_BWD(NVV, THREADS)                                                                                            \
@@ -776,11 +785,11 @@ void launch_rmsnorm_bwd(const void* dy, int64_t dy_stride, const void* dy2, int6
 // heads: a, b; hd 64, 128 or 256; rot a multiple of 16
 // src_last: tokens from there on read that row of src (tokens or more: every token its own)
 void launch_heads_fwd(const void* src, int64_t src_stride, const void* const* w, const int* heads, void* out, float* rstd, int tokens, int src_last, float eps,
-                      const int64_t* positions, const float* cos_t, const float* sin_t, int64_t max_pos, int hd, int rot, cudaStream_t stream) {
+                      const int64_t* positions, const float* cos_t, const float* sin_t, int64_t max_pos, int hd, int rot, const int* live, cudaStream_t stream) {
   if (tokens <= 0) return;
   typedef const __nv_bfloat16* In;
   const HeadsFwdArgs a{(In)src, src_stride, {(In)w[0], (In)w[1]}, {heads[0], heads[1]}, (__nv_bfloat16*)out, rstd, tokens, src_last, eps,
-                       HeadsRope{positions, cos_t, sin_t, max_pos, rot}};
+                       HeadsRope{positions, cos_t, sin_t, max_pos, rot}, live};
   const int64_t blocks = ((int64_t)tokens * (heads[0] + heads[1]) * (hd / 8) + 255) / 256;
   const int grid = (int)(blocks < 16 * kNumSM ? blocks : 16 * kNumSM);
   count_launch(1);
@@ -799,7 +808,7 @@ int64_t repeated_part_floats(int rows, int heads, int hd) { return (int64_t)repe
 void launch_heads_bwd(const void* const* d, const int64_t* d_stride, const int* split, const void* src, int64_t src_stride, const void* const* w,
                       const float* rstd, float* const* partial, void* const* dw, const int* accumulate, const int* heads, void* dst, int64_t dst_stride,
                       int tokens, int all_tokens, float* part, const int64_t* positions, const float* cos_t, const float* sin_t, int64_t max_pos, int hd,
-                      int rot, cudaStream_t stream) {
+                      int rot, const int* live, cudaStream_t stream) {
   if (tokens <= 0) return;
   typedef const __nv_bfloat16* In;
   const bool repeated = all_tokens > tokens;
@@ -831,6 +840,7 @@ void launch_heads_bwd(const void* const* d, const int64_t* d_stride, const int* 
   a.dst_stride = dst_stride;
   a.tokens = tokens;
   a.rope = HeadsRope{positions, cos_t, sin_t, max_pos, rot};
+  a.live = live;
   const int grid = (int)((groups * (hd / 8) + 255) / 256);
   count_launch(1);
   SB200_HEADS(heads_bwd_kernel, grid, a);

@@ -22,8 +22,13 @@ __device__ __forceinline__ int block_scan(int v, Op op, int* scratch) {
   __syncthreads();
   if (lane == 31) scratch[warp] = v;
   __syncthreads();
-  int before = scratch[0];
-  for (int w = 1; w < warp; ++w) before = op(before, scratch[w]);
+  int up_to = scratch[lane];  // every warp scans the 32 sums itself: no serial walk over them
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, up_to, o);
+    if (lane >= o) up_to = op(up_to, u);
+  }
+  const int before = __shfl_sync(0xffffffffu, up_to, max(warp - 1, 0));
   return warp > 0 ? op(v, before) : v;
 }
 
@@ -152,6 +157,146 @@ peagle_spec_kernel(const int64_t* __restrict__ anchor, const int64_t* __restrict
   hi[r] = pad ? 0 : (int)(a0 + 1);
   if (extra != nullptr)
     for (int e = 1; e < num_depths; ++e) extra[(int64_t)r * (num_depths - 1) + e - 1] = d >= e && !pad ? table[(int64_t)e * T + a] : -1;
+}
+
+// ---- rows that a step needs --------------------------------------------------------------------------------------
+// In a training-time-test step row t is wanted where its loss in some pass s < S (label and target row t + s, loss_mask[t + s])
+// or its run of correct passes (loss_mask[t]) counts; every other row only serves as context keys of pass 0.  The verifier's
+// row u is wanted where some wanted comparison reads it.  Block 0 lists the first, block 1 the second, ascending, as
+// index (row of the step -> row of the batch) and inverse (-1: not listed).  The count is rounded up to 256, so that no GEMM
+// or attention tile and no contraction step of 128 straddles it, by rows that nobody asked for (the last ones): they are
+// computed like any other and their gradients are exact zeros.
+constexpr int kKept = 16;  // rounds of which the flags stay in shared memory: 131072 rows
+__global__ void __launch_bounds__(kT)
+wanted_rows_kernel(const uint8_t* __restrict__ mask, int T, int S, int64_t* __restrict__ index, int* __restrict__ inverse, int* __restrict__ count) {
+  pdl_begin();
+  __shared__ int scratch[32], total, carry;
+  __shared__ uint8_t kept[kKept * kT];
+  const int dir = blockIdx.x == 0 ? 1 : -1, rounds = (T + kT * kPer - 1) / (kT * kPer);
+  index += (int64_t)blockIdx.x * T;
+  inverse += (int64_t)blockIdx.x * T;
+  auto wanted = [&](int round) {  // bit j: row i0 + j
+    const int i0 = (round * kT + threadIdx.x) * kPer;
+    unsigned bits = 0;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j)
+      for (int s = 0; s < S; ++s) {
+        const int u = i0 + j + dir * s;
+        if (i0 + j < T && u >= 0 && u < T && mask[u] != 0) bits |= 1u << j;
+      }
+    return bits;
+  };
+  int mine = 0;
+  for (int round = 0; round < rounds; ++round) {
+    const unsigned bits = wanted(round);
+    if (round < kKept) kept[round * kT + threadIdx.x] = (uint8_t)bits;
+    mine += __popc(bits);
+  }
+  const auto plus = [](int a, int b) { return a + b; };
+  const int up_to = block_scan(mine, plus, scratch);
+  if (threadIdx.x == kT - 1) total = up_to;
+  if (threadIdx.x == 0) carry = 0;
+  __syncthreads();
+  const int n = total, live = min(T, max(256, (n + 255) & ~255)), drop = T - live;  // the first `drop` unwanted rows stay out
+  for (int round = 0; round < rounds; ++round) {
+    const unsigned bits = round < kKept ? kept[round * kT + threadIdx.x] : wanted(round);
+    const int here = __popc(bits), from = carry, upto = rounds == 1 ? up_to : block_scan(here, plus, scratch);
+    int rank = from + upto - here;  // wanted rows before this one
+    const int i0 = (round * kT + threadIdx.x) * kPer;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+      const int i = i0 + j, unwanted = i - rank;
+      if (i >= T) break;
+      const bool want = bits >> j & 1, in = want || unwanted >= drop;
+      const int at = rank + max(0, unwanted - drop);
+      inverse[i] = in ? at : -1;
+      if (in) index[at] = i;
+      rank += want;
+    }
+    __syncthreads();
+    if (threadIdx.x == kT - 1) carry = from + upto;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) count[blockIdx.x] = live;
+}
+
+// What the passes read of the listed rows: ids, positions and label masks shifted by the pass, the verifier's listed row to
+// compare with (-1: none), the first run of correct passes, key intervals, and each later pass's own keys of the earlier ones.
+struct StepRows {
+  const uint8_t* mask;
+  const int64_t *ids, *positions;
+  const int* interval[2];  // [2, T] lo and hi (optional)
+  const int64_t* index;
+  const int *inverse, *count;  // of both lists
+  int T, S;
+  int64_t *ids_out, *positions_out;  // [S, T]
+  uint8_t *mask_out, *prev_out;      // [S, T], [T]
+  int* target_row;                   // [S, T]
+  int* interval_out[2];              // [2, T]
+  int* extra;                        // pass s from row T s (s - 1) / 2 on: [T, s]
+};
+__global__ void __launch_bounds__(256) step_rows_kernel(const StepRows p) {
+  pdl_begin();
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= p.T) return;
+  const bool on = i < p.count[0];
+  const int64_t t = on ? p.index[i] : 0;
+  p.prev_out[i] = on && p.mask[t] != 0;
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+    if (p.interval[k] != nullptr) {
+      p.interval_out[k][i] = on ? p.interval[k][t] : 0;
+      p.interval_out[k][p.T + i] = on ? p.interval[k][p.T + t] : 0;
+    }
+  for (int s = 0; s < p.S; ++s) {
+    const int64_t u = t + s, at = (int64_t)s * p.T + i;
+    const bool in = on && u < p.T;
+    p.ids_out[at] = in ? p.ids[u] : 0;
+    p.positions_out[at] = on ? p.positions[t] + s : 0;
+    p.mask_out[at] = in && p.mask[u] != 0;
+    p.target_row[at] = in ? p.inverse[p.T + u] : -1;
+    int* extra = p.extra + (int64_t)p.T * (s * (s - 1) / 2) + (int64_t)i * s;
+    for (int j = 0; j < s; ++j) extra[j] = on ? j * p.T + i : -1;
+  }
+}
+
+// Rows of up to two matrices at once (blockIdx.y), 16 bytes per thread.  Taken: out[r] = x[index[r]] for the rows in use.
+struct RowCopies {
+  const __nv_bfloat16* from[2];
+  int64_t stride[2];
+  __nv_bfloat16* to[2];
+  int W[2];
+  int rows;
+};
+__global__ void __launch_bounds__(256) take_rows_kernel(const RowCopies p, const int64_t* __restrict__ index, const int* __restrict__ live) {
+  pdl_begin();
+  const bool second = blockIdx.y != 0;
+  const __nv_bfloat16* x = second ? p.from[1] : p.from[0];
+  __nv_bfloat16* out = second ? p.to[1] : p.to[0];
+  const int64_t stride = second ? p.stride[1] : p.stride[0];
+  const int W = second ? p.W[1] : p.W[0], per = W >> 3;
+  const int64_t total = (int64_t)live_rows(live, p.rows) * per;
+  for (int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x; e < total; e += (int64_t)gridDim.x * 256) {
+    const int64_t r = e / per;
+    const int c = (int)(e - r * per) * 8;
+    st8(out + r * W + c, ld8(x + index[r] * stride + c));
+  }
+}
+// the way back: out[t] = d[inverse[t]], zero where the row was not taken
+__global__ void __launch_bounds__(256) put_rows_kernel(const RowCopies p, const int* __restrict__ inverse) {
+  pdl_begin();
+  const bool second = blockIdx.y != 0;
+  const __nv_bfloat16* d = second ? p.from[1] : p.from[0];
+  __nv_bfloat16* out = second ? p.to[1] : p.to[0];
+  const int64_t stride = second ? p.stride[1] : p.stride[0];
+  const int W = second ? p.W[1] : p.W[0], per = W >> 3;
+  const int64_t total = (int64_t)p.rows * per;
+  const float zero[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  for (int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x; e < total; e += (int64_t)gridDim.x * 256) {
+    const int64_t t = e / per;
+    const int c = (int)(e - t * per) * 8, from = inverse[t];
+    st8(out + t * W + c, from >= 0 ? ld8(d + (int64_t)from * stride + c) : pack8(zero));
+  }
 }
 
 // Gradient rows of an embedding from ids in ascending order (`order`: where each came from), summed in fp32 in a fixed order
@@ -301,6 +446,47 @@ void launch_peagle_spec(const int64_t* anchor, const int64_t* depth, const bool*
   }
   count_launch(1);
   launch_pdl(rows::peagle_spec_kernel, grid, 256, 0, stream, anchor, depth, row_valid, doc, doc_lo, n, T, num_depths, window, (const int*)table, lo, hi, extra);
+}
+void launch_step_rows(const uint8_t* mask, const int64_t* ids, const int64_t* positions, const int* const* interval, int T, int S, int64_t* index,
+                      int* inverse, int* count, int64_t* ids_out, int64_t* positions_out, uint8_t* mask_out, uint8_t* prev_out, int* target_row,
+                      int* const* interval_out, int* extra, cudaStream_t stream) {
+  if (T <= 0) return;
+  count_launch(2);
+  launch_pdl(rows::wanted_rows_kernel, 2, rows::kT, 0, stream, mask, T, S, index, inverse, count);
+  const rows::StepRows p{mask, ids, positions, {interval[0], interval[1]}, index, inverse, count, T, S, ids_out, positions_out, mask_out, prev_out,
+                         target_row, {interval_out[0], interval_out[1]}, extra};
+  launch_pdl(rows::step_rows_kernel, (T + 255) / 256, 256, 0, stream, p);
+}
+static rows::RowCopies row_copies(int n, const void* const* from, const int64_t* stride, const int* W, void* const* to, int rows, dim3* grid) {
+  rows::RowCopies p{};
+  int64_t most = 0;
+  for (int i = 0; i < n; ++i) {
+    p.from[i] = (const __nv_bfloat16*)from[i];
+    p.stride[i] = stride[i];
+    p.to[i] = (__nv_bfloat16*)to[i];
+    p.W[i] = W[i];
+    const int64_t blocks = ((int64_t)rows * (W[i] >> 3) + 255) / 256;
+    most = blocks > most ? blocks : most;
+  }
+  p.rows = rows;
+  *grid = dim3((unsigned)(most < 16 * kNumSM ? (most > 0 ? most : 1) : 16 * kNumSM), n);
+  return p;
+}
+// n: 1 or 2 matrices of the same rows
+void launch_take_rows(int n, const void* const* x, const int64_t* stride, const int* W, void* const* out, const int64_t* index, const int* live, int rows,
+                      cudaStream_t stream) {
+  if (rows <= 0) return;
+  dim3 grid;
+  const rows::RowCopies p = row_copies(n, x, stride, W, out, rows, &grid);
+  count_launch(1);
+  launch_pdl(rows::take_rows_kernel, grid, 256, 0, stream, p, index, live);
+}
+void launch_put_rows(int n, const void* const* d, const int64_t* stride, const int* W, void* const* out, const int* inverse, int rows, cudaStream_t stream) {
+  if (rows <= 0) return;
+  dim3 grid;
+  const rows::RowCopies p = row_copies(n, d, stride, W, out, rows, &grid);
+  count_launch(1);
+  launch_pdl(rows::put_rows_kernel, grid, 256, 0, stream, p, inverse);
 }
 int embedding_bwd_partial_rows(int n) { return n > rows::kSlice ? ((n - 1) / rows::kSlice + 1) * 2 : 0; }
 void launch_embedding_bwd(const int64_t* ids, const int64_t* order, const void* d, int64_t d_stride, int n, int H, int64_t vocab, int64_t padding, void* dw,

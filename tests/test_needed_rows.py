@@ -1,0 +1,215 @@
+"""EAGLE-3 steps over the rows that a loss term or counter reads: the plan, the kernels that stop at a device-side row count,
+and the whole pass against the pass over all rows."""
+
+import copy
+
+import pytest
+import torch
+
+from conftest import make_tiny_batch, make_tiny_eagle3
+
+import speculators_b200 as sb
+from speculators_b200 import ops
+from speculators_b200.layer_config import TransformerLayerConfig
+from speculators_b200.models.eagle3 import Eagle3DraftModel, Eagle3SpeculatorConfig
+from speculators_b200.models.eagle3.attention import causal_document_interval
+
+
+def _mask(kind: str, T: int, device="cpu") -> torch.Tensor:
+    g = torch.Generator().manual_seed(T)
+    m = torch.zeros(T, dtype=torch.bool)
+    if kind == "spans":
+        m = (torch.rand((T + 31) // 32, generator=g) < 0.5).repeat_interleave(32)[:T]
+    elif kind == "scattered":
+        m = torch.rand(T, generator=g) < 0.2
+    elif kind == "all":
+        m[:] = True
+    elif kind == "ends":
+        m[0] = m[-1] = True
+    return m.to(device)
+
+
+KINDS = ["spans", "scattered", "all", "none", "ends"]
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("layers", [1, 2])
+def test_pass_over_needed_rows_equals_the_whole_pass(tiny_verifier_dir, tiny_vocab_maps, monkeypatch, kind, layers):
+    model = make_tiny_eagle3(tiny_verifier_dir, tiny_vocab_maps, num_layers=layers)
+    kwargs, _ = sb.Eagle3DraftModel.get_trainer_kwargs(loss_fn="kl_div", ttt_steps=3, ttt_step_loss_decay=0.8)
+    batch = make_tiny_batch()
+    batch["loss_mask"] = _mask(kind, batch["loss_mask"].shape[1])[None]
+    results = []
+    for needed in (False, True):
+        monkeypatch.setattr(Eagle3DraftModel, "_takes_needed_rows", lambda *_, n=needed: n)
+        model.zero_grad()
+        _, loss, metrics = model(**batch, **kwargs)
+        loss.backward()
+        results.append((metrics, {n: p.grad.clone() for n, p in model.named_parameters() if p.grad is not None}))
+    (metrics, grads), (metrics_needed, grads_needed) = results
+    assert metrics.keys() == metrics_needed.keys() and grads.keys() == grads_needed.keys()
+    for k, v in metrics.items():
+        torch.testing.assert_close(metrics_needed[k], v, rtol=1e-5, atol=1e-6, msg=k)
+    for n, v in grads.items():
+        torch.testing.assert_close(grads_needed[n], v, rtol=1e-4, atol=1e-5 * float(v.abs().max()) + 1e-9, msg=n)
+
+
+# --------------------------------------------------------------------------- on a GPU
+@pytest.mark.gpu
+@pytest.mark.parametrize("T", [1, 255, 256, 257, 1000, 1024, 8192, 8200, 20011])
+@pytest.mark.parametrize("kind", KINDS)
+def test_plan(T, kind):
+    S = 3
+    g = torch.Generator().manual_seed(0)
+    doc = torch.arange(T) // 300
+    doc[T - T // 50 :] = -1
+    mask, ids, pos = _mask(kind, T), torch.randint(0, 1000, (T,), generator=g), torch.arange(T) % 300
+    iv = causal_document_interval(doc, 64)
+    full = causal_document_interval(doc, None)
+    ref = ops.step_rows(mask, ids, pos, [iv, full], S)
+    got = ops.step_rows(mask.cuda(), ids.cuda(), pos.cuda(), [tuple(t.cuda() for t in iv), causal_document_interval(doc.cuda(), None)], S)
+    for index, live, ref_index, ref_live in ((got.index, got.live, ref.index, ref.live), (got.target_index, got.target_live, ref.target_index, ref.target_live)):
+        n, want = int(live), int(ref_live)
+        assert n == min(T, max(256, -(-want // 256) * 256))
+        rows = index[:n].cpu()
+        assert (rows[1:] > rows[:-1]).all() and set(ref_index[:want].tolist()) <= set(rows.tolist())
+    n = int(got.live)
+    rows = got.index[:n].cpu()
+    inverse = torch.full((T,), -1, dtype=torch.int32)
+    inverse[rows] = torch.arange(n, dtype=torch.int32)
+    assert torch.equal(got.inverse.cpu(), inverse)
+    target_rows = got.target_index[: int(got.target_live)].cpu()
+    target_inverse = torch.full((T + S,), -1, dtype=torch.int32)
+    target_inverse[target_rows] = torch.arange(len(target_rows), dtype=torch.int32)
+    assert torch.equal(got.prev_correct.cpu(), torch.cat([mask[rows], torch.zeros(T - n, dtype=torch.bool)]))
+    for (lo, hi), (want_lo, want_hi) in zip(got.intervals, (iv, full)):
+        assert torch.equal(lo[:n].cpu(), want_lo[rows]) and torch.equal(hi[:n].cpu(), want_hi[rows]) and not lo[n:].any() and not hi[n:].any()
+    padded_mask, padded_ids = torch.cat([mask, mask.new_zeros(S)]), torch.cat([ids, ids.new_zeros(S)])
+    for s in range(S):
+        assert torch.equal(got.ids[s, :n].cpu(), padded_ids[rows + s]) and not got.ids[s, n:].any()
+        assert torch.equal(got.positions[s, :n].cpu(), pos[rows] + s)
+        assert torch.equal(got.mask[s, :n].cpu(), padded_mask[rows + s]) and not got.mask[s, n:].any()
+        assert torch.equal(got.target_row[s, :n].cpu(), target_inverse[rows + s]) and (got.target_row[s, n:] == -1).all()
+        wanted = padded_mask[rows + s] | mask[rows] & (rows + s < T)
+        assert (got.target_row[s, :n].cpu()[wanted] >= 0).all()
+        if s:
+            want = torch.arange(s)[None, :] * T + torch.arange(n)[:, None]
+            assert torch.equal(got.extra[s][:n].cpu().long(), want) and (got.extra[s][n:] == -1).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("variant", [0, 3, 4, 5, 10, 11, 12, 13])
+@pytest.mark.parametrize("live", [256, 768, 1001])
+def test_products_stop_at_the_count(variant, live):
+    """Rows behind hold NaN: neither read (weight gradient, which sums over them) nor written."""
+    T, M, N = 1001, 384, 1032
+    g = torch.Generator(device="cuda").manual_seed(variant * 7 + live)
+    a = torch.randn(T, M, generator=g, device="cuda").bfloat16()
+    w = torch.randn(N, M, generator=g, device="cuda").bfloat16()
+    dy = torch.randn(T, N, generator=g, device="cuda").bfloat16()
+    a[live:], dy[live:] = float("nan"), float("nan")
+    count, status = torch.tensor([live], dtype=torch.int32, device="cuda"), ops.gemm_status(a.device)
+    res = torch.randn(T, N, generator=g, device="cuda").bfloat16()
+    out, summed, dx = (torch.full((T, k), 7.0, dtype=torch.bfloat16, device="cuda") for k in (N, N, M))
+    dw = torch.full((N, M), 7.0, dtype=torch.bfloat16, device="cuda")
+    ops.native().gemm_tn_variant(a, w, out, None, 0, status, variant, count)
+    ops.native().gemm_tn_variant(a, w, summed, res, 2, status, variant, count)
+    ops.native().gemm_variant(dy, w, dx, 0, False, True, status, variant, count)
+    ops.native().gemm_variant(dy, a, dw, 0, True, True, status, variant, count)
+    af, wf, df = a[:live].float(), w.float(), dy[:live].float()
+    for got, want in ((out[:live], af @ wf.T), (summed[:live], af @ wf.T + res[:live].float()), (dx[:live], df @ wf), (dw, df.T @ af)):
+        assert float((got.float() - want).norm() / want.norm()) < 4e-3  # one rounding to bf16 (2^-9 at most, relative)
+    for t in (out, summed, dx):
+        assert (t[live:] == 7.0).all()
+    assert int(status) == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lives", [(256, 512, None), (None, 256, 768), (1001, 1001, 256)])
+def test_weight_gradient_parts_stop_at_their_counts(lives):
+    T, M, N = 1001, 2560, 2048
+    g = torch.Generator(device="cuda").manual_seed(1)
+    dys, xs, counts, want = [], [], [], 0
+    for live in lives:
+        dy, x = (torch.randn(T, k, generator=g, device="cuda").bfloat16() for k in (M, N))
+        n = T if live is None else live
+        dy[n:], x[n:] = float("nan"), float("nan")
+        want = want + dy[:n].float().T @ x[:n].float()
+        dys.append(dy), xs.append(x)
+        counts.append(torch.empty(0, dtype=torch.int32, device="cuda") if live is None else torch.tensor([live], dtype=torch.int32, device="cuda"))
+    dw = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+    status = ops.gemm_status(dw.device)
+    ops.native().gemm_wgrad_parts_rows(dys, xs, dw, False, status, counts)
+    assert float((dw.float() - want).norm() / want.norm()) < 4e-3 and int(status) == 0
+
+
+def _model(layers, head_dim, qwen, inter, window):
+    cfg = dict(architectures=["Qwen3ForCausalLM" if qwen else "LlamaForCausalLM"], model_type="qwen3" if qwen else "llama", hidden_size=256, num_hidden_layers=layers,
+               num_attention_heads=4, num_key_value_heads=2, head_dim=head_dim, intermediate_size=inter, vocab_size=1024, rms_norm_eps=1e-5, rope_theta=10000.0,
+               max_position_embeddings=4096, hidden_act="silu")
+    if window:
+        cfg.update(sliding_window=200, layer_types=["sliding_attention"] + ["full_attention"] * (layers - 1))
+    torch.manual_seed(0)
+    model = Eagle3DraftModel(Eagle3SpeculatorConfig(transformer_layer_config=TransformerLayerConfig(**cfg), draft_vocab_size=512, norm_before_residual=bool(window),
+                                                    norm_before_fc=True, norm_output=qwen, eagle_aux_hidden_state_layer_ids=[2, 5, 8]))
+    model.load_verifier_weights()
+    with torch.no_grad():
+        model.embed_tokens.weight.normal_(0.0, 1.0)
+        model.lm_head.weight.normal_(0.0, 0.1)
+        model.verifier_lm_head.weight.copy_(model.lm_head.weight)
+    kept = torch.arange(512) * 2
+    t2d = torch.zeros(1024, dtype=torch.bool)
+    t2d[kept] = True
+    model.load_vocab_mappings(t2d, kept - torch.arange(512))
+    return model.cuda().bfloat16()
+
+
+def _gpu_batch(T, kind):
+    g = torch.Generator().manual_seed(T)
+    doc = torch.arange(T) // max(1, T // 3)
+    doc[T - 17 :] = -1
+    mask = _mask(kind, T)
+    mask[T - 17 :] = False
+    return {"input_ids": torch.randint(0, 1024, (1, T), generator=g).cuda(), "hidden_states": torch.randn(1, T, 768, generator=g).bfloat16().cuda(),
+            "verifier_last_hidden_states": torch.randn(1, T, 256, generator=g).bfloat16().cuda(), "document_ids": doc[None].cuda(),
+            "loss_mask": mask[None].cuda(), "position_ids": (torch.arange(T) % 400)[None].cuda()}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T", [513, 777, 1536])
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("layers,head_dim,qwen,inter,window", [(1, 64, False, 688, True), (1, 128, True, 512, True), (2, 128, False, 512, False), (1, 256, True, 512, False)])
+def test_gpu_pass_over_needed_rows(monkeypatch, T, kind, layers, head_dim, qwen, inter, window):
+    model, batch = _model(layers, head_dim, qwen, inter, window), _gpu_batch(T, kind)
+    kwargs, _ = Eagle3DraftModel.get_trainer_kwargs(loss_fn="kl_div", ttt_steps=3, ttt_step_loss_decay=0.8)
+    results = []
+    for needed in (False, True):
+        monkeypatch.setattr(Eagle3DraftModel, "_takes_needed_rows", lambda *_, n=needed: n)
+        for p in model.parameters():
+            p.grad = None
+        poison = [torch.full((1 << 27,), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(4)]
+        del poison  # what the pass allocates and does not write holds NaN
+        _, loss, metrics = model(**batch, **kwargs)
+        loss.backward()
+        results.append(({k: v.float().cpu() for k, v in metrics.items()}, {n: p.grad.float() for n, p in model.named_parameters() if p.grad is not None}))
+    (metrics, grads), (metrics_needed, grads_needed) = results
+    assert metrics.keys() == metrics_needed.keys() and grads.keys() == grads_needed.keys()
+    for k, v in metrics.items():  # the same bits per row; fp32 sums in another order
+        torch.testing.assert_close(metrics_needed[k], v, rtol=2e-4, atol=1e-6, msg=k)
+    for n, v in grads.items():
+        # gradients round to bf16 (2^-9) on the way and at the end; sums over rows and queries take another order in between
+        assert torch.isfinite(grads_needed[n]).all(), n
+        assert float((grads_needed[n] - v).norm()) <= 1e-2 * float(v.norm()) + 1e-12, (n, float((grads_needed[n] - v).norm() / v.norm()))
+    ops.check_gemm_status()
+
+
+@pytest.mark.gpu
+def test_gpu_what_is_not_one_fused_loss_takes_all_rows():
+    model, batch = _model(1, 64, False, 512, False), _gpu_batch(777, "spans")
+    for loss_fn, implementation, want in (("kl_div", "fused", True), ("ce", "fused", True), ("kl_div", "eager", False), ('{"ce": 0.5, "tv": 0.5}', "fused", False), ("nla", "fused", False)):
+        kwargs, _ = Eagle3DraftModel.get_trainer_kwargs(loss_fn=loss_fn, loss_implementation=implementation, ttt_steps=2, ttt_step_loss_decay=1.0)
+        assert model._takes_needed_rows(2100, batch["loss_mask"], kwargs["loss_config"], 2) is want, loss_fn
+    assert not model._takes_needed_rows(2100, None, None, 2) and not model._takes_needed_rows(2047, batch["loss_mask"], None, 2)
+    tokens, loss, _ = model(**batch, ttt_steps=2)  # draft tokens of every row
+    assert len(tokens) == 2 and tokens[0].shape == (1, 777)
+    assert not copy.deepcopy(model).float()._takes_needed_rows(2100, batch["loss_mask"], None, 2)
