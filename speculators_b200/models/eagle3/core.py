@@ -35,20 +35,12 @@ from speculators_b200.model import DraftVocabMixin, SpeculatorModel
 from speculators_b200.models.eagle3.attention import causal_document_interval, ttt_attn_spec
 from speculators_b200.models.eagle3.config import Eagle3SpeculatorConfig
 from speculators_b200.models.eagle3.metrics import compute_metrics, compute_metrics_from_hidden, compute_metrics_of_rows, step_tail_is_fused
-from speculators_b200.models.layers import MLP, Attention, DecoderLayer, Linear, RMSNorm, RotaryTable
+from speculators_b200.models.layers import MLP, NEEDED_ROWS_FROM, Attention, DecoderLayer, Linear, RMSNorm, RotaryTable, takes_listed_rows
 from speculators_b200.models.utils import resolve_target_layer_ids
 from speculators_b200.ops import AttnSpec
 from speculators_b200.proposals.greedy import GreedyTokenProposalConfig
 
 __all__ = ["Eagle3DraftModel", "Eagle3FirstLayer"]
-
-# Rows x width from which on a step leaves out rows that nothing reads.  Listing them and copying queries and residuals costs
-# four launches (20 us of a step); ms a step with all rows and with the needed ones, half of the rows supervised in spans of 64:
-#   width 256:  513 rows 0.555 and 0.580, 1500 rows 0.723 and 0.731, 2048 rows 0.949 and 0.917, 4096 rows 1.200 and 1.129
-#   width 1024: 257 rows 1.134 and 1.136, 513 rows 1.351 and 1.345, 1500 rows 2.051 and 1.873
-#   width 4096: 257 rows 4.54 and 4.14, 800 rows 7.15 and 5.77, 1500 rows 10.77 and 8.14
-# A batch that is supervised throughout pays 1 to 2 % at any of these sizes.
-_NEEDED_ROWS_FROM = 1 << 19
 
 
 class Eagle3FirstLayer(nn.Module):
@@ -152,20 +144,13 @@ class Eagle3DraftModel(DraftVocabMixin, SpeculatorModel):
     def _takes_needed_rows(self, rows: int, loss_mask, loss_config, ttt_steps: int) -> bool:
         """Whether a step may leave out the rows that no loss term or counter reads (``ops.step_rows``): the loss and counters
         run as one fused tail over listed rows, and every operator in between is a kernel that stops at the count."""
-        if loss_mask is None or rows <= 256 or rows * self.hidden_size < _NEEDED_ROWS_FROM or ttt_steps <= 0 or not step_tail_is_fused(loss_config) or not ops.own_gemm_enabled() or ops.fused_head_enabled():
+        if loss_mask is None or rows <= 256 or rows * self.hidden_size < NEEDED_ROWS_FROM or ttt_steps <= 0 or not step_tail_is_fused(loss_config):
             return False
-        linears = [self.lm_head, self.verifier_lm_head]
-        for i, layer in enumerate(self.layers):
-            if type(layer) is not (DecoderLayer if i else Eagle3FirstLayer) or type(layer.self_attn) is not Attention or type(layer.mlp) is not MLP:
-                return False
-            linears += [layer.self_attn.qkv_proj, layer.self_attn.o_proj, layer.mlp.gate_up_proj, layer.mlp.down_proj]
-        attn = self.layers[0].self_attn
-        return (
-            all(p.is_cuda and p.dtype == torch.bfloat16 for p in (*self.layers.parameters(), self.norm.weight, self.verifier_norm.weight, *(m.weight for m in linears)))
-            and all(m.bias is None and getattr(m, "row_parallel", None) is None and m.weight.is_contiguous() and m.weight.data_ptr() % 16 == 0
-                    and m.weight.shape[0] % 8 == 0 and m.weight.shape[1] % 8 == 0 for m in linears)
-            and self.layers[0].mlp.hidden_act in ("silu", "swish") and attn.hd in (64, 128, 256) and attn.rot % 16 == 0 and self.hidden_size <= 32768
-        )
+        if not loss_mask.is_cuda or loss_mask.numel() != rows or ops.fused_head_enabled() or self.hidden_size > 32768:
+            return False
+        return (all(type(layer) is (DecoderLayer if i else Eagle3FirstLayer) for i, layer in enumerate(self.layers))
+                and takes_listed_rows(self.layers, self.lm_head, self.verifier_lm_head)
+                and all(n.weight.dtype == torch.bfloat16 for n in (self.norm, self.verifier_norm)))
 
     def _forward_needed_rows(self, hidden, verifier_hidden, ids, mask, positions, intervals, ttt_steps: int, decay: float, loss_config):
         """``forward`` over the rows that a loss term or counter reads (``ops.step_rows``); same loss, metrics and gradients.
@@ -176,7 +161,7 @@ class Eagle3DraftModel(DraftVocabMixin, SpeculatorModel):
         of the rows supervised: 8B, 2048 tokens 13.9 -> 11.7 ms, 8192 tokens 68.3 -> 52.2, validation of 5003 12.6 -> 8.2."""
         T = ids.shape[0]
         full_iv, win_iv = intervals
-        rows = ops.step_rows(mask, ids, positions, [iv for iv in intervals if iv is not None], ttt_steps)
+        rows = ops.step_rows(mask, ids.long(), positions, [iv for iv in intervals if iv is not None], ttt_steps)
         taken = iter(rows.intervals)
         taken_full, taken_win = (next(taken) if iv is not None else None for iv in intervals)
         with torch.no_grad():

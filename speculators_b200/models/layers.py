@@ -30,8 +30,10 @@ __all__ = [
     "FusedLinear",
     "Linear",
     "MLP",
+    "NEEDED_ROWS_FROM",
     "RMSNorm",
     "RotaryTable",
+    "takes_listed_rows",
 ]
 
 
@@ -323,6 +325,33 @@ class MLP(nn.Module):
             gate, up = gate_up.chunk(2, dim=-1)
             hidden = _GATE_ACTIVATIONS[self.hidden_act](gate) * up
         return self.down_proj(hidden, residual=residual, live=live)
+
+
+# Rows x width from which on an EAGLE-3 or MTP step leaves out rows that nothing reads.  Listing them and copying queries and residuals costs
+# four launches (20 us of a step); ms a step with all rows and with the needed ones, half of the rows supervised in spans of 64:
+#   width 256:  513 rows 0.555 and 0.580, 1500 rows 0.723 and 0.731, 2048 rows 0.949 and 0.917, 4096 rows 1.200 and 1.129
+#   width 1024: 257 rows 1.134 and 1.136, 513 rows 1.351 and 1.345, 1500 rows 2.051 and 1.873
+#   width 4096: 257 rows 4.54 and 4.14, 800 rows 7.15 and 5.77, 1500 rows 10.77 and 8.14
+# A batch that is supervised throughout pays 1 to 2 % at any of these sizes.
+NEEDED_ROWS_FROM = 1 << 19
+
+
+def takes_listed_rows(layers, *linears: nn.Module) -> bool:
+    """Whether decoder layers (``self_attn``, ``mlp``) and further linear layers may run over the rows that ``ops.step_rows``
+    lists: every operator between them is a kernel that stops at the device's row count."""
+    linears = list(linears)
+    for layer in layers:
+        attn, mlp = layer.self_attn, layer.mlp
+        if type(attn) is not Attention or type(mlp) is not MLP or mlp.hidden_act not in ("silu", "swish") or attn.hd not in (64, 128, 256) or attn.rot % 16:
+            return False
+        linears += [attn.qkv_proj, attn.o_proj, mlp.gate_up_proj, mlp.down_proj]
+    return (
+        ops.own_gemm_enabled()
+        and all(p.is_cuda and p.dtype == torch.bfloat16 for layer in layers for p in layer.parameters())
+        and all(getattr(m, "bias", None) is None and getattr(m, "row_parallel", None) is None and m.weight.is_cuda and m.weight.dtype == torch.bfloat16
+                and m.weight.is_contiguous() and m.weight.data_ptr() % 16 == 0 and m.weight.shape[0] % 8 == 0 and m.weight.shape[1] % 8 == 0
+                and m.weight.shape[1] <= 1 << 20 for m in linears)
+    )
 
 
 class DecoderLayer(nn.Module):

@@ -36,7 +36,7 @@ from torch import nn
 
 from speculators_b200 import ops
 from speculators_b200.layer_config import TransformerLayerConfig
-from speculators_b200.models.layers import FusedLinear, Linear, RotaryTable
+from speculators_b200.models.layers import FusedLinear, Linear, RotaryTable, takes_listed_rows
 from speculators_b200.models.mtp.model_definitions import _MTPMixin
 from speculators_b200.ops import AttnSpec
 from speculators_b200.ops.moe import moe_experts, moe_experts_ok
@@ -52,11 +52,11 @@ class ZeroCenteredRMSNorm(nn.Module):
         self.weight = nn.Parameter(torch.zeros(hidden_size))
         self.variance_epsilon = eps
 
-    def forward(self, x: torch.Tensor) -> torch.Tensor:
-        return ops.rms_norm(x, self.weight, self.variance_epsilon, centred=True)
+    def forward(self, x: torch.Tensor, live: torch.Tensor | None = None) -> torch.Tensor:
+        return ops.rms_norm(x, self.weight, self.variance_epsilon, centred=True, live=live)
 
-    def fork(self, x: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
-        return ops.rms_norm_fork(x, self.weight, self.variance_epsilon, centred=True)
+    def fork(self, x: torch.Tensor, live: torch.Tensor | None = None) -> tuple[torch.Tensor, torch.Tensor]:
+        return ops.rms_norm_fork(x, self.weight, self.variance_epsilon, centred=True, live=live)
 
 
 class GatedAttention(nn.Module):
@@ -74,8 +74,12 @@ class GatedAttention(nn.Module):
         self.q_norm = ZeroCenteredRMSNorm(self.hd, config.rms_norm_eps)
         self.k_norm = ZeroCenteredRMSNorm(self.hd, config.rms_norm_eps)
 
-    def forward(self, x, positions, rotary: RotaryTable, spec: AttnSpec, residual: torch.Tensor | None = None) -> torch.Tensor:
+    def forward(self, x, positions, rotary: RotaryTable, spec: AttnSpec, residual: torch.Tensor | None = None,
+                rows: ops.StepRows | None = None) -> torch.Tensor:
+        """``rows``: the inputs are of all rows, queries, ``spec`` and the result of those that ``ops.step_rows`` lists."""
         T = x.shape[0]
+        if rows is not None:
+            return self._listed_queries(x, positions, rotary, spec, residual, rows)
         qg = self.q_proj(x).view(T, self.nh, 2 * self.hd)
         split = ops.split_gated_query(qg, self.q_norm.weight, self.q_norm.variance_epsilon)
         if split is not None:
@@ -94,6 +98,18 @@ class GatedAttention(nn.Module):
         out = ops.masked_attention(q, k, v, spec, scale=self.scaling).reshape(T, self.nh * self.hd)
         return self.o_proj(out * torch.sigmoid(gate), residual=residual)
 
+    def _listed_queries(self, x, positions, rotary, spec, residual, rows: ops.StepRows) -> torch.Tensor:
+        T, live = x.shape[0], rows.live
+        k = self.k_norm(self.k_proj(x).view(T, self.nkv, self.hd))
+        k = ops.rope_(k, positions, rotary.cos, rotary.sin, self.nkv, self.hd, self.rot)
+        v = self.v_proj(x).view(T, self.nkv, self.hd)
+        x, residual = ops.take_rows(rows.index, rows.inverse, live, x, residual)
+        qg = self.q_proj(x, live=live).view(T, self.nh, 2 * self.hd)
+        q, gate = ops.split_gated_query(qg, self.q_norm.weight, self.q_norm.variance_epsilon, live * self.nh)
+        q = ops.rope_(q, rows.positions[0], rotary.cos, rotary.sin, self.nh, self.hd, self.rot)
+        out = ops.masked_attention(q, k, v, spec, scale=self.scaling)
+        return self.o_proj(ops.gated(out, gate).view(T, self.nh * self.hd), residual=residual, live=live)
+
 
 class _Experts(nn.Module):
     def __init__(self, num_local: int, hidden: int, inter: int):
@@ -111,11 +127,11 @@ class _SharedExpert(nn.Module):
         self.gate_up_proj = FusedLinear(hidden, ["gate_proj", "up_proj"], [inter, inter]).attach(self, "gate_up_proj")
         self.down_proj = Linear(inter, hidden)
 
-    def forward(self, x: torch.Tensor) -> torch.Tensor:
-        hidden = ops.linear_swiglu(x, self.gate_up_proj.weight)
+    def forward(self, x: torch.Tensor, live: torch.Tensor | None = None) -> torch.Tensor:
+        hidden = ops.linear_swiglu(x, self.gate_up_proj.weight, live)
         if hidden is None:
-            hidden = ops.swiglu(self.gate_up_proj(x))
-        return self.down_proj(hidden)
+            hidden = ops.swiglu(self.gate_up_proj(x, live), live)
+        return self.down_proj(hidden, live=live)
 
 
 def expert_forward(x: torch.Tensor, expert_ids: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor) -> torch.Tensor:
@@ -229,19 +245,20 @@ class SparseMoeBlock(nn.Module):
             if full is not None and full.shape[0] == self.num_experts and self.num_local != self.num_experts:
                 state_dict[key] = full[self.ep_rank * self.num_local : (self.ep_rank + 1) * self.num_local]
 
-    def route(self, x: torch.Tensor):
-        probs = torch.softmax(self.gate(x).float(), dim=-1)
+    def route(self, x: torch.Tensor, live: torch.Tensor | None = None):
+        logits = ops.only_live(self.gate(x, live=live), live)  # what nobody wrote must not choose an expert
+        probs = torch.softmax(logits.float(), dim=-1)
         top_p, top_e = torch.topk(probs, self.top_k, dim=-1)
         if self.norm_topk_prob:
             top_p = top_p / top_p.sum(dim=-1, keepdim=True)
         return top_p.to(x.dtype), top_e
 
-    def forward(self, x: torch.Tensor, residual: torch.Tensor | None = None) -> torch.Tensor:
-        """The block's output, plus ``residual`` when given."""
+    def forward(self, x: torch.Tensor, residual: torch.Tensor | None = None, live: torch.Tensor | None = None) -> torch.Tensor:
+        """The block's output, plus ``residual`` when given.  ``live`` (tokens in use): only where ``moe_experts_ok``."""
         if self.ep_size == 1 and moe_experts_ok(x, self.experts.gate_up_proj, self.experts.down_proj):
-            top_p, top_e = self.route(x)
-            shared, gate = (None, None) if self.shared_expert is None else (self.shared_expert(x), self.shared_expert_gate(x))
-            return moe_experts(x, top_p, top_e, self.experts.gate_up_proj, self.experts.down_proj, shared, gate, residual)
+            top_p, top_e = self.route(x, live)
+            shared, gate = (None, None) if self.shared_expert is None else (self.shared_expert(x, live), self.shared_expert_gate(x, live=live))
+            return moe_experts(x, top_p, top_e, self.experts.gate_up_proj, self.experts.down_proj, shared, gate, residual, live)
         out = self._sorted_forward(x)
         return out if residual is None else residual + out
 
@@ -355,11 +372,13 @@ class MoEDecoderLayer(nn.Module):
         self.input_layernorm = ZeroCenteredRMSNorm(H, eps)
         self.post_attention_layernorm = ZeroCenteredRMSNorm(H, eps)
 
-    def forward(self, x, positions, rotary, spec) -> torch.Tensor:
+    def forward(self, x, positions, rotary, spec, rows=None) -> torch.Tensor:
+        """``rows``: as in ``GatedAttention``."""
+        live = None if rows is None else rows.live
         normed, x = self.input_layernorm.fork(x)
-        x = self.self_attn(normed, positions, rotary, spec, residual=x)
-        normed, x = self.post_attention_layernorm.fork(x)
-        return self.mlp(normed, residual=x)
+        x = self.self_attn(normed, positions, rotary, spec, residual=x, rows=rows)
+        normed, x = self.post_attention_layernorm.fork(x, live)
+        return self.mlp(normed, residual=x, live=live)
 
 
 class MoEMTPLayer(_MTPMixin, MoEDecoderLayer):
@@ -370,6 +389,19 @@ class MoEMTPLayer(_MTPMixin, MoEDecoderLayer):
         MoEDecoderLayer.__init__(self, config, layer_idx, ep_group=ep_group)
         self._setup_mtp_modules(config, norm_cls=ZeroCenteredRMSNorm)
 
-    def forward(self, hidden_states, token_embeddings, positions, rotary, spec):
+    def takes_listed_rows(self) -> bool:
+        """Whether ``rows`` may be given: all experts on this rank, every operator a kernel that stops at the row count."""
+        attn, mlp = self.self_attn, self.mlp
+        linears = [attn.q_proj, attn.k_proj, attn.v_proj, attn.o_proj, mlp.gate]
+        if mlp.shared_expert is not None:
+            linears += [mlp.shared_expert.gate_up_proj, mlp.shared_expert.down_proj]
+            if mlp.shared_expert_gate.bias is not None:
+                return False
+        width = self.final_layernorm.weight.numel()
+        return (takes_listed_rows([], *linears) and all(p.dtype == torch.bfloat16 for p in self.parameters()) and attn.hd in (64, 128, 256) and attn.rot % 16 == 0
+                and width <= 32768 and mlp.ep_size == 1 and moe_experts_ok(mlp.gate.weight, mlp.experts.gate_up_proj, mlp.experts.down_proj))
+
+    def forward(self, hidden_states, token_embeddings, positions, rotary, spec, rows=None):
+        """``rows``: the inputs are of all rows, the result and ``spec`` of those that ``ops.step_rows`` lists."""
         x = self.combine(hidden_states, token_embeddings)
-        return self.final_layernorm(MoEDecoderLayer.forward(self, x, positions, rotary, spec))
+        return self.final_layernorm(MoEDecoderLayer.forward(self, x, positions, rotary, spec, rows), None if rows is None else rows.live)

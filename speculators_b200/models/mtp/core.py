@@ -20,7 +20,7 @@ from torch import nn
 from speculators_b200 import ops
 from speculators_b200.config import SpeculatorsConfig, VerifierConfig
 from speculators_b200.model import DraftVocabMixin, SpeculatorModel
-from speculators_b200.models.layers import RotaryTable
+from speculators_b200.models.layers import NEEDED_ROWS_FROM, RotaryTable, takes_listed_rows
 from speculators_b200.models.mtp.config import MTPSpeculatorConfig
 from speculators_b200.models.mtp.model_definitions import build_mtp_layer
 from speculators_b200.ops import AttnSpec
@@ -54,6 +54,8 @@ class MTPDraftModel(DraftVocabMixin, SpeculatorModel):
     _keys_to_ignore_on_save: ClassVar[list[str]] = ["embed_tokens.weight", "lm_head.weight", "verifier_lm_head.weight"]
     _keys_to_ignore_on_load_missing: ClassVar[list[str]] = ["embed_tokens.weight", "lm_head.weight", "verifier_lm_head.weight", "t2d", "d2t"]
     cuda_graph_safe: ClassVar[bool] = True
+    # what a caller adds that takes the loss and the metrics and leaves the logits (``Trainer``)
+    loss_only_kwargs: ClassVar[dict] = {"return_logits": False}
 
     def __init__(self, config: MTPSpeculatorConfig, ep_group=None):
         """``ep_group`` (mixture-of-experts heads only): split the experts over this process group
@@ -88,8 +90,14 @@ class MTPDraftModel(DraftVocabMixin, SpeculatorModel):
         if hasattr(self, "verifier_lm_head"):
             del self.verifier_lm_head  # MTP trains against token ids, not verifier logits
 
+    def _takes_needed_rows(self, rows: int, mask: torch.Tensor) -> bool:
+        return rows > 256 and rows * self.hidden_size >= NEEDED_ROWS_FROM and mask.is_cuda and takes_listed_rows([], self.lm_head)
+
     def forward(self, input_ids, hidden_states, attention_mask=None, position_ids=None, loss_mask=None,
-                step_weights: list[float] | None = None, return_dict: bool = True, **_: Any):
+                step_weights: list[float] | None = None, return_dict: bool = True, return_logits: bool = True, **_: Any):
+        """``return_logits=False``: the first result is an empty list, and rows without a label take part in no product whose
+        result the loss does not depend on - the head of every step, and the last step's queries, MLP and norms (60 % of the
+        rows with a label: 8B, 2000 tokens 22.2 -> 20.1 ms, 4096 tokens with 256 experts 30.5 -> 27.5)."""
         del attention_mask, return_dict
         ids = input_ids.reshape(-1).long()
         device = ids.device
@@ -113,23 +121,36 @@ class MTPDraftModel(DraftVocabMixin, SpeculatorModel):
             return all_logits, total, metrics
         pos = positions[:valid_len]
         idx = torch.arange(valid_len, device=device, dtype=torch.int32)
-        spec = AttnSpec(lo=torch.zeros_like(idx), hi=idx + 1)  # plain causal, as in the reference
+        interval = torch.stack([torch.zeros_like(idx), idx + 1])  # plain causal, as in the reference
+        spec = AttnSpec(lo=interval[0], hi=interval[1])
         current = hidden_states.reshape(T, -1).to(dtype)
         mask = loss_mask.reshape(-1) if loss_mask is not None else None
+        layer, rows = self.mtp_layers[0], None
+        if not return_logits and mask is not None and self._takes_needed_rows(valid_len, mask):
+            # row t is wanted where one of its labels, t + 2 and on, is in the mask
+            rows = ops.step_rows((mask != 0)[2:], ids[2:], pos, [(spec.lo, spec.hi)], steps, targets=False)
         for step in range(steps):
             with torch.no_grad():
                 emb = self.embed_tokens(ids[step + 1 : step + 1 + valid_len]).to(dtype)
-            out = self.mtp_layers[0](current[:valid_len], emb, pos, self.rotary_emb, spec)
-            logits = ops.linear(out, self.lm_head.weight)
-            all_logits.append(logits.unsqueeze(0))
-            labels = ids[step + 2 : step + 2 + valid_len]
-            keep = mask[step + 2 : step + 2 + valid_len] != 0 if mask is not None else torch.ones_like(labels, dtype=torch.bool)
-            per_row = ops.token_cross_entropy(logits, labels, keep)
+            if rows is not None and step + 1 == steps and getattr(layer, "takes_listed_rows", bool)():
+                lo, hi = rows.intervals[0]  # nothing reads the last step's states but its head
+                head_in = layer(current[:valid_len], emb, pos, self.rotary_emb, AttnSpec(lo=lo, hi=hi), rows=rows)
+            else:
+                current = layer(current[:valid_len], emb, pos, self.rotary_emb, spec)
+                head_in = current if rows is None else ops.take_rows(rows.index, rows.inverse, rows.live, current)[0]
+            if rows is None:
+                labels, live = ids[step + 2 : step + 2 + valid_len], None
+                keep = mask[step + 2 : step + 2 + valid_len] != 0 if mask is not None else torch.ones_like(labels, dtype=torch.bool)
+            else:
+                labels, keep, live = rows.ids[step], rows.mask[step], rows.live
+            logits = ops.linear(head_in, self.lm_head.weight, live=live)
+            if return_logits:
+                all_logits.append(logits.unsqueeze(0))
+            per_row = ops.token_cross_entropy(logits, labels, keep, live)
             weight = step_weights[step] if step_weights is not None else 1.0
             step_loss = weight * per_row.sum() / keep.sum().clamp(min=1)
             total = total + step_loss
             metrics[f"loss_step_{step}"] = step_loss.detach().clone()
-            current = out
         metrics["loss_sum"] = total.detach().clone()
         metrics["loss_total"] = torch.ones((), device=device)
         return all_logits, total, metrics

@@ -14,7 +14,7 @@ import torch
 from torch import nn
 
 from speculators_b200.layer_config import TransformerLayerConfig
-from speculators_b200.models.layers import DecoderLayer, Linear, RMSNorm
+from speculators_b200.models.layers import DecoderLayer, Linear, RMSNorm, takes_listed_rows
 
 __all__ = ["MTPLayer", "MTPLayerMixin", "build_mtp_layer", "mtp_model_classes", "resolve_model_type"]
 
@@ -47,9 +47,14 @@ class MTPLayer(_MTPMixin, DecoderLayer):
         DecoderLayer.__init__(self, config, layer_idx)
         self._setup_mtp_modules(config)
 
-    def forward(self, hidden_states, token_embeddings, positions, rotary, spec):
+    def takes_listed_rows(self) -> bool:
+        return takes_listed_rows([self])
+
+    def forward(self, hidden_states, token_embeddings, positions, rotary, spec, rows=None):
+        """``rows``: the inputs are of all rows, the result and ``spec`` of those that ``ops.step_rows`` lists."""
         x = self.combine(hidden_states, token_embeddings)
-        return self.final_layernorm(DecoderLayer.forward(self, x, positions, rotary, spec))
+        x = DecoderLayer.forward(self, x, positions, rotary, spec, rows=rows, dense=rows is not None)
+        return self.final_layernorm(x, None if rows is None else rows.live)
 
 
 MTPLayerMixin = _MTPMixin  # public name (src/speculators/models/mtp/model_definitions.py:73)

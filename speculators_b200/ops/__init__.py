@@ -52,6 +52,7 @@ __all__ = [
     "matmul_tn",
     "masked_attention_reference",
     "native",
+    "only_live",
     "norm_rope_heads",
     "repeat_rows",
     "rms_norm",
@@ -127,7 +128,8 @@ def check_gemm_status() -> None:
 
 # ``live`` (here and below): an int32 tensor on the device that says how many of the rows hold anything (``step_rows``).  The
 # kernels neither read nor write the rows behind; what runs elsewhere takes all rows, and a sum over rows leaves those out.
-def _without_unused(x2: torch.Tensor, live: torch.Tensor | None) -> torch.Tensor:
+def only_live(x2: torch.Tensor, live: torch.Tensor | None) -> torch.Tensor:
+    """``x2`` with zeros in the rows from ``live`` on."""
     if live is None:
         return x2
     used = torch.arange(x2.shape[0], device=x2.device) < live
@@ -448,7 +450,7 @@ def _linear_backward(x2, weight, rows, use, dy, need_dx: bool, need_dw: bool, li
     if need_dx:
         dx = _dgrad_gemm(dy2, w, live=live) if own else dy2 @ w
     if need_dw and not own:
-        dy2, x2 = _without_unused(dy2, live), _without_unused(x2, live)
+        dy2, x2 = only_live(dy2, live), only_live(x2, live)
     if need_dw:
         flat = getattr(weight, "_flat_grad", None)
         if flat is not None and own and _gemm_operand_ok(flat if r0 is None else flat[r0:r1]) and x2.shape[0] > 0:
@@ -464,7 +466,7 @@ def _linear_backward(x2, weight, rows, use, dy, need_dx: bool, need_dw: bool, li
         elif flat is not None:
             if use is not None:
                 use.left()
-            dy2, x2 = (_without_unused(t, live if own else None) for t in (dy2, x2))
+            dy2, x2 = (only_live(t, live if own else None) for t in (dy2, x2))
             target, accumulate = _param_grad_target(weight)[:2] if r0 is None else _row_grad_target(weight, r0, r1)
             if accumulate:
                 target.addmm_(dy2.t(), x2)
@@ -477,7 +479,7 @@ def _linear_backward(x2, weight, rows, use, dy, need_dx: bool, need_dw: bool, li
             if own and _gemm_operand_ok(dw[r0:r1]):
                 _wgrad_gemm(dy2, x2, dw[r0:r1], accumulate=False, live=live)
             else:
-                dy2, x2 = (_without_unused(t, live if own else None) for t in (dy2, x2))
+                dy2, x2 = (only_live(t, live if own else None) for t in (dy2, x2))
                 dw[r0:r1] = dy2.t() @ x2
     return dx, dw
 
@@ -944,25 +946,26 @@ class StepRows(NamedTuple):
     extra: list  # per pass: None, then int32 [T, pass]
 
 
-def step_rows(mask: torch.Tensor, ids: torch.Tensor, positions: torch.Tensor, intervals: list, passes: int) -> StepRows:
+def step_rows(mask: torch.Tensor, ids: torch.Tensor, positions: torch.Tensor, intervals: list, passes: int, targets: bool = True) -> StepRows:
     """Which rows of a packed batch the passes of a training-time-test step need, the batch in their order.
 
     Pass ``s`` compares row ``t`` with the verifier's row ``t + s`` where ``mask[t + s]`` is set, and follows the rows that
     were right in every pass from where ``mask[t]`` is.  A later pass sees a row's own keys of the passes before and nothing
     else of them, so a row that no comparison reads serves as context keys in pass 0 only.  ``mask`` bool / uint8 ``[T]``,
     ``intervals``: up to two key intervals ``(lo, hi)`` of the rows.  Rows are listed in ascending order; the count is a
-    multiple of 256 or all of them (on the CPU exact), filled up with rows that nobody asked for."""
-    T = ids.shape[0]
+    multiple of 256 or all of them (on the CPU exact), filled up with rows that nobody asked for.  Without ``targets`` (labels
+    instead of a verifier's rows) ``mask`` and ``ids`` may reach past the rows, of which there are as many as ``positions``."""
+    T, N = positions.shape[0], ids.shape[0]
     if _use_native(ids):
         both = [lo._base if lo._base is not None and lo._base is hi._base and lo._base.shape == (2, T) else torch.stack([lo, hi]) for lo, hi in intervals]
-        index, inverse, count, ids, positions, mask, prev, target_row, spans, extra = native().step_rows(mask.contiguous(), ids, positions, both, passes)
+        index, inverse, count, ids, positions, mask, prev, target_row, spans, extra = native().step_rows(mask.contiguous(), ids.contiguous(), positions.contiguous(), both, passes, targets)
         offsets = [T * s * (s - 1) // 2 for s in range(passes)]
         extra = [None] + [extra.view(-1)[offsets[s] : offsets[s] + T * s].view(T, s) for s in range(1, passes)]
         return StepRows(index[0], inverse[0], count[:1], index[1], count[1:], ids, positions, mask, prev, target_row, [(s[0], s[1]) for s in spans], extra)
     m = torch.cat([mask.bool(), torch.zeros(passes, dtype=torch.bool)])
     lists = []
     for wanted in (torch.stack([m[s : s + T] for s in range(passes)]).any(0),
-                   torch.stack([torch.cat([torch.zeros(s, dtype=torch.bool), m[: T - s]]) for s in range(passes) if s < T]).any(0)):
+                   torch.stack([torch.cat([torch.zeros(s, dtype=torch.bool), m[: T - s]]) for s in range(passes) if s < T]).any(0) & targets):
         at = wanted.nonzero().view(-1)
         inverse = torch.full((T,), -1, dtype=torch.int32)
         inverse[at] = torch.arange(at.numel(), dtype=torch.int32)
@@ -970,13 +973,13 @@ def step_rows(mask: torch.Tensor, ids: torch.Tensor, positions: torch.Tensor, in
     (index, inverse, live), (target_index, target_inverse, target_live) = lists
     on = torch.arange(T) < live
     u = index + torch.arange(passes)[:, None]
-    there = on & (u < T)
-    u = u.clamp(max=T - 1)
+    there = on & (u < N)
+    u = u.clamp(max=N - 1)
     zero = torch.zeros((), dtype=torch.long)
     extra = [None] + [torch.where(on[:, None], torch.arange(s, dtype=torch.int32) * T + torch.arange(T, dtype=torch.int32)[:, None], -1) for s in range(1, passes)]
     return StepRows(index, inverse, live, target_index, target_live, torch.where(there, ids[u], zero),
                     torch.where(on, positions[index] + torch.arange(passes)[:, None], zero), there & m[u], on & m[index],
-                    torch.where(there, target_inverse[u], -1), [tuple(torch.where(on, v[index], 0) for v in pair) for pair in intervals], extra)
+                    torch.where(there, target_inverse[u.clamp(max=T - 1)], -1), [tuple(torch.where(on, v[index], 0) for v in pair) for pair in intervals], extra)
 
 
 class _TakeRowsFn(torch.autograd.Function):
@@ -999,7 +1002,7 @@ def take_rows(index: torch.Tensor, inverse: torch.Tensor, live: torch.Tensor, *x
     (zero on the CPU).  The gradient is a row copy, zero where a row was not taken."""
     if _use_native(index):
         return _TakeRowsFn.apply(index, inverse, live, *(_grad_rows(x, x.shape[1]) for x in xs))
-    return tuple(_without_unused(x[index], live) for x in xs)
+    return tuple(only_live(x[index], live) for x in xs)
 
 
 def rms_norm_taken(x: torch.Tensor, weight: torch.Tensor, eps: float, index: torch.Tensor, live: torch.Tensor) -> torch.Tensor:
@@ -1008,7 +1011,7 @@ def rms_norm_taken(x: torch.Tensor, weight: torch.Tensor, eps: float, index: tor
         y = torch.empty((index.shape[0], x.shape[1]), dtype=x.dtype, device=x.device)
         native().norm_fwd(_grad_rows(x, x.shape[1]), weight, index, y, None, eps, False, live)
         return y
-    return rms_norm(_without_unused(x[index], live), weight, eps)
+    return rms_norm(only_live(x[index], live), weight, eps)
 
 
 # --------------------------------------------------------------------------- repeated rows, embedding
@@ -1076,19 +1079,19 @@ class _SplitGatedQueryFn(torch.autograd.Function):
     ``[T, heads, 2 * hd]`` buffer, into the other half of which ``_GatedFn`` has put the gate's gradient."""
 
     @staticmethod
-    def forward(ctx, qg, weight, eps):
+    def forward(ctx, qg, weight, eps, live):
         T, heads, two = qg.shape
         hd = two // 2
         x2 = qg.view(T * heads, two)[:, :hd]
         q = torch.empty((T, heads, hd), dtype=qg.dtype, device=qg.device)
         rstd = torch.empty(T * heads, dtype=torch.float32, device=qg.device)
-        native().norm_fwd(x2, weight, None, q.view(T * heads, hd), rstd, eps, True)
-        ctx.save_for_backward(qg, weight, rstd)
+        native().norm_fwd(x2, weight, None, q.view(T * heads, hd), rstd, eps, True, live)
+        ctx.save_for_backward(qg, weight, rstd, live)
         return q, qg[..., hd:]
 
     @staticmethod
     def backward(ctx, dq, dgate):
-        qg, weight, rstd = ctx.saved_tensors
+        qg, weight, rstd, live = ctx.saved_tensors
         T, heads, two = qg.shape
         hd = two // 2
         in_place = (dgate.dtype == qg.dtype and dgate.stride() == (heads * two, two, 1) and dgate.storage_offset() == hd
@@ -1100,8 +1103,8 @@ class _SplitGatedQueryFn(torch.autograd.Function):
             d[..., hd:] = dgate
         rows = T * heads
         dw, accumulate, attached = _param_grad_target(weight) if ctx.needs_input_grad[1] else (None, False, False)
-        native().rmsnorm_bwd(_grad_rows(dq, hd), None, qg.view(rows, two)[:, :hd], weight, rstd, None, d.view(rows, two)[:, :hd], dw, accumulate, True)
-        return d, None if attached else dw, None
+        native().rmsnorm_bwd(_grad_rows(dq, hd), None, qg.view(rows, two)[:, :hd], weight, rstd, None, d.view(rows, two)[:, :hd], dw, accumulate, True, live)
+        return d, None if attached else dw, None, None
 
 
 class _GatedFn(torch.autograd.Function):
@@ -1118,12 +1121,12 @@ class _GatedFn(torch.autograd.Function):
         return native().gate_mul_bwd(dy.contiguous(), out, gate, dgate), dgate
 
 
-def split_gated_query(qg: torch.Tensor, weight: torch.Tensor, eps: float):
+def split_gated_query(qg: torch.Tensor, weight: torch.Tensor, eps: float, live: torch.Tensor | None = None):
     """Query and gate of a gated attention from the ``[T, heads, 2 * hd]`` projection: the query normalised with a zero-centred
-    weight, the gate as a view.  ``None`` where the kernels do not take the tensor and the caller runs the steps one by one."""
+    weight, the gate as a view (``live``: heads in use, of all tokens).  ``None`` where the kernels do not take the tensor and the caller runs the steps one by one."""
     if not (_norm_native(qg) and qg.is_contiguous() and qg.shape[-1] % 16 == 0):
         return None
-    return _SplitGatedQueryFn.apply(qg, weight, eps)
+    return _SplitGatedQueryFn.apply(qg, weight, eps, live)
 
 
 def gated(out: torch.Tensor, gate: torch.Tensor) -> torch.Tensor:
@@ -1362,27 +1365,27 @@ def fused_row_loss(op: str, logits, targets, shift: int = 0, rows: int | None = 
 
 class _TokenCEFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, logits, labels, keep):
+    def forward(ctx, logits, labels, keep, live):
         loss, stats = native().ce_label_fwd(logits, labels, keep)
-        ctx.save_for_backward(logits, stats)
+        ctx.save_for_backward(logits, stats, live)
         return loss
 
     @staticmethod
     def backward(ctx, dloss):
-        logits, stats = ctx.saved_tensors
+        logits, stats, live = ctx.saved_tensors
         # the CE backward only needs the saved label (stats[4]) and the draft statistics
-        d = native().loss_bwd(LOSS_OPS["ce"], logits, logits, dloss.contiguous().float(), stats, 0, logits.shape[0])
-        return d, None, None
+        d = native().loss_bwd_scaled(LOSS_OPS["ce"], logits, logits, dloss.contiguous().float(), None, stats, 0, logits.shape[0], None, live)
+        return d, None, None, None
 
 
-def token_cross_entropy(logits: torch.Tensor, labels: torch.Tensor, keep: torch.Tensor | None = None) -> torch.Tensor:
+def token_cross_entropy(logits: torch.Tensor, labels: torch.Tensor, keep: torch.Tensor | None = None, live: torch.Tensor | None = None) -> torch.Tensor:
     """Per-row cross-entropy of ``logits [n, V]`` against integer ``labels [n]``;
-    rows with ``keep == False`` contribute 0 (and no gradient)."""
+    rows with ``keep == False`` contribute 0 (and no gradient).  ``live``: see ``step_rows``; no row behind it is kept."""
     if _use_native(logits):
         if logits.stride(-1) != 1:
             logits = logits.contiguous()
         keep_b = keep.to(torch.bool).contiguous() if keep is not None else None
-        return _TokenCEFn.apply(logits, labels.long().contiguous(), keep_b)
+        return _TokenCEFn.apply(logits, labels.long().contiguous(), keep_b, live)
     loss = F.cross_entropy(logits.float(), labels.long(), reduction="none")
     return loss if keep is None else torch.where(keep.bool(), loss, torch.zeros_like(loss))
 

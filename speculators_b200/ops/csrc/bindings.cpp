@@ -33,7 +33,7 @@ void launch_document_interval(const int64_t*, int, int, int*, int*, cudaStream_t
 void launch_compact(const bool*, int, int64_t*, int*, cudaStream_t);
 void launch_cod_step(const int64_t*, const int64_t*, int, const bool*, int, int, int, unsigned char*, int64_t*, int64_t*, int64_t*, int64_t*, int*, cudaStream_t);
 void launch_peagle_spec(const int64_t*, const int64_t*, const bool*, const int64_t*, const int*, int, int, int, int, int*, int*, int*, int*, cudaStream_t);
-void launch_step_rows(const uint8_t*, const int64_t*, const int64_t*, const int* const*, int, int, int64_t*, int*, int*, int64_t*, int64_t*, uint8_t*, uint8_t*,
+void launch_step_rows(const uint8_t*, const int64_t*, const int64_t*, const int* const*, int, int, int, int64_t*, int*, int*, int64_t*, int64_t*, uint8_t*, uint8_t*,
                       int*, int* const*, int*, cudaStream_t);
 void launch_take_rows(int, const void* const*, const int64_t*, const int*, void* const*, const int64_t*, const int*, int, cudaStream_t);
 void launch_put_rows(int, const void* const*, const int64_t*, const int*, void* const*, const int*, int, cudaStream_t);
@@ -46,12 +46,12 @@ void launch_rope_merge(const void* const*, const int64_t*, const int*, const int
 void launch_gate_mul_fwd(const void*, const void*, void*, int, int, int, int64_t, int, cudaStream_t);
 void launch_gate_mul_bwd(const void*, const void*, const void*, void*, void*, int, int, int, int64_t, int, int64_t, cudaStream_t);
 int moe_plan_blocks(int);
-int launch_moe_plan(const int64_t*, int, int, int, int*, int*, int*, int*, int*, cudaStream_t);
+int launch_moe_plan(const int64_t*, int, int, int, int*, int*, int*, int*, int*, const int*, int, cudaStream_t);
 void launch_moe_gather(const void*, int64_t, const int*, const int*, int, void*, int, int, cudaStream_t);
-void launch_moe_gather_bwd(const void*, const int*, int, void*, int, int, cudaStream_t);
-void launch_moe_combine(const void*, const int*, const void*, int, const void*, const void*, const void*, void*, int, int, cudaStream_t);
+void launch_moe_gather_bwd(const void*, const int*, int, void*, int, int, const int*, cudaStream_t);
+void launch_moe_combine(const void*, const int*, const void*, int, const void*, const void*, const void*, void*, int, int, const int*, cudaStream_t);
 void launch_moe_combine_bwd(const void*, const void*, const int*, const int*, const void*, int, void*, void*, const void*, const void*, void*, void*, int, int, int,
-                            cudaStream_t);
+                            const int*, cudaStream_t);
 int launch_gemm_grouped_swiglu(const void*, const void*, void*, void*, int, int, int, int64_t, int64_t, const int*, const int*, int, int*, cudaStream_t);
 void launch_rope(void*, const int64_t*, const float*, const float*, int64_t, int, int, int, int64_t,
                  int64_t, float, const int*, cudaStream_t);
@@ -346,19 +346,19 @@ std::tuple<Tensor, Tensor, Tensor> peagle_spec(const Tensor& anchor, const Tenso
                             lo.data_ptr<int>(), hi.data_ptr<int>(), extras ? extra.data_ptr<int>() : nullptr, cur_stream());
   return {lo, hi, extra};
 }
-// The rows a training-time-test step of S passes needs (see wanted_rows_kernel): every tensor is fully written.
+// The rows a training-time-test step of S passes needs (see wanted_rows_kernel).  Without targets the second list stays unwritten.
 // -> (index int64[2, T], inverse int32[2, T], count int32[2]; ids, positions int64[S, T], mask bool[S, T], prev bool[T], target_row int32[S, T],
 //     intervals int32[n, 2, T] as given, extra keys int32[S (S - 1) / 2, T] flat)
 std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor> step_rows(const Tensor& mask, const Tensor& ids, const Tensor& positions,
-                                                                                                     const std::vector<Tensor>& intervals, int64_t passes) {
-  const int64_t T = ids.numel(), S = passes;
-  TORCH_CHECK(T > 0 && T < (int64_t{1} << 31) / std::max<int64_t>(S * S, 1) && S >= 1 && intervals.size() <= 2 && positions.numel() == T && mask.numel() == T &&
-              mask.is_cuda());
+                                                                                                     const std::vector<Tensor>& intervals, int64_t passes, bool targets) {
+  const int64_t T = positions.numel(), N = ids.numel(), S = passes;
+  TORCH_CHECK(T > 0 && T < (int64_t{1} << 31) / std::max<int64_t>(S * S, 1) && S >= 1 && intervals.size() <= 2 && N >= T && mask.numel() == N &&
+              mask.is_cuda() && (!targets || N == T));
   c10::cuda::CUDAGuard guard(ids.device());
   const auto l = ids.options().dtype(at::kLong), n = ids.options().dtype(at::kInt), b = ids.options().dtype(at::kBool);
   Tensor index = at::empty({2, T}, l), inverse = at::empty({2, T}, n), count = at::empty({2}, n);
   Tensor ids_out = at::empty({S, T}, l), pos_out = at::empty({S, T}, l), mask_out = at::empty({S, T}, b), prev = at::empty({T}, b);
-  Tensor target_row = at::empty({S, T}, n), spans = at::empty({(int64_t)intervals.size(), 2, T}, n), extra = at::empty({S * (S - 1) / 2, T}, n);
+  Tensor target_row = at::empty({targets ? S : 0, T}, n), spans = at::empty({(int64_t)intervals.size(), 2, T}, n), extra = at::empty({S * (S - 1) / 2, T}, n);
   const int* in[2] = {nullptr, nullptr};
   int* out[2] = {nullptr, nullptr};
   for (size_t k = 0; k < intervals.size(); ++k) {
@@ -367,9 +367,9 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tenso
     in[k] = intervals[k].data_ptr<int>();
     out[k] = spans.select(0, (int64_t)k).data_ptr<int>();
   }
-  sb200::launch_step_rows(row_flags(mask, T), long_ptr(ids, "ids"), long_ptr(positions, "positions"), in, (int)T, (int)S, index.data_ptr<int64_t>(),
+  sb200::launch_step_rows(row_flags(mask, N), long_ptr(ids, "ids"), long_ptr(positions, "positions"), in, (int)T, (int)N, (int)S, index.data_ptr<int64_t>(),
                           inverse.data_ptr<int>(), count.data_ptr<int>(), ids_out.data_ptr<int64_t>(), pos_out.data_ptr<int64_t>(),
-                          reinterpret_cast<uint8_t*>(mask_out.data_ptr()), reinterpret_cast<uint8_t*>(prev.data_ptr()), target_row.data_ptr<int>(), out,
+                          reinterpret_cast<uint8_t*>(mask_out.data_ptr()), reinterpret_cast<uint8_t*>(prev.data_ptr()), targets ? target_row.data_ptr<int>() : nullptr, out,
                           extra.data_ptr<int>(), cur_stream());
   return {index, inverse, count, ids_out, pos_out, mask_out, prev, target_row, spans, extra};
 }
@@ -494,7 +494,8 @@ Tensor gate_mul_bwd(const Tensor& dy, const Tensor& out, const Tensor& gate, Ten
 
 // ---- mixture-of-experts row movement ---------------------------------------------------------------
 // expert int64[T, k] -> (seg int32[E + 1], 256-row tile prefix int32[E + 1], slot_row int32[T * k], row_slot int32[capacity]).
-std::tuple<Tensor, Tensor, Tensor, Tensor> moe_plan(const Tensor& expert, int64_t E, int64_t capacity) {
+std::tuple<Tensor, Tensor, Tensor, Tensor> moe_plan(const Tensor& expert, int64_t E, int64_t capacity, int64_t k, const c10::optional<Tensor>& live) {
+  TORCH_CHECK(k >= 1 && expert.numel() % k == 0, "moe_plan: k slots per token");
   TORCH_CHECK(expert.is_cuda() && expert.scalar_type() == at::kLong && expert.is_contiguous() && expert.numel() > 0);
   TORCH_CHECK(E >= 1 && E <= 1024 && capacity >= (expert.numel() + 127 * E + 127) / 128 * 128, "moe_plan: at most 1024 experts and room for every padded segment");
   c10::cuda::CUDAGuard guard(expert.device());
@@ -503,7 +504,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> moe_plan(const Tensor& expert, int64_
   Tensor hist = at::empty({sb200::moe_plan_blocks(n), E}, opt), seg = at::empty({E + 1}, opt), tiles = at::empty({E + 1}, opt);
   Tensor slot_row = at::empty({n}, opt), row_slot = at::empty({capacity}, opt);
   const int rc = sb200::launch_moe_plan(expert.data_ptr<int64_t>(), n, (int)E, (int)capacity, hist.data_ptr<int>(), seg.data_ptr<int>(), tiles.data_ptr<int>(),
-                                        slot_row.data_ptr<int>(), row_slot.data_ptr<int>(), cur_stream());
+                                        slot_row.data_ptr<int>(), row_slot.data_ptr<int>(), used_rows(live), (int)k, cur_stream());
   TORCH_CHECK(rc == 0, "moe_plan launch failed (", rc, ")");
   return {seg, tiles, slot_row, row_slot};
 }
@@ -523,13 +524,13 @@ Tensor moe_gather(const Tensor& x, const Tensor& row_slot, const Tensor& seg, in
   sb200::launch_moe_gather(x.data_ptr(), x.stride(0), int_ptr(row_slot, 1, "row_slot"), rows_used_of(seg), (int)k, out.data_ptr(), (int)cap, (int)H, cur_stream());
   return out;
 }
-Tensor moe_gather_bwd(const Tensor& d_pad, const Tensor& slot_row, int64_t k) {
+Tensor moe_gather_bwd(const Tensor& d_pad, const Tensor& slot_row, int64_t k, const c10::optional<Tensor>& live) {
   check_rows(d_pad, "d_pad");
   TORCH_CHECK(d_pad.is_contiguous() && d_pad.size(1) % 8 == 0 && slot_row.numel() % k == 0);
   const int64_t T = slot_row.numel() / k, H = d_pad.size(1);
   c10::cuda::CUDAGuard guard(d_pad.device());
   Tensor dx = at::empty({T, H}, d_pad.options());
-  sb200::launch_moe_gather_bwd(d_pad.data_ptr(), int_ptr(slot_row, 1, "slot_row"), (int)k, dx.data_ptr(), (int)T, (int)H, cur_stream());
+  sb200::launch_moe_gather_bwd(d_pad.data_ptr(), int_ptr(slot_row, 1, "slot_row"), (int)k, dx.data_ptr(), (int)T, (int)H, used_rows(live), cur_stream());
   return dx;
 }
 const void* token_rows(const c10::optional<Tensor>& t, int64_t T, int64_t W, const char* name) {
@@ -538,7 +539,7 @@ const void* token_rows(const c10::optional<Tensor>& t, int64_t T, int64_t W, con
   return t->data_ptr();
 }
 Tensor moe_combine(const Tensor& y_pad, const Tensor& slot_row, const Tensor& p, const c10::optional<Tensor>& shared, const c10::optional<Tensor>& gate,
-                   const c10::optional<Tensor>& residual) {
+                   const c10::optional<Tensor>& residual, const c10::optional<Tensor>& live) {
   check_rows(y_pad, "y_pad");
   TORCH_CHECK(y_pad.is_contiguous() && p.dim() == 2 && p.is_contiguous() && p.scalar_type() == at::kBFloat16 && p.numel() == slot_row.numel());
   TORCH_CHECK(shared.has_value() == gate.has_value(), "moe_combine: the shared expert comes with its gate");
@@ -546,12 +547,13 @@ Tensor moe_combine(const Tensor& y_pad, const Tensor& slot_row, const Tensor& p,
   c10::cuda::CUDAGuard guard(y_pad.device());
   Tensor out = at::empty({T, H}, y_pad.options());
   sb200::launch_moe_combine(y_pad.data_ptr(), int_ptr(slot_row, 1, "slot_row"), p.data_ptr(), (int)k, token_rows(shared, T, H, "shared"), token_rows(gate, T, 1, "gate"),
-                            token_rows(residual, T, H, "residual"), out.data_ptr(), (int)T, (int)H, cur_stream());
+                            token_rows(residual, T, H, "residual"), out.data_ptr(), (int)T, (int)H, used_rows(live), cur_stream());
   return out;
 }
 // -> (dy_pad, dp, dshared, dgate); the last two empty without a shared expert
 std::tuple<Tensor, Tensor, Tensor, Tensor> moe_combine_bwd(const Tensor& dout, const Tensor& y_pad, const Tensor& row_slot, const Tensor& seg, const Tensor& p,
-                                                           const c10::optional<Tensor>& shared, const c10::optional<Tensor>& gate) {
+                                                           const c10::optional<Tensor>& shared, const c10::optional<Tensor>& gate,
+                                                           const c10::optional<Tensor>& live) {
   check_rows(y_pad, "y_pad");
   const int64_t T = p.size(0), k = p.size(1), H = y_pad.size(1), cap = row_slot.numel();
   TORCH_CHECK(y_pad.is_contiguous() && y_pad.size(0) == cap && p.is_contiguous() && p.scalar_type() == at::kBFloat16);
@@ -560,7 +562,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> moe_combine_bwd(const Tensor& dout, c
   Tensor dshared = at::empty({shared.has_value() ? T : 0, H}, y_pad.options()), dgate = at::empty({shared.has_value() ? T : 0, 1}, y_pad.options());
   sb200::launch_moe_combine_bwd(token_rows(dout, T, H, "dout"), y_pad.data_ptr(), int_ptr(row_slot, 1, "row_slot"), rows_used_of(seg), p.data_ptr(), (int)k,
                                 dy_pad.data_ptr(), dp.data_ptr(), token_rows(shared, T, H, "shared"), token_rows(gate, T, 1, "gate"), dshared.data_ptr(),
-                                dgate.data_ptr(), (int)T, (int)cap, (int)H, cur_stream());
+                                dgate.data_ptr(), (int)T, (int)cap, (int)H, used_rows(live), cur_stream());
   return {dy_pad, dp, dshared, dgate};
 }
 
@@ -1439,11 +1441,12 @@ TORCH_LIBRARY(sb200, m) {
   m.def("embedding_bwd", &embedding_bwd);
   m.def("gate_mul_fwd", &gate_mul_fwd);
   m.def("gate_mul_bwd", &gate_mul_bwd);
-  m.def("moe_plan", &moe_plan);
+  m.def("moe_plan(Tensor expert, int E, int capacity, int k=1, Tensor? live=None) -> (Tensor, Tensor, Tensor, Tensor)", &moe_plan);
   m.def("moe_gather", &moe_gather);
-  m.def("moe_gather_bwd", &moe_gather_bwd);
-  m.def("moe_combine", &moe_combine);
-  m.def("moe_combine_bwd", &moe_combine_bwd);
+  m.def("moe_gather_bwd(Tensor d_pad, Tensor slot_row, int k, Tensor? live=None) -> Tensor", &moe_gather_bwd);
+  m.def("moe_combine(Tensor y_pad, Tensor slot_row, Tensor p, Tensor? shared, Tensor? gate, Tensor? residual, Tensor? live=None) -> Tensor", &moe_combine);
+  m.def("moe_combine_bwd(Tensor dout, Tensor y_pad, Tensor row_slot, Tensor seg, Tensor p, Tensor? shared, Tensor? gate, Tensor? live=None) -> "
+        "(Tensor, Tensor, Tensor, Tensor)", &moe_combine_bwd);
   m.def("gemm_grouped_swiglu", &gemm_grouped_swiglu);
   m.def("rope_(Tensor x, Tensor positions, Tensor cos, Tensor sin, int heads, int hd, int rot, float sign, Tensor? live=None) -> ()", &rope_);
   m.def("loss_fwd", &loss_fwd);

@@ -13,7 +13,7 @@
 //                     dshared = sigmoid(g) dout, dg = <shared, dout> sigmoid'(g)
 //
 // All of them are bound by memory: a row is read and written once, 16 bytes per thread and access, one block per row.
-// Rows past seg[E] exist in the buffers (their capacity is the worst case) but are neither read nor written.
+// `live` (optional, device): tokens in use; the slots of the others are not placed.  Rows past seg[E] exist in the buffers (their capacity is the worst case) but are neither read nor written.
 #include "common.cuh"
 
 namespace sb200 {
@@ -24,8 +24,9 @@ constexpr int kPlanThreads = 1024;
 constexpr int kMaxExperts = 1024;
 
 __global__ void __launch_bounds__(kPlanThreads)
-count_kernel(const int64_t* __restrict__ expert, int n_slots, int E, int* __restrict__ hist) {
+count_kernel(const int64_t* __restrict__ expert, int n_slots, int E, int* __restrict__ hist, const int* __restrict__ live, int k) {
   pdl_begin();
+  n_slots = live_rows(live, n_slots / k) * k;
   __shared__ int count[kMaxExperts];
   for (int e = threadIdx.x; e < E; e += kPlanThreads) count[e] = 0;
   __syncthreads();
@@ -57,8 +58,9 @@ __device__ __forceinline__ void scan_segments(const int* total, int E, int* seg,
 
 __global__ void __launch_bounds__(kPlanThreads)
 place_kernel(const int64_t* __restrict__ expert, int n_slots, int E, int capacity, const int* __restrict__ hist, int* __restrict__ seg_out,
-             int* __restrict__ tiles_out, int* __restrict__ slot_row, int* __restrict__ row_slot) {
+             int* __restrict__ tiles_out, int* __restrict__ slot_row, int* __restrict__ row_slot, const int* __restrict__ live, int k) {
   pdl_begin();
+  n_slots = live_rows(live, n_slots / k) * k;
   __shared__ int total[kMaxExperts], before[kMaxExperts], seg[kMaxExperts + 1], tiles[kMaxExperts + 1];
   extern __shared__ unsigned short warp_count[];  // [32][E]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -124,9 +126,11 @@ gather_kernel(const __nv_bfloat16* __restrict__ x, int64_t x_stride, const int* 
 }
 
 __global__ void __launch_bounds__(kThreads)
-gather_bwd_kernel(const __nv_bfloat16* __restrict__ d_pad, const int* __restrict__ slot_row, int k, __nv_bfloat16* __restrict__ dx, int H) {
+gather_bwd_kernel(const __nv_bfloat16* __restrict__ d_pad, const int* __restrict__ slot_row, int k, __nv_bfloat16* __restrict__ dx, int H,
+                  const int* __restrict__ live) {
   pdl_begin();
   const int64_t t = blockIdx.x;
+  if (live != nullptr && t >= *live) return;
   for (int c = threadIdx.x * 8; c < H; c += kThreads * 8) {
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll 5
@@ -145,9 +149,10 @@ __device__ __forceinline__ float sigmoid(float g) { return 1.f / (1.f + __expf(-
 __global__ void __launch_bounds__(kThreads)
 combine_kernel(const __nv_bfloat16* __restrict__ y_pad, const int* __restrict__ slot_row, const __nv_bfloat16* __restrict__ p, int k,
                const __nv_bfloat16* __restrict__ shared, const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __restrict__ residual,
-               __nv_bfloat16* __restrict__ out, int H) {
+               __nv_bfloat16* __restrict__ out, int H, const int* __restrict__ live) {
   pdl_begin();
   const int64_t t = blockIdx.x;
+  if (live != nullptr && t >= *live) return;
   const float s = shared != nullptr ? sigmoid(__bfloat162float(gate[t])) : 0.f;
   for (int c = threadIdx.x * 8; c < H; c += kThreads * 8) {
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, v[8];
@@ -177,11 +182,13 @@ __global__ void __launch_bounds__(kThreads)
 combine_bwd_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ y_pad, const int* __restrict__ row_slot,
                    const int* __restrict__ rows_used, const __nv_bfloat16* __restrict__ p, int k, __nv_bfloat16* __restrict__ dy_pad,
                    __nv_bfloat16* __restrict__ dp, const __nv_bfloat16* __restrict__ shared, const __nv_bfloat16* __restrict__ gate,
-                   __nv_bfloat16* __restrict__ dshared, __nv_bfloat16* __restrict__ dgate, int tokens, int H) {
+                   __nv_bfloat16* __restrict__ dshared, __nv_bfloat16* __restrict__ dgate, int tokens, int H,
+                   const int* __restrict__ live) {
   pdl_begin();
   __shared__ float scratch[33];
   if ((int)blockIdx.x < tokens) {  // shared expert
     const int64_t t = blockIdx.x;
+    if (live != nullptr && t >= *live) return;
     const float s = sigmoid(__bfloat162float(gate[t]));
     float dot = 0.f;
     for (int c = threadIdx.x * 8; c < H; c += kThreads * 8) {
@@ -226,11 +233,11 @@ static int row_blocks(int rows) { return rows < 16 * kNumSM ? rows : 16 * kNumSM
 
 int moe_plan_blocks(int n_slots) { return (n_slots + moe::kPlanThreads - 1) / moe::kPlanThreads; }
 
-// hist: int[moe_plan_blocks(n_slots) * E] scratch
+// hist: int[moe_plan_blocks(n_slots) * E] scratch; k: slots per token
 int launch_moe_plan(const int64_t* expert, int n_slots, int E, int capacity, int* hist, int* seg, int* tiles, int* slot_row, int* row_slot,
-                    cudaStream_t stream) {
+                    const int* live, int k, cudaStream_t stream) {
   using namespace moe;
-  if (E < 1 || E > kMaxExperts || n_slots < 1) return -1;
+  if (E < 1 || E > kMaxExperts || n_slots < 1 || k < 1) return -1;
   const int blocks = moe_plan_blocks(n_slots), smem = 32 * E * (int)sizeof(unsigned short);
   static PerDeviceOnce configured;
   if (configured.needed()) {
@@ -238,8 +245,8 @@ int launch_moe_plan(const int64_t* expert, int n_slots, int E, int capacity, int
     configured.mark();
   }
   count_launch(2);
-  launch_pdl(count_kernel, blocks, kPlanThreads, 0, stream, expert, n_slots, E, hist);
-  launch_pdl(place_kernel, blocks, kPlanThreads, smem, stream, expert, n_slots, E, capacity, hist, seg, tiles, slot_row, row_slot);
+  launch_pdl(count_kernel, blocks, kPlanThreads, 0, stream, expert, n_slots, E, hist, live, k);
+  launch_pdl(place_kernel, blocks, kPlanThreads, smem, stream, expert, n_slots, E, capacity, hist, seg, tiles, slot_row, row_slot, live, k);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
@@ -251,23 +258,24 @@ void launch_moe_gather(const void* x, int64_t x_stride, const int* row_slot, con
   launch_pdl(moe::gather_kernel, row_blocks(capacity), moe::kThreads, 0, stream, (In)x, x_stride, row_slot, rows_used, k, (Out)out, H);
 }
 
-void launch_moe_gather_bwd(const void* d_pad, const int* slot_row, int k, void* dx, int tokens, int H, cudaStream_t stream) {
+void launch_moe_gather_bwd(const void* d_pad, const int* slot_row, int k, void* dx, int tokens, int H, const int* live, cudaStream_t stream) {
   count_launch(1);
-  launch_pdl(moe::gather_bwd_kernel, tokens, moe::kThreads, 0, stream, (In)d_pad, slot_row, k, (Out)dx, H);
+  launch_pdl(moe::gather_bwd_kernel, tokens, moe::kThreads, 0, stream, (In)d_pad, slot_row, k, (Out)dx, H, live);
 }
 
 void launch_moe_combine(const void* y_pad, const int* slot_row, const void* p, int k, const void* shared, const void* gate, const void* residual,
-                        void* out, int tokens, int H, cudaStream_t stream) {
+                        void* out, int tokens, int H, const int* live, cudaStream_t stream) {
   count_launch(1);
-  launch_pdl(moe::combine_kernel, tokens, moe::kThreads, 0, stream, (In)y_pad, slot_row, (In)p, k, (In)shared, (In)gate, (In)residual, (Out)out, H);
+  launch_pdl(moe::combine_kernel, tokens, moe::kThreads, 0, stream, (In)y_pad, slot_row, (In)p, k, (In)shared, (In)gate, (In)residual, (Out)out, H, live);
 }
 
 void launch_moe_combine_bwd(const void* dout, const void* y_pad, const int* row_slot, const int* rows_used, const void* p, int k, void* dy_pad, void* dp,
-                            const void* shared, const void* gate, void* dshared, void* dgate, int tokens, int capacity, int H, cudaStream_t stream) {
+                            const void* shared, const void* gate, void* dshared, void* dgate, int tokens, int capacity, int H, const int* live,
+                            cudaStream_t stream) {
   count_launch(1);
   const int shared_blocks = shared != nullptr ? tokens : 0;
   launch_pdl(moe::combine_bwd_kernel, shared_blocks + row_blocks(capacity), moe::kThreads, 0, stream, (In)dout, (In)y_pad, row_slot, rows_used, (In)p, k,
-             (Out)dy_pad, (Out)dp, (In)shared, (In)gate, (Out)dshared, (Out)dgate, shared_blocks, H);
+             (Out)dy_pad, (Out)dp, (In)shared, (In)gate, (Out)dshared, (Out)dgate, shared_blocks, H, live);
 }
 
 }  // namespace sb200

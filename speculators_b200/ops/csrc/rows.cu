@@ -163,12 +163,13 @@ peagle_spec_kernel(const int64_t* __restrict__ anchor, const int64_t* __restrict
 // In a training-time-test step row t is wanted where its loss in some pass s < S (label and target row t + s, loss_mask[t + s])
 // or its run of correct passes (loss_mask[t]) counts; every other row only serves as context keys of pass 0.  The verifier's
 // row u is wanted where some wanted comparison reads it.  Block 0 lists the first, block 1 the second, ascending, as
-// index (row of the step -> row of the batch) and inverse (-1: not listed).  The count is rounded up to 256, so that no GEMM
+// index (row of the step -> row of the batch) and inverse (-1: not listed).  Labels may reach past the rows (N >= T of them; there
+// is no verifier's list then).  The count is rounded up to 256, so that no GEMM
 // or attention tile and no contraction step of 128 straddles it, by rows that nobody asked for (the last ones): they are
 // computed like any other and their gradients are exact zeros.
 constexpr int kKept = 16;  // rounds of which the flags stay in shared memory: 131072 rows
 __global__ void __launch_bounds__(kT)
-wanted_rows_kernel(const uint8_t* __restrict__ mask, int T, int S, int64_t* __restrict__ index, int* __restrict__ inverse, int* __restrict__ count) {
+wanted_rows_kernel(const uint8_t* __restrict__ mask, int T, int N, int S, int64_t* __restrict__ index, int* __restrict__ inverse, int* __restrict__ count) {
   pdl_begin();
   __shared__ int scratch[32], total, carry;
   __shared__ uint8_t kept[kKept * kT];
@@ -182,7 +183,7 @@ wanted_rows_kernel(const uint8_t* __restrict__ mask, int T, int S, int64_t* __re
     for (int j = 0; j < kPer; ++j)
       for (int s = 0; s < S; ++s) {
         const int u = i0 + j + dir * s;
-        if (i0 + j < T && u >= 0 && u < T && mask[u] != 0) bits |= 1u << j;
+        if (i0 + j < T && u >= 0 && u < N && mask[u] != 0) bits |= 1u << j;
       }
     return bits;
   };
@@ -228,7 +229,7 @@ struct StepRows {
   const int* interval[2];  // [2, T] lo and hi (optional)
   const int64_t* index;
   const int *inverse, *count;  // of both lists
-  int T, S;
+  int T, N, S;
   int64_t *ids_out, *positions_out;  // [S, T]
   uint8_t *mask_out, *prev_out;      // [S, T], [T]
   int* target_row;                   // [S, T]
@@ -250,11 +251,11 @@ __global__ void __launch_bounds__(256) step_rows_kernel(const StepRows p) {
     }
   for (int s = 0; s < p.S; ++s) {
     const int64_t u = t + s, at = (int64_t)s * p.T + i;
-    const bool in = on && u < p.T;
+    const bool in = on && u < p.N;
     p.ids_out[at] = in ? p.ids[u] : 0;
     p.positions_out[at] = on ? p.positions[t] + s : 0;
     p.mask_out[at] = in && p.mask[u] != 0;
-    p.target_row[at] = in ? p.inverse[p.T + u] : -1;
+    if (p.target_row != nullptr) p.target_row[at] = in ? p.inverse[p.T + u] : -1;
     int* extra = p.extra + (int64_t)p.T * (s * (s - 1) / 2) + (int64_t)i * s;
     for (int j = 0; j < s; ++j) extra[j] = on ? j * p.T + i : -1;
   }
@@ -447,13 +448,14 @@ void launch_peagle_spec(const int64_t* anchor, const int64_t* depth, const bool*
   count_launch(1);
   launch_pdl(rows::peagle_spec_kernel, grid, 256, 0, stream, anchor, depth, row_valid, doc, doc_lo, n, T, num_depths, window, (const int*)table, lo, hi, extra);
 }
-void launch_step_rows(const uint8_t* mask, const int64_t* ids, const int64_t* positions, const int* const* interval, int T, int S, int64_t* index,
+// target_row == nullptr: no list of the verifier's rows (needed where N > T)
+void launch_step_rows(const uint8_t* mask, const int64_t* ids, const int64_t* positions, const int* const* interval, int T, int N, int S, int64_t* index,
                       int* inverse, int* count, int64_t* ids_out, int64_t* positions_out, uint8_t* mask_out, uint8_t* prev_out, int* target_row,
                       int* const* interval_out, int* extra, cudaStream_t stream) {
   if (T <= 0) return;
   count_launch(2);
-  launch_pdl(rows::wanted_rows_kernel, 2, rows::kT, 0, stream, mask, T, S, index, inverse, count);
-  const rows::StepRows p{mask, ids, positions, {interval[0], interval[1]}, index, inverse, count, T, S, ids_out, positions_out, mask_out, prev_out,
+  launch_pdl(rows::wanted_rows_kernel, target_row != nullptr ? 2 : 1, rows::kT, 0, stream, mask, T, N, S, index, inverse, count);
+  const rows::StepRows p{mask, ids, positions, {interval[0], interval[1]}, index, inverse, count, T, N, S, ids_out, positions_out, mask_out, prev_out,
                          target_row, {interval_out[0], interval_out[1]}, extra};
   launch_pdl(rows::step_rows_kernel, (T + 255) / 256, 256, 0, stream, p);
 }

@@ -29,27 +29,27 @@ def moe_experts_ok(x: torch.Tensor, gate_up: torch.Tensor, down: torch.Tensor) -
 
 class _MoEExpertsFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, top_p, top_e, w_gu, w_d, shared, gate, residual, uses):
+    def forward(ctx, x, top_p, top_e, w_gu, w_d, shared, gate, residual, uses, live):
         nat, status = ops.native(), ops.gemm_status(x.device)
         k, E = top_e.shape[1], w_gu.shape[0]
         capacity = (top_e.numel() + 127 * E + 127) // 128 * 128  # worst case: every expert's tail padded by 127 rows
-        seg, tiles, slot_row, row_slot = nat.moe_plan(top_e, E, capacity)
+        seg, tiles, slot_row, row_slot = nat.moe_plan(top_e, E, capacity, k, live)
         x_pad = nat.moe_gather(x, row_slot, seg, k)
         gate_up, h = nat.gemm_grouped_swiglu(x_pad, w_gu, seg, tiles, status)
         y_pad = torch.empty((capacity, w_d.shape[1]), dtype=x.dtype, device=x.device)
         nat.gemm_grouped_rows(h, w_d, y_pad, False, seg, tiles, status)
-        out = nat.moe_combine(y_pad, slot_row, top_p, shared, gate, residual)
-        ctx.save_for_backward(x_pad, gate_up, h, y_pad, top_p, w_gu, w_d, shared, gate, seg, tiles, slot_row, row_slot)
+        out = nat.moe_combine(y_pad, slot_row, top_p, shared, gate, residual, live)
+        ctx.save_for_backward(x_pad, gate_up, h, y_pad, top_p, w_gu, w_d, shared, gate, seg, tiles, slot_row, row_slot, live)
         ctx.with_residual, ctx.uses = residual is not None, uses
         return out
 
     @staticmethod
     def backward(ctx, dout):
-        x_pad, gate_up, h, y_pad, top_p, w_gu, w_d, shared, gate, seg, tiles, slot_row, row_slot = ctx.saved_tensors
+        x_pad, gate_up, h, y_pad, top_p, w_gu, w_d, shared, gate, seg, tiles, slot_row, row_slot, live = ctx.saved_tensors
         nat, status = ops.native(), ops.gemm_status(dout.device)
         need = ctx.needs_input_grad
         dout = dout.contiguous()
-        dy_pad, dp, dshared, dgate = nat.moe_combine_bwd(dout, y_pad, row_slot, seg, top_p, shared, gate)
+        dy_pad, dp, dshared, dgate = nat.moe_combine_bwd(dout, y_pad, row_slot, seg, top_p, shared, gate, live)
 
         def weight_gradient(needed, dy, rows, w, use):
             if not needed:
@@ -78,18 +78,18 @@ class _MoEExpertsFn(torch.autograd.Function):
             if need[0]:
                 dx_pad = torch.empty_like(x_pad)
                 nat.gemm_grouped_rows(dgu, w_gu, dx_pad, True, seg, tiles, status)
-                dx = nat.moe_gather_bwd(dx_pad, slot_row, top_p.shape[1])
+                dx = nat.moe_gather_bwd(dx_pad, slot_row, top_p.shape[1], live)
         with_shared = shared is not None
-        return dx, dp, None, dw_gu, dw_d, dshared if with_shared else None, dgate if with_shared else None, dout if ctx.with_residual else None, None
+        return dx, dp, None, dw_gu, dw_d, dshared if with_shared else None, dgate if with_shared else None, dout if ctx.with_residual else None, None, None
 
 
-def moe_experts(x, top_p, top_e, gate_up, down, shared=None, shared_gate=None, residual=None) -> torch.Tensor:
+def moe_experts(x, top_p, top_e, gate_up, down, shared=None, shared_gate=None, residual=None, live=None) -> torch.Tensor:
     """``sum_j top_p[t, j] * expert_{top_e[t, j]}(x[t]) (+ sigmoid(shared_gate[t]) * shared[t]) (+ residual[t])`` for
     operands that ``moe_experts_ok`` accepts; ``x [T, H]``, ``top_e`` int64 and ``top_p`` of ``x``'s dtype ``[T, k]``,
-    ``shared_gate`` ``[T, 1]`` before its sigmoid."""
+    ``shared_gate`` ``[T, 1]`` before its sigmoid.  ``live``: tokens in use (``ops.step_rows``); the others go to no expert."""
     def rows(t):
         return None if t is None else t.contiguous()
 
     grad = torch.is_grad_enabled()
     uses = tuple(ops._note_use(w, "experts") if grad and w.requires_grad else None for w in (gate_up, down))  # noqa: SLF001
-    return _MoEExpertsFn.apply(rows(x), rows(top_p), rows(top_e), gate_up, down, rows(shared), rows(shared_gate), rows(residual), uses)
+    return _MoEExpertsFn.apply(rows(x), rows(top_p), rows(top_e), gate_up, down, rows(shared), rows(shared_gate), rows(residual), uses, live)

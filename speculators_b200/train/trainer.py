@@ -234,7 +234,7 @@ class _GraphedStep:
         static_in = {k: torch.empty(v.shape, dtype=v.dtype, device=dev) for k, v in batch.items() if isinstance(v, torch.Tensor)}
         for k, v in static_in.items():
             v.copy_(batch[k], non_blocking=True)
-        kwargs = tr.config.train_call_kwargs or {}
+        kwargs = tr.loss_only(tr.config.train_call_kwargs)
         side = self._capture_stream(dev)
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):
@@ -333,6 +333,10 @@ class Trainer:
         self.setup_trainer()
         self.setup_model()
         self.setup_optimizer()
+
+    def loss_only(self, call_kwargs: dict | None) -> dict:
+        """What the model is called with: the configured arguments, and what lets it leave out results that nobody takes here."""
+        return {**getattr(self.model, "loss_only_kwargs", {}), **(call_kwargs or {})}
 
     # ------------------------------------------------------------------ setup
     def _training_state_path(self, epoch) -> Path:
@@ -471,7 +475,7 @@ class Trainer:
             self.timer.mark("fetch")
             with nvtx_range("forward"):
                 self.engine.zero_grad()
-                _, loss, metrics = self.model(**dev_batch, **(self.config.train_call_kwargs or {}))
+                _, loss, metrics = self.model(**dev_batch, **self.loss_only(self.config.train_call_kwargs))
             self.timer.mark("fwd")
             with nvtx_range("backward"):
                 loss.backward()
@@ -736,7 +740,7 @@ class Trainer:
         for i, batch in enumerate(self.val_loader):
             self._maybe_val_sync(i)
             dev_batch = {k: v.to(device, non_blocking=True) if isinstance(v, torch.Tensor) else v for k, v in batch.items()}
-            _, _loss, metrics = self.model(**dev_batch, **(self.config.val_call_kwargs or {}))
+            _, _loss, metrics = self.model(**dev_batch, **self.loss_only(self.config.val_call_kwargs))
             for k, v in metrics.items():
                 accumulated[k] = v.float() if k not in accumulated else accumulated[k] + v.float()
         val_metrics: dict[str, float] = {}

@@ -205,11 +205,85 @@ def test_gpu_pass_over_needed_rows(monkeypatch, T, kind, layers, head_dim, qwen,
 
 @pytest.mark.gpu
 def test_gpu_what_is_not_one_fused_loss_takes_all_rows():
-    model, batch = _model(1, 64, False, 512, False), _gpu_batch(777, "spans")
+    model, batch = _model(1, 64, False, 512, False), _gpu_batch(2100, "spans")
     for loss_fn, implementation, want in (("kl_div", "fused", True), ("ce", "fused", True), ("kl_div", "eager", False), ('{"ce": 0.5, "tv": 0.5}', "fused", False), ("nla", "fused", False)):
         kwargs, _ = Eagle3DraftModel.get_trainer_kwargs(loss_fn=loss_fn, loss_implementation=implementation, ttt_steps=2, ttt_step_loss_decay=1.0)
         assert model._takes_needed_rows(2100, batch["loss_mask"], kwargs["loss_config"], 2) is want, loss_fn
-    assert not model._takes_needed_rows(2100, None, None, 2) and not model._takes_needed_rows(2047, batch["loss_mask"], None, 2)
+    assert not model._takes_needed_rows(2100, None, None, 2) and not model._takes_needed_rows(2047, batch["loss_mask"][:, :2047], None, 2)
     tokens, loss, _ = model(**batch, ttt_steps=2)  # draft tokens of every row
-    assert len(tokens) == 2 and tokens[0].shape == (1, 777)
+    assert len(tokens) == 2 and tokens[0].shape == (1, 2100)
     assert not copy.deepcopy(model).float()._takes_needed_rows(2100, batch["loss_mask"], None, 2)
+
+
+# --------------------------------------------------------------------------- multi-token prediction
+def _mtp(experts: int, hidden: int, head_dim: int, vocab: int):
+    from speculators_b200.config import SpeculatorsConfig, VerifierConfig
+    from speculators_b200.models.mtp import MTPDraftModel, MTPSpeculatorConfig
+    from speculators_b200.proposals.greedy import GreedyTokenProposalConfig
+
+    cfg = dict(architectures=["Qwen3ForCausalLM"], model_type="qwen3", hidden_size=hidden, num_hidden_layers=4, num_attention_heads=4, num_key_value_heads=2,
+               head_dim=head_dim, intermediate_size=2 * hidden, vocab_size=vocab, rms_norm_eps=1e-6, rope_theta=10000.0, max_position_embeddings=4096,
+               hidden_act="silu")
+    if experts:
+        cfg.update(architectures=["Qwen3NextForCausalLM"], model_type="qwen3_next", partial_rotary_factor=0.25, num_experts=experts, num_experts_per_tok=2,
+                   moe_intermediate_size=256, shared_expert_intermediate_size=256, norm_topk_prob=True, decoder_sparse_step=1, mlp_only_layers=[])
+    torch.manual_seed(0)
+    model = MTPDraftModel(MTPSpeculatorConfig(transformer_layer_config=TransformerLayerConfig(**cfg), speculators_config=SpeculatorsConfig(
+        algorithm="mtp", proposal_methods=[GreedyTokenProposalConfig(speculative_tokens=3)], default_proposal_method="greedy",
+        verifier=VerifierConfig(name_or_path=None, architectures=cfg["architectures"]))))
+    model.load_verifier_weights()
+    with torch.no_grad():
+        model.embed_tokens.weight.normal_(0.0, 1.0)
+        model.lm_head.weight.normal_(0.0, 0.1)
+    model.embed_tokens.weight.requires_grad_(False)
+    model.lm_head.weight.requires_grad_(False)
+    return model
+
+
+def _mtp_results(model, batch, monkeypatch):
+    results = []
+    for needed in (False, True):
+        monkeypatch.setattr(type(model), "_takes_needed_rows", lambda *_, n=needed: n)
+        for p in model.parameters():
+            p.grad = None
+        if batch["input_ids"].is_cuda:
+            poison = [torch.full((1 << 27,), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(4)]
+            del poison
+        logits, loss, metrics = model(**batch, return_logits=False, step_weights=[0.5, 0.3, 0.2])
+        assert logits == []
+        loss.backward()
+        results.append((metrics, {n: p.grad.float() for n, p in model.named_parameters() if p.grad is not None}))
+    return results
+
+
+@pytest.mark.parametrize("kind", KINDS)
+def test_mtp_step_over_needed_rows_equals_the_whole_step(monkeypatch, kind):
+    T, model = 50, _mtp(0, 32, 8, 64)
+    batch = {"input_ids": torch.randint(0, 64, (1, T)), "hidden_states": torch.randn(1, T, 32), "loss_mask": _mask(kind, T)[None]}
+    monkeypatch.setattr(type(model.mtp_layers[0]), "takes_listed_rows", lambda _: True)
+    (metrics, grads), (metrics_needed, grads_needed) = _mtp_results(model, batch, monkeypatch)
+    assert metrics.keys() == metrics_needed.keys() and grads.keys() == grads_needed.keys()
+    for k, v in metrics.items():
+        torch.testing.assert_close(metrics_needed[k], v, rtol=1e-5, atol=1e-6, msg=k)
+    for n, v in grads.items():
+        torch.testing.assert_close(grads_needed[n], v, rtol=1e-4, atol=1e-5 * float(v.abs().max()) + 1e-9, msg=n)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T", [516, 777, 1540])
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("experts,head_dim", [(0, 128), (0, 64), (8, 256)])
+def test_gpu_mtp_step_over_needed_rows(monkeypatch, T, kind, experts, head_dim):
+    g = torch.Generator().manual_seed(T)
+    model = _mtp(experts, 512, head_dim, 1000).cuda().bfloat16()
+    assert model.mtp_layers[0].takes_listed_rows()
+    batch = {"input_ids": torch.randint(0, 1000, (1, T), generator=g).cuda(), "hidden_states": torch.randn(1, T, 512, generator=g).bfloat16().cuda(),
+             "loss_mask": _mask(kind, T)[None].cuda()}
+    (metrics, grads), (metrics_needed, grads_needed) = _mtp_results(model, batch, monkeypatch)
+    assert metrics.keys() == metrics_needed.keys() and grads.keys() == grads_needed.keys()
+    for k, v in metrics.items():
+        torch.testing.assert_close(metrics_needed[k], v, rtol=2e-4, atol=1e-6, msg=k)
+    for n, v in grads.items():  # as for EAGLE-3
+        assert torch.isfinite(grads_needed[n]).all(), n
+        assert float((grads_needed[n] - v).norm()) <= 1e-2 * float(v.norm()) + 1e-12, (n, float((grads_needed[n] - v).norm() / v.norm()))
+    ops.check_gemm_status()
