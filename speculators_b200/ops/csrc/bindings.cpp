@@ -6,7 +6,12 @@
 
 #include "attention_params.h"
 #include "ep_a2a.h"
+#include "gemm_split.h"
 #include <ATen/ATen.h>
+
+#include <algorithm>
+#include <deque>
+#include <mutex>
 
 namespace sb200 {
 int rmsnorm_bwd_partial_rows(int rows, int H, bool with_dx);
@@ -61,13 +66,14 @@ int launch_loss_bwd(int, const void*, const void*, const float*, const float*, c
                     int64_t, int64_t, int64_t, int, const int*, const int*, cudaStream_t);
 int64_t launch_count();
 int launch_gemm_tn_tcgen05(const void*, const void*, void*, const void*, int, int, int, int64_t, int64_t, int64_t, int64_t, int,
-                           int*, int, const int*, cudaStream_t);
+                           int*, int, const int*, SplitSpace*, cudaStream_t);
 int launch_gemm_tcgen05(const void*, const void*, void*, const void*, int, int, int, int64_t, int64_t, int64_t, int64_t, int, int, int,
-                        int*, int, const int*, cudaStream_t);
-int launch_gemm_parts(int, const void* const*, const void* const*, const int*, const int64_t*, const int64_t*, const int* const*, void*, int, int, int64_t, int, int*, cudaStream_t);
+                        int*, int, const int*, SplitSpace*, cudaStream_t);
+int launch_gemm_parts(int, const void* const*, const void* const*, const int*, const int64_t*, const int64_t*, const int* const*, void*, int, int, int64_t, int, int*,
+                      SplitSpace*, cudaStream_t);
 int launch_gemm_grouped_parts(int, const void* const*, const void* const*, const int*, const int64_t*, const int64_t*, const int* const*, void*, int, int, int,
                               const int*, int, int*, cudaStream_t);
-int launch_gemm_stack(const void*, const void*, void*, const void*, int, int, int, int, int, int, float, float, int, int*, cudaStream_t);
+int launch_gemm_stack(const void*, const void*, void*, const void*, int, int, int, int, int, int, float, float, int, int*, SplitSpace*, cudaStream_t);
 void launch_moe_group_plan(const int*, int, int*, int*, cudaStream_t);
 int launch_gemm_grouped(const void*, const void*, void*, int, int, int, int64_t, int64_t, int64_t, int, int, int, const int*, const int*, int, int*,
                         cudaStream_t);
@@ -130,6 +136,65 @@ const uint8_t* row_flags(const c10::optional<Tensor>& t, int64_t rows) {
   TORCH_CHECK((t->scalar_type() == at::kBool || t->scalar_type() == at::kByte) && t->is_contiguous() && t->numel() >= rows, "bool / uint8 row flags expected");
   return reinterpret_cast<const uint8_t*>(t->data_ptr());
 }
+
+// ---- memory of GEMMs that divide tiles ---------------------------------------------------------------------
+// Partial sums come from the caching allocator, for the launch alone.  Counters and flags have to be zero when the kernel starts,
+// and a launch of a captured graph finds them used at its next replay: they come in slabs of kSlots launches that one memset
+// zeroes, on the launch's stream and - under capture - as a node of the graph, in whose memory the slab then is.  A slot
+// serves one launch.  The slab in use is kept per stream and capture (the last kSlabs of them, 300 KB each); one that is
+// dropped goes back to the allocator in its stream's order, behind the launches that use it.
+struct SyncSlabs {
+  static constexpr int kSlots = 64, kSlabs = 32;
+  struct Slab {
+    int device;
+    cudaStream_t stream;
+    unsigned long long capture;  // 0: none
+    Tensor memory;
+    int used;
+  };
+  std::mutex mutex;
+  std::deque<Slab> slabs;  // the least recently made first
+  static SyncSlabs& instance() {
+    static SyncSlabs* all = new SyncSlabs;  // outlives the threads and the driver: never destroyed
+    return *all;
+  }
+  int* slot(const Tensor& near, cudaStream_t stream) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    if (cudaStreamGetCaptureInfo(stream, &status, &id) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    if (status != cudaStreamCaptureStatusActive) id = 0;
+    const int ints = (sb200::gemm_split_sync_ints() + 31) / 32 * 32, device = near.get_device();
+    std::lock_guard<std::mutex> lock(mutex);
+    auto it = std::find_if(slabs.begin(), slabs.end(), [&](const Slab& s) { return s.device == device && s.stream == stream; });
+    if (it != slabs.end() && (it->capture != id || it->used == kSlots)) {
+      slabs.erase(it);
+      it = slabs.end();
+    }
+    if (it == slabs.end()) {
+      Slab s{device, stream, id, at::empty({(int64_t)kSlots * ints}, near.options().dtype(at::kInt)), 0};
+      if (cudaMemsetAsync(s.memory.data_ptr(), 0, s.memory.nbytes(), stream) != cudaSuccess) return nullptr;
+      if (slabs.size() == kSlabs) slabs.pop_front();
+      slabs.push_back(std::move(s));
+      it = slabs.end() - 1;
+    }
+    return it->memory.data_ptr<int>() + (int64_t)it->used++ * ints;
+  }
+};
+struct TorchSplitSpace : sb200::SplitSpace {
+  const Tensor& near;
+  Tensor partial;
+  explicit TorchSplitSpace(const Tensor& t) : near(t) {}
+  bool get(float** sums, int** sync) override {
+    *sync = SyncSlabs::instance().slot(near, cur_stream());
+    if (*sync == nullptr) return false;
+    partial = at::empty({sb200::gemm_split_floats()}, near.options().dtype(at::kFloat));
+    *sums = partial.data_ptr<float>();
+    return true;
+  }
+};
 
 void norm_fwd(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& row_index, Tensor y,
               c10::optional<Tensor> rstd, double eps, bool centred, const c10::optional<Tensor>& live) {
@@ -721,8 +786,9 @@ void gemm_wgrad_parts_rows(const std::vector<Tensor>& dy, const std::vector<Tens
   }
   TORCH_CHECK(status.is_cuda() && status.scalar_type() == at::kInt && status.numel() >= 1);
   c10::cuda::CUDAGuard guard(dw.device());
+  TorchSplitSpace space(dw);
   const int rc = sb200::launch_gemm_parts((int)n, a, b, K, lda, ldb, rows_of, dw.data_ptr(), (int)M, (int)N, dw.stride(0), accumulate ? 1 : 0, status.data_ptr<int>(),
-                                          cur_stream());
+                                          &space, cur_stream());
   TORCH_CHECK(rc == 0, "gemm_wgrad_parts launch failed (", rc, ")");
 }
 
@@ -1187,9 +1253,10 @@ void gemm_tn_variant(const Tensor& a, const Tensor& b, Tensor out, const c10::op
   }
   TORCH_CHECK(epilogue != 2 || res != nullptr, "gemm_tn: epilogue 2 needs a residual");
   c10::cuda::CUDAGuard guard(a.device());
+  TorchSplitSpace space(a);
   const int rc = sb200::launch_gemm_tn_tcgen05(a.data_ptr(), b.data_ptr(), out.data_ptr(), res, (int)a.size(0), (int)b.size(0),
                                                (int)a.size(1), a.stride(0), b.stride(0), out.stride(0), ldr, (int)epilogue,
-                                               status.data_ptr<int>(), (int)variant, used_rows(live), cur_stream());
+                                               status.data_ptr<int>(), (int)variant, used_rows(live), variant == 6 ? &space : nullptr, cur_stream());
   TORCH_CHECK(rc == 0, "gemm_tn launch failed (", rc, ")");
 }
 
@@ -1215,9 +1282,10 @@ void gemm_variant(const Tensor& a, const Tensor& b, Tensor out, int64_t epilogue
   TORCH_CHECK(K == Kb && out.size(0) == M && out.size(1) == N, "gemm: shape mismatch");
   TORCH_CHECK(status.scalar_type() == at::kInt && status.numel() >= 1);
   c10::cuda::CUDAGuard guard(a.device());
+  TorchSplitSpace space(a);
   const int rc = sb200::launch_gemm_tcgen05(a.data_ptr(), b.data_ptr(), out.data_ptr(), nullptr, (int)M, (int)N, (int)K, a.stride(0),
                                             b.stride(0), out.stride(0), 0, (int)epilogue, a_mn ? 1 : 0, b_mn ? 1 : 0,
-                                            status.data_ptr<int>(), (int)variant, used_rows(live), cur_stream());
+                                            status.data_ptr<int>(), (int)variant, used_rows(live), variant == 0 || variant == 6 ? &space : nullptr, cur_stream());
   TORCH_CHECK(rc == 0, "gemm launch failed (", rc, ")");
 }
 
@@ -1238,8 +1306,9 @@ void gemm_stack(const Tensor& a, const Tensor& b, Tensor out, const c10::optiona
     TORCH_CHECK(addend->is_cuda() && addend->scalar_type() == at::kBFloat16 && addend->is_contiguous() && addend->sizes() == out.sizes(), "gemm_stack: addend");
   TORCH_CHECK(status.is_cuda() && status.scalar_type() == at::kInt && status.numel() >= 1);
   c10::cuda::CUDAGuard guard(a.device());
+  TorchSplitSpace space(a);
   const int rc = sb200::launch_gemm_stack(a.data_ptr(), b.data_ptr(), out.data_ptr(), addend.has_value() ? addend->data_ptr() : nullptr, (int)B, (int)M, (int)N,
-                                          (int)K, a_mn ? 1 : 0, b_mn ? 1 : 0, (float)alpha, (float)beta, symmetric ? 1 : 0, status.data_ptr<int>(), cur_stream());
+                                          (int)K, a_mn ? 1 : 0, b_mn ? 1 : 0, (float)alpha, (float)beta, symmetric ? 1 : 0, status.data_ptr<int>(), &space, cur_stream());
   TORCH_CHECK(rc == 0, "gemm_stack launch failed (", rc, ")");
 }
 

@@ -39,6 +39,7 @@
 // returns.  Nothing traps and nothing spins forever.
 #include <atomic>
 
+#include "gemm_split.h"
 #include "loss_stats.cuh"
 #include "remember.h"
 #include "tcgen05_utils.cuh"
@@ -55,7 +56,7 @@ constexpr int TMEM_COLS = 512;
 // gate in columns 0..127 and up in 128..255); the epilogue stores both halves into C[M, 2 I] (kept for the backward
 // pass) and silu(gate) * up into h[M, I].
 enum Epilogue : int { kStore = 0, kAccumulate = 1, kAddResidual = 2, kSwiGLU = 3 };
-enum Status : int { kOk = kStatusOk, kTimeoutProducer = 1, kTimeoutMma = 2, kTimeoutEpilogue = 3 };
+enum Status : int { kOk = kStatusOk, kTimeoutProducer = 1, kTimeoutMma = 2, kTimeoutEpilogue = 3, kTimeoutPartial = 4 };
 
 // Row statistics in the epilogue (the lm_head product fused with the row loss): next to
 // storing the logits tile, every thread reduces its row's 256 columns of the tile, together with
@@ -128,7 +129,138 @@ struct Params {
   // Device-side row count of the activations (live_rows).  It bounds M, and where both operands are MN-major (a weight
   // gradient, which sums over the rows) K.  A multiple of 256 or all rows: no tile and no contraction step straddles it.
   const int* live;
+  // Tiles divided between pairs (SplitPlan): partial sums [round][pair][CTA][epilogue warp][1024] float4 and, zero at launch, one
+  // flag per (round, pair, CTA, epilogue warp) behind a start counter.  nullptr: none are.
+  float4* partial;
+  int* sync;
 };
+
+// ---- a part-filled last wave, its tiles divided -------------------------------------------------------------------
+// 74 pairs walk the tiles in whole waves, and the last one is usually part-filled: 80 tiles take as long as 148.  What is left
+// over after the whole waves is divided instead (us before and after: 1280 x 4096 x 4096 43.9 and 34.7, 1280 x 4096 x 14336
+// 141 and 104, 1280 x 4096 x 151936 1572 and 1041, 2560 x 4096 x 14336 229 and 196, 1777 x 6144 x 4096 67 and 63): `parts` pairs take a tile, each an equal part of its contraction, in one or
+// two rounds (left[0], then left[1] tiles).  All parts but the last leave their sums in fp32 in global memory (256 KB a pair, which
+// stay in L2) and raise a flag per epilogue warp; the counterparts in the pair with the last part add them to their
+// accumulator, in the order of the contraction, before the epilogue.  The same bits on every run.
+//   The pairs of one part walk neighbouring tiles in step, as in a whole wave, and so share operand panels in L2.  Dividing
+// all steps evenly (each pair a contiguous range of the tiles' contraction steps) balances better and loses that: 1024 x
+// 8192 x 28672 took 465 us so, 321 undivided - every panel came from memory once per tile.
+//   The rounds come first.  A pair waits for pairs with a lower number only, and numbers go by the order in which pairs start
+// (a counter): whoever is waited for is running already, and waits for nobody who is not.
+constexpr int kMostParts = 8;
+constexpr int kSplitSync = 1 + 2 * 74 * 16;  // ints of `sync`: the counter, then flags of (round, pair, CTA, epilogue warp)
+struct SplitPlan {
+  int whole;    // tiles in whole waves; the rest are divided
+  int left[2];  // tiles of the two rounds
+  int parts[2];
+  int steps;    // contraction steps of a pair on its way through (the longest part of each round)
+  float us;     // predicted, above a launch's fixed part
+};
+// Round i of `left` tiles in `parts` parts: 0.56 us a step, and for writing, waiting for and adding sums 2.5 us and 1.2 a part.
+// Without whole waves behind them the rounds have nothing to hide that behind (256 x 4096 x 14336: 46.6 us where this says 31).
+constexpr float kStepUs = 0.56f, kRoundUs = 2.5f, kPartUs = 1.2f, kSplitGainUs = 2.f, kAloneUs = 20.f;
+__host__ __device__ inline SplitPlan split_plan(int tiles, int kb, int pairs) {
+  const int waves = tiles / pairs, rest = tiles - waves * pairs;
+  SplitPlan s{tiles, {0, 0}, {1, 1}, kb * (waves + (rest > 0)), 0.f};
+  s.us = kStepUs * s.steps;
+  if (rest == 0) return s;
+  auto consider = [&](int n0, int c0, int n1, int c1) {
+    if (c0 < 2 || kb < 2 * c0 || n0 * c0 > pairs || (n1 > 0 && (c1 < 2 || kb < 2 * c1 || n1 * c1 > pairs))) return;
+    const int steps = kb * waves + (kb + c0 - 1) / c0 + (n1 > 0 ? (kb + c1 - 1) / c1 : 0);
+    const float us = kStepUs * steps + kRoundUs + kPartUs * c0 + (n1 > 0 ? kRoundUs + kPartUs * c1 : 0.f);
+    if (us + (waves > 0 ? kSplitGainUs : kAloneUs) < kStepUs * kb * (waves + 1) && (s.left[0] == 0 || us < s.us)) s = SplitPlan{waves * pairs, {n0, n1}, {c0, n1 > 0 ? c1 : 1}, steps, us};
+  };
+  const int fit = pairs / rest;
+  for (int c = 2; c <= kMostParts; ++c) {
+    if (c <= fit) consider(rest, c, 0, 0);
+    const int half = pairs / 2, behind = rest - half;  // two parts for as many tiles as that takes, then the others
+    if (behind > 0 && c <= pairs / behind) consider(half, 2, behind, c);
+  }
+  return s;
+}
+
+// The pieces of tiles that one pair works on, in order: its parts of divided tiles, then whole tiles.
+template <bool DIVIDE>
+struct Pieces {  // whole tiles only
+  int tile;
+  static constexpr int k0 = 0, steps = 0, round = -1, part = 0;
+  int next;
+  __device__ __forceinline__ explicit Pieces(int number) : next(number) {}
+  __device__ __forceinline__ bool advance(const SplitPlan& s, int, int, int pairs) {
+    tile = next;
+    next += pairs;
+    return tile < s.whole;
+  }
+};
+template <>
+struct Pieces<true> {
+  int tile, k0, steps;  // this piece: contraction steps k0 .. k0 + steps of the tile
+  int round, part;      // of a divided tile; round -1: a whole one
+  int at, next;
+  __device__ __forceinline__ explicit Pieces(int number) : round(-1), part(0), at(0), next(number) {}
+  __device__ __forceinline__ bool advance(const SplitPlan& s, int kb, int number, int pairs) {
+    while (at < 2) {
+      const int i = at++, n = i == 0 ? s.left[0] : s.left[1], c = i == 0 ? s.parts[0] : s.parts[1];
+      if (number >= n * c) continue;
+      round = i;
+      part = number / n;
+      tile = s.whole + (i == 0 ? 0 : s.left[0]) + number - part * n;
+      k0 = part * kb / c;
+      steps = (part + 1) * kb / c - k0;
+      return true;
+    }
+    round = -1;
+    if (next >= s.whole) return false;
+    tile = next;
+    k0 = 0;
+    steps = kb;
+    next += pairs;
+    return true;
+  }
+};
+
+// A warp's 32 rows x 128 columns of the accumulator, four columns at a time, lanes (rows) side by side.
+__device__ __forceinline__ void split_put(float4* to, uint32_t tmem, int lane) {
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    uint32_t r[32];
+    tmem_ld32(tmem + c * 32, r);
+    tmem_ld_wait();
+#pragma unroll
+    for (int v = 0; v < 8; ++v)
+      __stcg(to + (c * 8 + v) * 32 + lane, make_float4(__uint_as_float(r[v * 4]), __uint_as_float(r[v * 4 + 1]), __uint_as_float(r[v * 4 + 2]), __uint_as_float(r[v * 4 + 3])));
+  }
+}
+__device__ __forceinline__ void split_add(const float4* from, uint32_t tmem, int lane) {
+#pragma unroll 1
+  for (int c = 0; c < 4; ++c) {
+    uint32_t r[32];
+    float4 o[8];
+#pragma unroll
+    for (int v = 0; v < 8; ++v) o[v] = __ldcg(from + (c * 8 + v) * 32 + lane);
+    tmem_ld32(tmem + c * 32, r);
+    tmem_ld_wait();
+#pragma unroll
+    for (int v = 0; v < 8; ++v) {
+      const float add[4] = {o[v].x, o[v].y, o[v].z, o[v].w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) r[v * 4 + j] = __float_as_uint(__uint_as_float(r[v * 4 + j]) + add[j]);
+    }
+    tmem_st32(tmem + c * 32, r);
+  }
+  tmem_st_wait();
+}
+// One lane's bounded wait for a flag; false = gave up (status word set) or another role already failed.
+__device__ __forceinline__ bool flag_wait(const int* flag, int* status, int code) {
+  for (uint32_t i = 0; i < POLL_LIMIT; ++i) {
+    int up;
+    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(up) : "l"(flag) : "memory");
+    if (up != 0) return true;
+    if ((i & 0xfff) == 0xfff && *reinterpret_cast<volatile int*>(status) != kStatusOk) return false;
+  }
+  atomicCAS(status, kStatusOk, code);
+  return false;
+}
 
 __device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16(x)); }
 struct Scaling {
@@ -596,6 +728,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   const int tiles_m = (p.M + BM - 1) / BM, tiles = tiles_m * ((p.N + S_TILE_N - 1) / S_TILE_N);
   const int z = (int)(blockIdx.x >> log_splits) / tiles, tile = (int)(blockIdx.x >> log_splits) - z * tiles;
   const int m0 = (tile % tiles_m) * BM, n0 = (tile / tiles_m) * S_TILE_N;
+  int M = p.M, all_kb = (p.K + S_STEP_K - 1) / S_STEP_K;
   if (threadIdx.x == 0) {
     for (int s = 0; s < S_STAGES; ++s) {
       mbar_init(smem_addr(&bar_full[s]), 1);
@@ -613,10 +746,12 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   fence_after_sync();
   const uint32_t tmem_base = tmem_base_slot;
   pdl_begin();
-  constexpr bool kSumsRows = A_MN && B_MN;
-  const int M = kSumsRows ? p.M : live_rows(p.live, p.M), K = kSumsRows ? live_rows(p.live, p.K) : p.K;
-  const bool dead = m0 >= M;  // the whole cluster: nothing is loaded, multiplied or stored
-  const int all_kb = dead ? 0 : (K + S_STEP_K - 1) / S_STEP_K;
+  constexpr bool kSumsRows = A_MN && B_MN;  // nothing to sum: zeros (a dead tile of the other layouts stores nothing)
+  if (p.live != nullptr) {
+    if (kSumsRows) all_kb = (live_rows(p.live, p.K) + S_STEP_K - 1) / S_STEP_K;
+    else M = live_rows(p.live, p.M);
+    if (m0 >= M) all_kb = 0;  // for the whole cluster: nothing is loaded, multiplied or stored
+  }
   const int kb0 = (split * all_kb) >> log_splits, num_kb = (((split + 1) * all_kb) >> log_splits) - kb0;
   if (log_splits > 0) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // waited for before the first remote store
 
@@ -678,12 +813,12 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16);
       if (p.staged) {
         const uint32_t stage = smem_addr(smem + S_STAGES * S_STAGE_BYTES) + quarter * 4096;
-        store_accumulator_staged<S_TILE_N>(p, sc, &map_c, &map_c, stage, taddr, m0 + quarter * 32, n0, z, pre, m0 + quarter * 32 < M, false, num_kb == 0, lane);
+        store_accumulator_staged<S_TILE_N>(p, sc, &map_c, &map_c, stage, taddr, m0 + quarter * 32, n0, z, pre, m0 + quarter * 32 < M, false, kSumsRows && num_kb == 0, lane);
         stage_wait();
       } else if (pre.tile_ok) {
-        store_accumulator_prefetched<S_TILE_N>(p, sc, taddr, row, n0, z, pre, num_kb == 0);
+        store_accumulator_prefetched<S_TILE_N>(p, sc, taddr, row, n0, z, pre, kSumsRows && num_kb == 0);
       } else {
-        store_accumulator<S_TILE_N>(p, sc, taddr, row, n0, z, M, num_kb == 0);
+        store_accumulator<S_TILE_N>(p, sc, taddr, row, n0, z, M, kSumsRows && num_kb == 0);
       }
     }
   } else {
@@ -799,7 +934,9 @@ __device__ __forceinline__ int more_steps(const Params& p, const MoreParts& more
 }
 __device__ __forceinline__ int more_steps(const Params&, const NoParts&, const PartSteps<false>&, int, int) { return 0; }
 
-template <int KSUB, bool A_MN = false, bool B_MN = false, bool PARTS = false>
+// DIVIDE: the tiles of a part-filled last wave may be divided between pairs (an instance of its own: what that takes in registers
+// cost undivided products 2 %).
+template <int KSUB, bool A_MN = false, bool B_MN = false, bool PARTS = false, bool DIVIDE = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P_THREADS, 1)
 gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_h, const Params p,
@@ -807,17 +944,19 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   static_assert(!PARTS || (A_MN && B_MN), "parts are those of weight gradients");
+  static_assert(!DIVIDE || !PARTS, "a contraction in parts is not divided");
   static_assert(KSUB == 2 || (!A_MN && !B_MN), "MN-major operands are staged as 128-row boxes: KSUB must be 2");
   constexpr int P_STAGES = 6 / KSUB;
   constexpr int P_STAGE_BYTES = KSUB * P_SUB_BYTES;
   constexpr int STAGE_K = KSUB * BK;
   __shared__ __align__(8) uint64_t bar_full[P_STAGES], bar_empty[P_STAGES], bar_acc_full[2], bar_acc_empty[2];
   __shared__ uint32_t tmem_base_slot;
+  __shared__ int ticket_slot;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
-  const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
+  const int num_pairs = gridDim.x >> 1;
   if (threadIdx.x == 0) {
     for (int s = 0; s < P_STAGES; ++s) {
       mbar_init(smem_addr(&bar_full[s]), 1);   // the leader's expect_tx arrival; bytes come from both CTAs' copies
@@ -842,17 +981,27 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   const int M = kSumsRows ? p.M : live_rows(p.live, p.M), K = kSumsRows ? live_rows(p.live, p.K) : p.K;
   const int tiles_m = (M + P_TILE_M - 1) / P_TILE_M, tiles_n = (p.N + P_TILE_N - 1) / P_TILE_N;
   const int num_kb = (K + STAGE_K - 1) / STAGE_K;
-  [[maybe_unused]] const PartSteps<PARTS> steps(more);
+  [[maybe_unused]] const PartSteps<PARTS> part_kb(more);
   const int num_tiles = p.grp.mode == kGroupRows ? p.grp.tile_start[p.grp.num_groups] * tiles_n
                         : p.grp.mode == kGroupK  ? p.grp.num_groups * tiles_m * tiles_n
                                                  : p.batch * (p.symmetric ? tiles_m * (tiles_m + 1) / 2 : tiles_m * tiles_n);
+  SplitPlan plan{num_tiles, {0, 0}, {1, 1}, 0, 0.f};
+  if (DIVIDE) plan = split_plan(num_tiles, num_kb, num_pairs);
+  int number = blockIdx.x >> 1;  // which pair this is; where tiles are divided in the order of starting
+  if (DIVIDE && plan.left[0] > 0) {
+    if (leader && threadIdx.x == 0) ticket_slot = atomicAdd(p.sync, 1);
+    __syncwarp();
+    cluster_sync_all();
+    asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(number) : "r"(map_to_cta(smem_addr(&ticket_slot), 0)) : "memory");
+  }
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (both CTAs)
     if (elect_one()) {
       uint32_t stage = 0, phase = 0;
       bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
+      for (Pieces<DIVIDE> it(number); ok && it.advance(plan, num_kb, number, num_pairs);) {
+        const int tile = it.tile;
         const TileInfo ti = decode_tile<B_MN>(p, M, tile, tiles_m, tiles_n, num_kb, (int)rank);
         auto load_steps = [&](const CUtensorMap* ma, const CUtensorMap* mb, int a_k0, int b_k0, int count) {
           for (int kb = 0; kb < count; ++kb) {
@@ -874,11 +1023,11 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             if (++stage == P_STAGES) { stage = 0; phase ^= 1; }
           }
         };
-        load_steps(&map_a, &map_b, ti.a_k0, ti.b_k0, ti.num_kb);
+        load_steps(&map_a, &map_b, ti.a_k0 + it.k0 * STAGE_K, ti.b_k0 + it.k0 * STAGE_K, DIVIDE ? it.steps : ti.num_kb);
         if constexpr (PARTS) {
           for (int i = 0; i < more.n && ok; ++i) {
             int k0;
-            const int count = part_steps(p, more, steps, i, tile, tiles_m * tiles_n, k0);
+            const int count = part_steps(p, more, part_kb, i, tile, tiles_m * tiles_n, k0);
             load_steps(&more.a[i], &more.b[i], k0, k0, count);
           }
         }
@@ -897,12 +1046,13 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       uint32_t stage = 0, phase = 0;
       bool ok = true;
       int local = 0;
-      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++local) {
+      for (Pieces<DIVIDE> it(number); ok && it.advance(plan, num_kb, number, num_pairs); ++local) {
         const int acc = local & 1;
         if (!(ok = mbar_wait(smem_addr(&bar_acc_empty[acc]), ((local >> 1) & 1) ^ 1, p.status, kTimeoutMma))) break;
         fence_after_sync();
         const uint32_t tmem_d = tmem_base + acc * BN;
-        const int tile_kb = decode_tile<B_MN>(p, M, tile, tiles_m, tiles_n, num_kb, 0).num_kb + more_steps(p, more, steps, tile, tiles_m * tiles_n);
+        const int tile_kb = DIVIDE ? it.steps
+                                    : decode_tile<B_MN>(p, M, it.tile, tiles_m, tiles_n, num_kb, 0).num_kb + more_steps(p, more, part_kb, it.tile, tiles_m * tiles_n);
         for (int kb = 0; kb < tile_kb; ++kb) {
           if (!(ok = mbar_wait(smem_addr(&bar_full[stage]), phase, p.status, kTimeoutMma))) break;
           fence_after_sync();
@@ -934,25 +1084,48 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const uint32_t stage = smem_addr(smem + P_RING_BYTES) + (warp - 2) * 4096;
     bool ok = true;
     int local = 0;
-    for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++local) {
-      const int acc = local & 1;
+    for (Pieces<DIVIDE> it(number); ok && it.advance(plan, num_kb, number, num_pairs); ++local) {
+      const int acc = local & 1, tile = it.tile;
+      const int parts = !DIVIDE || it.round < 0 ? 1 : it.round == 0 ? plan.parts[0] : plan.parts[1];
+      const bool hands_over = DIVIDE && it.part + 1 < parts;  // another pair finishes the tile
       const TileInfo ti = decode_tile<B_MN>(p, M, tile, tiles_m, tiles_n, num_kb, (int)rank);
       const int row = ti.c_row0 + quarter * 32 + lane, n0 = ti.n0 + chalf * P_EPI_COLS;
-      const bool zero = ti.num_kb + more_steps(p, more, steps, tile, tiles_m * tiles_n) == 0;
+      const bool zero = ti.num_kb + more_steps(p, more, part_kb, tile, tiles_m * tiles_n) == 0;
       RowPrefetch<P_EPI_COLS> pre;
       const bool with_stats = p.rs.targets != nullptr, gated = p.epilogue == kSwiGLU;
       if (with_stats) prefetch_targets<P_EPI_COLS>(p, row, n0, pre);
+      else if (hands_over) pre.tile_ok = pre.valid = false;
       else if (p.staged && !gated) prefetch_addend_staged<P_EPI_COLS>(p, row, n0, ti.z, ti.row_end, pre);
       else if (!gated) prefetch_addend<P_EPI_COLS>(p, row, n0, ti.z, ti.row_end, pre);
       ok = mbar_wait(smem_addr(&bar_acc_full[acc]), (local >> 1) & 1, p.status, kTimeoutEpilogue);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       fence_after_sync();
-      const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN + chalf * P_EPI_COLS;
+      const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN, taddr = lane_base + chalf * P_EPI_COLS;
+      if (DIVIDE && parts > 1) {
+        auto slot = [&](int pair) { return ((it.round * num_pairs + pair) * 2 + (int)rank) * 8 + warp - 2; };
+        if (hands_over) {
+          split_put(p.partial + (int64_t)slot(number) * 1024, taddr, lane);
+          __threadfence();
+          __syncwarp();
+          if (lane == 0) asm volatile("st.release.gpu.global.s32 [%0], 1;" ::"l"(p.sync + 1 + slot(number)) : "memory");
+          fence_before_sync();
+          mbar_arrive_cluster_relaxed(acc_empty_leader[acc]);
+          continue;
+        }
+        const int n = it.round == 0 ? plan.left[0] : plan.left[1];
+        for (int other = number - n * it.part; other < number && ok; other += n) {
+          if (lane == 0) ok = flag_wait(p.sync + 1 + slot(other), p.status, kTimeoutPartial);
+          ok = __shfl_sync(0xffffffffu, ok, 0);
+          __syncwarp();
+          if (ok) split_add(p.partial + (int64_t)slot(other) * 1024, taddr, lane);
+        }
+        if (!ok) break;
+      }
       const int row0 = ti.c_row0 + quarter * 32;
       const Scaling sc{p.alpha, p.beta};
       if (gated)  // this warp: gate columns 64 * chalf .. + 63 of the tile and the same up columns
-        store_accumulator_swiglu(p, &map_c, &map_h, stage, tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN + chalf * 64, row0, ti.n0 + chalf * 64,
+        store_accumulator_swiglu(p, &map_c, &map_h, stage, lane_base + chalf * 64, row0, ti.n0 + chalf * 64,
                                  row0 < ti.row_end, lane);
       else if (with_stats) store_accumulator_with_stats<P_EPI_COLS>(p, taddr, row, n0, ti.tile_n * 2 + chalf, tiles_n * 2, pre);
       else if (p.staged) store_accumulator_staged<P_EPI_COLS>(p, sc, &map_c, &map_h, stage, taddr, row0, n0, ti.z, pre, row0 < ti.row_end, ti.mirror, zero, lane);
@@ -1165,7 +1338,7 @@ static cudaError_t launch_small(int a_mn, int b_mn, int tiles, int log_splits, i
   return cudaLaunchKernelEx(&cfg, tc::gemm_small_kernel<false, false>, map_a, map_b, map_c, p, log_splits);
 }
 
-enum Variant : int { kPairK64 = 2, kPair = 3, kSplit2 = 4, kSplit4 = 5, kSmall = 10, kSmall2 = 11, kSmall4 = 12, kSmall8 = 13 };
+enum Variant : int { kPairK64 = 2, kPair = 3, kSplit2 = 4, kSplit4 = 5, kPairDivided = 6, kSmall = 10, kSmall2 = 11, kSmall4 = 12, kSmall8 = 13 };
 constexpr int kMaxPairs = kNumSM / 2;
 
 // 256x256 tiles of a stack of products (of a symmetric one: the diagonal and what lies above it).
@@ -1200,21 +1373,30 @@ static int resident_clusters(int size) {
 // exchange of partial sums) plus its 128-wide contraction steps; the constants (us) are fits to launches inside CUDA
 // graphs at 128 .. 3072 rows and columns and contractions of 128 .. 32000, all three layouts:
 //   pair tiles     7.0 + 0.56 / step and wave     (2048 x 1024 x 1024: 10.9 us; 1000 x 2048 x 8192: 43.8)
+//   the same with the tiles of a part-filled last wave divided: 8.0 + what split_plan says, 26.0 with no whole wave
+//                                                  (1280 x 4096 x 4096: 43.9 -> 34.7; 768 x 2048 x 32000: 85.6 -> 78.5)
 //   128 x 64 tiles 3.3 + 0.34 / step and wave     (1024 x 1024 x 1024: 6.7; 128 x 256 x 256: 4.0)
 //   the same, contraction over 2, 4, 8 CTAs: 5.0 + 0.34 / step, one wave only   (128 x 512 x 2048: 6.1 at 8, 8.6 unsplit)
 //   pair tiles over 2, 4 pairs: 10.8 + 0.66 / step, one wave only               (1000 x 2048 x 8192: 31.9 at 2)
 // Several waves of small tiles are bound by L2-to-SM traffic, so they pay a full wave each; the model drops them
 // quickly.  Products of more than about two waves of pair tiles always come out as pair tiles.
-static int choose_variant(int M, int N, int K, int batch, int symmetric) {
+// divide: tiles may be divided between pairs.  Gradients' products may; a forward product, whose rows give the same bits in a batch
+// of any size (with all rows or only the needed ones), is not divided by what is left over of its tiles.
+static int choose_variant(int M, int N, int K, int batch, int symmetric, bool divide) {
   using namespace tc;
   const int64_t small = (int64_t)((M + BM - 1) / BM) * ((N + S_TILE_N - 1) / S_TILE_N) * batch;
   const int64_t big = pair_tile_count(M, N, batch, 0);
   const int steps = (K + 127) / 128;
   int best = kPair;
-  float t = 7.0f + 0.56f * steps * ((pair_tile_count(M, N, batch, symmetric) + kMaxPairs - 1) / kMaxPairs);
+  const int64_t pair_tiles = pair_tile_count(M, N, batch, symmetric);
+  float t = 7.0f + 0.56f * steps * ((pair_tiles + kMaxPairs - 1) / kMaxPairs);
   auto consider = [&](int variant, float us) {
     if (us < t) { t = us; best = variant; }
   };
+  if (divide && pair_tiles < (1 << 20)) {
+    const SplitPlan s = split_plan((int)pair_tiles, steps, kMaxPairs);
+    if (s.left[0] > 0) consider(kPairDivided, (s.whole > 0 ? 8.0f : 26.0f) + s.us);
+  }
   if (small <= 4 * kNumSM) consider(kSmall, 2.0f + (1.3f + 0.34f * steps) * ((small + kNumSM - 1) / kNumSM));
   for (int log = 1; log <= 3; ++log)
     if (steps >= (2 << log) && small <= resident_clusters(1 << log)) consider(kSmall + log, 5.0f + 0.34f * ((steps + (1 << log) - 1) >> log));
@@ -1222,6 +1404,21 @@ static int choose_variant(int M, int N, int K, int batch, int symmetric) {
     if (steps >= (4 << log) && big <= resident_clusters(2 << log)) consider(log == 1 ? kSplit2 : kSplit4, 10.8f + 0.66f * ((steps + (1 << log) - 1) >> log));
   return best;
 }
+
+// Space for the partial sums of divided tiles: what a product in this form may need, 0 if it never divides any.  rows_vary: M is
+// only the most that the device may ask for.
+static bool may_split(int M, int N, int K, int batch, int symmetric, bool rows_vary) {
+  const int kb = (K + 127) / 128;
+  for (int m = M; m > 0; m -= tc::P_TILE_M) {
+    const int64_t tiles = pair_tile_count(m, N, batch, symmetric);
+    if (tiles < (1 << 20) && tc::split_plan((int)tiles, kb, kMaxPairs).left[0] > 0) return true;
+    if (!rows_vary) break;
+  }
+  return false;
+}
+int64_t gemm_split_floats() { return (int64_t)2 * kMaxPairs * 2 * 8 * 1024 * 4; }
+int gemm_split_sync_ints() { return tc::kSplitSync; }
+static_assert(kMaxPairs == 74, "kSplitSync counts the pairs");
 
 // Further uses of a weight whose gradient is one product (see MoreParts); the first is the plain a, b, K.
 struct PartsSpec {
@@ -1248,12 +1445,12 @@ struct BatchSpec {
 // lda / ldb / ldc / ldr in elements; operand rows must be 16-byte aligned (ld multiple of 8).
 // `status` is a device int the kernel writes a non-zero code to if a bounded wait ran out.
 // variant: 0 = choose (choose_variant), 1 or 10 .. 13 = 128x64 tiles on one CTA or a cluster of 2, 4, 8 CTAs, 2 = CTA pairs with 64-wide K stages (K-major only),
-// 3 = CTA pairs with 128-wide K stages, 4 / 5 = clusters of two / four pairs that split the contraction of a tile.
+// 3 = CTA pairs with 128-wide K stages (6 = the same, the tiles of a part-filled last wave divided; needs `space`), 4 / 5 = clusters of two / four pairs that split the contraction of a tile.
 static int launch_gemm_impl(const void* a, const void* b, void* c, const void* residual, int M, int N, int K, int64_t lda,
                             int64_t ldb, int64_t ldc, int64_t ldr, int epilogue, int a_mn, int b_mn, int* status, int variant,
                             const void* stats_targets, int64_t stats_ldt, int stats_t_rows, int stats_shift, float* stats_partial,
                             const tc::Grouping* grp, cudaStream_t stream, const tc::Scatter* scatter = nullptr, void* gated_h = nullptr,
-                            int64_t gated_ldh = 0, const BatchSpec* batched = nullptr, const PartsSpec* parts = nullptr, const int* live = nullptr) {
+                            int64_t gated_ldh = 0, const BatchSpec* batched = nullptr, const PartsSpec* parts = nullptr, const int* live = nullptr, SplitSpace* space = nullptr) {
   using namespace tc;
   static const BatchSpec one{};
   const BatchSpec& bs = batched != nullptr ? *batched : one;
@@ -1266,6 +1463,8 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
     bool ok = allow_smem(gemm_tn_2cta_kernel<1>, smem_pair) && allow_smem(gemm_tn_2cta_kernel<2>, smem_pair) &&
               allow_smem(gemm_tn_2cta_kernel<2, false, true>, smem_pair) && allow_smem(gemm_tn_2cta_kernel<2, true, false>, smem_pair) &&
               allow_smem(gemm_tn_2cta_kernel<2, true, true>, smem_pair) && allow_smem(gemm_tn_2cta_kernel<2, true, true, true>, smem_pair);
+    ok = ok && allow_smem(gemm_tn_2cta_kernel<2, false, false, false, true>, smem_pair) && allow_smem(gemm_tn_2cta_kernel<2, false, true, false, true>, smem_pair) &&
+         allow_smem(gemm_tn_2cta_kernel<2, true, false, false, true>, smem_pair) && allow_smem(gemm_tn_2cta_kernel<2, true, true, false, true>, smem_pair);
     ok = ok && allow_smem(gemm_split_kernel<2, false, false>, smem_pair) && allow_smem(gemm_split_kernel<2, false, true>, smem_pair) &&
          allow_smem(gemm_split_kernel<2, true, false>, smem_pair) && allow_smem(gemm_split_kernel<2, true, true>, smem_pair);
     ok = ok && allow_smem(gemm_split_kernel<4, false, false>, smem_pair) && allow_smem(gemm_split_kernel<4, false, true>, smem_pair) &&
@@ -1277,11 +1476,14 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
   }
   const bool mn = a_mn || b_mn;
   const bool plain = stats_targets == nullptr && grp == nullptr && scatter == nullptr && epilogue != kSwiGLU;
-  if (variant == 0) variant = plain ? choose_variant(M, N, K, bs.batch, symmetric) : kPair;
+  if (variant == 0) variant = plain ? choose_variant(M, N, K, bs.batch, symmetric, space != nullptr) : kPair;
   if (variant == 1) variant = kSmall;
-  if (variant < kPairK64 || variant > kSmall8 || (variant > kSplit4 && variant < kSmall)) return -4;
+  if (variant < kPairK64 || variant > kSmall8 || (variant > kPairDivided && variant < kSmall)) return -4;
   if (variant == kPairK64 && mn) return -4;
   if (variant > kPair && !plain) return -4;
+  // How many rows there are is known on the device only: it decides whether there is anything to divide
+  const bool divide = variant == kPairDivided || (variant == kPair && plain && live != nullptr && !(a_mn && b_mn));
+  if (variant == kPairDivided) variant = kPair;
   const bool pairs = variant < kSmall;
   CUtensorMap map_a, map_b;
   constexpr int mn_rows = 2 * BK;  // contraction rows of a transposed operand's box
@@ -1294,7 +1496,7 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
   if (rc) return rc;
   Params p{(__nv_bfloat16*)c, (const __nv_bfloat16*)residual, M, N, K, ldc, ldr, epilogue, status, RowStatsOut{nullptr, 0, 0, 0, nullptr},
            Grouping{kGroupNone, 0, nullptr, nullptr}, Scatter{}, (__nv_bfloat16*)gated_h, gated_ldh, 0, bs.alpha, bs.beta, bs.batch,
-           bs.c_stride, bs.r_stride, 0, live};
+           bs.c_stride, bs.r_stride, 0, live, nullptr, nullptr};
   if (live != nullptr && (grp != nullptr || scatter != nullptr || stats_targets != nullptr || bs.batch != 1 || (a_mn && !b_mn))) return -10;
   if (epilogue == kSwiGLU) {
     if (!pairs || a_mn || b_mn || (grp != nullptr && grp->mode != kGroupRows) || stats_targets != nullptr || scatter != nullptr || gated_h == nullptr || (N & 255) || (ldc & 7) ||
@@ -1357,8 +1559,12 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
       more.live[i] = parts->live[i];
     }
   }
-  count_launch(1);
   const int pair_tiles = (int)pair_tile_count(M, N, bs.batch, p.symmetric);
+  if (divide && space != nullptr && parts == nullptr &&
+      may_split(M, N, K, bs.batch, p.symmetric, live != nullptr && !(a_mn && b_mn)) && space->get(reinterpret_cast<float**>(&p.partial), &p.sync)) {
+    if (p.sync == nullptr || p.partial == nullptr) return -11;
+  }
+  count_launch(1);
   if (variant >= kSmall && variant <= kSmall8) {
     const int log_splits = variant - kSmall;
     const int tiles = ((M + BM - 1) / BM) * ((N + S_TILE_N - 1) / S_TILE_N) * bs.batch;
@@ -1369,9 +1575,13 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
     launch_split<4>(a_mn, b_mn, pair_tiles, smem_pair, stream, map_a, map_b, p);
   } else {
     // grouped: the number of tiles is known on the device only; every pair looks for work
-    const int tiles = grp != nullptr ? kMaxPairs : pair_tiles;
+    const int tiles = grp != nullptr || p.sync != nullptr ? kMaxPairs : pair_tiles;  // (divided tiles occupy every pair)
     const int grid = 2 * (tiles < kMaxPairs ? tiles : kMaxPairs);
     if (more.n > 0) launch_pdl(gemm_tn_2cta_kernel<2, true, true, true>, grid, P_THREADS, smem_pair, stream, map_a, map_b, map_c, map_h, p, more);
+    else if (p.sync != nullptr && a_mn && b_mn) launch_pdl(gemm_tn_2cta_kernel<2, true, true, false, true>, grid, P_THREADS, smem_pair, stream, map_a, map_b, map_c, map_h, p, NoParts{});
+    else if (p.sync != nullptr && a_mn) launch_pdl(gemm_tn_2cta_kernel<2, true, false, false, true>, grid, P_THREADS, smem_pair, stream, map_a, map_b, map_c, map_h, p, NoParts{});
+    else if (p.sync != nullptr && b_mn) launch_pdl(gemm_tn_2cta_kernel<2, false, true, false, true>, grid, P_THREADS, smem_pair, stream, map_a, map_b, map_c, map_h, p, NoParts{});
+    else if (p.sync != nullptr) launch_pdl(gemm_tn_2cta_kernel<2, false, false, false, true>, grid, P_THREADS, smem_pair, stream, map_a, map_b, map_c, map_h, p, NoParts{});
     else if (a_mn && b_mn) launch_pdl(gemm_tn_2cta_kernel<2, true, true>, grid, P_THREADS, smem_pair, stream, map_a, map_b, map_c, map_h, p, NoParts{});
     else if (a_mn) launch_pdl(gemm_tn_2cta_kernel<2, true, false>, grid, P_THREADS, smem_pair, stream, map_a, map_b, map_c, map_h, p, NoParts{});
     else if (b_mn) launch_pdl(gemm_tn_2cta_kernel<2, false, true>, grid, P_THREADS, smem_pair, stream, map_a, map_b, map_c, map_h, p, NoParts{});
@@ -1383,20 +1593,21 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
 
 int launch_gemm_tcgen05(const void* a, const void* b, void* c, const void* residual, int M, int N, int K, int64_t lda,
                         int64_t ldb, int64_t ldc, int64_t ldr, int epilogue, int a_mn, int b_mn, int* status, int variant, const int* live,
-                        cudaStream_t stream) {
+                        SplitSpace* space, cudaStream_t stream) {
   return launch_gemm_impl(a, b, c, residual, M, N, K, lda, ldb, ldc, ldr, epilogue, a_mn, b_mn, status, variant, nullptr, 0, 0, 0, nullptr, nullptr, stream,
-                          nullptr, nullptr, 0, nullptr, nullptr, live);
+                          nullptr, nullptr, 0, nullptr, nullptr, live, space);
 }
 
 int launch_gemm_tn_tcgen05(const void* a, const void* b, void* c, const void* residual, int M, int N, int K, int64_t lda,
-                           int64_t ldb, int64_t ldc, int64_t ldr, int epilogue, int* status, int variant, const int* live, cudaStream_t stream) {
-  return launch_gemm_tcgen05(a, b, c, residual, M, N, K, lda, ldb, ldc, ldr, epilogue, 0, 0, status, variant, live, stream);
+                           int64_t ldb, int64_t ldc, int64_t ldr, int epilogue, int* status, int variant, const int* live, SplitSpace* space,
+                           cudaStream_t stream) {
+  return launch_gemm_tcgen05(a, b, c, residual, M, N, K, lda, ldb, ldc, ldr, epilogue, 0, 0, status, variant, live, space, stream);
 }
 
 // c[M, N] (+)= sum_i a_i[K_i, M]^T . b_i[K_i, N]: one launch where pair tiles are the form for the whole contraction, else one each
 // (small products are not bound by their epilogue, and have better forms).
 int launch_gemm_parts(int n, const void* const* a, const void* const* b, const int* K, const int64_t* lda, const int64_t* ldb, const int* const* live,
-                      void* c, int M, int N, int64_t ldc, int accumulate, int* status, cudaStream_t stream) {
+                      void* c, int M, int N, int64_t ldc, int accumulate, int* status, SplitSpace* space, cudaStream_t stream) {
   if (n < 1 || n > tc::kMoreParts + 1) return -9;
   int total = 0;
   PartsSpec parts;
@@ -1413,12 +1624,12 @@ int launch_gemm_parts(int n, const void* const* a, const void* const* b, const i
     parts.live[i - 1] = live[i];
   }
   parts.n = n - 1;
-  if (n > 1 && choose_variant(M, N, total, 1, 0) == kPair)
+  if (n > 1 && choose_variant(M, N, total, 1, 0, false) == kPair)
     return launch_gemm_impl(a[0], b[0], c, nullptr, M, N, K[0], lda[0], ldb[0], ldc, 0, accumulate ? 1 : 0, 1, 1, status, kPair, nullptr, 0, 0, 0, nullptr,
                             nullptr, stream, nullptr, nullptr, 0, nullptr, &parts, live[0]);
   for (int i = 0; i < n; ++i) {
     const int rc = launch_gemm_impl(a[i], b[i], c, nullptr, M, N, K[i], lda[i], ldb[i], ldc, 0, accumulate || i > 0 ? 1 : 0, 1, 1, status, 0, nullptr, 0, 0, 0,
-                                    nullptr, nullptr, stream, nullptr, nullptr, 0, nullptr, nullptr, live[i]);
+                                    nullptr, nullptr, stream, nullptr, nullptr, 0, nullptr, nullptr, live[i], space);
     if (rc) return rc;
   }
   return 0;
@@ -1429,7 +1640,7 @@ int launch_gemm_parts(int n, const void* const* a, const void* const* b, const i
 // All stacks dense: [batch, rows, cols].  `symmetric`: the caller knows that the product is (a Gram matrix, a power of a
 // symmetric matrix): only tiles on and above the diagonal are computed.
 int launch_gemm_stack(const void* a, const void* b, void* c, const void* addend, int batch, int M, int N, int K, int a_mn, int b_mn, float alpha,
-                      float beta, int symmetric, int* status, cudaStream_t stream) {
+                      float beta, int symmetric, int* status, SplitSpace* space, cudaStream_t stream) {
   BatchSpec bs;
   bs.batch = batch;
   bs.a_stride = (int64_t)M * K;
@@ -1439,7 +1650,7 @@ int launch_gemm_stack(const void* a, const void* b, void* c, const void* addend,
   bs.beta = beta;
   bs.symmetric = symmetric != 0;
   return launch_gemm_impl(a, b, c, addend, M, N, K, a_mn ? M : K, b_mn ? N : K, N, N, addend != nullptr ? tc::kAddResidual : tc::kStore, a_mn, b_mn, status, 0,
-                          nullptr, 0, 0, 0, nullptr, nullptr, stream, nullptr, nullptr, 0, &bs);
+                          nullptr, 0, 0, 0, nullptr, nullptr, stream, nullptr, nullptr, 0, &bs, nullptr, nullptr, space);
 }
 
 // ---- row-parallel product with the reduce-scatter's transfer in the epilogue -----------------
