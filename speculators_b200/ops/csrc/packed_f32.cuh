@@ -1,0 +1,28 @@
+// Two fp32 values in a register pair: one instruction for both.
+#pragma once
+
+namespace sb200 {
+
+typedef unsigned long long float2x;
+__device__ __forceinline__ float2x both(float lo, float hi) {
+  float2x r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 apart(float2x v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ float2x fma2(float2x a, float2x b, float2x c) {
+  float2x r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ float2x add2(float2x a, float2x b) {
+  float2x r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+}  // namespace sb200
