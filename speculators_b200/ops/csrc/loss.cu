@@ -1,7 +1,8 @@
 // Row-wise distillation losses between draft logits and verifier logits.
 //
-// One CTA per row.  Forward streams over the row pair and collects the online-softmax statistics (max, sum-exp) and the
-// argmax of both rows, and for the KL divergence its cross term; the other divergences are reduced in a second pass.  Nothing of size [rows, V] is
+// One CTA per row.  Forward makes two streaming passes over the row pair: pass 1
+// collects the online-softmax statistics (max, sum-exp) and the argmax of both
+// rows, pass 2 reduces the selected divergence.  Nothing of size [rows, V] is
 // written.  Backward recomputes both softmaxes from the saved statistics and
 // writes d(logits) in bf16 with the closed forms
 //     kl   : dp - tp
@@ -22,170 +23,68 @@
 namespace sb200 {
 
 enum LossOp : int { kOpKL = 0, kOpRKL = 1, kOpJSD = 2, kOpCE = 3, kOpTV = 4 };
-constexpr int kLossThreads = 512, kFwdThreads = 256;
+constexpr int kLossThreads = 512;
 constexpr int kNumStats = 5;  // m_d, z_d, m_t, z_t, per-op extra
 
-// One thread's share of a row: running maximum, sum of exponentials against it, and the column at which the vector of eight
-// starts that holds the maximum first (which of the eight is looked up once, at the end of the row).  KL: and the cross term.
-struct Share {
-  float m = -INFINITY, z = 0.f, A = 0.f;
-  int col = 0x7fffffff;
-};
-__device__ __forceinline__ float max8(const bf16x8& v) {
-  const __nv_bfloat162 m = __hmax2(__hmax2(v.v[0], v.v[1]), __hmax2(v.v[2], v.v[3]));
-  return fmaxf(__low2float(m), __high2float(m));
-}
-// A new maximum moves the sums; most vectors bring none.
-__device__ __forceinline__ void raise(Share& s, float to, int col) {
-  if (to > s.m) {
-    const float by = __expf(s.m - to);
-    s.z *= by;
-    s.A *= by;
-    s.m = to;
-    s.col = col;
-  }
-}
-__device__ __forceinline__ float reference(const Share& s) { return s.m == -INFINITY ? 0.f : s.m; }
-
-// Two fp32 values in a register pair: one instruction for both.
-typedef unsigned long long float2x;
-__device__ __forceinline__ float2x both(float lo, float hi) {
-  float2x r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ float2 apart(float2x v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ float2x fma2(float2x a, float2x b, float2x c) {
-  float2x r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ float2x add2(float2x a, float2x b) {
-  float2x r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ float2x widen(const __nv_bfloat162& v) {
-  const uint32_t w = *reinterpret_cast<const uint32_t*>(&v);
-  return both(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
-}
-__device__ __forceinline__ float exp_base2(float v) {
-  float r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
-  return r;
-}
-constexpr float kLog2E = 1.4426950408889634f;
-// e^(x - m) = 2^(x log2 e - m log2 e) in one multiply-add needs m log2 e to be finite: not where everything so far is -inf or the
-// type's lowest value
-constexpr float kFiniteFrom = -1e38f;
-__device__ __forceinline__ float2x exp2x(float2x x, float2x log2e, float2x minus_m) {
-  const float2 a = apart(fma2(x, log2e, minus_m));
-  return both(exp_base2(a.x), exp_base2(a.y));
-}
-
-__device__ __forceinline__ void add8(Share& s, const bf16x8& v, int col) {
-  raise(s, max8(v), col);
-  if (s.m < kFiniteFrom) {
-    float x[8];
-    unpack8(v, x);
-    const float m = reference(s);
-    for (int j = 0; j < 8; ++j) s.z += __expf(x[j] - m);
-    return;
-  }
-  const float2x log2e = both(kLog2E, kLog2E), minus_m = both(-s.m * kLog2E, -s.m * kLog2E);
-  float2x add = both(0.f, 0.f);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) add = add2(add, exp2x(widen(v.v[i]), log2e, minus_m));
-  const float2 sum = apart(add);
-  s.z += sum.x + sum.y;
-}
-// The target row's, with A = sum_v e^{t_v - m}(t_v - x_v): sum_v p_v (t_v - x_v) = A / Z needs no second read of the rows.
-__device__ __forceinline__ void add8_kl(Share& s, const bf16x8& tv, const bf16x8& xv, int col) {
-  raise(s, max8(tv), col);
-  if (s.m >= kFiniteFrom) {
-    const float2x log2e = both(kLog2E, kLog2E), minus_m = both(-s.m * kLog2E, -s.m * kLog2E), minus = both(-1.f, -1.f);
-    float2x add = both(0.f, 0.f), add_a = both(0.f, 0.f);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float2x t = widen(tv.v[i]), e = exp2x(t, log2e, minus_m);
-      add = add2(add, e);
-      add_a = fma2(e, fma2(widen(xv.v[i]), minus, t), add_a);
-    }
-    const float2 a = apart(add_a), sum = apart(add);
-    if (fabsf(a.x + a.y) <= 3.4e38f) {  // else an infinite logit is among them
-      s.z += sum.x + sum.y;
-      s.A += a.x + a.y;
-      return;
-    }
-  }
-  float t[8], x[8];
-  unpack8(tv, t);
-  unpack8(xv, x);
-  const float m = reference(s);
-  for (int j = 0; j < 8; ++j) {
-    const float e = __expf(t[j] - m);
-    s.z += e;
-    if (e > 0.f) s.A += e * (t[j] - x[j]);  // zero-probability targets contribute nothing
-  }
-}
-__device__ __forceinline__ void add1(Share& s, float x, float other, int col, bool cross) {
-  raise(s, x, col);
-  const float e = __expf(x - reference(s));
-  s.z += e;
-  if (cross && e > 0.f) s.A += e * (x - other);
-}
-__device__ __forceinline__ void merge(Share& a, const Share& b) {
-  const float m = fmaxf(a.m, b.m), ra = a.m == -INFINITY ? 0.f : __expf(a.m - m), rb = b.m == -INFINITY ? 0.f : __expf(b.m - m);
-  a.z = a.z * ra + b.z * rb;
-  a.A = a.A * ra + b.A * rb;
-  if (b.m > a.m || (b.m == a.m && b.col < a.col)) a.col = b.col;
-  a.m = m;
-}
-// Over the block, the same in every thread: shuffles, one exchange, and the warps' shares in order.
-template <int WARPS>
-__device__ __forceinline__ void merge_block(Share& s, Share (&slots)[WARPS]) {
+// Combine per-thread stats across the block.  Result valid in every thread.
+__device__ __forceinline__ void block_combine(RowStats& s, float* scratch, int* iscratch) {
+  const float M = block_max(s.m, scratch);
+  const float z = (s.m == -INFINITY) ? 0.f : s.z * __expf(s.m - M);
+  const float Z = block_sum(z, scratch);
+  // argmax with lowest-index tie break
+  float bv = s.best;
+  int bi = s.best_idx;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
-    Share b;
-    b.m = __shfl_xor_sync(0xffffffffu, s.m, o);
-    b.z = __shfl_xor_sync(0xffffffffu, s.z, o);
-    b.A = __shfl_xor_sync(0xffffffffu, s.A, o);
-    b.col = __shfl_xor_sync(0xffffffffu, s.col, o);
-    merge(s, b);
+    const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+    if (ov > bv || (ov == bv && oi < bi)) {
+      bv = ov;
+      bi = oi;
+    }
   }
-  if ((threadIdx.x & 31) == 0) slots[threadIdx.x >> 5] = s;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   __syncthreads();
-  s = slots[0];
+  if (lane == 0) {
+    scratch[warp] = bv;
+    iscratch[warp] = bi;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    bv = lane < nwarp ? scratch[lane] : -INFINITY;
+    bi = lane < nwarp ? iscratch[lane] : 0x7fffffff;
 #pragma unroll
-  for (int w = 1; w < WARPS; ++w) merge(s, slots[w]);
-}
-// Column of the row's maximum (the first one).
-__device__ __forceinline__ int first_max(const Share& s, const __nv_bfloat16* row, int vec_end) {
-  if (s.col >= vec_end) return s.col;
-  for (int j = 0; j < 8; ++j)
-    if (__bfloat162float(row[s.col + j]) == s.m) return s.col + j;
-  return s.col;
+    for (int o = 16; o > 0; o >>= 1) {
+      const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+      if (ov > bv || (ov == bv && oi < bi)) {
+        bv = ov;
+        bi = oi;
+      }
+    }
+    if (lane == 0) {
+      scratch[32] = bv;
+      iscratch[32] = bi;
+    }
+  }
+  __syncthreads();
+  s.m = M;
+  s.z = Z;
+  s.best = scratch[32];
+  s.best_idx = iscratch[32];
+  __syncthreads();
 }
 
-// Bound by issue and the special-function units before memory: an exponential per column and row, and beside it what the
-// maximum, its column and the sums take.  So the maximum comes from packed comparisons and its column is kept per vector of
-// eight, the sums are packed pairs, rescaling waits for a new maximum, two vectors are in flight, and the block meets once a row.  us before and after:
-// KL 1280 x 32000 56 and 47, 4096 x 32000 161 and 122; total variation (a second pass) 222 and 185; labels 2460 x 151936
-// 172 and 150 (reading takes 25, 80, 160 and 114).
-template <int OP, int THREADS>
-__global__ void __launch_bounds__(THREADS, 1536 / THREADS)
+template <int OP>
+__global__ void __launch_bounds__(kLossThreads)
 loss_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* __restrict__ targets,
                 const uint8_t* __restrict__ active, const uint8_t* __restrict__ also, const int64_t* __restrict__ labels,
                 float* __restrict__ loss, float* __restrict__ stats, int* __restrict__ argmax_d,
                 int* __restrict__ argmax_t, int rows, int V, int64_t ld_logits, int64_t ld_targets,
                 int shift, const int* __restrict__ target_row) {
   pdl_begin();
-  __shared__ Share slots[2][THREADS / 32];
   __shared__ float scratch[33];
+  __shared__ int iscratch[33];
   const int r = blockIdx.x;
   if (r >= rows) return;
   float* st = stats + r;
@@ -207,46 +106,54 @@ loss_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* _
   const bool vec_ok = ((V & 7) == 0) && ((ld_logits & 7) == 0) && ((ld_targets & 7) == 0);
   const int nvec = vec_ok ? (V >> 3) : 0;
 
-  Share sd, stt;
-  auto take = [&](const bf16x8& a, const bf16x8& b, int v) {
-    add8(sd, a, v << 3);
+  RowStats sd{-INFINITY, 0.f, -INFINITY, 0x7fffffff}, stt{-INFINITY, 0.f, -INFINITY, 0x7fffffff};
+  float kl_a = 0.f;  // OP == kOpKL: the cross term, accumulated in the same pass
+  for (int v = threadIdx.x; v < nvec; v += kLossThreads) {
+    float a[8], b[8];
+    unpack8(ld8(x + (v << 3)), a);
+    online_update(sd, a, v << 3);
     if (has_t) {
-      if (OP == kOpKL) add8_kl(stt, b, a, v << 3);
-      else add8(stt, b, v << 3);
+      unpack8(ld8(t + (v << 3)), b);
+      if (OP == kOpKL) online_update_kl(stt, kl_a, b, a, v << 3);
+      else online_update(stt, b, v << 3);
     }
-  };
-  int v = threadIdx.x;
-  for (; v + THREADS < nvec; v += 2 * THREADS) {
-    const bf16x8 a0 = ld8(x + (v << 3)), a1 = ld8(x + ((v + THREADS) << 3));
-    bf16x8 b0 = a0, b1 = a1;
-    if (has_t) {
-      b0 = ld8(t + (v << 3));
-      b1 = ld8(t + ((v + THREADS) << 3));
-    }
-    take(a0, b0, v);
-    take(a1, b1, v + THREADS);
   }
-  if (v < nvec) {
-    const bf16x8 a0 = ld8(x + (v << 3));
-    take(a0, has_t ? ld8(t + (v << 3)) : a0, v);
-  }
-  for (int c = (nvec << 3) + threadIdx.x; c < V; c += THREADS) {
+  for (int c = (nvec << 3) + threadIdx.x; c < V; c += kLossThreads) {
     const float xc = __bfloat162float(x[c]);
-    add1(sd, xc, 0.f, c, false);
-    if (has_t) add1(stt, __bfloat162float(t[c]), xc, c, OP == kOpKL);
+    online_update_scalar(sd, xc, c);
+    if (has_t) {
+      if (OP == kOpKL) online_update_kl_scalar(stt, kl_a, __bfloat162float(t[c]), xc, c);
+      else online_update_scalar(stt, __bfloat162float(t[c]), c);
+    }
   }
-  if (has_t) merge_block(stt, slots[1]);
-  merge_block(sd, slots[0]);
+  const float my_mt = stt.m;  // this thread's running max of the target row, before the block-wide combine
+  block_combine(sd, scratch, iscratch);
+  if (has_t) {
+    block_combine(stt, scratch, iscratch);
+  } else {
+    stt.m = 0.f;
+    stt.z = 1.f;
+    int lab = labels ? (int)labels[tr] : 0;
+    stt.best_idx = lab < 0 ? 0 : (lab >= V ? V - 1 : lab);
+  }
   const float lse_d = sd.m + __logf(sd.z);
-  float lse_t = 0.f;
-  if (has_t) lse_t = stt.m + __logf(stt.z);
+  const float lse_t = stt.m + __logf(stt.z);
 
   float acc0 = 0.f, acc1 = 0.f;
-  if (OP != kOpCE && OP != kOpKL) {
+  if (OP == kOpCE) {
+    if (threadIdx.x == 0) acc0 = lse_d - __bfloat162float(x[stt.best_idx]);
+  } else if (OP == kOpKL) {
+    // sum_v p_v (t_v - x_v) = (sum over threads of A rescaled to the row max) / Z_t; thread 0 adds
+    // the normaliser terms once so that the block sum below yields the row's KL directly
+    acc0 = (my_mt == -INFINITY) ? 0.f : kl_a * __expf(my_mt - stt.m) / stt.z;
+    if (threadIdx.x == 0) acc0 += lse_d - lse_t;
+  } else {
     auto body = [&](float xv, float tv) {
       const float ldp = xv - lse_d, ltp = tv - lse_t;
       const float dp = __expf(ldp), tp = __expf(ltp);
-      if (OP == kOpRKL) {
+      if (OP == kOpKL) {
+        if (tp > 0.f) acc0 += tp * (ltp - ldp);
+      } else if (OP == kOpRKL) {
         if (dp > 0.f) acc0 += dp * (ldp - ltp);
       } else if (OP == kOpJSD) {
         const float mx = fmaxf(ldp, ltp);
@@ -258,40 +165,29 @@ loss_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* _
         if (dp <= tp) acc1 += dp;
       }
     };
-    for (int v = threadIdx.x; v < nvec; v += THREADS) {
+    for (int v = threadIdx.x; v < nvec; v += kLossThreads) {
       float a[8], b[8];
       unpack8(ld8(x + (v << 3)), a);
       unpack8(ld8(t + (v << 3)), b);
 #pragma unroll
       for (int j = 0; j < 8; ++j) body(a[j], b[j]);
     }
-    for (int c = (nvec << 3) + threadIdx.x; c < V; c += THREADS)
+    for (int c = (nvec << 3) + threadIdx.x; c < V; c += kLossThreads)
       body(__bfloat162float(x[c]), __bfloat162float(t[c]));
-    acc0 = block_sum(acc0, scratch);
-    if (OP == kOpJSD || OP == kOpTV) acc1 = block_sum(acc1, scratch);
   }
+  acc0 = block_sum(acc0, scratch);
+  if (OP == kOpJSD || OP == kOpTV) acc1 = block_sum(acc1, scratch);
   if (threadIdx.x == 0) {
-    int best_t;
-    if (has_t) {
-      best_t = first_max(stt, t, nvec << 3);
-    } else {
-      const int64_t lab = labels ? labels[tr] : 0;
-      best_t = lab < 0 ? 0 : (lab >= V ? V - 1 : (int)lab);
-      stt.m = 0.f;
-      stt.z = 1.f;
-    }
     float L, extra;
-    if (OP == kOpKL) {
-      L = extra = stt.A / stt.z + lse_d - lse_t;  // sum_v p_v (t_v - x_v) and the normalisers
-    } else if (OP == kOpRKL) {
+    if (OP == kOpKL || OP == kOpRKL) {
       L = acc0;
       extra = acc0;
     } else if (OP == kOpJSD) {
       L = 0.5f * (acc0 + acc1);
       extra = acc1;
     } else if (OP == kOpCE) {
-      L = lse_d - __bfloat162float(x[best_t]);
-      extra = (float)best_t;
+      L = acc0;
+      extra = (float)stt.best_idx;
     } else {
       L = 1.f - acc0;
       extra = acc1;
@@ -302,8 +198,8 @@ loss_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* _
     st[(int64_t)2 * rows] = stt.m;
     st[(int64_t)3 * rows] = stt.z;
     st[(int64_t)4 * rows] = extra;
-    if (argmax_d) argmax_d[r] = first_max(sd, x, nvec << 3);
-    if (argmax_t) argmax_t[r] = best_t;
+    if (argmax_d) argmax_d[r] = sd.best_idx;
+    if (argmax_t) argmax_t[r] = stt.best_idx;
   }
 }
 
@@ -380,7 +276,7 @@ int launch_loss_fwd(int op, const void* logits, const void* targets, const uint8
   if (targets == nullptr && (labels == nullptr || op != kOpCE)) return -3;
   count_launch(1);
 #define SB200_LF(OPV)                                                                            \
-  launch_pdl(loss_fwd_kernel<OPV, kFwdThreads>, rows, kFwdThreads, 0, stream,                              \
+  launch_pdl(loss_fwd_kernel<OPV>, rows, kLossThreads, 0, stream,                                         \
       (const __nv_bfloat16*)logits, (const __nv_bfloat16*)targets, active, also, labels, loss, stats,   \
       argmax_d, argmax_t, rows, V, ld_logits, ld_targets, shift, target_row)
   switch (op) {
