@@ -119,8 +119,9 @@ struct Params {
   __nv_bfloat16* h;  // kSwiGLU: [M, N / 2] output, row stride ldh
   int64_t ldh;
   int staged;        // 1: C (and h) leave through shared memory and TMA stores (map_c, map_h)
-  // result = alpha * product (+ beta * addend) (+ diagonal on its diagonal), in fp32 and rounded once; 1, 1, 0 is the plain epilogue
-  float alpha, beta, diagonal;
+  // result = alpha * product (+ beta * addend), rounded where separate element-wise passes over bf16 tensors would round:
+  // alpha * bf16(product) and beta * addend each to bf16 before the sum; alpha = beta = 1 is the plain epilogue
+  float alpha, beta;
   // a stack of `batch` products: the z-th of each operand's stack, elements apart
   int batch;
   int64_t c_batch, r_batch;
@@ -261,25 +262,22 @@ __device__ __forceinline__ bool flag_wait(const int* flag, int* status, int code
   return false;
 }
 
+__device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16(x)); }
 struct Scaling {
-  float alpha, beta, diagonal;
+  float alpha, beta;
   // (the plain epilogue skips the arithmetic as a whole: the conditions are uniform)
   template <int N>
-  __device__ __forceinline__ void product(float (&f)[N], int row, int col) const {  // N columns from col on
+  __device__ __forceinline__ void product(float (&f)[N]) const {
     if (alpha != 1.f) {
 #pragma unroll
-      for (int j = 0; j < N; ++j) f[j] *= alpha;
-    }
-    if (diagonal != 0.f) {
-#pragma unroll
-      for (int j = 0; j < N; ++j) f[j] += row == col + j ? diagonal : 0.f;
+      for (int j = 0; j < N; ++j) f[j] = bf16_round(alpha * bf16_round(f[j]));
     }
   }
   template <int N>
   __device__ __forceinline__ void add(float (&f)[N], const float (&o)[N]) const {
     if (beta != 1.f) {
 #pragma unroll
-      for (int j = 0; j < N; ++j) f[j] = fmaf(beta, o[j], f[j]);
+      for (int j = 0; j < N; ++j) f[j] += bf16_round(beta * o[j]);
     } else {
 #pragma unroll
       for (int j = 0; j < N; ++j) f[j] += o[j];
@@ -409,7 +407,7 @@ __device__ __forceinline__ void store_accumulator(const Params& p, const Scaling
           float f[8];
 #pragma unroll
           for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(r[v * 8 + j]);
-          sc.product(f, row, col0 + v * 8);
+          sc.product(f);
           if (p.epilogue == kAccumulate) {
             float o[8];
             unpack8(ld8(crow + c * 32 + v * 8), o);
@@ -432,7 +430,7 @@ __device__ __forceinline__ void store_accumulator(const Params& p, const Scaling
         for (int j = 0; j < 32; ++j) {
           if (col0 + j < p.N) {
             float f[1] = {__uint_as_float(r[j])};
-            sc.product(f, row, col0 + j);
+            sc.product(f);
             if (p.epilogue != kStore) {
               const float o[1] = {__bfloat162float((p.epilogue == kAccumulate ? crow : rrow)[c * 32 + j])};
               sc.add(f, o);
@@ -564,7 +562,7 @@ __device__ __forceinline__ void store_accumulator_prefetched(const Params& p, co
       unpack8(*reinterpret_cast<const bf16x8*>(&pre.v[c * 4 + v]), o);
 #pragma unroll
       for (int j = 0; j < 8; ++j) f[j] = zero ? 0.f : __uint_as_float(r[v * 8 + j]);
-      sc.product(f, row, n0 + c * 32 + v * 8);
+      sc.product(f);
       sc.add(f, o);
       packed[v] = pack8(f);
     }
@@ -584,7 +582,7 @@ __device__ __forceinline__ void store_vec4(const Params& p, const Scaling& sc, c
   __nv_bfloat16* out = p.c + z * p.c_batch + (int64_t)row * p.ldc + col0;
   const __nv_bfloat16* add = p.epilogue == kAccumulate ? out : p.residual + z * p.r_batch + (int64_t)row * p.ldr + col0;
   float f[4] = {t.x, t.y, t.z, t.w}, o[4];
-  sc.product(f, row, col0);
+  sc.product(f);
   const bool full = col0 + 4 <= p.N && (p.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(p.c) & 7) == 0;
   if (p.epilogue != kStore) {
     for (int j = 0; j < 4; ++j) o[j] = col0 + j < p.N ? __bfloat162float(add[j]) : 0.f;
@@ -619,7 +617,7 @@ __device__ __forceinline__ void store_accumulator_staged(const Params& p, const 
         float f[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) f[j] = zero ? 0.f : __uint_as_float(r[v * 8 + j]);
-        sc.product(f, row0 + lane, n0 + c * 32 + v * 8);
+        sc.product(f);
         if (p.epilogue != kStore) {
           float o[8];
           unpack8(*reinterpret_cast<const bf16x8*>(&pre.v[c * 4 + v]), o);
@@ -758,7 +756,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   if (log_splits > 0) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // waited for before the first remote store
 
   bool ok = true;
-  const Scaling sc{p.alpha, p.beta, p.diagonal};
+  const Scaling sc{p.alpha, p.beta};
   const int quarter = warp & 3, row = m0 + quarter * 32 + lane;
   if (warp == 0) {
     if (elect_one()) {
@@ -1125,7 +1123,7 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         if (!ok) break;
       }
       const int row0 = ti.c_row0 + quarter * 32;
-      const Scaling sc{p.alpha, p.beta, p.diagonal};
+      const Scaling sc{p.alpha, p.beta};
       if (gated)  // this warp: gate columns 64 * chalf .. + 63 of the tile and the same up columns
         store_accumulator_swiglu(p, &map_c, &map_h, stage, lane_base + chalf * 64, row0, ti.n0 + chalf * 64,
                                  row0 < ti.row_end, lane);
@@ -1200,7 +1198,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   const int kb0 = split * per_kb, num_kb = max(0, min(per_kb, all_kb - kb0));
 
   bool ok = true;
-  const Scaling sc{p.alpha, p.beta, p.diagonal};
+  const Scaling sc{p.alpha, p.beta};
   const int quarter = warp & 3, chalf = (warp - 2) >> 2;
   if (warp == 0) {
     if (elect_one()) {
@@ -1437,7 +1435,7 @@ struct PartsSpec {
 struct BatchSpec {
   int batch = 1;
   int64_t a_stride = 0, b_stride = 0, c_stride = 0, r_stride = 0;
-  float alpha = 1.f, beta = 1.f, diagonal = 0.f;
+  float alpha = 1.f, beta = 1.f;
   bool symmetric = false;
 };
 
@@ -1497,7 +1495,7 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
             : make_map_bf16_stack(&map_b, b, b_stack * N, K, ldb, pairs ? P_HALF : S_TILE_N, bs.batch, bs.b_stride);
   if (rc) return rc;
   Params p{(__nv_bfloat16*)c, (const __nv_bfloat16*)residual, M, N, K, ldc, ldr, epilogue, status, RowStatsOut{nullptr, 0, 0, 0, nullptr},
-           Grouping{kGroupNone, 0, nullptr, nullptr}, Scatter{}, (__nv_bfloat16*)gated_h, gated_ldh, 0, bs.alpha, bs.beta, bs.diagonal, bs.batch,
+           Grouping{kGroupNone, 0, nullptr, nullptr}, Scatter{}, (__nv_bfloat16*)gated_h, gated_ldh, 0, bs.alpha, bs.beta, bs.batch,
            bs.c_stride, bs.r_stride, 0, live, nullptr, nullptr};
   if (live != nullptr && (grp != nullptr || scatter != nullptr || stats_targets != nullptr || bs.batch != 1 || (a_mn && !b_mn))) return -10;
   if (epilogue == kSwiGLU) {
@@ -1638,11 +1636,11 @@ int launch_gemm_parts(int n, const void* const* a, const void* const* b, const i
 }
 
 // ---- stacks of products (Newton-Schulz iterations of equally shaped matrices) ----------------------
-// c[z] = alpha * op(a[z]) * op(b[z])^T (+ beta * addend[z]) (+ diagonal * I), as in Params.
+// c[z] = alpha * op(a[z]) * op(b[z])^T (+ beta * addend[z]), rounded as in Params.
 // All stacks dense: [batch, rows, cols].  `symmetric`: the caller knows that the product is (a Gram matrix, a power of a
 // symmetric matrix): only tiles on and above the diagonal are computed.
 int launch_gemm_stack(const void* a, const void* b, void* c, const void* addend, int batch, int M, int N, int K, int a_mn, int b_mn, float alpha,
-                      float beta, float diagonal, int symmetric, int* status, SplitSpace* space, cudaStream_t stream) {
+                      float beta, int symmetric, int* status, SplitSpace* space, cudaStream_t stream) {
   BatchSpec bs;
   bs.batch = batch;
   bs.a_stride = (int64_t)M * K;
@@ -1650,7 +1648,6 @@ int launch_gemm_stack(const void* a, const void* b, void* c, const void* addend,
   bs.c_stride = bs.r_stride = (int64_t)M * N;
   bs.alpha = alpha;
   bs.beta = beta;
-  bs.diagonal = diagonal;
   bs.symmetric = symmetric != 0;
   return launch_gemm_impl(a, b, c, addend, M, N, K, a_mn ? M : K, b_mn ? N : K, N, N, addend != nullptr ? tc::kAddResidual : tc::kStore, a_mn, b_mn, status, 0,
                           nullptr, 0, 0, 0, nullptr, nullptr, stream, nullptr, nullptr, 0, &bs, nullptr, nullptr, space);

@@ -893,57 +893,28 @@ def _newton_schulz(g: torch.Tensor, steps: int, normalise: bool = True) -> torch
     tall = x.shape[0] > x.shape[1]
     for _ in range(steps):
         gram = ops.matmul_tn(x, x) if tall else ops.matmul_nt(x, x)
-        poly = b * gram.float() + c * ops.matmul_nn(gram, gram).float()
-        poly.diagonal().add_(a)
-        poly = poly.to(x.dtype)
-        x = ops.matmul_nn(x, poly) if tall else ops.matmul_nn(poly, x)
+        poly = b * gram + c * ops.matmul_nn(gram, gram)
+        nxt = a * x
+        x = ops.matmul_nn(x, poly, out=nxt, accumulate=True) if tall else ops.matmul_nn(poly, x, out=nxt, accumulate=True)
     return x.to(g.dtype)
-
-
-# Sides' ratio from which on two iterations share a Gram matrix (five of them, us one by one and in pairs: 5 x 1024 x 2048 297 and 297,
-# 5 x 1024 x 3072 358 and 334, 4096 x 12288 2548 and 1997, 28672 x 4096 5168 and 3612, 151936 x 256 524 and 361; 256 x 512 65 and 68).
-_NS_PAIRS_FROM = 2.5
 
 
 def _newton_schulz_stack(x: torch.Tensor, y: torch.Tensor, steps: int) -> None:
     """``_newton_schulz`` of a normalised CUDA bf16 stack ``[batch, m, n]``, alternating between ``x`` and the equally shaped
-    ``y``: the result is in ``y`` after an odd number of steps, else in ``x``.
-
-    One iteration is ``X <- P(G) X`` with ``P = a I + b G + c G^2`` and ``G`` the Gram matrix on the short side; ``P`` is formed
-    in the epilogue of ``G^2`` and rounded once.  ``P`` and ``G`` commute, so the next iteration's Gram matrix is ``P^2 G``: two
-    iterations share one, as ``X <- P' P X``, and what they do on the short side alone is symmetric and computed on and above
-    the diagonal only - ``3 m^2 n + 5 m^3`` FLOPs instead of ``6 m^2 n + 2 m^3`` for two, m the short side.  No more than two:
-    ``G`` holds the squares of the singular values, and what bf16 leaves of the small ones does not survive a third.
-
-    Relative error against the same polynomial in fp64, five steps, 256 x 2048 with Gaussian entries and with singular values over
-    two and four decades: 0.0080, 0.030, 0.042; iteration by iteration 0.0087, 0.024, 0.057; with ``b G + c G^2`` and
-    ``a X`` rounded on their own, as separate passes, 0.025, 0.042, 0.099."""
+    ``y``: the result is in ``y`` after an odd number of steps, else in ``x``.  Three launches per iteration: the sums
+    ``b G + c G^2`` and ``a X + X P`` are formed in the products' epilogues (rounded like the single-matrix form), and the Gram
+    matrix and its square, being symmetric, are computed on and above the diagonal only (``3 m^2 n + m^3`` FLOPs per
+    iteration instead of ``4 m^2 n + 2 m^3``, m the short side)."""
     a, b, c = 3.4445, -4.7750, 2.0315
     batch, rows, cols = x.shape
     tall = rows > cols
     short = min(rows, cols)
     nat, status = ops.native(), ops.gemm_status(x.device)
-    spare = [torch.empty((batch, short, short), dtype=x.dtype, device=x.device) for _ in range(4)]
-    # pairs of iterations come in twos, so that the result ends where it is expected
-    pairs = steps // 4 * 2 if max(rows, cols) >= _NS_PAIRS_FROM * short else 0
+    gram, poly = (torch.empty((batch, short, short), dtype=x.dtype, device=x.device) for _ in range(2))
     src, dst = x, y
-
-    def polynomial(gram, out):
-        nat.gemm_stack(gram, gram, out, gram, False, False, c, b, True, status, a)
-
-    def product(left, right, out):  # of symmetric matrices that commute
-        nat.gemm_stack(left, right, out, None, False, False, 1.0, 0.0, True, status)
-
-    for i in range(steps - pairs):
-        gram, poly, other, last = spare
+    for _ in range(steps):
         nat.gemm_stack(src, src, gram, None, tall, tall, 1.0, 0.0, True, status)
-        polynomial(gram, poly)
-        if i < pairs:
-            product(poly, gram, other)
-            product(poly, other, gram)  # P^2 G
-            polynomial(gram, other)
-            product(other, poly, last)
-            poly = last
+        nat.gemm_stack(gram, gram, poly, gram, False, False, c, b, True, status)
         left, right = (src, poly) if tall else (poly, src)  # symmetric poly: either orientation of it is the same
-        nat.gemm_stack(left, right, dst, None, False, not tall, 1.0, 0.0, False, status)
+        nat.gemm_stack(left, right, dst, src, False, not tall, 1.0, a, False, status)
         src, dst = dst, src
