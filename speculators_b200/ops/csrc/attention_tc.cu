@@ -30,6 +30,8 @@
 // All waits are bounded (tcgen05_utils.cuh): a role that runs out of budget records a code
 // in the status word, every role then leaves its loop, the CTA meets at the final barrier,
 // frees its TMEM and returns.
+#include <type_traits>
+
 #include "attention_params.h"
 #include "packed_f32.cuh"
 #include "tcgen05_utils.cuh"
@@ -440,8 +442,8 @@ attn_fwd_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 // and head, 128 wide: ~3000 there, 1890 here, 2 x 1700 of a pair's 3780 in the exponentials (a lone warp of its scheduler takes 11.5
 // clocks for one with its scaling, sum and rounding).  P shares its slot's columns with S (all 512 are taken), so the next S waits
 // for the P V product; the latter starts on the first 64 keys a quarter of the exponentials early.
-// Forward, us, one-head kernel and this one: 32 / 8 heads causal 2048 tokens 65.5 and 53, 8192 tokens 64 wide 589 and 462, 64 / 8
-// heads 4096 tokens 363 and 290, 9 documents in 8192 tokens 212 and 156, 512 anchored blocks of 16 over 4096 tokens 252 and 186.
+// Forward, us, one-head kernel and this one: 32 / 8 heads causal 2048 tokens 65.5 and 53, 8192 tokens 64 wide 589 and 445, 64 / 8
+// heads 4096 tokens 363 and 285, 9 documents in 8192 tokens 212 and 154, 512 anchored blocks of 16 over 4096 tokens 252 and 184.
 // Same results to the bit: the sums run over the same halves of a tile in the same order.
 template <int HD>
 __global__ void __launch_bounds__(PAIR_THREADS, 1)
@@ -683,36 +685,42 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_con
       // P overwrites the first half of the scores' columns as the A operand of the P.V product: key k of the row sits in the
       // 16-bit half (k & 1) of column k / 2.  The product starts on the first 64 keys while the last 32 are still to come.
       const float2x sc2 = both(sc, sc), minus_m = both(-m_sub, -m_sub);
-      float2x csum[2];
-      uint32_t pk[32];
+      auto probabilities = [&](auto masked) {
+        float2x csum[2];
+        uint32_t pk[32];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        if ((c & 1) == 0) csum[0] = csum[1] = both(0.f, 0.f);
-        if (seen & (1u << c)) {
+        for (int c = 0; c < 4; ++c) {
+          if ((c & 1) == 0) csum[0] = csum[1] = both(0.f, 0.f);
+          if (!masked.value || (seen & (1u << c))) {
 #pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            const float2 x = apart(fma2(both(__uint_as_float(r[c][i]), __uint_as_float(r[c][i + 1])), sc2, minus_m));
-            const float p0 = ex2(x.x), p1 = ex2(x.y);
-            csum[c & 1] = add2(csum[c & 1], both(p0, p1));
-            const __nv_bfloat162 h2 = __floats2bfloat162_rn(p0, p1);
-            pk[(c & 1) * 16 + (i >> 1)] = *reinterpret_cast<const uint32_t*>(&h2);
+            for (int i = 0; i < 32; i += 2) {
+              const float2 x = apart(fma2(both(__uint_as_float(r[c][i]), __uint_as_float(r[c][i + 1])), sc2, minus_m));
+              const float p0 = ex2(x.x), p1 = ex2(x.y);
+              csum[c & 1] = add2(csum[c & 1], both(p0, p1));
+              const __nv_bfloat162 h2 = __floats2bfloat162_rn(p0, p1);
+              pk[(c & 1) * 16 + (i >> 1)] = *reinterpret_cast<const uint32_t*>(&h2);
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) pk[(c & 1) * 16 + i] = 0;
           }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) pk[(c & 1) * 16 + i] = 0;
+          if (c & 1) {
+            tmem_st32(tmem_s + (c >> 1) * 32, pk);
+            const float2 a = apart(csum[0]), b = apart(csum[1]);
+            l[c >> 1] = l[c >> 1] * alpha + ((a.x + a.y) + (b.x + b.y));
+          }
+          if (c >= 2) {
+            tmem_st_wait();
+            fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_addr(&bar_p_ready[slot][c - 2]));
+          }
         }
-        if (c & 1) {
-          tmem_st32(tmem_s + (c >> 1) * 32, pk);
-          const float2 a = apart(csum[0]), b = apart(csum[1]);
-          l[c >> 1] = l[c >> 1] * alpha + ((a.x + a.y) + (b.x + b.y));
-        }
-        if (c >= 2) {
-          tmem_st_wait();
-          fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(smem_addr(&bar_p_ready[slot][c - 2]));
-        }
-      }
+      };
+      if (full)
+        probabilities(std::false_type{});  // no branch between the groups: they are worked on together
+      else
+        probabilities(std::true_type{});
     }
 
     // the finished output row comes back into registers
