@@ -20,10 +20,21 @@
 //     grouped queries the CTAs of a group write fp32 partials that a reduction kernel sums
 //     in head order.
 //
+// The products of a tile and its element-wise work take turns in both kernels (all 512 columns of TMEM are taken: S and dP of one
+// tile), so the latter counts: scaling and differences two to an instruction, groups of 32 x 32 that a warp sees wholly or not
+// at all without a test per element, and no branch between the groups of a tile that is seen as a whole.  In the dQ kernel S and
+// dP are released as soon as they are in registers.  Backward, us before and after: 32 / 8 heads causal 8192 tokens 64 wide 1626 and
+// 1479, 64 / 8 heads 4096 tokens 128 wide 1128 and 1053, 512 anchored blocks of 16 over 4096 tokens 847 and 686.  (Halves of 64
+// queries in turn in the dK / dV kernel, with the products of one under the other's exponentials: 1132 -> 1202; a product of
+// 128 x 64 costs as much shared memory bandwidth in its A operand as one of 128 x 128.)
+//
 // All waits are bounded: a role that runs out of budget records a code in the status word;
 // the element-wise threads then keep walking their loops without waiting (so that no
 // partner is left alone at a named barrier) and store nothing.
+#include <type_traits>
+
 #include "attention_params.h"
+#include "packed_f32.cuh"
 #include "tcgen05_utils.cuh"
 
 namespace sb200 {
@@ -65,12 +76,6 @@ __device__ __forceinline__ void mma_ts(uint32_t tmem_d, uint32_t a0, uint32_t a1
     const uint32_t a = kk < 4 ? a0 + kk * 8 : a1 + (kk - 4) * 8;
     umma_bf16_ts(tmem_d, a, smem_desc_mnmajor_sw128(b_tile + kk * 2048, SUB_BYTES), idesc, accumulate || kk != 0);
   }
-}
-
-// like tc::store_rows_f32, adding into global memory (several query heads of a group meet on one KV head)
-template <int W>
-__device__ __forceinline__ void atomic_rows_f32(unsigned char* stage, const float (&vals)[W], float* gbase, int64_t row_stride, int rows_valid, int lane) {
-  stage_rows_f32(stage, vals, rows_valid, lane, [&](int r, int c, float4 v) { atomicAdd(reinterpret_cast<float4*>(gbase + (int64_t)r * row_stride + c), v); });
 }
 
 __device__ __forceinline__ void pair_barrier(int quarter) { asm volatile("bar.sync %0, 64;" ::"r"(1 + quarter) : "memory"); }
@@ -282,6 +287,8 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
     const unsigned char* do_row = do_s + half_at + prow * 128;  // ... and of dO
     const float delta = row_ok ? p.delta[(int64_t)h * p.Tq + row] : 0.f;  // rowsum(dO * O), from attn_delta_kernel
 
+    const float2x sc2 = both(sc, sc), minus_lse = both(-lse, -lse), minus_delta = both(-delta, -delta);
+
     for (int t = 0; t < n_tiles; ++t) {
       if (ok) ok = mbar_wait(smem_addr(&bar_sdp_full), t & 1, status, kTimeoutDqCompute);
       ok = __all_sync(0xffffffffu, ok);
@@ -290,32 +297,45 @@ attn_bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
       const int key0 = (ext ? q0 : (j0 + t) * BN) + colh;
       const int tlo = ext ? elo : lo, thi = ext ? ehi : hi;
       const bool full = __all_sync(0xffffffffu, tlo <= key0 && thi >= key0 + 64);
-      uint32_t pk[32];
+      uint32_t pk[32], s[2][32], d[2][32];
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
-        uint32_t s[32], d[32];
-        tmem_ld32(lane_base + COL_S + colh + c * 32, s);
-        tmem_ld32(lane_base + COL_DP + colh + c * 32, d);
-        tmem_ld_wait();
-        if (c == 1) {  // S and dP of the tile are in registers: the next tile's products may overwrite them
-          fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(smem_addr(&bar_sdp_free));
-        }
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          float pr0 = ex2(fmaf(__uint_as_float(s[i]), sc, -lse));
-          float pr1 = ex2(fmaf(__uint_as_float(s[i + 1]), sc, -lse));
-          if (!full) {
-            const int key = key0 + c * 32 + i;
-            if (key < tlo || key >= thi) pr0 = 0.f;
-            if (key + 1 < tlo || key + 1 >= thi) pr1 = 0.f;
-          }
-          const float ds0 = pr0 * (__uint_as_float(d[i]) - delta);
-          const float ds1 = pr1 * (__uint_as_float(d[i + 1]) - delta);
-          pk[c * 16 + (i >> 1)] = pack_bf16(ds0, ds1);
-        }
+        tmem_ld32(lane_base + COL_S + colh + c * 32, s[c]);
+        tmem_ld32(lane_base + COL_DP + colh + c * 32, d[c]);
       }
+      tmem_ld_wait();
+      // S and dP of the tile are in registers: the next tile's products may overwrite them while this one is worked on
+      fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_addr(&bar_sdp_free));
+      auto gradients = [&](auto masked) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int from = tlo - (key0 + c * 32), to = thi - (key0 + c * 32);  // the row's keys in this group of 32
+          if (masked.value && !__any_sync(0xffffffffu, from < 32 && to > 0)) {  // none that any row of the warp sees
+#pragma unroll
+            for (int i = 0; i < 16; ++i) pk[c * 16 + i] = 0;
+            continue;
+          }
+          const bool all = !masked.value || __all_sync(0xffffffffu, from <= 0 && to >= 32);
+          const uint32_t mask = from >= 32 || to <= 0 ? 0u : (to >= 32 ? ~0u : (1u << to) - 1) & (from <= 0 ? ~0u : ~0u << from);
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) {
+            const float2 x = apart(fma2(both(__uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1])), sc2, minus_lse));
+            float pr0 = ex2(x.x), pr1 = ex2(x.y);
+            if (masked.value && !all) {
+              if (!(mask & (1u << i))) pr0 = 0.f;
+              if (!(mask & (2u << i))) pr1 = 0.f;
+            }
+            const float2 dd = apart(add2(both(__uint_as_float(d[c][i]), __uint_as_float(d[c][i + 1])), minus_delta));
+            pk[c * 16 + (i >> 1)] = pack_bf16(pr0 * dd.x, pr1 * dd.y);
+          }
+        }
+      };
+      if (full)
+        gradients(std::false_type{});  // no branch between the groups: they are worked on together
+      else
+        gradients(std::true_type{});
       if (t > 0) {
         // the previous dS K product has retired: its dS block (and, one tile on, this one) is free
         if (ok) ok = mbar_wait(smem_addr(&bar_dq_done), (t - 1) & 1, status, kTimeoutDqCompute);
@@ -448,8 +468,10 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                        const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                        const AttnParams p, int n_range_tiles, int ext_mode, int* status) {
   // ext_mode (block-structured extras): the key tiles are tiles of the extra K / V tensors (the caller passes their
-  // tensor maps as map_k / map_v); key tile j is seen by query tile j alone, under the block mask, and the result is
-  // added (fp32 atomics over the query heads of a group) into dke / dve.
+  // tensor maps as map_k / map_v), and key tile j is seen by query tile j alone, under the block mask.  A CTA per KV head
+  // takes the query heads of its group one after the other and writes the rounded sums.  (A CTA per query head had one tile
+  // each, nothing to overlap, and met the others in fp32 atomics over zeros that were converted afterwards: 512 blocks of 16,
+  // 32 / 8 heads, 204 us and the fill and conversion besides; now 87 us.)
   constexpr int TILE_BYTES = kTile<HD>, HO = HD / 2, STAGE = HD * 128;  // HO: head-dim columns of a thread; STAGE: staging bytes of a warp
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -460,16 +482,16 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   __shared__ __align__(8) uint64_t bar_kv, bar_qdo_full[2], bar_qdo_empty[2], bar_s_full, bar_dp_full, bar_p_ready, bar_ds_ready,
       bar_dv_done, bar_dk_done;
   __shared__ uint32_t tmem_base_slot;
-  // per-query statistics of the query tile in flight, two buffers
-  __shared__ __align__(16) float st_lse[2][BM];
-  __shared__ __align__(16) float st_delta[2][BM];
+  // per-query statistics (-lse, -delta, keys) of the query tile in flight, two buffers
+  __shared__ __align__(16) float st_mlse[2][BM];
+  __shared__ __align__(16) float st_mdelta[2][BM];
   __shared__ __align__(16) int st_lo[2][BM];
   __shared__ __align__(16) int st_hi[2][BM];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int h = blockIdx.x, j = blockIdx.y;  // key tile 0 is seen by the most queries under a causal mask: first
+  const int j = blockIdx.y;  // key tile 0 is seen by the most queries under a causal mask: first
   const int group = p.nh / p.nkv;
-  const int kvh = h / group;
+  const int h0 = ext_mode ? blockIdx.x * group : blockIdx.x, kvh = h0 / group;
   const int key_base = j * BN;
 
   if (threadIdx.x == 0) {
@@ -510,7 +532,9 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     }
   }
   const int i0 = ext_mode ? j : (qmax > qmin ? qmin / BM : 0);
-  const int n_tiles = ext_mode ? (j * BM < p.Tq ? 1 : 0) : (qmax > qmin ? (qmax + BM - 1) / BM - i0 : 0);
+  const int n_tiles = ext_mode ? (j * BM < p.Tq ? group : 0) : (qmax > qmin ? (qmax + BM - 1) / BM - i0 : 0);
+  // the t-th query tile: the next rows of one head, or the same rows of the group's next head
+  const int row_step = ext_mode ? 0 : BM, head_step = ext_mode ? 1 : 0;
   const int n_keys = ext_mode ? p.Te : p.Tc;
 
   if (warp == 0) {
@@ -524,7 +548,7 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         if (!mbar_wait(smem_addr(&bar_qdo_empty[st]), ((t >> 1) & 1) ^ 1, status, kTimeoutDkvProducer)) break;
         const uint32_t full = smem_addr(&bar_qdo_full[st]);
         mbar_expect_tx(full, 2 * TILE_BYTES);
-        const int r0 = (i0 + t) * BM;
+        const int r0 = i0 * BM + t * row_step, h = h0 + t * head_step;
         const uint32_t qa = smem_addr(q_s + st * TILE_BYTES), da = smem_addr(do_s + st * TILE_BYTES);
         load_tile<HD>(qa, &map_q, full, h * HD, r0);
         load_tile<HD>(da, &map_do, full, h * HD, r0);
@@ -584,14 +608,14 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     bool ok = true;
 
     // statistics of query `i0 * BM + ..` go through registers one tile ahead
-    float ld_a = 0.f, ld_b = 0.f;  // lse, delta (ct < 128) or lo, hi as bit patterns (ct >= 128)
+    float ld_a = 0.f, ld_b = 0.f;  // -lse, -delta (ct < 128) or lo, hi as bit patterns (ct >= 128)
     uint32_t ld_full = 1;
     auto fetch_stats = [&](int t) {
-      const int r = (i0 + t) * BM + (ct & (BM - 1));
+      const int r = i0 * BM + t * row_step + (ct & (BM - 1)), h = h0 + t * head_step;
       const bool in = r < p.Tq;
       if (ct < BM) {
-        ld_a = in ? p.lse2[(int64_t)h * p.Tq + r] : INFINITY;
-        ld_b = in ? p.delta[(int64_t)h * p.Tq + r] : 0.f;
+        ld_a = in ? -p.lse2[(int64_t)h * p.Tq + r] : -INFINITY;
+        ld_b = in ? -p.delta[(int64_t)h * p.Tq + r] : 0.f;
         ld_full = 1;
       } else {
         int l = in ? p.lo[r] : 0x7fffffff;
@@ -608,8 +632,8 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     auto stash_stats = [&](int t) {
       const int b = t & 1, c = ct & (BM - 1);
       if (ct < BM) {
-        st_lse[b][c] = ld_a;
-        st_delta[b][c] = ld_b;
+        st_mlse[b][c] = ld_a;
+        st_mdelta[b][c] = ld_b;
       } else {
         st_lo[b][c] = __float_as_int(ld_a);
         st_hi[b][c] = __float_as_int(ld_b);
@@ -619,6 +643,9 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       fetch_stats(0);
       stash_stats(0);
     }
+
+    const float2x sc2 = both(sc, sc);
+    const int warp_key0 = key_base + quarter * 32;
 
     for (int t = 0; t < n_tiles; ++t) {
       // all 256 threads meet: statistics of tile t are visible, and `full` says whether every
@@ -634,6 +661,16 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           : "memory");
       if (t + 1 < n_tiles) fetch_stats(t + 1);  // in flight during the tile's work
       const int b = t & 1;
+      // of 32 queries, the warp's 32 keys are mostly seen by all or by none
+      bool some[2] = {true, true}, all[2] = {true, true};
+      if (!full) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int l = st_lo[b][colh + c * 32 + lane], hgh = st_hi[b][colh + c * 32 + lane];
+          some[c] = __any_sync(0xffffffffu, l < warp_key0 + 32 && hgh > warp_key0 && l < hgh);
+          all[c] = __all_sync(0xffffffffu, l <= warp_key0 && hgh >= warp_key0 + 32);
+        }
+      }
 
       if (ok) ok = mbar_wait(smem_addr(&bar_s_full), t & 1, status, kTimeoutDkvCompute);
       ok = __all_sync(0xffffffffu, ok);
@@ -643,30 +680,42 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       for (int c = 0; c < 2; ++c) tmem_ld32(lane_base + COL_ST + colh + c * 32, s[c]);
       tmem_ld_wait();
       uint32_t pk[32];
+      auto probabilities = [&](auto masked) {
 #pragma unroll
-      for (int c = 0; c < 2; ++c)
+        for (int c = 0; c < 2; ++c) {
+          if (masked.value && !some[c]) {
 #pragma unroll
-        for (int i = 0; i < 32; i += 4) {
-          const int qi = colh + c * 32 + i;
-          const float4 l4 = *reinterpret_cast<const float4*>(&st_lse[b][qi]);
-          float pr[4];
-          pr[0] = ex2(fmaf(__uint_as_float(s[c][i]), sc, -l4.x));
-          pr[1] = ex2(fmaf(__uint_as_float(s[c][i + 1]), sc, -l4.y));
-          pr[2] = ex2(fmaf(__uint_as_float(s[c][i + 2]), sc, -l4.z));
-          pr[3] = ex2(fmaf(__uint_as_float(s[c][i + 3]), sc, -l4.w));
-          if (!full) {
-            const int4 lo4 = *reinterpret_cast<const int4*>(&st_lo[b][qi]);
-            const int4 hi4 = *reinterpret_cast<const int4*>(&st_hi[b][qi]);
-            if (key < lo4.x || key >= hi4.x) pr[0] = 0.f;
-            if (key < lo4.y || key >= hi4.y) pr[1] = 0.f;
-            if (key < lo4.z || key >= hi4.z) pr[2] = 0.f;
-            if (key < lo4.w || key >= hi4.w) pr[3] = 0.f;
+            for (int i = 0; i < 32; ++i) s[c][i] = 0u;
+#pragma unroll
+            for (int i = 0; i < 16; ++i) pk[c * 16 + i] = 0u;
+            continue;
           }
 #pragma unroll
-          for (int u = 0; u < 4; ++u) s[c][i + u] = __float_as_uint(pr[u]);
-          pk[c * 16 + (i >> 1)] = pack_bf16(pr[0], pr[1]);
-          pk[c * 16 + (i >> 1) + 1] = pack_bf16(pr[2], pr[3]);
+          for (int i = 0; i < 32; i += 4) {
+            const int qi = colh + c * 32 + i;
+            const float4 l4 = *reinterpret_cast<const float4*>(&st_mlse[b][qi]);
+            const float2 x = apart(fma2(both(__uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1])), sc2, both(l4.x, l4.y)));
+            const float2 y = apart(fma2(both(__uint_as_float(s[c][i + 2]), __uint_as_float(s[c][i + 3])), sc2, both(l4.z, l4.w)));
+            float pr[4] = {ex2(x.x), ex2(x.y), ex2(y.x), ex2(y.y)};
+            if (masked.value && !all[c]) {
+              const int4 lo4 = *reinterpret_cast<const int4*>(&st_lo[b][qi]);
+              const int4 hi4 = *reinterpret_cast<const int4*>(&st_hi[b][qi]);
+              if (key < lo4.x || key >= hi4.x) pr[0] = 0.f;
+              if (key < lo4.y || key >= hi4.y) pr[1] = 0.f;
+              if (key < lo4.z || key >= hi4.z) pr[2] = 0.f;
+              if (key < lo4.w || key >= hi4.w) pr[3] = 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) s[c][i + u] = __float_as_uint(pr[u]);
+            pk[c * 16 + (i >> 1)] = pack_bf16(pr[0], pr[1]);
+            pk[c * 16 + (i >> 1) + 1] = pack_bf16(pr[2], pr[3]);
+          }
         }
+      };
+      if (full)
+        probabilities(std::false_type{});  // no branch between the two groups: they are worked on together
+      else
+        probabilities(std::true_type{});
       tmem_st32(lane_base + COL_ST + colh, pk);  // P^T over the first half of this thread's own S^T columns
       tmem_st_wait();
       fence_before_sync();
@@ -684,13 +733,11 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       for (int c = 0; c < 2; ++c)
 #pragma unroll
         for (int i = 0; i < 32; i += 4) {
-          const float4 d4 = *reinterpret_cast<const float4*>(&st_delta[b][colh + c * 32 + i]);
-          const float ds0 = __uint_as_float(s[c][i]) * (__uint_as_float(d[c][i]) - d4.x);
-          const float ds1 = __uint_as_float(s[c][i + 1]) * (__uint_as_float(d[c][i + 1]) - d4.y);
-          const float ds2 = __uint_as_float(s[c][i + 2]) * (__uint_as_float(d[c][i + 2]) - d4.z);
-          const float ds3 = __uint_as_float(s[c][i + 3]) * (__uint_as_float(d[c][i + 3]) - d4.w);
-          pk[c * 16 + (i >> 1)] = pack_bf16(ds0, ds1);
-          pk[c * 16 + (i >> 1) + 1] = pack_bf16(ds2, ds3);
+          const float4 d4 = *reinterpret_cast<const float4*>(&st_mdelta[b][colh + c * 32 + i]);
+          const float2 x = apart(add2(both(__uint_as_float(d[c][i]), __uint_as_float(d[c][i + 1])), both(d4.x, d4.y)));
+          const float2 y = apart(add2(both(__uint_as_float(d[c][i + 2]), __uint_as_float(d[c][i + 3])), both(d4.z, d4.w)));
+          pk[c * 16 + (i >> 1)] = pack_bf16(__uint_as_float(s[c][i]) * x.x, __uint_as_float(s[c][i + 1]) * x.y);
+          pk[c * 16 + (i >> 1) + 1] = pack_bf16(__uint_as_float(s[c][i + 2]) * y.x, __uint_as_float(s[c][i + 3]) * y.y);
         }
       tmem_st32(lane_base + COL_DPT + colh, pk);  // dS^T over the first half of this thread's own dP^T columns
       tmem_st_wait();
@@ -725,12 +772,11 @@ attn_bwd_dkv_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       if (__all_sync(0xffffffffu, ok)) {
         // whole rows through the warp's staging area (the Q / dO stages are idle by now)
         unsigned char* stage = q_s + (warp - 2) * STAGE;
-        const int warp_key0 = key_base + quarter * 32;
         const int64_t off0 = ((int64_t)warp_key0 * p.nkv + kvh) * HD + colo;
         if (ext_mode)
-          atomic_rows_f32(stage, acc, (which ? p.dve : p.dke) + off0, (int64_t)p.nkv * HD, n_keys - warp_key0, lane);
+          store_rows_bf16(stage, acc, 1.f, (which ? p.dve16 : p.dke16) + off0, (int64_t)p.nkv * HD, n_keys - warp_key0, lane);
         else if (p.dkv_part != nullptr)
-          store_rows_f32(stage, acc, p.dkv_part + (int64_t)(h - kvh * group) * 2 * plane + which * plane + off0, (int64_t)p.nkv * HD,
+          store_rows_f32(stage, acc, p.dkv_part + (int64_t)(h0 - kvh * group) * 2 * plane + which * plane + off0, (int64_t)p.nkv * HD,
                            p.Tc - warp_key0, lane);
         else
           store_rows_bf16(stage, acc, 1.f, (which ? p.dv : p.dk) + off0, (int64_t)p.nkv * HD, p.Tc - warp_key0, lane);
@@ -773,7 +819,7 @@ static int launch_bwd(const AttnParams& p, int* tile_qmin, int* tile_qmax, int* 
   if (rc) return rc;
   CUtensorMap map_ke = map_k, map_ve = map_v;
   if (p.ext_block > 0) {
-    if (p.E != 0 || BM % p.ext_block != 0 || p.ke == nullptr || p.ve == nullptr || p.dke == nullptr || p.dve == nullptr) return -4;
+    if (p.E != 0 || BM % p.ext_block != 0 || p.ke == nullptr || p.ve == nullptr || p.dke16 == nullptr || p.dve16 == nullptr) return -4;
     rc = tc::make_map_bf16(&map_ke, p.ke, p.Te, (int64_t)p.nkv * HD, p.ke_rs, BN);
     if (rc) return rc;
     rc = tc::make_map_bf16(&map_ve, p.ve, p.Te, (int64_t)p.nkv * HD, p.ve_rs, BN);
@@ -795,7 +841,7 @@ static int launch_bwd(const AttnParams& p, int* tile_qmin, int* tile_qmax, int* 
   launch_pdl(attn_bwd_dkv_tc_kernel<HD>, grid_kv, THREADS, kSmem<HD>, stream, map_q, map_do, map_k, map_v, p, (p.Tc + kAttnKeyTile - 1) / kAttnKeyTile, 0, status);
   if (p.ext_block > 0) {  // gradients of the extra keys: one key tile per query tile, read from the extra tensors
     count_launch(1);
-    dim3 grid_ext(p.nh, (p.Te + BN - 1) / BN);
+    dim3 grid_ext(p.nkv, (p.Te + BN - 1) / BN);
     launch_pdl(attn_bwd_dkv_tc_kernel<HD>, grid_ext, THREADS, kSmem<HD>, stream, map_q, map_do, map_ke, map_ve, p, 0, 1, status);
   }
   if (p.dkv_part != nullptr) {

@@ -35,6 +35,8 @@ struct AttnParams {
   int64_t dq_rs;
   float* dke;            // [Te, nkv, HD] fp32 (atomics)
   float* dve;
+  __nv_bfloat16* dke16;  // [Te, nkv, HD]: the gradients of block-structured extras
+  __nv_bfloat16* dve16;
   __nv_bfloat16* dk;     // [Tc, nkv, HD] contiguous
   __nv_bfloat16* dv;
   float* dkv_part;       // [group, 2, Tc, nkv, HD] fp32 per-query-head partials of dK / dV (grouped-query attention only)

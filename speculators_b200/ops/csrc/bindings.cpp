@@ -1436,7 +1436,13 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> attn_bwd(
   Tensor dv = at::empty({k.size(0), k.size(1), hd}, q.options());
   Tensor delta = at::empty({q.size(1), q.size(0)}, lse2.options());
   Tensor dke, dve;
-  if (p.E > 0 || p.ext_block > 0) {
+  if (p.ext_block > 0) {
+    const Tensor both = at::empty({2, p.Te, p.nkv, hd}, q.options());
+    dke = both.select(0, 0);
+    dve = both.select(0, 1);
+    p.dke16 = (__nv_bfloat16*)dke.data_ptr();
+    p.dve16 = (__nv_bfloat16*)dve.data_ptr();
+  } else if (p.E > 0) {
     const Tensor both = at::zeros({2, p.Te, p.nkv, hd}, lse2.options());
     dke = both.select(0, 0);
     dve = both.select(0, 1);
@@ -1470,7 +1476,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> attn_bwd(
                  : impl == 1 ? sb200::launch_attn_bwd_tc(p, (int)hd, qmin.data_ptr<int>(), qmax.data_ptr<int>(), status->data_ptr<int>(), cur_stream())
                            : sb200::launch_attn_bwd(p, (int)hd, qmin.data_ptr<int>(), qmax.data_ptr<int>(), cur_stream());
   TORCH_CHECK(rc == 0, "attn_bwd launch failed (", rc, ")");
-  if (dke.numel() > 0) {  // both gradients of the extra keys in the inputs' type with one conversion
+  if (p.E > 0) {  // both gradients of the extra keys in the inputs' type with one conversion
     const Tensor both = at::as_strided(dke, {2, p.Te, p.nkv, hd}, {(int64_t)p.Te * p.nkv * hd, p.nkv * hd, hd, 1}).to(q.scalar_type());
     dke = both.select(0, 0);
     dve = both.select(0, 1);
