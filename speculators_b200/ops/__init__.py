@@ -108,7 +108,7 @@ def gemm_status(device: torch.device) -> torch.Tensor:
 
 
 _WAIT_CODES = {
-    1: "GEMM producer", 2: "GEMM MMA issuer", 3: "GEMM epilogue",
+    1: "GEMM producer", 2: "GEMM MMA issuer", 3: "GEMM epilogue", 4: "GEMM partial sums of a divided tile",
     31: "attention forward producer", 32: "attention forward MMA issuer", 33: "attention forward softmax",
     41: "attention dQ producer", 42: "attention dQ MMA issuer", 43: "attention dQ element-wise warps",
     44: "attention dK/dV producer", 45: "attention dK/dV MMA issuer", 46: "attention dK/dV element-wise warps",
