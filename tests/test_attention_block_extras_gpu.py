@@ -22,6 +22,8 @@ def test_gradients(heads, kv, blocks, block, head_dim):
                     extra_block=block)
     ke, ve = ke.requires_grad_(), ve.requires_grad_()
     masked_attention(q.requires_grad_(), k, v, spec, ke, ve).backward(go)
+    again = torch.autograd.grad(masked_attention(q, k, v, spec, ke, ve), (ke, ve), go)
+    assert torch.equal(again[0], ke.grad) and torch.equal(again[1], ve.grad)  # the heads of a group meet in a fixed order
 
     seen = torch.cat([torch.arange(context, device="cuda") < hi[:, None], rows[:, None] // block == rows // block], 1)
     group, scale = heads // kv, head_dim**-0.5
