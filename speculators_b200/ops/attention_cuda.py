@@ -38,7 +38,7 @@ def _tensor_core_shape(q: torch.Tensor, ext_idx: torch.Tensor | None) -> bool:
     is filled by 128 resident rows and leaves none to stage individually addressed extra keys in); 64 from 513 query rows on -
     up to there a head is a few key tiles, and setting up tensor memory costs what the products save (128 tokens, 4 heads:
     10 / 55 us forward / backward on mma.sync, 11 / 61 here; 512 tokens 15 / 61 and 15 / 68; 1001 tokens, 32 heads 42 / 117
-    and 26 / 73; 8192 tokens 1189 / 3543 and 593 / 1644)."""
+    and 26 / 73; 8192 tokens 1189 / 3543 and 445 / 1479)."""
     hd = q.shape[2]
     return hd == 128 or (hd == 64 and q.shape[0] > 512) or (hd == 256 and ext_idx is None)
 
