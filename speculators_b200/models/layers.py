@@ -34,6 +34,7 @@ __all__ = [
     "RMSNorm",
     "RotaryTable",
     "takes_listed_rows",
+    "unobserved",
 ]
 
 
@@ -336,9 +337,20 @@ class MLP(nn.Module):
 NEEDED_ROWS_FROM = 1 << 19
 
 
+def unobserved(*modules: nn.Module) -> bool:
+    """Whether nobody looks into ``modules``: no hook, of a module in their trees or of all modules, that would get to see the
+    listed rows, moved together and with unwritten rows behind them, in the place of the batch's."""
+    if torch.nn.modules.module._has_any_global_hook():  # noqa: SLF001
+        return False
+    return not any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks  # noqa: SLF001
+                   for module in modules for m in module.modules())
+
+
 def takes_listed_rows(layers, *linears: nn.Module) -> bool:
     """Whether decoder layers (``self_attn``, ``mlp``) and further linear layers may run over the rows that ``ops.step_rows``
-    lists: every operator between them is a kernel that stops at the device's row count."""
+    lists: every operator between them is a kernel that stops at the device's row count, and nobody watches."""
+    if not unobserved(*layers):
+        return False
     linears = list(linears)
     for layer in layers:
         attn, mlp = layer.self_attn, layer.mlp

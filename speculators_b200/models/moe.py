@@ -36,7 +36,7 @@ from torch import nn
 
 from speculators_b200 import ops
 from speculators_b200.layer_config import TransformerLayerConfig
-from speculators_b200.models.layers import FusedLinear, Linear, RotaryTable, takes_listed_rows
+from speculators_b200.models.layers import FusedLinear, Linear, RotaryTable, takes_listed_rows, unobserved
 from speculators_b200.models.mtp.model_definitions import _MTPMixin
 from speculators_b200.ops import AttnSpec
 from speculators_b200.ops.moe import moe_experts, moe_experts_ok
@@ -390,7 +390,9 @@ class MoEMTPLayer(_MTPMixin, MoEDecoderLayer):
         self._setup_mtp_modules(config, norm_cls=ZeroCenteredRMSNorm)
 
     def takes_listed_rows(self) -> bool:
-        """Whether ``rows`` may be given: all experts on this rank, every operator a kernel that stops at the row count."""
+        """Whether ``rows`` may be given: all experts on this rank, every operator a kernel that stops at the row count, no hooks."""
+        if not unobserved(self):
+            return False
         attn, mlp = self.self_attn, self.mlp
         linears = [attn.q_proj, attn.k_proj, attn.v_proj, attn.o_proj, mlp.gate]
         if mlp.shared_expert is not None:

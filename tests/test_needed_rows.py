@@ -287,3 +287,93 @@ def test_gpu_mtp_step_over_needed_rows(monkeypatch, T, kind, experts, head_dim):
         assert torch.isfinite(grads_needed[n]).all(), n
         assert float((grads_needed[n] - v).norm()) <= 1e-2 * float(v.norm()) + 1e-12, (n, float((grads_needed[n] - v).norm() / v.norm()))
     ops.check_gemm_status()
+
+
+# --------------------------------------------------------------------------- who watches sees the whole batch
+def _poison():
+    torch.cuda.empty_cache()  # nothing older is handed out
+    held = [torch.full((1 << 27,), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(4)]
+    del held  # what a pass allocates and does not write holds NaN
+
+
+def _watched(model, where, seen):
+    """A hook, of one kind or another, that keeps what the module at ``where`` takes or gives."""
+    place, _, kind = where.partition(":")
+    module = {"layer": lambda: model.layers[0], "mlp": lambda: model.layers[0].mlp, "norm": lambda: model.norm, "verifier_norm": lambda: model.verifier_norm,
+              "embed_tokens": lambda: model.embed_tokens}[place]()
+
+    def keep(tensors):
+        seen.append([t.detach().clone() for t in (tensors if isinstance(tensors, tuple) else (tensors,)) if isinstance(t, torch.Tensor)])
+
+    if kind == "pre":
+        return module.register_forward_pre_hook(lambda m, args: keep(args))
+    if kind == "backward":
+        return module.register_full_backward_hook(lambda m, taken, given: keep(given))
+    if kind == "global":
+        return torch.nn.modules.module.register_module_forward_hook(lambda m, args, out: keep(out) if m is module else None)
+    return module.register_forward_hook(lambda m, args, out: keep(out))
+
+
+@pytest.mark.parametrize("register", ["register_forward_hook", "register_forward_pre_hook", "register_full_backward_hook", "register_full_backward_pre_hook"])
+def test_hooks_are_noticed(register):
+    from speculators_b200.models.layers import unobserved
+
+    layer = _mtp(0, 32, 8, 64).mtp_layers[0]
+    for module in (layer, layer.mlp.down_proj):
+        handle = getattr(module, register)(lambda *_: None)
+        assert not unobserved(layer) and not unobserved(torch.nn.Identity(), layer)
+        handle.remove()
+        assert unobserved(layer)
+    handle = torch.nn.modules.module.register_module_forward_pre_hook(lambda *_: None)
+    assert not unobserved(layer)
+    handle.remove()
+    assert unobserved(layer)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("where", ["layer", "layer:pre", "layer:backward", "mlp", "mlp:global", "norm", "verifier_norm", "embed_tokens"])
+def test_gpu_hooks_see_the_rows_of_the_batch(monkeypatch, where):
+    model, batch = _model(1, 64, False, 688, True), _gpu_batch(2100, "spans")
+    kwargs, _ = Eagle3DraftModel.get_trainer_kwargs(loss_fn="kl_div", ttt_steps=3, ttt_step_loss_decay=0.8)
+    results = []
+    for whole in (True, False):
+        with monkeypatch.context() as patched:
+            if whole:
+                patched.setattr(Eagle3DraftModel, "_takes_needed_rows", lambda *_: False)
+            seen = []
+            handle = _watched(model, where, seen)
+            _poison()
+            _, loss, _ = model(**batch, **kwargs)
+            loss.backward()
+            handle.remove()
+            results.append(seen)
+    want, got = results
+    assert len(got) == len(want) == (1 if where == "verifier_norm" else 3)
+    for a, b in zip(got, want):
+        assert len(a) == len(b) > 0
+        for x, y in zip(a, b):  # the same route: the same bits but for the atomics behind the gradients of irregular extra keys
+            assert x.shape == y.shape and float((x.float() - y.float()).norm()) <= 1e-2 * float(y.float().norm())
+    assert model._takes_needed_rows(2100, batch["loss_mask"], kwargs["loss_config"], 3)  # and nobody watches any more
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("experts", [0, 8])
+def test_gpu_mtp_hooks_see_the_rows_of_the_batch(experts):
+    T = 1540
+    model = _mtp(experts, 512, 256 if experts else 64, 1000).cuda().bfloat16()
+    batch = {"input_ids": torch.randint(0, 1000, (1, T)).cuda(), "hidden_states": torch.randn(1, T, 512).bfloat16().cuda(), "loss_mask": _mask("spans", T)[None].cuda()}
+    results = []
+    for kwargs in ({"return_logits": True}, {"return_logits": False}):
+        seen = []
+        with torch.no_grad():
+            handle = model.mtp_layers[0].register_forward_hook(lambda m, args, out: seen.append(out.clone()))
+            _poison()
+            model(**batch, **kwargs)
+            handle.remove()
+        results.append(seen)
+    want, got = results
+    assert len(want) == len(got) == 3
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+
+
