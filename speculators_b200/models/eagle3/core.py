@@ -35,7 +35,7 @@ from speculators_b200.model import DraftVocabMixin, SpeculatorModel
 from speculators_b200.models.eagle3.attention import causal_document_interval, ttt_attn_spec
 from speculators_b200.models.eagle3.config import Eagle3SpeculatorConfig
 from speculators_b200.models.eagle3.metrics import compute_metrics, compute_metrics_from_hidden, compute_metrics_of_rows, step_tail_is_fused
-from speculators_b200.models.layers import MLP, NEEDED_ROWS_FROM, Attention, DecoderLayer, Linear, RMSNorm, RotaryTable, takes_listed_rows, unobserved
+from speculators_b200.models.layers import MLP, NEEDED_ROWS_FROM, Attention, DecoderLayer, Linear, RMSNorm, RotaryTable, stops_at_count, takes_listed_rows, unobserved
 from speculators_b200.models.utils import resolve_target_layer_ids
 from speculators_b200.ops import AttnSpec
 from speculators_b200.proposals.greedy import GreedyTokenProposalConfig
@@ -43,6 +43,7 @@ from speculators_b200.proposals.greedy import GreedyTokenProposalConfig
 __all__ = ["Eagle3DraftModel", "Eagle3FirstLayer"]
 
 
+@stops_at_count
 class Eagle3FirstLayer(nn.Module):
     """Decoder block whose attention reads ``cat([embeds, hidden])`` (2H): both
     halves are normalised separately, the residual is the hidden half (normalised
@@ -143,14 +144,14 @@ class Eagle3DraftModel(DraftVocabMixin, SpeculatorModel):
     # ------------------------------------------------------------------ forward
     def _takes_needed_rows(self, rows: int, loss_mask, loss_config, ttt_steps: int) -> bool:
         """Whether a step may leave out the rows that no loss term or counter reads (``ops.step_rows``): the loss and counters
-        run as one fused tail over listed rows, every operator in between is a kernel that stops at the count, and no hook
-        waits for the batch's rows."""
+        run as one fused tail over listed rows, every operator in between is a kernel that stops at the count, and no hook or
+        module of the caller's waits for the batch's rows."""
         if loss_mask is None or rows <= 256 or rows * self.hidden_size < NEEDED_ROWS_FROM or ttt_steps <= 0 or not step_tail_is_fused(loss_config):
             return False
         if not loss_mask.is_cuda or loss_mask.numel() != rows or ops.fused_head_enabled() or self.hidden_size > 32768:
             return False
         return (all(type(layer) is (DecoderLayer if i else Eagle3FirstLayer) for i, layer in enumerate(self.layers))
-                and unobserved(self.embed_tokens, self.norm, self.verifier_norm)
+                and type(self.norm) is type(self.verifier_norm) is RMSNorm and unobserved(self.embed_tokens, self.norm, self.verifier_norm)
                 and takes_listed_rows(self.layers, self.lm_head, self.verifier_lm_head)
                 and all(n.weight.dtype == torch.bfloat16 for n in (self.norm, self.verifier_norm)))
 

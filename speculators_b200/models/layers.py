@@ -33,11 +33,33 @@ __all__ = [
     "NEEDED_ROWS_FROM",
     "RMSNorm",
     "RotaryTable",
+    "stops_at_count",
     "takes_listed_rows",
     "unobserved",
 ]
 
 
+_ROW_MODULES: set[type] = {nn.Embedding}
+
+
+def stops_at_count(cls: type) -> type:
+    """Class decorator: a module of this class runs over the rows in use alone (``live``, ``rows``), or row by row.  A class
+    derived from it says so itself or counts as one that reads all rows."""
+    _ROW_MODULES.add(cls)
+    return cls
+
+
+def unobserved(*modules: nn.Module) -> bool:
+    """Whether nobody looks into ``modules``: no hook, of a module in their trees or of all modules, that would get to see the
+    listed rows, moved together and with unwritten rows behind them, in the place of the batch's; and no module that would
+    run over those, of a class of its own or with its ``forward`` replaced."""
+    if torch.nn.modules.module._has_any_global_hook():  # noqa: SLF001
+        return False
+    return not any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks  # noqa: SLF001
+                   or type(m) not in _ROW_MODULES or "forward" in vars(m) for module in modules for m in module.modules())
+
+
+@stops_at_count
 class RMSNorm(nn.Module):
     def __init__(self, hidden_size: int, eps: float = 1e-6):
         super().__init__()
@@ -60,6 +82,7 @@ def _init_linear_(weight: torch.Tensor, std: float = 0.02) -> None:
         weight.normal_(mean=0.0, std=std)
 
 
+@stops_at_count
 class Linear(nn.Module):
     """Bias-optional linear layer; weight ``[out, in]`` like ``nn.Linear``."""
 
@@ -82,6 +105,7 @@ class Linear(nn.Module):
         return f"in={self.in_features}, out={self.out_features}, bias={self.bias is not None}"
 
 
+@stops_at_count
 class FusedLinear(nn.Module):
     """Several projections of the same input stored as one ``[sum(out), in]`` weight.
 
@@ -212,6 +236,7 @@ class RotaryTable(nn.Module):
             self._build(int(max_pos * 2))
 
 
+@stops_at_count
 class Attention(nn.Module):
     """Grouped-query self-attention over an ``AttnSpec`` mask.
 
@@ -299,6 +324,7 @@ _GATE_ACTIVATIONS = {
 }
 
 
+@stops_at_count
 class MLP(nn.Module):
     """Gated MLP ``down(act(gate(x)) * up(x))``.  SiLU (every supported verifier family's default)
     runs on the fused SwiGLU kernel; the other activations the reference accepts through
@@ -337,15 +363,6 @@ class MLP(nn.Module):
 NEEDED_ROWS_FROM = 1 << 19
 
 
-def unobserved(*modules: nn.Module) -> bool:
-    """Whether nobody looks into ``modules``: no hook, of a module in their trees or of all modules, that would get to see the
-    listed rows, moved together and with unwritten rows behind them, in the place of the batch's."""
-    if torch.nn.modules.module._has_any_global_hook():  # noqa: SLF001
-        return False
-    return not any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks  # noqa: SLF001
-                   for module in modules for m in module.modules())
-
-
 def takes_listed_rows(layers, *linears: nn.Module) -> bool:
     """Whether decoder layers (``self_attn``, ``mlp``) and further linear layers may run over the rows that ``ops.step_rows``
     lists: every operator between them is a kernel that stops at the device's row count, and nobody watches."""
@@ -366,6 +383,7 @@ def takes_listed_rows(layers, *linears: nn.Module) -> bool:
     )
 
 
+@stops_at_count
 class DecoderLayer(nn.Module):
     """Pre-norm decoder block (Llama / Qwen3 layout)."""
 

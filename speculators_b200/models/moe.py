@@ -36,7 +36,7 @@ from torch import nn
 
 from speculators_b200 import ops
 from speculators_b200.layer_config import TransformerLayerConfig
-from speculators_b200.models.layers import FusedLinear, Linear, RotaryTable, takes_listed_rows, unobserved
+from speculators_b200.models.layers import FusedLinear, Linear, RotaryTable, stops_at_count, takes_listed_rows, unobserved
 from speculators_b200.models.mtp.model_definitions import _MTPMixin
 from speculators_b200.ops import AttnSpec
 from speculators_b200.ops.moe import moe_experts, moe_experts_ok
@@ -44,6 +44,7 @@ from speculators_b200.ops.moe import moe_experts, moe_experts_ok
 __all__ = ["GatedAttention", "MoEDecoderLayer", "MoEMTPLayer", "SparseMoeBlock", "ZeroCenteredRMSNorm", "expert_forward"]
 
 
+@stops_at_count
 class ZeroCenteredRMSNorm(nn.Module):
     """``x / rms(x) * (1 + weight)`` with the weight initialised to zero."""
 
@@ -59,6 +60,7 @@ class ZeroCenteredRMSNorm(nn.Module):
         return ops.rms_norm_fork(x, self.weight, self.variance_epsilon, centred=True, live=live)
 
 
+@stops_at_count
 class GatedAttention(nn.Module):
     def __init__(self, config: TransformerLayerConfig, layer_idx: int):
         super().__init__()
@@ -111,6 +113,7 @@ class GatedAttention(nn.Module):
         return self.o_proj(ops.gated(out, gate).view(T, self.nh * self.hd), residual=residual, live=live)
 
 
+@stops_at_count
 class _Experts(nn.Module):
     def __init__(self, num_local: int, hidden: int, inter: int):
         super().__init__()
@@ -118,6 +121,7 @@ class _Experts(nn.Module):
         self.down_proj = nn.Parameter(torch.empty(num_local, hidden, inter).normal_(std=0.02))
 
 
+@stops_at_count
 class _SharedExpert(nn.Module):
     """The always-on expert: a gated MLP with the gate | up projections stored as one weight (one GEMM with the
     activation in its epilogue on CUDA); its state dict keeps the ``gate_proj`` / ``up_proj`` / ``down_proj`` names."""
@@ -210,6 +214,7 @@ def _grouped_expert_forward(x_sorted: torch.Tensor, counts: torch.Tensor, gate_u
     return expert_forward(x_sorted, ids, gate_up, down)
 
 
+@stops_at_count
 class SparseMoeBlock(nn.Module):
     def __init__(self, config: TransformerLayerConfig, ep_group=None):
         super().__init__()
@@ -381,6 +386,7 @@ class MoEDecoderLayer(nn.Module):
         return self.mlp(normed, residual=x, live=live)
 
 
+@stops_at_count
 class MoEMTPLayer(_MTPMixin, MoEDecoderLayer):
     """``ep_group``: process group over which the experts are split (expert parallelism); ``None``
     keeps all experts on every rank."""
@@ -390,7 +396,8 @@ class MoEMTPLayer(_MTPMixin, MoEDecoderLayer):
         self._setup_mtp_modules(config, norm_cls=ZeroCenteredRMSNorm)
 
     def takes_listed_rows(self) -> bool:
-        """Whether ``rows`` may be given: all experts on this rank, every operator a kernel that stops at the row count, no hooks."""
+        """Whether ``rows`` may be given: all experts on this rank, every operator a kernel that stops at the row count, nobody
+        watches (``unobserved``)."""
         if not unobserved(self):
             return False
         attn, mlp = self.self_attn, self.mlp

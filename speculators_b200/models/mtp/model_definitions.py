@@ -14,7 +14,7 @@ import torch
 from torch import nn
 
 from speculators_b200.layer_config import TransformerLayerConfig
-from speculators_b200.models.layers import DecoderLayer, Linear, RMSNorm, takes_listed_rows
+from speculators_b200.models.layers import DecoderLayer, Linear, RMSNorm, stops_at_count, takes_listed_rows
 
 __all__ = ["MTPLayer", "MTPLayerMixin", "build_mtp_layer", "mtp_model_classes", "resolve_model_type"]
 
@@ -40,6 +40,7 @@ class _MTPMixin:
         return self.input_proj(torch.cat([self.token_layernorm(token_embeddings), self.hidden_layernorm(hidden_states)], dim=-1))
 
 
+@stops_at_count
 class MTPLayer(_MTPMixin, DecoderLayer):
     """Dense decoder block variant."""
 

@@ -377,3 +377,97 @@ def test_gpu_mtp_hooks_see_the_rows_of_the_batch(experts):
         assert torch.equal(a, b)
 
 
+
+
+class _WithAdapter(torch.nn.Module):
+    """What ``_adapted`` puts behind a linear layer: a trained path over every row that comes in."""
+
+    def __init__(self, width_in: int, width_out: int):
+        super().__init__()
+        self.a, self.b = torch.nn.Parameter(torch.randn(8, width_in) * 0.05), torch.nn.Parameter(torch.randn(width_out, 8) * 0.05)
+
+    def forward(self, x):
+        return x @ self.a.T @ self.b.T
+
+
+def _adapted(linear, as_class: bool):
+    linear.adapter = _WithAdapter(linear.in_features, linear.out_features).to(linear.weight.device, linear.weight.dtype)
+    base = type(linear).forward
+    if as_class:
+        class Adapted(type(linear)):
+            def forward(self, x, residual=None, live=None):
+                return base(self, x, residual=residual, live=live) + self.adapter(x)
+
+        linear.__class__ = Adapted
+    else:
+        linear.forward = lambda x, residual=None, live=None: base(linear, x, residual=residual, live=live) + linear.adapter(x)
+
+
+def test_modules_of_the_users_own_are_noticed():
+    from speculators_b200.models.layers import RMSNorm, unobserved
+
+    class Own(RMSNorm):
+        pass
+
+    for experts in (0, 8):
+        layer = _mtp(experts, 512, 256, 64).mtp_layers[0]
+        assert unobserved(layer)
+        norm = layer.final_layernorm
+        layer.final_layernorm = Own(512)
+        assert not unobserved(layer)
+        layer.final_layernorm = norm
+        assert unobserved(layer)
+        norm.forward = lambda x, live=None: x
+        assert not unobserved(layer)
+
+
+@pytest.mark.gpu
+def test_gpu_a_verifier_norm_of_the_users_own_is_called(monkeypatch):
+    """Whatever it has for weights."""
+    model, batch = _model(1, 64, False, 688, True), _gpu_batch(2100, "spans")
+    kwargs, _ = Eagle3DraftModel.get_trainer_kwargs(loss_fn="kl_div", ttt_steps=3, ttt_step_loss_decay=0.8)
+
+    class Halved(type(model.verifier_norm)):
+        def forward(self, x):
+            return super().forward(x) * 0.5
+
+    halved = Halved(256).cuda().bfloat16()
+    for norm in (halved, torch.nn.Identity()):
+        model.verifier_norm = norm
+        losses = []
+        for whole in (True, False):
+            with monkeypatch.context() as patched, torch.no_grad():
+                if whole:
+                    patched.setattr(Eagle3DraftModel, "_takes_needed_rows", lambda *_: False)
+                losses.append(float(model(**batch, **kwargs)[1]))
+        assert losses[0] == losses[1]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("as_class", [True, False])
+@pytest.mark.parametrize("algorithm", ["eagle3", "mtp"])
+def test_gpu_modules_of_the_users_own_run_over_the_rows_of_the_batch(monkeypatch, algorithm, as_class):
+    torch.manual_seed(3)
+    if algorithm == "eagle3":
+        model, batch = _model(1, 64, False, 688, True), _gpu_batch(2100, "spans")
+        kwargs, _ = Eagle3DraftModel.get_trainer_kwargs(loss_fn="kl_div", ttt_steps=3, ttt_step_loss_decay=0.8)
+    else:
+        model = _mtp(0, 512, 64, 1000).cuda().bfloat16()
+        batch = {"input_ids": torch.randint(0, 1000, (1, 1540)).cuda(), "hidden_states": torch.randn(1, 1540, 512).bfloat16().cuda(), "loss_mask": _mask("spans", 1540)[None].cuda()}
+        kwargs = {"return_logits": False}
+    _adapted(model.layers[0].mlp.down_proj, as_class)
+    results = []
+    for whole in (True, False):
+        with monkeypatch.context() as patched:
+            if whole:
+                patched.setattr(type(model), "_takes_needed_rows", lambda *_: False)
+            for p in model.parameters():
+                p.grad = None
+            _poison()
+            _, loss, _ = model(**batch, **kwargs)
+            loss.backward()
+            results.append([float(loss)] + [p.grad.float() for p in model.layers[0].mlp.down_proj.adapter.parameters()])
+    (loss, *grads), (loss_got, *grads_got) = results
+    assert abs(loss_got - loss) <= 2e-4 * abs(loss)
+    for got, want in zip(grads_got, grads):  # rounded to bf16 on the way, sums in another order (MTP's head takes the listed rows)
+        assert float((got - want).norm()) <= 1e-2 * float(want.norm())
