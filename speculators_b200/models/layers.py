@@ -36,6 +36,7 @@ __all__ = [
     "stops_at_count",
     "takes_listed_rows",
     "unobserved",
+    "watched",
 ]
 
 
@@ -49,14 +50,18 @@ def stops_at_count(cls: type) -> type:
     return cls
 
 
+def watched(module: nn.Module) -> bool:
+    """Whether somebody gets to see what ``module`` itself takes and gives: a hook, its own or one of all modules, or a
+    ``forward`` put in the place of its class's."""
+    return bool(torch.nn.modules.module._has_any_global_hook() or module._forward_hooks or module._forward_pre_hooks  # noqa: SLF001
+                or module._backward_hooks or module._backward_pre_hooks or "forward" in vars(module))  # noqa: SLF001
+
+
 def unobserved(*modules: nn.Module) -> bool:
-    """Whether nobody looks into ``modules``: no hook, of a module in their trees or of all modules, that would get to see the
-    listed rows, moved together and with unwritten rows behind them, in the place of the batch's; and no module that would
-    run over those, of a class of its own or with its ``forward`` replaced."""
-    if torch.nn.modules.module._has_any_global_hook():  # noqa: SLF001
-        return False
-    return not any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks  # noqa: SLF001
-                   or type(m) not in _ROW_MODULES or "forward" in vars(m) for module in modules for m in module.modules())
+    """Whether nobody looks into ``modules``: none in their trees is watched, by what would get to see the listed rows, moved
+    together and with unwritten rows behind them, in the place of the batch's, and none is of a class of its own, which would
+    run over those."""
+    return not any(type(m) not in _ROW_MODULES or watched(m) for module in modules for m in module.modules())
 
 
 @stops_at_count

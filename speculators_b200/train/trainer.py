@@ -33,6 +33,7 @@ import torch
 import torch.distributed as dist
 
 from speculators_b200.model import SpeculatorModel
+from speculators_b200.models.layers import watched
 from speculators_b200.parallel.distributed import get_local_rank, get_rank, is_distributed, set_training_group, training_rank
 from speculators_b200.parallel.engine import EngineConfig, TrainEngine
 from speculators_b200.train.checkpointer import Checkpointer
@@ -335,8 +336,14 @@ class Trainer:
         self.setup_optimizer()
 
     def loss_only(self, call_kwargs: dict | None) -> dict:
-        """What the model is called with: the configured arguments, and what lets it leave out results that nobody takes here."""
-        return {**getattr(self.model, "loss_only_kwargs", {}), **(call_kwargs or {})}
+        """What the model is called with: the configured arguments, and what lets it leave out results that nobody takes.  They
+        are taken here for their loss and metrics alone; but a hook on the model, or a ``forward`` of another class than the
+        one that offers to leave something out, may read the rest."""
+        model = self.model
+        offers = next((cls for cls in type(model).__mro__ if "loss_only_kwargs" in vars(cls)), None)
+        if offers is None or type(model).forward is not offers.forward or watched(model):
+            return dict(call_kwargs or {})
+        return {**offers.loss_only_kwargs, **(call_kwargs or {})}
 
     # ------------------------------------------------------------------ setup
     def _training_state_path(self, epoch) -> Path:

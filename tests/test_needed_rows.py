@@ -471,3 +471,39 @@ def test_gpu_modules_of_the_users_own_run_over_the_rows_of_the_batch(monkeypatch
     assert abs(loss_got - loss) <= 2e-4 * abs(loss)
     for got, want in zip(grads_got, grads):  # rounded to bf16 on the way, sums in another order (MTP's head takes the listed rows)
         assert float((got - want).norm()) <= 1e-2 * float(want.norm())
+
+
+def test_trainer_asks_for_logits_that_somebody_takes():
+    from types import SimpleNamespace
+
+    from speculators_b200.models.mtp import MTPDraftModel
+    from speculators_b200.train import Trainer
+
+    class Reads(MTPDraftModel):
+        def forward(self, *args, **kwargs):
+            logits, loss, metrics = super().forward(*args, **kwargs)
+            metrics["peak"] = logits[0].max()
+            return logits, loss, metrics
+
+    class Keeps(MTPDraftModel):
+        pass
+
+    def asked(model):
+        return Trainer.loss_only(SimpleNamespace(model=model), {"step_weights": None})
+
+    def of(cls):
+        model = _mtp(0, 32, 8, 64)
+        model.__class__ = cls
+        return model
+
+    lean, full = {"return_logits": False, "step_weights": None}, {"step_weights": None}
+    assert asked(of(MTPDraftModel)) == lean and asked(of(Keeps)) == lean
+    assert asked(of(Reads)) == full
+    model = of(MTPDraftModel)
+    handle = model.register_forward_hook(lambda m, args, out: None)
+    assert asked(model) == full
+    handle.remove()
+    assert asked(model) == lean
+    model.forward = lambda *args, **kwargs: MTPDraftModel.forward(model, *args, **kwargs)
+    assert asked(model) == full
+    assert asked(torch.nn.Identity()) == full
