@@ -110,7 +110,7 @@ class GatedAttention(nn.Module):
         q, gate = ops.split_gated_query(qg, self.q_norm.weight, self.q_norm.variance_epsilon, live * self.nh)
         q = ops.rope_(q, rows.positions[0], rotary.cos, rotary.sin, self.nh, self.hd, self.rot)
         out = ops.masked_attention(q, k, v, spec, scale=self.scaling)
-        return self.o_proj(ops.gated(out, gate).view(T, self.nh * self.hd), residual=residual, live=live)
+        return self.o_proj(ops.gated(out, gate, live).view(T, self.nh * self.hd), residual=residual, live=live)
 
 
 @stops_at_count

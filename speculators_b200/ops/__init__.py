@@ -129,11 +129,17 @@ def check_gemm_status() -> None:
 # ``live`` (here and below): an int32 tensor on the device that says how many of the rows hold anything (``step_rows``).  The
 # kernels neither read nor write the rows behind; what runs elsewhere takes all rows, and a sum over rows leaves those out.
 def only_live(x2: torch.Tensor, live: torch.Tensor | None) -> torch.Tensor:
-    """``x2`` with zeros in the rows from ``live`` on."""
+    """``x2`` (rows first) with zeros in the rows from ``live`` on."""
     if live is None:
         return x2
     used = torch.arange(x2.shape[0], device=x2.device) < live
-    return torch.where(used[:, None], x2, torch.zeros((), dtype=x2.dtype, device=x2.device))
+    return torch.where(used.view(-1, *[1] * (x2.dim() - 1)), x2, torch.zeros((), dtype=x2.dtype, device=x2.device))
+
+
+def _settled(d: torch.Tensor | None, live: torch.Tensor | None) -> torch.Tensor | None:
+    """A gradient that a backward pass hands on.  Nothing reads its rows from ``live`` on but autograd's anomaly detection, which
+    looks for NaN in all of them: zeros for it."""
+    return d if d is None or live is None or not (torch.is_anomaly_enabled() and torch.is_anomaly_check_nan_enabled()) else only_live(d, live)
 
 
 def _forward_gemm(x2: torch.Tensor, w: torch.Tensor, residual: torch.Tensor | None, live: torch.Tensor | None = None) -> torch.Tensor:
@@ -481,7 +487,7 @@ def _linear_backward(x2, weight, rows, use, dy, need_dx: bool, need_dw: bool, li
             else:
                 dy2, x2 = (only_live(t, live if own else None) for t in (dy2, x2))
                 dw[r0:r1] = dy2.t() @ x2
-    return dx, dw
+    return _settled(dx, live), dw
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = None, residual: torch.Tensor | None = None,
@@ -589,7 +595,7 @@ def _norm_backward(dy, dy2, x2, weight, rstd, residual_grad, need_dx: bool, need
     dw, accumulate, attached = _param_grad_target(weight) if need_dw else (None, False, False)
     if need_dx or need_dw:
         native().rmsnorm_bwd(dy, dy2, x2, weight, rstd, residual_grad if need_dx else None, dx, dw, accumulate, centred, live)
-    return dx, None if attached else dw
+    return _settled(dx, live), None if attached else dw
 
 
 class _RMSNormPairFn(torch.autograd.Function):
@@ -729,7 +735,7 @@ class _SwiGLUFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dh):
         gate_up, live = ctx.saved_tensors
-        return native().swiglu_bwd_rows(dh.contiguous(), gate_up, live), None
+        return _settled(native().swiglu_bwd_rows(dh.contiguous(), gate_up, live), live), None
 
 
 class _GateUpSwiGLUFn(torch.autograd.Function):
@@ -849,7 +855,7 @@ class _RopeSplitFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dq, dk, dv):
         *tables, live = ctx.saved_tensors
-        return _unrotate(dq, dk, dv, *tables, *ctx.cfg, live), None, None, None, None, None, None, None, None, None
+        return _settled(_unrotate(dq, dk, dv, *tables, *ctx.cfg, live), live), None, None, None, None, None, None, None, None, None
 
 
 # --------------------------------------------------------------------------- per-head norms and rotation
@@ -894,7 +900,7 @@ class _NormRopeHeadsFn(torch.autograd.Function):
         dw_a, acc_a, flat_a = _param_grad_target(w_a) if ctx.needs_input_grad[1] else (None, False, False)
         dw_b, acc_b, flat_b = _param_grad_target(w_b) if nb and ctx.needs_input_grad[2] else (None, False, False)
         d = native().heads_bwd(rows, src.shape[0] if split is None else split, src, rstd, w_a, na, w_b, nb, nv, dw_a, acc_a, dw_b, acc_b, positions, cos_t, sin_t, hd, rot, repeated, live)
-        return d, None if flat_a else dw_a, None if flat_b else dw_b, None, None, None, None, None, None, None, None, None, None
+        return _settled(d, live), None if flat_a else dw_a, None if flat_b else dw_b, None, None, None, None, None, None, None, None, None, None
 
 
 def norm_rope_heads(src: torch.Tensor, w_a, w_b, eps: float, positions, cos_t, sin_t, heads: tuple[int, int, int], hd: int, rot: int,
@@ -1104,21 +1110,21 @@ class _SplitGatedQueryFn(torch.autograd.Function):
         rows = T * heads
         dw, accumulate, attached = _param_grad_target(weight) if ctx.needs_input_grad[1] else (None, False, False)
         native().rmsnorm_bwd(_grad_rows(dq, hd), None, qg.view(rows, two)[:, :hd], weight, rstd, None, d.view(rows, two)[:, :hd], dw, accumulate, True, live)
-        return d, None if attached else dw, None, None
+        return _settled(d.view(rows, two), live).view(qg.shape), None if attached else dw, None, None
 
 
 class _GatedFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, out, gate):
-        ctx.save_for_backward(out, gate)
+    def forward(ctx, out, gate, live):
+        ctx.save_for_backward(out, gate, live)
         return native().gate_mul_fwd(out, gate)
 
     @staticmethod
     def backward(ctx, dy):
-        out, gate = ctx.saved_tensors
+        out, gate, live = ctx.saved_tensors
         T, heads, hd = out.shape
         dgate = torch.empty((T, heads, gate.stride(1)), dtype=out.dtype, device=out.device)[..., -hd:]  # of a projection: its second half
-        return native().gate_mul_bwd(dy.contiguous(), out, gate, dgate), dgate
+        return _settled(native().gate_mul_bwd(dy.contiguous(), out, gate, dgate), live), _settled(dgate, live), None
 
 
 def split_gated_query(qg: torch.Tensor, weight: torch.Tensor, eps: float, live: torch.Tensor | None = None):
@@ -1129,9 +1135,10 @@ def split_gated_query(qg: torch.Tensor, weight: torch.Tensor, eps: float, live: 
     return _SplitGatedQueryFn.apply(qg, weight, eps, live)
 
 
-def gated(out: torch.Tensor, gate: torch.Tensor) -> torch.Tensor:
-    """``out * sigmoid(gate)`` for ``[T, heads, hd]`` CUDA tensors, ``gate`` as ``split_gated_query`` returns it."""
-    return _GatedFn.apply(out.contiguous(), gate)
+def gated(out: torch.Tensor, gate: torch.Tensor, live: torch.Tensor | None = None) -> torch.Tensor:
+    """``out * sigmoid(gate)`` for ``[T, heads, hd]`` CUDA tensors, ``gate`` as ``split_gated_query`` returns it (``live``: tokens
+    in use; the kernels run over all)."""
+    return _GatedFn.apply(out.contiguous(), gate, live)
 
 
 def rope_split(qkv, positions, cos_t, sin_t, heads: int, hd: int, rot: int, nq: int, nk: int, live: torch.Tensor | None = None):
@@ -1278,7 +1285,7 @@ class _StepLossFn(torch.autograd.Function):
         logits, targets, stats, weight, target_row, live = ctx.saved_tensors
         op, shift, rows = ctx.cfg
         d = native().loss_bwd_scaled(op, logits, targets, weight, dtotal.float(), stats, shift, rows, target_row, live)
-        return d, None, dtotal if ctx.needs_input_grad[2] else None, None, None, None, None, None, None, None, None, None
+        return _settled(d, live), None, dtotal if ctx.needs_input_grad[2] else None, None, None, None, None, None, None, None, None, None
 
 
 def ttt_step_loss(op: str, logits, targets, earlier, shift: int, rows: int, mask, prev_correct, decay: float, eps: float, target_row=None, live=None):
@@ -1375,7 +1382,7 @@ class _TokenCEFn(torch.autograd.Function):
         logits, stats, live = ctx.saved_tensors
         # the CE backward only needs the saved label (stats[4]) and the draft statistics
         d = native().loss_bwd_scaled(LOSS_OPS["ce"], logits, logits, dloss.contiguous().float(), None, stats, 0, logits.shape[0], None, live)
-        return d, None, None, None
+        return _settled(d, live), None, None, None
 
 
 def token_cross_entropy(logits: torch.Tensor, labels: torch.Tensor, keep: torch.Tensor | None = None, live: torch.Tensor | None = None) -> torch.Tensor:

@@ -49,7 +49,8 @@ class _MoEExpertsFn(torch.autograd.Function):
         nat, status = ops.native(), ops.gemm_status(dout.device)
         need = ctx.needs_input_grad
         dout = dout.contiguous()
-        dy_pad, dp, dshared, dgate = nat.moe_combine_bwd(dout, y_pad, row_slot, seg, top_p, shared, gate, live)
+        dy_pad, *grads = nat.moe_combine_bwd(dout, y_pad, row_slot, seg, top_p, shared, gate, live)
+        dp, dshared, dgate = (ops._settled(d, live) if d.numel() else d for d in grads)  # noqa: SLF001
 
         def weight_gradient(needed, dy, rows, w, use):
             if not needed:
@@ -78,7 +79,7 @@ class _MoEExpertsFn(torch.autograd.Function):
             if need[0]:
                 dx_pad = torch.empty_like(x_pad)
                 nat.gemm_grouped_rows(dgu, w_gu, dx_pad, True, seg, tiles, status)
-                dx = nat.moe_gather_bwd(dx_pad, slot_row, top_p.shape[1], live)
+                dx = ops._settled(nat.moe_gather_bwd(dx_pad, slot_row, top_p.shape[1], live), live)  # noqa: SLF001
         with_shared = shared is not None
         return dx, dp, None, dw_gu, dw_d, dshared if with_shared else None, dgate if with_shared else None, dout if ctx.with_residual else None, None, None
 

@@ -2,6 +2,7 @@
 and the whole pass against the pass over all rows."""
 
 import copy
+import warnings
 
 import pytest
 import torch
@@ -507,3 +508,31 @@ def test_trainer_asks_for_logits_that_somebody_takes():
     model.forward = lambda *args, **kwargs: MTPDraftModel.forward(model, *args, **kwargs)
     assert asked(model) == full
     assert asked(torch.nn.Identity()) == full
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("algorithm", ["eagle3", "eagle3 head norms", "mtp", "mtp experts"])
+@pytest.mark.parametrize("forward_too", [True, False])
+def test_gpu_anomaly_detection_finds_nothing_in_a_sound_step(monkeypatch, algorithm, forward_too):
+    """It looks for NaN in every gradient, also in rows that nobody wrote."""
+    if algorithm.startswith("eagle3"):
+        qwen = algorithm.endswith("norms")
+        model, batch = _model(2 if qwen else 1, 64, qwen, 688, True), _gpu_batch(2100, "spans")
+        kwargs, _ = Eagle3DraftModel.get_trainer_kwargs(loss_fn="kl_div", ttt_steps=3, ttt_step_loss_decay=0.8)
+    else:
+        experts = 8 if algorithm.endswith("experts") else 0
+        model = _mtp(experts, 512, 256 if experts else 64, 1000).cuda().bfloat16()
+        batch = {"input_ids": torch.randint(0, 1000, (1, 1540)).cuda(), "hidden_states": torch.randn(1, 1540, 512).bfloat16().cuda(), "loss_mask": _mask("spans", 1540)[None].cuda()}
+        kwargs = {"return_logits": False}
+    taken = []
+    monkeypatch.setattr(ops, "step_rows", lambda *args, made=ops.step_rows, **kw: taken.append(1) or made(*args, **kw))
+    with warnings.catch_warnings():
+        warnings.simplefilter("ignore")  # that it is slow
+        with torch.autograd.set_detect_anomaly(forward_too):
+            _poison()
+            _, loss, _ = model(**batch, **kwargs)
+        _poison()
+        with torch.autograd.set_detect_anomaly(True):
+            loss.backward()
+    assert taken and torch.isfinite(loss)
+    assert all(torch.isfinite(p.grad).all() for p in model.parameters() if p.grad is not None)
