@@ -56,6 +56,13 @@ def test_pass_over_needed_rows_equals_the_whole_pass(tiny_verifier_dir, tiny_voc
 
 
 # --------------------------------------------------------------------------- on a GPU
+def _poison():
+    """What is allocated from here on and not written holds NaN: free memory does, and nothing freed earlier is left beside it."""
+    torch.cuda.empty_cache()
+    held = [torch.full((1 << 27,), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(4)]
+    del held
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("T", [1, 255, 256, 257, 1000, 1024, 8192, 8200, 20011])
 @pytest.mark.parametrize("kind", KINDS)
@@ -188,8 +195,7 @@ def test_gpu_pass_over_needed_rows(monkeypatch, T, kind, layers, head_dim, qwen,
         monkeypatch.setattr(Eagle3DraftModel, "_takes_needed_rows", lambda *_, n=needed: n)
         for p in model.parameters():
             p.grad = None
-        poison = [torch.full((1 << 27,), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(4)]
-        del poison  # what the pass allocates and does not write holds NaN
+        _poison()
         _, loss, metrics = model(**batch, **kwargs)
         loss.backward()
         results.append(({k: v.float().cpu() for k, v in metrics.items()}, {n: p.grad.float() for n, p in model.named_parameters() if p.grad is not None}))
@@ -248,8 +254,7 @@ def _mtp_results(model, batch, monkeypatch):
         for p in model.parameters():
             p.grad = None
         if batch["input_ids"].is_cuda:
-            poison = [torch.full((1 << 27,), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(4)]
-            del poison
+            _poison()
         logits, loss, metrics = model(**batch, return_logits=False, step_weights=[0.5, 0.3, 0.2])
         assert logits == []
         loss.backward()
@@ -291,12 +296,6 @@ def test_gpu_mtp_step_over_needed_rows(monkeypatch, T, kind, experts, head_dim):
 
 
 # --------------------------------------------------------------------------- who watches sees the whole batch
-def _poison():
-    torch.cuda.empty_cache()  # nothing older is handed out
-    held = [torch.full((1 << 27,), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(4)]
-    del held  # what a pass allocates and does not write holds NaN
-
-
 def _watched(model, where, seen):
     """A hook, of one kind or another, that keeps what the module at ``where`` takes or gives."""
     place, _, kind = where.partition(":")
@@ -536,3 +535,45 @@ def test_gpu_anomaly_detection_finds_nothing_in_a_sound_step(monkeypatch, algori
             loss.backward()
     assert taken and torch.isfinite(loss)
     assert all(torch.isfinite(p.grad).all() for p in model.parameters() if p.grad is not None)
+
+
+# --------------------------------------------------------------------------- one graph, batches of any density
+@pytest.mark.gpu
+@pytest.mark.parametrize("algorithm", ["eagle3", "mtp", "mtp experts"])
+def test_gpu_one_graph_replayed_over_masks_of_any_density(monkeypatch, tmp_path, algorithm):
+    """The rows are listed inside the graph: a replay with fewer or more of them than the capture had gives that batch's gradients."""
+    from speculators_b200.train import Trainer, TrainerConfig
+    from speculators_b200.train.synthetic import SyntheticLoader
+
+    if algorithm == "eagle3":
+        model, batch = _model(1, 64, False, 688, True), _gpu_batch(2100, "all")
+        kwargs, _ = Eagle3DraftModel.get_trainer_kwargs(loss_fn="kl_div", ttt_steps=3, ttt_step_loss_decay=0.8)
+        T, cls = 2100, Eagle3DraftModel
+        lossy = batch["loss_mask"].clone()
+    else:
+        experts = 8 if algorithm.endswith("experts") else 0
+        T, model = 1540, _mtp(experts, 512, 256 if experts else 64, 1000).cuda().bfloat16()
+        g = torch.Generator().manual_seed(1)
+        batch = {"input_ids": torch.randint(0, 1000, (1, T), generator=g).cuda(), "hidden_states": torch.randn(1, T, 512, generator=g).bfloat16().cuda()}
+        lossy, kwargs, cls = torch.ones(1, T, dtype=torch.bool, device="cuda"), {"step_weights": [0.5, 0.3, 0.2]}, type(model)
+    g = torch.Generator().manual_seed(5)
+    at = torch.rand((T + 31) // 32, generator=g).repeat_interleave(32)[:T].cuda()[None]
+
+    def trainer(graph):
+        return Trainer(copy.deepcopy(model), TrainerConfig(lr=0.0, weight_decay=0.0, num_epochs=1, save_path=str(tmp_path), train_call_kwargs=kwargs, scheduler_type="none",
+                                                           log_freq=10**9, use_cuda_graph=graph, device="cuda:0"), SyntheticLoader([batch], 1))
+
+    graphed, eager = trainer(True), trainer(False)
+    for density in (0.6, 0.0, 1.0, 0.2, 0.6, 0.0, 0.2, 1.0):
+        one = dict(batch, loss_mask=lossy & (at < density))
+        loss, _ = graphed.train_step(one)
+        loss, grads = float(loss), graphed.engine.flat_g.float().clone()
+        with monkeypatch.context() as patched:
+            patched.setattr(cls, "_takes_needed_rows", lambda *_: False)
+            want, _ = eager.train_step(one)
+            want, want_grads = float(want), eager.engine.flat_g.float().clone()
+        assert len(graphed._graphed.cache) == 1
+        assert abs(loss - want) <= 2e-4 * abs(want) + 1e-6, density
+        # bf16 gradients, sums over rows and queries in another order
+        assert torch.isfinite(grads).all() and float((grads - want_grads).norm()) <= 1e-2 * float(want_grads.norm()) + 1e-12, density
+    ops.check_gemm_status()
