@@ -862,6 +862,11 @@ static int launch_fwd(const AttnParams& p, int* status, cudaStream_t stream) {
   // Pairs need an even group, and a wave and a half of them: half as many blocks of nearly twice the length leave a short grid
   // waiting for the longest.  32 / 8 heads, us one head and pairs a block: 777 tokens (0.75 waves of pairs) 24.6 and 28.7, 1100
   // (0.97) 32.8 and 35.6, 1500 (1.3) 45.1 and 43, 2048 (1.7) 65.5 and 53; 16 / 8 heads 3000 tokens (1.3) 67.6 and 73.7.
+  // Of listed rows (step_rows) the grid holds more tiles than have keys, and theirs see keys further apart than a short batch's
+  // tiles do, so the rule goes by all of them; one head and pairs, without extra keys | with two a row:
+  //   2048 tokens, 512 rows listed 37.9 and 50.2 | 64.5 and 76.8; 1024: 46.0 and 48.1 | 80.8 and 74.7; 1280: 52.1 and 46.1 | 95.3 and 91.1;
+  //   1792: 62.5 and 52.2 | 113.7 and 105.3; 64 / 8 heads 1536 tokens, 512: 48.1 and 44.0 | 90.9 and 72.5; 16 / 8 heads 4096 tokens, 1024: 42.0 and
+  //   54.3 | 68.6 and 82.9, 2560: 62.3 and 52.2 | 107.5 and 99.3.  It loses where a short grid has a quarter of its rows listed.
   const int tiles = (p.Tq + BM - 1) / BM;
   if ((p.nh / p.nkv) % 2 == 0 && (int64_t)p.nh * tiles >= 3 * kNumSM)
     launch_pdl(attn_fwd_pair_kernel<HD>, dim3(p.nh / 2, tiles), PAIR_THREADS, pair_smem_bytes, stream, map_q, map_k, map_v, map_ke, map_ve, p, status);

@@ -141,7 +141,7 @@ const uint8_t* row_flags(const c10::optional<Tensor>& t, int64_t rows) {
 // Partial sums come from the caching allocator, for the launch alone.  Counters and flags have to be zero when the kernel starts,
 // and a launch of a captured graph finds them used at its next replay: they come in slabs of kSlots launches that one memset
 // zeroes, on the launch's stream and - under capture - as a node of the graph, in whose memory the slab then is.  A slot
-// serves one launch.  The slab in use is kept per stream and capture (the last kSlabs of them, 300 KB each); one that is
+// serves one launch.  The slab in use is kept per stream and capture (the last kSlabs of them, 600 KB each); one that is
 // dropped goes back to the allocator in its stream's order, behind the launches that use it.
 struct SyncSlabs {
   static constexpr int kSlots = 64, kSlabs = 32;

@@ -1380,6 +1380,10 @@ static int resident_clusters(int size) {
 //   pair tiles over 2, 4 pairs: 10.8 + 0.66 / step, one wave only               (1000 x 2048 x 8192: 31.9 at 2)
 // Several waves of small tiles are bound by L2-to-SM traffic, so they pay a full wave each; the model drops them
 // quickly.  Products of more than about two waves of pair tiles always come out as pair tiles.
+// Where the device's count bounds the rows, M is the most there can be: a captured launch serves any count, and
+// so does the choice.  It stays the best form, or within 2 us of it, down to half the rows: 1001 x 2048 x 8192 with 1001, 768 and 512 rows in
+// use: 2 pairs 41.0, 38.9 and 38.9, pair tiles 53.2, 53.2 and 51.2, 128 x 64 tiles 57.3, 56.2 and 36.9; 1001 x 3072 x 4096: pair tiles
+// 34.8, 32.8 and 32.8, 128 x 64 tiles 49.2, 38.9 and 34.8.
 // divide: tiles may be divided between pairs.  Gradients' products may; a forward product, whose rows give the same bits in a batch
 // of any size (with all rows or only the needed ones), is not divided by what is left over of its tiles.
 static int choose_variant(int M, int N, int K, int batch, int symmetric, bool divide) {
