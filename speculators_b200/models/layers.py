@@ -371,8 +371,9 @@ NEEDED_ROWS_FROM = 1 << 19
 
 def takes_listed_rows(layers, *linears: nn.Module) -> bool:
     """Whether decoder layers (``self_attn``, ``mlp``) and further linear layers may run over the rows that ``ops.step_rows``
-    lists: every operator between them is a kernel that stops at the device's row count, and nobody watches."""
-    if not unobserved(*layers):
+    lists: every operator between them is a kernel that stops at the device's row count, nobody
+    watches, and what is saved for the backward pass goes through no hook of the caller's, which would pack unwritten rows too."""
+    if not unobserved(*layers) or torch._C._autograd._top_saved_tensors_default_hooks(True) is not None:  # noqa: SLF001
         return False
     linears = list(linears)
     for layer in layers:

@@ -577,3 +577,38 @@ def test_gpu_one_graph_replayed_over_masks_of_any_density(monkeypatch, tmp_path,
         # bf16 gradients, sums over rows and queries in another order
         assert torch.isfinite(grads).all() and float((grads - want_grads).norm()) <= 1e-2 * float(want_grads.norm()) + 1e-12, density
     ops.check_gemm_status()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("algorithm", ["eagle3", "mtp"])
+def test_gpu_saved_tensor_hooks_get_tensors_of_the_batch(monkeypatch, algorithm):
+    """A hook that packs what is saved by its largest value: no row may hold what nobody wrote."""
+    if algorithm == "eagle3":
+        model, batch = _model(1, 64, False, 688, True), _gpu_batch(2100, "spans")
+        kwargs, _ = Eagle3DraftModel.get_trainer_kwargs(loss_fn="kl_div", ttt_steps=3, ttt_step_loss_decay=0.8)
+    else:
+        model = _mtp(0, 512, 64, 1000).cuda().bfloat16()
+        batch = {"input_ids": torch.randint(0, 1000, (1, 1540)).cuda(), "hidden_states": torch.randn(1, 1540, 512).bfloat16().cuda(), "loss_mask": _mask("spans", 1540)[None].cuda()}
+        kwargs = {"return_logits": False}
+    largest = []
+
+    def pack(t):
+        if t.is_floating_point() and t.numel():
+            largest.append(t.detach().abs().max())
+        return t
+
+    results = []
+    for whole in (True, False):
+        with monkeypatch.context() as patched:
+            if whole:
+                patched.setattr(type(model), "_takes_needed_rows", lambda *_: False)
+            largest.clear()
+            _poison()
+            with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t):
+                _, loss, _ = model(**batch, **kwargs)
+            results.append(torch.stack([v.float() for v in largest]))
+    assert torch.isfinite(results[0]).sum() == torch.isfinite(results[1]).sum() and results[0].shape == results[1].shape
+    taken = []
+    monkeypatch.setattr(ops, "step_rows", lambda *args, made=ops.step_rows, **kw: taken.append(1) or made(*args, **kw))
+    model(**batch, **kwargs)
+    assert taken
