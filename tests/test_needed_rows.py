@@ -612,3 +612,19 @@ def test_gpu_saved_tensor_hooks_get_tensors_of_the_batch(monkeypatch, algorithm)
     monkeypatch.setattr(ops, "step_rows", lambda *args, made=ops.step_rows, **kw: taken.append(1) or made(*args, **kw))
     model(**batch, **kwargs)
     assert taken
+
+
+@pytest.mark.gpu
+def test_gpu_forward_mode_is_refused_as_before(monkeypatch):
+    from torch.autograd import forward_ad
+
+    model, batch = _model(1, 64, False, 688, True), _gpu_batch(2100, "spans")
+    kwargs, _ = Eagle3DraftModel.get_trainer_kwargs(loss_fn="kl_div", ttt_steps=3, ttt_step_loss_decay=0.8)
+    states = batch["verifier_last_hidden_states"]
+    for whole in (True, False):
+        with monkeypatch.context() as patched, forward_ad.dual_level():
+            if whole:
+                patched.setattr(Eagle3DraftModel, "_takes_needed_rows", lambda *_: False)
+            dual = forward_ad.make_dual(states, torch.ones_like(states))
+            with pytest.raises(Exception, match="jvp"):
+                model(**dict(batch, verifier_last_hidden_states=dual), **kwargs)
