@@ -50,18 +50,33 @@ def stops_at_count(cls: type) -> type:
     return cls
 
 
+def _tree(modules) -> list[nn.Module]:
+    """``modules`` and what is below them.  A list that grows as it is walked: ``modules()`` and ``parameters()``, which look
+    for what comes twice, take three times as long, and a small step waits for the host."""
+    found = list(modules)
+    for m in found:
+        found += [child for child in m._modules.values() if child is not None]  # noqa: SLF001
+    return found
+
+
+def _has_own_hook(module: nn.Module) -> bool:
+    return bool(module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks  # noqa: SLF001
+                or "forward" in module.__dict__)
+
+
 def watched(module: nn.Module) -> bool:
     """Whether somebody gets to see what ``module`` itself takes and gives: a hook, its own or one of all modules, or a
     ``forward`` put in the place of its class's."""
-    return bool(torch.nn.modules.module._has_any_global_hook() or module._forward_hooks or module._forward_pre_hooks  # noqa: SLF001
-                or module._backward_hooks or module._backward_pre_hooks or "forward" in vars(module))  # noqa: SLF001
+    return bool(torch.nn.modules.module._has_any_global_hook()) or _has_own_hook(module)  # noqa: SLF001
 
 
 def unobserved(*modules: nn.Module) -> bool:
     """Whether nobody looks into ``modules``: none in their trees is watched, by what would get to see the listed rows, moved
     together and with unwritten rows behind them, in the place of the batch's, and none is of a class of its own, which would
     run over those."""
-    return not any(type(m) not in _ROW_MODULES or watched(m) for module in modules for m in module.modules())
+    if torch.nn.modules.module._has_any_global_hook():  # noqa: SLF001
+        return False
+    return all(type(m) in _ROW_MODULES and not _has_own_hook(m) for m in _tree(modules))
 
 
 @stops_at_count
@@ -383,7 +398,7 @@ def takes_listed_rows(layers, *linears: nn.Module) -> bool:
         linears += [attn.qkv_proj, attn.o_proj, mlp.gate_up_proj, mlp.down_proj]
     return (
         ops.own_gemm_enabled()
-        and all(p.is_cuda and p.dtype == torch.bfloat16 for layer in layers for p in layer.parameters())
+        and all(p is None or p.is_cuda and p.dtype == torch.bfloat16 for m in _tree(layers) for p in m._parameters.values())  # noqa: SLF001
         and all(getattr(m, "bias", None) is None and getattr(m, "row_parallel", None) is None and m.weight.is_cuda and m.weight.dtype == torch.bfloat16
                 and m.weight.is_contiguous() and m.weight.data_ptr() % 16 == 0 and m.weight.shape[0] % 8 == 0 and m.weight.shape[1] % 8 == 0
                 and m.weight.shape[1] <= 1 << 20 for m in linears)

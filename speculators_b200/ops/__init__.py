@@ -1011,21 +1011,14 @@ def take_rows(index: torch.Tensor, inverse: torch.Tensor, live: torch.Tensor, *x
     return tuple(only_live(x[index], live) for x in xs)
 
 
-class _RMSNormTakenFn(torch.autograd.Function):
-    """No gradient either way: a function, so that forward mode and ``torch.func`` refuse it as they do ``rms_norm``."""
-
-    @staticmethod
-    def forward(ctx, x, weight, eps, index, live):
-        y = torch.empty((index.shape[0], x.shape[1]), dtype=x.dtype, device=x.device)
-        native().norm_fwd(_grad_rows(x, x.shape[1]), weight, index, y, None, eps, False, live)
-        ctx.mark_non_differentiable(y)
-        return y
-
-
 def rms_norm_taken(x: torch.Tensor, weight: torch.Tensor, eps: float, index: torch.Tensor, live: torch.Tensor) -> torch.Tensor:
     """``rms_norm`` of the rows ``index`` of ``x``, where nothing is differentiated."""
     if _norm_native(x):
-        return _RMSNormTakenFn.apply(x, weight, eps, index, live)
+        if torch.autograd.forward_ad._current_level >= 0 or torch._C._are_functorch_transforms_active():  # noqa: SLF001
+            rms_norm(x, weight, eps)  # for its refusal: a tangent or a batch dimension would get lost in a bare kernel call
+        y = torch.empty((index.shape[0], x.shape[1]), dtype=x.dtype, device=x.device)
+        native().norm_fwd(_grad_rows(x, x.shape[1]), weight, index, y, None, eps, False, live)
+        return y
     return rms_norm(only_live(x[index], live), weight, eps)
 
 

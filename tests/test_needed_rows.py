@@ -620,7 +620,7 @@ def test_gpu_forward_mode_is_refused_as_before(monkeypatch):
 
     model, batch = _model(1, 64, False, 688, True), _gpu_batch(2100, "spans")
     kwargs, _ = Eagle3DraftModel.get_trainer_kwargs(loss_fn="kl_div", ttt_steps=3, ttt_step_loss_decay=0.8)
-    states = batch["verifier_last_hidden_states"]
+    states, losses = batch["verifier_last_hidden_states"], []
     for whole in (True, False):
         with monkeypatch.context() as patched, forward_ad.dual_level():
             if whole:
@@ -628,3 +628,6 @@ def test_gpu_forward_mode_is_refused_as_before(monkeypatch):
             dual = forward_ad.make_dual(states, torch.ones_like(states))
             with pytest.raises(Exception, match="jvp"):
                 model(**dict(batch, verifier_last_hidden_states=dual), **kwargs)
+            with torch.no_grad():
+                losses.append(float(model(**batch, **kwargs)[1]))  # without a tangent it runs
+    assert abs(losses[0] - losses[1]) <= 2e-4 * abs(losses[0])
