@@ -262,7 +262,13 @@ __device__ __forceinline__ bool flag_wait(const int* flag, int* status, int code
   return false;
 }
 
-__device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16(x)); }
+// both rounded to bf16
+__device__ __forceinline__ void bf16_round2(float& a, float& b) {
+  const __nv_bfloat162 t = __floats2bfloat162_rn(a, b);
+  const uint32_t w = *reinterpret_cast<const uint32_t*>(&t);
+  a = __uint_as_float(w << 16);
+  b = __uint_as_float(w & 0xffff0000u);
+}
 struct Scaling {
   float alpha, beta;
   // (the plain epilogue skips the arithmetic as a whole: the conditions are uniform)
@@ -270,17 +276,27 @@ struct Scaling {
   __device__ __forceinline__ void product(float (&f)[N]) const {
     if (alpha != 1.f) {
 #pragma unroll
-      for (int j = 0; j < N; ++j) f[j] = bf16_round(alpha * bf16_round(f[j]));
+      for (int j = 0; j < N; j += 2) {
+        float pad = 0.f, &second = j + 1 < N ? f[j + 1 < N ? j + 1 : j] : pad;
+        bf16_round2(f[j], second);
+        f[j] *= alpha;
+        second *= alpha;
+        bf16_round2(f[j], second);
+      }
     }
   }
   template <int N>
   __device__ __forceinline__ void add(float (&f)[N], const float (&o)[N]) const {
-    if (beta != 1.f) {
 #pragma unroll
-      for (int j = 0; j < N; ++j) f[j] += bf16_round(beta * o[j]);
-    } else {
-#pragma unroll
-      for (int j = 0; j < N; ++j) f[j] += o[j];
+    for (int j = 0; j < N; j += 2) {
+      float a = o[j], b = j + 1 < N ? o[j + 1 < N ? j + 1 : j] : 0.f;
+      if (beta != 1.f) {
+        a *= beta;
+        b *= beta;
+        bf16_round2(a, b);
+      }
+      f[j] += a;
+      if (j + 1 < N) f[j + 1 < N ? j + 1 : j] += b;
     }
   }
 };
@@ -519,16 +535,31 @@ __device__ __forceinline__ bool tile_reads_vectorised(const Params& p, int n0) {
   return true;
 }
 
-// Staged stores take every tile (N is a multiple of 8 then): a chunk past the edge reads as zeros.
+// Staged stores take every tile (N is a multiple of 8 then): a chunk past the edge reads as zeros.  The addend of a warp's 32
+// rows comes in whole 128-byte lines, four rows of 64 columns a load (v[h * 8 + j]: row j * 4 + lane / 8, columns h * 64 +
+// 8 * (lane % 8)), and meets its row in the staging area.  Loaded with a row per lane, 16 bytes each, every load touched 32
+// lines and the addend's loads set the pace of a tile (us a wave of pair tiles, 4096 x 9472, at contractions of 128 and 1024: residual 8.7 and 9.9,
+// now 5.4 and 8.3; accumulate 8.6 and 10.2, now 4.7 and 8.1; scaled by alpha and beta 10.8 and 11.0, now 6.5 and 8.8).
 template <int W>
-__device__ __forceinline__ void prefetch_addend_staged(const Params& p, int row, int n0, int z, int row_end, RowPrefetch<W>& pre) {
-  pre.tile_ok = true;
-  pre.valid = row < row_end;
-  if (p.epilogue == kStore) return;
-  const __nv_bfloat16* src = p.epilogue == kAccumulate ? p.c + z * p.c_batch + (int64_t)row * p.ldc + n0 : p.residual + z * p.r_batch + (int64_t)row * p.ldr + n0;
+__device__ __forceinline__ void prefetch_addend_staged(const Params& p, int row0, int n0, int z, int row_end, int lane, int h, RowPrefetch<W>& pre) {
+  const int row = row0 + (lane >> 3), col = n0 + h * 64 + (lane & 7) * 8;
+  const int64_t ld = p.epilogue == kAccumulate ? p.ldc : p.ldr;
+  const __nv_bfloat16* src = (p.epilogue == kAccumulate ? p.c + z * p.c_batch : p.residual + z * p.r_batch) + (int64_t)row * ld + col;
+  if (row0 + 32 <= row_end && n0 + h * 64 + 64 <= p.N) {
 #pragma unroll
-  for (int i = 0; i < W / 8; ++i)
-    pre.v[i] = pre.valid && n0 + i * 8 < p.N ? __ldg(reinterpret_cast<const uint4*>(src) + i) : make_uint4(0u, 0u, 0u, 0u);
+    for (int j = 0; j < 8; ++j) pre.v[h * 8 + j] = __ldg(reinterpret_cast<const uint4*>(src + j * 4 * ld));
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      pre.v[h * 8 + j] = row + j * 4 < row_end && col < p.N ? __ldg(reinterpret_cast<const uint4*>(src + j * 4 * ld)) : make_uint4(0u, 0u, 0u, 0u);
+  }
+}
+template <int W>
+__device__ __forceinline__ void prefetch_addend_staged(const Params& p, int row0, int n0, int z, int row_end, int lane, RowPrefetch<W>& pre) {
+  pre.tile_ok = pre.valid = true;
+  if (p.epilogue == kStore) return;
+#pragma unroll
+  for (int h = 0; h < W / 64; ++h) prefetch_addend_staged<W>(p, row0, n0, z, row_end, lane, h, pre);
 }
 
 template <int W>
@@ -598,35 +629,56 @@ __device__ __forceinline__ void store_vec4(const Params& p, const Scaling& sc, c
 }
 
 // One warp's 32 rows x W columns through its 4 KB staging area, 64 columns at a time.  `row0`: C row of lane 0;
-// `live`: the rows exist; the addend of a reading epilogue is in `pre` (pre.tile_ok) or read here.
-template <int W>
-__device__ __forceinline__ void store_accumulator_staged(const Params& p, const Scaling& sc, const CUtensorMap* map_c, const CUtensorMap* map_t, uint32_t stage,
-                                                         uint32_t taddr, int row0, int n0, int z, const RowPrefetch<W>& pre, bool live, bool mirror,
-                                                         bool zero, int lane) {
+// `live`: the rows exist.  ADD: the epilogue reads, its addend is in `pre` (prefetch_addend_staged) and `ahead(h)` is called
+// where the registers of the 64 columns h are free for the next tile's.  Instances of their own for what an epilogue does not
+// do: with the tests in between a plain tile took 4.0 us where it takes 2.2 (contraction of 128; from 768 on the products are longer).
+template <int W, bool ADD, bool SCALED, typename Ahead>
+__device__ __forceinline__ void store_accumulator_staged_as(const Scaling& sc, const CUtensorMap* map_c, const CUtensorMap* map_t, uint32_t stage, uint32_t taddr,
+                                                            int row0, int n0, int N, int z, RowPrefetch<W>& pre, bool live, bool mirror, bool zero, int lane,
+                                                            const Ahead& ahead) {
 #pragma unroll
   for (int h = 0; h < W / 64; ++h) {
     stage_wait();
+    if (ADD) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) stage_put8(stage, j * 4 + (lane >> 3), lane & 7, *reinterpret_cast<const bf16x8*>(&pre.v[h * 8 + j]));
+      __syncwarp();
+      ahead(h);
+    }
 #pragma unroll
     for (int q = 0; q < 2; ++q) {
-      const int c = h * 2 + q;
       uint32_t r[32];
-      tmem_ld32(taddr + c * 32, r);
+      uint4 own[4];
+      tmem_ld32(taddr + (h * 2 + q) * 32, r);
+      if (ADD) {
+#pragma unroll
+        for (int v = 0; v < 4; ++v) own[v] = stage_get8(stage, lane, q * 4 + v);
+      }
       tmem_ld_wait();
+      if (zero) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) r[j] = 0u;
+      }
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
         float f[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) f[j] = zero ? 0.f : __uint_as_float(r[v * 8 + j]);
-        sc.product(f);
-        if (p.epilogue != kStore) {
+        for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(r[v * 8 + j]);
+        if (SCALED) sc.product(f);
+        if (ADD) {
           float o[8];
-          unpack8(*reinterpret_cast<const bf16x8*>(&pre.v[c * 4 + v]), o);
-          sc.add(f, o);
+          unpack8(*reinterpret_cast<const bf16x8*>(&own[v]), o);
+          if (SCALED) {
+            sc.add(f, o);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) f[j] += o[j];
+          }
         }
         stage_put8(stage, lane, q * 4 + v, pack8(f));
       }
     }
-    const bool inside = live && n0 + h * 64 < p.N;
+    const bool inside = live && n0 + h * 64 < N;
     stage_store(stage, map_c, n0 + h * 64, row0, z, inside);
     if (mirror) {  // 64 rows (this half's columns) of 32 elements (the warp's rows); the lanes of a store are neighbours
       stage_wait();
@@ -644,6 +696,19 @@ __device__ __forceinline__ void store_accumulator_staged(const Params& p, const 
       stage_store(stage, map_t, row0, n0 + h * 64, z, inside);
     }
   }
+}
+struct NothingAhead {
+  __device__ __forceinline__ void operator()(int) const {}
+};
+template <int W, typename Ahead = NothingAhead>
+__device__ __forceinline__ void store_accumulator_staged(const Params& p, const Scaling& sc, const CUtensorMap* map_c, const CUtensorMap* map_t, uint32_t stage,
+                                                         uint32_t taddr, int row0, int n0, int z, RowPrefetch<W>& pre, bool live, bool mirror, bool zero,
+                                                         int lane, const Ahead& ahead = Ahead()) {
+  const bool scaled = sc.alpha != 1.f || sc.beta != 1.f;
+  if (p.epilogue == kStore && !scaled) store_accumulator_staged_as<W, false, false>(sc, map_c, map_t, stage, taddr, row0, n0, p.N, z, pre, live, mirror, zero, lane, ahead);
+  else if (p.epilogue == kStore) store_accumulator_staged_as<W, false, true>(sc, map_c, map_t, stage, taddr, row0, n0, p.N, z, pre, live, mirror, zero, lane, ahead);
+  else if (!scaled) store_accumulator_staged_as<W, true, false>(sc, map_c, map_t, stage, taddr, row0, n0, p.N, z, pre, live, mirror, zero, lane, ahead);
+  else store_accumulator_staged_as<W, true, true>(sc, map_c, map_t, stage, taddr, row0, n0, p.N, z, pre, live, mirror, zero, lane, ahead);
 }
 
 // ---- logits tile + row statistics ------------------------------------------------------------
@@ -804,7 +869,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     }
   } else if (log_splits == 0) {
     RowPrefetch<S_TILE_N> pre;
-    if (p.staged) prefetch_addend_staged<S_TILE_N>(p, row, n0, z, M, pre);
+    if (p.staged) prefetch_addend_staged<S_TILE_N>(p, m0 + quarter * 32, n0, z, M, lane, pre);
     else prefetch_addend<S_TILE_N>(p, row, n0, z, M, pre);
     ok = mbar_wait(smem_addr(&bar_acc_full), 0, p.status, kTimeoutEpilogue);
     ok = __all_sync(0xffffffffu, ok);
@@ -1082,6 +1147,7 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     const int chalf = (warp - 2) >> 2;    // columns 128 * chalf .. + 127 of the tile
     const uint32_t acc_empty_leader[2] = {map_to_cta(smem_addr(&bar_acc_empty[0]), 0), map_to_cta(smem_addr(&bar_acc_empty[1]), 0)};
     const uint32_t stage = smem_addr(smem + P_RING_BYTES) + (warp - 2) * 4096;
+    RowPrefetch<P_EPI_COLS> pre;
     bool ok = true;
     int local = 0;
     for (Pieces<DIVIDE> it(number); ok && it.advance(plan, num_kb, number, num_pairs); ++local) {
@@ -1091,12 +1157,11 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       const TileInfo ti = decode_tile<B_MN>(p, M, tile, tiles_m, tiles_n, num_kb, (int)rank);
       const int row = ti.c_row0 + quarter * 32 + lane, n0 = ti.n0 + chalf * P_EPI_COLS;
       const bool zero = ti.num_kb + more_steps(p, more, part_kb, tile, tiles_m * tiles_n) == 0;
-      RowPrefetch<P_EPI_COLS> pre;
       const bool with_stats = p.rs.targets != nullptr, gated = p.epilogue == kSwiGLU;
       if (with_stats) prefetch_targets<P_EPI_COLS>(p, row, n0, pre);
       else if (hands_over) pre.tile_ok = pre.valid = false;
-      else if (p.staged && !gated) prefetch_addend_staged<P_EPI_COLS>(p, row, n0, ti.z, ti.row_end, pre);
-      else if (!gated) prefetch_addend<P_EPI_COLS>(p, row, n0, ti.z, ti.row_end, pre);
+      else if (p.staged && !gated && (DIVIDE || local == 0)) prefetch_addend_staged<P_EPI_COLS>(p, ti.c_row0 + quarter * 32, n0, ti.z, ti.row_end, lane, pre);
+      else if (!gated && !p.staged) prefetch_addend<P_EPI_COLS>(p, row, n0, ti.z, ti.row_end, pre);
       ok = mbar_wait(smem_addr(&bar_acc_full[acc]), (local >> 1) & 1, p.status, kTimeoutEpilogue);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
@@ -1128,7 +1193,16 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         store_accumulator_swiglu(p, &map_c, &map_h, stage, lane_base + chalf * 64, row0, ti.n0 + chalf * 64,
                                  row0 < ti.row_end, lane);
       else if (with_stats) store_accumulator_with_stats<P_EPI_COLS>(p, taddr, row, n0, ti.tile_n * 2 + chalf, tiles_n * 2, pre);
-      else if (p.staged) store_accumulator_staged<P_EPI_COLS>(p, sc, &map_c, &map_h, stage, taddr, row0, n0, ti.z, pre, row0 < ti.row_end, ti.mirror, zero, lane);
+      else if (p.staged) {
+        const int following = tile + num_pairs;
+        TileInfo tn{};
+        auto ahead = [&](int h) {
+          if (DIVIDE || following >= plan.whole) return;
+          if (h == 0) tn = decode_tile<B_MN>(p, M, following, tiles_m, tiles_n, num_kb, (int)rank);
+          prefetch_addend_staged<P_EPI_COLS>(p, tn.c_row0 + quarter * 32, tn.n0 + chalf * P_EPI_COLS, tn.z, tn.row_end, lane, h, pre);
+        };
+        store_accumulator_staged<P_EPI_COLS>(p, sc, &map_c, &map_h, stage, taddr, row0, n0, ti.z, pre, row0 < ti.row_end, ti.mirror, zero, lane, ahead);
+      }
       else if (pre.tile_ok) store_accumulator_prefetched<P_EPI_COLS>(p, sc, taddr, row, n0, ti.z, pre, zero);
       else store_accumulator<P_EPI_COLS>(p, sc, taddr, row, n0, ti.z, ti.row_end, zero);
       fence_before_sync();
@@ -1532,12 +1606,7 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
   // Stores through staging: C must be a matrix that TMA can address, and a warp's 32 rows must not straddle an expert.
   CUtensorMap map_c = map_a, map_h = map_a;
   const bool reads_ok = epilogue != kAddResidual || ((ldr & 7) == 0 && (reinterpret_cast<uintptr_t>(residual) & 15) == 0);
-  // An epilogue that reads C or a residual on pair tiles stores whole sectors straight from registers: with the addend's loads
-  // it is the epilogue that sets the pace at short contractions, and waiting for the staging area to be read lengthens it
-  // (weight gradients added up: 24576 x 4096 x 736 195 us staged, 175 direct; 4096 x 14336 x 2048 214 and 194).
-  const bool direct = (epilogue == kAccumulate || epilogue == kAddResidual) && variant == kPair && !symmetric && (N & 127) == 0 && (ldc & 15) == 0 &&
-                      (reinterpret_cast<uintptr_t>(c) & 31) == 0;
-  if (!direct && scatter == nullptr && stats_targets == nullptr && (N & 7) == 0 && (ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(c) & 15) == 0 && reads_ok &&
+  if (scatter == nullptr && stats_targets == nullptr && (N & 7) == 0 && (ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(c) & 15) == 0 && reads_ok &&
       (grp == nullptr || grp->mode == kGroupRows || (M & 127) == 0)) {
     const int64_t rows = grp != nullptr && grp->mode == kGroupK ? (int64_t)grp->num_groups * M : M;
     rc = make_map_bf16_stack(&map_c, c, rows, N, ldc, 32, bs.batch, bs.c_stride);

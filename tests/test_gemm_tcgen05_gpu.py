@@ -281,3 +281,29 @@ def test_grouped_weight_gradient_over_several_uses(counts):
     ops.native().gemm_grouped_wgrad_parts(dys, xs, dw, False, segs, plan.mtile_start, ops.gemm_status(dw.device))
     ops.check_gemm_status()
     assert (dw.float() - want).abs().max() <= 0.01 * want.abs().max()
+
+
+# Several tiles per pair (the addend of one is fetched while the one before is stored), ragged rows and columns, one contraction step and
+# several.  Small integers: every sum is exact in fp32, so only the one rounding at the end is left and the results are equal.
+@pytest.mark.parametrize("M,N,K", [(2560, 2568, 64), (2433, 2312, 64), (4864, 1288, 200), (1024, 512, 64)])
+@pytest.mark.parametrize("epilogue", [0, 1, 2])
+def test_an_addend_meets_its_rows_and_columns(M, N, K, epilogue):
+    gen = torch.Generator(device="cuda").manual_seed(M + N)
+    draw = lambda *s: torch.randint(-2, 3, s, generator=gen, device="cuda").bfloat16()
+    a, b, add = draw(M, K), draw(N, K), torch.randint(-128, 129, (M, N), generator=gen, device="cuda").bfloat16()
+    out = add.clone() if epilogue == 1 else torch.full((M, N), float("nan"), device="cuda", dtype=torch.bfloat16)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    ops.native().gemm_tn_variant(a, b, out, add if epilogue == 2 else None, epilogue, status, 3, None)
+    want = a.float() @ b.float().t() + (add.float() if epilogue else 0.0)
+    assert int(status.item()) == 0 and torch.equal(out, want.bfloat16())
+
+
+def test_a_scaled_addend_is_rounded_like_separate_passes():
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    draw = lambda *s: torch.randint(-2, 3, s, generator=gen, device="cuda").bfloat16()
+    a, b, add = draw(5, 1032, 72), draw(5, 72, 1288), torch.randn(5, 1032, 1288, generator=gen, device="cuda").bfloat16()
+    out, status = torch.empty_like(add), torch.zeros(1, dtype=torch.int32, device="cuda")
+    ops.native().gemm_stack(a, b, out, add, False, True, 2.0315, -4.775, False, status)
+    alpha, beta = (torch.tensor(c, device="cuda") for c in (2.0315, -4.775))
+    want = (alpha * (a.float() @ b.float()).bfloat16().float()).bfloat16().float() + (beta * add.float()).bfloat16().float()
+    assert int(status.item()) == 0 and torch.equal(out, want.bfloat16())
