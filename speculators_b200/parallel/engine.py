@@ -597,6 +597,7 @@ class TrainEngine:
             self._muon_adjusts = torch.tensor(adjust, dtype=torch.float32, device=dev)
             self._muon_inv_norm = torch.zeros(len(owned), dtype=torch.float32, device=dev)
             self._muon_places = [at for _o, _n, at in table]
+            self._muon_streams = [torch.cuda.Stream(dev) for _ in range(min(len(self._muon_groups), _MUON_STREAMS) - 1)]
             for (i, p, o), place in zip(owned, self._muon_places):
                 n = p.numel()
                 master = self._muon_master[place : place + n].view(p.shape)
@@ -612,22 +613,44 @@ class TrainEngine:
         return 0.2 * math.sqrt(max(rows, cols)) if self.cfg.muon_adjust_lr_fn == "match_rms_adamw" else math.sqrt(max(1.0, rows / cols))
 
     def _muon_update_stacks(self, g: torch.Tensor, lr_ratio: float) -> None:
-        """The CUDA form: two element-wise launches for all matrices around one Newton-Schulz iteration per shape."""
+        """The CUDA form: two element-wise launches for all matrices around one Newton-Schulz iteration per shape.
+
+        An iteration is a chain of 15 products, most of which leave SMs idle (50 tiles on 74 pairs, a Gram matrix of one tile), so
+        the chains of different shapes run on streams of their own, joined before the update: with one stream, two, three and one
+        a shape, DSpark 0.6B takes 9.77, 9.22, 9.10 and 9.04 ms a step, EAGLE-3 with Muon 0.83, 0.67, 0.61 and 0.54 ms at the plumbing size
+        (128 rows), 5.9 and 5.5 at head dim 64 (1001 rows); where the products fill
+        the chip nothing changes (8B widths, the optimizer step alone: 19.1 and 18.9).  The Gram
+        matrices and polynomials of all shapes are allocated at the same time then."""
         cfg, nat = self.cfg, ops.native()
         upd = torch.empty(self._muon_momentum.shape, dtype=torch.bfloat16, device=self.device)
         other = torch.empty_like(upd)  # the iteration alternates between the two; the result is where it ends
         result = other if cfg.muon_ns_steps % 2 else upd
         nat.muon_momentum(g, self._muon_momentum, upd, self._muon_table, self._muon_chunks, self._muon_first_chunk, self.hyper, self.norm_sq,
                           cfg.muon_momentum, True, self._muon_inv_norm)
-        for start, count, rows, cols, k in self._muon_groups:
-            if rows % 8 == 0 and cols % 8 == 0 and ops.own_gemm_enabled() and cfg.muon_ns_steps > 0:
-                x, y = (t[start : start + count * rows * cols].view(count, rows, cols) for t in (upd, other))
-                _newton_schulz_stack(x, y, cfg.muon_ns_steps)
-                continue
-            for j in range(k, k + count):
-                place = self._muon_places[j]
-                one = upd[place : place + rows * cols].view(rows, cols)
-                result[place : place + rows * cols].view(rows, cols).copy_(_newton_schulz(one, cfg.muon_ns_steps, normalise=False))
+        main = torch.cuda.current_stream(self.device)
+        load = dict.fromkeys([main, *self._muon_streams], 0.0)  # each shape's chain on the stream with the least work so far
+        try:
+            for stream in self._muon_streams:
+                stream.wait_stream(main)
+            for start, count, rows, cols, k in sorted(self._muon_groups, key=_ns_work, reverse=True):
+                stream = min(load, key=load.get)
+                load[stream] += _ns_work((start, count, rows, cols, k))
+                with torch.cuda.stream(stream):
+                    if rows % 8 == 0 and cols % 8 == 0 and ops.own_gemm_enabled() and cfg.muon_ns_steps > 0:
+                        x, y = (t[start : start + count * rows * cols].view(count, rows, cols) for t in (upd, other))
+                        _newton_schulz_stack(x, y, cfg.muon_ns_steps)
+                        continue
+                    for j in range(k, k + count):
+                        place = self._muon_places[j]
+                        one = upd[place : place + rows * cols].view(rows, cols)
+                        result[place : place + rows * cols].view(rows, cols).copy_(_newton_schulz(one, cfg.muon_ns_steps, normalise=False))
+        except BaseException:
+            with contextlib.suppress(RuntimeError):  # a capture that the exception ended, too
+                for stream in self._muon_streams:
+                    main.wait_stream(stream)
+            raise
+        for stream in self._muon_streams:
+            main.wait_stream(stream)
         nat.muon_apply(self._muon_master, result, self.flat_w, self._muon_table, self._muon_chunks, self._muon_adjusts, self.hyper, lr_ratio, cfg.muon_weight_decay)
 
     def _muon_update(self, g: torch.Tensor) -> None:
@@ -880,6 +903,16 @@ def _can_access_peer(a: int, b: int) -> bool:
         return bool(torch.cuda.can_device_access_peer(a, b))
     except Exception:  # noqa: BLE001 - an unknown device index counts as "no"
         return False
+
+
+_MUON_STREAMS = 8  # at most, the caller's among them
+
+
+def _ns_work(group: tuple[int, int, int, int, int]) -> float:
+    """Work of a stack's iteration, for dividing stacks among streams; a launch's fixed part counts for narrow ones."""
+    _start, count, rows, cols, _k = group
+    m, n = min(rows, cols), max(rows, cols)
+    return count * (3.0 * m * m * n + 1.0 * m**3) + 1e10
 
 
 def _newton_schulz(g: torch.Tensor, steps: int, normalise: bool = True) -> torch.Tensor:

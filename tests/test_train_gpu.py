@@ -237,6 +237,38 @@ def test_muon_on_gpu_tracks_the_fp32_engine():
         assert (w - g_).abs().max() < tol * moved + 1e-4, (name, float((w - g_).abs().max()), float(moved))
 
 
+@pytest.mark.parametrize("graph", [False, True])
+def test_muon_chains_on_streams_of_their_own_give_the_same_update(graph):
+    """Shapes from one tile to many, more of them than streams, one that is not a multiple of 8 (library products)."""
+    from torch import nn
+
+    from speculators_b200.parallel import engine as engine_module
+
+    shapes = [(64, 64), (72, 264), (264, 72), (128, 4096), (4096, 128), (512, 512), (1032, 1032), (2048, 520), (520, 2048), (36, 60)]
+
+    def weights(streams):
+        torch.manual_seed(0)
+        net = nn.Module()
+        for i, shape in enumerate(shapes * 2):
+            net.register_parameter(f"w{i}", nn.Parameter(torch.randn(shape) * 0.02))
+        eng = engine_module.TrainEngine(net, engine_module.EngineConfig(lr=1e-3, optimizer="muon", compute_dtype=torch.bfloat16), device="cuda:0")
+        assert len(eng._muon_streams) == engine_module._MUON_STREAMS - 1
+        if not streams:
+            eng._muon_streams = []
+        eng.flat_g.copy_(torch.randn(eng.flat_g.shape, generator=torch.Generator().manual_seed(1)))
+        eng.step()
+        if graph:
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g):
+                eng.step()
+            for _ in range(3):
+                g.replay()
+        torch.cuda.synchronize()
+        return eng.flat_w.clone()
+
+    assert torch.equal(weights(True), weights(False))
+
+
 @pytest.mark.parametrize("name", ["kl_div", "ce"])
 def test_fused_head_and_default_head_give_the_same_passes(name, monkeypatch):
     """The switch ``SB200_FUSED_HEAD`` has a tail of its own behind its row losses: running loss, counters, ``prev_correct`` and
