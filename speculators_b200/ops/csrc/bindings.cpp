@@ -73,7 +73,8 @@ int launch_gemm_parts(int, const void* const*, const void* const*, const int*, c
                       SplitSpace*, cudaStream_t);
 int launch_gemm_grouped_parts(int, const void* const*, const void* const*, const int*, const int64_t*, const int64_t*, const int* const*, void*, int, int, int,
                               const int*, int, int*, cudaStream_t);
-int launch_gemm_stack(const void*, const void*, void*, const void*, int, int, int, int, int, int, float, float, int, int*, SplitSpace*, cudaStream_t);
+int launch_gemm_stack(const void*, const void*, void*, const void*, int, int, int, int, int, int, float, float, int, float, int, int*, SplitSpace*,
+                      cudaStream_t);
 void launch_moe_group_plan(const int*, int, int*, int*, cudaStream_t);
 int launch_gemm_grouped(const void*, const void*, void*, int, int, int, int64_t, int64_t, int64_t, int, int, int, const int*, const int*, int, int*,
                         cudaStream_t);
@@ -1293,10 +1294,11 @@ void gemm(const Tensor& a, const Tensor& b, Tensor out, int64_t epilogue, bool a
   gemm_variant(a, b, out, epilogue, a_mn, b_mn, status, 0, live);
 }
 
-// Stacks of products: out[z] = alpha op(a[z]) @ op(b[z])^T (+ beta addend[z]), rounded as separate bf16 passes would round.
+// Stacks of products: out[z] = alpha op(a[z]) @ op(b[z])^T (+ beta addend[z]), rounded as separate bf16 passes would round; with a
+// `diagonal` (+ diagonal I), in fp32 and rounded once.
 // Operands as in gemm, each a dense [batch, ., .] stack; symmetric: the caller knows that the products are.
 void gemm_stack(const Tensor& a, const Tensor& b, Tensor out, const c10::optional<Tensor>& addend, bool a_mn, bool b_mn, double alpha, double beta,
-                bool symmetric, Tensor status) {
+                bool symmetric, Tensor status, c10::optional<double> diagonal) {
   for (const Tensor* t : std::initializer_list<const Tensor*>{&a, &b, &out})
     TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kBFloat16 && t->dim() == 3 && t->is_contiguous(), "gemm_stack: contiguous bf16 [batch, rows, cols] expected");
   const int64_t B = a.size(0), M = a_mn ? a.size(2) : a.size(1), K = a_mn ? a.size(1) : a.size(2), N = b_mn ? b.size(2) : b.size(1);
@@ -1308,7 +1310,8 @@ void gemm_stack(const Tensor& a, const Tensor& b, Tensor out, const c10::optiona
   c10::cuda::CUDAGuard guard(a.device());
   TorchSplitSpace space(a);
   const int rc = sb200::launch_gemm_stack(a.data_ptr(), b.data_ptr(), out.data_ptr(), addend.has_value() ? addend->data_ptr() : nullptr, (int)B, (int)M, (int)N,
-                                          (int)K, a_mn ? 1 : 0, b_mn ? 1 : 0, (float)alpha, (float)beta, symmetric ? 1 : 0, status.data_ptr<int>(), &space, cur_stream());
+                                          (int)K, a_mn ? 1 : 0, b_mn ? 1 : 0, (float)alpha, (float)beta,
+                                          diagonal.has_value() ? 1 : 0, (float)diagonal.value_or(0.0), symmetric ? 1 : 0, status.data_ptr<int>(), &space, cur_stream());
   TORCH_CHECK(rc == 0, "gemm_stack launch failed (", rc, ")");
 }
 
@@ -1560,7 +1563,8 @@ TORCH_LIBRARY(sb200, m) {
   m.def("gemm_tn(Tensor a, Tensor b, Tensor out, Tensor? residual, int epilogue, Tensor status, Tensor? live=None) -> ()", &gemm_tn);
   m.def("gemm(Tensor a, Tensor b, Tensor out, int epilogue, bool a_mn, bool b_mn, Tensor status, Tensor? live=None) -> ()", &gemm);
   m.def("gemm_variant(Tensor a, Tensor b, Tensor out, int epilogue, bool a_mn, bool b_mn, Tensor status, int variant, Tensor? live=None) -> ()", &gemm_variant);
-  m.def("gemm_stack", &gemm_stack);
+  m.def("gemm_stack(Tensor a, Tensor b, Tensor out, Tensor? addend, bool a_mn, bool b_mn, float alpha, float beta, bool symmetric, Tensor status, "
+        "float? diagonal=None) -> ()", &gemm_stack);
   m.def("lmhead_loss_fwd", &lmhead_loss_fwd);
   m.def("moe_group_plan", &moe_group_plan);
   m.def("gemm_grouped_rows", &gemm_grouped_rows);

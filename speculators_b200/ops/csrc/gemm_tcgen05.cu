@@ -120,8 +120,10 @@ struct Params {
   int64_t ldh;
   int staged;        // 1: C (and h) leave through shared memory and TMA stores (map_c, map_h)
   // result = alpha * product (+ beta * addend), rounded where separate element-wise passes over bf16 tensors would round:
-  // alpha * bf16(product) and beta * addend each to bf16 before the sum; alpha = beta = 1 is the plain epilogue
-  float alpha, beta;
+  // alpha * bf16(product) and beta * addend each to bf16 before the sum; alpha = beta = 1 is the plain epilogue.
+  // once: alpha * product + beta * addend + diagonal on its diagonal, in fp32 and rounded once
+  float alpha, beta, diagonal;
+  int once;
   // a stack of `batch` products: the z-th of each operand's stack, elements apart
   int batch;
   int64_t c_batch, r_batch;
@@ -270,11 +272,20 @@ __device__ __forceinline__ void bf16_round2(float& a, float& b) {
   b = __uint_as_float(w & 0xffff0000u);
 }
 struct Scaling {
-  float alpha, beta;
+  float alpha, beta, diagonal;
+  int once;
+  __device__ __forceinline__ explicit Scaling(const Params& p) : alpha(p.alpha), beta(p.beta), diagonal(p.diagonal), once(p.once) {}
   // (the plain epilogue skips the arithmetic as a whole: the conditions are uniform)
   template <int N>
-  __device__ __forceinline__ void product(float (&f)[N]) const {
-    if (alpha != 1.f) {
+  __device__ __forceinline__ void product(float (&f)[N], int row, int col) const {  // N columns from col on
+    if (once) {
+#pragma unroll
+      for (int j = 0; j < N; ++j) f[j] *= alpha;
+      if ((unsigned)(row - col) < (unsigned)N) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) f[j] += row == col + j ? diagonal : 0.f;
+      }
+    } else if (alpha != 1.f) {
 #pragma unroll
       for (int j = 0; j < N; j += 2) {
         float pad = 0.f, &second = j + 1 < N ? f[j + 1 < N ? j + 1 : j] : pad;
@@ -287,6 +298,11 @@ struct Scaling {
   }
   template <int N>
   __device__ __forceinline__ void add(float (&f)[N], const float (&o)[N]) const {
+    if (once) {
+#pragma unroll
+      for (int j = 0; j < N; ++j) f[j] = fmaf(beta, o[j], f[j]);
+      return;
+    }
 #pragma unroll
     for (int j = 0; j < N; j += 2) {
       float a = o[j], b = j + 1 < N ? o[j + 1 < N ? j + 1 : j] : 0.f;
@@ -423,7 +439,7 @@ __device__ __forceinline__ void store_accumulator(const Params& p, const Scaling
           float f[8];
 #pragma unroll
           for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(r[v * 8 + j]);
-          sc.product(f);
+          sc.product(f, row, col0 + v * 8);
           if (p.epilogue == kAccumulate) {
             float o[8];
             unpack8(ld8(crow + c * 32 + v * 8), o);
@@ -446,7 +462,7 @@ __device__ __forceinline__ void store_accumulator(const Params& p, const Scaling
         for (int j = 0; j < 32; ++j) {
           if (col0 + j < p.N) {
             float f[1] = {__uint_as_float(r[j])};
-            sc.product(f);
+            sc.product(f, row, col0 + j);
             if (p.epilogue != kStore) {
               const float o[1] = {__bfloat162float((p.epilogue == kAccumulate ? crow : rrow)[c * 32 + j])};
               sc.add(f, o);
@@ -593,7 +609,7 @@ __device__ __forceinline__ void store_accumulator_prefetched(const Params& p, co
       unpack8(*reinterpret_cast<const bf16x8*>(&pre.v[c * 4 + v]), o);
 #pragma unroll
       for (int j = 0; j < 8; ++j) f[j] = zero ? 0.f : __uint_as_float(r[v * 8 + j]);
-      sc.product(f);
+      sc.product(f, row, n0 + c * 32 + v * 8);
       sc.add(f, o);
       packed[v] = pack8(f);
     }
@@ -613,7 +629,7 @@ __device__ __forceinline__ void store_vec4(const Params& p, const Scaling& sc, c
   __nv_bfloat16* out = p.c + z * p.c_batch + (int64_t)row * p.ldc + col0;
   const __nv_bfloat16* add = p.epilogue == kAccumulate ? out : p.residual + z * p.r_batch + (int64_t)row * p.ldr + col0;
   float f[4] = {t.x, t.y, t.z, t.w}, o[4];
-  sc.product(f);
+  sc.product(f, row, col0);
   const bool full = col0 + 4 <= p.N && (p.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(p.c) & 7) == 0;
   if (p.epilogue != kStore) {
     for (int j = 0; j < 4; ++j) o[j] = col0 + j < p.N ? __bfloat162float(add[j]) : 0.f;
@@ -664,7 +680,7 @@ __device__ __forceinline__ void store_accumulator_staged_as(const Scaling& sc, c
         float f[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(r[v * 8 + j]);
-        if (SCALED) sc.product(f);
+        if (SCALED) sc.product(f, row0 + lane, n0 + h * 64 + q * 32 + v * 8);
         if (ADD) {
           float o[8];
           unpack8(*reinterpret_cast<const bf16x8*>(&own[v]), o);
@@ -704,7 +720,7 @@ template <int W, typename Ahead = NothingAhead>
 __device__ __forceinline__ void store_accumulator_staged(const Params& p, const Scaling& sc, const CUtensorMap* map_c, const CUtensorMap* map_t, uint32_t stage,
                                                          uint32_t taddr, int row0, int n0, int z, RowPrefetch<W>& pre, bool live, bool mirror, bool zero,
                                                          int lane, const Ahead& ahead = Ahead()) {
-  const bool scaled = sc.alpha != 1.f || sc.beta != 1.f;
+  const bool scaled = sc.alpha != 1.f || sc.beta != 1.f || sc.once;
   if (p.epilogue == kStore && !scaled) store_accumulator_staged_as<W, false, false>(sc, map_c, map_t, stage, taddr, row0, n0, p.N, z, pre, live, mirror, zero, lane, ahead);
   else if (p.epilogue == kStore) store_accumulator_staged_as<W, false, true>(sc, map_c, map_t, stage, taddr, row0, n0, p.N, z, pre, live, mirror, zero, lane, ahead);
   else if (!scaled) store_accumulator_staged_as<W, true, false>(sc, map_c, map_t, stage, taddr, row0, n0, p.N, z, pre, live, mirror, zero, lane, ahead);
@@ -821,7 +837,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   if (log_splits > 0) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // waited for before the first remote store
 
   bool ok = true;
-  const Scaling sc{p.alpha, p.beta};
+  const Scaling sc(p);
   const int quarter = warp & 3, row = m0 + quarter * 32 + lane;
   if (warp == 0) {
     if (elect_one()) {
@@ -1188,7 +1204,7 @@ gemm_tn_2cta_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         if (!ok) break;
       }
       const int row0 = ti.c_row0 + quarter * 32;
-      const Scaling sc{p.alpha, p.beta};
+      const Scaling sc(p);
       if (gated)  // this warp: gate columns 64 * chalf .. + 63 of the tile and the same up columns
         store_accumulator_swiglu(p, &map_c, &map_h, stage, lane_base + chalf * 64, row0, ti.n0 + chalf * 64,
                                  row0 < ti.row_end, lane);
@@ -1272,7 +1288,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   const int kb0 = split * per_kb, num_kb = max(0, min(per_kb, all_kb - kb0));
 
   bool ok = true;
-  const Scaling sc{p.alpha, p.beta};
+  const Scaling sc(p);
   const int quarter = warp & 3, chalf = (warp - 2) >> 2;
   if (warp == 0) {
     if (elect_one()) {
@@ -1513,7 +1529,8 @@ struct PartsSpec {
 struct BatchSpec {
   int batch = 1;
   int64_t a_stride = 0, b_stride = 0, c_stride = 0, r_stride = 0;
-  float alpha = 1.f, beta = 1.f;
+  float alpha = 1.f, beta = 1.f, diagonal = 0.f;
+  bool once = false;
   bool symmetric = false;
 };
 
@@ -1573,7 +1590,7 @@ static int launch_gemm_impl(const void* a, const void* b, void* c, const void* r
             : make_map_bf16_stack(&map_b, b, b_stack * N, K, ldb, pairs ? P_HALF : S_TILE_N, bs.batch, bs.b_stride);
   if (rc) return rc;
   Params p{(__nv_bfloat16*)c, (const __nv_bfloat16*)residual, M, N, K, ldc, ldr, epilogue, status, RowStatsOut{nullptr, 0, 0, 0, nullptr},
-           Grouping{kGroupNone, 0, nullptr, nullptr}, Scatter{}, (__nv_bfloat16*)gated_h, gated_ldh, 0, bs.alpha, bs.beta, bs.batch,
+           Grouping{kGroupNone, 0, nullptr, nullptr}, Scatter{}, (__nv_bfloat16*)gated_h, gated_ldh, 0, bs.alpha, bs.beta, bs.diagonal, bs.once ? 1 : 0, bs.batch,
            bs.c_stride, bs.r_stride, 0, live, nullptr, nullptr};
   if (live != nullptr && (grp != nullptr || scatter != nullptr || stats_targets != nullptr || bs.batch != 1 || (a_mn && !b_mn))) return -10;
   if (epilogue == kSwiGLU) {
@@ -1709,11 +1726,11 @@ int launch_gemm_parts(int n, const void* const* a, const void* const* b, const i
 }
 
 // ---- stacks of products (Newton-Schulz iterations of equally shaped matrices) ----------------------
-// c[z] = alpha * op(a[z]) * op(b[z])^T (+ beta * addend[z]), rounded as in Params.
+// c[z] = alpha * op(a[z]) * op(b[z])^T (+ beta * addend[z]), rounded as in Params; with `once` (+ diagonal * I) and rounded once.
 // All stacks dense: [batch, rows, cols].  `symmetric`: the caller knows that the product is (a Gram matrix, a power of a
 // symmetric matrix): only tiles on and above the diagonal are computed.
 int launch_gemm_stack(const void* a, const void* b, void* c, const void* addend, int batch, int M, int N, int K, int a_mn, int b_mn, float alpha,
-                      float beta, int symmetric, int* status, SplitSpace* space, cudaStream_t stream) {
+                      float beta, int once, float diagonal, int symmetric, int* status, SplitSpace* space, cudaStream_t stream) {
   BatchSpec bs;
   bs.batch = batch;
   bs.a_stride = (int64_t)M * K;
@@ -1721,6 +1738,8 @@ int launch_gemm_stack(const void* a, const void* b, void* c, const void* addend,
   bs.c_stride = bs.r_stride = (int64_t)M * N;
   bs.alpha = alpha;
   bs.beta = beta;
+  bs.diagonal = diagonal;
+  bs.once = once != 0;
   bs.symmetric = symmetric != 0;
   return launch_gemm_impl(a, b, c, addend, M, N, K, a_mn ? M : K, b_mn ? N : K, N, N, addend != nullptr ? tc::kAddResidual : tc::kStore, a_mn, b_mn, status, 0,
                           nullptr, 0, 0, 0, nullptr, nullptr, stream, nullptr, nullptr, 0, &bs, nullptr, nullptr, space);
