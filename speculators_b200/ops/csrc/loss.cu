@@ -19,6 +19,7 @@
 // accuracy metrics need no extra pass over the vocabulary.
 #include "common.cuh"
 #include "loss_stats.cuh"
+#include "packed_f32.cuh"
 
 namespace sb200 {
 
@@ -26,65 +27,146 @@ enum LossOp : int { kOpKL = 0, kOpRKL = 1, kOpJSD = 2, kOpCE = 3, kOpTV = 4 };
 constexpr int kLossThreads = 512;
 constexpr int kNumStats = 5;  // m_d, z_d, m_t, z_t, per-op extra
 
-// Combine per-thread stats across the block.  Result valid in every thread.
-__device__ __forceinline__ void block_combine(RowStats& s, float* scratch, int* iscratch) {
-  const float M = block_max(s.m, scratch);
-  const float z = (s.m == -INFINITY) ? 0.f : s.z * __expf(s.m - M);
-  const float Z = block_sum(z, scratch);
-  // argmax with lowest-index tie break
-  float bv = s.best;
-  int bi = s.best_idx;
+// One thread's share of a row: running maximum, sum of exponentials against it, and the column where the vector of eight starts
+// that brought the maximum (which of the eight is looked up once a row); columns behind the last whole vector on their own.
+// Sums are formed in the order of the columns, eight at a time, as online_update forms them.
+struct Share {
+  float m = -INFINITY, z = 0.f;
+  int col = 0x7fffffff;
+};
+__device__ __forceinline__ float max8(const bf16x8& v) {
+  const __nv_bfloat162 m = __hmax2(__hmax2(v.v[0], v.v[1]), __hmax2(v.v[2], v.v[3]));
+  return fmaxf(__low2float(m), __high2float(m));
+}
+__device__ __forceinline__ float2x widen(const __nv_bfloat162& v) {
+  const uint32_t w = *reinterpret_cast<const uint32_t*>(&v);
+  return both(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+}
+// e^v = 2^(v log2 e) of two differences
+__device__ __forceinline__ float2 exp_pair(float2x v) {
+  constexpr float kLog2E = 1.4426950408889634f;
+  const float2 s = apart(mul2(v, both(kLog2E, kLog2E)));
+  float2 e;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(s.x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(s.y));
+  return e;
+}
+// The new maximum and what it makes of the sums so far.
+__device__ __forceinline__ float raise(Share& s, float vmax, int col) {
+  const float m_new = fmaxf(s.m, vmax), by = __expf(s.m - m_new);
+  s.col = vmax > s.m ? col : s.col;
+  s.m = m_new;
+  return by;
+}
+__device__ __forceinline__ void add8(Share& s, const bf16x8& v, int col) {
+  const float by = raise(s, max8(v), col);
+  const float2x minus_m = both(-s.m, -s.m);
+  float add = 0.f;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-    if (ov > bv || (ov == bv && oi < bi)) {
-      bv = ov;
-      bi = oi;
-    }
+  for (int i = 0; i < 4; ++i) {
+    const float2 e = exp_pair(add2(widen(v.v[i]), minus_m));
+    add += e.x;
+    add += e.y;
   }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  __syncthreads();
-  if (lane == 0) {
-    scratch[warp] = bv;
-    iscratch[warp] = bi;
-  }
-  __syncthreads();
-  if (warp == 0) {
-    bv = lane < nwarp ? scratch[lane] : -INFINITY;
-    bi = lane < nwarp ? iscratch[lane] : 0x7fffffff;
+  s.z = fmaf(s.z, by, add);
+}
+// The target row's, with A = sum_v e^{t_v - m}(t_v - x_v) (see online_update_kl).
+__device__ __forceinline__ void add8_kl(Share& s, float& A, const bf16x8& tv, const bf16x8& xv, int col) {
+  const float by = raise(s, max8(tv), col);
+  const float2x minus_m = both(-s.m, -s.m), minus = both(-1.f, -1.f);
+  float add = 0.f, add_a = 0.f;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (ov > bv || (ov == bv && oi < bi)) {
-        bv = ov;
-        bi = oi;
-      }
-    }
-    if (lane == 0) {
-      scratch[32] = bv;
-      iscratch[32] = bi;
+  for (int i = 0; i < 4; ++i) {
+    const float2x t = widen(tv.v[i]);
+    const float2 e = exp_pair(add2(t, minus_m)), d = apart(fma2(widen(xv.v[i]), minus, t));
+    add += e.x;
+    add += e.y;
+    add_a = fmaf(e.x, d.x, add_a);
+    add_a = fmaf(e.y, d.y, add_a);
+  }
+  if (add_a != add_a) {  // an infinite logit is among them: zero-probability targets contribute nothing
+    float t[8], x[8];
+    unpack8(tv, t);
+    unpack8(xv, x);
+    add = add_a = 0.f;
+    for (int j = 0; j < 8; ++j) {
+      const float e = __expf(t[j] - s.m);
+      add += e;
+      if (e > 0.f) add_a = fmaf(e, t[j] - x[j], add_a);
     }
   }
-  __syncthreads();
-  s.m = M;
-  s.z = Z;
-  s.best = scratch[32];
-  s.best_idx = iscratch[32];
-  __syncthreads();
+  s.z = fmaf(s.z, by, add);
+  A = fmaf(A, by, add_a);
+}
+__device__ __forceinline__ void add1(Share& s, float x, int col) {
+  const float by = raise(s, x, col);
+  s.z = fmaf(s.z, by, __expf(x - s.m));
+}
+__device__ __forceinline__ void add1_kl(Share& s, float& A, float t, float x, int col) {
+  const float by = raise(s, t, col), e = __expf(t - s.m);
+  s.z = fmaf(s.z, by, e);
+  A = fmaf(A, by, e > 0.f ? e * (t - x) : 0.f);
 }
 
+// Meetings of the block.  Every warp finishes the reduction for itself, in the order block_sum takes, so that a meeting is one barrier.
+constexpr int kLossWarps = kLossThreads / 32;
+struct Meeting {
+  float m[2][kLossWarps], z[2][kLossWarps], acc[2][kLossWarps];
+  int col[2][kLossWarps];
+};
+__device__ __forceinline__ float over_warps_sum(const float* of) {
+  const int lane = threadIdx.x & 31;
+  return warp_sum(lane < kLossWarps ? of[lane] : 0.f);
+}
+// Row `i`'s share over the block; meet_max, a barrier, meet_sum, a barrier, met.
+__device__ __forceinline__ void meet_max(const Share& s, Meeting& at, int i) {
+  const float m = warp_max(s.m);
+  const int col = __reduce_min_sync(0xffffffffu, s.m == m ? s.col : 0x7fffffff);
+  if ((threadIdx.x & 31) == 0) {
+    at.m[i][threadIdx.x >> 5] = m;
+    at.col[i][threadIdx.x >> 5] = col;
+  }
+}
+__device__ __forceinline__ void meet_sum(Share& s, Meeting& at, int i) {
+  const int lane = threadIdx.x & 31;
+  const float wm = lane < kLossWarps ? at.m[i][lane] : -INFINITY, M = warp_max(wm);
+  s.col = __reduce_min_sync(0xffffffffu, lane < kLossWarps && wm == M ? at.col[i][lane] : 0x7fffffff);
+  const float z = warp_sum((s.m == -INFINITY) ? 0.f : s.z * __expf(s.m - M));
+  if (lane == 0) at.z[i][threadIdx.x >> 5] = z;
+  s.m = M;
+}
+__device__ __forceinline__ void met(Share& s, const Meeting& at, int i) { s.z = over_warps_sum(at.z[i]); }
+__device__ __forceinline__ float block_sum_in(float v, float* of) {
+  v = warp_sum(v);
+  if ((threadIdx.x & 31) == 0) of[threadIdx.x >> 5] = v;
+  __syncthreads();
+  return over_warps_sum(of);
+}
+// Column of the row's maximum, the first one.
+__device__ __forceinline__ int first_max(const Share& s, const __nv_bfloat16* row, int vec_end) {
+  if (s.col >= vec_end) return s.col;
+  for (int j = 0; j < 8; ++j)
+    if (__bfloat162float(row[s.col + j]) == s.m) return s.col + j;
+  return s.col;
+}
+
+// Bound by issue and the special-function units before memory: an exponential per column and row, and beside it what the maximum,
+// its column and the sums take.  So the maximum comes from packed comparisons, its column is kept per vector of eight and looked up
+// once a row, differences and scalings are packed pairs, and a row takes three barriers (23 before).  Sums keep their order.  The
+// KL divergence does best with three blocks an SM and one vector of each row in flight, the others with two and what registers
+// the compiler likes (us, two vectors and one: KL 4096 x 32000 143 and 130, total variation 168 and 195, labels 2460 x 151936 144 and
+// 175; bounded to 32 registers the labels took 268).  us before and after: KL 1001 x 32000 45.7 and 38.7, 4096 x 32000 159 and 129,
+// total variation 220 and 168, cross-entropy 8192 x 32000 253 and 205, labels 300 x 151936 38.5 and 29.8, 2460 x 151936 170 and 144
+// (reading takes 20, 80, 80, 160, 14 and 114).
 template <int OP>
-__global__ void __launch_bounds__(kLossThreads)
+__global__ void __launch_bounds__(kLossThreads, OP == kOpKL ? 3 : 0)
 loss_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* __restrict__ targets,
                 const uint8_t* __restrict__ active, const uint8_t* __restrict__ also, const int64_t* __restrict__ labels,
                 float* __restrict__ loss, float* __restrict__ stats, int* __restrict__ argmax_d,
                 int* __restrict__ argmax_t, int rows, int V, int64_t ld_logits, int64_t ld_targets,
                 int shift, const int* __restrict__ target_row) {
   pdl_begin();
-  __shared__ float scratch[33];
-  __shared__ int iscratch[33];
+  __shared__ Meeting at;
   const int r = blockIdx.x;
   if (r >= rows) return;
   float* st = stats + r;
@@ -106,42 +188,71 @@ loss_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* _
   const bool vec_ok = ((V & 7) == 0) && ((ld_logits & 7) == 0) && ((ld_targets & 7) == 0);
   const int nvec = vec_ok ? (V >> 3) : 0;
 
-  RowStats sd{-INFINITY, 0.f, -INFINITY, 0x7fffffff}, stt{-INFINITY, 0.f, -INFINITY, 0x7fffffff};
+  Share sd, stt;
   float kl_a = 0.f;  // OP == kOpKL: the cross term, accumulated in the same pass
-  for (int v = threadIdx.x; v < nvec; v += kLossThreads) {
-    float a[8], b[8];
-    unpack8(ld8(x + (v << 3)), a);
-    online_update(sd, a, v << 3);
+  auto take = [&](const bf16x8& a, const bf16x8& b, int v) {
+    add8(sd, a, v << 3);
     if (has_t) {
-      unpack8(ld8(t + (v << 3)), b);
-      if (OP == kOpKL) online_update_kl(stt, kl_a, b, a, v << 3);
-      else online_update(stt, b, v << 3);
+      if (OP == kOpKL) add8_kl(stt, kl_a, b, a, v << 3);
+      else add8(stt, b, v << 3);
+    }
+  };
+  int v = threadIdx.x;
+  if constexpr (OP == kOpKL) {
+    for (; v < nvec; v += kLossThreads) {
+      const bf16x8 a0 = ld8(x + (v << 3));
+      take(a0, has_t ? ld8(t + (v << 3)) : a0, v);
+    }
+  } else {
+    for (; v + kLossThreads < nvec; v += 2 * kLossThreads) {
+      const bf16x8 a0 = ld8(x + (v << 3)), a1 = ld8(x + ((v + kLossThreads) << 3));
+      bf16x8 b0 = a0, b1 = a1;
+      if (has_t) {
+        b0 = ld8(t + (v << 3));
+        b1 = ld8(t + ((v + kLossThreads) << 3));
+      }
+      take(a0, b0, v);
+      take(a1, b1, v + kLossThreads);
+    }
+    if (v < nvec) {
+      const bf16x8 a0 = ld8(x + (v << 3));
+      take(a0, has_t ? ld8(t + (v << 3)) : a0, v);
     }
   }
   for (int c = (nvec << 3) + threadIdx.x; c < V; c += kLossThreads) {
     const float xc = __bfloat162float(x[c]);
-    online_update_scalar(sd, xc, c);
+    add1(sd, xc, c);
     if (has_t) {
-      if (OP == kOpKL) online_update_kl_scalar(stt, kl_a, __bfloat162float(t[c]), xc, c);
-      else online_update_scalar(stt, __bfloat162float(t[c]), c);
+      if (OP == kOpKL) add1_kl(stt, kl_a, __bfloat162float(t[c]), xc, c);
+      else add1(stt, __bfloat162float(t[c]), c);
     }
   }
   const float my_mt = stt.m;  // this thread's running max of the target row, before the block-wide combine
-  block_combine(sd, scratch, iscratch);
+  meet_max(sd, at, 0);
+  if (has_t) meet_max(stt, at, 1);
+  __syncthreads();
+  meet_sum(sd, at, 0);
+  if (has_t) meet_sum(stt, at, 1);
+  __syncthreads();
+  met(sd, at, 0);
   if (has_t) {
-    block_combine(stt, scratch, iscratch);
+    met(stt, at, 1);
   } else {
     stt.m = 0.f;
     stt.z = 1.f;
     int lab = labels ? (int)labels[tr] : 0;
-    stt.best_idx = lab < 0 ? 0 : (lab >= V ? V - 1 : lab);
+    stt.col = lab < 0 ? 0 : (lab >= V ? V - 1 : lab);
   }
+  auto best_of_target = [&]() { return has_t ? first_max(stt, t, nvec << 3) : stt.col; };
   const float lse_d = sd.m + __logf(sd.z);
   const float lse_t = stt.m + __logf(stt.z);
 
   float acc0 = 0.f, acc1 = 0.f;
   if (OP == kOpCE) {
-    if (threadIdx.x == 0) acc0 = lse_d - __bfloat162float(x[stt.best_idx]);
+    if (threadIdx.x == 0) {
+      const int c = best_of_target();  // none in a row of nothing but -inf or NaN
+      acc0 = c < V ? lse_d - __bfloat162float(x[c]) : __int_as_float(0x7fffffff);
+    }
   } else if (OP == kOpKL) {
     // sum_v p_v (t_v - x_v) = (sum over threads of A rescaled to the row max) / Z_t; thread 0 adds
     // the normaliser terms once so that the block sum below yields the row's KL directly
@@ -175,10 +286,11 @@ loss_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* _
     for (int c = (nvec << 3) + threadIdx.x; c < V; c += kLossThreads)
       body(__bfloat162float(x[c]), __bfloat162float(t[c]));
   }
-  acc0 = block_sum(acc0, scratch);
-  if (OP == kOpJSD || OP == kOpTV) acc1 = block_sum(acc1, scratch);
+  if (OP != kOpCE) acc0 = block_sum_in(acc0, at.acc[0]);
+  if (OP == kOpJSD || OP == kOpTV) acc1 = block_sum_in(acc1, at.acc[1]);
   if (threadIdx.x == 0) {
     float L, extra;
+    const int best_t = OP == kOpCE || argmax_t ? best_of_target() : 0;
     if (OP == kOpKL || OP == kOpRKL) {
       L = acc0;
       extra = acc0;
@@ -187,7 +299,7 @@ loss_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* _
       extra = acc1;
     } else if (OP == kOpCE) {
       L = acc0;
-      extra = (float)stt.best_idx;
+      extra = (float)best_t;
     } else {
       L = 1.f - acc0;
       extra = acc1;
@@ -198,8 +310,8 @@ loss_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* _
     st[(int64_t)2 * rows] = stt.m;
     st[(int64_t)3 * rows] = stt.z;
     st[(int64_t)4 * rows] = extra;
-    if (argmax_d) argmax_d[r] = sd.best_idx;
-    if (argmax_t) argmax_t[r] = stt.best_idx;
+    if (argmax_d) argmax_d[r] = first_max(sd, x, nvec << 3);
+    if (argmax_t) argmax_t[r] = best_t;
   }
 }
 

@@ -19,6 +19,11 @@ __device__ __forceinline__ float2x fma2(float2x a, float2x b, float2x c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
+__device__ __forceinline__ float2x mul2(float2x a, float2x b) {
+  float2x r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
 __device__ __forceinline__ float2x add2(float2x a, float2x b) {
   float2x r;
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
