@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import torch
 
+from speculators_b200 import ops
 from speculators_b200.models.eagle3.attention import causal_document_interval
 from speculators_b200.ops import AttnSpec
 
@@ -19,13 +20,20 @@ __all__ = ["anchor_block_attn_spec", "create_anchor_block_mask_mod", "dense_anch
 
 
 def anchor_block_attn_spec(document_ids, anchor_positions, block_size: int, sliding_window: int | None = None,
-                           sliding_window_non_causal: bool = False) -> AttnSpec:
+                           sliding_window_non_causal: bool = False, doc_lo: torch.Tensor | None = None) -> AttnSpec:
+    """``doc_lo``: ``causal_document_interval(document_ids)[0]``, for several specs of the same documents."""
     doc = document_ids.reshape(-1)
     device = doc.device
     a = anchor_positions.to(device=device, dtype=torch.long).reshape(-1)
     n = a.numel()
+    causal_in_block = sliding_window is not None and not sliding_window_non_causal
+    if doc_lo is None:
+        doc_lo, _ = causal_document_interval(doc, None)
+    if doc.is_cuda and doc.dtype == torch.int64:  # one launch
+        lo, hi, extra = ops.native().anchor_spec(doc.contiguous(), doc_lo, a.contiguous(), int(block_size), -1 if sliding_window is None else int(sliding_window),
+                                                 causal_in_block)
+        return AttnSpec(lo=lo, hi=hi, extra_idx=extra, extra_block=int(block_size), extra_block_causal=bool(causal_in_block))
     qa = a.repeat_interleave(block_size)
-    doc_lo, _ = causal_document_interval(doc, None)
     lo = doc_lo[qa].to(torch.int64)
     if sliding_window is not None:
         lo = torch.maximum(lo, qa - int(sliding_window))
@@ -36,7 +44,6 @@ def anchor_block_attn_spec(document_ids, anchor_positions, block_size: int, slid
     slot = torch.arange(block_size, device=device)
     block = torch.arange(n, device=device).repeat_interleave(block_size)
     extra = (block[:, None] * block_size + slot[None, :]).to(torch.int32)
-    causal_in_block = sliding_window is not None and not sliding_window_non_causal
     if causal_in_block:
         q_slot = slot.repeat(n)
         extra = torch.where(slot[None, :] <= q_slot[:, None], extra, torch.full_like(extra, -1))

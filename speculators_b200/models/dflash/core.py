@@ -27,6 +27,7 @@ from speculators_b200.models.dflash.config import DFlashSpeculatorConfig
 from speculators_b200.models.dflash.metrics import compute_metrics
 from speculators_b200.models.dflash.model_definitions import DFlashDecoderLayer
 from speculators_b200.models.dflash.utils import get_base_indices_for_anchored_blocks, select_anchors
+from speculators_b200.models.eagle3.attention import causal_document_interval
 from speculators_b200.models.layers import Linear, RMSNorm, RotaryTable
 from speculators_b200.models.utils import resolve_target_layer_ids
 from speculators_b200.proposals.greedy import GreedyTokenProposalConfig
@@ -95,19 +96,31 @@ class DFlashDraftModel(DraftVocabMixin, SpeculatorModel):
         ids = input_ids.reshape(-1)
 
         anchors, anchor_valid = select_anchors(loss_mask, num_anchors, B)
-        full_spec = anchor_block_attn_spec(doc, anchors, B, None) if self.uses_full_attn else None
+        doc_lo, _ = causal_document_interval(doc, None)
+        full_spec = anchor_block_attn_spec(doc, anchors, B, None, doc_lo=doc_lo) if self.uses_full_attn else None
         win_spec = (
-            anchor_block_attn_spec(doc, anchors, B, self.sliding_window, self.sliding_window_non_causal)
+            anchor_block_attn_spec(doc, anchors, B, self.sliding_window, self.sliding_window_non_causal, doc_lo=doc_lo)
             if self.uses_sliding_window_attn else None
         )
-        block_ids = torch.full((num_anchors * B,), self.mask_token_id, dtype=torch.long, device=device)
-        block_ids[::B] = ids[anchors]
+        one_launch = ids.is_cuda and ids.dtype == torch.int64 and loss_mask.dtype == torch.bool and positions.numel() == ids.numel() == loss_mask.numel() == T
+        if one_launch:
+            block_ids, noise_positions, block_index, target_index, aligned = ops.native().anchor_slots(
+                anchors, anchor_valid, ids.contiguous(), positions.contiguous(), loss_mask.reshape(-1).contiguous(), B, self.mask_token_id,
+                bool(self.config.sample_from_anchor))
+        else:
+            block_ids = torch.full((num_anchors * B,), self.mask_token_id, dtype=torch.long, device=device)
+            block_ids[::B] = ids[anchors]
+            noise_positions = get_base_indices_for_anchored_blocks(positions[anchors], B)
+            block_index = get_base_indices_for_anchored_blocks(anchors, B)
+            target_index = (block_index if self.config.sample_from_anchor else block_index - 1) % T
+            aligned = loss_mask.reshape(-1)[block_index % T].clone()
+            aligned = aligned * anchor_valid.repeat_interleave(B).to(aligned.dtype)
+            aligned = aligned * (block_index < T).to(aligned.dtype)
+            if not self.config.sample_from_anchor:
+                aligned[::B] = 0
         noise = self.embed_tokens(block_ids).to(dtype)
         context = self.hidden_norm(self.fc(hidden_states.reshape(T, -1).to(dtype)))
-        noise_positions = get_base_indices_for_anchored_blocks(positions[anchors], B)
         all_positions = torch.cat([positions, noise_positions])
-        block_index = get_base_indices_for_anchored_blocks(anchors, B)
-        target_index = (block_index if self.config.sample_from_anchor else block_index - 1) % T
         with torch.no_grad():
             vl = verifier_last_hidden_states.reshape(T, -1).to(dtype)[target_index]
             targets = ops.linear(self.verifier_norm(vl), self.verifier_lm_head.weight)
@@ -116,11 +129,6 @@ class DFlashDraftModel(DraftVocabMixin, SpeculatorModel):
             noise = layer(noise, context, noise_positions, all_positions, self.rotary_emb, spec)
         hidden = self.norm(noise)
         logits = ops.linear(hidden, self.lm_head.weight)
-        aligned = loss_mask.reshape(-1)[block_index % T].clone()
-        aligned = aligned * anchor_valid.repeat_interleave(B).to(aligned.dtype)
-        aligned = aligned * (block_index < T).to(aligned.dtype)
-        if not self.config.sample_from_anchor:
-            aligned[::B] = 0
         return hidden.unsqueeze(0), logits.unsqueeze(0), targets.unsqueeze(0), aligned.unsqueeze(0), block_index
 
     def forward(self, hidden_states, input_ids, loss_mask, verifier_last_hidden_states, document_ids, position_ids=None,

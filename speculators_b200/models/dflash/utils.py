@@ -5,7 +5,7 @@ the loss-masked positions (the last ``block_size`` positions are never anchors),
 returns them sorted and padded with zeros, plus a validity flag per slot
 (src/speculators/models/dflash/utils.py:21-67).  It is written with fixed output
 shapes and without reading anything back to the host -- a random key per
-position, ``topk`` of the keys -- so the training step stays capturable in a
+position, the smallest keys taken -- so the training step stays capturable in a
 CUDA graph; the reference uses ``nonzero`` + ``randperm``, which yields the same
 distribution but synchronises.
 """
@@ -13,6 +13,8 @@ distribution but synchronises.
 from __future__ import annotations
 
 import torch
+
+from speculators_b200 import ops
 
 __all__ = ["get_base_indices_for_anchored_blocks", "select_anchors"]
 
@@ -28,6 +30,8 @@ def select_anchors(loss_mask: torch.Tensor, num_anchors: int, block_size: int):
         raise ValueError(f"Expected [B, T], got {loss_mask.shape}")
     if block_size <= 0:
         raise ValueError(f"Expected block size > 0, got {block_size}")
+    if loss_mask.is_cuda:  # one launch
+        return ops.native().select_anchors(loss_mask[0].bool().contiguous(), torch.rand(loss_mask.shape[1], device=loss_mask.device), num_anchors, block_size)
     valid = loss_mask[0].bool().clone()
     valid[-block_size:] = False
     T = valid.shape[0]

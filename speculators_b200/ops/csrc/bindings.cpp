@@ -35,6 +35,10 @@ void launch_heads_bwd(const void* const*, const int64_t*, const int*, const void
                       cudaStream_t);
 void launch_repeated_rows_sum(const void*, int64_t, int, int, float*, void*, int64_t, cudaStream_t);
 void launch_document_interval(const int64_t*, int, int, int*, int*, cudaStream_t);
+void launch_select_anchors(const bool*, const float*, int, int, int, int, int64_t*, bool*, cudaStream_t);
+void launch_anchor_spec(const int64_t*, const int*, int, const int64_t*, int, int, int, int, int*, int*, int*, cudaStream_t);
+void launch_anchor_slots(const int64_t*, const bool*, const int64_t*, const int64_t*, const bool*, int, int, int, int64_t, int, int64_t*, int64_t*, int64_t*,
+                         int64_t*, bool*, cudaStream_t);
 void launch_compact(const bool*, int, int64_t*, int*, cudaStream_t);
 void launch_cod_step(const int64_t*, const int64_t*, int, const bool*, int, int, int, unsigned char*, int64_t*, int64_t*, int64_t*, int64_t*, int*, cudaStream_t);
 void launch_peagle_spec(const int64_t*, const int64_t*, const bool*, const int64_t*, const int*, int, int, int, int, int*, int*, int*, int*, cudaStream_t);
@@ -373,6 +377,45 @@ std::tuple<Tensor, Tensor> document_interval(const Tensor& doc, int64_t window) 
   Tensor lo = both.select(0, 0), hi = both.select(0, 1);
   sb200::launch_document_interval(d, (int)doc.numel(), (int)window, lo.data_ptr<int>(), hi.data_ptr<int>(), cur_stream());
   return {lo, hi};
+}
+// mask bool[T], keys fp32[T] in [0, 1) -> (anchors int64[slots] ascending and padded with zeros, which of them are, bool[slots])
+std::tuple<Tensor, Tensor> select_anchors(const Tensor& mask, const Tensor& keys, int64_t slots, int64_t block) {
+  const int64_t T = mask.numel();
+  const bool* m = bool_ptr(mask, T, "mask");
+  TORCH_CHECK(keys.is_cuda() && keys.scalar_type() == at::kFloat && keys.is_contiguous() && keys.numel() == T, "select_anchors: a float32 key per row expected");
+  TORCH_CHECK(slots >= 0 && block > 0 && T < (int64_t(1) << 31) - 65536 && slots < (int64_t(1) << 31) - 65536);
+  c10::cuda::CUDAGuard guard(mask.device());
+  Tensor anchors = at::empty({slots}, mask.options().dtype(at::kLong)), picked = at::empty({slots}, mask.options());
+  sb200::launch_select_anchors(m, keys.data_ptr<float>(), (int)T, (int)std::min<int64_t>(block, T), (int)slots, (int)std::min(slots, T),
+                               anchors.data_ptr<int64_t>(), picked.data_ptr<bool>(), cur_stream());
+  return {anchors, picked};
+}
+// doc_lo int32[T]: start of each row's document; window < 0: none -> lo, hi int32[n * block], extra int32[n * block, block]
+std::tuple<Tensor, Tensor, Tensor> anchor_spec(const Tensor& doc, const Tensor& doc_lo, const Tensor& anchors, int64_t block, int64_t window, bool causal) {
+  const int64_t T = doc.numel(), n = anchors.numel();
+  const int64_t *d = long_ptr(doc, "document_ids"), *a = long_ptr(anchors, "anchors");
+  TORCH_CHECK(doc_lo.is_cuda() && doc_lo.scalar_type() == at::kInt && doc_lo.is_contiguous() && doc_lo.numel() == T, "doc_lo: int32 per row expected");
+  TORCH_CHECK(block > 0 && n * block * block < (int64_t(1) << 31) * 64 && n * block < (int64_t(1) << 31));
+  c10::cuda::CUDAGuard guard(doc.device());
+  auto opt = doc_lo.options();
+  Tensor lo = at::empty({n * block}, opt), hi = at::empty({n * block}, opt), extra = at::empty({n * block, block}, opt);
+  sb200::launch_anchor_spec(d, doc_lo.data_ptr<int>(), (int)T, a, (int)n, (int)block, (int)std::min<int64_t>(window, (int64_t(1) << 31) - 1), causal ? 1 : 0,
+                            lo.data_ptr<int>(), hi.data_ptr<int>(), extra.data_ptr<int>(), cur_stream());
+  return {lo, hi, extra};
+}
+// anchors as select_anchors gives them -> token, position, row, target row (int64[n * block]), counted (bool[n * block])
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> anchor_slots(const Tensor& anchors, const Tensor& picked, const Tensor& ids, const Tensor& positions,
+                                                                const Tensor& mask, int64_t block, int64_t mask_token, bool from_anchor) {
+  const int64_t T = mask.numel(), n = anchors.numel(), N = n * block;
+  const int64_t *a = long_ptr(anchors, "anchors"), *i = long_ptr(ids, "ids"), *pos = long_ptr(positions, "positions");
+  const bool *pk = bool_ptr(picked, n, "picked"), *m = bool_ptr(mask, T, "mask");
+  TORCH_CHECK(ids.numel() == T && positions.numel() == T && T > 0 && block > 0 && N < (int64_t(1) << 31));
+  c10::cuda::CUDAGuard guard(anchors.device());
+  Tensor of = at::empty({4, N}, anchors.options()), counts = at::empty({N}, mask.options());
+  Tensor token = of.select(0, 0), position = of.select(0, 1), index = of.select(0, 2), target = of.select(0, 3);
+  sb200::launch_anchor_slots(a, pk, i, pos, m, (int)T, (int)n, (int)block, mask_token, from_anchor ? 1 : 0, token.data_ptr<int64_t>(), position.data_ptr<int64_t>(),
+                             index.data_ptr<int64_t>(), target.data_ptr<int64_t>(), counts.data_ptr<bool>(), cur_stream());
+  return {token, position, index, target, counts};
 }
 // positions of the set entries -> (int64[T] of which the first count are filled, int32[1] count)
 std::tuple<Tensor, Tensor> compact_rows(const Tensor& valid) {
@@ -1513,6 +1556,9 @@ TORCH_LIBRARY(sb200, m) {
         "Tensor? target_row=None, Tensor? live=None) -> Tensor", &loss_bwd_scaled);
   m.def("repeated_rows_sum", &repeated_rows_sum);
   m.def("document_interval", &document_interval);
+  m.def("select_anchors", &select_anchors);
+  m.def("anchor_spec", &anchor_spec);
+  m.def("anchor_slots", &anchor_slots);
   m.def("compact_rows", &compact_rows);
   m.def("cod_step", &cod_step);
   m.def("peagle_spec", &peagle_spec);

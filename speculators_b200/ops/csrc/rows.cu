@@ -421,7 +421,125 @@ embedding_join_kernel(const int64_t* __restrict__ ids, const float* __restrict__
   }
 }
 
+// ---- anchored blocks (DFlash, DSpark) ------------------------------------------------------------
+// Up to `take_most` of the valid rows, the ones with the smallest keys (keys in [0, 1), ties to the lower row), ascending, padded with
+// zeros; a flag per slot.  The last `block` rows are never anchors.  One block: the k-th smallest key by its bits, eight at a time
+// (positive floats order like their bits), then an ordered compaction.  As a top-k of the keys, a sort of the picks and the
+// arithmetic around them it was 25 launches: 512 of 3000 rows, blocks of 8, took 85 us, now 11, and with the two specs and the slots' indices
+// (70 launches) 190 us, now 27.
+__global__ void __launch_bounds__(kT)
+select_anchors_kernel(const bool* __restrict__ mask, const float* __restrict__ keys, int T, int block, int slots, int take_most, int64_t* __restrict__ anchors,
+                      bool* __restrict__ picked) {
+  pdl_begin();
+  __shared__ int scratch[32], total, hist[256], sh_digit, sh_below, cutoff;
+  const int usable = T - block;  // rows from there on are never anchors
+  auto valid = [&](int i) { return i < usable && mask[i]; };
+  auto bits = [&](int i) { return __float_as_uint(keys[i]); };
+  for (int i = threadIdx.x; i < slots; i += kT) {
+    anchors[i] = 0;
+    picked[i] = false;
+  }
+  int mine = 0;
+  for (int i = threadIdx.x; i < usable; i += kT) mine += mask[i] ? 1 : 0;
+  block_scan(mine, [](int a, int b) { return a + b; }, scratch);
+  __syncthreads();
+  int n = 0;
+  for (int w = 0; w < 32; ++w) n += scratch[w];
+  const int take = min(take_most, n);
+  unsigned thr = 0xffffffffu;
+  int last = T;  // equal keys count up to this row
+  if (take < n && take > 0) {
+    unsigned prefix = 0, known = 0;
+    int need = take;  // of the keys that share the digits found so far
+    for (int shift = 24; shift >= 0; shift -= 8) {
+      for (int i = threadIdx.x; i < 256; i += kT) hist[i] = 0;
+      __syncthreads();
+      for (int i = threadIdx.x; i < usable; i += kT)
+        if (mask[i] && (bits(i) & known) == prefix) atomicAdd(&hist[(bits(i) >> shift) & 255], 1);
+      __syncthreads();
+      const int h = threadIdx.x < 256 ? hist[threadIdx.x] : 0;
+      const int upto = block_scan(h, [](int a, int b) { return a + b; }, scratch);
+      if (threadIdx.x < 256 && upto >= need && upto - h < need) {
+        sh_digit = threadIdx.x;
+        sh_below = upto - h;
+      }
+      __syncthreads();
+      prefix |= (unsigned)sh_digit << shift;
+      known |= 255u << shift;
+      need -= sh_below;
+      if (shift == 0) total = hist[sh_digit];
+      __syncthreads();
+    }
+    thr = prefix;
+    if (total > need) {  // more keys equal the last one taken than are wanted
+      compact(usable, [&](int i) { return mask[i] && bits(i) == thr; }, [&](int rank, int i) { if (rank == need - 1) cutoff = i; }, scratch, &total);
+      last = cutoff;
+    }
+  }
+  if (take > 0)
+    compact(usable, [&](int i) { return valid(i) && (bits(i) < thr || (bits(i) == thr && i <= last)); },
+            [&](int rank, int i) { anchors[rank] = i; picked[rank] = true; }, scratch, &total);
+}
+
+// Context interval of a block's rows - the anchor's document before the anchor, inside the window if there is one - and the rows of the
+// block as extra keys (up to the row itself with `causal`).  One thread an extra key.
+__global__ void __launch_bounds__(256)
+anchor_spec_kernel(const int64_t* __restrict__ doc, const int* __restrict__ doc_lo, int T, const int64_t* __restrict__ anchors, int n, int block, int window,
+                   int causal, int* __restrict__ lo, int* __restrict__ hi, int* __restrict__ extra) {
+  pdl_begin();
+  const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  const int64_t row = e / block;
+  if (row >= (int64_t)n * block) return;
+  const int slot = (int)(e - row * block);
+  const int64_t blk = row / block;
+  extra[e] = !causal || slot <= (int)(row - blk * block) ? (int)(blk * block) + slot : -1;
+  if (slot != 0) return;
+  const int64_t a = anchors[blk];
+  const bool seen = a >= 0 && a < T && doc[a] != -1;
+  const int first = seen ? doc_lo[a] : 0;
+  lo[row] = !seen ? 0 : window >= 0 ? max(first, (int)a - window) : first;
+  hi[row] = seen ? (int)a : 0;
+}
+
+// What a block's slots read: token, position, row of the packed sequence, row of the targets, and whether a loss counts there.
+__global__ void __launch_bounds__(256)
+anchor_slots_kernel(const int64_t* __restrict__ anchors, const bool* __restrict__ picked, const int64_t* __restrict__ ids, const int64_t* __restrict__ positions,
+                    const bool* __restrict__ mask, int T, int n, int block, int64_t mask_token, int from_anchor, int64_t* __restrict__ token,
+                    int64_t* __restrict__ position, int64_t* __restrict__ index, int64_t* __restrict__ target, bool* __restrict__ counts) {
+  pdl_begin();
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= n * block) return;
+  const int blk = i / block, slot = i - blk * block;
+  const int64_t a = anchors[blk], at = a + slot;
+  token[i] = slot == 0 ? ids[a] : mask_token;
+  position[i] = positions[a] + slot;
+  index[i] = at;
+  const int64_t t = from_anchor ? at : at - 1;
+  target[i] = t < 0 ? t + T : t % T;
+  counts[i] = picked[blk] && at < T && mask[at] && (from_anchor || slot != 0);
+}
+
 }  // namespace rows
+
+void launch_select_anchors(const bool* mask, const float* keys, int T, int block, int slots, int take_most, int64_t* anchors, bool* picked, cudaStream_t stream) {
+  count_launch(1);
+  launch_pdl(rows::select_anchors_kernel, 1, rows::kT, 0, stream, mask, keys, T, block, slots, take_most, anchors, picked);
+}
+void launch_anchor_spec(const int64_t* doc, const int* doc_lo, int T, const int64_t* anchors, int n, int block, int window, int causal, int* lo, int* hi,
+                        int* extra, cudaStream_t stream) {
+  const int64_t elements = (int64_t)n * block * block;
+  if (elements <= 0) return;
+  count_launch(1);
+  launch_pdl(rows::anchor_spec_kernel, (int)((elements + 255) / 256), 256, 0, stream, doc, doc_lo, T, anchors, n, block, window, causal, lo, hi, extra);
+}
+void launch_anchor_slots(const int64_t* anchors, const bool* picked, const int64_t* ids, const int64_t* positions, const bool* mask, int T, int n, int block,
+                         int64_t mask_token, int from_anchor, int64_t* token, int64_t* position, int64_t* index, int64_t* target, bool* counts,
+                         cudaStream_t stream) {
+  if (n * block <= 0) return;
+  count_launch(1);
+  launch_pdl(rows::anchor_slots_kernel, (n * block + 255) / 256, 256, 0, stream, anchors, picked, ids, positions, mask, T, n, block, mask_token, from_anchor, token,
+             position, index, target, counts);
+}
 
 void launch_document_interval(const int64_t* doc, int T, int window, int* lo, int* hi, cudaStream_t stream) {
   if (T <= 0) return;

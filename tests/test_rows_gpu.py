@@ -126,3 +126,47 @@ def test_embedding_gradient_of_frequent_ids(lengths, H, padding, attached):
     want, size = (torch.zeros(w.shape, dtype=torch.double, device="cuda").index_add_(0, ids[keep], 2 * x.double()[keep]) for x in (d, d.abs()))
     # fp32 sums of at most max(lengths) terms; the sum is rounded to bf16, and so is its double
     assert ((got - want).abs() <= 2.0**-8 * want.abs() + max(lengths) * 2.0**-24 * size).all()
+
+
+# ---- anchored blocks --------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("T,slots,block", [(1, 4, 8), (8, 4, 8), (9, 4, 8), (100, 200, 8), (700, 64, 16), (8192, 512, 8), (8193, 512, 16), (20000, 3000, 4)])
+@pytest.mark.parametrize("density", [0.0, 0.02, 0.6, 1.0])
+@pytest.mark.parametrize("distinct", [True, False])
+def test_anchors_are_the_smallest_keys_in_order(T, slots, block, density, distinct):
+    g = torch.Generator(device="cuda").manual_seed(T + slots)
+    mask = torch.rand(T, generator=g, device="cuda") < density
+    keys = torch.rand(T, generator=g, device="cuda")
+    if not distinct:  # few keys: many equal the last one taken
+        keys = (keys * 3).floor() / 3
+    anchors, picked = ops.native().select_anchors(mask, keys, slots, block)
+    valid = [i for i in range(max(T - block, 0)) if mask[i]] if T < 1000 else torch.nonzero(mask[: T - block]).flatten().tolist()
+    k = keys.tolist()
+    want = sorted(sorted(valid, key=lambda i: (k[i], i))[: min(slots, T)])
+    assert anchors.tolist() == want + [0] * (slots - len(want)) and picked.tolist() == [True] * len(want) + [False] * (slots - len(want))
+
+
+@pytest.mark.parametrize("window,non_causal", [(None, False), (5, False), (5, True), (10**6, False)])
+@pytest.mark.parametrize("block", [1, 3, 8])
+def test_anchor_specs_and_slots_match_their_definition(window, non_causal, block):
+    from speculators_b200.models.dflash.attention import anchor_block_attn_spec
+
+    T, mask_token = 90, 77
+    doc = torch.tensor([0] * 20 + [1] * 31 + [2] * 29 + [-1] * 10)
+    anchors, picked = torch.tensor([0, 3, 19, 20, 50, 79, 81, 89, 0, 0]), torch.tensor([True] * 8 + [False] * 2)
+    want = anchor_block_attn_spec(doc, anchors, block, window, non_causal)
+    got = anchor_block_attn_spec(doc.cuda(), anchors.cuda(), block, window, non_causal)
+    for a, b in ((got.lo, want.lo), (got.hi, want.hi), (got.extra_idx, want.extra_idx)):
+        assert a.dtype == b.dtype and torch.equal(a.cpu(), b)
+    assert (got.extra_block, got.extra_block_causal) == (want.extra_block, want.extra_block_causal)
+
+    ids, positions, mask = torch.arange(T) * 3 + 1, torch.arange(T) % 31, torch.arange(T) % 4 != 1
+    index = (anchors[:, None] + torch.arange(block)).reshape(-1)
+    for from_anchor in (False, True):
+        token = torch.full((len(index),), mask_token)
+        token[::block] = ids[anchors]
+        counts = mask[index % T] & picked.repeat_interleave(block) & (index < T)
+        if not from_anchor:
+            counts[::block] = False
+        want = token, (positions[anchors][:, None] + torch.arange(block)).reshape(-1), index, (index if from_anchor else index - 1) % T, counts
+        got = ops.native().anchor_slots(anchors.cuda(), picked.cuda(), ids.cuda(), positions.cuda(), mask.cuda(), block, mask_token, from_anchor)
+        assert all(torch.equal(a.cpu(), b) for a, b in zip(got, want))
