@@ -23,7 +23,7 @@ import torch
 from torch import nn
 
 from speculators_b200 import ops
-from speculators_b200.models.layers import Linear
+from speculators_b200.models.layers import Linear, unobserved
 
 __all__ = ["ConfidenceHead", "MarkovHead"]
 
@@ -47,7 +47,12 @@ class MarkovHead(nn.Module):
             self.joint_proj = Linear(2 * r + hidden_size, 3 * r, bias=True)  # input order [s; e; h]
 
     def prev_embeddings(self, token_ids: torch.Tensor) -> torch.Tensor:
-        return self.markov_w1(token_ids.long())
+        table, ids = self.markov_w1, token_ids.long()
+        if (not hasattr(table.weight, "_flat_grad") or type(table) is not nn.Embedding or not unobserved(table) or table.max_norm is not None
+                or table.sparse or table.scale_grad_by_freq):
+            return table(ids)
+        # under the training engine: rows of the gradient straight into its buffer, where autograd's own is a table of zeros that is added to it
+        return ops.embedding(ids, table.weight, table.padding_idx).view(*ids.shape, -1)
 
     # ------------------------------------------------------------------ features f_k
     def features(self, prev_emb: torch.Tensor, hidden_states: torch.Tensor | None) -> torch.Tensor:
