@@ -24,14 +24,18 @@ def _is_fused(fn) -> bool:
     return getattr(fn, "__module__", "") == fused.__name__
 
 
-def rowwise_terms(loss_config: LossConfig, logits2d, targets2d, shift: int, rows: int, active=None):
-    """-> ``({name: loss[rows]}, argmax_logits[rows], argmax_targets[rows])``."""
+def rowwise_terms(loss_config: LossConfig, logits2d, targets2d, shift: int, rows: int, active=None, target_row=None, tv_out: list | None = None):
+    """-> ``({name: loss[rows]}, argmax_logits[rows], argmax_targets[rows])``.  ``target_row``: the row of the targets that each row is
+    compared with, in place of a shift.  ``tv_out`` (optional): takes the rows' total variation where it comes with a term."""
     out: dict[str, torch.Tensor] = {}
     am_d = am_t = None
 
     def prim(op: str):
         nonlocal am_d, am_t
-        loss, a, b = fused_row_loss(op, logits2d, targets2d, shift=shift, rows=rows, active=active)
+        with_tv = tv_out is not None and not tv_out and op == "kl_div"
+        loss, a, b, *tv = fused_row_loss(op, logits2d, targets2d, shift=shift, rows=rows, active=active, target_row=target_row, with_tv=with_tv)
+        if with_tv:
+            tv_out.extend(tv)
         if am_d is None:
             am_d, am_t = a, b
         return loss
@@ -49,9 +53,9 @@ def rowwise_terms(loss_config: LossConfig, logits2d, targets2d, shift: int, rows
                 out[name] = lam * prim("kl_div") + (1.0 - lam) * tv
         else:
             lg = logits2d[:rows].unsqueeze(0)
-            tg = targets2d[shift : shift + rows].unsqueeze(0)
+            tg = (targets2d[shift : shift + rows] if target_row is None else targets2d[target_row[:rows].long()]).unsqueeze(0)
             out[name] = fn(lg, tg).reshape(rows)
     if am_d is None:
         am_d = logits2d[:rows].argmax(-1)
-        am_t = targets2d[shift : shift + rows].argmax(-1)
+        am_t = targets2d.argmax(-1)[target_row[:rows].long()] if target_row is not None else targets2d[shift : shift + rows].argmax(-1)
     return out, am_d, am_t

@@ -20,11 +20,13 @@ def block_decay_fn(per_position_loss_weight: str, loss_mask, block_size: int, ga
     return partial(dflash_loss_decay, gamma=gamma, sample_from_anchor=sample_from_anchor)
 
 
-def weighted_terms(loss_config: LossConfig, logits, targets, loss_mask, pos_idx, decay_fn):
-    """-> (loss, {term scalars}, pred_ids, target_ids)"""
+def weighted_terms(loss_config: LossConfig, logits, targets, loss_mask, pos_idx, decay_fn, target_row=None, tv_out: list | None = None):
+    """-> (loss, {term scalars}, pred_ids, target_ids).  Rows without a loss are skipped: they weigh nothing in a sum or counter.
+    ``target_row``, ``tv_out`` as in ``rowwise_terms``."""
     n = logits.shape[1]
     per_term, pred_ids, target_ids = rowwise_terms(
-        loss_config, logits.reshape(n, -1), targets.reshape(n, -1), shift=0, rows=n, active=None
+        loss_config, logits.reshape(n, -1), targets.reshape(targets.shape[1], -1), shift=0, rows=n, active=loss_mask.reshape(-1) != 0,
+        target_row=target_row, tv_out=tv_out,
     )
     loss = torch.zeros((), device=logits.device, dtype=torch.float32)
     parts = {}
@@ -37,14 +39,14 @@ def weighted_terms(loss_config: LossConfig, logits, targets, loss_mask, pos_idx,
 
 
 def compute_metrics(logits, targets, loss_mask, block_size: int = 1, gamma: float = 4.0, loss_config: LossConfig | None = None,
-                    per_position_loss_weight: str = "fixed-exp-decay", dpace_alpha: float = 0.5, sample_from_anchor: bool = False):
+                    per_position_loss_weight: str = "fixed-exp-decay", dpace_alpha: float = 0.5, sample_from_anchor: bool = False, target_row=None):
     if loss_config is None:
         loss_config = {"kl_div": (kl_div_loss, 1.0)}
     device = logits.device
     n = logits.shape[1]
     pos_idx = (torch.arange(n, device=device) % block_size).unsqueeze(0)
     decay = block_decay_fn(per_position_loss_weight, loss_mask, block_size, gamma, dpace_alpha, sample_from_anchor)
-    loss, parts, pred_ids, target_ids = weighted_terms(loss_config, logits, targets, loss_mask, pos_idx, decay)
+    loss, parts, pred_ids, target_ids = weighted_terms(loss_config, logits, targets, loss_mask, pos_idx, decay, target_row)
     correct, total = compute_accuracy_multi_step(pred_ids.unsqueeze(0), target_ids.unsqueeze(0), loss_mask, pos_idx, block_size)
     one = torch.ones((), device=device)
     metrics = {"loss_sum": loss.detach().clone(), "loss_total": one}
@@ -54,13 +56,9 @@ def compute_metrics(logits, targets, loss_mask, block_size: int = 1, gamma: floa
     start = 0 if sample_from_anchor else 1
     metrics["full_acc_sum"] = correct[start:].sum()
     metrics["full_acc_total"] = total[start:].sum()
-    eal = torch.zeros((), device=device)
-    run = torch.ones((), device=device)
     for pos in range(start, block_size):
         metrics[f"position_{pos}_acc_sum"] = correct[pos]
         metrics[f"position_{pos}_acc_total"] = total[pos]
-        run = run * (correct[pos] / total[pos].clamp(min=1.0))
-        eal = eal + run
-    metrics["eal_sum"] = eal
+    metrics["eal_sum"] = (correct[start:] / total[start:].clamp(min=1.0)).cumprod(0).sum()
     metrics["eal_total"] = one.clone()
     return loss, metrics

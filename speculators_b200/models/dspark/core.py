@@ -110,7 +110,7 @@ class DSparkDraftModel(DFlashDraftModel):
     def forward(self, hidden_states, input_ids, loss_mask, verifier_last_hidden_states, document_ids, position_ids=None,
                 loss_config: LossConfig | None = None, tv_loss_fn=tv_loss, gamma: float = 4.0, max_anchors: int = 3072,
                 confidence_head_alpha: float = 1.0, per_position_loss_weight: str = "fixed-exp-decay", dpace_alpha: float = 0.5, **kwargs):
-        hidden, logits, targets, slot_mask, block_index = self._backbone_forward(
+        hidden, logits, targets, slot_mask, block_index, target_row = self._backbone_forward(
             hidden_states, input_ids, loss_mask, verifier_last_hidden_states, document_ids, position_ids, max_anchors=max_anchors
         )
         logits, confidence = self._apply_heads(hidden, logits, self._previous_tokens(input_ids, block_index, max_anchors))
@@ -118,6 +118,6 @@ class DSparkDraftModel(DFlashDraftModel):
             logits, targets, confidence, slot_mask, self.block_size, loss_config=loss_config or {"kl_div": (kl_div_loss, 1.0)},
             tv_loss_fn=tv_loss_fn, gamma=gamma, confidence_head_alpha=confidence_head_alpha,
             per_position_loss_weight=per_position_loss_weight, dpace_alpha=dpace_alpha,
-            sample_from_anchor=self.config.sample_from_anchor,
+            sample_from_anchor=self.config.sample_from_anchor, target_row=target_row,
         )
         return None, loss, metrics

@@ -16,6 +16,7 @@ from torch.nn.functional import binary_cross_entropy_with_logits
 from speculators_b200.losses import LossConfig, tv_loss
 from speculators_b200.models.dflash.metrics import block_decay_fn, weighted_terms
 from speculators_b200.models.metrics import compute_accuracy_multi_step
+from speculators_b200.ops import fused_row_loss
 
 __all__ = ["compute_metrics"]
 
@@ -34,16 +35,24 @@ def _confidence_loss(bce: torch.Tensor, mask_f: torch.Tensor, weights: torch.Ten
 
 def compute_metrics(logits, targets, confidence_logits, loss_mask, block_size: int, loss_config: LossConfig, tv_loss_fn=tv_loss,
                     gamma: float = 4.0, confidence_head_alpha: float = 1.0, per_position_loss_weight: str = "fixed-exp-decay",
-                    dpace_alpha: float = 0.5, sample_from_anchor: bool = True):
+                    dpace_alpha: float = 0.5, sample_from_anchor: bool = True, target_row=None):
     device = logits.device
     n = logits.shape[1]
     first = 0 if sample_from_anchor else 1
     slot = (torch.arange(n, device=device) % block_size).unsqueeze(0)
     decay = block_decay_fn(per_position_loss_weight, loss_mask, block_size, gamma, dpace_alpha, sample_from_anchor)
-    loss, parts, pred_ids, target_ids = weighted_terms(loss_config, logits, targets, loss_mask, slot, decay)
+    tv: list[torch.Tensor] | None = [] if tv_loss_fn is tv_loss and logits.is_cuda else None
+    loss, parts, pred_ids, target_ids = weighted_terms(loss_config, logits, targets, loss_mask, slot, decay, target_row, tv)
 
     with torch.no_grad():
-        accept = 1.0 - tv_loss_fn(logits.detach(), targets)  # [1, n] analytic acceptance rate
+        # [1, n] analytic acceptance rate: next to the divergence where that is the loss, on the rows with a loss; else a pass of its own
+        if tv:
+            accept = 1.0 - tv[0].unsqueeze(0)
+        elif tv is not None:
+            accept = 1.0 - fused_row_loss("tv", logits.detach().reshape(n, -1), targets.reshape(targets.shape[1], -1), rows=n,
+                                          active=loss_mask.reshape(-1) != 0, target_row=target_row)[0].unsqueeze(0)
+        else:
+            accept = 1.0 - tv_loss_fn(logits.detach(), targets if target_row is None else targets[:, target_row.long()])
         mask_f = loss_mask.to(accept.dtype)
         drafted = _per_block(mask_f, block_size, first)
         accept_run = (_per_block(accept, block_size, first) * drafted).cumprod(dim=-1)

@@ -1180,19 +1180,20 @@ def _row_loss_ref(op: str, logits, targets):
 
 class _RowLossFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, logits, targets, op, shift, rows, active):
-        loss, stats, am_d, am_t = native().loss_fwd(op, logits, targets, active, shift, rows)
-        ctx.save_for_backward(logits, targets, stats)
+    def forward(ctx, logits, targets, op, shift, rows, active, target_row=None, with_tv=False):
+        loss, stats, am_d, am_t, tv = native().loss_fwd_tv(op, logits, targets, active, None, shift, rows, target_row, with_tv)
+        ctx.save_for_backward(logits, targets, stats, target_row)
         ctx.cfg = (op, shift, rows)
-        ctx.mark_non_differentiable(am_d, am_t)
-        return loss, am_d, am_t
+        out = (am_d, am_t, tv) if with_tv else (am_d, am_t)
+        ctx.mark_non_differentiable(*out)
+        return loss, *out
 
     @staticmethod
-    def backward(ctx, dloss, _a, _b):
-        logits, targets, stats = ctx.saved_tensors
+    def backward(ctx, dloss, *_):
+        logits, targets, stats, target_row = ctx.saved_tensors
         op, shift, rows = ctx.cfg
-        d = native().loss_bwd(op, logits, targets, dloss.contiguous().float(), stats, shift, rows)
-        return d, None, None, None, None, None
+        d = native().loss_bwd_scaled(op, logits, targets, dloss.contiguous().float(), None, stats, shift, rows, target_row)
+        return d, None, None, None, None, None, None, None
 
 
 class _LmHeadLossFn(torch.autograd.Function):
@@ -1340,11 +1341,12 @@ def fused_row_loss_raw(op: str, logits, targets, shift: int, rows: int, active):
     return _RowLossFn.apply(logits, targets, LOSS_OPS[op], shift, rows, active)
 
 
-def fused_row_loss(op: str, logits, targets, shift: int = 0, rows: int | None = None, active=None):
-    """Per-row loss between ``logits[r]`` and ``targets[r + shift]`` for ``r < rows``.
+def fused_row_loss(op: str, logits, targets, shift: int = 0, rows: int | None = None, active=None, target_row=None, with_tv: bool = False):
+    """Per-row loss between ``logits[r]`` and ``targets[r + shift]`` (``targets[target_row[r]]`` with int32 ``target_row``) for
+    ``r < rows``.
 
-    Returns ``(loss[rows] fp32, argmax_logits[rows], argmax_targets[rows])``.
-    ``active`` (bool[rows], optional) marks rows worth computing; inactive rows get
+    Returns ``(loss[rows] fp32, argmax_logits[rows], argmax_targets[rows])``, and for ``kl_div`` ``with_tv`` also the rows' total
+    variation (no gradient).  ``active`` (bool[rows], optional) marks rows worth computing; inactive rows get
     loss 0 and sentinel argmaxes (-1 / -2, never equal).  Gradients flow to
     ``logits`` only; the buffer that comes back has ``logits.shape`` with rows
     ``>= rows`` zeroed.
@@ -1352,24 +1354,25 @@ def fused_row_loss(op: str, logits, targets, shift: int = 0, rows: int | None = 
     if logits.dim() != 2 or targets.dim() != 2:
         raise ValueError("fused_row_loss expects [rows, V] inputs")
     if rows is None:
-        rows = min(logits.shape[0], targets.shape[0] - shift)
+        rows = logits.shape[0] if target_row is not None else min(logits.shape[0], targets.shape[0] - shift)
     if _use_native(logits):
         if logits.stride(-1) != 1:
             logits = logits.contiguous()
         if targets.stride(-1) != 1:
             targets = targets.contiguous()
-        loss, am_d, am_t = _RowLossFn.apply(logits, targets, LOSS_OPS[op], shift, rows, active)
-        return loss, am_d.long(), am_t.long()
+        loss, am_d, am_t, *tv = _RowLossFn.apply(logits, targets, LOSS_OPS[op], shift, rows, active, target_row, with_tv)
+        return loss, am_d.long(), am_t.long(), *tv
     lg = logits[:rows]
-    tg = targets[shift : shift + rows]
+    tg = targets[target_row.long()[:rows]] if target_row is not None else targets[shift : shift + rows]
     loss = _row_loss_ref(op, lg, tg)
+    tv = [_row_loss_ref("tv", lg.detach(), tg)] if with_tv else []
     am_d, am_t = lg.argmax(-1), tg.argmax(-1)
     if active is not None:
         act = active.bool()
-        loss = torch.where(act, loss, torch.zeros_like(loss))
+        loss, *tv = (torch.where(act, v, torch.zeros_like(v)) for v in (loss, *tv))
         am_d = torch.where(act, am_d, torch.full_like(am_d, -1))
         am_t = torch.where(act, am_t, torch.full_like(am_t, -2))
-    return loss, am_d, am_t
+    return loss, am_d, am_t, *tv
 
 
 class _TokenCEFn(torch.autograd.Function):

@@ -65,7 +65,7 @@ int launch_gemm_grouped_swiglu(const void*, const void*, void*, void*, int, int,
 void launch_rope(void*, const int64_t*, const float*, const float*, int64_t, int, int, int, int64_t,
                  int64_t, float, const int*, cudaStream_t);
 int launch_loss_fwd(int, const void*, const void*, const uint8_t*, const uint8_t*, const int64_t*, float*, float*, int*,
-                    int*, int, int, int64_t, int64_t, int, const int*, cudaStream_t);
+                    int*, int, int, int64_t, int64_t, int, const int*, float*, cudaStream_t);
 int launch_loss_bwd(int, const void*, const void*, const float*, const float*, const float*, void*, int, int, int,
                     int64_t, int64_t, int64_t, int, const int*, const int*, cudaStream_t);
 int64_t launch_count();
@@ -700,9 +700,9 @@ const int* row_targets(const c10::optional<Tensor>& t, int64_t rows) {
 }
 
 // target_row: rows of `targets` to compare with, in place of a shift (they are not checked against its size)
-std::tuple<Tensor, Tensor, Tensor, Tensor> loss_fwd_either(int64_t op, const Tensor& logits, const Tensor& targets, const c10::optional<Tensor>& active,
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> loss_fwd_tv(int64_t op, const Tensor& logits, const Tensor& targets, const c10::optional<Tensor>& active,
                                                            const c10::optional<Tensor>& also, int64_t shift, int64_t rows,
-                                                           const c10::optional<Tensor>& target_row) {
+                                                           const c10::optional<Tensor>& target_row, bool with_tv) {
   TORCH_CHECK(logits.is_cuda() && targets.is_cuda());
   TORCH_CHECK(logits.scalar_type() == at::kBFloat16 && targets.scalar_type() == at::kBFloat16);
   TORCH_CHECK(logits.dim() == 2 && targets.dim() == 2 && logits.stride(1) == 1 &&
@@ -714,12 +714,19 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> loss_fwd_either(int64_t op, const Ten
   Tensor stats = at::empty({5, rows}, fopt);
   Tensor am_d = at::empty({rows}, logits.options().dtype(at::kInt));
   Tensor am_t = at::empty({rows}, logits.options().dtype(at::kInt));
+  Tensor tv = at::empty({with_tv ? rows : 0}, fopt);
   const int rc = sb200::launch_loss_fwd((int)op, logits.data_ptr(), targets.data_ptr(), row_flags(active, rows), row_flags(also, rows), nullptr,
                                         loss.data_ptr<float>(), stats.data_ptr<float>(),
                                         am_d.data_ptr<int>(), am_t.data_ptr<int>(), (int)rows,
                                         (int)logits.size(1), logits.stride(0), targets.stride(0),
-                                        (int)shift, row_targets(target_row, rows), cur_stream());
+                                        (int)shift, row_targets(target_row, rows), with_tv ? tv.data_ptr<float>() : nullptr, cur_stream());
   TORCH_CHECK(rc == 0, "loss_fwd: unknown op ", op);
+  return {loss, stats, am_d, am_t, tv};
+}
+std::tuple<Tensor, Tensor, Tensor, Tensor> loss_fwd_either(int64_t op, const Tensor& logits, const Tensor& targets, const c10::optional<Tensor>& active,
+                                                           const c10::optional<Tensor>& also, int64_t shift, int64_t rows,
+                                                           const c10::optional<Tensor>& target_row) {
+  auto [loss, stats, am_d, am_t, tv] = loss_fwd_tv(op, logits, targets, active, also, shift, rows, target_row, false);
   return {loss, stats, am_d, am_t};
 }
 std::tuple<Tensor, Tensor, Tensor, Tensor> loss_fwd(int64_t op, const Tensor& logits, const Tensor& targets, const c10::optional<Tensor>& active, int64_t shift,
@@ -895,7 +902,7 @@ std::tuple<Tensor, Tensor> ce_label_fwd(const Tensor& logits, const Tensor& labe
   }
   const int rc = sb200::launch_loss_fwd(3, logits.data_ptr(), nullptr, act, nullptr, labels.data_ptr<int64_t>(), loss.data_ptr<float>(),
                                         stats.data_ptr<float>(), nullptr, nullptr, (int)rows, (int)logits.size(1),
-                                        logits.stride(0), logits.stride(0), 0, nullptr, cur_stream());
+                                        logits.stride(0), logits.stride(0), 0, nullptr, nullptr, cur_stream());
   TORCH_CHECK(rc == 0, "ce_label_fwd failed (", rc, ")");
   return {loss, stats};
 }
@@ -1552,6 +1559,8 @@ TORCH_LIBRARY(sb200, m) {
         "Tensor", &rope_merge);
   m.def("loss_fwd_either(int op, Tensor logits, Tensor targets, Tensor? active, Tensor? also, int shift, int rows, Tensor? target_row=None) -> "
         "(Tensor, Tensor, Tensor, Tensor)", &loss_fwd_either);
+  m.def("loss_fwd_tv(int op, Tensor logits, Tensor targets, Tensor? active, Tensor? also, int shift, int rows, Tensor? target_row, bool with_tv) -> "
+        "(Tensor, Tensor, Tensor, Tensor, Tensor)", &loss_fwd_tv);
   m.def("loss_bwd_scaled(int op, Tensor logits, Tensor targets, Tensor grad_out, Tensor? grad_scale, Tensor stats, int shift, int rows, "
         "Tensor? target_row=None, Tensor? live=None) -> Tensor", &loss_bwd_scaled);
   m.def("repeated_rows_sum", &repeated_rows_sum);

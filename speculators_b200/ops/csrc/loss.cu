@@ -23,7 +23,8 @@
 
 namespace sb200 {
 
-enum LossOp : int { kOpKL = 0, kOpRKL = 1, kOpJSD = 2, kOpCE = 3, kOpTV = 4 };
+// kOpKLTV: the KL divergence, and the total variation next to it (forward only)
+enum LossOp : int { kOpKL = 0, kOpRKL = 1, kOpJSD = 2, kOpCE = 3, kOpTV = 4, kOpKLTV = 5 };
 constexpr int kLossThreads = 512;
 constexpr int kNumStats = 5;  // m_d, z_d, m_t, z_t, per-op extra
 
@@ -159,13 +160,14 @@ __device__ __forceinline__ int first_max(const Share& s, const __nv_bfloat16* ro
 // total variation 220 and 168, cross-entropy 8192 x 32000 253 and 205, labels 300 x 151936 38.5 and 29.8, 2460 x 151936 170 and 144
 // (reading takes 20, 80, 80, 160, 14 and 114).
 template <int OP>
-__global__ void __launch_bounds__(kLossThreads, OP == kOpKL ? 3 : 0)
+__global__ void __launch_bounds__(kLossThreads, OP == kOpKL || OP == kOpKLTV ? 3 : 0)
 loss_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* __restrict__ targets,
                 const uint8_t* __restrict__ active, const uint8_t* __restrict__ also, const int64_t* __restrict__ labels,
                 float* __restrict__ loss, float* __restrict__ stats, int* __restrict__ argmax_d,
                 int* __restrict__ argmax_t, int rows, int V, int64_t ld_logits, int64_t ld_targets,
-                int shift, const int* __restrict__ target_row) {
+                int shift, const int* __restrict__ target_row, float* __restrict__ tv) {
   pdl_begin();
+  constexpr bool KL = OP == kOpKL || OP == kOpKLTV;
   __shared__ Meeting at;
   const int r = blockIdx.x;
   if (r >= rows) return;
@@ -174,6 +176,7 @@ loss_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* _
   if (tr < 0 || (active && !active[r] && !(also && also[r]))) {
     if (threadIdx.x == 0) {
       loss[r] = 0.f;
+      if (OP == kOpKLTV) tv[r] = 0.f;
 #pragma unroll
       for (int k = 0; k < kNumStats; ++k) st[(int64_t)k * rows] = 0.f;
       if (argmax_d) argmax_d[r] = -1;
@@ -189,16 +192,16 @@ loss_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* _
   const int nvec = vec_ok ? (V >> 3) : 0;
 
   Share sd, stt;
-  float kl_a = 0.f;  // OP == kOpKL: the cross term, accumulated in the same pass
+  float kl_a = 0.f;  // KL: the cross term, accumulated in the same pass
   auto take = [&](const bf16x8& a, const bf16x8& b, int v) {
     add8(sd, a, v << 3);
     if (has_t) {
-      if (OP == kOpKL) add8_kl(stt, kl_a, b, a, v << 3);
+      if (KL) add8_kl(stt, kl_a, b, a, v << 3);
       else add8(stt, b, v << 3);
     }
   };
   int v = threadIdx.x;
-  if constexpr (OP == kOpKL) {
+  if constexpr (KL) {
     for (; v < nvec; v += kLossThreads) {
       const bf16x8 a0 = ld8(x + (v << 3));
       take(a0, has_t ? ld8(t + (v << 3)) : a0, v);
@@ -223,7 +226,7 @@ loss_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* _
     const float xc = __bfloat162float(x[c]);
     add1(sd, xc, c);
     if (has_t) {
-      if (OP == kOpKL) add1_kl(stt, kl_a, __bfloat162float(t[c]), xc, c);
+      if (KL) add1_kl(stt, kl_a, __bfloat162float(t[c]), xc, c);
       else add1(stt, __bfloat162float(t[c]), c);
     }
   }
@@ -253,18 +256,19 @@ loss_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* _
       const int c = best_of_target();  // none in a row of nothing but -inf or NaN
       acc0 = c < V ? lse_d - __bfloat162float(x[c]) : __int_as_float(0x7fffffff);
     }
-  } else if (OP == kOpKL) {
+  } else if (KL) {
     // sum_v p_v (t_v - x_v) = (sum over threads of A rescaled to the row max) / Z_t; thread 0 adds
     // the normaliser terms once so that the block sum below yields the row's KL directly
     acc0 = (my_mt == -INFINITY) ? 0.f : kl_a * __expf(my_mt - stt.m) / stt.z;
     if (threadIdx.x == 0) acc0 += lse_d - lse_t;
-  } else {
+  }
+  if (OP != kOpCE && OP != kOpKL) {
+    float acc0b = 0.f;
+    float& acc = OP == kOpKLTV ? acc0b : acc0;
     auto body = [&](float xv, float tv) {
       const float ldp = xv - lse_d, ltp = tv - lse_t;
       const float dp = __expf(ldp), tp = __expf(ltp);
-      if (OP == kOpKL) {
-        if (tp > 0.f) acc0 += tp * (ltp - ldp);
-      } else if (OP == kOpRKL) {
+      if (OP == kOpRKL) {
         if (dp > 0.f) acc0 += dp * (ldp - ltp);
       } else if (OP == kOpJSD) {
         const float mx = fmaxf(ldp, ltp);
@@ -272,8 +276,8 @@ loss_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* _
         if (tp > 0.f) acc0 += tp * (ltp - lm);
         if (dp > 0.f) acc1 += dp * (ldp - lm);
       } else {  // TV
-        acc0 += fminf(dp, tp);
-        if (dp <= tp) acc1 += dp;
+        acc += fminf(dp, tp);
+        if (OP == kOpTV && dp <= tp) acc1 += dp;
       }
     };
     for (int v = threadIdx.x; v < nvec; v += kLossThreads) {
@@ -285,13 +289,14 @@ loss_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* _
     }
     for (int c = (nvec << 3) + threadIdx.x; c < V; c += kLossThreads)
       body(__bfloat162float(x[c]), __bfloat162float(t[c]));
+    if (OP == kOpKLTV) acc1 = acc0b;
   }
   if (OP != kOpCE) acc0 = block_sum_in(acc0, at.acc[0]);
-  if (OP == kOpJSD || OP == kOpTV) acc1 = block_sum_in(acc1, at.acc[1]);
+  if (OP == kOpJSD || OP == kOpTV || OP == kOpKLTV) acc1 = block_sum_in(acc1, at.acc[1]);
   if (threadIdx.x == 0) {
     float L, extra;
     const int best_t = OP == kOpCE || argmax_t ? best_of_target() : 0;
-    if (OP == kOpKL || OP == kOpRKL) {
+    if (KL || OP == kOpRKL) {
       L = acc0;
       extra = acc0;
     } else if (OP == kOpJSD) {
@@ -305,6 +310,7 @@ loss_fwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* _
       extra = acc1;
     }
     loss[r] = L;
+    if (OP == kOpKLTV) tv[r] = 1.f - acc1;
     st[0] = sd.m;
     st[(int64_t)rows] = sd.z;
     st[(int64_t)2 * rows] = stt.m;
@@ -380,23 +386,29 @@ loss_bwd_kernel(const __nv_bfloat16* __restrict__ logits, const __nv_bfloat16* _
 }
 
 // active / also (optional): rows marked in neither are skipped.  target_row (optional): the row of `targets` that each row is
-// compared with, instead of its own + shift; rows with a negative one are skipped.
+// compared with, instead of its own + shift; rows with a negative one are skipped.  tv (optional, with the KL divergence): the rows'
+// total variation, 0 where skipped.
 int launch_loss_fwd(int op, const void* logits, const void* targets, const uint8_t* active, const uint8_t* also,
                     const int64_t* labels, float* loss, float* stats, int* argmax_d, int* argmax_t, int rows, int V,
-                    int64_t ld_logits, int64_t ld_targets, int shift, const int* target_row, cudaStream_t stream) {
+                    int64_t ld_logits, int64_t ld_targets, int shift, const int* target_row, float* tv, cudaStream_t stream) {
   if (rows <= 0) return 0;
+  if (tv != nullptr) {
+    if (op != kOpKL || targets == nullptr) return -4;
+    op = kOpKLTV;
+  }
   if (targets == nullptr && (labels == nullptr || op != kOpCE)) return -3;
   count_launch(1);
 #define SB200_LF(OPV)                                                                            \
   launch_pdl(loss_fwd_kernel<OPV>, rows, kLossThreads, 0, stream,                                         \
       (const __nv_bfloat16*)logits, (const __nv_bfloat16*)targets, active, also, labels, loss, stats,   \
-      argmax_d, argmax_t, rows, V, ld_logits, ld_targets, shift, target_row)
+      argmax_d, argmax_t, rows, V, ld_logits, ld_targets, shift, target_row, tv)
   switch (op) {
     case kOpKL: SB200_LF(kOpKL); break;
     case kOpRKL: SB200_LF(kOpRKL); break;
     case kOpJSD: SB200_LF(kOpJSD); break;
     case kOpCE: SB200_LF(kOpCE); break;
     case kOpTV: SB200_LF(kOpTV); break;
+    case kOpKLTV: SB200_LF(kOpKLTV); break;
     default: return -1;
   }
 #undef SB200_LF

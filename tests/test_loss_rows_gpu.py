@@ -67,6 +67,23 @@ def test_infinite_logits_of_improbable_tokens(op):
     _check(op, x, t)
 
 
+@pytest.mark.parametrize("V", [7, 512, 4104, 32000])
+def test_divergence_and_variation_of_listed_target_rows_in_one_pass(V):
+    g = torch.Generator(device="cuda").manual_seed(V)
+    x, t = (torch.randn(n, V, generator=g, device="cuda").bfloat16().mul_(3) for n in (33, 9))
+    to = torch.randint(0, 9, (33,), generator=g, device="cuda", dtype=torch.int32)
+    active = torch.rand(33, generator=g, device="cuda") < 0.7
+    x.requires_grad_(True)
+    loss, am_d, am_t, tv = ops.fused_row_loss("kl_div", x, t, active=active, target_row=to, with_tv=True)
+    loss.sum().backward()
+    got, x.grad = x.grad, None
+    rows = t[to.long()]
+    want, want_d, want_t = ops.fused_row_loss("kl_div", x, rows, active=active)  # the same sums in the same order
+    want.sum().backward()
+    assert torch.equal(loss, want) and torch.equal(am_d, want_d) and torch.equal(am_t, want_t) and torch.equal(got, x.grad)
+    assert torch.equal(tv, ops.fused_row_loss("tv", x.detach(), rows, active=active)[0]) and not tv.requires_grad
+
+
 def test_the_first_of_equal_maxima():
     x = torch.zeros(4, 4100, device="cuda", dtype=torch.bfloat16)
     t = x.clone()
