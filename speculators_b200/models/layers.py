@@ -93,6 +93,13 @@ class RMSNorm(nn.Module):
         """``(self(x), x)``: the input of a pre-norm block and its residual branch."""
         return ops.rms_norm_fork(x, self.weight, self.variance_epsilon, live=live)
 
+    def of_sum(self, x: torch.Tensor, add: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
+        """``(x + add, self(x + add))``: a block's result, its residual added, and the next block's input."""
+        if type(self) is not RMSNorm or not unobserved(self):
+            x = x + add
+            return x, self(x)
+        return ops.add_rms_norm(x, add, self.weight, self.variance_epsilon)
+
     def extra_repr(self) -> str:
         return f"{tuple(self.weight.shape)}, eps={self.variance_epsilon}"
 
@@ -295,7 +302,8 @@ class Attention(nn.Module):
                                        rotary.sin, (self.nh, self.nkv, self.nkv), self.hd, self.rot, split, repeated, live)
         if repeated:
             qkv = ops.repeat_rows(qkv, T)
-        q, k, v = ops.rope_split(qkv, positions, rotary.cos, rotary.sin, self.nh + self.nkv, self.hd, self.rot, nq, nk, live)
+        q, k, v = ops.rope_split(qkv, positions, rotary.cos, rotary.sin, self.nh + self.nkv, self.hd, self.rot, nq, nk, live,
+                                 unseen=not torch.is_grad_enabled() and unobserved(self.qkv_proj))
         q, k, v = q.view(T, self.nh, self.hd), k.view(T, self.nkv, self.hd), v.view(T, self.nkv, self.hd)
         return (q, k, v) if split is None else (q, k[:split], k[split:], v[:split], v[split:])
 

@@ -672,6 +672,16 @@ def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float, centred: bool = 
     return _rms_norm_ref(x, weight, eps, centred)
 
 
+def add_rms_norm(x: torch.Tensor, add: torch.Tensor, weight: torch.Tensor, eps: float) -> tuple[torch.Tensor, torch.Tensor]:
+    """``(x + add, rms_norm(x + add))``, in one launch where no gradient is asked for."""
+    if (_norm_native(x) and not torch.is_grad_enabled() and x.dim() == 2 and x.shape[1] > 256 and add.shape == x.shape and add.dtype == x.dtype
+            and weight.dtype == x.dtype and all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (x, add, weight))
+            and torch.autograd.forward_ad._current_level < 0):
+        return native().add_rmsnorm_fwd(x, add, weight, eps)
+    x = x + add
+    return x, rms_norm(x, weight, eps)
+
+
 def rms_norm_fork(x: torch.Tensor, weight: torch.Tensor, eps: float, centred: bool = False,
                   live: torch.Tensor | None = None) -> tuple[torch.Tensor, torch.Tensor]:
     """``(rms_norm(x), x)`` for a pre-norm block: the second result is the residual branch."""
@@ -1143,13 +1153,19 @@ def gated(out: torch.Tensor, gate: torch.Tensor, live: torch.Tensor | None = Non
     return _GatedFn.apply(out.contiguous(), gate, live)
 
 
-def rope_split(qkv, positions, cos_t, sin_t, heads: int, hd: int, rot: int, nq: int, nk: int, live: torch.Tensor | None = None):
+def rope_split(qkv, positions, cos_t, sin_t, heads: int, hd: int, rot: int, nq: int, nk: int, live: torch.Tensor | None = None,
+               unseen: bool = False):
     """``rope_`` on the first ``heads`` heads of ``qkv`` ([T, nq + nk + nv]) followed by
     the split into ``(q [T, nq], k [T, nk], v [T, rest])``.  On CUDA the buffer is
     rotated in place and the results are views of it: the caller must own ``qkv``
-    (a fresh projection output) and must not modify the views in place."""
+    (a fresh projection output) and must not modify the views in place.  ``unseen``: nobody else holds it either, so that it is
+    rotated in place without a gradient too (else a view is copied first)."""
     if _use_native(qkv) and qkv.requires_grad and torch.is_grad_enabled():
         return _RopeSplitFn.apply(qkv, positions, cos_t, sin_t, heads, hd, rot, nq, nk, live)
+    if unseen and _use_native(qkv) and not torch.is_grad_enabled() and qkv.dim() == 2 and qkv.stride(-1) == 1 and torch.autograd.forward_ad._current_level < 0:
+        out = qkv.detach()  # (``rope_`` would work on a copy of a view)
+        native().rope_(out, positions, cos_t, sin_t, heads, hd, rot, 1.0, live)
+        return out[:, :nq], out[:, nq : nq + nk], out[:, nq + nk :]
     out = rope_(qkv, positions, cos_t, sin_t, heads, hd, rot)
     return out[:, :nq], out[:, nq : nq + nk], out[:, nq + nk :]
 

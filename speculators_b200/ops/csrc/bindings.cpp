@@ -15,6 +15,7 @@
 
 namespace sb200 {
 int rmsnorm_bwd_partial_rows(int rows, int H, bool with_dx);
+void launch_add_rmsnorm_fwd(const void*, const void*, const void*, void*, void*, int, int, float, cudaStream_t);
 void launch_rmsnorm_fwd(const void*, const void*, const int64_t*, void*, float*, int, int, int64_t,
                         int64_t, float, int64_t, int, const int*, cudaStream_t);
 struct BoundsRecord {
@@ -228,6 +229,19 @@ void norm_fwd(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& row
   c10::cuda::CUDAGuard guard(x.device());
   sb200::launch_rmsnorm_fwd(x.data_ptr(), w.data_ptr(), idx, y.data_ptr(), rs, rows, H, x.stride(0),
                             y.stride(0), (float)eps, x.size(0), centred ? 1 : 0, used_rows(live), cur_stream());
+}
+// -> (x + add, its norm); contiguous bf16 [rows, H]
+std::tuple<Tensor, Tensor> add_rmsnorm_fwd(const Tensor& x, const Tensor& add, const Tensor& w, double eps) {
+  for (const Tensor* t : std::initializer_list<const Tensor*>{&x, &add})
+    TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kBFloat16 && t->dim() == 2 && t->is_contiguous() && (reinterpret_cast<uintptr_t>(t->data_ptr()) & 15) == 0,
+                "add_rmsnorm_fwd: contiguous bf16 [rows, H] expected");
+  const int64_t H = x.size(1);
+  TORCH_CHECK(add.sizes() == x.sizes() && H % 8 == 0 && H > 256 && H <= 32768, "add_rmsnorm_fwd: shapes");
+  TORCH_CHECK(w.is_cuda() && w.scalar_type() == at::kBFloat16 && w.is_contiguous() && w.numel() == H && (reinterpret_cast<uintptr_t>(w.data_ptr()) & 15) == 0);
+  c10::cuda::CUDAGuard guard(x.device());
+  Tensor sum = at::empty_like(x), y = at::empty_like(x);
+  sb200::launch_add_rmsnorm_fwd(x.data_ptr(), add.data_ptr(), w.data_ptr(), sum.data_ptr(), y.data_ptr(), (int)x.size(0), (int)H, (float)eps, cur_stream());
+  return {sum, y};
 }
 void rmsnorm_fwd(const Tensor& x, const Tensor& w, const c10::optional<Tensor>& row_index, Tensor y, c10::optional<Tensor> rstd, double eps,
                  const c10::optional<Tensor>& live) {
@@ -1541,6 +1555,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> attn_bwd(
 
 TORCH_LIBRARY(sb200, m) {
   // a trailing `live` (int32[1] on the device): how many of the rows are in use
+  m.def("add_rmsnorm_fwd", &add_rmsnorm_fwd);
   m.def("rmsnorm_fwd(Tensor x, Tensor w, Tensor? row_index, Tensor y, Tensor? rstd, float eps, Tensor? live=None) -> ()", &rmsnorm_fwd);
   m.def("norm_fwd(Tensor x, Tensor w, Tensor? row_index, Tensor y, Tensor? rstd, float eps, bool centred, Tensor? live=None) -> ()", &norm_fwd);
   m.def("rmsnorm_bwd(Tensor dy, Tensor? dy2, Tensor x, Tensor w, Tensor rstd, Tensor? add, Tensor? dx, Tensor? dw, bool accumulate_dw, bool centred, "

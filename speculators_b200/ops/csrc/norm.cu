@@ -61,19 +61,25 @@ __device__ __forceinline__ float row_sum(float v, float (&scratch)[2][THREADS / 
 // and evens out how many rows its blocks walk.
 template <int NV, int THREADS> constexpr int kFwdBlocks = THREADS == 512 ? 1 : NV == 2 ? 5 : NV == 4 ? 4 : 2;
 
-template <int NV, int THREADS>
+// ADD: the row is x + add, rounded as a sum of its own would be, kept in `sum` and normalised from registers: a block of a decoder
+// hands its result to the next norm without reading it back, and a launch less (1777 x 4096: 8 + 10 us apart).
+struct NormAdd {
+  const __nv_bfloat16* add;
+  __nv_bfloat16* sum;
+};
+template <int NV, int THREADS, bool ADD = false>
 __global__ void __launch_bounds__(THREADS, kFwdBlocks<NV, THREADS>)
 rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                    const int64_t* __restrict__ row_index, __nv_bfloat16* __restrict__ y,
                    float* __restrict__ rstd_out, int rows, int H, int64_t x_stride,
-                   int64_t y_stride, float eps, int64_t src_rows, NormWeight nw, const int* __restrict__ live) {
+                   int64_t y_stride, float eps, int64_t src_rows, NormWeight nw, const int* __restrict__ live, const NormAdd ad) {
   pdl_begin();
   rows = live_rows(live, rows);
   __shared__ float scratch[2][THREADS / 32];
   const int nvec = H >> 3;
-  bf16x8 cur[NV], next[NV];
+  bf16x8 cur[NV], next[NV], cur_add[ADD ? NV : 1], next_add[ADD ? NV : 1];
   bool ok = false, next_ok = false;  // false only in the debug build
-  auto fetch = [&](int r, bf16x8 (&to)[NV]) -> bool {
+  auto fetch = [&](int r, bf16x8 (&to)[NV], bf16x8 (&to_add)[ADD ? NV : 1]) -> bool {
     const int64_t src = row_index ? row_index[r] : (int64_t)r;
     if (!SB200_IN_RANGE(src, src_rows, 1)) return false;
     const __nv_bfloat16* xr = x + src * x_stride;
@@ -81,13 +87,30 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
     for (int i = 0; i < NV; ++i) {
       const int v = threadIdx.x + i * THREADS;
       if (v < nvec) to[i] = ld8(xr + (v << 3));
+      if (ADD && v < nvec) to_add[ADD ? i : 0] = ld8(ad.add + (int64_t)r * H + (v << 3));
     }
     return true;
   };
   int r = blockIdx.x, slot = 0;
-  if (r < rows) ok = fetch(r, cur);
+  if (r < rows) ok = fetch(r, cur, cur_add);
   for (; r < rows; r += gridDim.x, slot ^= 1) {
-    if (r + (int)gridDim.x < rows) next_ok = fetch(r + gridDim.x, next);  // in flight during this row's reduction
+    if (r + (int)gridDim.x < rows) next_ok = fetch(r + gridDim.x, next, next_add);  // in flight during this row's reduction
+    if (ADD) {
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const int v = threadIdx.x + i * THREADS;
+        if (v < nvec) {
+          float a[8], b[8];
+          unpack8(cur[i], a);
+          unpack8(cur_add[ADD ? i : 0], b);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) a[j] += b[j];
+          cur[i] = pack8(a);
+          st8(ad.sum + (int64_t)r * H + (v << 3), cur[i]);
+        }
+        cur_add[ADD ? i : 0] = next_add[ADD ? i : 0];
+      }
+    }
     float ss = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
@@ -734,6 +757,27 @@ SB200_BOUNDS_READER(read_bounds_norm)
 
 // src_rows: number of rows of `x` (what `row_index` may address).
 // live (optional, device): how many of the rows are in use.
+static int norm_fwd_grid(int rows, int H, int blocks) {
+  if (H <= 4096 && rows <= 16 * kNumSM) return rows;
+  const int most = blocks * kNumSM, rounds = (rows + most - 1) / most;
+  return (rows + rounds - 1) / rounds;
+}
+
+// sum = x + add, y = norm(sum); dense rows of H elements (above kNarrowMaxH, a multiple of 8)
+void launch_add_rmsnorm_fwd(const void* x, const void* add, const void* w, void* sum, void* y, int rows, int H, float eps, cudaStream_t stream) {
+  if (rows <= 0) return;
+  count_launch(1);
+#define SB200_ADD(NVV, THREADS)                                                                                                                   \
+  launch_pdl(rmsnorm_fwd_kernel<NVV, THREADS, true>, norm_fwd_grid(rows, H, kFwdBlocks<NVV, THREADS>), THREADS, 0, stream, (const __nv_bfloat16*)x, \
+             (const __nv_bfloat16*)w, (const int64_t*)nullptr, (__nv_bfloat16*)y, (float*)nullptr, rows, H, (int64_t)H, (int64_t)H, eps, (int64_t)rows, \
+             NormWeight{false}, (const int*)nullptr, NormAdd{(const __nv_bfloat16*)add, (__nv_bfloat16*)sum})
+  if (H <= 4096) SB200_ADD(2, 256);
+  else if (H <= 8192) SB200_ADD(4, 256);
+  else if (H <= 16384) SB200_ADD(8, 256);
+  else SB200_ADD(8, 512);
+#undef SB200_ADD
+}
+
 void launch_rmsnorm_fwd(const void* x, const void* w, const int64_t* row_index, void* y,
                         float* rstd, int rows, int H, int64_t x_stride, int64_t y_stride, float eps,
                         int64_t src_rows, int centred, const int* live, cudaStream_t stream) {
@@ -751,14 +795,10 @@ void launch_rmsnorm_fwd(const void* x, const void* w, const int64_t* row_index, 
   // 4096 33.8 and 35.9).  From memory it is level or gains a tenth there (8192 x 2048 28.7 and 26.8, 2368 x 4096 18.4 and
   // 16.4) and 15 to 20 % on wide rows, where a block's loads are long (1536 x 24576 57 and 47, from L2 51 and 42).  The line
   // gives few narrow rows, which the step's kernels find in L2, a block each.
-  auto grid = [&](int blocks) {
-    if (H <= 4096 && rows <= 16 * kNumSM) return rows;
-    const int most = blocks * kNumSM, rounds = (rows + most - 1) / most;
-    return (rows + rounds - 1) / rounds;
-  };
+  auto grid = [&](int blocks) { return norm_fwd_grid(rows, H, blocks); };
 #define SB200_FWD(NVV, THREADS)                                                                                          \
   launch_pdl(rmsnorm_fwd_kernel<NVV, THREADS>, grid(kFwdBlocks<NVV, THREADS>), THREADS, 0, stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, row_index, \
-             (__nv_bfloat16*)y, rstd, rows, H, x_stride, y_stride, eps, src_rows, nw, live)
+             (__nv_bfloat16*)y, rstd, rows, H, x_stride, y_stride, eps, src_rows, nw, live, NormAdd{nullptr, nullptr})
   if (H <= 4096) SB200_FWD(2, 256);
   else if (H <= 8192) SB200_FWD(4, 256);
   else if (H <= 16384) SB200_FWD(8, 256);

@@ -243,7 +243,9 @@ class TensorParallelVerifier:
         shift = 1 if self.layers_counted else 0
         if self.layers_counted and 0 in layer_ids:
             taken[0] = h
-        for i in range(int(self.cfg.num_hidden_layers)):
+        layers = int(self.cfg.num_hidden_layers)
+        normed = None  # the layer's input behind its norm, where the layer before has formed it
+        for i in range(layers):
             layer = self._layer(i)
             if fused:
                 # o_proj / down_proj: product, sum over the ranks and residual add in two kernels; the result
@@ -251,8 +253,13 @@ class TensorParallelVerifier:
                 h = layer.self_attn(layer.input_layernorm(h), pos, self.rotary, spec, residual=h)
                 h = layer.mlp(layer.post_attention_layernorm(h), residual=h)
             else:
-                h = h + self._reduce(layer.self_attn(layer.input_layernorm(h), pos, self.rotary, spec))
-                h = h + self._reduce(layer.mlp(layer.post_attention_layernorm(h)))
+                attended = self._reduce(layer.self_attn(layer.input_layernorm(h) if normed is None else normed, pos, self.rotary, spec))
+                h, normed = layer.post_attention_layernorm.of_sum(h, attended)
+                out = self._reduce(layer.mlp(normed))
+                if self.resident and i + 1 < layers:  # (else one layer is held at a time)
+                    h, normed = self._layer(i + 1).input_layernorm.of_sum(h, out)
+                else:
+                    h, normed = h + out, None
             if i + shift in layer_ids:
                 taken[i + shift] = h.clone() if fused else h
             del layer

@@ -138,3 +138,12 @@ def test_weight_gradients_beside_the_backward_pass(rows, K, N):
     zf = zf @ wf.t() if N >= K else yf
     (zf.pow(2).mean() + (wf * 0.5).sum()).backward()
     assert (got - wf.grad).abs().max() <= 0.02 * wf.grad.abs().max()
+
+
+@pytest.mark.parametrize("rows,H", [(1, 264), (77, 1024), (2368, 4096), (2369, 4096), (3000, 4104), (900, 8192), (901, 12296), (700, 24576)])
+def test_a_sum_and_its_norm_in_one_launch_give_the_same_bits(rows, H):
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x, add, w = (torch.randn(*s, generator=g, device="cuda").bfloat16() for s in ((rows, H), (rows, H), (H,)))
+    with torch.no_grad():
+        total, normed = ops.add_rms_norm(x, add, w, 1e-6)
+        assert torch.equal(total, x + add) and torch.equal(normed, ops.rms_norm(x + add, w, 1e-6))
