@@ -27,6 +27,7 @@ from speculators_b200.ops import AttnSpec
 __all__ = [
     "Attention",
     "DecoderLayer",
+    "decoder_layer_fwd",
     "FusedLinear",
     "Linear",
     "MLP",
@@ -431,3 +432,31 @@ class DecoderLayer(nn.Module):
         x = self.self_attn(normed, positions, rotary, spec, past, ctx_len, residual=x, rows=rows, dense=dense)
         normed, x = self.post_attention_layernorm.fork(x, live)
         return self.mlp(normed, residual=x, live=live)
+
+
+def decoder_layer_fwd(layer: DecoderLayer, h: torch.Tensor, normed: torch.Tensor | None, next_norm: RMSNorm | None, positions, rotary: RotaryTable, spec):
+    """A decoder layer's result without a gradient, in one call of the extension: ``(h, next_norm(h) or None)``, or ``None`` where
+    its modules have to be called (other devices, types or activations, biases, a watched module).  ``normed``: the layer's input
+    behind its first norm, if the layer before has formed it.  The launches are those of the modules."""
+    from speculators_b200.ops import attention_cuda
+
+    attn, mlp = layer.self_attn, layer.mlp
+    if (not h.is_cuda or h.dtype != torch.bfloat16 or torch.is_grad_enabled() or torch.autograd.forward_ad._current_level >= 0
+            or type(layer) is not DecoderLayer or type(attn) is not Attention or type(mlp) is not MLP or not unobserved(layer)
+            or (next_norm is not None and not unobserved(next_norm)) or mlp.hidden_act not in ("silu", "swish")
+            or not ops.own_gemm_enabled() or not ops.fused_swiglu_enabled() or attention_cuda.FWD_IMPL != "tc"):
+        return None
+    qkv, o, gate_up, down = attn.qkv_proj, attn.o_proj, mlp.gate_up_proj, mlp.down_proj
+    if (any(m.bias is not None for m in (qkv, o, gate_up, down)) or o.row_parallel is not None or down.row_parallel is not None
+            or (attn.q_norm is None) != (attn.k_norm is None) or spec.extra_idx is not None):
+        return None
+    q_norm, k_norm = attn.q_norm, attn.k_norm
+    first, post = layer.input_layernorm, layer.post_attention_layernorm
+    out = ops.native().decoder_layer_fwd(
+        h, normed, first.weight, qkv.weight, None if q_norm is None else q_norm.weight, None if k_norm is None else k_norm.weight, o.weight, post.weight,
+        gate_up.weight, down.weight, None if next_norm is None else next_norm.weight, positions, rotary.cos, rotary.sin, spec.lo, spec.hi, attn.nh, attn.nkv,
+        attn.hd, attn.rot, first.variance_epsilon, 0.0 if q_norm is None else q_norm.variance_epsilon, post.variance_epsilon,
+        0.0 if next_norm is None else next_norm.variance_epsilon, attn.scaling, attention_cuda.tensor_core_shape(h.shape[0], attn.hd, None), ops.gemm_status(h.device))
+    if not out:
+        return None
+    return out[0], out[1] if next_norm is not None else None

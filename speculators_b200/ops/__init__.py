@@ -767,15 +767,19 @@ class _GateUpSwiGLUFn(torch.autograd.Function):
         return dx, dw, None, None
 
 
+def fused_swiglu_enabled() -> bool:
+    import os
+
+    return os.environ.get("SB200_FUSED_SWIGLU", "1") != "0"
+
+
 def linear_swiglu(x: torch.Tensor, weight: torch.Tensor, live: torch.Tensor | None = None) -> torch.Tensor | None:
     """``swiglu(linear(x, weight))`` for a stacked ``[gate; up]`` weight in one launch: the
     activation is formed in the GEMM's epilogue from the accumulator (``SB200_FUSED_SWIGLU=0``
     switches it off).  ``None`` when the operands do not suit the kernel (other dtype or device,
     intermediate size not a multiple of 128) and the caller should run the two steps."""
-    import os
-
     x2 = x.reshape(-1, x.shape[-1])
-    if (not own_gemm_enabled() or os.environ.get("SB200_FUSED_SWIGLU", "1") == "0" or not _gemm_operand_ok(x2) or not _gemm_operand_ok(weight)
+    if (not own_gemm_enabled() or not fused_swiglu_enabled() or not _gemm_operand_ok(x2) or not _gemm_operand_ok(weight)
             or weight.shape[0] % 256 or weight.shape[1] != x2.shape[1]):
         return None
     use = _note_use(weight, None, None) if weight.requires_grad and torch.is_grad_enabled() else None

@@ -33,14 +33,13 @@ def _rows_ok(t: torch.Tensor) -> torch.Tensor:
     return t.contiguous()
 
 
-def _tensor_core_shape(q: torch.Tensor, ext_idx: torch.Tensor | None) -> bool:
+def tensor_core_shape(rows: int, hd: int, ext_idx: torch.Tensor | None) -> bool:
     """Whether the tcgen05 kernels take the call: head dim 128; 256 without extra keys (its own kernels, whose shared memory
     is filled by 128 resident rows and leaves none to stage individually addressed extra keys in); 64 from 513 query rows on -
     up to there a head is a few key tiles, and setting up tensor memory costs what the products save (128 tokens, 4 heads:
     10 / 55 us forward / backward on mma.sync, 11 / 61 here; 512 tokens 15 / 61 and 15 / 68; 1001 tokens, 32 heads 42 / 117
     and 26 / 73; 8192 tokens 1189 / 3543 and 445 / 1479)."""
-    hd = q.shape[2]
-    return hd == 128 or (hd == 64 and q.shape[0] > 512) or (hd == 256 and ext_idx is None)
+    return hd == 128 or (hd == 64 and rows > 512) or (hd == 256 and ext_idx is None)
 
 
 class _MaskedAttentionFn(torch.autograd.Function):
@@ -49,7 +48,7 @@ class _MaskedAttentionFn(torch.autograd.Function):
         q, k, v = _rows_ok(q), _rows_ok(k), _rows_ok(v)
         if ext_idx is not None:
             k_ext, v_ext = _rows_ok(k_ext), _rows_ok(v_ext)
-        tc_shape = _tensor_core_shape(q, ext_idx)
+        tc_shape = tensor_core_shape(q.shape[0], q.shape[2], ext_idx)
         tc_fwd, tc_bwd = FWD_IMPL == "tc" and tc_shape, BWD_IMPL == "tc" and tc_shape
         # block-structured extras run as one more key tile on the tensor cores; both directions must take
         # that route (or neither), since the forward's statistics feed the backward either way
@@ -69,7 +68,7 @@ class _MaskedAttentionFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout):
         q, k, v, out, lse2, lo, hi, k_ext, v_ext, ext_idx = ctx.saved_tensors
-        if BWD_IMPL == "tc" and _tensor_core_shape(q, ext_idx):
+        if BWD_IMPL == "tc" and tensor_core_shape(q.shape[0], q.shape[2], ext_idx):
             from speculators_b200.ops import gemm_status
 
             impl, status = 1, gemm_status(q.device)

@@ -1479,6 +1479,51 @@ std::tuple<Tensor, Tensor> attn_fwd_tc(const Tensor& q, const Tensor& k, const T
   return {out, lse2};
 }
 
+// A decoder layer's forward without a gradient: norm, projection, head norms and rotation, attention, projection, sum and norm,
+// gated MLP, sum (and the next layer's norm, given its weight).  Called one by one from Python its nine launches take 200 us of
+// the host, more than they take on the device up to some 1000 rows of a narrow decoder; from here about 40.
+// -> (result, its norm if w_next), or nothing where the operands are not what the kernels take (the caller's modules then do).
+std::vector<Tensor> decoder_layer_fwd(const Tensor& h, const c10::optional<Tensor>& normed, const Tensor& w_in, const Tensor& w_qkv, const c10::optional<Tensor>& w_q,
+                                      const c10::optional<Tensor>& w_k, const Tensor& w_o, const Tensor& w_post, const Tensor& w_gate_up, const Tensor& w_down,
+                                      const c10::optional<Tensor>& w_next, const Tensor& positions, const Tensor& cos_t, const Tensor& sin_t, const Tensor& lo,
+                                      const Tensor& hi, int64_t nh, int64_t nkv, int64_t hd, int64_t rot, double eps_in, double eps_heads, double eps_post,
+                                      double eps_next, double scale, bool tensor_cores, const Tensor& status) {
+  auto dense = [&](const Tensor& t, std::initializer_list<int64_t> shape) {
+    return t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.device() == h.device() && t.sizes() == c10::IntArrayRef(shape) && t.is_contiguous() &&
+           (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0;
+  };
+  if (h.dim() != 2 || w_down.dim() != 2 || nh <= 0 || nkv <= 0) return {};
+  const int64_t T = h.size(0), H = h.size(1), I = w_down.size(1), nq = nh * hd, nk = nkv * hd;
+  const bool heads = w_q.has_value();
+  if (T <= 0 || H % 8 || H <= 256 || H > 32768 || I % 128 || nh % nkv || (hd != 64 && hd != 128 && hd != 256) || rot > hd || rot % (heads ? 16 : 2)) return {};
+  if (!dense(h, {T, H}) || (normed.has_value() && !dense(*normed, {T, H})) || !dense(w_in, {H}) || !dense(w_qkv, {nq + 2 * nk, H}) || !dense(w_o, {H, nq}) ||
+      !dense(w_post, {H}) || !dense(w_gate_up, {2 * I, H}) || !dense(w_down, {H, I}) || (w_next.has_value() && !dense(*w_next, {H})))
+    return {};
+  if (heads && (!w_k.has_value() || !dense(*w_q, {hd}) || !dense(*w_k, {hd}))) return {};
+  if (positions.scalar_type() != at::kLong || !positions.is_contiguous() || positions.numel() != T) return {};
+  c10::cuda::CUDAGuard guard(h.device());
+  const c10::optional<Tensor> none;
+  auto product = [&](const Tensor& x, const Tensor& w) {
+    Tensor out = at::empty({T, w.size(0)}, h.options());
+    gemm_tn(x, w, out, none, 0, status, none);
+    return out;
+  };
+  Tensor x;
+  if (normed.has_value()) x = *normed;
+  else norm_fwd(h, w_in, none, x = at::empty_like(h), none, eps_in, false, none);
+  const Tensor qkv = product(x, w_qkv);
+  Tensor qk = qkv;
+  if (heads) qk = std::get<0>(heads_fwd(qkv, w_q, nh, w_k, nkv, eps_heads, positions, cos_t, sin_t, hd, rot, false, none));
+  else rope_(qkv, positions, cos_t, sin_t, nh + nkv, hd, rot, 1.0, none);
+  const Tensor q = qk.narrow(1, 0, nq).unflatten(1, {nh, hd}), k = qk.narrow(1, nq, nk).unflatten(1, {nkv, hd}), v = qkv.narrow(1, nq + nk, nk).unflatten(1, {nkv, hd});
+  Tensor out = std::get<0>(tensor_cores ? attn_fwd_tc(q, k, v, lo, hi, none, none, none, scale, status, 0, false) : attn_fwd(q, k, v, lo, hi, none, none, none, scale));
+  auto [mid, mid_normed] = add_rmsnorm_fwd(h, product(out.view({T, nq}), w_o), w_post, eps_post);
+  const Tensor down = product(std::get<1>(gemm_swiglu(mid_normed, w_gate_up, status, none)), w_down);
+  if (!w_next.has_value()) return {mid + down};
+  auto [next, next_normed] = add_rmsnorm_fwd(mid, down, *w_next, eps_next);
+  return {next, next_normed};
+}
+
 std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> attn_bwd(
     const Tensor& dout, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& out, const Tensor& lse2,
     const Tensor& lo, const Tensor& hi, const c10::optional<Tensor>& ke, const c10::optional<Tensor>& ve,
@@ -1556,6 +1601,9 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> attn_bwd(
 TORCH_LIBRARY(sb200, m) {
   // a trailing `live` (int32[1] on the device): how many of the rows are in use
   m.def("add_rmsnorm_fwd", &add_rmsnorm_fwd);
+  m.def("decoder_layer_fwd(Tensor h, Tensor? normed, Tensor w_in, Tensor w_qkv, Tensor? w_q, Tensor? w_k, Tensor w_o, Tensor w_post, Tensor w_gate_up, "
+        "Tensor w_down, Tensor? w_next, Tensor positions, Tensor cos_t, Tensor sin_t, Tensor lo, Tensor hi, int nh, int nkv, int hd, int rot, float eps_in, "
+        "float eps_heads, float eps_post, float eps_next, float scale, bool tensor_cores, Tensor status) -> Tensor[]", &decoder_layer_fwd);
   m.def("rmsnorm_fwd(Tensor x, Tensor w, Tensor? row_index, Tensor y, Tensor? rstd, float eps, Tensor? live=None) -> ()", &rmsnorm_fwd);
   m.def("norm_fwd(Tensor x, Tensor w, Tensor? row_index, Tensor y, Tensor? rstd, float eps, bool centred, Tensor? live=None) -> ()", &norm_fwd);
   m.def("rmsnorm_bwd(Tensor dy, Tensor? dy2, Tensor x, Tensor w, Tensor rstd, Tensor? add, Tensor? dx, Tensor? dw, bool accumulate_dw, bool centred, "

@@ -29,7 +29,7 @@ import torch.distributed as dist
 
 from speculators_b200.layer_config import TransformerLayerConfig
 from speculators_b200.models.eagle3.attention import causal_document_interval
-from speculators_b200.models.layers import DecoderLayer, RotaryTable
+from speculators_b200.models.layers import DecoderLayer, RotaryTable, decoder_layer_fwd
 from speculators_b200.ops import AttnSpec
 from speculators_b200.verifier.model import _seeded
 
@@ -247,7 +247,11 @@ class TensorParallelVerifier:
         normed = None  # the layer's input behind its norm, where the layer before has formed it
         for i in range(layers):
             layer = self._layer(i)
-            if fused:
+            after = self._layer(i + 1).input_layernorm if self.resident and not fused and i + 1 < layers else None  # (else one layer is held at a time)
+            whole = decoder_layer_fwd(layer, h, normed, after, pos, self.rotary, spec) if self.world == 1 and not fused else None
+            if whole is not None:
+                h, normed = whole
+            elif fused:
                 # o_proj / down_proj: product, sum over the ranks and residual add in two kernels; the result
                 # alternates between two peer buffers, so what is kept beyond the next call is copied
                 h = layer.self_attn(layer.input_layernorm(h), pos, self.rotary, spec, residual=h)
@@ -256,10 +260,7 @@ class TensorParallelVerifier:
                 attended = self._reduce(layer.self_attn(layer.input_layernorm(h) if normed is None else normed, pos, self.rotary, spec))
                 h, normed = layer.post_attention_layernorm.of_sum(h, attended)
                 out = self._reduce(layer.mlp(normed))
-                if self.resident and i + 1 < layers:  # (else one layer is held at a time)
-                    h, normed = self._layer(i + 1).input_layernorm.of_sum(h, out)
-                else:
-                    h, normed = h + out, None
+                h, normed = after.of_sum(h, out) if after is not None else (h + out, None)
             if i + shift in layer_ids:
                 taken[i + shift] = h.clone() if fused else h
             del layer

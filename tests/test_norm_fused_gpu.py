@@ -147,3 +147,28 @@ def test_a_sum_and_its_norm_in_one_launch_give_the_same_bits(rows, H):
     with torch.no_grad():
         total, normed = ops.add_rms_norm(x, add, w, 1e-6)
         assert torch.equal(total, x + add) and torch.equal(normed, ops.rms_norm(x + add, w, 1e-6))
+
+
+@pytest.mark.parametrize("family,hd", [("llama", 64), ("llama", 128), ("qwen3", 128), ("qwen3", 256)])
+@pytest.mark.parametrize("rows", [1, 100, 513, 2500])
+def test_a_decoder_layer_in_one_call_gives_the_bits_of_its_modules(family, hd, rows, monkeypatch):
+    from speculators_b200.verifier import tp
+
+    cfg = {"architectures": ["LlamaForCausalLM"], "model_type": family, "hidden_size": 512, "num_hidden_layers": 3, "num_attention_heads": 4,
+           "num_key_value_heads": 2, "head_dim": hd, "intermediate_size": 640, "vocab_size": 128, "rms_norm_eps": 1e-5, "rope_theta": 10000.0,
+           "max_position_embeddings": 4096, "hidden_act": "silu"}
+    verifier = tp.TensorParallelVerifier(cfg, seed=1, device="cuda", dtype=torch.bfloat16, resident=True)
+    ids, doc = torch.randint(0, 128, (1, rows), device="cuda"), (torch.arange(rows, device="cuda") // 400).unsqueeze(0)
+    taken = []
+    fwd = tp.decoder_layer_fwd
+    monkeypatch.setattr(tp, "decoder_layer_fwd", lambda *a: taken.append(fwd(*a)) or taken[-1])
+    got = verifier.forward(ids, [0, 2], doc)
+    assert len(taken) == 3 and all(t is not None for t in taken)
+    monkeypatch.setattr(tp, "decoder_layer_fwd", lambda *a: None)
+    want = verifier.forward(ids, [0, 2], doc)
+    assert all(torch.equal(got[k], want[k]) for k in want)
+    seen = []
+    verifier._layers[1].mlp.down_proj.register_forward_hook(lambda m, i, o: seen.append(o.shape))  # its layer's modules are called
+    monkeypatch.setattr(tp, "decoder_layer_fwd", fwd)
+    again = verifier.forward(ids, [0, 2], doc)
+    assert len(seen) == 1 and all(torch.equal(again[k], want[k]) for k in want)
