@@ -55,6 +55,7 @@ void launch_rope_merge(const void* const*, const int64_t*, const int*, const int
                        int, float, const int*, cudaStream_t);
 void launch_gate_mul_fwd(const void*, const void*, void*, int, int, int, int64_t, int, cudaStream_t);
 void launch_gate_mul_bwd(const void*, const void*, const void*, void*, void*, int, int, int, int64_t, int, int64_t, cudaStream_t);
+int launch_topk_rows(const float*, int, int, int, int64_t*, cudaStream_t);
 int moe_plan_blocks(int);
 int launch_moe_plan(const int64_t*, int, int, int, int*, int*, int*, int*, int*, const int*, int, cudaStream_t);
 void launch_moe_gather(const void*, int64_t, const int*, const int*, int, void*, int, int, cudaStream_t);
@@ -617,6 +618,15 @@ Tensor gate_mul_bwd(const Tensor& dy, const Tensor& out, const Tensor& gate, Ten
 
 // ---- mixture-of-experts row movement ---------------------------------------------------------------
 // expert int64[T, k] -> (seg int32[E + 1], 256-row tile prefix int32[E + 1], slot_row int32[T * k], row_slot int32[capacity]).
+// columns of the k largest of every row, descending, equal ones by column: fp32 [rows, E <= 1024] -> int64 [rows, k]
+Tensor topk_rows(const Tensor& p, int64_t k) {
+  TORCH_CHECK(p.is_cuda() && p.scalar_type() == at::kFloat && p.dim() == 2 && p.is_contiguous() && p.size(1) <= 1024 && k >= 1 && k <= p.size(1), "topk_rows");
+  c10::cuda::CUDAGuard guard(p.device());
+  Tensor index = at::empty({p.size(0), k}, p.options().dtype(at::kLong));
+  const int rc = sb200::launch_topk_rows(p.data_ptr<float>(), (int)p.size(0), (int)p.size(1), (int)k, index.data_ptr<int64_t>(), cur_stream());
+  TORCH_CHECK(rc == 0, "topk_rows launch failed (", rc, ")");
+  return index;
+}
 std::tuple<Tensor, Tensor, Tensor, Tensor> moe_plan(const Tensor& expert, int64_t E, int64_t capacity, int64_t k, const c10::optional<Tensor>& live) {
   TORCH_CHECK(k >= 1 && expert.numel() % k == 0, "moe_plan: k slots per token");
   TORCH_CHECK(expert.is_cuda() && expert.scalar_type() == at::kLong && expert.is_contiguous() && expert.numel() > 0);
@@ -1637,6 +1647,7 @@ TORCH_LIBRARY(sb200, m) {
   m.def("embedding_bwd", &embedding_bwd);
   m.def("gate_mul_fwd", &gate_mul_fwd);
   m.def("gate_mul_bwd", &gate_mul_bwd);
+  m.def("topk_rows", &topk_rows);
   m.def("moe_plan(Tensor expert, int E, int capacity, int k=1, Tensor? live=None) -> (Tensor, Tensor, Tensor, Tensor)", &moe_plan);
   m.def("moe_gather", &moe_gather);
   m.def("moe_gather_bwd(Tensor d_pad, Tensor slot_row, int k, Tensor? live=None) -> Tensor", &moe_gather_bwd);

@@ -23,6 +23,40 @@ constexpr int kThreads = 256;
 constexpr int kPlanThreads = 1024;
 constexpr int kMaxExperts = 1024;
 
+// The k largest of a row's values, descending, equal ones by index (NaN counts as the largest, as torch.topk has it).  A warp a
+// row, PER values a lane in registers as keys that order like the values; k rounds of a warp-wide maximum.  Bound by the rounds'
+// shuffles: 4092 rows of 256, 10 of them, 7 us; a top-k and its sort took 74.
+template <int PER>
+__global__ void __launch_bounds__(256) topk_rows_kernel(const float* __restrict__ p, int rows, int E, int k, int64_t* __restrict__ index) {
+  pdl_begin();
+  const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (r >= rows) return;
+  unsigned key[PER];
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    const int e = j * 32 + lane;
+    const unsigned b = e < E ? __float_as_uint(p[(int64_t)r * E + e]) : 0xffffffffu;  // (a place behind the row: the lowest key)
+    const bool nan = (b & 0x7fffffffu) > 0x7f800000u;
+    key[j] = e >= E ? 0u : nan ? 0xffffffffu : b > 0x80000000u ? ~b : b | 0x80000000u;  // (-0 equals 0)
+  }
+  for (int i = 0; i < k; ++i) {
+    unsigned best = 0;
+    int at = 0;
+#pragma unroll
+    for (int j = PER - 1; j >= 0; --j)
+      if (key[j] >= best) {  // the lowest of equal ones
+        best = key[j];
+        at = j * 32 + lane;
+      }
+    const unsigned top = __reduce_max_sync(0xffffffffu, best);
+    const int e = (int)__reduce_min_sync(0xffffffffu, best == top ? (unsigned)at : 0xffffffffu);
+#pragma unroll
+    for (int j = 0; j < PER; ++j)
+      if (j * 32 + lane == e) key[j] = 0u;
+    if (lane == 0) index[(int64_t)r * k + i] = e;
+  }
+}
+
 __global__ void __launch_bounds__(kPlanThreads)
 count_kernel(const int64_t* __restrict__ expert, int n_slots, int E, int* __restrict__ hist, const int* __restrict__ live, int k) {
   pdl_begin();
@@ -231,6 +265,18 @@ combine_bwd_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* 
 
 static int row_blocks(int rows) { return rows < 16 * kNumSM ? rows : 16 * kNumSM; }
 
+int launch_topk_rows(const float* p, int rows, int E, int k, int64_t* index, cudaStream_t stream) {
+  if (rows <= 0) return 0;
+  if (E < 1 || E > moe::kMaxExperts || k < 1 || k > E) return -1;
+  count_launch(1);
+  const int grid = (rows + 7) / 8;
+  if (E <= 64) launch_pdl(moe::topk_rows_kernel<2>, grid, 256, 0, stream, p, rows, E, k, index);
+  else if (E <= 128) launch_pdl(moe::topk_rows_kernel<4>, grid, 256, 0, stream, p, rows, E, k, index);
+  else if (E <= 256) launch_pdl(moe::topk_rows_kernel<8>, grid, 256, 0, stream, p, rows, E, k, index);
+  else if (E <= 512) launch_pdl(moe::topk_rows_kernel<16>, grid, 256, 0, stream, p, rows, E, k, index);
+  else launch_pdl(moe::topk_rows_kernel<32>, grid, 256, 0, stream, p, rows, E, k, index);
+  return 0;
+}
 int moe_plan_blocks(int n_slots) { return (n_slots + moe::kPlanThreads - 1) / moe::kPlanThreads; }
 
 // hist: int[moe_plan_blocks(n_slots) * E] scratch; k: slots per token

@@ -86,3 +86,17 @@ def test_merged_rotation_gradient_has_the_bits_of_the_separate_steps(hd, rot, st
     want = dq.contiguous().clone()
     nat.rope_(want, *args, nq, hd, rot, -1.0)
     assert torch.equal(nat.rope_merge(dq, None, None, False, *args, hd, rot, -1.0), want)
+
+
+@pytest.mark.parametrize("E", [1, 31, 64, 65, 256, 512, 1000])
+@pytest.mark.parametrize("ties", [False, True])
+def test_topk_rows(E, ties):
+    g = torch.Generator(device="cuda").manual_seed(E)
+    p = torch.randn(37, E, generator=g, device="cuda")
+    if ties:
+        p = (p * 2).round()
+        p[0], p[1, E // 2], p[2, 0] = 0.0, float("nan"), float("-inf")
+    for k in {1, min(E, 10), min(E, 32)}:
+        got = ops.native().topk_rows(p, k)
+        keyed = torch.where(p.isnan(), torch.full_like(p, float("inf")), p)
+        assert torch.equal(got, torch.sort(keyed, dim=-1, descending=True, stable=True).indices[:, :k])
