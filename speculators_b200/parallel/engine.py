@@ -951,7 +951,7 @@ def _newton_schulz_stack(x: torch.Tensor, y: torch.Tensor, steps: int) -> None:
     than two: ``G`` holds the squares of the singular values, and what bf16 leaves of the small ones does not survive a third.
 
     Narrow ones form ``b G + c G^2`` and ``a X + X P`` in the products' epilogues, rounded like the single-matrix form: the drafts
-    of several narrow layers (DSpark) amplify last bits of an update by what their loss gradient is worth, so they keep those.
+    of several narrow layers (DSpark) amplify the last bits of an update up to the size of their gradients, so they keep those bits.
 
     Relative error against the same polynomial in fp64, five steps, Gaussian entries and spread over two and four decades, sums rounded
     on their own and now: 2048 x 8192 0.018, 0.029, 0.048 and 0.009, 0.016, 0.025; 28672 x 4096 0.019, 0.024, 0.040 and
