@@ -34,6 +34,7 @@ __all__ = [
     "NEEDED_ROWS_FROM",
     "RMSNorm",
     "RotaryTable",
+    "norm_of_sum",
     "stops_at_count",
     "takes_listed_rows",
     "unobserved",
@@ -94,15 +95,17 @@ class RMSNorm(nn.Module):
         """``(self(x), x)``: the input of a pre-norm block and its residual branch."""
         return ops.rms_norm_fork(x, self.weight, self.variance_epsilon, live=live)
 
-    def of_sum(self, x: torch.Tensor, add: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
-        """``(x + add, self(x + add))``: a block's result, its residual added, and the next block's input."""
-        if type(self) is not RMSNorm or not unobserved(self):
-            x = x + add
-            return x, self(x)
-        return ops.add_rms_norm(x, add, self.weight, self.variance_epsilon)
-
     def extra_repr(self) -> str:
         return f"{tuple(self.weight.shape)}, eps={self.variance_epsilon}"
+
+
+def norm_of_sum(norm: nn.Module, x: torch.Tensor, add: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
+    """``(x + add, norm(x + add))``: a block's result, its residual added, and the next block's input; one launch for an ``RMSNorm``
+    that nobody watches, any other module is called."""
+    if type(norm) is RMSNorm and unobserved(norm):
+        return ops.add_rms_norm(x, add, norm.weight, norm.variance_epsilon)
+    x = x + add
+    return x, norm(x)
 
 
 def _init_linear_(weight: torch.Tensor, std: float = 0.02) -> None:

@@ -29,7 +29,7 @@ import torch.distributed as dist
 
 from speculators_b200.layer_config import TransformerLayerConfig
 from speculators_b200.models.eagle3.attention import causal_document_interval
-from speculators_b200.models.layers import DecoderLayer, RotaryTable, decoder_layer_fwd
+from speculators_b200.models.layers import DecoderLayer, RotaryTable, decoder_layer_fwd, norm_of_sum
 from speculators_b200.ops import AttnSpec
 from speculators_b200.verifier.model import _seeded
 
@@ -258,9 +258,9 @@ class TensorParallelVerifier:
                 h = layer.mlp(layer.post_attention_layernorm(h), residual=h)
             else:
                 attended = self._reduce(layer.self_attn(layer.input_layernorm(h) if normed is None else normed, pos, self.rotary, spec))
-                h, normed = layer.post_attention_layernorm.of_sum(h, attended)
+                h, normed = norm_of_sum(layer.post_attention_layernorm, h, attended)
                 out = self._reduce(layer.mlp(normed))
-                h, normed = after.of_sum(h, out) if after is not None else (h + out, None)
+                h, normed = norm_of_sum(after, h, out) if after is not None else (h + out, None)
             if i + shift in layer_ids:
                 taken[i + shift] = h.clone() if fused else h
             del layer

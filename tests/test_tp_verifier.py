@@ -3,6 +3,7 @@ all-reduced) must reproduce the single-device forward of the same seeded random 
 
 import os
 
+import pytest
 import torch
 import torch.distributed as dist
 import torch.multiprocessing as mp
@@ -131,3 +132,16 @@ def test_row_parallel_biases_are_refused(monkeypatch):
         TensorParallelVerifier(dict(CFG, attention_bias=True))
     with pytest.raises(ValueError, match="mlp_bias"):
         TensorParallelVerifier(dict(CFG, mlp_bias=True))
+
+
+@pytest.mark.parametrize("which", ["input_layernorm", "post_attention_layernorm"])
+def test_a_norm_of_another_class_is_called(which):
+    ids, doc, pos = _inputs()
+    verifier = TensorParallelVerifier(CFG, seed=3, resident=True)
+    want = verifier.forward(ids, [0, 2], document_ids=doc, position_ids=pos)
+    for layer in verifier._layers.values():
+        norm = torch.nn.RMSNorm(CFG["hidden_size"], eps=CFG["rms_norm_eps"])
+        norm.load_state_dict(getattr(layer, which).state_dict())
+        setattr(layer, which, norm)
+    got = verifier.forward(ids, [0, 2], document_ids=doc, position_ids=pos)
+    assert all(torch.allclose(got[k], want[k], atol=2e-5, rtol=1e-4) for k in want)
