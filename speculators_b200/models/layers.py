@@ -437,22 +437,33 @@ class DecoderLayer(nn.Module):
         return self.mlp(normed, residual=x, live=live)
 
 
+def _of_one_call(layer: nn.Module, next_norm: nn.Module | None) -> bool:
+    """Whether ``decoder_layer_fwd`` does what calling the modules does: every one of the class whose formula it has (other norms
+    have a ``weight`` and an epsilon, too), none watched, no bias, no exchange between ranks."""
+    if type(layer) is not DecoderLayer or not unobserved(layer) or (next_norm is not None and not unobserved(next_norm)):
+        return False
+    attn, mlp = layer.self_attn, layer.mlp
+    if type(attn) is not Attention or type(mlp) is not MLP or mlp.hidden_act not in ("silu", "swish"):
+        return False
+    heads = [attn.q_norm, attn.k_norm] if attn.q_norm is not None or attn.k_norm is not None else []
+    norms = [layer.input_layernorm, layer.post_attention_layernorm, *heads, *([] if next_norm is None else [next_norm])]
+    return (all(type(n) is RMSNorm for n in norms)
+            and all(type(m) is FusedLinear and m.bias is None for m in (attn.qkv_proj, mlp.gate_up_proj))
+            and all(type(m) is Linear and m.bias is None and m.row_parallel is None for m in (attn.o_proj, mlp.down_proj)))
+
+
 def decoder_layer_fwd(layer: DecoderLayer, h: torch.Tensor, normed: torch.Tensor | None, next_norm: RMSNorm | None, positions, rotary: RotaryTable, spec):
     """A decoder layer's result without a gradient, in one call of the extension: ``(h, next_norm(h) or None)``, or ``None`` where
     its modules have to be called (other devices, types or activations, biases, a watched module).  ``normed``: the layer's input
     behind its first norm, if the layer before has formed it.  The launches are those of the modules."""
     from speculators_b200.ops import attention_cuda
 
-    attn, mlp = layer.self_attn, layer.mlp
     if (not h.is_cuda or h.dtype != torch.bfloat16 or torch.is_grad_enabled() or torch.autograd.forward_ad._current_level >= 0
-            or type(layer) is not DecoderLayer or type(attn) is not Attention or type(mlp) is not MLP or not unobserved(layer)
-            or (next_norm is not None and not unobserved(next_norm)) or mlp.hidden_act not in ("silu", "swish")
-            or not ops.own_gemm_enabled() or not ops.fused_swiglu_enabled() or attention_cuda.FWD_IMPL != "tc"):
+            or spec.extra_idx is not None or not ops.own_gemm_enabled() or not ops.fused_swiglu_enabled() or attention_cuda.FWD_IMPL != "tc"
+            or not _of_one_call(layer, next_norm)):
         return None
+    attn, mlp = layer.self_attn, layer.mlp
     qkv, o, gate_up, down = attn.qkv_proj, attn.o_proj, mlp.gate_up_proj, mlp.down_proj
-    if (any(m.bias is not None for m in (qkv, o, gate_up, down)) or o.row_parallel is not None or down.row_parallel is not None
-            or (attn.q_norm is None) != (attn.k_norm is None) or spec.extra_idx is not None):
-        return None
     q_norm, k_norm = attn.q_norm, attn.k_norm
     first, post = layer.input_layernorm, layer.post_attention_layernorm
     out = ops.native().decoder_layer_fwd(

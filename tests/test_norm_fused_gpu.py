@@ -172,3 +172,21 @@ def test_a_decoder_layer_in_one_call_gives_the_bits_of_its_modules(family, hd, r
     monkeypatch.setattr(tp, "decoder_layer_fwd", fwd)
     again = verifier.forward(ids, [0, 2], doc)
     assert len(seen) == 1 and all(torch.equal(again[k], want[k]) for k in want)
+
+
+@pytest.mark.parametrize("which", ["input_layernorm", "post_attention_layernorm"])
+def test_a_layer_with_a_centred_norm_is_not_one_call_of_the_plain_one(which, monkeypatch):
+    from speculators_b200.models.moe import ZeroCenteredRMSNorm
+    from speculators_b200.verifier import tp
+
+    cfg = {"architectures": ["LlamaForCausalLM"], "model_type": "llama", "hidden_size": 512, "num_hidden_layers": 3, "num_attention_heads": 4,
+           "num_key_value_heads": 2, "head_dim": 128, "intermediate_size": 640, "vocab_size": 128, "rms_norm_eps": 1e-5, "rope_theta": 10000.0,
+           "max_position_embeddings": 4096, "hidden_act": "silu"}
+    verifier = tp.TensorParallelVerifier(cfg, seed=1, device="cuda", dtype=torch.bfloat16, resident=True)
+    ids = torch.randint(0, 128, (1, 100), device="cuda")
+    verifier.forward(ids, [0])
+    setattr(verifier._layers[1], which, ZeroCenteredRMSNorm(512).to("cuda", torch.bfloat16))
+    got = verifier.forward(ids, [0, 1, 2])
+    monkeypatch.setattr(tp, "decoder_layer_fwd", lambda *a: None)
+    want = verifier.forward(ids, [0, 1, 2])
+    assert all(torch.equal(got[k], want[k]) for k in want)

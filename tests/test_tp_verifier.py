@@ -8,6 +8,7 @@ import torch
 import torch.distributed as dist
 import torch.multiprocessing as mp
 
+from speculators_b200.layer_config import TransformerLayerConfig
 from speculators_b200.verifier import RandomVerifier, TensorParallelVerifier
 
 CFG = dict(architectures=["Qwen3ForCausalLM"], model_type="qwen3", hidden_size=64, intermediate_size=96, num_hidden_layers=3,
@@ -145,3 +146,21 @@ def test_a_norm_of_another_class_is_called(which):
         setattr(layer, which, norm)
     got = verifier.forward(ids, [0, 2], document_ids=doc, position_ids=pos)
     assert all(torch.allclose(got[k], want[k], atol=2e-5, rtol=1e-4) for k in want)
+
+
+def test_only_layers_of_plain_modules_are_one_call():
+    from speculators_b200.models import layers
+    from speculators_b200.models.moe import ZeroCenteredRMSNorm
+
+    def fresh(**changes):
+        return layers.DecoderLayer(TransformerLayerConfig(**{**CFG, **changes}), 0)
+
+    assert layers._of_one_call(fresh(), None) and layers._of_one_call(fresh(model_type="llama"), fresh().input_layernorm)
+    assert not layers._of_one_call(fresh(hidden_act="gelu"), None) and not layers._of_one_call(fresh(mlp_bias=True), None)
+    for path in ("input_layernorm", "post_attention_layernorm", "self_attn.q_norm", "self_attn.k_norm"):
+        layer = fresh()
+        parent, name = layer.get_submodule(path.rpartition(".")[0]), path.rpartition(".")[2]
+        setattr(parent, name, ZeroCenteredRMSNorm(getattr(parent, name).weight.numel()))
+        assert not layers._of_one_call(layer, None), path
+    assert not layers._of_one_call(fresh(), ZeroCenteredRMSNorm(CFG["hidden_size"]))
+    assert not layers._of_one_call(fresh(), torch.nn.RMSNorm(CFG["hidden_size"]))
