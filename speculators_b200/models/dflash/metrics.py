@@ -11,7 +11,7 @@ from speculators_b200.losses import LossConfig, dflash_loss_decay, dpace_loss_de
 from speculators_b200.losses.rowwise import rowwise_terms
 from speculators_b200.models.metrics import compute_accuracy_multi_step
 
-__all__ = ["block_decay_fn", "compute_metrics", "weighted_terms"]
+__all__ = ["block_decay_fn", "compute_metrics", "target_rows", "weighted_terms"]
 
 
 def block_decay_fn(per_position_loss_weight: str, loss_mask, block_size: int, gamma: float, dpace_alpha: float, sample_from_anchor: bool):
@@ -20,12 +20,17 @@ def block_decay_fn(per_position_loss_weight: str, loss_mask, block_size: int, ga
     return partial(dflash_loss_decay, gamma=gamma, sample_from_anchor=sample_from_anchor)
 
 
+def target_rows(targets, n: int, target_row):
+    """``[rows, V]``: those of the ``n`` slots, or of the packed sequence if ``target_row`` lists what the slots are compared with."""
+    return targets.reshape(n if target_row is None else targets.shape[-2], -1)
+
+
 def weighted_terms(loss_config: LossConfig, logits, targets, loss_mask, pos_idx, decay_fn, target_row=None, tv_out: list | None = None):
     """-> (loss, {term scalars}, pred_ids, target_ids).  Rows without a loss are skipped: they weigh nothing in a sum or counter.
     ``target_row``, ``tv_out`` as in ``rowwise_terms``."""
     n = logits.shape[1]
     per_term, pred_ids, target_ids = rowwise_terms(
-        loss_config, logits.reshape(n, -1), targets.reshape(targets.shape[1], -1), shift=0, rows=n, active=loss_mask.reshape(-1) != 0,
+        loss_config, logits.reshape(n, -1), target_rows(targets, n, target_row), shift=0, rows=n, active=loss_mask.reshape(-1) != 0,
         target_row=target_row, tv_out=tv_out,
     )
     loss = torch.zeros((), device=logits.device, dtype=torch.float32)

@@ -14,7 +14,7 @@ import torch
 from torch.nn.functional import binary_cross_entropy_with_logits
 
 from speculators_b200.losses import LossConfig, tv_loss
-from speculators_b200.models.dflash.metrics import block_decay_fn, weighted_terms
+from speculators_b200.models.dflash.metrics import block_decay_fn, target_rows, weighted_terms
 from speculators_b200.models.metrics import compute_accuracy_multi_step
 from speculators_b200.ops import fused_row_loss
 
@@ -49,7 +49,7 @@ def compute_metrics(logits, targets, confidence_logits, loss_mask, block_size: i
         if tv:
             accept = 1.0 - tv[0].unsqueeze(0)
         elif tv is not None:
-            accept = 1.0 - fused_row_loss("tv", logits.detach().reshape(n, -1), targets.reshape(targets.shape[1], -1), rows=n,
+            accept = 1.0 - fused_row_loss("tv", logits.detach().reshape(n, -1), target_rows(targets, n, target_row), rows=n,
                                           active=loss_mask.reshape(-1) != 0, target_row=target_row)[0].unsqueeze(0)
         else:
             accept = 1.0 - tv_loss_fn(logits.detach(), targets if target_row is None else targets[:, target_row.long()])

@@ -104,3 +104,16 @@ def test_skipped_rows_get_no_gradient_whatever_the_upstream_weight():
         row, _, _ = ops.fused_row_loss(op, y, t, active=keep)
         row.sum().backward()
         assert (row[~keep] == 0).all() and (y.grad[~keep] == 0).all()
+
+
+def test_block_metrics_take_targets_without_a_batch_dimension():
+    from speculators_b200.models.dflash.metrics import compute_metrics as dflash_metrics
+    from speculators_b200.models.dspark.metrics import compute_metrics as dspark_metrics
+
+    x, t = _pair(T=8)
+    mask = torch.tensor([[True, True, False, True, True, False, True, True]])
+    config = losses.resolve_loss_config("kl_div")
+    for metrics in (lambda targets: dflash_metrics(x, targets, mask, 4, loss_config=config),
+                    lambda targets: dspark_metrics(x, targets, torch.zeros(1, 8), mask, 4, config)):
+        (want, counters), (got, flat_counters) = metrics(t), metrics(t[0])
+        assert torch.equal(got, want) and all(torch.equal(flat_counters[k], counters[k]) for k in counters)
