@@ -49,7 +49,7 @@ class MarkovHead(nn.Module):
     def prev_embeddings(self, token_ids: torch.Tensor) -> torch.Tensor:
         table, ids = self.markov_w1, token_ids.long()
         if (not hasattr(table.weight, "_flat_grad") or type(table) is not nn.Embedding or not unobserved(table) or table.max_norm is not None
-                or table.sparse or table.scale_grad_by_freq):
+                or table.sparse or table.scale_grad_by_freq or ops.gradient_watched(table.weight)):
             return table(ids)
         # under the training engine: rows of the gradient straight into its buffer, where autograd's own is a table of zeros that is added to it
         return ops.embedding(ids, table.weight, table.padding_idx).view(*ids.shape, -1)

@@ -557,6 +557,13 @@ def _param_grad_target(weight: torch.Tensor, beside: bool = False) -> tuple[torc
     return flat, not fresh, True
 
 
+def gradient_watched(p: torch.Tensor) -> bool:
+    """Whether a hook of the caller's waits for the gradient of ``p`` (the training engine's own does not count): a gradient that
+    goes straight into the flat buffer passes it by."""
+    hooks = (p._backward_hooks or {}).values()  # noqa: SLF001
+    return any(not getattr(h, "of_engine", False) for h in hooks) or bool(getattr(p, "_post_accumulate_grad_hooks", None))
+
+
 def clear_fresh_grad(p: torch.Tensor) -> None:
     """Zero what no gradient has been stored into since the engine's ``zero_grad``: all of the flat view
     (``_grad_fresh`` is ``True``) or the row intervals that ``_row_grad_target`` has left."""

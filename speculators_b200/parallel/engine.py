@@ -400,6 +400,7 @@ class TrainEngine:
                 ops.clear_fresh_grad(ref())
                 return g
 
+            on_grad.of_engine = True
             return on_grad
 
         for p in self.params:

@@ -263,3 +263,27 @@ def test_dflash_family_parity_with_reference(algo, tiny_verifier_dir, tiny_vocab
 def test_mtp_step_weights():
     w = compute_step_weights(0.6, 3)
     assert abs(sum(w) - 1) < 1e-9 and abs(w[1] / w[0] - 0.6) < 1e-9
+
+
+@pytest.mark.parametrize("kind", [None, "register_hook", "register_post_accumulate_grad_hook", "register_forward_hook"])
+def test_a_hook_on_the_markov_table_gets_its_gradient(kind, monkeypatch):
+    """Under the training engine the table's gradient goes past autograd, but only where nobody waits for it."""
+    from speculators_b200.models.dspark import model_definitions
+
+    head = model_definitions.MarkovHead(verifier_vocab_size=16, draft_vocab_size=16, markov_rank=8, hidden_size=8)
+    table = head.markov_w1
+    table.weight._flat_grad = torch.zeros_like(table.weight)
+
+    def of_engine(g):
+        return g
+
+    of_engine.of_engine = True
+    table.weight.register_hook(of_engine)
+    seen, direct = [], []
+    monkeypatch.setattr(model_definitions.ops, "embedding", lambda ids, w, pad: direct.append(1) or torch.nn.functional.embedding(ids, w, pad))
+    if kind == "register_forward_hook":
+        table.register_forward_hook(lambda m, i, o: seen.append(1))
+    elif kind is not None:
+        getattr(table.weight, kind)(lambda g: seen.append(1))
+    head.prev_embeddings(torch.tensor([[1, 2], [3, 1]])).sum().backward()
+    assert (direct, seen) == (([1], []) if kind is None else ([], [1]))
