@@ -28,7 +28,7 @@ from speculators_b200.models.dflash.metrics import compute_metrics
 from speculators_b200.models.dflash.model_definitions import DFlashDecoderLayer
 from speculators_b200.models.dflash.utils import get_base_indices_for_anchored_blocks, select_anchors
 from speculators_b200.models.eagle3.attention import causal_document_interval
-from speculators_b200.models.layers import Linear, RMSNorm, RotaryTable
+from speculators_b200.models.layers import Linear, RMSNorm, RotaryTable, unobserved
 from speculators_b200.models.utils import resolve_target_layer_ids
 from speculators_b200.proposals.greedy import GreedyTokenProposalConfig
 
@@ -124,8 +124,10 @@ class DFlashDraftModel(DraftVocabMixin, SpeculatorModel):
         all_positions = torch.cat([positions, noise_positions])
         with torch.no_grad():
             vl = verifier_last_hidden_states.reshape(T, -1).to(dtype)
-            # slots share rows of the sequence: the verifier's head runs over whichever are fewer (8B, 8192 slots of 4096 rows: 0.8 ms less)
-            target_row = target_index.to(torch.int32) if vl.is_cuda and T < target_index.numel() else None
+            # slots share rows of the sequence: the verifier's head runs over whichever are fewer (8B, 8192 slots of 4096 rows: 0.8 ms less);
+            # who watches the norm, or has put another in its place, gets the slots
+            shared = vl.is_cuda and T < target_index.numel() and unobserved(self.verifier_norm)
+            target_row = target_index.to(torch.int32) if shared else None
             targets = ops.linear(self.verifier_norm(vl if target_row is not None else vl[target_index]), self.verifier_lm_head.weight)
         for li, layer in enumerate(self.layers):
             spec = win_spec if li in self.sliding_window_indices else full_spec

@@ -80,6 +80,22 @@ def test_gpu_loss_matches_cpu_fp32(algo, head_dim, tmp_path):
     assert all(torch.isfinite(v).all() for v in metrics.values() if torch.is_tensor(v))
 
 
+@pytest.mark.parametrize("algo", ["dflash", "dspark"])
+def test_a_hook_on_the_verifier_norm_sees_the_slots(algo, tmp_path):
+    model, kwargs = _build(algo, tmp_path, 128)
+    model.to("cuda", torch.bfloat16)
+    batch = {k: v.cuda() for k, v in _batch().items()}
+    assert kwargs["max_anchors"] * 8 > batch["input_ids"].shape[1]  # more slots than rows: by themselves they would share targets
+    torch.manual_seed(3)
+    _, want, _ = model(**batch, **kwargs)
+    seen = []
+    model.verifier_norm.register_forward_hook(lambda m, i, o: seen.append((i[0].shape, o.shape)))
+    torch.manual_seed(3)
+    _, loss, _ = model(**batch, **kwargs)
+    slots = torch.Size((kwargs["max_anchors"] * 8, HIDDEN))
+    assert seen == [(slots, slots)] and torch.equal(loss, want)
+
+
 @pytest.mark.parametrize("algo", ["dflash", "dspark", "peagle"])
 def test_cuda_graph_steps(algo, tmp_path, monkeypatch):
     # P-EAGLE's step is graph-capturable only with the fixed-shape COD sampler (opt-in)
