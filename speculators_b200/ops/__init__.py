@@ -682,7 +682,7 @@ def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float, centred: bool = 
 def add_rms_norm(x: torch.Tensor, add: torch.Tensor, weight: torch.Tensor, eps: float) -> tuple[torch.Tensor, torch.Tensor]:
     """``(x + add, rms_norm(x + add))``, in one launch where no gradient is asked for."""
     if (_norm_native(x) and not torch.is_grad_enabled() and x.dim() == 2 and x.shape[1] > 256 and add.shape == x.shape and add.dtype == x.dtype
-            and weight.dtype == x.dtype and all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (x, add, weight))
+            and weight.dtype == x.dtype and all(t.device == x.device and t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (x, add, weight))
             and torch.autograd.forward_ad._current_level < 0):
         return native().add_rmsnorm_fwd(x, add, weight, eps)
     x = x + add

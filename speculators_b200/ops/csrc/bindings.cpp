@@ -132,6 +132,11 @@ void check_rows(const Tensor& t, const char* name) {
               " rows must be 16-byte aligned");
 }
 
+// Operands that plain operators would have refused to combine.
+void check_same_device(const Tensor& t, std::initializer_list<const Tensor*> others) {
+  for (const Tensor* o : others) TORCH_CHECK(o->device() == t.device(), "expected tensors on one device, got ", t.device(), " and ", o->device());
+}
+
 // rows_used (optional int32[1] on the device): rows past it are left alone.
 const int* used_rows(const c10::optional<Tensor>& rows_used) {
   if (!rows_used.has_value()) return nullptr;
@@ -236,6 +241,7 @@ std::tuple<Tensor, Tensor> add_rmsnorm_fwd(const Tensor& x, const Tensor& add, c
   for (const Tensor* t : std::initializer_list<const Tensor*>{&x, &add})
     TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kBFloat16 && t->dim() == 2 && t->is_contiguous() && (reinterpret_cast<uintptr_t>(t->data_ptr()) & 15) == 0,
                 "add_rmsnorm_fwd: contiguous bf16 [rows, H] expected");
+  check_same_device(x, {&add, &w});
   const int64_t H = x.size(1);
   TORCH_CHECK(add.sizes() == x.sizes() && H % 8 == 0 && H > 256 && H <= 32768, "add_rmsnorm_fwd: shapes");
   TORCH_CHECK(w.is_cuda() && w.scalar_type() == at::kBFloat16 && w.is_contiguous() && w.numel() == H && (reinterpret_cast<uintptr_t>(w.data_ptr()) & 15) == 0);
@@ -398,6 +404,7 @@ std::tuple<Tensor, Tensor> select_anchors(const Tensor& mask, const Tensor& keys
   const int64_t T = mask.numel();
   const bool* m = bool_ptr(mask, T, "mask");
   TORCH_CHECK(keys.is_cuda() && keys.scalar_type() == at::kFloat && keys.is_contiguous() && keys.numel() == T, "select_anchors: a float32 key per row expected");
+  check_same_device(mask, {&keys});
   TORCH_CHECK(slots >= 0 && block > 0 && T < (int64_t(1) << 31) - 65536 && slots < (int64_t(1) << 31) - 65536);
   c10::cuda::CUDAGuard guard(mask.device());
   Tensor anchors = at::empty({slots}, mask.options().dtype(at::kLong)), picked = at::empty({slots}, mask.options());
@@ -410,6 +417,7 @@ std::tuple<Tensor, Tensor, Tensor> anchor_spec(const Tensor& doc, const Tensor& 
   const int64_t T = doc.numel(), n = anchors.numel();
   const int64_t *d = long_ptr(doc, "document_ids"), *a = long_ptr(anchors, "anchors");
   TORCH_CHECK(doc_lo.is_cuda() && doc_lo.scalar_type() == at::kInt && doc_lo.is_contiguous() && doc_lo.numel() == T, "doc_lo: int32 per row expected");
+  check_same_device(doc, {&doc_lo, &anchors});
   TORCH_CHECK(block > 0 && n * block * block < (int64_t(1) << 31) * 64 && n * block < (int64_t(1) << 31));
   c10::cuda::CUDAGuard guard(doc.device());
   auto opt = doc_lo.options();
@@ -424,6 +432,7 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> anchor_slots(const Tensor& an
   const int64_t T = mask.numel(), n = anchors.numel(), N = n * block;
   const int64_t *a = long_ptr(anchors, "anchors"), *i = long_ptr(ids, "ids"), *pos = long_ptr(positions, "positions");
   const bool *pk = bool_ptr(picked, n, "picked"), *m = bool_ptr(mask, T, "mask");
+  check_same_device(anchors, {&picked, &ids, &positions, &mask});
   TORCH_CHECK(ids.numel() == T && positions.numel() == T && T > 0 && block > 0 && N < (int64_t(1) << 31));
   c10::cuda::CUDAGuard guard(anchors.device());
   Tensor of = at::empty({4, N}, anchors.options()), counts = at::empty({N}, mask.options());
@@ -1511,6 +1520,8 @@ std::vector<Tensor> decoder_layer_fwd(const Tensor& h, const c10::optional<Tenso
     return {};
   if (heads && (!w_k.has_value() || !dense(*w_q, {hd}) || !dense(*w_k, {hd}))) return {};
   if (positions.scalar_type() != at::kLong || !positions.is_contiguous() || positions.numel() != T) return {};
+  for (const Tensor* t : std::initializer_list<const Tensor*>{&positions, &cos_t, &sin_t, &lo, &hi})
+    if (t->device() != h.device()) return {};
   c10::cuda::CUDAGuard guard(h.device());
   const c10::optional<Tensor> none;
   auto product = [&](const Tensor& x, const Tensor& w) {

@@ -164,3 +164,16 @@ def test_only_layers_of_plain_modules_are_one_call():
         assert not layers._of_one_call(layer, None), path
     assert not layers._of_one_call(fresh(), ZeroCenteredRMSNorm(CFG["hidden_size"]))
     assert not layers._of_one_call(fresh(), torch.nn.RMSNorm(CFG["hidden_size"]))
+
+
+def test_a_sum_of_two_devices_is_refused(monkeypatch):
+    from speculators_b200 import ops
+
+    def native():
+        raise AssertionError("a kernel would read one device's memory on another")
+
+    monkeypatch.setattr(ops, "_norm_native", lambda x: True)
+    monkeypatch.setattr(ops, "native", native)
+    x = torch.zeros(2, 512, dtype=torch.bfloat16)
+    with torch.no_grad(), pytest.raises(RuntimeError, match="device"):
+        ops.add_rms_norm(x, torch.zeros_like(x, device="meta"), torch.ones(512, dtype=torch.bfloat16), 1e-6)
