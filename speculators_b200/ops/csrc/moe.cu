@@ -25,7 +25,8 @@ constexpr int kMaxExperts = 1024;
 
 // The k largest of a row's values, descending, equal ones by index (NaN counts as the largest, as torch.topk has it).  A warp a
 // row, PER values a lane in registers as keys that order like the values; k rounds of a warp-wide maximum.  Bound by the rounds'
-// shuffles: 4092 rows of 256, 10 of them, 7 us; a top-k and its sort took 74.
+// shuffles: 4092 rows of 256, 10 of them, 7 us; a top-k and its sort took 74.  The routing does not call it: equal probabilities are
+// common there and keep the order that torch.topk gives them.
 template <int PER>
 __global__ void __launch_bounds__(256) topk_rows_kernel(const float* __restrict__ p, int rows, int E, int k, int64_t* __restrict__ index) {
   pdl_begin();
