@@ -933,12 +933,10 @@ def _newton_schulz(g: torch.Tensor, steps: int, normalise: bool = True) -> torch
     return x.to(g.dtype)
 
 
-# Short side from which on the polynomial is rounded once, and sides' ratio from which on two of its iterations share a Gram matrix
-# (us, five iterations, sums rounded on their own and now: 2048 x 2048 345 and 314, 3072 x 4096 792 and 708, 2048 x 6144 572 and 471,
-# 2048 x 8192 711 and 551, 16384 x 2048 952 and 706, 4096 x 12288 2452 and 2131, 28672 x 4096 5623 and 3779).  In pairs 1024 x 2048
-# took what it did one by one.  Stacks of a short side of 1024 would gain as much (5 x 6144 x 1024 706 and 485): see below.
+# Short side from which on the polynomial is rounded once (us, five iterations, sums rounded on their own and once: 2048 x 2048 378 and
+# 339, 3072 x 4096 796 and 716, 2048 x 6144 557 and 514, 2048 x 8192 754 and 669, 16384 x 2048 964 and 919, 4096 x 12288 2370 and 2350, 28672 x
+# 4096 5190 and 5140).  Stacks of a short side of 1024 keep the bits that they had: see below.
 _NS_ONCE_FROM = 2048
-_NS_PAIRS_FROM = 2.5
 
 
 def _newton_schulz_stack(x: torch.Tensor, y: torch.Tensor, steps: int) -> None:
@@ -946,45 +944,29 @@ def _newton_schulz_stack(x: torch.Tensor, y: torch.Tensor, steps: int) -> None:
     ``y``: the result is in ``y`` after an odd number of steps, else in ``x``.  The Gram matrix and its square, being symmetric,
     are computed on and above the diagonal only.
 
-    Wide matrices: one iteration is ``X <- P(G) X`` with ``P = a I + b G + c G^2`` formed in the epilogue of ``G^2`` and rounded
-    once.  ``P`` and ``G`` commute, so the next iteration's Gram matrix is ``P^2 G``: where the sides differ enough, two iterations
-    share one, as ``X <- P' P X``, ``3 m^2 n + 5 m^3`` FLOPs for two instead of ``6 m^2 n + 2 m^3``, m the short side.  No more
-    than two: ``G`` holds the squares of the singular values, and what bf16 leaves of the small ones does not survive a third.
+    Wide matrices: one iteration is ``X <- P(G) X`` with ``P = a I + b G + c G^2`` formed in fp32 in the epilogue of ``G^2`` and rounded
+    once.  (``P`` and ``G`` commute, so the next iteration's Gram matrix is ``P^2 G``.  Two iterations on one Gram matrix take less time
+    but round that to bf16, and what this leaves of the small singular values can be half as far off again as in the form below:
+    2048 x 8192, one in sixteen at 1 and the rest at 0.2, 0.030 where that form has 0.021 and this one 0.013.)
 
     Narrow ones form ``b G + c G^2`` and ``a X + X P`` in the products' epilogues, rounded like the single-matrix form: the drafts
     of several narrow layers (DSpark) amplify the last bits of an update up to the size of their gradients, so they keep those bits.
 
     Relative error against the same polynomial in fp64, five steps, Gaussian entries and spread over two and four decades, sums rounded
-    on their own and now: 2048 x 8192 0.018, 0.029, 0.048 and 0.009, 0.016, 0.025; 28672 x 4096 0.019, 0.024, 0.040 and
-    0.011, 0.013, 0.020; 3072 x 4096 0.017, 0.024, 0.039 and 0.008, 0.016, 0.026."""
+    on their own and once: 2048 x 8192 0.018, 0.028, 0.048 and 0.007, 0.018, 0.031; 4096 x 14336 0.019, 0.023, 0.039 and
+    0.009, 0.016, 0.025; 3072 x 4096 0.017, 0.021, 0.038 and 0.008, 0.014, 0.025.  None of eighteen more spectra, of two levels among them, is
+    further off once rounded."""
     a, b, c = 3.4445, -4.7750, 2.0315
     batch, rows, cols = x.shape
     tall = rows > cols
-    short, long = min(rows, cols), max(rows, cols)
+    short = min(rows, cols)
     nat, status = ops.native(), ops.gemm_status(x.device)
     once = short >= _NS_ONCE_FROM
-    # pairs of iterations come in twos, so that the result ends where it is expected
-    pairs = steps // 4 * 2 if once and long >= _NS_PAIRS_FROM * short else 0
-    spare = [torch.empty((batch, short, short), dtype=x.dtype, device=x.device) for _ in range(4 if pairs else 2)]
+    gram, poly = (torch.empty((batch, short, short), dtype=x.dtype, device=x.device) for _ in range(2))
     src, dst = x, y
-
-    def polynomial(gram, out):
-        nat.gemm_stack(gram, gram, out, gram, False, False, c, b, True, status, a if once else None)
-
-    def product(left, right, out):  # of symmetric matrices that commute
-        nat.gemm_stack(left, right, out, None, False, False, 1.0, 0.0, True, status)
-
-    for i in range(steps - pairs):
-        gram, poly = spare[:2]
+    for _ in range(steps):
         nat.gemm_stack(src, src, gram, None, tall, tall, 1.0, 0.0, True, status)
-        polynomial(gram, poly)
-        if i < pairs:
-            other, last = spare[2:]
-            product(poly, gram, other)
-            product(poly, other, gram)  # P^2 G
-            polynomial(gram, other)
-            product(other, poly, last)
-            poly = last
+        nat.gemm_stack(gram, gram, poly, gram, False, False, c, b, True, status, a if once else None)
         left, right = (src, poly) if tall else (poly, src)  # symmetric poly: either orientation of it is the same
         nat.gemm_stack(left, right, dst, None if once else src, False, not tall, 1.0, 0.0 if once else a, False, status)
         src, dst = dst, src

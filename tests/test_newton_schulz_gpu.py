@@ -47,3 +47,24 @@ def test_diagonal_is_added_before_the_one_rounding():
     ops.native().gemm_stack(x, x, out, x, False, False, 0.5, -1.5, False, status, 2.25)
     want = 0.5 * x.double() @ x.double().mT - 1.5 * x.double() + 2.25 * torch.eye(264, device="cuda", dtype=torch.float64)
     assert float(((out.double() - want).abs() / want.abs().clamp(min=1e-2)).max()) <= 2**-8 and int(status) == 0
+
+
+@pytest.mark.parametrize("rows,cols", [(2048, 6144), (8192, 2048), (3072, 4096)])
+@pytest.mark.parametrize("share,low", [(0.1, 0.1), (1 / 16, 0.2), (0.5, 0.5)])
+def test_wide_stacks_are_no_further_off_than_with_sums_rounded_on_their_own(rows, cols, share, low, monkeypatch):
+    """A share of the singular values at one, the others lower."""
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    short, long = min(rows, cols), max(rows, cols)
+    u, v = (torch.linalg.qr(torch.randn(n, short, generator=g, device="cuda", dtype=torch.float64))[0] for n in (short, long))
+    x = (u * torch.where(torch.arange(short, device="cuda") < share * short, 1.0, low)) @ v.mT
+    x = ((x if rows < cols else x.mT) / x.norm()).bfloat16()[None].contiguous()
+    want = _exact(x, 5)
+
+    def off():
+        work, other = x.clone(), torch.empty_like(x)
+        engine._newton_schulz_stack(work, other, 5)
+        return float((other.double() - want).norm() / want.norm())
+
+    now = off()
+    monkeypatch.setattr(engine, "_NS_ONCE_FROM", 1 << 30)
+    assert now <= off()
