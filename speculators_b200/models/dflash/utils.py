@@ -30,7 +30,7 @@ def select_anchors(loss_mask: torch.Tensor, num_anchors: int, block_size: int):
         raise ValueError(f"Expected [B, T], got {loss_mask.shape}")
     if block_size <= 0:
         raise ValueError(f"Expected block size > 0, got {block_size}")
-    if loss_mask.is_cuda:  # one launch
+    if loss_mask.is_cuda and torch.get_default_dtype() == torch.float32:  # one launch; keys of another type are compared below
         return ops.native().select_anchors(loss_mask[0].bool().contiguous(), torch.rand(loss_mask.shape[1], device=loss_mask.device), num_anchors, block_size)
     valid = loss_mask[0].bool().clone()
     valid[-block_size:] = False

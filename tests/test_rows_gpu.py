@@ -170,3 +170,17 @@ def test_anchor_specs_and_slots_match_their_definition(window, non_causal, block
         want = token, (positions[anchors][:, None] + torch.arange(block)).reshape(-1), index, (index if from_anchor else index - 1) % T, counts
         got = ops.native().anchor_slots(anchors.cuda(), picked.cuda(), ids.cuda(), positions.cuda(), mask.cuda(), block, mask_token, from_anchor)
         assert all(torch.equal(a.cpu(), b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float64])
+def test_anchors_are_chosen_under_another_default_type(dtype):
+    from speculators_b200.models.dflash.utils import select_anchors
+
+    mask = torch.zeros(1, 50, dtype=torch.bool, device="cuda")
+    mask[0, [3, 7, 30, 45]] = True
+    torch.set_default_dtype(dtype)
+    try:
+        anchors, picked = select_anchors(mask, 5, 8)
+    finally:
+        torch.set_default_dtype(torch.float32)
+    assert anchors.tolist() == [3, 7, 30, 0, 0] and picked.tolist() == [True] * 3 + [False] * 2
