@@ -29,7 +29,7 @@ def anchor_block_attn_spec(document_ids, anchor_positions, block_size: int, slid
     causal_in_block = sliding_window is not None and not sliding_window_non_causal
     if doc_lo is None:
         doc_lo, _ = causal_document_interval(doc, None)
-    if doc.is_cuda and doc.dtype == torch.int64:  # one launch
+    if doc.is_cuda and doc.dtype == torch.int64 and (sliding_window is None or sliding_window >= 0):  # one launch
         lo, hi, extra = ops.native().anchor_spec(doc.contiguous(), doc_lo, a.contiguous(), int(block_size), -1 if sliding_window is None else int(sliding_window),
                                                  causal_in_block)
         return AttnSpec(lo=lo, hi=hi, extra_idx=extra, extra_block=int(block_size), extra_block_causal=bool(causal_in_block))

@@ -184,3 +184,15 @@ def test_anchors_are_chosen_under_another_default_type(dtype):
     finally:
         torch.set_default_dtype(torch.float32)
     assert anchors.tolist() == [3, 7, 30, 0, 0] and picked.tolist() == [True] * 3 + [False] * 2
+
+
+@pytest.mark.parametrize("window", [0, 1, -1, -3, 2**40])
+@pytest.mark.parametrize("non_causal", [False, True])
+def test_anchor_specs_of_any_window(window, non_causal):
+    from speculators_b200.models.dflash.attention import anchor_block_attn_spec
+
+    doc, anchors = torch.tensor([0] * 20 + [1] * 31 + [-1] * 10), torch.tensor([0, 3, 19, 20, 50, 55])
+    want = anchor_block_attn_spec(doc, anchors, 4, window, non_causal)
+    got = anchor_block_attn_spec(doc.cuda(), anchors.cuda(), 4, window, non_causal)
+    for a, b in ((got.lo, want.lo), (got.hi, want.hi), (got.extra_idx, want.extra_idx)):
+        assert torch.equal(a.cpu(), b)
