@@ -18,6 +18,11 @@ from speculators_b200 import ops
 
 __all__ = ["get_base_indices_for_anchored_blocks", "select_anchors"]
 
+# Longest row whose anchors one block chooses.  It passes over the row six times or more, which top-k and sort share among many (us, 64
+# and 3072 anchors among 90 % of the rows, one block and the launches below: 3000 rows 15 and 100, 13 and 150; 32768 38 and 157, 42
+# and 198; 65536 90 and 160, 95 and 204; 131072 191 and 158, 198 and 211; 1048576 1420 and 258, 1440 and 307).
+_ONE_BLOCK_ROWS = 65536
+
 
 def get_base_indices_for_anchored_blocks(anchor_positions: torch.Tensor, block_size: int) -> torch.Tensor:
     """``[num_anchors] -> [num_anchors * block_size]``: anchor, anchor+1, ..."""
@@ -30,7 +35,8 @@ def select_anchors(loss_mask: torch.Tensor, num_anchors: int, block_size: int):
         raise ValueError(f"Expected [B, T], got {loss_mask.shape}")
     if block_size <= 0:
         raise ValueError(f"Expected block size > 0, got {block_size}")
-    if loss_mask.is_cuda and torch.get_default_dtype() == torch.float32:  # one launch; keys of another type are compared below
+    # one launch (keys of another type are compared below)
+    if loss_mask.is_cuda and loss_mask.shape[1] <= _ONE_BLOCK_ROWS and torch.get_default_dtype() == torch.float32:
         return ops.native().select_anchors(loss_mask[0].bool().contiguous(), torch.rand(loss_mask.shape[1], device=loss_mask.device), num_anchors, block_size)
     valid = loss_mask[0].bool().clone()
     valid[-block_size:] = False

@@ -196,3 +196,20 @@ def test_anchor_specs_of_any_window(window, non_causal):
     got = anchor_block_attn_spec(doc.cuda(), anchors.cuda(), 4, window, non_causal)
     for a, b in ((got.lo, want.lo), (got.hi, want.hi), (got.extra_idx, want.extra_idx)):
         assert torch.equal(a.cpu(), b)
+
+
+@pytest.mark.parametrize("T", [65536, 65537, 140000])
+@pytest.mark.parametrize("density", [0.001, 0.6])
+def test_anchors_of_long_rows(T, density, monkeypatch):
+    from speculators_b200.models.dflash import utils
+
+    mask = torch.rand(1, T, device="cuda") < density
+    if T > 65536:  # one block is no match for a long row
+        monkeypatch.setattr(utils.ops, "native", lambda: pytest.fail("a long row in one block"))
+    torch.manual_seed(T)
+    anchors, picked = utils.select_anchors(mask, 300, 8)
+    torch.manual_seed(T)
+    keys = torch.rand(T, device="cuda").where(mask[0] & (torch.arange(T, device="cuda") < T - 8), 2.0)
+    want = torch.sort(torch.sort(keys, stable=True).indices[: min(300, int((keys < 2).sum()))]).values
+    n = len(want)
+    assert torch.equal(anchors[:n], want) and picked[:n].all() and not picked[n:].any() and not anchors[n:].any()
