@@ -62,7 +62,9 @@ __device__ __forceinline__ float row_sum(float v, float (&scratch)[2][THREADS / 
 template <int NV, int THREADS> constexpr int kFwdBlocks = THREADS == 512 ? 1 : NV == 2 ? 5 : NV == 4 ? 4 : 2;
 
 // ADD: the row is x + add, rounded as a sum of its own would be, kept in `sum` and normalised from registers: a block of a decoder
-// hands its result to the next norm without reading it back, and a launch less (1777 x 4096: 8 + 10 us apart).
+// hands its result to the next norm without reading it back, and a launch less.  Its two reads take the registers that hold the next row
+// otherwise; with that too, rows went through local memory (us: a sum and a norm apart, with the next row, now: 1777 x 4096 21.5, 20.5,
+// 18.5; 8192 x 4096 73, 74, 59; 500 x 8192 15.4, 20.4, 14.4; 8192 x 8192 128, 170, 105; 8192 x 32768 484, 720, 448).
 struct NormAdd {
   const __nv_bfloat16* add;
   __nv_bfloat16* sum;
@@ -77,7 +79,7 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
   rows = live_rows(live, rows);
   __shared__ float scratch[2][THREADS / 32];
   const int nvec = H >> 3;
-  bf16x8 cur[NV], next[NV], cur_add[ADD ? NV : 1], next_add[ADD ? NV : 1];
+  bf16x8 cur[NV], next[ADD ? 1 : NV], cur_add[ADD ? NV : 1];
   bool ok = false, next_ok = false;  // false only in the debug build
   auto fetch = [&](int r, bf16x8 (&to)[NV], bf16x8 (&to_add)[ADD ? NV : 1]) -> bool {
     const int64_t src = row_index ? row_index[r] : (int64_t)r;
@@ -92,10 +94,12 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
     return true;
   };
   int r = blockIdx.x, slot = 0;
-  if (r < rows) ok = fetch(r, cur, cur_add);
+  if (!ADD && r < rows) ok = fetch(r, cur, cur_add);
   for (; r < rows; r += gridDim.x, slot ^= 1) {
-    if (r + (int)gridDim.x < rows) next_ok = fetch(r + gridDim.x, next, next_add);  // in flight during this row's reduction
-    if (ADD) {
+    if constexpr (!ADD) {
+      if (r + (int)gridDim.x < rows) next_ok = fetch(r + gridDim.x, next, cur_add);  // in flight during this row's reduction
+    } else {
+      ok = fetch(r, cur, cur_add);
 #pragma unroll
       for (int i = 0; i < NV; ++i) {
         const int v = threadIdx.x + i * THREADS;
@@ -108,7 +112,6 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
           cur[i] = pack8(a);
           st8(ad.sum + (int64_t)r * H + (v << 3), cur[i]);
         }
-        cur_add[ADD ? i : 0] = next_add[ADD ? i : 0];
       }
     }
     float ss = 0.f;
@@ -137,9 +140,9 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
         for (int j = 0; j < 8; ++j) o[j] = nw.apply(xv[j] * rstd, wv[j]);
         st8(yr + (v << 3), pack8(o));
       }
-      cur[i] = next[i];
+      if (!ADD) cur[i] = next[ADD ? 0 : i];
     }
-    ok = next_ok;
+    if (!ADD) ok = next_ok;
   }
 }
 
