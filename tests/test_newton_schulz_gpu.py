@@ -68,3 +68,18 @@ def test_wide_stacks_are_no_further_off_than_with_sums_rounded_on_their_own(rows
     now = off()
     monkeypatch.setattr(engine, "_NS_ONCE_FROM", 1 << 30)
     assert now <= off()
+
+
+@pytest.mark.parametrize("batch,n", [(1, 2048), (2, 2048), (1, 2056), (1, 3072)])
+def test_symmetric_polynomial_on_pair_tiles(batch, n):
+    """Sizes that take tiles of 256 x 256: addends a tile ahead, mirrored stores, a diagonal in both halves, at 3072 divided tiles."""
+    g = torch.Generator(device="cuda").manual_seed(n + batch)
+    x = torch.randn(batch, n, n, generator=g, device="cuda") * 0.02
+    x = (x + x.mT).bfloat16()
+    out, status = torch.empty_like(x), ops.gemm_status(x.device)
+    ops.native().gemm_stack(x, x, out, x, False, False, 2.0315, -4.7750, True, status, 3.4445)
+    eye = 3.4445 * torch.eye(n, device="cuda", dtype=torch.float64)
+    want = 2.0315 * x.double() @ x.double() - 4.7750 * x.double() + eye
+    size = 2.0315 * x.double().abs() @ x.double().abs() + 4.7750 * x.double().abs() + eye
+    # one rounding to bf16, and n terms added in fp32
+    assert ((out.double() - want).abs() <= 2.0**-8 * want.abs() + n * 2.0**-24 * size).all() and int(status) == 0
