@@ -274,10 +274,14 @@ __device__ __forceinline__ void bf16_round2(float& a, float& b) {
 struct Scaling {
   float alpha, beta, diagonal;
   int once;
-  __device__ __forceinline__ explicit Scaling(const Params& p) : alpha(p.alpha), beta(p.beta), diagonal(p.diagonal), once(p.once) {}
-  // (the plain epilogue skips the arithmetic as a whole: the conditions are uniform)
+  bool plain;
+  __device__ __forceinline__ explicit Scaling(const Params& p)
+      : alpha(p.alpha), beta(p.beta), diagonal(p.diagonal), once(p.once), plain(!p.once && p.alpha == 1.f && p.beta == 1.f) {}
+  // (the plain epilogue skips the arithmetic as a whole behind one uniform test each: with the other forms' tests in between split
+  // products took 1 to 2 % more, 2048 x 1024 x 3072 with a residual 22.7 us instead of 22.2)
   template <int N>
   __device__ __forceinline__ void product(float (&f)[N], int row, int col) const {  // N columns from col on
+    if (plain) return;
     if (once) {
 #pragma unroll
       for (int j = 0; j < N; ++j) f[j] *= alpha;
@@ -298,6 +302,11 @@ struct Scaling {
   }
   template <int N>
   __device__ __forceinline__ void add(float (&f)[N], const float (&o)[N]) const {
+    if (plain) {
+#pragma unroll
+      for (int j = 0; j < N; ++j) f[j] += o[j];
+      return;
+    }
     if (once) {
 #pragma unroll
       for (int j = 0; j < N; ++j) f[j] = fmaf(beta, o[j], f[j]);
@@ -720,7 +729,7 @@ template <int W, typename Ahead = NothingAhead>
 __device__ __forceinline__ void store_accumulator_staged(const Params& p, const Scaling& sc, const CUtensorMap* map_c, const CUtensorMap* map_t, uint32_t stage,
                                                          uint32_t taddr, int row0, int n0, int z, RowPrefetch<W>& pre, bool live, bool mirror, bool zero,
                                                          int lane, const Ahead& ahead = Ahead()) {
-  const bool scaled = sc.alpha != 1.f || sc.beta != 1.f || sc.once;
+  const bool scaled = !sc.plain;
   if (p.epilogue == kStore && !scaled) store_accumulator_staged_as<W, false, false>(sc, map_c, map_t, stage, taddr, row0, n0, p.N, z, pre, live, mirror, zero, lane, ahead);
   else if (p.epilogue == kStore) store_accumulator_staged_as<W, false, true>(sc, map_c, map_t, stage, taddr, row0, n0, p.N, z, pre, live, mirror, zero, lane, ahead);
   else if (!scaled) store_accumulator_staged_as<W, true, false>(sc, map_c, map_t, stage, taddr, row0, n0, p.N, z, pre, live, mirror, zero, lane, ahead);
