@@ -626,7 +626,6 @@ Tensor gate_mul_bwd(const Tensor& dy, const Tensor& out, const Tensor& gate, Ten
 }
 
 // ---- mixture-of-experts row movement ---------------------------------------------------------------
-// expert int64[T, k] -> (seg int32[E + 1], 256-row tile prefix int32[E + 1], slot_row int32[T * k], row_slot int32[capacity]).
 // columns of the k largest of every row, descending, equal ones by column: fp32 [rows, E <= 1024] -> int64 [rows, k]
 Tensor topk_rows(const Tensor& p, int64_t k) {
   TORCH_CHECK(p.is_cuda() && p.scalar_type() == at::kFloat && p.dim() == 2 && p.is_contiguous() && p.size(1) <= 1024 && k >= 1 && k <= p.size(1), "topk_rows");
@@ -636,6 +635,7 @@ Tensor topk_rows(const Tensor& p, int64_t k) {
   TORCH_CHECK(rc == 0, "topk_rows launch failed (", rc, ")");
   return index;
 }
+// expert int64[T, k] -> (seg int32[E + 1], 256-row tile prefix int32[E + 1], slot_row int32[T * k], row_slot int32[capacity]).
 std::tuple<Tensor, Tensor, Tensor, Tensor> moe_plan(const Tensor& expert, int64_t E, int64_t capacity, int64_t k, const c10::optional<Tensor>& live) {
   TORCH_CHECK(k >= 1 && expert.numel() % k == 0, "moe_plan: k slots per token");
   TORCH_CHECK(expert.is_cuda() && expert.scalar_type() == at::kLong && expert.is_contiguous() && expert.numel() > 0);

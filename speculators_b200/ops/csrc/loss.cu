@@ -18,7 +18,6 @@
 // steps of EAGLE-3 align their targets) and both argmaxes are by-products, so the
 // accuracy metrics need no extra pass over the vocabulary.
 #include "common.cuh"
-#include "loss_stats.cuh"
 #include "packed_f32.cuh"
 
 namespace sb200 {
@@ -30,7 +29,7 @@ constexpr int kNumStats = 5;  // m_d, z_d, m_t, z_t, per-op extra
 
 // One thread's share of a row: running maximum, sum of exponentials against it, and the column where the vector of eight starts
 // that brought the maximum (which of the eight is looked up once a row); columns behind the last whole vector on their own.
-// Sums are formed in the order of the columns, eight at a time, as online_update forms them.
+// Sums are formed in the order of the columns, eight at a time, as online_update (loss_stats.cuh) forms them.
 struct Share {
   float m = -INFINITY, z = 0.f;
   int col = 0x7fffffff;
@@ -71,7 +70,7 @@ __device__ __forceinline__ void add8(Share& s, const bf16x8& v, int col) {
   }
   s.z = fmaf(s.z, by, add);
 }
-// The target row's, with A = sum_v e^{t_v - m}(t_v - x_v) (see online_update_kl).
+// The target row's, with A = sum_v e^{t_v - m}(t_v - x_v) (see online_update_kl in loss_stats.cuh).
 __device__ __forceinline__ void add8_kl(Share& s, float& A, const bf16x8& tv, const bf16x8& xv, int col) {
   const float by = raise(s, max8(tv), col);
   const float2x minus_m = both(-s.m, -s.m), minus = both(-1.f, -1.f);
@@ -153,7 +152,7 @@ __device__ __forceinline__ int first_max(const Share& s, const __nv_bfloat16* ro
 
 // Bound by issue and the special-function units before memory: an exponential per column and row, and beside it what the maximum,
 // its column and the sums take.  So the maximum comes from packed comparisons, its column is kept per vector of eight and looked up
-// once a row, differences and scalings are packed pairs, and a row takes three barriers (23 before).  Sums keep their order.  The
+// once a row, differences and scalings are packed pairs, and a row takes two to four barriers, by loss (23 before).  Sums keep their order.  The
 // KL divergence does best with three blocks an SM and one vector of each row in flight, the others with two and what registers
 // the compiler likes (us, two vectors and one: KL 4096 x 32000 143 and 130, total variation 168 and 195, labels 2460 x 151936 144 and
 // 175; bounded to 32 registers the labels took 268).  us before and after: KL 1001 x 32000 45.7 and 38.7, 4096 x 32000 159 and 129,

@@ -1,6 +1,6 @@
 // Online-softmax statistics of a logits row (and, for the KL divergence, of the target row with
-// the cross term carried along), shared by the row-loss kernels and by the GEMM epilogue that
-// computes the same statistics tile by tile.
+// the cross term carried along) for the GEMM epilogue that computes them tile by tile.  The row-loss
+// kernels form the same statistics from whole rows, in packed pairs (loss.cu).
 #pragma once
 #include "common.cuh"
 
@@ -54,28 +54,6 @@ __device__ __forceinline__ void online_update_kl(RowStats& s, float& A, const fl
 #pragma unroll
     for (int j = 7; j >= 0; --j)
       if (t[j] == vmax) s.best_idx = col0 + j;
-  }
-}
-
-__device__ __forceinline__ void online_update_kl_scalar(RowStats& s, float& A, float t, float x, int col) {
-  const float m_new = fmaxf(s.m, t);
-  const float e = __expf(t - m_new), resc = __expf(s.m - m_new);
-  s.z = s.z * resc + e;
-  A = A * resc + (e > 0.f ? e * (t - x) : 0.f);
-  s.m = m_new;
-  if (t > s.best) {
-    s.best = t;
-    s.best_idx = col;
-  }
-}
-
-__device__ __forceinline__ void online_update_scalar(RowStats& s, float x, int col) {
-  const float m_new = fmaxf(s.m, x);
-  s.z = s.z * __expf(s.m - m_new) + __expf(x - m_new);
-  s.m = m_new;
-  if (x > s.best) {
-    s.best = x;
-    s.best_idx = col;
   }
 }
 

@@ -758,8 +758,6 @@ int rmsnorm_bwd_partial_rows(int rows, int H, bool with_dx) {
 
 SB200_BOUNDS_READER(read_bounds_norm)
 
-// src_rows: number of rows of `x` (what `row_index` may address).
-// live (optional, device): how many of the rows are in use.
 static int norm_fwd_grid(int rows, int H, int blocks) {
   if (H <= 4096 && rows <= 16 * kNumSM) return rows;
   const int most = blocks * kNumSM, rounds = (rows + most - 1) / most;
@@ -781,6 +779,8 @@ void launch_add_rmsnorm_fwd(const void* x, const void* add, const void* w, void*
 #undef SB200_ADD
 }
 
+// src_rows: number of rows of `x` (what `row_index` may address).
+// live (optional, device): how many of the rows are in use.
 void launch_rmsnorm_fwd(const void* x, const void* w, const int64_t* row_index, void* y,
                         float* rstd, int rows, int H, int64_t x_stride, int64_t y_stride, float eps,
                         int64_t src_rows, int centred, const int* live, cudaStream_t stream) {

@@ -954,7 +954,7 @@ def _newton_schulz_stack(x: torch.Tensor, y: torch.Tensor, steps: int) -> None:
 
     Relative error against the same polynomial in fp64, five steps, Gaussian entries and spread over two and four decades, sums rounded
     on their own and once: 2048 x 8192 0.018, 0.028, 0.048 and 0.007, 0.018, 0.031; 4096 x 14336 0.019, 0.023, 0.039 and
-    0.009, 0.016, 0.025; 3072 x 4096 0.017, 0.021, 0.038 and 0.008, 0.014, 0.025.  None of eighteen more spectra, of two levels among them, is
+    0.009, 0.016, 0.025; 3072 x 4096 0.017, 0.021, 0.038 and 0.008, 0.014, 0.025.  None of nineteen more spectra, of two levels among them, is
     further off once rounded."""
     a, b, c = 3.4445, -4.7750, 2.0315
     batch, rows, cols = x.shape
