@@ -4,8 +4,7 @@ import pytest
 import torch
 
 from speculators_b200 import ops
-from speculators_b200.layer_config import TransformerLayerConfig
-from speculators_b200.models.moe import SparseMoeBlock, expert_forward
+from speculators_b200.models.moe import expert_forward
 from speculators_b200.ops.moe import moe_experts, moe_experts_ok
 
 pytestmark = pytest.mark.gpu
@@ -105,6 +104,9 @@ def test_topk_rows(E, ties):
 
 @pytest.mark.parametrize("E,k", [(16, 4), (256, 10)])
 def test_equal_experts_are_chosen_in_the_order_of_topk(E, k):
+    from speculators_b200.layer_config import TransformerLayerConfig
+    from speculators_b200.models.moe import SparseMoeBlock
+
     cfg = TransformerLayerConfig(hidden_size=256, num_hidden_layers=1, num_attention_heads=4, num_key_value_heads=2, head_dim=64, intermediate_size=256,
                                  vocab_size=512, model_type="qwen3_next", num_experts=E, num_experts_per_tok=k, moe_intermediate_size=128)
     torch.manual_seed(E)
